@@ -75,9 +75,11 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
     uint64_t* v_empty = bars + 7;       // [2]
     uint64_t* s_full = bars + 9;        // [2]
     uint64_t* p_full = bars + 11;       // [2]
-    uint64_t* pv_done = bars + 13;      // [1]
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 14);
-    int* s_meta = reinterpret_cast<int*>(bars + 15);     // [0] sequence, [1] first token, [2] tokens, [3] first K/V row, [4] K/V tiles
+    // [2] P V of the even / odd tiles done.  Two, because a row warp may be two products ahead: it can finish the last softmax
+    // before the product of the tile before has been issued, and one barrier's parity cannot tell that product from its own
+    uint64_t* pv_done = bars + 13;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 15);
+    int* s_meta = reinterpret_cast<int*>(bars + 16);     // [0] sequence, [1] first token, [2] tokens, [3] first K/V row, [4] K/V tiles
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = p.status;
@@ -88,8 +90,8 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
             mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
             mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
             mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128);
+            mbar_init(&pv_done[i], 1);
         }
-        mbar_init(pv_done, 1);
         mbar_init_fence();
         tma_prefetch_desc(&qmap);
         tma_prefetch_desc(&kmap);
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
                         umma_ts(tbase + cO, tbase + cS + st * BK + ks * 8, umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_o,
                                 (j > 0 || ks > 0) ? 1u : 0u);
                     umma_commit(&v_empty[st]);
-                    umma_commit(pv_done);
+                    umma_commit(&pv_done[st]);
                 }
                 __syncwarp();
             }
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
                 // accumulator rows already hold products (j > 0): rescale them when any row of the warp changes reference
                 const bool scale_acc = __any_sync(0xffffffffu, raise && j > 0);
                 if (scale_acc) {
-                    ok = mbar_wait(pv_done, (j - 1) & 1, status) && ok;
+                    ok = mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, status) && ok;
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < D; c0 += 32) {
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
             }
             // ---- epilogue
             if (nblk > 0) {
-                ok = mbar_wait(pv_done, (nblk - 1) & 1, status) && ok;
+                ok = mbar_wait(&pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status) && ok;
                 tc_fence_after();
             }
             const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;

@@ -1,0 +1,46 @@
+"""Sizes at which the size rules of the launches change: short and mid-sized tile lists of the selected-attention kernels
+(the scheduling runs of the backward get shorter with the list), and long rows of K/V tiles of range attention."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from fsa.ops.FSA_topk_sparse_attention import sel_attn_bwd, sel_attn_fwd
+from fsa.ops.range_attention import compressed_attention_core
+from fsa.synthetic import make_cu_seqlens, make_qkv, make_topk_idx
+from oracle.sel_attn_oracle import sel_attn_forward_backward
+
+DEV = "cuda:0"
+
+
+def _close(got, ref, name):
+    err = (got.float().cpu() - ref).abs()
+    scale = max(1.0, float(ref.abs().max()) / 2.0)
+    assert float(err.max()) <= 2e-2 * scale, f"{name}: max-abs {float(err.max()):.3e}"
+    assert float(err.mean()) <= 1e-3 * scale, f"{name}: mean-abs {float(err.mean()):.3e}"
+
+
+@pytest.mark.parametrize("seqlens,Hk,G,T", [([1], 1, 1, 2), ([1100], 1, 2, 16), ([2371, 200], 2, 2, 16), ([1500, 33], 2, 8, 16)])
+def test_scheduling_runs_of_short_lists(seqlens, Hk, G, T):
+    d, bs, N = 128, 64, sum(seqlens)
+    q, k, v, do = make_qkv(N, Hk * G, Hk, d, 300 + N)
+    idx, cu = make_topk_idx(seqlens, Hk, T, bs, 301 + N), make_cu_seqlens(seqlens)
+    ref = sel_attn_forward_backward(q, k, v, do, idx, bs, cu, d ** -0.5)
+    qc, kc, vc, dc, ic, cc = (x.to(DEV) for x in (q, k, v, do, idx, cu))
+    o, lse, ws = sel_attn_fwd(qc, kc, vc, ic, bs, cc, d ** -0.5, check_status=True)
+    grads = sel_attn_bwd(qc, kc, vc, o, lse, dc, ic, bs, cc, d ** -0.5, ws, check_status=True)
+    for name, got, want in zip(("o", "dq", "dk", "dv"), (o, *grads), (ref[0], *ref[2:])):
+        _close(got, want, name)
+
+
+def test_long_rows_are_the_same_every_time():
+    """Row warps run up to two P V products ahead of the tensor core: the last products must be waited for all the same."""
+    N, ks, st = 20011, 32, 16
+    C = (N - ks) // st + 1
+    g = torch.Generator(device=DEV).manual_seed(1)
+    q, k, v = (torch.randn(n, h, 128, device=DEV, generator=g).to(torch.bfloat16) for n, h in ((N, 32), (C, 8), (C, 8)))
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=DEV) for n in (N, C))
+    o0, lse0 = compressed_attention_core(q, k, v, ks, st, cu_q, cu_k, C)
+    for _ in range(4):
+        o, lse = compressed_attention_core(q, k, v, ks, st, cu_q, cu_k, C)
+        assert torch.equal(o, o0) and torch.equal(lse, lse0)
