@@ -143,6 +143,18 @@ static int env_int(const char* name, int dflt) {
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
+// Tiles per scheduling run of the persistent kernels: `most` when there are plenty of tiles, fewer when runs of that length
+// would leave SMs without work or with a last run of their own to wait for -- a run is a serial chain on one SM (a backward
+// tile takes about 2.7 us, so the 128 tiles of a 512-token problem took 86 us in four runs of 32 and take 12 in 128 runs of
+// one).  Four runs per SM keep the imbalance of the last round small; a shorter run costs the backward one more dK / dV slab
+// (64 KB written and read), which is why long lists keep long runs.  A function of the shape alone: forward and backward
+// must cut the same list alike.
+static int sched_run(const SelShape& s, int most) {
+    const int64_t tiles = ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT;
+    const int64_t run = tiles / (4 * 148);
+    return (int)(run < 1 ? 1 : run > most ? most : run);
+}
+
 static int make_shape(int64_t N, int B, int Hq, int Hk, int D, int T, int BK, SelShape* s, int64_t Nk = -1) {
     if (Nk < 0) Nk = N;
     if (N < 0 || B < 0 || Hq <= 0 || Hk <= 0 || T <= 0 || BK <= 0) return FSA_ERR_BAD_ARG;
@@ -161,9 +173,9 @@ static int make_shape(int64_t N, int B, int Hq, int Hk, int D, int T, int BK, Se
     s->C = (int)C;
     s->NC = (int)((N + C - 1) / C);
     if (s->NC < 1) s->NC = 1;
-    // tiles per scheduling run of the backward (FSA_SEL_RUN overrides; read once)
+    // tiles per scheduling run of the backward (FSA_SEL_RUN overrides; read once): see sched_run
     static const int env_run = env_int("FSA_SEL_RUN", 0);
-    s->RB = env_run > 0 ? env_run : 32;
+    s->RB = env_run > 0 ? env_run : sched_run(*s, 32);
     if ((int64_t)s->Hk * s->NBmax >= ((int64_t)1 << 30)) return FSA_ERR_UNSUPPORTED;
     if ((int64_t)s->Hk * s->NBmax * s->NC >= ((int64_t)1 << 31)) return FSA_ERR_UNSUPPORTED;
     if (Hk > 65535) return FSA_ERR_UNSUPPORTED;
@@ -299,7 +311,7 @@ static int sel_fwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
     SelFwdArgs a;
     a.q = q; a.q_sn = q_sn; a.q_sh = q_sh; a.sm_scale = sm_scale;
     static const int env_run = env_int("FSA_SEL_RUN", 0);
-    a.run = env_run;
+    a.run = env_run > 0 ? env_run : sched_run(s, 8);
     a.opart = scratch;
     a.ml = (float2*)((char*)scratch + align_up(prow * D * 2, 1024));
     a.o = o; a.o_sn = o_sn; a.o_sh = o_sh; a.lse = lse;

@@ -891,7 +891,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     p.s = s; p.ix = ix;
     p.scale_log2 = a.sm_scale * 1.4426950408889634f;
     p.opart = (ET*)a.opart; p.ml = a.ml;
-    p.run = a.run > 0 ? a.run : 8;
+    p.run = a.run;
     p.bd = a.bd;
     p.dbg = 0;
 #ifdef FSA_TIMING

@@ -24,7 +24,7 @@ struct SelFwdArgs {
     const void* q;            // used by the unpipelined kernel (arbitrary strides)
     int64_t q_sn, q_sh;
     float sm_scale;
-    int run;                  // tiles per scheduling run; 0 = default
+    int run;                  // tiles per scheduling run
     void* opart;              // [max_tiles * 128, D] input dtype
     float2* ml;               // [Hq, N, T] statistics (capacity max_tiles * 128 pairs)
     void* o;
@@ -47,7 +47,7 @@ struct SelBwdArgs {
     const int* topk_idx;
     const int* cu;
     float sm_scale;
-    int run;           // tiles per scheduling run; 0 = default
+    int run;           // tiles per scheduling run
     // scratch
     float* delta;      // [Hq, N]
     void* dq_part;     // [max_tiles * nsub * 128, D] input dtype
