@@ -298,7 +298,7 @@ static int sel_fwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
 
     SelIndex ix = sel_index_carve(index_ws, s);
     prof_begin(FSA_KERNEL_SEL_INDEX, stream);
-    cudaError_t e = sel_build_index(topk_idx, cu_seqlens, bd, s, ix, index_ws, stream);
+    cudaError_t e = sel_build_index(topk_idx, cu_seqlens, bd, s, ix, stream);
     prof_end(FSA_KERNEL_SEL_INDEX, stream);
     if (e != cudaSuccess) return cuda_fail(e);
 
@@ -464,7 +464,7 @@ int fsa_range_attn_index(const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_
     if (index_ws_bytes < sel_index_bytes(s)) return FSA_ERR_WORKSPACE;
     SelIndex ix = sel_index_carve(index_ws, s);
     prof_begin(FSA_KERNEL_SEL_INDEX, stream);
-    cudaError_t e = sel_build_index(nullptr, cu_seqlens_q, SelBounds{cu_seqlens_k, kv_lo, kv_hi}, s, ix, index_ws, stream);
+    cudaError_t e = sel_build_index(nullptr, cu_seqlens_q, SelBounds{cu_seqlens_k, kv_lo, kv_hi}, s, ix, stream);
     prof_end(FSA_KERNEL_SEL_INDEX, stream);
     if (e != cudaSuccess) return cuda_fail(e);
     return FSA_OK;

@@ -65,8 +65,6 @@ struct SelIndex {
     int* key_cnt;    // [Hk * NBmax]       entries per key
     int* key_tile;   // [Hk * NBmax + 1]   first tile of every key (exclusive scan of ceil(count / TPT))
     int* key_seg;    // [Hk * NBmax + 1]   first segment of every key
-    int* row0;       // [NBmax]            first global K/V row of block gb
-    int* nrow;       // [NBmax]            K/V rows of block gb (the last block of a sequence may be short)
     int4* tile_rec;  // [max_tiles]   per tile {first K/V row of the block, entries | kv head << 8, key, first segment of the key}
     int2* tile_aux;  // [max_tiles]   per tile {first tile of its key, tiles of its key}
     uint32_t* entries;  // [max_tiles * TPT]  packed entries in TILE ORDER: entry e of tile j at j * TPT + e,
@@ -93,7 +91,6 @@ inline int64_t sel_index_bytes(const SelShape& s) {
     b += align_up(HG * s.NC * s.IW * 4, 256);
     b += align_up(HG * 4, 256);
     b += align_up((HG + 1) * 4, 256) * 2;
-    b += align_up((int64_t)s.NBmax * 4, 256) * 2;
     b += align_up(sel_max_tiles(s) * 16, 256);
     b += align_up(sel_max_tiles(s) * 8, 256);
     b += align_up(sel_max_tiles(s) * s.TPT * 4, 256);
@@ -111,18 +108,12 @@ inline SelIndex sel_index_carve(void* ws, const SelShape& s) {
     ix.key_cnt = (int*)p;   p += align_up(HG * 4, 256);
     ix.key_tile = (int*)p;  p += align_up((HG + 1) * 4, 256);
     ix.key_seg = (int*)p;   p += align_up((HG + 1) * 4, 256);
-    ix.row0 = (int*)p;      p += align_up((int64_t)s.NBmax * 4, 256);
-    ix.nrow = (int*)p;      p += align_up((int64_t)s.NBmax * 4, 256);
     ix.tile_rec = (int4*)p; p += align_up(sel_max_tiles(s) * 16, 256);
     ix.tile_aux = (int2*)p; p += align_up(sel_max_tiles(s) * 8, 256);
     ix.entries = (uint32_t*)p; p += align_up(sel_max_tiles(s) * s.TPT * 4, 256);
     ix.pos = (int*)p;
     return ix;
 }
-// bytes from the start of the workspace that must be zero before the index build (the header: every other word is
-// written before it is read)
-inline int64_t sel_index_zero_bytes(const SelShape&) { return align_up(64 * 4, 256); }
-
 // sequence of token n: largest b with cu[b] <= n
 __device__ __forceinline__ int find_seq(const int* __restrict__ cu, int B, int n) {
     int lo = 0, hi = B;   // invariant: cu[lo] <= n < cu[hi]
@@ -131,6 +122,19 @@ __device__ __forceinline__ int find_seq(const int* __restrict__ cu, int B, int n
         if (__ldg(cu + mid) <= n) lo = mid; else hi = mid;
     }
     return lo;
+}
+
+// First K/V row of block gb (gb = cu_k[b] / BK + b + j for block j of sequence b) and its number of rows, which is <= 0 for
+// the ids between two sequences that no block has.
+__device__ __forceinline__ int2 block_rows(const int* __restrict__ ck, int B, int BK, int gb) {
+    int lo = 0, hi = B;   // largest b with cu_k[b] / BK + b <= gb
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(ck + mid) / BK + mid <= gb) lo = mid; else hi = mid;
+    }
+    const int k0 = __ldg(ck + lo), k1 = __ldg(ck + lo + 1);
+    const int row0 = k0 + (gb - (k0 / BK + lo)) * BK;
+    return make_int2(row0, min(BK, k1 - row0));
 }
 
 // Block of slot `sl` of token n, or -1.  List mode: a slot is usable when 0 <= id <= t_local / BK

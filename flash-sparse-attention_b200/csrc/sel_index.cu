@@ -16,6 +16,9 @@
 //   5. fill    the CTAs of step 1 again: the same counting pass gives every warp its first position inside each key,
 //              a second pass over the same tokens writes entries and positions.
 // Entries of a key are in ascending order of (chunk, warp range, 32-token group, slot): ascending token groups.
+// Short problems run all steps in one launch (sel_index_small).
+#include <cooperative_groups.h>
+
 #include "sel_launch.cuh"
 
 namespace fsa {
@@ -61,8 +64,8 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
                 int r0 = 0;
                 const int id = !active ? -1 : in_regs ? ids[j] : list ? __ldg(row + sl) : 0;
                 int gb = active ? entry_block_ctx(tc, bd, s.BK, n, sl, id, &r0) : -1;
-                if (gb >= s.NBmax) {   // only a malformed range can do this: skip the entry, record it
-                    atomicMax(ix.header, (int)kStatusBadIndex);
+                if (gb >= s.NBmax) {   // only a malformed range can do this: skip the entry, record it (once: the header is
+                    if (FILL) atomicMax(ix.header, (int)kStatusBadIndex);      // cleared between the two passes)
                     gb = -1;
                 }
                 __syncwarp();
@@ -216,42 +219,125 @@ __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) 
     if (tid == 0) {
         ix.key_tile[HG] = carry_b;
         ix.key_seg[HG] = carry_c;
+        ix.header[0] = kStatusOk;
         ix.header[1] = carry_b;
         ix.header[2] = carry_a;
         ix.header[3] = carry_c;
     }
 }
 
-// Step 4: tile records and the padding of the tile-ordered entry list: one warp per key.  The block's first K/V row
-// and its row count follow from the block id: gb = cu_k[b] / BK + b + j for block j of sequence b.
+// Tile records of one key (a warp), and the unused slots of its last tile.
+__device__ __forceinline__ void write_tiles(const SelShape& s, const SelIndex& ix, const int* __restrict__ ck, int h, int gb, int cnt,
+                                            int t0, int seg0, int lane) {
+    const int hg = h * s.NBmax + gb, nt = (cnt + s.TPT - 1) / s.TPT;
+    const int row0 = block_rows(ck, s.B, s.BK, gb).x;
+    for (int t = lane; t < nt; t += 32) {
+        ix.tile_rec[t0 + t] = make_int4(row0, min(s.TPT, cnt - t * s.TPT) | (h << 8), hg, seg0);
+        ix.tile_aux[t0 + t] = make_int2(t0, nt);
+    }
+    const int used = cnt - (nt - 1) * s.TPT;
+    for (int e = used + lane; e < s.TPT; e += 32) ix.entries[(int64_t)(t0 + nt - 1) * s.TPT + e] = 0xFFFFFFFFu;
+}
+
+// Step 4: tile records and the padding of the tile-ordered entry list: one warp per key.
 __global__ void __launch_bounds__(256) sel_index_tiles(const int* __restrict__ cu, SelBounds bd, SelShape s, SelIndex ix) {
     const int lane = threadIdx.x & 31;
     const int hg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (hg >= s.Hk * s.NBmax) return;
     const int cnt = ix.key_cnt[hg];
     if (cnt == 0) return;
-    const int t0 = ix.key_tile[hg], nt = (cnt + s.TPT - 1) / s.TPT;
-    const int h = hg / s.NBmax, gb = hg - h * s.NBmax;
+    const int h = hg / s.NBmax;
+    write_tiles(s, ix, bd.cu_k ? bd.cu_k : cu, h, hg - h * s.NBmax, cnt, ix.key_tile[hg], ix.key_seg[hg], lane);
+}
+
+// All five steps in one launch, for short problems: one CTA per kv head, the CTAs of a cluster exchange the numbers of tiles
+// and segments of their heads through distributed shared memory.  What bounds a short build is the latency of its launches
+// and dependent steps: 512 tokens x 2 heads took 24 us in five kernels and a memset.  The list is the same one (a warp takes
+// a contiguous range of 32-token groups either way).  Used up to kSmallTokens tokens, where the passes over the tokens (four
+// groups a warp) cost about what the launches do, and up to 8 heads (the cluster) and kSmallKeys blocks (a thread each).
+constexpr int kSmallTokens = 4096, kSmallKeys = 1024, kSmallWarps = 32;
+
+// Exclusive prefix of v over the CTA's 1024 threads; *total = the sum.
+__device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total) {
+    const int lane = tid & 31, warp = tid >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int base = 0, all = 0;
+    const int w = wsum[lane];
+    all = __reduce_add_sync(0xffffffffu, w);
+    base = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+    __syncthreads();
+    *total = all;
+    return base + incl - v;
+}
+
+__global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* __restrict__ topk_idx, const int* __restrict__ cu, SelBounds bd,
+                                                                  SelShape s, SelIndex ix) {
+    namespace cg = cooperative_groups;
+    extern __shared__ int sm[];   // [warps][NBmax] counts, then positions; [NBmax] entries, [NBmax] first tile, [NBmax] first segment of a key
+    __shared__ int wsum[32], mine[2];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, NB = s.NBmax;
+    int *s_cnt = sm + kSmallWarps * NB, *s_t0 = s_cnt + NB, *s_seg = s_t0 + NB;
     const int* ck = bd.cu_k ? bd.cu_k : cu;
-    int lo = 0, hi = s.B;   // largest b with cu_k[b] / BK + b <= gb
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(ck + mid) / s.BK + mid <= gb) lo = mid; else hi = mid;
+    for (int i = tid; i < kSmallWarps * NB; i += blockDim.x) sm[i] = 0;
+    __syncthreads();
+    chunk_pass<false>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
+    __syncthreads();
+    int cnt = 0;
+    if (tid < NB) {
+        for (int w = 0; w < kSmallWarps; ++w) {
+            const int v = sm[w * NB + tid];
+            sm[w * NB + tid] = cnt;            // this warp's first position inside the key
+            cnt += v;
+        }
     }
-    const int k0 = __ldg(ck + lo), k1 = __ldg(ck + lo + 1);
-    const int row0 = k0 + (gb - (k0 / s.BK + lo)) * s.BK;
-    if (lane == 0) {
-        ix.row0[gb] = row0;                     // (the same values from every kv head)
-        ix.nrow[gb] = min(s.BK, k1 - row0);
+    int entries = 0, tiles = 0, segs = 0;
+    cta_prefix(cnt, wsum, tid, &entries);
+    const int nt = (cnt + s.TPT - 1) / s.TPT;
+    int t0 = cta_prefix(nt, wsum, tid, &tiles);
+    // tiles and entries of the heads before this one, and of all
+    if (tid == 0) { mine[0] = tiles; mine[1] = entries; }
+    cluster.sync();
+    int all_tiles = 0, all_entries = 0;
+    for (int r = 0; r < s.Hk; ++r) {
+        const int* other = cluster.map_shared_rank(mine, r);
+        if (r < h) t0 += other[0];
+        all_tiles += other[0];
+        all_entries += other[1];
     }
-    const int seg0 = ix.key_seg[hg];
-    for (int t = lane; t < nt; t += 32) {
-        ix.tile_rec[t0 + t] = make_int4(row0, min(s.TPT, cnt - t * s.TPT) | (h << 8), hg, seg0);
-        ix.tile_aux[t0 + t] = make_int2(t0, nt);
+    cluster.sync();                            // everybody has read before the words are used again
+    int seg = cta_prefix(nt > 0 ? (t0 + nt - 1) / s.RB - t0 / s.RB + 1 : 0, wsum, tid, &segs);
+    if (tid == 0) mine[0] = segs;
+    if (tid == 0 && h == 0) {
+        ix.header[0] = kStatusOk; ix.header[1] = all_tiles; ix.header[2] = all_entries;
+        ix.key_tile[s.Hk * NB] = all_tiles;
     }
-    // unused slots of the last tile
-    const int used = cnt - (nt - 1) * s.TPT;
-    for (int e = used + lane; e < s.TPT; e += 32) ix.entries[(int64_t)(t0 + nt - 1) * s.TPT + e] = 0xFFFFFFFFu;
+    cluster.sync();
+    int all_segs = 0;
+    for (int r = 0; r < s.Hk; ++r) {
+        const int v = cluster.map_shared_rank(mine, r)[0];
+        if (r < h) seg += v;
+        all_segs += v;
+    }
+    if (tid < NB) {
+        const int hg = h * NB + tid;
+        ix.key_cnt[hg] = cnt; ix.key_tile[hg] = t0; ix.key_seg[hg] = seg;
+        s_cnt[tid] = cnt; s_t0[tid] = t0; s_seg[tid] = seg;
+        for (int w = 0; w < kSmallWarps; ++w) sm[w * NB + tid] += t0 * s.TPT;
+    }
+    if (tid == 0 && h == 0) { ix.header[3] = all_segs; ix.key_seg[s.Hk * NB] = all_segs; }
+    __syncthreads();
+    for (int gb = warp; gb < NB; gb += kSmallWarps)
+        if (s_cnt[gb] > 0) write_tiles(s, ix, ck, h, gb, s_cnt[gb], s_t0[gb], s_seg[gb], lane);
+    chunk_pass<true>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
+    cluster.sync();                            // no CTA leaves while another reads its shared memory
 }
 
 // warps per CTA of the chunk kernels so that the per-warp histograms fit in shared memory; 0: the problem does not fit
@@ -266,10 +352,25 @@ int sel_index_warps(const SelShape& s) {
 }
 
 cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds& bd, const SelShape& s, const SelIndex& ix,
-                            void* ws, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(ws, 0, sel_index_zero_bytes(s), stream);
-    if (e != cudaSuccess) return e;
-    if ((int64_t)s.Hk * s.N == 0) return cudaSuccess;
+                            cudaStream_t stream) {
+    cudaError_t e;
+    if ((int64_t)s.Hk * s.N == 0) return cudaMemsetAsync(ix.header, 0, 64 * 4, stream);
+    if (s.N <= kSmallTokens && s.Hk <= 8 && s.NBmax <= kSmallKeys) {
+        const int smem = (kSmallWarps + 3) * s.NBmax * 4;
+        e = cudaFuncSetAttribute(sel_index_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, (unsigned)s.Hk);
+        cfg.blockDim = dim3(kSmallWarps * 32);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1; at.val.clusterDim.y = (unsigned)s.Hk; at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, sel_index_small, topk_idx, cu, bd, s, ix);
+    }
     const int nw = s.IW;
     if (nw == 0) return cudaErrorInvalidValue;
     const int smem = nw * s.NBmax * 4;

@@ -14,7 +14,7 @@ void prof_end(int kernel_id, cudaStream_t stream);
 int sel_index_warps(const SelShape& s);
 
 cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds& bd, const SelShape& s, const SelIndex& ix,
-                            void* ws, cudaStream_t stream);
+                            cudaStream_t stream);
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

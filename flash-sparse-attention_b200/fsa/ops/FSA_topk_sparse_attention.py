@@ -9,12 +9,13 @@ from __future__ import annotations
 
 import math
 import os
-from ctypes import byref, c_int, c_int64
+from ctypes import byref, c_int
 from typing import Any, Optional
 
 import torch
 
 from fsa import _lib
+from fsa._host import host
 
 __all__ = ["FSA_topk_sparse_attention", "FSATopkSparseAttention", "sel_attn_fwd", "sel_attn_bwd"]
 
@@ -40,70 +41,38 @@ def _alloc_bytes(n: int, device) -> torch.Tensor:
     return torch.empty(max(int(n), 16), dtype=torch.uint8, device=device)
 
 
+def _status(index_ws, what):
+    st = c_int(0)
+    _lib.check(_lib.lib().fsa_read_status(_lib.ptr(index_ws), _lib.current_stream(index_ws.device), byref(st)), what)
+
+
 def sel_attn_fwd(q, k, v, topk_idx, block_size, cu_seqlens, sm_scale, check_status: bool = False):
     """Run the forward kernels.  Returns ``(o, lse, index_ws)``; ``index_ws`` holds the
     block->entries inversion the backward reuses."""
     assert q.is_cuda, "the sm_100a kernels need CUDA tensors (no CPU fallback)"
-    L = _lib.lib()
-    N, Hq, D = q.shape
-    Hk = k.shape[1]
-    T = topk_idx.shape[-1]
-    B = cu_seqlens.shape[0] - 1
-    q, k, v = _prep(q), _prep(k, True), _prep(v, True)
-    topk_idx = topk_idx.contiguous()
-    cu_seqlens = cu_seqlens.contiguous()
-    dev = q.device
-    nb = c_int64(0)
-    _lib.check(L.fsa_sel_index_bytes(N, B, Hq, Hk, T, block_size, byref(nb)), "fsa_sel_index_bytes")
-    index_ws = _alloc_bytes(nb.value, dev)
-    _lib.check(L.fsa_sel_fwd_scratch_bytes(N, B, Hq, Hk, D, T, block_size, byref(nb)), "fsa_sel_fwd_scratch_bytes")
-    scratch = _alloc_bytes(nb.value, dev)
-    o = torch.empty((N, Hq, D), dtype=q.dtype, device=dev)
-    lse = torch.empty((Hq, N), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        rc = L.fsa_sel_fwd(
-            _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(topk_idx), _lib.ptr(cu_seqlens),
-            N, B, Hq, Hk, D, T, block_size, _lib.DTYPE_CODE[q.dtype],
-            q.stride(0), q.stride(1), k.stride(0), v.stride(0), float(sm_scale),
-            _lib.ptr(o), o.stride(0), o.stride(1), _lib.ptr(lse),
-            _lib.ptr(index_ws), index_ws.numel(), _lib.ptr(scratch), scratch.numel(), _lib.current_stream(dev),
-        )
-        _lib.check(rc, "fsa_sel_fwd")
-        if check_status or _CHECK_STATUS:
-            st = c_int(0)
-            _lib.check(L.fsa_read_status(_lib.ptr(index_ws), _lib.current_stream(dev), byref(st)), "fsa_sel_fwd status")
+    o, lse, index_ws = host().sel_fwd(q, k, v, topk_idx, block_size, cu_seqlens, float(sm_scale))
+    if check_status or _CHECK_STATUS:
+        _status(index_ws, "fsa_sel_fwd status")
     return o, lse, index_ws
 
 
 def sel_attn_bwd(q, k, v, o, lse, do, topk_idx, block_size, cu_seqlens, sm_scale, index_ws, check_status: bool = False):
     """Run the backward kernels.  Returns ``(dq, dk, dv)``."""
-    L = _lib.lib()
-    N, Hq, D = q.shape
-    Hk = k.shape[1]
-    T = topk_idx.shape[-1]
-    B = cu_seqlens.shape[0] - 1
-    q, k, v, o, do = _prep(q), _prep(k, True), _prep(v, True), _prep(o), _prep(do)
-    topk_idx = topk_idx.contiguous()
-    dev = q.device
-    nb = c_int64(0)
-    _lib.check(L.fsa_sel_bwd_scratch_bytes(N, B, Hq, Hk, D, T, block_size, byref(nb)), "fsa_sel_bwd_scratch_bytes")
-    scratch = _alloc_bytes(nb.value, dev)
-    dq = torch.empty((N, Hq, D), dtype=q.dtype, device=dev)
-    dk = torch.empty((N, Hk, D), dtype=q.dtype, device=dev)
-    dv = torch.empty((N, Hk, D), dtype=q.dtype, device=dev)
-    with torch.cuda.device(dev):
-        rc = L.fsa_sel_bwd(
-            _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse), _lib.ptr(do),
-            _lib.ptr(topk_idx), _lib.ptr(cu_seqlens), N, B, Hq, Hk, D, T, block_size, _lib.DTYPE_CODE[q.dtype],
-            q.stride(0), q.stride(1), k.stride(0), v.stride(0), o.stride(0), o.stride(1), do.stride(0), do.stride(1),
-            float(sm_scale), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv),
-            _lib.ptr(index_ws), index_ws.numel(), _lib.ptr(scratch), scratch.numel(), _lib.current_stream(dev),
-        )
-        _lib.check(rc, "fsa_sel_bwd")
-        if check_status or _CHECK_STATUS:
-            st = c_int(0)
-            _lib.check(L.fsa_read_status(_lib.ptr(index_ws), _lib.current_stream(dev), byref(st)), "fsa_sel_bwd status")
+    dq, dk, dv = host().sel_bwd(q, k, v, o, lse, do, topk_idx, block_size, cu_seqlens, float(sm_scale), index_ws)
+    if check_status or _CHECK_STATUS:
+        _status(index_ws, "fsa_sel_bwd status")
     return dq, dk, dv
+
+
+def _check_args(q, k, v, topk_idx, block_size, cu_seqlens_q, cu_seqlens_k):
+    assert q.is_cuda, "the sm_100a kernels need CUDA tensors (no CPU fallback)"
+    assert q.dtype == torch.bfloat16 or q.dtype == torch.float16
+    assert q.dtype == k.dtype and k.dtype == v.dtype
+    assert topk_idx.dtype == torch.int32
+    assert cu_seqlens_q.dtype == torch.int32 and cu_seqlens_k.dtype == torch.int32
+    assert block_size in {32, 64, 128, 256}
+    assert q.shape[1] % k.shape[1] == 0
+    assert topk_idx.shape[0] == k.shape[1] and topk_idx.shape[1] == q.shape[0]
 
 
 class FSATopkSparseAttention(torch.autograd.Function):
@@ -112,13 +81,7 @@ class FSATopkSparseAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, topk_idx, block_size, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, sm_scale=None):
-        assert q.dtype == torch.bfloat16 or q.dtype == torch.float16
-        assert q.dtype == k.dtype and k.dtype == v.dtype
-        assert topk_idx.dtype == torch.int32
-        assert cu_seqlens_q.dtype == torch.int32 and cu_seqlens_k.dtype == torch.int32
-        assert block_size in {32, 64, 128, 256}
-        assert q.shape[1] % k.shape[1] == 0
-        assert topk_idx.shape[0] == k.shape[1] and topk_idx.shape[1] == q.shape[0]
+        _check_args(q, k, v, topk_idx, block_size, cu_seqlens_q, cu_seqlens_k)
         if sm_scale is None:
             sm_scale = 1 / math.sqrt(q.shape[-1])
         o, lse, index_ws = sel_attn_fwd(q, k, v, topk_idx, block_size, cu_seqlens_q, sm_scale)
@@ -157,5 +120,7 @@ def FSA_topk_sparse_attention(
     Returns:
         attention output ``[total_len, num_q_heads, head_dim]``
     """
-    # the reference computes max_seqlen with a host sync (:1986); the kernels here do not need it
-    return FSATopkSparseAttention.apply(q, k, v, topk_idx, block_size, cu_seqlens, cu_seqlens, None, None, softmax_scale)
+    # the reference computes max_seqlen with a host sync (:1986); the kernels here do not need it.  The same function as
+    # FSATopkSparseAttention, with the autograd node in native code too.
+    _check_args(q, k, v, topk_idx, block_size, cu_seqlens, cu_seqlens)
+    return host().sel_attention(q, k, v, topk_idx, block_size, cu_seqlens, q.shape[-1] ** -0.5 if softmax_scale is None else float(softmax_scale))
