@@ -569,14 +569,8 @@ static cudaError_t launch_partial_tma(DecodeParams p, const CUtensorMap& kmap, c
     p.nst = min(max((p.chunk + kDecKT - 1) / kDecKT * p.rpp, 1), 3);
     const size_t smem = (size_t)p.nst * STAGE_BYTES + 1024 /* alignment slack */ + 1024 /* barriers, statistics */;
     auto kern = decode_partial_tma<D, HI, ET>;
-    static int attr_dev_mask = 0;                          // the attribute is per device; set it once for each
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!(attr_dev_mask >> (dev & 31) & 1)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * STAGE_BYTES + 2048);
-        if (e != cudaSuccess) return e;
-        attr_dev_mask |= 1 << (dev & 31);
-    }
+    const cudaError_t e = allow_smem((const void*)kern, 3 * STAGE_BYTES + 2048);
+    if (e != cudaSuccess) return e;
     kern<<<(unsigned)((int64_t)p.B * p.Hk * p.NP * p.nchunk), 160, smem, stream>>>(p, kmap, vmap);
     return cudaGetLastError();
 }
@@ -615,8 +609,7 @@ extern "C" int fsa_decode_attn_partial(const void* q, const void* k, const void*
     CUtensorMap kmap, vmap;
     if (kv_rows <= 0) return FSA_ERR_BAD_ARG;
     {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return FSA_ERR_CUDA;   // binds the context
+        if (int rc_ctx = ensure_context()) return rc_ctx;
         int rc = make_tile_map(&kmap, k, dtype, kv_rows, (int64_t)num_kv_heads * head_dim, kv_stride_n, kDecKT);
         if (rc) return rc;
         rc = make_tile_map(&vmap, v, dtype, kv_rows, (int64_t)num_kv_heads * head_dim, kv_stride_n, kDecKT);
@@ -681,7 +674,7 @@ extern "C" int fsa_decode_select_topk(const float* scores, int64_t scores_ld, in
     if (smem > 200 * 1024) return FSA_ERR_UNSUPPORTED;
     (void)cudaGetLastError();
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(decode_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem((const void*)decode_topk_kernel, (int)smem);
         if (e != cudaSuccess) return FSA_ERR_CUDA;
     }
     decode_topk_kernel<<<(unsigned)(batch * num_kv_heads), 256, smem, (cudaStream_t)stream>>>(p);

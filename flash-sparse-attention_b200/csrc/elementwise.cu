@@ -349,7 +349,7 @@ static int run_gate_fwd(const void* x, int64_t x_sn, const void* wg, const void*
                         int HD, void* out, void* gate, cudaStream_t stream) {
     const int smem = 3 * hidden * 2;
     auto kern = gate_proj_mix_fwd_kernel<ET>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FSA_ERR_CUDA;
+    if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
     const int64_t want = (N + 7) / 8;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
     kern<<<grid, 256, smem, stream>>>((const ET*)x, x_sn, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, N, hidden, HD,
@@ -363,7 +363,7 @@ static int run_gate_bwd(const void* x, int64_t x_sn, const void* wg, const void*
                         float* partial, cudaStream_t stream) {
     const int smem = 3 * hidden * 2;
     auto kern = gate_proj_mix_bwd_kernel<ET>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FSA_ERR_CUDA;
+    if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
     const int64_t want = (N + 7) / 8;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
     kern<<<grid, 256, smem, stream>>>((const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,

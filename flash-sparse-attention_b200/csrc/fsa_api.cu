@@ -86,6 +86,19 @@ int make_tile_map_3d_box(CUtensorMap* map, const void* base, int dtype, int64_t 
     return FSA_OK;
 }
 
+cudaError_t allow_smem(const void* kern, int bytes) {
+    struct Seen { const void* kern; int dev, bytes; };
+    static thread_local Seen seen[128];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    Seen& c = seen[(((uintptr_t)kern >> 4) ^ ((uintptr_t)kern >> 11)) & 127];      // a collision only costs the call
+    if (c.kern == kern && c.dev == dev && c.bytes >= bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) c = Seen{kern, dev, bytes};
+    return e;
+}
+
 int device_sm_count(int* out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -127,11 +140,14 @@ void prof_end(int id, cudaStream_t stream) {
 // thread; a thread that has only ever been handed device pointers (an autograd worker) may not
 // have one yet.  cudaSetDevice on the current device binds it.
 int ensure_context() {
+    static thread_local int bound = -1;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e);
+    if (dev == bound) return FSA_OK;
     e = cudaSetDevice(dev);
     if (e != cudaSuccess) return cuda_fail(e);
+    bound = dev;
     return FSA_OK;
 }
 

@@ -144,7 +144,7 @@ template <int D, typename ET>
 static cudaError_t launch_lc(const LcParams& p, const CUtensorMap& amap, const CUtensorMap& wmap, cudaStream_t stream) {
     constexpr int smem = kLcStages * (128 * 128 + 64 * D * 2) + 256;
     auto kern = linear_compress_fwd_kernel<D, ET>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((unsigned)((p.n_cmp + 127) / 128), (unsigned)p.H), 192, smem, stream>>>(p, amap, wmap);
     return cudaGetLastError();
@@ -163,8 +163,7 @@ extern "C" int fsa_linear_compress_fwd(const void* x, int64_t x_stride_n, const 
     if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || (bias && ((uintptr_t)bias & 15)) || (x_stride_n % 8)) return FSA_ERR_BAD_ARG;
     if (x_stride_n < (int64_t)num_heads * head_dim) return FSA_ERR_BAD_ARG;
     (void)cudaGetLastError();
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return FSA_ERR_CUDA;   // binds the context
+    if (int rc_ctx = ensure_context()) return rc_ctx;
     CUtensorMap wmap;
     int rc = make_tile_map(&wmap, w, dtype, (int64_t)num_heads * kernel_size * head_dim, head_dim, head_dim, 64);
     if (rc) return rc;

@@ -157,7 +157,7 @@ template <int D, typename ET>
 static cudaError_t launch_dx(const LcDxParams& p, const CUtensorMap& ymap, const CUtensorMap& wmap, cudaStream_t stream) {
     constexpr int smem = kLcDxStages * (128 * 128 + D * 128) + 256;
     auto kern = linear_compress_dx_kernel<D, ET>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     const int m_rows = (p.L + p.stride - 1) / p.stride;
     kern<<<dim3((unsigned)((m_rows + 127) / 128), (unsigned)p.H, (unsigned)(p.stride / p.phases)), 192, smem, stream>>>(p, ymap, wmap);
@@ -319,7 +319,7 @@ template <int D, typename ET>
 static cudaError_t launch_dw(const LcDwParams<ET>& p, cudaStream_t stream) {
     constexpr int smem = kLcDwStages * (2 + D / 64) * 128 * 128 + 256;
     auto kern = linear_compress_dw_kernel<D, ET>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((unsigned)(p.ks / (128 / D)), (unsigned)p.H), 256, smem, stream>>>(p);
     return cudaGetLastError();
@@ -386,8 +386,7 @@ extern "C" int fsa_linear_compress_bwd(const void* x, int64_t x_stride_n, const 
         if (seqlens_host[b] >= kernel_size) total_y += (seqlens_host[b] - kernel_size) / kernel_stride + 1;
     if (total_y > 0 && !dy) return FSA_ERR_BAD_ARG;
     (void)cudaGetLastError();
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return FSA_ERR_CUDA;   // binds the context
+    if (int rc_ctx = ensure_context()) return rc_ctx;
     cudaStream_t stream = (cudaStream_t)stream_;
     return dtype == FSA_DTYPE_BF16
                ? run_bwd<__nv_bfloat16>(x, x_stride_n, w, dy, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size,

@@ -26,7 +26,6 @@ namespace fsa {
 int make_tile_map(CUtensorMap* map, const void* base, int dtype, int64_t rows, int64_t cols, int64_t row_stride, int box_rows);
 int make_tile_map_3d_box(CUtensorMap* map, const void* base, int dtype, int64_t d0, int64_t d1, int64_t d2, int64_t stride1,
                          int64_t stride2, int box1, int box2);
-int ensure_context();
 int device_sm_count(int* out);
 
 struct RangeDenseParams {
@@ -352,7 +351,7 @@ static cudaError_t launch_rd(const RangeDenseParams& p, const CUtensorMap& qmap,
                              const CUtensorMap& omap, int max_tiles, cudaStream_t stream) {
     constexpr int smem = kTileRows * D * 2 + 4 * kRdBK * D * 2 + 256;
     auto kern = range_fwd_dense<D, ET>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(FSA_KERNEL_RANGE_DENSE, stream);
     kern<<<dim3((unsigned)max_tiles, (unsigned)p.Hk), kRdThreads, smem, stream>>>(p, qmap, kmap, vmap, omap);
@@ -722,14 +721,14 @@ cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& 
     cudaError_t e;
     if (dtype == kBF16) {
         auto kern = range_bwd_dq_dense<__nv_bfloat16>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         prof_begin(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
         kern<<<grid, kDqThreads, smem, stream>>>(p, qmap, domap, kmap, vmap, dqmap);
         prof_end(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
     } else {
         auto kern = range_bwd_dq_dense<__half>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         prof_begin(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
         kern<<<grid, kDqThreads, smem, stream>>>(p, qmap, domap, kmap, vmap, dqmap);

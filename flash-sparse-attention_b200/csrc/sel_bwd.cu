@@ -450,6 +450,7 @@ __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restri
     constexpr int D = 128, KT = 64;
     const int hg = blockIdx.x;
     if (hg == s.Hk * s.NBmax) {
+        if (blockIdx.y > 0) return;
         const int64_t first = (int64_t)__ldg(ck + s.B) * s.Hk * (D / 8), last = s.Nk * s.Hk * (D / 8);
         for (int64_t i = first + threadIdx.x; i < last; i += blockDim.x) {
             reinterpret_cast<uint4*>(dk)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -461,12 +462,13 @@ __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restri
     const int2 rn = block_rows(ck, s.B, s.BK, gb);
     const int row0 = rn.x, nkeys = min(KT, rn.y);     // rows past the end of the sequence belong to the next sequence's block
     const int seg0 = ix.key_seg[hg], nseg = ix.key_seg[hg + 1] - seg0;
-    // a warp per K/V row (32 lanes x 16 bytes = the row's 128 floats); the CTA's 8 warps walk the block's rows of dK, then dV,
-    // four rows in flight per warp
+    // a warp per K/V row (32 lanes x 16 bytes = the row's 128 floats), four rows in flight per warp; the CTA's 8 warps take 32
+    // of the 64 rows of dK and 64 rows of dV (blockIdx.y: a block with many short segments would be a serial chain otherwise)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float4* base = reinterpret_cast<const float4*>(slabs + (int64_t)seg0 * (2 * KT * D)) + lane;
     constexpr int kSegStride = 2 * KT * D / 4, kRowStride = D / 4;       // in float4
-    for (int r0 = warp * 4; r0 < 2 * KT; r0 += 32) {
+    {
+        const int r0 = (blockIdx.y * 8 + warp) * 4;
         float4 acc[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -550,7 +552,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     } else {
         auto kern = sel_bwd_main<D, ET>;
         constexpr int smem = SelBwdCfg<D>::kBytes;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         int per_sm = (int)(512 / SelBwdCfg<D>::kCols);
         int by_smem = (227 * 1024) / (smem + 2048);
@@ -571,7 +573,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     if (kv_elems > 0) {
         if (pipelined) {
             if constexpr (D == 128)
-                sel_bwd_dkdv_reduce<ET><<<(unsigned)(s.Hk * s.NBmax + 1), 256, 0, stream>>>(a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix,
+                sel_bwd_dkdv_reduce<ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), 4), 256, 0, stream>>>(a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix,
                                                                                             (ET*)a.dk, (ET*)a.dv);
         } else {
             int64_t n4 = kv_elems / 4;

@@ -630,7 +630,7 @@ static cudaError_t launch_pipe(const SelBwdArgs& a, const SelShape& s, const Sel
     p.dq_part = (ET*)a.dq_part; p.slabs = a.slabs;
     p.no_dq = no_dq ? 1 : 0;
     auto kern = sel_bwd_pipe<ET>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bwdpipe::kBytes);
+    cudaError_t e = allow_smem((const void*)kern, bwdpipe::kBytes);
     if (e != cudaSuccess) return e;
     prof_begin(2, stream);
     kern<<<num_sms, bwdpipe::kThreads, bwdpipe::kBytes, stream>>>(p, kmap, vmap, dqmap);

@@ -905,7 +905,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
         if constexpr (kPipelined) {
             auto kern = sel_fwd_main<D, BK, ET>;
             constexpr int smem = SelFwdCfg<D, BK>::kBytes;
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = allow_smem((const void*)kern, smem);
             if (e != cudaSuccess) return e;
             prof_begin(0, stream);
             kern<<<num_sms, kFwdThreads, smem, stream>>>(p, (const ET*)a.q, a.q_sn, a.q_sh, *a.kmap, *a.vmap, *a.omap);
@@ -914,7 +914,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     } else {
         auto kern = sel_fwd_simple<D, BK, ET>;
         constexpr int smem = SelFwdSimpleSmem<D, BK>::kBytes;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         constexpr int tmem_per_cta = (int)tmem_cols_pow2(BK + D);
         int per_sm = 512 / tmem_per_cta;

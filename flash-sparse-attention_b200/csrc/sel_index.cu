@@ -357,7 +357,7 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     if ((int64_t)s.Hk * s.N == 0) return cudaMemsetAsync(ix.header, 0, 64 * 4, stream);
     if (s.N <= kSmallTokens && s.Hk <= 8 && s.NBmax <= kSmallKeys) {
         const int smem = (kSmallWarps + 3) * s.NBmax * 4;
-        e = cudaFuncSetAttribute(sel_index_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)sel_index_small, smem);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, (unsigned)s.Hk);
@@ -374,9 +374,9 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     const int nw = s.IW;
     if (nw == 0) return cudaErrorInvalidValue;
     const int smem = nw * s.NBmax * 4;
-    e = cudaFuncSetAttribute(sel_index_chunk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = allow_smem((const void*)sel_index_chunk<false>, smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(sel_index_chunk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = allow_smem((const void*)sel_index_chunk<true>, smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)s.NC, (unsigned)s.Hk);
     const int HG = s.Hk * s.NBmax;

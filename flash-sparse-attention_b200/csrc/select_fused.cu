@@ -240,12 +240,12 @@ static cudaError_t launch_tl(const SelFusedParams& p, const CUtensorMap& qmap, c
     cudaError_t e;
     if (p.T_out <= 16) {
         auto kern = select_topk_fused_kernel<D, ET, A, BS, 16>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
     } else {
         auto kern = select_topk_fused_kernel<D, ET, A, BS, 32>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
     }
@@ -281,8 +281,7 @@ extern "C" int fsa_select_topk_fused(const void* q, int64_t q_stride_n, const vo
     if (total_tokens == 0 || batch == 0) return FSA_OK;
     const int A = kernel_size / kernel_stride, BS = block_size / kernel_stride;
     (void)cudaGetLastError();
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return FSA_ERR_CUDA;   // binds the context
+    if (int rc_ctx = ensure_context()) return rc_ctx;
     CUtensorMap qmap, kmap;
     int rc = make_tile_map(&qmap, q, dtype, total_tokens, (int64_t)num_q_heads * head_dim, q_stride_n, kSfRows);
     if (rc) return rc;

@@ -141,7 +141,7 @@ extern "C" int fsa_select_topk_seq(const float* qk, int64_t ld, const float* lse
     size_t smem = (size_t)4 * (p.smem_p + max_blocks + 64) * sizeof(float);
     if (smem > 200 * 1024) return FSA_ERR_UNSUPPORTED;
     (void)cudaGetLastError();
-    cudaError_t e = cudaFuncSetAttribute(select_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void*)select_topk_kernel, (int)smem);
     if (e != cudaSuccess) return FSA_ERR_CUDA;
     int64_t warps = (int64_t)num_kv_heads * seq_len;
     select_topk_kernel<<<(unsigned)((warps + 3) / 4), 128, smem, (cudaStream_t)stream_>>>(p);

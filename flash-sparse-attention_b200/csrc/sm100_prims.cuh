@@ -16,6 +16,13 @@
 
 namespace fsa {
 
+// Host side of every launch (fsa_api.cu).
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize), once per thread, device and kernel (the driver call costs about as much
+// as a launch)
+cudaError_t allow_smem(const void* kern, int bytes);
+// Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
+int ensure_context();
+
 // ----------------------------------------------------------------------------------------
 // status word: kernels never trap and never spin forever.  A wait that runs out records
 // where it gave up; the host reads the word after the launch.
