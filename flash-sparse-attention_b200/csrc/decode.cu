@@ -32,6 +32,9 @@ struct DecodeParams {
     float* scores;          // optional [B, Hk, scores_ld]: scaled logits (log2 units) of the group's FIRST head, range 0 only
     int64_t scores_ld;
     int nst;                // pipeline stages of the TMA kernel
+    // compressed mode (rng_lo null, R = 1): the rows of sequence b are [row0[b], row0[b] + its visible compressed tokens)
+    const int *seq_len, *row0;
+    int ks, stride;
     int rpp, NP;            // ranges per partial (one online softmax over rpp consecutive ranges), partial groups = ceil(R / rpp)
 };
 
@@ -90,7 +93,14 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
     const int* rhi = p.rng_hi + ((int64_t)b * p.Hk + h) * p.R;
     // rows [lo, lo + n) of range j that fall into this CTA's chunk
     auto bounds = [&](int j, int& lo, int& n) {
-        const int lo_r = rlo[j], hi_r = rhi[j];
+        int lo_r, hi_r;
+        if (p.rng_lo) {
+            lo_r = rlo[j]; hi_r = rhi[j];
+        } else {
+            const int len = __ldg(p.seq_len + b);
+            lo_r = __ldg(p.row0 + b);
+            hi_r = lo_r + (len >= p.ks ? (len - p.ks) / p.stride + 1 : 0);
+        }
         lo = lo_r + c * p.chunk;
         n = lo_r < 0 ? 0 : max(min(hi_r, lo + p.chunk) - lo, 0);
     };
@@ -585,48 +595,63 @@ static cudaError_t dispatch_g(int G, const DecodeParams& p, const CUtensorMap* k
 
 using namespace fsa;
 
+// Checks, tensor maps and launch shared by the two entry points of the partial attention.
+static int run_partial(DecodeParams& p, int64_t kv_rows, int head_dim, int dtype, float sm_scale, void* stream) {
+    if (!p.q || !p.k || !p.v || !p.o_part || !p.ml) return FSA_ERR_BAD_ARG;
+    if (p.B <= 0 || p.Hk <= 0 || p.Hq % p.Hk || p.R <= 0 || p.chunk <= 0 || p.nchunk <= 0) return FSA_ERR_BAD_ARG;
+    if ((p.kv_sn % 8) || ((uintptr_t)p.k & 15) || ((uintptr_t)p.v & 15)) return FSA_ERR_BAD_ARG;
+    if (p.rpp < 1 || (p.rpp > 1 && p.nchunk != 1)) return FSA_ERR_BAD_ARG;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    if (head_dim != 128 && head_dim != 64) return FSA_ERR_UNSUPPORTED;
+    if (kv_rows <= 0) return FSA_ERR_BAD_ARG;
+    p.scale_log2 = sm_scale * 1.4426950408889634f;
+    p.nst = 1;
+    p.NP = (p.R + p.rpp - 1) / p.rpp;
+    (void)cudaGetLastError();
+    // K/V rows are streamed by TMA (tensor maps over [kv_rows, Hk * D])
+    CUtensorMap kmap, vmap;
+    int rc = ensure_context();
+    if (rc) return rc;
+    rc = make_tile_map(&kmap, p.k, dtype, kv_rows, (int64_t)p.Hk * head_dim, p.kv_sn, kDecKT);
+    if (rc) return rc;
+    rc = make_tile_map(&vmap, p.v, dtype, kv_rows, (int64_t)p.Hk * head_dim, p.kv_sn, kDecKT);
+    if (rc) return rc;
+    const int G = p.Hq / p.Hk;
+    cudaError_t e;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dtype == FSA_DTYPE_BF16) {
+        if (head_dim == 128) e = dispatch_g<128, __nv_bfloat16>(G, p, &kmap, &vmap, st);
+        else e = dispatch_g<64, __nv_bfloat16>(G, p, &kmap, &vmap, st);
+    } else {
+        if (head_dim == 128) e = dispatch_g<128, __half>(G, p, &kmap, &vmap, st);
+        else e = dispatch_g<64, __half>(G, p, &kmap, &vmap, st);
+    }
+    if (e == cudaErrorInvalidValue) return FSA_ERR_UNSUPPORTED;
+    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
 extern "C" int fsa_decode_attn_partial(const void* q, const void* k, const void* v, int64_t kv_rows, int64_t kv_stride_n, const int32_t* rng_lo,
                                        const int32_t* rng_hi, int batch, int num_q_heads, int num_kv_heads, int head_dim,
                                        int num_ranges, int ranges_per_partial, int chunk, int num_chunks, int dtype, float sm_scale, float* o_part,
                                        float* ml, float* scores, int64_t scores_ld, void* stream) {
-    if (!q || !k || !v || !rng_lo || !rng_hi || !o_part || !ml) return FSA_ERR_BAD_ARG;
-    if (batch <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads || num_ranges <= 0 || chunk <= 0 || num_chunks <= 0)
-        return FSA_ERR_BAD_ARG;
-    if ((kv_stride_n % 8) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15)) return FSA_ERR_BAD_ARG;
-    const int G = num_q_heads / num_kv_heads;
-    DecodeParams p;
+    if (!rng_lo || !rng_hi) return FSA_ERR_BAD_ARG;
+    DecodeParams p = {};
     p.q = q; p.k = k; p.v = v; p.kv_sn = kv_stride_n; p.rng_lo = rng_lo; p.rng_hi = rng_hi;
-    p.B = batch; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.R = num_ranges; p.chunk = chunk; p.nchunk = num_chunks;
-    p.scale_log2 = sm_scale * 1.4426950408889634f;
-    p.o_part = o_part; p.ml = (float2*)ml; p.scores = scores; p.scores_ld = scores_ld; p.nst = 1;
-    if (ranges_per_partial < 1 || (ranges_per_partial > 1 && num_chunks != 1)) return FSA_ERR_BAD_ARG;
-    p.rpp = ranges_per_partial;
-    p.NP = (num_ranges + ranges_per_partial - 1) / ranges_per_partial;
-    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
-    if (head_dim != 128 && head_dim != 64) return FSA_ERR_UNSUPPORTED;
-    (void)cudaGetLastError();
-    // K/V rows are streamed by TMA (tensor maps over [kv_rows, Hk * D])
-    CUtensorMap kmap, vmap;
-    if (kv_rows <= 0) return FSA_ERR_BAD_ARG;
-    {
-        if (int rc_ctx = ensure_context()) return rc_ctx;
-        int rc = make_tile_map(&kmap, k, dtype, kv_rows, (int64_t)num_kv_heads * head_dim, kv_stride_n, kDecKT);
-        if (rc) return rc;
-        rc = make_tile_map(&vmap, v, dtype, kv_rows, (int64_t)num_kv_heads * head_dim, kv_stride_n, kDecKT);
-        if (rc) return rc;
-    }
-    const CUtensorMap *km = &kmap, *vm = &vmap;
-    cudaError_t e = cudaErrorInvalidValue;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (dtype == FSA_DTYPE_BF16) {
-        if (head_dim == 128) e = dispatch_g<128, __nv_bfloat16>(G, p, km, vm, st);
-        else e = dispatch_g<64, __nv_bfloat16>(G, p, km, vm, st);
-    } else {
-        if (head_dim == 128) e = dispatch_g<128, __half>(G, p, km, vm, st);
-        else e = dispatch_g<64, __half>(G, p, km, vm, st);
-    }
-    if (e == cudaErrorInvalidValue) return FSA_ERR_UNSUPPORTED;
-    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+    p.B = batch; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.R = num_ranges; p.chunk = chunk; p.nchunk = num_chunks; p.rpp = ranges_per_partial;
+    p.o_part = o_part; p.ml = (float2*)ml; p.scores = scores; p.scores_ld = scores_ld;
+    return run_partial(p, kv_rows, head_dim, dtype, sm_scale, stream);
+}
+
+extern "C" int fsa_decode_cmp_partial(const void* q, const void* cmp_k, const void* cmp_v, int64_t cmp_rows, int64_t cmp_stride_n, const int32_t* seq_len,
+                                      const int32_t* cmp_row0, int batch, int num_q_heads, int num_kv_heads, int head_dim, int kernel_size,
+                                      int kernel_stride, int chunk, int num_chunks, int dtype, float sm_scale, float* o_part, float* ml,
+                                      float* scores, int64_t scores_ld, void* stream) {
+    if (!seq_len || !cmp_row0 || kernel_size <= 0 || kernel_stride <= 0) return FSA_ERR_BAD_ARG;
+    DecodeParams p = {};
+    p.q = q; p.k = cmp_k; p.v = cmp_v; p.kv_sn = cmp_stride_n; p.seq_len = seq_len; p.row0 = cmp_row0; p.ks = kernel_size; p.stride = kernel_stride;
+    p.B = batch; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.R = 1; p.chunk = chunk; p.nchunk = num_chunks; p.rpp = 1;
+    p.o_part = o_part; p.ml = (float2*)ml; p.scores = scores; p.scores_ld = scores_ld;
+    return run_partial(p, cmp_rows, head_dim, dtype, sm_scale, stream);
 }
 
 extern "C" int fsa_lse_merge(const float* o_part, const float* ml, int64_t rows, int num_partials, int part_stride, int head_dim, int out_dtype,

@@ -1,0 +1,637 @@
+// The small kernels of a one-GPU decode step around decode_partial_tma (decode.cu): projections of a few rows, the append of
+// the new token with its gate, the incremental compressor, and merge + top-k + row ranges.  A step moves megabytes through
+// kernels of a few microseconds, so what bounds it is the number of launches and dependent steps: 63 launches (torch glue
+// around the library's kernels) took 180 us of GPU time for eight requests whose bytes need 25.
+//
+// Replaces the host-side glue of the reference's step (fsa_preview/module/fsa_decode.py:84-199: projections, torch.cat of
+// the caches, the incremental compressor fsa_preview/ops/linear_compress_decode.py:14-76, gate).
+#include "../../include/fsa_sm100.h"
+
+#include <cooperative_groups.h>
+#include <initializer_list>
+
+#include "sm100_prims.cuh"
+
+namespace fsa {
+
+template <typename ET> __device__ __forceinline__ float round_et(float v) {
+    return ElemTraits<ET>::unpack2(ElemTraits<ET>::pack2(v, 0.f)).x;
+}
+
+template <typename ET>
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (ElemTraits<ET>::kIsBF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// ------------------------------------------------------------------------------------------------ projections
+// y_i[b, :] = x[b, :] W_i^T for up to four weight matrices [rows_i, K] and up to 16 rows of x, in one launch.  Bound by
+// reading the weights once (K/V/Q projections of a 4096-wide layer: 50 MB, 8 us), so the layout serves the loads: a CTA =
+// 16 weight rows, its 8 warps split K, every lane loads 16 bytes of two weight rows and of its x row and uses them as MMA
+// fragments as they are (the k index inside a group of 32 is permuted alike in both operands, which a sum does not notice).
+// The warp-level MMA only has to keep up with the loads.  One library GEMM per matrix took 44 us for the four of a layer at
+// one request; above 16 rows the library's tiles are the better choice.
+struct DecodeProjParams {
+    const void* w[4];
+    void* y[4];
+    int64_t y_stride[4];
+    int rows[4];
+    int tile0[5];        // first 16-row tile of every matrix; tile0[n] = total
+    int n;
+    const void* x;
+    int64_t x_stride;
+    int B, K;
+};
+
+template <int NT, typename ET>
+__global__ void __launch_bounds__(256) decode_proj_kernel(const DecodeProjParams p) {
+    __shared__ float red[8][16][8 * NT + 1];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+    int m = 0;
+    while (m + 1 < p.n && (int)blockIdx.x >= p.tile0[m + 1]) ++m;
+    const int row0 = ((int)blockIdx.x - p.tile0[m]) * 16, rows = p.rows[m];
+    const int kw = p.K >> 3;                       // this warp's share of K (a multiple of 32)
+    // rows past the end of the matrix (and of x) repeat its last row: their products are dropped below
+    const ET* w0 = (const ET*)p.w[m] + (int64_t)min(row0 + gid, rows - 1) * p.K + warp * kw + tig * 8;
+    const ET* w1 = (const ET*)p.w[m] + (int64_t)min(row0 + gid + 8, rows - 1) * p.K + warp * kw + tig * 8;
+    const ET* xr[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) xr[t] = (const ET*)p.x + (int64_t)min(t * 8 + gid, p.B - 1) * p.x_stride + warp * kw + tig * 8;
+    float c[NT][4];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kw; k += 32) {
+        const uint4 a = __ldcs(reinterpret_cast<const uint4*>(w0 + k)), b = __ldcs(reinterpret_cast<const uint4*>(w1 + k));
+        uint4 xv[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) xv[t] = __ldg(reinterpret_cast<const uint4*>(xr[t] + k));
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            mma_16816<ET>(c[t], a.x, b.x, a.y, b.y, xv[t].x, xv[t].y);
+            mma_16816<ET>(c[t], a.z, b.z, a.w, b.w, xv[t].z, xv[t].w);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        red[warp][gid][t * 8 + tig * 2] = c[t][0];
+        red[warp][gid][t * 8 + tig * 2 + 1] = c[t][1];
+        red[warp][gid + 8][t * 8 + tig * 2] = c[t][2];
+        red[warp][gid + 8][t * 8 + tig * 2 + 1] = c[t][3];
+    }
+    __syncthreads();
+    for (int i = tid; i < 16 * 8 * NT; i += 256) {
+        const int r = i & 15, b = i >> 4;
+        if (b >= p.B || row0 + r >= rows) continue;
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red[w][r][b];
+        ((ET*)p.y[m])[(int64_t)b * p.y_stride[m] + row0 + r] = (ET)s;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ append
+// One CTA per sequence: rotates q and k of the new token at its position t = seq_len[b] (inv_freq null: they come rotated),
+// writes k, v to row t of the cache and the raw k, v to the compressor's ring, gate = sigmoid(z) with z given or computed
+// here (z = gx Wg^T), and advances seq_len.  Rounding points are those of the separate modules: cos / sin, z and the sigmoid
+// in the activation dtype.
+struct DecodeAppendParams {
+    const void *q_in, *k_in, *v_in;      // [B, Hq, D], [B, Hk, D]
+    void* q_out;                         // [B, Hq, D] rotated (may be q_in); unused without inv_freq
+    void *k_cache, *v_cache;             // [B * cap + 1, Hk, D]; the last row takes what does not fit
+    void *k_tail, *v_tail;               // [B * ks + 1, Hk, D]
+    const float* inv_freq;               // [D / 2] or null
+    int* seq_len;
+    const int* seq_row0;
+    int64_t spare_row;                   // B * cap
+    int cap, ks;
+    const void* z;                       // [B, 3] gate logits or null
+    const void *gx, *gw;                 // [B, glen], [3, glen]
+    int glen;
+    void* gate;                          // [B, 3]
+    int Hq, Hk, D;
+};
+
+template <typename ET>
+__device__ __forceinline__ float sigmoid_et(float z) { return round_et<ET>(1.f / (1.f + __expf(-z))); }
+
+template <typename ET>
+__global__ void __launch_bounds__(256) decode_append_kernel(const DecodeAppendParams p) {
+    __shared__ float s_cos[128], s_sin[128];
+    __shared__ float s_z[3][8];
+    const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int t = p.seq_len[b];
+    const int half = p.D / 2;
+    const bool rot = p.inv_freq != nullptr;
+    if (rot && tid < half) {
+        const float a = (float)t * p.inv_freq[tid];
+        s_cos[tid] = round_et<ET>(cosf(a));
+        s_sin[tid] = round_et<ET>(sinf(a));
+    }
+    if (!p.z) {
+        const uint4* x = reinterpret_cast<const uint4*>((const ET*)p.gx + (int64_t)b * p.glen);
+        const uint4* w = reinterpret_cast<const uint4*>((const ET*)p.gw);
+        const int nv = p.glen / 8;
+        float acc[3] = {0.f, 0.f, 0.f};
+        for (int i = tid; i < nv; i += 256) {
+            const uint4 xv = __ldg(x + i);
+            const uint32_t* px = &xv.x;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const uint4 wv = __ldg(w + (int64_t)j * nv + i);
+                const uint32_t* pw = &wv.x;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = ElemTraits<ET>::unpack2(px[e]), g = ElemTraits<ET>::unpack2(pw[e]);
+                    acc[j] = fmaf(f.x, g.x, fmaf(f.y, g.y, acc[j]));
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+            if (lane == 0) s_z[j][warp] = acc[j];
+        }
+    }
+    __syncthreads();
+    if (tid < 3) {
+        float z = 0.f;
+        if (p.z) z = (float)((const ET*)p.z)[b * 3 + tid];
+        else {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) z += s_z[tid][w];
+            z = round_et<ET>(z);
+        }
+        ((ET*)p.gate)[b * 3 + tid] = (ET)sigmoid_et<ET>(z);
+    }
+    const int64_t row = t < p.cap ? (int64_t)p.seq_row0[b] + t : p.spare_row, ring = (int64_t)b * p.ks + t % p.ks;
+    const int hv = half / 8;                         // 16-byte vectors per half row
+    const int nq = rot ? p.Hq * hv : 0, nk = p.Hk * hv;
+    for (int i = tid; i < nq + 2 * nk; i += 256) {
+        const bool is_q = i < nq, is_k = !is_q && i < nq + nk;
+        const int j = is_q ? i : is_k ? i - nq : i - nq - nk;
+        const int h = j / hv, v = j - h * hv, H = is_q ? p.Hq : p.Hk;
+        const ET* src = (const ET*)(is_q ? p.q_in : is_k ? p.k_in : p.v_in) + ((int64_t)b * H + h) * p.D + v * 8;
+        const uint4 a = *reinterpret_cast<const uint4*>(src), c = *reinterpret_cast<const uint4*>(src + half);
+        uint4 o1 = a, o2 = c;
+        if (rot && (is_q || is_k)) {
+            const uint32_t *pa = &a.x, *pc = &c.x;
+            uint32_t *q1 = &o1.x, *q2 = &o2.x;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 x1 = ElemTraits<ET>::unpack2(pa[e]), x2 = ElemTraits<ET>::unpack2(pc[e]);
+                const float cx = s_cos[v * 8 + 2 * e], cy = s_cos[v * 8 + 2 * e + 1], sx = s_sin[v * 8 + 2 * e], sy = s_sin[v * 8 + 2 * e + 1];
+                q1[e] = ElemTraits<ET>::pack2(x1.x * cx - x2.x * sx, x1.y * cy - x2.y * sy);
+                q2[e] = ElemTraits<ET>::pack2(x1.x * sx + x2.x * cx, x1.y * sy + x2.y * cy);
+            }
+        }
+        ET* dst = is_q ? (ET*)p.q_out + ((int64_t)b * p.Hq + h) * p.D + v * 8
+                       : (ET*)(is_k ? p.k_cache : p.v_cache) + (row * p.Hk + h) * p.D + v * 8;
+        *reinterpret_cast<uint4*>(dst) = o1;
+        *reinterpret_cast<uint4*>(dst + half) = o2;
+        if (!is_q) {
+            ET* tail = (ET*)(is_k ? p.k_tail : p.v_tail) + (ring * p.Hk + h) * p.D + v * 8;
+            *reinterpret_cast<uint4*>(tail) = a;
+            *reinterpret_cast<uint4*>(tail + half) = c;
+        }
+    }
+    if (tid == 0) p.seq_len[b] = t + 1;              // (everybody read it before the barrier above)
+}
+
+// ------------------------------------------------------------------------------------------------ incremental compressor
+// For every sequence whose length seq_len[b] (after the append) completes a window: y = ring rows (oldest first) W[h], rounded,
+// plus the position-embedding bias pe W (keys), rotated at m * stride (keys, with inv_freq), to row m of the compressed
+// cache.  A cluster of 8 CTAs per (kv head, K or V) splits the ks * D reduction; their partial sums meet in distributed
+// shared memory.  Sequences are taken eight at a time; when none completes a window, which is most steps of a small batch,
+// no weight is read and the launch ends at once (a batched library GEMM over all sequences read 17 MB every step: 35 us).
+struct DecodeCompressParams {
+    const void *k_tail, *v_tail;         // [B * ks + 1, Hk, D] rings
+    const void *wk, *wv;                 // [Hk, ks * D, D]
+    const void* pe;                      // [Hk, ks, D] or null
+    const float* inv_freq;               // [D / 2] or null
+    const int* seq_len;
+    const int* cmp_row0;
+    void *cmp_k, *cmp_v;                 // [rows, Hk, D]
+    int B, Hk, ks, stride, cmp_cap;
+};
+
+constexpr int kDcSplit = 8, kDcSeqs = 8, kDcPitch = 12;
+
+template <int D, typename ET>
+__global__ void __launch_bounds__(256) decode_compress_kernel(const DecodeCompressParams p) {
+    namespace cg = cooperative_groups;
+    constexpr int CG = D / 8, KL = 256 / CG;          // 16-byte column groups, reduction lanes
+    extern __shared__ __align__(16) float dcs[];      // [KS][kDcPitch] inputs, later [8][kDcSeqs + 1][D] sums of the warps
+    __shared__ float part[(kDcSeqs + 1) * D], s_y[D];
+    __shared__ int s_act[kDcSeqs], s_n, s_next;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x, h = blockIdx.y;
+    const bool is_k = blockIdx.z == 0;
+    const int KS = p.ks * D / kDcSplit;
+    const ET* tail = (const ET*)(is_k ? p.k_tail : p.v_tail);
+    const ET* w = (const ET*)(is_k ? p.wk : p.wv) + ((int64_t)h * p.ks * D + (int64_t)rank * KS) * D;
+    const ET* pe = is_k && p.pe ? (const ET*)p.pe + (int64_t)h * p.ks * D + (int64_t)rank * KS : nullptr;
+    const int cgi = tid % CG, kl = tid / CG;
+    for (int next = 0;;) {
+        if (warp == 0) {
+            int n = 0, b0 = next;
+            for (; b0 < p.B && n < kDcSeqs; b0 += 32) {
+                const int b = b0 + lane;
+                const int len = b < p.B ? p.seq_len[b] : 0;
+                unsigned m = __ballot_sync(0xffffffffu, len >= p.ks && (len - p.ks) % p.stride == 0);
+                int last = 31;
+                while (m && n < kDcSeqs) {
+                    last = __ffs(m) - 1;
+                    if (lane == 0) s_act[n] = b0 + last;
+                    ++n;
+                    m &= m - 1;
+                }
+                if (n == kDcSeqs) { b0 += last + 1; break; }
+            }
+            if (lane == 0) { s_n = n; s_next = b0; }
+        }
+        __syncthreads();
+        const int n = s_n;
+        if (n == 0) break;                             // (the same for every CTA of the cluster)
+        for (int i = tid; i < KS * kDcPitch; i += 256) {
+            const int e = i / kDcPitch, a = i - e * kDcPitch;
+            float x = 0.f;
+            if (a < n) {
+                const int b = s_act[a], kk = rank * KS + e, o = kk / D, d = kk - o * D;
+                x = (float)tail[(((int64_t)b * p.ks + (p.seq_len[b] + o) % p.ks) * p.Hk + h) * D + d];
+            } else if (a == kDcSeqs && pe) {
+                x = (float)pe[e];
+            }
+            dcs[i] = x;
+        }
+        __syncthreads();
+        float acc[kDcSeqs + 1][8];
+#pragma unroll
+        for (int a = 0; a <= kDcSeqs; ++a)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
+#pragma unroll 4
+        for (int e = kl; e < KS; e += KL) {
+            const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)e * D) + cgi);
+            const uint32_t* pw = &wv.x;
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 t = ElemTraits<ET>::unpack2(pw[j]);
+                f[2 * j] = t.x; f[2 * j + 1] = t.y;
+            }
+            const float4 x0 = *reinterpret_cast<const float4*>(dcs + e * kDcPitch), x1 = *reinterpret_cast<const float4*>(dcs + e * kDcPitch + 4);
+            const float xs[kDcSeqs + 1] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, dcs[e * kDcPitch + 8]};
+#pragma unroll
+            for (int a = 0; a <= kDcSeqs; ++a)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[a][j] = fmaf(xs[a], f[j], acc[a][j]);
+        }
+        __syncthreads();
+        // lanes of a warp that share a column group, then the warps, then the cluster
+#pragma unroll
+        for (int a = 0; a <= kDcSeqs; ++a)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+#pragma unroll
+                for (int o = CG; o < 32; o <<= 1) acc[a][j] += __shfl_xor_sync(0xffffffffu, acc[a][j], o);
+                if (lane < CG) dcs[(warp * (kDcSeqs + 1) + a) * D + cgi * 8 + j] = acc[a][j];
+            }
+        __syncthreads();
+        for (int i = tid; i < (kDcSeqs + 1) * D; i += 256) {
+            float s = 0.f;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) s += dcs[v * (kDcSeqs + 1) * D + i];
+            part[i] = s;
+        }
+        cluster.sync();
+        if (rank < n) {
+            const int b = s_act[rank], m = (p.seq_len[b] - p.ks) / p.stride;
+            if (tid < D) {
+                float y = 0.f, bias = 0.f;
+#pragma unroll
+                for (int r = 0; r < kDcSplit; ++r) {
+                    const float* other = cluster.map_shared_rank(part, r);
+                    y += other[rank * D + tid];
+                    bias += other[kDcSeqs * D + tid];
+                }
+                y = round_et<ET>(y);
+                if (pe) y = round_et<ET>(y + round_et<ET>(bias));
+                s_y[tid] = y;
+            }
+            __syncthreads();
+            if (tid < D && m < p.cmp_cap) {
+                float y = s_y[tid];
+                if (is_k && p.inv_freq) {
+                    const int i = tid % (D / 2);
+                    const float ang = (float)(m * p.stride) * p.inv_freq[i];
+                    const float c = round_et<ET>(cosf(ang)), s = round_et<ET>(sinf(ang));
+                    const float x1 = s_y[i], x2 = s_y[i + D / 2];
+                    y = tid < D / 2 ? x1 * c - x2 * s : x1 * s + x2 * c;
+                }
+                ((ET*)(is_k ? p.cmp_k : p.cmp_v))[((int64_t)(p.cmp_row0[b] + m) * p.Hk + h) * D + tid] = (ET)y;
+            }
+        }
+        next = s_next;
+        cluster.sync();                                // the partial sums have been read
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ merge, top-k, row ranges
+// Between the two attention passes of a step, one CTA per (sequence, kv head): LSE merge of the compressed branch's partials
+// of the G heads, the top-k blocks from the scores of the group's first head (the rule of decode_topk_kernel), and the cache
+// rows of the selected blocks and of the sliding window (the rule of decode_ranges_kernel).  The top-k works on keys (bf16
+// score, then the complement of the id, so that equal scores go to the lower id): every warp takes the best of its share with
+// warp-wide maxima, then one warp takes the best of those -- two barriers instead of two per selected block (64 sequences of
+// 2048 blocks: 34 us in the kernel with a CTA-wide maximum per selected block).
+struct DecodeSelectParams {
+    const float* o_part;     // [B, Hq, P, D]
+    const float2* ml;        // [B, Hq, P]
+    const float* scores;     // [B, Hk, ld]
+    int64_t ld;
+    const int *seq_len, *seq_row0;
+    int B, Hk, G, D, P;
+    int ks, stride, BK, init_blocks, local_blocks, T, nw, max_blocks, window, npieces;
+    float w[16];
+    void* o_cmp;             // [B, Hq, D]
+    int32_t* topk;           // [B, Hk, T]
+    int *rng_lo, *rng_hi;    // [B, Hk, T + npieces]
+};
+
+// The `want` largest of the keys in[0 .. n), all different, none 0: to out[0 .. want) in descending order (0 when they run
+// out).  One warp; every lane looks after every 32nd key and looks again only when its own was taken.  Destroys the keys.
+__device__ __forceinline__ void warp_largest(uint32_t* in, int n, int want, uint32_t* out, int lane) {
+    auto best = [&](int& at) {
+        uint32_t m = 0;
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t v = in[i];
+            if (v > m) { m = v; at = i; }
+        }
+        return m;
+    };
+    int at = 0;
+    uint32_t mine = best(at);
+    for (int r = 0; r < want; ++r) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, mine);
+        if (lane == 0) out[r] = m;
+        if (m != 0 && mine == m) {
+            in[at] = 0;
+            mine = best(at);
+        }
+        __syncwarp();
+    }
+}
+
+template <typename ET>
+__global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectParams p) {
+    extern __shared__ uint32_t dks[];                 // [max_blocks] keys, then the probabilities
+    __shared__ float s_lse;
+    __shared__ uint32_t cand[8 * 64], sel[64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b = blockIdx.x / p.Hk, h = blockIdx.x % p.Hk;
+    const int len = p.seq_len[b], t = len - 1;
+    const int ncmp = len >= p.ks ? (len - p.ks) / p.stride + 1 : 0;
+    // ---- merge: a warp per head
+    for (int g = warp; g < p.G; g += 8) {
+        const int64_t row = (int64_t)b * p.Hk * p.G + h * p.G + g;
+        const float2* mlr = p.ml + row * p.P;
+        float M = -INFINITY;
+        for (int i = lane; i < p.P; i += 32) {
+            const float2 v = mlr[i];
+            if (v.y > 0.f) M = fmaxf(M, v.x);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        float L = 0.f;
+        for (int i = lane; i < p.P; i += 32) {
+            const float2 v = mlr[i];
+            if (v.y > 0.f) L += exp2f(v.x - M) * v.y;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        if (g == 0 && lane == 0) s_lse = L > 0.f ? M + log2f(L) : -INFINITY;
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+        const float* src = p.o_part + row * p.P * p.D;
+        for (int d = lane * 4; d < p.D; d += 128) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int i = 0; i < p.P; ++i) {
+                const float2 v = mlr[i];
+                if (v.y > 0.f) {
+                    const float wt = exp2f(v.x - M);
+                    const float4 x = *reinterpret_cast<const float4*>(src + (int64_t)i * p.D + d);
+                    acc.x = fmaf(wt, x.x, acc.x); acc.y = fmaf(wt, x.y, acc.y); acc.z = fmaf(wt, x.z, acc.z); acc.w = fmaf(wt, x.w, acc.w);
+                }
+            }
+            *reinterpret_cast<uint2*>((ET*)p.o_cmp + row * p.D + d) =
+                make_uint2(ElemTraits<ET>::pack2(acc.x * inv, acc.y * inv), ElemTraits<ET>::pack2(acc.z * inv, acc.w * inv));
+        }
+    }
+    __syncthreads();
+    // ---- block scores
+    const float lse = s_lse;
+    const float* row = p.scores + ((int64_t)b * p.Hk + h) * p.ld;
+    const int bq = t / p.BK, nb = t >= 0 ? min(bq + 1, p.max_blocks) : 0;
+    const int bstride = p.BK / p.stride, pad = p.ks / p.stride - 1;
+    float* pv = reinterpret_cast<float*>(dks + p.max_blocks);
+    const int cmax = min(min(ncmp, nb * bstride + p.nw), (int)p.ld);
+    for (int c0 = 0; c0 < cmax; c0 += 2048) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = c0 + j * 256 + tid;
+            v[j] = c < cmax ? row[c] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = c0 + j * 256 + tid;
+            if (c < cmax) pv[c] = exp2f(v[j] - lse);
+        }
+    }
+    __syncthreads();
+    for (int blk = tid; blk < nb; blk += 256) {
+        float s = 0.f;
+        for (int o = 0; o < p.nw; ++o) {
+            const int c = blk * bstride - pad + o;
+            const float v = (c >= 0 && c < cmax) ? pv[c] : 0.f;
+            s += v * p.w[o];
+        }
+        if (blk < p.init_blocks || (bq >= blk && bq < blk + p.local_blocks)) s = INFINITY;
+        // scores are >= 0: their bf16 words order like the scores
+        dks[blk] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16(s)) << 16 | (uint32_t)(65535 - blk);
+    }
+    __syncthreads();
+    // ---- top-k: the best T of every warp's share of the blocks, then the best T of those
+    const int nsel = min(p.T, nb);
+    const int share = (nb + 7) / 8, s0 = min(nb, warp * share), s1 = min(nb, s0 + share);
+    warp_largest(dks + s0, s1 - s0, nsel, cand + warp * nsel, lane);
+    __syncthreads();
+    if (warp == 0) warp_largest(cand, 8 * nsel, nsel, sel, lane);
+    __syncthreads();
+    int32_t* out = p.topk + ((int64_t)b * p.Hk + h) * p.T;
+    int* s_id = reinterpret_cast<int*>(cand);          // ascending ids, -1 behind them
+    if (tid < p.T) {
+        int id = -1, at = tid;
+        if (tid < nsel) {
+            id = 65535 - (int)(sel[tid] & 0xffffu);
+            at = 0;
+            for (int j = 0; j < nsel; ++j) at += 65535 - (int)(sel[j] & 0xffffu) < id;
+        }
+        s_id[at] = id;
+        out[at] = id;
+    }
+    __syncthreads();
+    // ---- cache rows of the selected blocks and of the window [max(0, t - window), t] in pieces of BK rows
+    const int R = p.T + p.npieces;
+    const int64_t r0 = ((int64_t)b * p.Hk + h) * R;
+    for (int r = tid; r < R; r += 256) {
+        int a = 0, e = 0;
+        if (len > 0) {
+            if (r < p.T) {
+                const int id = s_id[r];
+                if (id >= 0 && id <= t / p.BK) { a = id * p.BK; e = min(a + p.BK, len); }
+            } else {
+                a = max(0, t - p.window) + (r - p.T) * p.BK;
+                e = min(a + p.BK, len);
+            }
+        }
+        p.rng_lo[r0 + r] = a < e ? p.seq_row0[b] + a : -1;
+        p.rng_hi[r0 + r] = a < e ? p.seq_row0[b] + e : -1;
+    }
+}
+
+}  // namespace fsa
+
+using namespace fsa;
+
+static bool misaligned(std::initializer_list<const void*> ps) {
+    for (const void* p : ps)
+        if ((uintptr_t)p & 15) return true;
+    return false;
+}
+
+extern "C" int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k_dim, int num, const void* const* w, const int* rows,
+                               void* const* y, const int64_t* y_stride, int dtype, void* stream) {
+    if (!x || !w || !rows || !y || !y_stride || batch <= 0 || num <= 0 || k_dim <= 0) return FSA_ERR_BAD_ARG;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    if (num > 4 || batch > 16 || k_dim % 256) return FSA_ERR_UNSUPPORTED;
+    if ((x_stride % 8) || misaligned({x})) return FSA_ERR_BAD_ARG;
+    DecodeProjParams p;
+    p.n = num; p.x = x; p.x_stride = x_stride; p.B = batch; p.K = k_dim;
+    int tiles = 0;
+    for (int i = 0; i < num; ++i) {
+        if (!w[i] || !y[i] || rows[i] <= 0 || misaligned({w[i]})) return FSA_ERR_BAD_ARG;
+        p.w[i] = w[i]; p.y[i] = y[i]; p.y_stride[i] = y_stride[i]; p.rows[i] = rows[i]; p.tile0[i] = tiles;
+        tiles += (rows[i] + 15) / 16;
+    }
+    p.tile0[num] = tiles;
+    (void)cudaGetLastError();
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dtype == FSA_DTYPE_BF16) {
+        if (batch <= 8) decode_proj_kernel<1, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
+        else decode_proj_kernel<2, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
+    } else {
+        if (batch <= 8) decode_proj_kernel<1, __half><<<tiles, 256, 0, st>>>(p);
+        else decode_proj_kernel<2, __half><<<tiles, 256, 0, st>>>(p);
+    }
+    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
+extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void* v_in, void* q_out, void* k_cache, void* v_cache, void* k_tail,
+                                 void* v_tail, const float* inv_freq, int32_t* seq_len, const int32_t* seq_row0, int batch, int cap,
+                                 int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, const void* gate_logits, const void* gate_x,
+                                 const void* gate_w, int gate_dim, void* gate, int dtype, void* stream) {
+    if (!k_in || !v_in || !k_cache || !v_cache || !k_tail || !v_tail || !seq_len || !seq_row0 || !gate || batch <= 0 || cap <= 0) return FSA_ERR_BAD_ARG;
+    if (num_q_heads <= 0 || num_kv_heads <= 0 || kernel_size <= 0 || (inv_freq && (!q_in || !q_out))) return FSA_ERR_BAD_ARG;
+    if (!gate_logits && (!gate_x || !gate_w || gate_dim <= 0 || gate_dim % 8 || misaligned({gate_x, gate_w}))) return FSA_ERR_BAD_ARG;
+    if (misaligned({q_in, k_in, v_in, q_out, k_cache, v_cache, k_tail, v_tail})) return FSA_ERR_BAD_ARG;
+    if (head_dim % 16 || head_dim > 256) return FSA_ERR_UNSUPPORTED;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    DecodeAppendParams p;
+    p.q_in = q_in; p.k_in = k_in; p.v_in = v_in; p.q_out = q_out; p.k_cache = k_cache; p.v_cache = v_cache; p.k_tail = k_tail; p.v_tail = v_tail;
+    p.inv_freq = inv_freq; p.seq_len = seq_len; p.seq_row0 = seq_row0; p.spare_row = (int64_t)batch * cap; p.cap = cap; p.ks = kernel_size;
+    p.z = gate_logits; p.gx = gate_x; p.gw = gate_w; p.glen = gate_dim; p.gate = gate; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.D = head_dim;
+    (void)cudaGetLastError();
+    if (dtype == FSA_DTYPE_BF16) decode_append_kernel<__nv_bfloat16><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
+    else decode_append_kernel<__half><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
+    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
+template <int D, typename ET>
+static cudaError_t launch_compress(const DecodeCompressParams& p, cudaStream_t stream) {
+    const int in = p.ks * D / kDcSplit * kDcPitch, sums = 8 * (kDcSeqs + 1) * D;
+    const int smem = (in > sums ? in : sums) * 4;
+    auto kern = decode_compress_kernel<D, ET>;
+    cudaError_t e = allow_smem((const void*)kern, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kDcSplit, (unsigned)p.Hk, 2);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kDcSplit; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+extern "C" int fsa_decode_compress(const void* k_tail, const void* v_tail, const void* w_key, const void* w_value, const void* pe,
+                                   const float* inv_freq, const int32_t* seq_len, const int32_t* cmp_row0, void* cmp_k, void* cmp_v, int batch,
+                                   int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int cmp_cap, int dtype, void* stream) {
+    if (!k_tail || !v_tail || !w_key || !w_value || !seq_len || !cmp_row0 || !cmp_k || !cmp_v || batch <= 0 || num_kv_heads <= 0) return FSA_ERR_BAD_ARG;
+    if (kernel_size <= 0 || kernel_stride <= 0 || misaligned({w_key, w_value})) return FSA_ERR_BAD_ARG;
+    if ((head_dim != 64 && head_dim != 128) || kernel_size % 8 || kernel_size > 128 || num_kv_heads > 65535) return FSA_ERR_UNSUPPORTED;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    DecodeCompressParams p;
+    p.k_tail = k_tail; p.v_tail = v_tail; p.wk = w_key; p.wv = w_value; p.pe = pe; p.inv_freq = inv_freq; p.seq_len = seq_len; p.cmp_row0 = cmp_row0;
+    p.cmp_k = cmp_k; p.cmp_v = cmp_v; p.B = batch; p.Hk = num_kv_heads; p.ks = kernel_size; p.stride = kernel_stride; p.cmp_cap = cmp_cap;
+    (void)cudaGetLastError();
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e;
+    if (dtype == FSA_DTYPE_BF16) e = head_dim == 128 ? launch_compress<128, __nv_bfloat16>(p, st) : launch_compress<64, __nv_bfloat16>(p, st);
+    else e = head_dim == 128 ? launch_compress<128, __half>(p, st) : launch_compress<64, __half>(p, st);
+    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
+extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int num_partials, const float* scores, int64_t scores_ld,
+                                       const int32_t* seq_len, const int32_t* seq_row0, int batch, int num_q_heads, int num_kv_heads, int head_dim,
+                                       int kernel_size, int kernel_stride, int block_size, int init_blocks, int local_blocks, int topk,
+                                       int max_blocks, int window, int num_window_pieces, int dtype, void* o_cmp, int32_t* topk_idx,
+                                       int32_t* rng_lo, int32_t* rng_hi, void* stream) {
+    if (!o_part || !ml || !scores || !seq_len || !seq_row0 || !o_cmp || !topk_idx || !rng_lo || !rng_hi || batch <= 0 || num_partials <= 0) return FSA_ERR_BAD_ARG;
+    if (num_kv_heads <= 0 || num_q_heads % num_kv_heads || topk <= 0 || max_blocks <= 0 || num_window_pieces < 0 || kernel_stride <= 0 || block_size <= 0)
+        return FSA_ERR_BAD_ARG;
+    if (num_window_pieces > 0 && (int64_t)block_size * num_window_pieces < (int64_t)window + 1) return FSA_ERR_BAD_ARG;
+    if (head_dim % 4 || misaligned({o_part}) || ((uintptr_t)o_cmp & 7)) return FSA_ERR_BAD_ARG;
+    if (kernel_size % kernel_stride || block_size % kernel_stride || topk > 64 || max_blocks > 65535) return FSA_ERR_UNSUPPORTED;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    DecodeSelectParams p;
+    p.o_part = o_part; p.ml = (const float2*)ml; p.scores = scores; p.ld = scores_ld; p.seq_len = seq_len; p.seq_row0 = seq_row0;
+    p.B = batch; p.Hk = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.D = head_dim; p.P = num_partials;
+    p.ks = kernel_size; p.stride = kernel_stride; p.BK = block_size; p.init_blocks = init_blocks; p.local_blocks = local_blocks; p.T = topk;
+    p.max_blocks = max_blocks; p.window = window; p.npieces = num_window_pieces;
+    const int a = kernel_size / kernel_stride, bb = block_size / kernel_stride;
+    p.nw = a + bb - 1;
+    if (p.nw > 16) return FSA_ERR_UNSUPPORTED;
+    for (int i = 0; i < 16; ++i) p.w[i] = 0.f;
+    for (int i = 0; i < a; ++i)
+        for (int j = 0; j < bb; ++j) p.w[i + j] += 1.f;
+    p.o_cmp = o_cmp; p.topk = topk_idx; p.rng_lo = rng_lo; p.rng_hi = rng_hi;
+    const int64_t smem = 4 * ((int64_t)max_blocks + (int64_t)max_blocks * bb + p.nw);      // keys, probabilities the blocks can touch
+    if (smem > 200 * 1024) return FSA_ERR_UNSUPPORTED;
+    (void)cudaGetLastError();
+    const void* kern = dtype == FSA_DTYPE_BF16 ? (const void*)decode_select_kernel<__nv_bfloat16> : (const void*)decode_select_kernel<__half>;
+    if (smem > 48 * 1024 && allow_smem(kern, (int)smem) != cudaSuccess) return FSA_ERR_CUDA;
+    const unsigned grid = (unsigned)(batch * num_kv_heads);
+    if (dtype == FSA_DTYPE_BF16) decode_select_kernel<__nv_bfloat16><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
+    else decode_select_kernel<__half><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
+    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}

@@ -1,0 +1,162 @@
+// The one-GPU decode step in native code: scratch carved from one allocation, six to eight launches, no synchronisation (so
+// that a CUDA graph can hold it).
+#include "host_common.h"
+
+namespace fsa_host {
+
+struct DecodeCfg {
+    int ks, stride, bs, topk, init_blocks, local_blocks, window;
+    int64_t max_len;
+    double scale;      // 0: 1 / sqrt(head_dim)
+};
+
+static DecodeCfg cfg_of(const std::vector<int64_t>& c, double scale) {
+    TORCH_CHECK_VALUE(c.size() == 8, "decode settings");
+    return {(int)c[0], (int)c[1], (int)c[2], (int)c[3], (int)c[4], (int)c[5], (int)c[6], c[7], scale};
+}
+
+// Three branches of one token per sequence and their gate mix; q [B, Hq, D] rotated, gate [B, 3].
+static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cmp_k, const Tensor& cmp_v,
+                                            const Tensor& seq_len, const Tensor& seq_row0, const Tensor& cmp_row0, const Tensor& gate,
+                                            const DecodeCfg& c) {
+    const int B = (int)q.size(0), Hq = (int)q.size(1), D = (int)q.size(2), Hk = (int)k.size(1), dt = dtype_code(q);
+    TORCH_CHECK_VALUE(k.stride(2) == 1 && k.stride(1) == D && v.strides() == k.strides() && cmp_k.stride(2) == 1 && cmp_k.stride(1) == D &&
+                          cmp_v.strides() == cmp_k.strides(), "cache rows must be packed");
+    const float scale = (float)(c.scale > 0 ? c.scale : 1.0 / std::sqrt((double)D));
+    void* st = stream_of(q);
+    // Work per CTA of the two attention passes: as long as possible (few partials, a ring of loads that stays full) while about
+    // four CTAs per SM are left for each pass: a small batch is split finely, a full one takes 1024 rows / 16 blocks at a time.
+    const int64_t max_cmp = std::max<int64_t>(c.max_len >= c.ks ? (c.max_len - c.ks) / c.stride + 1 : 0, 1);
+    const int64_t per = (max_cmp * B * Hk + 4 * 148 - 1) / (4 * 148);
+    const int chunk = (int)std::min<int64_t>(1024, std::max<int64_t>(64, (per + 63) / 64 * 64));
+    const int nchunk = (int)((max_cmp + chunk - 1) / chunk);
+    const int npieces = (c.window + 1 + c.bs - 1) / c.bs, R = c.topk + npieces;
+    int rpp = 16;
+    while (rpp > 1 && (c.topk % rpp || (int64_t)B * Hk * ((R + rpp - 1) / rpp) < 2 * 148)) rpp /= 2;
+    const int ns = c.topk / rpp, nw = (npieces + rpp - 1) / rpp, P2 = ns + nw;
+    const int64_t ld = (int64_t)chunk * nchunk;
+    auto al = [](int64_t n) { return (n + 255) / 256 * 256; };
+    const int64_t rowsq = (int64_t)B * Hq;
+    const int64_t b_o1 = al(rowsq * nchunk * D * 4), b_m1 = al(rowsq * nchunk * 8), b_sc = al((int64_t)B * Hk * ld * 4),
+                  b_o2 = al(rowsq * P2 * D * 4), b_m2 = al(rowsq * P2 * 8), b_r = al((int64_t)B * Hk * R * 4), b_oc = al(rowsq * D * 2);
+    const Tensor scratch = bytes(b_o1 + b_m1 + b_sc + b_o2 + b_m2 + 2 * b_r + b_oc, q);
+    char* p = (char*)scratch.data_ptr();
+    auto take = [&](int64_t n) { char* r = p; p += n; return r; };
+    float* o1 = (float*)take(b_o1);
+    float* m1 = (float*)take(b_m1);
+    float* sc = (float*)take(b_sc);
+    float* o2 = (float*)take(b_o2);
+    float* m2 = (float*)take(b_m2);
+    int32_t* lo = (int32_t*)take(b_r);
+    int32_t* hi = (int32_t*)take(b_r);
+    void* oc = take(b_oc);
+    Tensor topk = i32({B, Hk, c.topk}, q), out = at::empty_like(q);
+    check(fsa_decode_cmp_partial(ptr(q), ptr(cmp_k), ptr(cmp_v), cmp_k.size(0), cmp_k.stride(0), iptr(seq_len), iptr(cmp_row0), B, Hq, Hk, D,
+                                 c.ks, c.stride, chunk, nchunk, dt, scale, o1, m1, sc, ld, st),
+          "fsa_decode_cmp_partial");
+    check(fsa_decode_merge_select(o1, m1, nchunk, sc, ld, iptr(seq_len), iptr(seq_row0), B, Hq, Hk, D, c.ks, c.stride, c.bs, c.init_blocks,
+                                  c.local_blocks, c.topk, (int)((c.max_len + c.bs - 1) / c.bs), c.window, npieces, dt, oc,
+                                  topk.data_ptr<int32_t>(), lo, hi, st),
+          "fsa_decode_merge_select");
+    check(fsa_decode_attn_partial(ptr(q), ptr(k), ptr(v), k.size(0), k.stride(0), lo, hi, B, Hq, Hk, D, R, rpp, c.bs, 1, dt, scale, o2, m2,
+                                  nullptr, 0, st),
+          "fsa_decode_attn_partial");
+    check(fsa_decode_finish(o2, m2, rowsq, ns, nw, P2, D, Hq, dt, oc, ptr(gate), ptr(out), st), "fsa_decode_finish");
+    return {out, topk};
+}
+
+std::tuple<Tensor, Tensor> decode_mixed(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cmp_k, const Tensor& cmp_v,
+                                        const Tensor& seq_len, const Tensor& seq_row0, const Tensor& cmp_row0, const Tensor& gate,
+                                        const std::vector<int64_t>& cfg, double scale) {
+    c10::cuda::CUDAGuard guard(q.device());
+    return attention(q.contiguous(), k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate.to(q.scalar_type()).contiguous(), cfg_of(cfg, scale));
+}
+
+// The buffers of a DecodeCache, in this order: k, v, cmp_k, cmp_v, k_tail, v_tail, seq_len, seq_row0, cmp_row0.
+using Cache = std::vector<Tensor>;
+
+// Append (with the gate from logits z, or from gx and its weight), compressor, attention.
+static std::tuple<Tensor, Tensor> step(const Tensor& q_in, const Tensor& k_new, const Tensor& v_new, Tensor q, const Tensor& inv_freq,
+                                       const Tensor& z, const Tensor& gx, const Tensor& gw, const Cache& t, const Tensor& w_key,
+                                       const Tensor& w_value, const Tensor& pe, bool compress, const DecodeCfg& c) {
+    TORCH_CHECK_VALUE(t.size() == 9, "cache buffers");
+    same_kind(k_new, {&v_new, &q, &gw, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &w_key, &w_value, &pe}, "decode step");
+    const int B = (int)k_new.size(0), Hk = (int)k_new.size(1), D = (int)k_new.size(2), Hq = (int)q.size(1), dt = dtype_code(k_new);
+    const int cap = (int)((t[0].size(0) - 1) / B), cmp_cap = (int)((t[2].size(0) - 1) / B);
+    const float* freq = inv_freq.defined() ? inv_freq.data_ptr<float>() : nullptr;
+    void* st = stream_of(k_new);
+    const Tensor gate = at::empty({B, 3}, k_new.options());
+    check(fsa_decode_append(ptr(q_in), ptr(k_new), ptr(v_new), ptr(q), ptr(t[0]), ptr(t[1]), ptr(t[4]), ptr(t[5]), freq,
+                            t[6].data_ptr<int32_t>(), iptr(t[7]), B, cap, Hq, Hk, D, c.ks, ptr(z), ptr(gx), ptr(gw),
+                            gx.defined() ? (int)gx.size(-1) : 0, ptr(gate), dt, st),
+          "fsa_decode_append");
+    if (compress)
+        check(fsa_decode_compress(ptr(t[4]), ptr(t[5]), ptr(w_key), ptr(w_value), ptr(pe), freq, iptr(t[6]), iptr(t[8]), ptr(t[2]), ptr(t[3]), B,
+                                  Hk, D, c.ks, c.stride, cmp_cap, dt, st),
+              "fsa_decode_compress");
+    return attention(q, t[0], t[1], t[2], t[3], t[6], t[7], t[8], gate, c);
+}
+
+// FlashSparseAttentionDecodeKernel.step: q, k_new, v_new in, [B, Hq * D] and the block ids out.
+std::tuple<Tensor, Tensor> decode_kernel_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gw, const Cache& t,
+                                              const Tensor& w_key, const Tensor& w_value, const Tensor& pe, bool compress,
+                                              const std::vector<int64_t>& cfg, double scale) {
+    c10::cuda::CUDAGuard guard(q_.device());
+    const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+    auto [y, ids] = step(q, k, v, q, Tensor(), Tensor(), q.view({q.size(0), -1}), gw, t, w_key, w_value, pe, compress, cfg_of(cfg, scale));
+    return {y.view({y.size(0), -1}), ids};
+}
+
+// Rows up to which the library's own skinny projection is used (one MMA tile of rows; above it a library GEMM's tiles are fuller).
+constexpr int kProjRows = 16;
+
+static void project(const Tensor& x, std::initializer_list<Tensor> ws, std::initializer_list<Tensor> ys) {
+    const void* w[4];
+    void* y[4];
+    int rows[4];
+    int64_t ystr[4];
+    int n = 0;
+    for (auto& t : ws) { w[n] = ptr(t); rows[n] = (int)t.size(0); ++n; }
+    n = 0;
+    for (auto& t : ys) { y[n] = ptr(t); ystr[n] = t.stride(0); ++n; }
+    check(fsa_decode_proj(ptr(x), x.stride(0), (int)x.size(0), (int)x.size(1), n, w, rows, y, ystr, dtype_code(x), stream_of(x)), "fsa_decode_proj");
+}
+
+// FlashSparseAttentionDecode.step: x [B, hidden] in, [B, hidden] and the block ids out.
+std::tuple<Tensor, Tensor> decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo,
+                                             const Tensor& gw, const Tensor& inv_freq, int64_t D, const Cache& t, const Tensor& w_key,
+                                             const Tensor& w_value, const Tensor& pe, bool compress, const std::vector<int64_t>& cfg, double scale) {
+    c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = x_.contiguous();
+    same_kind(x, {&wq, &wk, &wv, &wo, &gw}, "decode step");
+    const int64_t B = x.size(0), nq = wq.size(0), nk = wk.size(0);
+    const bool skinny = B <= kProjRows && x.size(1) % 256 == 0 && nq % 256 == 0 && ((uintptr_t)x.data_ptr() & 15) == 0;
+    Tensor q, k, v, z;
+    if (skinny) {
+        q = at::empty({B, nq}, x.options());
+        k = at::empty({B, nk}, x.options());
+        v = at::empty({B, nk}, x.options());
+        z = at::empty({B, 3}, x.options());
+        project(x, {wq, wk, wv, gw}, {q, k, v, z});
+    } else {
+        q = at::linear(x, wq);
+        k = at::linear(x, wk);
+        v = at::linear(x, wv);
+    }
+    q = q.view({B, nq / D, D});
+    auto [mixed, ids] = step(q, k.view({B, nk / D, D}), v.view({B, nk / D, D}), q, inv_freq, z, skinny ? Tensor() : x, gw, t, w_key, w_value, pe,
+                             compress, cfg_of(cfg, scale));
+    const Tensor m = mixed.view({B, nq});
+    if (!skinny) return {at::linear(m, wo), ids};
+    Tensor y = at::empty({B, wo.size(0)}, x.options());
+    project(m, {wo}, {y});
+    return {y, ids};
+}
+
+void bind_decode(pybind11::module& m) {
+    m.def("decode_mixed", &decode_mixed);
+    m.def("decode_kernel_step", &decode_kernel_step);
+    m.def("decode_layer_step", &decode_layer_step);
+}
+
+}  // namespace fsa_host

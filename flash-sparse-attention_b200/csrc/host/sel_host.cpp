@@ -95,5 +95,3 @@ void bind_sel(pybind11::module& m) {
 }
 
 }  // namespace fsa_host
-
-PYBIND11_MODULE(_fsa_host, m) { fsa_host::bind_sel(m); }

@@ -104,6 +104,18 @@ SIGNATURES = {
         [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
          c_float, c_void_p, c_void_p, c_void_p, c_int64, c_void_p],
     ),
+    "fsa_decode_proj": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "fsa_decode_append": (
+        c_int,
+        [c_void_p] * 9 + [c_void_p, c_void_p] + [c_int] * 6 + [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p]),
+    "fsa_decode_compress": (c_int, [c_void_p] * 10 + [c_int] * 7 + [c_void_p]),
+    "fsa_decode_cmp_partial": (
+        c_int,
+        [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p] + [c_int] * 9
+        + [c_float, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
+    "fsa_decode_merge_select": (
+        c_int,
+        [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p] + [c_int] * 14 + [c_void_p] * 5),
     "fsa_decode_read_status": (c_int, [c_void_p]),
     "fsa_decode_finish": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                   c_void_p]),

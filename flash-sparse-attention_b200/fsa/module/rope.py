@@ -98,12 +98,15 @@ class RotaryEmbedding(nn.Module):
     def inv_freq(self) -> torch.Tensor:
         return self._inv_freq
 
+    def inv_freq_on(self, device) -> torch.Tensor:
+        if self._inv_freq.device != device:
+            self._inv_freq = self._inv_freq.to(device)
+        return self._inv_freq
+
     @torch.no_grad()
     def generate_cos_sin(self, x: torch.Tensor, position_ids: torch.Tensor):
         """cos / sin ``[len, head_dim/2]`` for the given positions, angles in fp32, rounded to x.dtype (rope.py:102-124)."""
-        if self._inv_freq.device != position_ids.device:
-            self._inv_freq = self._inv_freq.to(position_ids.device)
-        freqs = position_ids.float()[:, None] * self._inv_freq[None, :]
+        freqs = position_ids.float()[:, None] * self.inv_freq_on(position_ids.device)[None, :]
         return (freqs.cos() * self.attention_scaling).to(x.dtype), (freqs.sin() * self.attention_scaling).to(x.dtype)
 
     def forward(self, x: torch.Tensor, cu_seqlens: torch.Tensor, start: int = 0, stride: int = 1, max_seqlen: int | None = None):

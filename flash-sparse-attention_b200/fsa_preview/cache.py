@@ -75,6 +75,17 @@ class DecodeCache:
         self.seq_len.copy_(torch.tensor(self.host_len, dtype=torch.int32))
 
     # ---------------------------------------------------------------- one token per sequence
+    def buffers(self):
+        """The tensors that the native step works on."""
+        return [self.k, self.v, self.cmp_k, self.cmp_v, self.k_tail, self.v_tail, self.seq_len, self.seq_row0, self.cmp_row0]
+
+    def advance(self) -> bool:
+        """Count one more token per sequence on the host; does the compressor have to run (it looks at the device-side lengths
+        itself, so it may run for nothing)?"""
+        ks, stride = self.ks, self.stride
+        self.host_len = new = [L + 1 for L in self.host_len]
+        return self.always_compress or any(L >= ks and (L - ks) % stride == 0 for L in new)
+
     @torch.no_grad()
     def append(self, k_raw: torch.Tensor, k_rot: torch.Tensor, v: torch.Tensor, compress_key: torch.Tensor,
                compress_value: torch.Tensor, intra_block_pe: Optional[torch.Tensor],
@@ -92,9 +103,7 @@ class DecodeCache:
         self.k_tail.index_copy_(0, ring, k_raw)
         self.v_tail.index_copy_(0, ring, v)
         self.seq_len += 1
-        new_host = [L + 1 for L in self.host_len]
-        self.host_len = new_host
-        if not self.always_compress and not any(L >= self.ks and (L - self.ks) % self.stride == 0 for L in new_host):
+        if not self.advance():
             return
         n = t + 1
         emit = (n >= self.ks) & ((n - self.ks) % self.stride == 0)

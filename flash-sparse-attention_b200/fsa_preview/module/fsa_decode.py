@@ -11,12 +11,14 @@ from typing import Optional, Sequence
 import torch
 
 from fsa import _lib
+from fsa._host import host
 from fsa.module.rope import RopeConfig, RotaryEmbedding
 from fsa.ops.gate import gate_mix
 from fsa.ops.linear_compress import compressed_seqlens, linear_compress
 from fsa_preview.cache import DecodeCache
 from fsa_preview.ops.compat import _linear_compress_decode
-from fsa_preview.ops.decode import Shard, nsa_decode_attention, nsa_decode_mixed
+from fsa_preview.module.fsa_decode_kernel import plain_gate, plain_linear
+from fsa_preview.ops.decode import Shard, nsa_decode_attention, step_settings
 
 
 class FlashSparseAttentionDecode(torch.nn.Module):
@@ -86,6 +88,14 @@ class FlashSparseAttentionDecode(torch.nn.Module):
     def step(self, x: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """``x [B, hidden]``: one new token per sequence -> ``[B, hidden]``; appends to ``cache``."""
         B = x.shape[0]
+        if (cache.shard.world == 1 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v)
+                and plain_linear(self.proj_o) and plain_gate(self.gate) and type(self.rope) is RotaryEmbedding):
+            compress = cache.advance()
+            y, self.last_topk_idx = host().decode_layer_step(
+                x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.proj_o.weight, self.gate[0].weight,
+                self.rope.inv_freq_on(x.device), self.head_dim, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
+                compress, step_settings(self, cache.max_len), 0.0)
+            return y
         pos = cache.seq_len.clone()                                   # position of the new token
         q = self.proj_q(x).view(B, self.num_q_heads, self.head_dim)
         k_new = self.proj_k(x).view(B, self.num_kv_heads, self.head_dim)
@@ -93,11 +103,6 @@ class FlashSparseAttentionDecode(torch.nn.Module):
         q = self.rope_at(q, pos)
         cache.append(k_new, self.rope_at(k_new, pos), v_new, self.compress_key, self.compress_value, self.intra_block_pe, self.rope_at)
         gate = self.gate(x)
-        if cache.shard.world == 1:
-            mixed, idx = nsa_decode_mixed(q, cache.k, cache.v, cache.cmp_k, cache.cmp_v, cache.seq_len, cache.seq_row0,
-                                          cache.cmp_row0, gate, max_len=cache.max_len, **self._nsa())
-            self.last_topk_idx = idx
-            return self.proj_o(mixed.flatten(1))
         oc, os_, ow, *_, idx = nsa_decode_attention(q, cache.k, cache.v, cache.cmp_k, cache.cmp_v, cache.seq_len, cache.seq_row0,
                                                     cache.cmp_row0, max_len=cache.max_len, shard=cache.shard, **self._nsa())
         self.last_topk_idx = idx

@@ -6,10 +6,21 @@ from typing import Optional
 
 import torch
 
+from fsa._host import host
 from fsa.ops.gate import gate_mix
 from fsa_preview.cache import DecodeCache
 from fsa_preview.ops.compat import _linear_compress_decode
-from fsa_preview.ops.decode import Shard, nsa_decode_attention, nsa_decode_mixed
+from fsa_preview.ops.decode import Shard, nsa_decode_attention, step_settings
+
+
+def plain_linear(m: torch.nn.Module) -> bool:
+    """Nothing but ``x W^T``: no subclass, bias or hook that a call of the module would run."""
+    return type(m) is torch.nn.Linear and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks)
+
+
+def plain_gate(m: torch.nn.Module) -> bool:
+    return (type(m) is torch.nn.Sequential and len(m) == 2 and plain_linear(m[0]) and type(m[1]) is torch.nn.Sigmoid
+            and not (m._forward_hooks or m._forward_pre_hooks or m[1]._forward_hooks or m[1]._forward_pre_hooks))
 
 
 class FlashSparseAttentionDecodeKernel(torch.nn.Module):
@@ -43,14 +54,15 @@ class FlashSparseAttentionDecodeKernel(torch.nn.Module):
     @torch.no_grad()
     def step(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """One token per sequence: ``q [B, Hq, d]``, ``k_new / v_new [B, Hk, d]`` -> ``[B, Hq*d]``; appends to ``cache``."""
+        if cache.shard.world == 1 and plain_gate(self.gate):
+            compress = cache.advance()
+            out, self.last_topk_idx = host().decode_kernel_step(
+                q, k_new, v_new, self.gate[0].weight, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
+                compress, step_settings(self, cache.max_len), 0.0)
+            return out
         cache.append(k_new, k_new, v_new, self.compress_key, self.compress_value, self.intra_block_pe, None)
         q = q.contiguous()
         gate = self.gate(q.view(q.shape[0], -1))
-        if cache.shard.world == 1:
-            mixed, idx = nsa_decode_mixed(q, cache.k, cache.v, cache.cmp_k, cache.cmp_v, cache.seq_len, cache.seq_row0,
-                                          cache.cmp_row0, gate, max_len=cache.max_len, **self._nsa())
-            self.last_topk_idx = idx
-            return mixed.flatten(1)
         oc, os_, ow, *_, idx = nsa_decode_attention(q, cache.k, cache.v, cache.cmp_k, cache.cmp_v, cache.seq_len, cache.seq_row0,
                                                     cache.cmp_row0, max_len=cache.max_len, shard=cache.shard, **self._nsa())
         self.last_topk_idx = idx

@@ -319,6 +319,45 @@ int fsa_decode_finish(const float* o_part, const float* ml, int64_t rows, int nu
                       int part_stride, int head_dim, int num_q_heads, int dtype, const void* o_cmp, const void* gate, void* out,
                       void* stream);
 
+/* ---- the fused kernels of a one-GPU step (what fsa_preview.module's step runs; the calls above are its parts) ----
+ *
+ * y_i[b, :] = x[b, :] W_i^T for up to four weight matrices [rows_i, k_dim] (contiguous) in one launch; batch <= 16,
+ * k_dim a multiple of 256 (else FSA_ERR_UNSUPPORTED: use a library GEMM).  Replaces the projections of
+ * fsa_preview/module/fsa_decode.py:76-83, :196. */
+int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k_dim, int num, const void* const* w, const int* rows,
+                    void* const* y, const int64_t* y_stride, int dtype, void* stream);
+
+/* Append one token per sequence: rotates q and k at position seq_len[b] (inv_freq null: they are rotated already and q is
+ * not touched), writes k and v to row seq_row0[b] + seq_len[b] of the caches and the raw k, v to the compressor's rings,
+ * gate[b, :] = sigmoid(gate_logits[b, :]) or sigmoid(gate_x[b, :] gate_w^T), then seq_len[b] += 1.  A token past `cap` goes
+ * to the spare row batch * cap.  fsa_preview/module/fsa_decode.py:84-139, :188. */
+int fsa_decode_append(const void* q_in, const void* k_in, const void* v_in, void* q_out, void* k_cache, void* v_cache, void* k_tail,
+                      void* v_tail, const float* inv_freq, int32_t* seq_len, const int32_t* seq_row0, int batch, int cap,
+                      int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, const void* gate_logits, const void* gate_x,
+                      const void* gate_w, int gate_dim, void* gate, int dtype, void* stream);
+
+/* The compressed token of every sequence whose length seq_len[b] completes a window, from the rings, to its row of the
+ * compressed caches (fsa_preview/ops/linear_compress_decode.py:14-76); keys get the bias of pe and, with inv_freq, are
+ * rotated at their window's first position. */
+int fsa_decode_compress(const void* k_tail, const void* v_tail, const void* w_key, const void* w_value, const void* pe,
+                        const float* inv_freq, const int32_t* seq_len, const int32_t* cmp_row0, void* cmp_k, void* cmp_v, int batch,
+                        int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int cmp_cap, int dtype, void* stream);
+
+/* fsa_decode_attn_partial over the visible compressed rows of every sequence (the ranges of fsa_decode_cmp_ranges without
+ * their arrays): num_chunks chunks of `chunk` rows. */
+int fsa_decode_cmp_partial(const void* q, const void* cmp_k, const void* cmp_v, int64_t cmp_rows, int64_t cmp_stride_n, const int32_t* seq_len,
+                           const int32_t* cmp_row0, int batch, int num_q_heads, int num_kv_heads, int head_dim, int kernel_size,
+                           int kernel_stride, int chunk, int num_chunks, int dtype, float sm_scale, float* o_part, float* ml,
+                           float* scores, int64_t scores_ld, void* stream);
+
+/* fsa_lse_merge of the compressed partials, fsa_decode_select_topk and fsa_decode_ranges (pieces of block_size rows) in one
+ * launch. */
+int fsa_decode_merge_select(const float* o_part, const float* ml, int num_partials, const float* scores, int64_t scores_ld,
+                            const int32_t* seq_len, const int32_t* seq_row0, int batch, int num_q_heads, int num_kv_heads, int head_dim,
+                            int kernel_size, int kernel_stride, int block_size, int init_blocks, int local_blocks, int topk,
+                            int max_blocks, int window, int num_window_pieces, int dtype, void* o_cmp, int32_t* topk_idx,
+                            int32_t* rng_lo, int32_t* rng_hi, void* stream);
+
 /* Top-k block ids for the decoded token of every sequence, from the scores buffer of the compressed branch
  * and its merged lse [B, Hq].  Same scoring, bf16 rounding and tie rule as fsa_select_topk_seq, evaluated at
  * t = seq_len[b] - 1 (the reference evaluates the "local blocks" rule at t = 0,
