@@ -380,7 +380,8 @@ __global__ void __launch_bounds__(256) decode_finish_kernel(const float* __restr
     const float g0 = (float)gate[b * 3], g1 = (float)gate[b * 3 + 1], g2 = (float)gate[b * 3 + 2];
     const float2* mlr = ml + row * PS;
     const float* src = o_part + row * PS * D;
-    float M[2], inv[2];
+    // lane i holds the weight of partial i of each segment (up to 32 per pass: longer lists take their weights from memory)
+    float inv[2], wl[2], M[2];
 #pragma unroll
     for (int seg = 0; seg < 2; ++seg) {
         const int p0 = seg ? ns : 0, pn = seg ? nw : ns;
@@ -392,27 +393,45 @@ __global__ void __launch_bounds__(256) decode_finish_kernel(const float* __restr
 #pragma unroll
         for (int o_ = 16; o_; o_ >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o_));
         float L = 0.f;
+        wl[seg] = 0.f;
         for (int i = lane; i < pn; i += 32) {
             float2 v = mlr[p0 + i];
-            if (v.y > 0.f) L += exp2f(v.x - m) * v.y;
+            const float w = v.y > 0.f ? exp2f(v.x - m) : 0.f;
+            if (i == lane) wl[seg] = w;
+            L += w * v.y;
         }
 #pragma unroll
         for (int o_ = 16; o_; o_ >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o_);
         M[seg] = m;
         inv[seg] = L > 0.f ? 1.f / L : 0.f;
     }
-    for (int d = lane * 4; d < D; d += 128) {
+    for (int d0 = 0; d0 < D; d0 += 128) {
+        const int d = d0 + lane * 4;
+        const bool in_row = d < D;
         float4 acc[2];
 #pragma unroll
         for (int seg = 0; seg < 2; ++seg) {
             const int p0 = seg ? ns : 0, pn = seg ? nw : ns;
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int i = 0; i < pn; ++i) {
-                const float2 v = mlr[p0 + i];
-                if (v.y > 0.f) {
-                    const float w = exp2f(v.x - M[seg]);
-                    const float4 x = *reinterpret_cast<const float4*>(src + (int64_t)(p0 + i) * D + d);
-                    a.x = fmaf(w, x.x, a.x); a.y = fmaf(w, x.y, a.y); a.z = fmaf(w, x.z, a.z); a.w = fmaf(w, x.w, a.w);
+            // eight rows in flight
+            for (int i0 = 0; i0 < pn; i0 += 8) {
+                float4 x[8];
+                float w[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int i = i0 + j;
+                    w[j] = 0.f;
+                    if (i < 32) w[j] = __shfl_sync(0xffffffffu, wl[seg], i & 31);
+                    else if (i < pn) {
+                        const float2 v = mlr[p0 + i];
+                        w[j] = v.y > 0.f ? exp2f(v.x - M[seg]) : 0.f;
+                    }
+                    if (i >= pn) w[j] = 0.f;
+                    x[j] = in_row && w[j] > 0.f ? *reinterpret_cast<const float4*>(src + (int64_t)(p0 + i) * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    a.x = fmaf(w[j], x[j].x, a.x); a.y = fmaf(w[j], x[j].y, a.y); a.z = fmaf(w[j], x[j].z, a.z); a.w = fmaf(w[j], x[j].w, a.w);
                 }
             }
             // round to the output type as the unfused path does
@@ -420,6 +439,7 @@ __global__ void __launch_bounds__(256) decode_finish_kernel(const float* __restr
             const float2 f0 = ElemTraits<ET>::unpack2(lo), f1 = ElemTraits<ET>::unpack2(hi);
             acc[seg] = make_float4(f0.x, f0.y, f1.x, f1.y);
         }
+        if (!in_row) continue;
         const uint2 cu_ = *reinterpret_cast<const uint2*>(o_cmp + row * D + d);
         const float2 c0 = ElemTraits<ET>::unpack2(cu_.x), c1 = ElemTraits<ET>::unpack2(cu_.y);
         uint2 o;

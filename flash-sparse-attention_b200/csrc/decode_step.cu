@@ -223,7 +223,7 @@ struct DecodeCompressParams {
 constexpr int kDcSplit = 8, kDcSeqs = 8, kDcPitch = 12;
 
 template <int D, typename ET>
-__global__ void __launch_bounds__(256) decode_compress_kernel(const DecodeCompressParams p) {
+__global__ void __launch_bounds__(256, 1) decode_compress_kernel(const DecodeCompressParams p) {
     namespace cg = cooperative_groups;
     constexpr int CG = D / 8, KL = 256 / CG;          // 16-byte column groups, reduction lanes
     extern __shared__ __align__(16) float dcs[];      // [KS][kDcPitch] inputs, later [8][kDcSeqs + 1][D] sums of the warps
@@ -259,16 +259,23 @@ __global__ void __launch_bounds__(256) decode_compress_kernel(const DecodeCompre
         __syncthreads();
         const int n = s_n;
         if (n == 0) break;                             // (the same for every CTA of the cluster)
-        for (int i = tid; i < KS * kDcPitch; i += 256) {
-            const int e = i / kDcPitch, a = i - e * kDcPitch;
-            float x = 0.f;
+        // eight inputs of one sequence (or of pe) per thread, transposed: the sequences of one input are adjacent
+        for (int i = tid; i < (kDcSeqs + 1) * (KS / 8); i += 256) {
+            const int a = i % (kDcSeqs + 1), e = i / (kDcSeqs + 1) * 8;
+            uint4 x = make_uint4(0u, 0u, 0u, 0u);
             if (a < n) {
                 const int b = s_act[a], kk = rank * KS + e, o = kk / D, d = kk - o * D;
-                x = (float)tail[(((int64_t)b * p.ks + (p.seq_len[b] + o) % p.ks) * p.Hk + h) * D + d];
+                x = *reinterpret_cast<const uint4*>(tail + (((int64_t)b * p.ks + (p.seq_len[b] + o) % p.ks) * p.Hk + h) * D + d);
             } else if (a == kDcSeqs && pe) {
-                x = (float)pe[e];
+                x = *reinterpret_cast<const uint4*>(pe + e);
             }
-            dcs[i] = x;
+            const uint32_t* px = &x.x;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = ElemTraits<ET>::unpack2(px[j]);
+                dcs[(e + 2 * j) * kDcPitch + a] = f.x;
+                dcs[(e + 2 * j + 1) * kDcPitch + a] = f.y;
+            }
         }
         __syncthreads();
         float acc[kDcSeqs + 1][8];
@@ -276,7 +283,7 @@ __global__ void __launch_bounds__(256) decode_compress_kernel(const DecodeCompre
         for (int a = 0; a <= kDcSeqs; ++a)
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
-#pragma unroll 4
+#pragma unroll 8
         for (int e = kl; e < KS; e += KL) {
             const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)e * D) + cgi);
             const uint32_t* pw = &wv.x;
@@ -364,43 +371,57 @@ struct DecodeSelectParams {
     int *rng_lo, *rng_hi;    // [B, Hk, T + npieces]
 };
 
-// The `want` largest of the keys in[0 .. n), all different, none 0: to out[0 .. want) in descending order (0 when they run
-// out).  One warp; every lane looks after every 32nd key and looks again only when its own was taken.  Destroys the keys.
-__device__ __forceinline__ void warp_largest(uint32_t* in, int n, int want, uint32_t* out, int lane) {
-    auto best = [&](int& at) {
-        uint32_t m = 0;
-        for (int i = lane; i < n; i += 32) {
-            const uint32_t v = in[i];
-            if (v > m) { m = v; at = i; }
-        }
-        return m;
-    };
-    int at = 0;
-    uint32_t mine = best(at);
-    for (int r = 0; r < want; ++r) {
-        const uint32_t m = __reduce_max_sync(0xffffffffu, mine);
-        if (lane == 0) out[r] = m;
-        if (m != 0 && mine == m) {
-            in[at] = 0;
-            mine = best(at);
+// The `want` <= 64 largest of the keys in[0 .. n), all different, none 0: to out[0 .. 64) in descending order, 0 behind them.
+// One warp, keys in registers: a round is one warp maximum and a handful of instructions.  More than 192 keys go in turns, the
+// best so far among the next ones.
+__device__ __forceinline__ void warp_largest(const uint32_t* in, int n, int want, uint32_t* out, int lane) {
+    constexpr int NR = 6;
+    out[lane] = 0; out[lane + 32] = 0;
+    __syncwarp();
+    int i0 = 0;
+    do {
+        uint32_t key[NR + 2];
+        key[0] = out[lane]; key[1] = out[lane + 32];
+#pragma unroll
+        for (int j = 0; j < NR; ++j) key[j + 2] = i0 + j * 32 + lane < n ? in[i0 + j * 32 + lane] : 0u;
+        __syncwarp();
+        for (int r = 0; r < want; ++r) {
+            uint32_t mine = key[0];
+#pragma unroll
+            for (int j = 1; j < NR + 2; ++j) mine = max(mine, key[j]);
+            const uint32_t m = __reduce_max_sync(0xffffffffu, mine);
+            if (lane == 0) out[r] = m;
+#pragma unroll
+            for (int j = 0; j < NR + 2; ++j) key[j] = key[j] == m ? 0u : key[j];
         }
         __syncwarp();
-    }
+        i0 += NR * 32;
+    } while (i0 < n);
 }
 
 template <typename ET>
 __global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectParams p) {
-    extern __shared__ uint32_t dks[];                 // [max_blocks] keys, then the probabilities
-    __shared__ float s_lse;
-    __shared__ uint32_t cand[8 * 64], sel[64];
+    extern __shared__ uint32_t dks[];                 // [max_blocks] keys, the probabilities, [G][P] merge weights
+    __shared__ float s_lse, s_inv[16];
+    __shared__ uint32_t cand[8 * 64], s_best[8 * 64], sel[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x / p.Hk, h = blockIdx.x % p.Hk;
     const int len = p.seq_len[b], t = len - 1;
     const int ncmp = len >= p.ks ? (len - p.ks) / p.stride + 1 : 0;
-    // ---- merge: a warp per head
+    const int bq = t / p.BK, nb = t >= 0 ? min(bq + 1, p.max_blocks) : 0;
+    const int bstride = p.BK / p.stride, pad = p.ks / p.stride - 1;
+    const int cmax = min(min(ncmp, nb * bstride + p.nw), (int)p.ld);
+    const float* row = p.scores + ((int64_t)b * p.Hk + h) * p.ld;
+    float* pv = reinterpret_cast<float*>(dks + p.max_blocks);
+    float* s_w = pv + p.max_blocks * bstride + p.nw;
+    // the first scores are on their way while the partials are merged
+    float v0[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v0[j] = j * 256 + tid < cmax ? row[j * 256 + tid] : 0.f;
+    // ---- merge: statistics and weights of a head by a warp, then the rows by all threads
+    const int64_t row0 = (int64_t)b * p.Hk * p.G + h * p.G;
     for (int g = warp; g < p.G; g += 8) {
-        const int64_t row = (int64_t)b * p.Hk * p.G + h * p.G + g;
-        const float2* mlr = p.ml + row * p.P;
+        const float2* mlr = p.ml + (row0 + g) * p.P;
         float M = -INFINITY;
         for (int i = lane; i < p.P; i += 32) {
             const float2 v = mlr[i];
@@ -411,50 +432,48 @@ __global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectPa
         float L = 0.f;
         for (int i = lane; i < p.P; i += 32) {
             const float2 v = mlr[i];
-            if (v.y > 0.f) L += exp2f(v.x - M) * v.y;
+            const float wt = v.y > 0.f ? exp2f(v.x - M) : 0.f;
+            L += wt * v.y;
+            s_w[g * p.P + i] = wt;
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-        if (g == 0 && lane == 0) s_lse = L > 0.f ? M + log2f(L) : -INFINITY;
-        const float inv = L > 0.f ? 1.f / L : 0.f;
-        const float* src = p.o_part + row * p.P * p.D;
-        for (int d = lane * 4; d < p.D; d += 128) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int i = 0; i < p.P; ++i) {
-                const float2 v = mlr[i];
-                if (v.y > 0.f) {
-                    const float wt = exp2f(v.x - M);
-                    const float4 x = *reinterpret_cast<const float4*>(src + (int64_t)i * p.D + d);
-                    acc.x = fmaf(wt, x.x, acc.x); acc.y = fmaf(wt, x.y, acc.y); acc.z = fmaf(wt, x.z, acc.z); acc.w = fmaf(wt, x.w, acc.w);
-                }
-            }
-            *reinterpret_cast<uint2*>((ET*)p.o_cmp + row * p.D + d) =
-                make_uint2(ElemTraits<ET>::pack2(acc.x * inv, acc.y * inv), ElemTraits<ET>::pack2(acc.z * inv, acc.w * inv));
+        if (lane == 0) {
+            s_inv[g] = L > 0.f ? 1.f / L : 0.f;
+            if (g == 0) s_lse = L > 0.f ? M + log2f(L) : -INFINITY;
         }
+    }
+    __syncthreads();
+    const float lse = s_lse;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (j * 256 + tid < cmax) pv[j * 256 + tid] = exp2f(v0[j] - lse);
+    for (int c = 2048 + tid; c < cmax; c += 256) pv[c] = exp2f(row[c] - lse);
+    for (int i = tid; i < p.G * (p.D / 4); i += 256) {
+        const int g = i / (p.D / 4), d = (i - g * (p.D / 4)) * 4;
+        const float* src = p.o_part + (row0 + g) * p.P * p.D + d;
+        const float* wg = s_w + g * p.P;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i0 = 0; i0 < p.P; i0 += 8) {
+            float4 x[8];
+            float wt[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                wt[j] = i0 + j < p.P ? wg[i0 + j] : 0.f;
+                x[j] = wt[j] > 0.f ? *reinterpret_cast<const float4*>(src + (int64_t)(i0 + j) * p.D) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                acc.x = fmaf(wt[j], x[j].x, acc.x); acc.y = fmaf(wt[j], x[j].y, acc.y);
+                acc.z = fmaf(wt[j], x[j].z, acc.z); acc.w = fmaf(wt[j], x[j].w, acc.w);
+            }
+        }
+        const float inv = s_inv[g];
+        *reinterpret_cast<uint2*>((ET*)p.o_cmp + (row0 + g) * p.D + d) =
+            make_uint2(ElemTraits<ET>::pack2(acc.x * inv, acc.y * inv), ElemTraits<ET>::pack2(acc.z * inv, acc.w * inv));
     }
     __syncthreads();
     // ---- block scores
-    const float lse = s_lse;
-    const float* row = p.scores + ((int64_t)b * p.Hk + h) * p.ld;
-    const int bq = t / p.BK, nb = t >= 0 ? min(bq + 1, p.max_blocks) : 0;
-    const int bstride = p.BK / p.stride, pad = p.ks / p.stride - 1;
-    float* pv = reinterpret_cast<float*>(dks + p.max_blocks);
-    const int cmax = min(min(ncmp, nb * bstride + p.nw), (int)p.ld);
-    for (int c0 = 0; c0 < cmax; c0 += 2048) {
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = c0 + j * 256 + tid;
-            v[j] = c < cmax ? row[c] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = c0 + j * 256 + tid;
-            if (c < cmax) pv[c] = exp2f(v[j] - lse);
-        }
-    }
-    __syncthreads();
     for (int blk = tid; blk < nb; blk += 256) {
         float s = 0.f;
         for (int o = 0; o < p.nw; ++o) {
@@ -470,9 +489,13 @@ __global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectPa
     // ---- top-k: the best T of every warp's share of the blocks, then the best T of those
     const int nsel = min(p.T, nb);
     const int share = (nb + 7) / 8, s0 = min(nb, warp * share), s1 = min(nb, s0 + share);
-    warp_largest(dks + s0, s1 - s0, nsel, cand + warp * nsel, lane);
+    warp_largest(dks + s0, s1 - s0, nsel, cand + warp * 64, lane);
     __syncthreads();
-    if (warp == 0) warp_largest(cand, 8 * nsel, nsel, sel, lane);
+    // the eight lists without the zeros behind them
+    if (tid < nsel)
+        for (int w = 0; w < 8; ++w) s_best[w * nsel + tid] = cand[w * 64 + tid];
+    __syncthreads();
+    if (warp == 0) warp_largest(s_best, 8 * nsel, nsel, sel, lane);
     __syncthreads();
     int32_t* out = p.topk + ((int64_t)b * p.Hk + h) * p.T;
     int* s_id = reinterpret_cast<int*>(cand);          // ascending ids, -1 behind them
@@ -611,7 +634,8 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
         return FSA_ERR_BAD_ARG;
     if (num_window_pieces > 0 && (int64_t)block_size * num_window_pieces < (int64_t)window + 1) return FSA_ERR_BAD_ARG;
     if (head_dim % 4 || misaligned({o_part}) || ((uintptr_t)o_cmp & 7)) return FSA_ERR_BAD_ARG;
-    if (kernel_size % kernel_stride || block_size % kernel_stride || topk > 64 || max_blocks > 65535) return FSA_ERR_UNSUPPORTED;
+    if (kernel_size % kernel_stride || block_size % kernel_stride || topk > 64 || max_blocks > 65535 || num_q_heads / num_kv_heads > 16)
+        return FSA_ERR_UNSUPPORTED;
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     DecodeSelectParams p;
     p.o_part = o_part; p.ml = (const float2*)ml; p.scores = scores; p.ld = scores_ld; p.seq_len = seq_len; p.seq_row0 = seq_row0;
@@ -625,7 +649,8 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
     for (int i = 0; i < a; ++i)
         for (int j = 0; j < bb; ++j) p.w[i + j] += 1.f;
     p.o_cmp = o_cmp; p.topk = topk_idx; p.rng_lo = rng_lo; p.rng_hi = rng_hi;
-    const int64_t smem = 4 * ((int64_t)max_blocks + (int64_t)max_blocks * bb + p.nw);      // keys, probabilities the blocks can touch
+    // keys, probabilities that the blocks can touch, merge weights
+    const int64_t smem = 4 * ((int64_t)max_blocks + (int64_t)max_blocks * bb + p.nw + (int64_t)p.G * num_partials);
     if (smem > 200 * 1024) return FSA_ERR_UNSUPPORTED;
     (void)cudaGetLastError();
     const void* kern = dtype == FSA_DTYPE_BF16 ? (const void*)decode_select_kernel<__nv_bfloat16> : (const void*)decode_select_kernel<__half>;

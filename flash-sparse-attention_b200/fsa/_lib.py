@@ -76,6 +76,9 @@ SIGNATURES = {
         c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p]),
     "fsa_linear_compress_fwd": (
         c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "fsa_compress_bias_scratch_bytes": (c_int64, [c_int, c_int]),
+    "fsa_compress_kv_fwd": (
+        c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4),
     "fsa_linear_compress_bwd": (
         c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                 c_void_p, c_void_p]),

@@ -201,6 +201,14 @@ int fsa_linear_compress_fwd(const void* x, int64_t x_stride_n, const void* w, co
                             int batch, int num_heads, int head_dim, int kernel_size, int kernel_stride, int dtype, void* y,
                             int32_t* status, void* stream);
 
+/* K and V compressed in one launch per 12 sequences, with the bias of the position embedding pe [H, ks, D] (or null) of the
+ * keys computed on the way: fsa_linear_compress_fwd twice plus the einsum of nsa_ref/ops/linear_compress.py:497-501.  v null:
+ * one tensor only.  scratch: fsa_compress_bias_scratch_bytes(), needed with pe. */
+int64_t fsa_compress_bias_scratch_bytes(int num_heads, int head_dim);
+int fsa_compress_kv_fwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
+                        const void* pe, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
+                        int kernel_stride, int dtype, void* yk, void* yv, float* scratch, void* stream);
+
 /* K/V compression backward without atomics: dx and dW of fsa_linear_compress_fwd from dy.  Replaces
  * linear_compress_bwd_kernel (nsa_ref/ops/linear_compress.py:135-292, launched at :401-470), which scatters both
  * gradients with fp32 tl.atomic_add (:275, :292); here every dx row and every dW row is written once from an fp32
