@@ -222,12 +222,16 @@ __global__ void __launch_bounds__(256) gate_proj_mix_fwd_kernel(const ET* __rest
 
 // Backward, per token: da = g0 do, db = g1 do, dc = g2 do; dg_j = sum(do * branch_j) rounded; dz_j = dg_j g_j (1 - g_j)
 // rounded (the sigmoid's backward in the activation dtype); dx[n, :] = sum_j dz_j Wg[j, :]; dz kept in fp32 for dWg.
-template <typename ET>
+// HV > 0: heads of HV 16-byte vectors; delta[j, h, n] = g_j sum over head h of do * branch_j, which is the sum of o dO that the
+// attention backward of branch j starts from (three passes over o and dO of their own otherwise: 0.79 ms of 64K tokens x 32
+// heads).
+template <int HV, typename ET>
 __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __restrict__ gate, const ET* __restrict__ wg,
                                                                 const ET* __restrict__ a, const ET* __restrict__ b,
                                                                 const ET* __restrict__ c, const ET* __restrict__ d_o, int64_t N,
                                                                 int hidden, int HD, ET* __restrict__ da, ET* __restrict__ db,
-                                                                ET* __restrict__ dc, ET* __restrict__ dx, float* __restrict__ dz) {
+                                                                ET* __restrict__ dc, ET* __restrict__ dx, float* __restrict__ dz,
+                                                                float* __restrict__ delta) {
     extern __shared__ __align__(16) uint8_t gsm[];
     uint4* sw = reinterpret_cast<uint4*>(gsm);
     const int hv = hidden / 8, vec = HD / 8;
@@ -256,18 +260,36 @@ __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __rest
                 if (v >= vec) continue;
                 const int64_t idx = n * vec + v;
                 const uint32_t *pd = &vd[u].x, *pa = &va[u].x, *pb = &vb[u].x, *pc = &vc[u].x;
+                float h0 = 0.f, h1 = 0.f, h2 = 0.f;       // this vector's share of its head
                 uint4 oa, ob, oc;
                 uint32_t *qa = &oa.x, *qb = &ob.x, *qc = &oc.x;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     float2 d = ElemTraits<ET>::unpack2(pd[i]);
                     float2 p = ElemTraits<ET>::unpack2(pa[i]), q = ElemTraits<ET>::unpack2(pb[i]), r = ElemTraits<ET>::unpack2(pc[i]);
-                    s0 += d.x * p.x + d.y * p.y;
-                    s1 += d.x * q.x + d.y * q.y;
-                    s2 += d.x * r.x + d.y * r.y;
+                    h0 += d.x * p.x + d.y * p.y;
+                    h1 += d.x * q.x + d.y * q.y;
+                    h2 += d.x * r.x + d.y * r.y;
                     qa[i] = ElemTraits<ET>::pack2(g0 * d.x, g0 * d.y);
                     qb[i] = ElemTraits<ET>::pack2(g1 * d.x, g1 * d.y);
                     qc[i] = ElemTraits<ET>::pack2(g2 * d.x, g2 * d.y);
+                }
+                s0 += h0; s1 += h1; s2 += h2;
+                if constexpr (HV > 0) {
+                    // (vec is a multiple of HV and HV divides 32: a head's vectors sit in neighbouring lanes of one iteration)
+                    const unsigned mask = HV == 32 ? 0xffffffffu : ((1u << HV) - 1) << (lane & ~(HV - 1));
+#pragma unroll
+                    for (int o = HV / 2; o; o >>= 1) {
+                        h0 += __shfl_xor_sync(mask, h0, o);
+                        h1 += __shfl_xor_sync(mask, h1, o);
+                        h2 += __shfl_xor_sync(mask, h2, o);
+                    }
+                    if ((lane & (HV - 1)) == 0) {
+                        const int64_t head = v / HV, heads = vec / HV;
+                        delta[head * N + n] = g0 * h0;
+                        delta[(heads + head) * N + n] = g1 * h1;
+                        delta[(2 * heads + head) * N + n] = g2 * h2;
+                    }
                 }
                 st_stream16(reinterpret_cast<uint4*>(da) + idx, oa);
                 st_stream16(reinterpret_cast<uint4*>(db) + idx, ob);
@@ -360,14 +382,14 @@ static int run_gate_fwd(const void* x, int64_t x_sn, const void* wg, const void*
 template <typename ET>
 static int run_gate_bwd(const void* x, int64_t x_sn, const void* wg, const void* gate, const void* a, const void* b, const void* c,
                         const void* d_o, int64_t N, int hidden, int HD, void* da, void* db, void* dc, void* dx, void* dwg, float* dz,
-                        float* partial, cudaStream_t stream) {
+                        float* partial, float* delta, int head_dim, cudaStream_t stream) {
     const int smem = 3 * hidden * 2;
-    auto kern = gate_proj_mix_bwd_kernel<ET>;
+    auto kern = !delta ? gate_proj_mix_bwd_kernel<0, ET> : head_dim == 128 ? gate_proj_mix_bwd_kernel<16, ET> : gate_proj_mix_bwd_kernel<8, ET>;
     if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
     const int64_t want = (N + 7) / 8;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
     kern<<<grid, 256, smem, stream>>>((const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,
-                                      HD, (ET*)da, (ET*)db, (ET*)dc, (ET*)dx, dz);
+                                      HD, (ET*)da, (ET*)db, (ET*)dc, (ET*)dx, dz, delta);
     const int chunk_tokens = (int)((N + kGateChunks - 1) / kGateChunks);
     const int chunks = (int)((N + chunk_tokens - 1) / chunk_tokens);
     gate_dw_partial_kernel<ET><<<dim3((unsigned)((hidden / 8 + 255) / 256), (unsigned)chunks), 256, 0, stream>>>((const ET*)x, x_sn, dz, N, hidden,
@@ -456,9 +478,10 @@ extern "C" int fsa_gate_proj_mix_fwd(const void* x, int64_t x_stride_n, const vo
     return FSA_ERR_BAD_ARG;
 }
 
-extern "C" int fsa_gate_proj_mix_bwd(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
+static int gate_bwd(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
                                      const void* c, const void* d_out, int64_t total, int hidden, int row_elems, int dtype, void* da, void* db,
-                                     void* dc, void* dx, void* dw_gate, float* scratch, int64_t scratch_bytes, void* stream) {
+                                     void* dc, void* dx, void* dw_gate, float* scratch, int64_t scratch_bytes, float* delta, int head_dim,
+                    void* stream) {
     if (total == 0) return FSA_OK;
     if (!x || !w_gate || !gate || !a || !b || !c || !d_out || !da || !db || !dc || !dx || !dw_gate || !scratch) return FSA_ERR_BAD_ARG;
     if (hidden <= 0 || hidden % 8 || row_elems % 8 || x_stride_n % 8) return FSA_ERR_BAD_ARG;
@@ -471,8 +494,25 @@ extern "C" int fsa_gate_proj_mix_bwd(const void* x, int64_t x_stride_n, const vo
     float* partial = scratch + (total * 3 + 3) / 4 * 4;
     (void)cudaGetLastError();
     if (dtype == FSA_DTYPE_BF16)
-        return run_gate_bwd<__nv_bfloat16>(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, row_elems, da, db, dc, dx, dw_gate, dz, partial, (cudaStream_t)stream);
+        return run_gate_bwd<__nv_bfloat16>(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, row_elems, da, db, dc, dx, dw_gate, dz, partial, delta, head_dim, (cudaStream_t)stream);
     if (dtype == FSA_DTYPE_FP16)
-        return run_gate_bwd<__half>(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, row_elems, da, db, dc, dx, dw_gate, dz, partial, (cudaStream_t)stream);
+        return run_gate_bwd<__half>(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, row_elems, da, db, dc, dx, dw_gate, dz, partial, delta, head_dim, (cudaStream_t)stream);
     return FSA_ERR_BAD_ARG;
+}
+
+extern "C" int fsa_gate_proj_mix_bwd(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
+                                     const void* c, const void* d_out, int64_t total, int hidden, int row_elems, int dtype, void* da, void* db,
+                                     void* dc, void* dx, void* dw_gate, float* scratch, int64_t scratch_bytes, void* stream) {
+    return gate_bwd(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, row_elems, dtype, da, db, dc, dx, dw_gate, scratch, scratch_bytes,
+                    nullptr, 0, stream);
+}
+
+extern "C" int fsa_gate_proj_mix_bwd_delta(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
+                                           const void* c, const void* d_out, int64_t total, int hidden, int num_heads, int head_dim, int dtype,
+                                           void* da, void* db, void* dc, void* dx, void* dw_gate, float* delta, float* scratch,
+                                           int64_t scratch_bytes, void* stream) {
+    if (!delta || num_heads <= 0) return FSA_ERR_BAD_ARG;
+    if (head_dim != 64 && head_dim != 128) return FSA_ERR_UNSUPPORTED;
+    return gate_bwd(x, x_stride_n, w_gate, gate, a, b, c, d_out, total, hidden, num_heads * head_dim, dtype, da, db, dc, dx, dw_gate, scratch,
+                    scratch_bytes, delta, head_dim, stream);
 }

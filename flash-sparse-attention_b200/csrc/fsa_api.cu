@@ -380,7 +380,7 @@ int fsa_sel_bwd_scratch_bytes(int64_t N, int B, int Hq, int Hk, int D, int T, in
 
 }  // extern "C"
 
-static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const void* k, const void* v, const void* o, const float* lse,
+static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, const void* q, const void* k, const void* v, const void* o, const float* lse,
                         const void* d_o, const int32_t* topk_idx, const int32_t* cu_seqlens, int64_t N, int B, int Hq, int Hk, int D, int T,
                 int BK, int dtype, int64_t q_sn, int64_t q_sh, int64_t k_sn, int64_t v_sn, int64_t o_sn, int64_t o_sh,
                 int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk, void* dv, void* index_ws,
@@ -395,7 +395,7 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     if (!(sm_scale > 0.f)) return FSA_ERR_BAD_ARG;
     if (N == 0) return FSA_OK;
-    if (!q || !k || !v || !o || !lse || !d_o || !cu_seqlens || !dq || !dk || !dv || !index_ws || !scratch)
+    if (!q || !k || !v || (!o && !delta) || !lse || !d_o || !cu_seqlens || !dq || !dk || !dv || !index_ws || !scratch)
         return FSA_ERR_BAD_ARG;
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dq) ||
         !aligned16(dk) || !aligned16(dv) || !aligned16(scratch) || !aligned16(index_ws))
@@ -422,7 +422,8 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
     a.lse = lse; a.topk_idx = topk_idx; a.cu = cu_seqlens; a.sm_scale = sm_scale;
     a.run = s.RB;
     char* sp = (char*)scratch;
-    a.delta = (float*)sp;   sp += align_up(N * Hq * 4, 1024);
+    a.delta = delta ? const_cast<float*>(delta) : (float*)sp;   sp += align_up(N * Hq * 4, 1024);
+    a.have_delta = delta != nullptr;
     a.dq_part = (void*)sp;  sp += bwd_dq_part_bytes(s);
     CUtensorMap dqmap;
     a.dqmap = nullptr;
@@ -449,7 +450,7 @@ int fsa_sel_bwd(const void* q, const void* k, const void* v, const void* o, cons
                 int BK, int dtype, int64_t q_sn, int64_t q_sh, int64_t k_sn, int64_t v_sn, int64_t o_sn, int64_t o_sh,
                 int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk, void* dv, void* index_ws,
                 int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream_) {
-    return sel_bwd_impl(SelBounds{nullptr, nullptr, nullptr}, N, q, k, v, o, lse, d_o, topk_idx, cu_seqlens, N, B, Hq, Hk, D, T, BK,
+    return sel_bwd_impl(SelBounds{nullptr, nullptr, nullptr}, N, nullptr, q, k, v, o, lse, d_o, topk_idx, cu_seqlens, N, B, Hq, Hk, D, T, BK,
                         dtype, q_sn, q_sh, k_sn, v_sn, o_sn, o_sh, do_sn, do_sh, sm_scale, dq, dk, dv, index_ws, index_ws_bytes,
                         scratch, scratch_bytes, stream_);
 }
@@ -461,9 +462,30 @@ int fsa_range_attn_bwd(const void* q, const void* k, const void* v, const void* 
                        float sm_scale, void* dq, void* dk, void* dv, void* index_ws, int64_t index_ws_bytes, void* scratch,
                        int64_t scratch_bytes, void* stream_) {
     if (!kv_hi || !cu_seqlens_k) return FSA_ERR_BAD_ARG;
-    return sel_bwd_impl(SelBounds{cu_seqlens_k, kv_lo, kv_hi}, Nk, q, k, v, o, lse, d_o, nullptr, cu_seqlens_q, N, B, Hq, Hk, D,
+    return sel_bwd_impl(SelBounds{cu_seqlens_k, kv_lo, kv_hi}, Nk, nullptr, q, k, v, o, lse, d_o, nullptr, cu_seqlens_q, N, B, Hq, Hk, D,
                         max_blocks, BK, dtype, q_sn, q_sh, k_sn, v_sn, o_sn, o_sh, do_sn, do_sh, sm_scale, dq, dk, dv, index_ws,
                         index_ws_bytes, scratch, scratch_bytes, stream_);
+}
+
+int fsa_sel_bwd_delta(const void* q, const void* k, const void* v, const float* lse, const void* d_o, const float* delta,
+                      const int32_t* topk_idx, const int32_t* cu_seqlens, int64_t N, int B, int Hq, int Hk, int D, int T, int BK, int dtype,
+                      int64_t q_sn, int64_t q_sh, int64_t k_sn, int64_t v_sn, int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk,
+                      void* dv, void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream_) {
+    if (!delta) return FSA_ERR_BAD_ARG;
+    return sel_bwd_impl(SelBounds{nullptr, nullptr, nullptr}, N, delta, q, k, v, nullptr, lse, d_o, topk_idx, cu_seqlens, N, B, Hq, Hk, D, T, BK,
+                        dtype, q_sn, q_sh, k_sn, v_sn, 0, 0, do_sn, do_sh, sm_scale, dq, dk, dv, index_ws, index_ws_bytes, scratch,
+                        scratch_bytes, stream_);
+}
+
+int fsa_range_attn_bwd_delta(const void* q, const void* k, const void* v, const float* lse, const void* d_o, const float* delta,
+                             const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi, int64_t N,
+                             int64_t Nk, int B, int Hq, int Hk, int D, int max_blocks, int BK, int dtype, int64_t q_sn, int64_t q_sh,
+                             int64_t k_sn, int64_t v_sn, int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk, void* dv,
+                             void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream_) {
+    if (!kv_hi || !cu_seqlens_k || !delta) return FSA_ERR_BAD_ARG;
+    return sel_bwd_impl(SelBounds{cu_seqlens_k, kv_lo, kv_hi}, Nk, delta, q, k, v, nullptr, lse, d_o, nullptr, cu_seqlens_q, N, B, Hq, Hk, D,
+                        max_blocks, BK, dtype, q_sn, q_sh, k_sn, v_sn, 0, 0, do_sn, do_sh, sm_scale, dq, dk, dv, index_ws, index_ws_bytes,
+                        scratch, scratch_bytes, stream_);
 }
 
 int fsa_range_attn_index(const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi,

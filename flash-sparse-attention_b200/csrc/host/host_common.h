@@ -54,7 +54,15 @@ inline bool wants_grad(std::initializer_list<const Tensor*> ts) {
     return false;
 }
 
+// selected attention (sel_host.cpp): o, lse and the index; dq, dk, dv from delta = sum_d o dO
+std::tuple<Tensor, Tensor, Tensor> sel_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, int64_t bs, const Tensor& cu,
+                                           double scale);
+std::tuple<Tensor, Tensor, Tensor> sel_bwd_delta(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& lse, const Tensor& dout,
+                                                 const float* delta, const Tensor& idx, int64_t bs, const Tensor& cu, double scale,
+                                                 const Tensor& ws);
+
 void bind_sel(pybind11::module& m);
 void bind_decode(pybind11::module& m);
+void bind_layer(pybind11::module& m);
 
 }  // namespace fsa_host

@@ -4,4 +4,5 @@
 PYBIND11_MODULE(_fsa_host, m) {
     fsa_host::bind_sel(m);
     fsa_host::bind_decode(m);
+    fsa_host::bind_layer(m);
 }

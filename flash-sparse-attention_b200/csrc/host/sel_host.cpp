@@ -52,6 +52,21 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q_, const Tensor& k_, c
     return {dq, dk, dv};
 }
 
+std::tuple<Tensor, Tensor, Tensor> sel_bwd_delta(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& lse, const Tensor& dout,
+                                                 const float* delta, const Tensor& idx, int64_t bs, const Tensor& cu, double scale,
+                                                 const Tensor& ws) {
+    const SelShapeArgs s = shape_of(q, k, idx, cu, bs);
+    int64_t nb = 0;
+    check(fsa_sel_bwd_scratch_bytes(s.N, s.B, s.Hq, s.Hk, s.D, s.T, s.bs, &nb), "fsa_sel_bwd_scratch_bytes");
+    const Tensor scratch = bytes(nb, q);
+    Tensor dq = at::empty_like(q), dk = at::empty({s.N, s.Hk, s.D}, q.options()), dv = at::empty_like(dk);
+    check(fsa_sel_bwd_delta(ptr(q), ptr(k), ptr(v), lse.data_ptr<float>(), ptr(dout), delta, iptr(idx), iptr(cu), s.N, s.B, s.Hq, s.Hk, s.D, s.T,
+                            s.bs, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1), (float)scale,
+                            ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
+          "fsa_sel_bwd_delta");
+    return {dq, dk, dv};
+}
+
 static void check_status(const Tensor& ws, const char* what) {
     static const bool on = [] {
         const char* v = getenv("FSA_CHECK_STATUS");

@@ -25,20 +25,29 @@ namespace fsa {
 int make_tile_map(CUtensorMap* map, const void* base, int dtype, int64_t rows, int64_t cols, int64_t row_stride, int box_rows);
 
 // ------------------------------------------------------------------------------------------------ dx
+// One launch takes up to kLbSeqs sequences (their tensor maps travel as kernel parameters) of up to two tensors (K and V).
+constexpr int kLbSeqs = 12, kLbTensors = 2;
+struct LcDxMaps {
+    CUtensorMap y[kLbTensors][kLbSeqs];     // dy of every sequence
+    CUtensorMap w[kLbTensors];
+};
 struct LcDxParams {
-    int n_cmp;          // windows of this sequence
-    int L;              // tokens of this sequence
-    int H, ks, stride;
-    int phases;         // phases per CTA
-    void* dx;           // first row of this sequence, [L, H, D] contiguous
+    int n_seq, H, ks, stride;
+    int phases;                 // phases per CTA
+    int tile0[kLbSeqs + 1];     // first tile (128 m) of every sequence
+    int n_cmp[kLbSeqs];         // windows of every sequence (0: no product, the gradient is the addends)
+    int L[kLbSeqs];             // tokens
+    int64_t tok0[kLbSeqs];      // first token
+    void* dx[kLbTensors];       // [N, H, D] contiguous
+    const void* add[kLbTensors][2];   // other gradients of the same tensor, added before the rounding (may be dx itself), or null
     int* status;
 };
+static_assert(sizeof(LcDxMaps) + sizeof(LcDxParams) <= 4096, "kernel parameters");
 
 constexpr int kLcDxStages = 4;
 
 template <int D, typename ET>
-__global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParams p, const __grid_constant__ CUtensorMap ymap,
-                                                                const __grid_constant__ CUtensorMap wmap) {
+__global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_constant__ LcDxMaps maps, const LcDxParams p) {
     constexpr int kA = 128 * 128, kB = D * 128;           // one stage: 128 rows of dy x 64 columns, D rows of W x 64 columns
     constexpr int KH = D / 64;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -51,7 +60,13 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
     uint64_t* acc_empty = bars + 2 * kLcDxStages + 2;   // [2]
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 2 * kLcDxStages + 4);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * 128, h = blockIdx.y, p0 = blockIdx.z * p.phases;
+    int seq = 0;
+    while (seq + 1 < p.n_seq && (int)blockIdx.x >= p.tile0[seq + 1]) ++seq;
+    const int tn = (int)blockIdx.y / p.H, h = (int)blockIdx.y % p.H;
+    const int m0 = ((int)blockIdx.x - p.tile0[seq]) * 128, p0 = blockIdx.z * p.phases;
+    const bool product = p.n_cmp[seq] > 0;
+    const CUtensorMap* ymap = &maps.y[tn][seq];
+    const CUtensorMap* wmap = &maps.w[tn];
     const int J = p.ks / p.stride;
     const int per_phase = J * KH;
     int* status = p.status;
@@ -59,8 +74,8 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
         for (int i = 0; i < kLcDxStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 128); }
         mbar_init_fence();
-        tma_prefetch_desc(&ymap);
-        tma_prefetch_desc(&wmap);
+        tma_prefetch_desc(ymap);
+        tma_prefetch_desc(wmap);
     }
     if (warp == 0) tmem_alloc(&tmem_slot, 2 * D);
     tc_fence_before();
@@ -71,7 +86,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
         // ---- producer: (dy shifted by j, W slice of offset p + j * stride), 64 reduction columns per stage
         bool ok = true;
         int i = 0;
-        for (int pi = 0; pi < p.phases && ok; ++pi) {
+        for (int pi = 0; pi < p.phases && ok && product; ++pi) {
             for (int q = 0; q < per_phase && ok; ++q, ++i) {
                 const int st = i % kLcDxStages;
                 if (lane == 0) {
@@ -79,10 +94,10 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
                     mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
                     const int j = q / KH, kh = q % KH;
                     const int k = p0 + pi + j * p.stride;
-                    tma_load_2d(smem_u32(sA + st * kA), &ymap, h * D + kh * 64, m0 - j, &full[st]);
+                    tma_load_2d(smem_u32(sA + st * kA), ymap, h * D + kh * 64, m0 - j, &full[st]);
 #pragma unroll
                     for (int nh = 0; nh < KH; ++nh)
-                        tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), &wmap, kh * 64, (h * p.ks + k) * D + nh * 64, &full[st]);
+                        tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), wmap, kh * 64, (h * p.ks + k) * D + nh * 64, &full[st]);
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
@@ -93,7 +108,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
         constexpr uint32_t idesc = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, false);
         bool ok = true;
         int i = 0;
-        for (int pi = 0; pi < p.phases && ok; ++pi) {
+        for (int pi = 0; pi < p.phases && ok && product; ++pi) {
             const int buf = pi & 1;
             ok = mbar_wait(&acc_empty[buf], ((pi >> 1) & 1) ^ 1, status) && ok;
             tc_fence_after();
@@ -122,25 +137,44 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
         bool ok = true;
         for (int pi = 0; pi < p.phases && ok; ++pi) {
             const int buf = pi & 1;
-            ok = mbar_wait(&acc_full[buf], (pi >> 1) & 1, status) && ok;
+            if (product) ok = mbar_wait(&acc_full[buf], (pi >> 1) & 1, status) && ok;
             tc_fence_after();
             const int64_t t = (int64_t)(m0 + r) * p.stride + p0 + pi;
-            const bool valid = ok && t < p.L;
-            ET* dst = reinterpret_cast<ET*>(p.dx) + (t * p.H + h) * D;
+            const bool valid = ok && t < p.L[seq];
+            const int64_t at = ((p.tok0[seq] + t) * p.H + h) * D;
+            ET* dst = reinterpret_cast<ET*>(p.dx[tn]) + at;
 #pragma unroll
             for (int cc = 0; cc < D; cc += 32) {
                 uint32_t v[32];
-                tmem_ld32(tbase + lane_off + buf * D + cc, v);
-                tmem_ld_wait();
+                if (product) {
+                    tmem_ld32(tbase + lane_off + buf * D + cc, v);
+                    tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = 0u;
+                }
                 if (valid) {
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
-                        uint4 u;
-                        u.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-                        u.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-                        u.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-                        u.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-                        *reinterpret_cast<uint4*>(dst + cc + q4 * 8) = u;
+                        float f[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[q4 * 8 + j]);
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {
+                            if (p.add[tn][a]) {
+                                const uint4 x = *reinterpret_cast<const uint4*>(reinterpret_cast<const ET*>(p.add[tn][a]) + at + cc + q4 * 8);
+                                const uint32_t* px = &x.x;
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float2 g = ElemTraits<ET>::unpack2(px[j]);
+                                    f[2 * j] += g.x;
+                                    f[2 * j + 1] += g.y;
+                                }
+                            }
+                        }
+                        *reinterpret_cast<uint4*>(dst + cc + q4 * 8) =
+                            make_uint4(ElemTraits<ET>::pack2(f[0], f[1]), ElemTraits<ET>::pack2(f[2], f[3]), ElemTraits<ET>::pack2(f[4], f[5]),
+                                       ElemTraits<ET>::pack2(f[6], f[7]));
                     }
                 }
             }
@@ -154,24 +188,29 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const LcDxParam
 }
 
 template <int D, typename ET>
-static cudaError_t launch_dx(const LcDxParams& p, const CUtensorMap& ymap, const CUtensorMap& wmap, cudaStream_t stream) {
+static cudaError_t launch_dx(const LcDxMaps& maps, const LcDxParams& p, int nt, cudaStream_t stream) {
     constexpr int smem = kLcDxStages * (128 * 128 + D * 128) + 256;
     auto kern = linear_compress_dx_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    const int m_rows = (p.L + p.stride - 1) / p.stride;
-    kern<<<dim3((unsigned)((m_rows + 127) / 128), (unsigned)p.H, (unsigned)(p.stride / p.phases)), 192, smem, stream>>>(p, ymap, wmap);
+    kern<<<dim3((unsigned)p.tile0[p.n_seq], (unsigned)(p.H * nt), (unsigned)(p.stride / p.phases)), 192, smem, stream>>>(maps, p);
     return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------------ dW
 template <typename ET>
 struct LcDwParams {
-    const ET* x;  int64_t x_sn;     // [N, H, D], token stride in elements
-    const ET* dy;                   // [sum n_b, H, D] contiguous
+    const ET* x[kLbTensors];  int64_t x_sn[kLbTensors];     // [N, H, D], token stride in elements
+    const ET* dy[kLbTensors];       // [sum n_b, H, D] contiguous
     const int32_t* cu;              // [batch + 1] token offsets
     int batch, H, ks, stride;
-    ET* dw;                         // [H, ks * D, D]
+    ET* dw[kLbTensors];             // [H, ks * D, D]
+    // bias of the position embedding (tensor 0 only; pe null: none): dW[h, r, :] += pe[h, r] dbias[h, :], dpe[h, r] = W[h, r, :] dbias[h, :],
+    // with dbias[h, :] the sum of its parts, rounded to the activation dtype
+    const ET *pe, *w;
+    ET* dpe;
+    const float* dbias;             // [parts][H][D]
+    int parts;
     int* status;
 };
 
@@ -191,7 +230,12 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
     uint64_t* acc_full = bars + 2 * kLcDwStages;
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 2 * kLcDwStages + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k0 = blockIdx.x * KPC, h = blockIdx.y;
+    const int k0 = blockIdx.x * KPC, h = blockIdx.y, tn = blockIdx.z;
+    const ET* x = p.x[tn];
+    const ET* dy = p.dy[tn];
+    const int64_t x_sn = p.x_sn[tn];
+    const bool with_pe = tn == 0 && p.pe != nullptr;
+    float* s_db = reinterpret_cast<float*>(bars + 2 * kLcDwStages + 2);      // [D] gradient of the bias
     int* status = p.status;
     if (tid == 0) {
         for (int i = 0; i < kLcDwStages; ++i) { mbar_init(&full[i], 128); mbar_init(&empty[i], 1); }
@@ -239,14 +283,14 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
                     const int r = xr0 + it * 8;
                     const bool valid = c0 + r < n;
                     const int64_t row = valid ? (int64_t)s_b + (int64_t)(c0 + r) * p.stride + x_k : 0;
-                    cp_async16(sx + sw128_chunk_off(r, xc & 7), p.x + row * p.x_sn + x_col, valid);
+                    cp_async16(sx + sw128_chunk_off(r, xc & 7), x + row * x_sn + x_col, valid);
                 }
 #pragma unroll
                 for (int it = 0; it < YIT; ++it) {
                     const int r = yr0 + it * YSTEP;
                     const bool valid = c0 + r < n;
                     const int64_t row = valid ? y0 + c0 + r : 0;
-                    cp_async16(sy + sw128_chunk_off(r, yc & 7), p.dy + (row * p.H + h) * D + yc * 8, valid);
+                    cp_async16(sy + sw128_chunk_off(r, yc & 7), dy + (row * p.H + h) * D + yc * 8, valid);
                 }
                 cp_async_mbar_arrive_noinc(&full[st]);
             }
@@ -282,11 +326,22 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
         const int r = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         bool ok = true;
+        const int64_t wrow = (int64_t)(h * p.ks + k0) * D + r;
+        float pe_r = 0.f, dpe = 0.f;
+        if (with_pe) {
+            if (r < D) {
+                float v = 0.f;
+                for (int i = 0; i < p.parts; ++i) v += __ldg(p.dbias + ((int64_t)i * p.H + h) * D + r);
+                s_db[r] = ElemTraits<ET>::unpack2(ElemTraits<ET>::pack2(v, 0.f)).x;
+            }
+            pe_r = (float)p.pe[wrow];
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         if (nitems > 0) {
             ok = mbar_wait(acc_full, 0, status);
             tc_fence_after();
         }
-        ET* dst = p.dw + ((int64_t)(h * p.ks + k0) * D + r) * D;
+        ET* dst = p.dw[tn] ? p.dw[tn] + wrow * D : nullptr;
 #pragma unroll
         for (int cc = 0; cc < D; cc += 32) {
             uint32_t v[32];
@@ -297,7 +352,22 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = 0u;
             }
-            if (ok) {
+            if (with_pe) {
+#pragma unroll
+                for (int q4 = 0; q4 < 4; ++q4) {
+                    const uint4 wv = __ldg(reinterpret_cast<const uint4*>(p.w + wrow * D + cc + q4 * 8));
+                    const uint32_t* pw = &wv.x;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = ElemTraits<ET>::unpack2(pw[j]);
+                        const float d0 = s_db[cc + q4 * 8 + 2 * j], d1 = s_db[cc + q4 * 8 + 2 * j + 1];
+                        dpe = fmaf(f.x, d0, fmaf(f.y, d1, dpe));
+                        v[q4 * 8 + 2 * j] = __float_as_uint(fmaf(pe_r, d0, __uint_as_float(v[q4 * 8 + 2 * j])));
+                        v[q4 * 8 + 2 * j + 1] = __float_as_uint(fmaf(pe_r, d1, __uint_as_float(v[q4 * 8 + 2 * j + 1])));
+                    }
+                }
+            }
+            if (ok && dst) {
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                     uint4 u;
@@ -309,6 +379,7 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
                 }
             }
         }
+        if (with_pe && p.dpe) p.dpe[wrow] = (ET)dpe;
     }
     tc_fence_before();
     __syncthreads();
@@ -316,54 +387,101 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
 }
 
 template <int D, typename ET>
-static cudaError_t launch_dw(const LcDwParams<ET>& p, cudaStream_t stream) {
-    constexpr int smem = kLcDwStages * (2 + D / 64) * 128 * 128 + 256;
+static cudaError_t launch_dw(const LcDwParams<ET>& p, int nt, cudaStream_t stream) {
+    constexpr int smem = kLcDwStages * (2 + D / 64) * 128 * 128 + 128 + D * 4;
     auto kern = linear_compress_dw_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3((unsigned)(p.ks / (128 / D)), (unsigned)p.H), 256, smem, stream>>>(p);
+    kern<<<dim3((unsigned)(p.ks / (128 / D)), (unsigned)p.H, (unsigned)nt), 256, smem, stream>>>(p);
     return cudaGetLastError();
 }
 
+// One tensor of a backward (K or V); dx and dw may be null.
+struct LcGrad {
+    const void* x;
+    int64_t x_sn;
+    const void *w, *dy;
+    void* dx;
+    const void* add[2];
+    void* dw;
+};
+struct LcPeGrad {
+    const void* pe;
+    void* dpe;
+    const float* dbias;
+    int parts;
+};
+
 template <typename ET>
-static int run_bwd(const void* x, int64_t x_stride_n, const void* w, const void* dy, const int32_t* cu_dev, const int32_t* seqlens_host,
-                   int batch, int H, int D, int ks, int stride, int dtype, void* dx, void* dw, int32_t* status, cudaStream_t stream) {
-    if (dx) {
-        CUtensorMap wmap;
-        int rc = make_tile_map(&wmap, w, dtype, (int64_t)H * ks * D, D, D, 64);
-        if (rc) return rc;
+static int run_bwd(const LcGrad* t, int nt, const LcPeGrad& pe, const int32_t* cu_dev, const int32_t* seqlens, int batch, int H, int D, int ks, int stride,
+                   int dtype, int32_t* status, cudaStream_t stream) {
+    if (t[0].dx) {
+        LcDxMaps maps;
+        LcDxParams p;
+        p.H = H; p.ks = ks; p.stride = stride; p.phases = stride < 4 ? stride : 4; p.status = status;
+        p.n_seq = 0; p.tile0[0] = 0;
+        for (int i = 0; i < nt; ++i) {
+            int rc = make_tile_map(&maps.w[i], t[i].w, dtype, (int64_t)H * ks * D, D, D, 64);
+            if (rc) return rc;
+            p.dx[i] = t[i].dx; p.add[i][0] = t[i].add[0]; p.add[i][1] = t[i].add[1];
+        }
         int64_t tok0 = 0, y0 = 0;
         const int64_t row_bytes = (int64_t)H * D * 2;
         for (int b = 0; b < batch; ++b) {
-            const int L = seqlens_host[b];
+            const int L = seqlens[b];
             if (L < 0) return FSA_ERR_BAD_ARG;
             const int n = L >= ks ? (L - ks) / stride + 1 : 0;
-            char* dx_b = (char*)dx + tok0 * row_bytes;
-            if (n == 0) {
-                // no window covers this sequence: its gradient is zero
-                if (L > 0 && cudaMemsetAsync(dx_b, 0, (size_t)(L * row_bytes), stream) != cudaSuccess) return FSA_ERR_CUDA;
-            } else {
-                CUtensorMap ymap;
-                rc = make_tile_map(&ymap, (const char*)dy + y0 * row_bytes, dtype, n, (int64_t)H * D, (int64_t)H * D, 128);
-                if (rc) return rc;
-                LcDxParams p;
-                p.n_cmp = n; p.L = L; p.H = H; p.ks = ks; p.stride = stride; p.phases = stride < 4 ? stride : 4;
-                p.dx = dx_b; p.status = status;
-                const cudaError_t e = D == 128 ? launch_dx<128, ET>(p, ymap, wmap, stream) : launch_dx<64, ET>(p, ymap, wmap, stream);
-                if (e != cudaSuccess) return FSA_ERR_CUDA;
+            if (L > 0) {
+                const int q = p.n_seq;
+                for (int i = 0; i < nt; ++i) {
+                    // (a sequence without a window loads nothing: any valid map does)
+                    int rc = make_tile_map(&maps.y[i][q], n > 0 ? (const char*)t[i].dy + y0 * row_bytes : (const char*)t[i].w, dtype, n > 0 ? n : 1,
+                                           n > 0 ? (int64_t)H * D : D, n > 0 ? (int64_t)H * D : D, 128);
+                    if (rc) return rc;
+                }
+                p.n_cmp[q] = n; p.L[q] = L; p.tok0[q] = tok0;
+                p.tile0[q + 1] = p.tile0[q] + ((L + stride - 1) / stride + 127) / 128;
+                ++p.n_seq;
             }
             tok0 += L;
             y0 += n;
+            if (p.n_seq == kLbSeqs || (b == batch - 1 && p.n_seq > 0)) {
+                const cudaError_t e = D == 128 ? launch_dx<128, ET>(maps, p, nt, stream) : launch_dx<64, ET>(maps, p, nt, stream);
+                if (e != cudaSuccess) return FSA_ERR_CUDA;
+                p.n_seq = 0;
+            }
         }
     }
-    if (dw) {
-        LcDwParams<ET> p;
-        p.x = (const ET*)x; p.x_sn = x_stride_n; p.dy = (const ET*)dy; p.cu = cu_dev;
-        p.batch = batch; p.H = H; p.ks = ks; p.stride = stride; p.dw = (ET*)dw; p.status = status;
-        const cudaError_t e = D == 128 ? launch_dw<128, ET>(p, stream) : launch_dw<64, ET>(p, stream);
+    if (t[0].dw || pe.dpe || (nt > 1 && t[1].dw)) {
+        LcDwParams<ET> p = {};
+        for (int i = 0; i < nt; ++i) {
+            p.x[i] = (const ET*)t[i].x; p.x_sn[i] = t[i].x_sn; p.dy[i] = (const ET*)t[i].dy; p.dw[i] = (ET*)t[i].dw;
+        }
+        p.cu = cu_dev; p.batch = batch; p.H = H; p.ks = ks; p.stride = stride; p.status = status;
+        p.pe = (const ET*)pe.pe; p.w = (const ET*)t[0].w; p.dpe = (ET*)pe.dpe; p.dbias = pe.dbias; p.parts = pe.parts;
+        const cudaError_t e = D == 128 ? launch_dw<128, ET>(p, nt, stream) : launch_dw<64, ET>(p, nt, stream);
         if (e != cudaSuccess) return FSA_ERR_CUDA;
     }
     return FSA_OK;
+}
+
+cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, cudaStream_t stream);
+
+constexpr int kBiasParts = 32;      // shares of the windows in the sum that is the bias's gradient
+
+static int check_bwd(const LcGrad& g, const int32_t* cu, const int32_t* seqlens, int batch, int H, int D, int ks, int stride, int dtype, int64_t* total) {
+    if (!g.x || !g.w || !cu || !seqlens || batch < 0 || H <= 0 || ks <= 0 || stride <= 0) return FSA_ERR_BAD_ARG;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    if (D != 64 && D != 128) return FSA_ERR_UNSUPPORTED;
+    if (ks % stride != 0 || (stride & (stride - 1)) != 0 || (ks & 1)) return FSA_ERR_UNSUPPORTED;
+    if (((uintptr_t)g.x & 15) || ((uintptr_t)g.w & 15) || ((uintptr_t)g.dy & 15) || ((uintptr_t)g.dx & 15) || ((uintptr_t)g.dw & 15) || (g.x_sn % 8))
+        return FSA_ERR_BAD_ARG;
+    if (((uintptr_t)g.add[0] & 15) || ((uintptr_t)g.add[1] & 15)) return FSA_ERR_BAD_ARG;
+    if (g.x_sn < (int64_t)H * D) return FSA_ERR_BAD_ARG;
+    *total = 0;
+    for (int b = 0; b < batch; ++b)
+        if (seqlens[b] >= ks) *total += (seqlens[b] - ks) / stride + 1;
+    return *total > 0 && !g.dy ? FSA_ERR_BAD_ARG : FSA_OK;
 }
 
 }  // namespace fsa
@@ -373,24 +491,41 @@ using namespace fsa;
 extern "C" int fsa_linear_compress_bwd(const void* x, int64_t x_stride_n, const void* w, const void* dy, const int32_t* cu_seqlens,
                                        const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
                                        int kernel_stride, int dtype, void* dx, void* dw, int32_t* status, void* stream_) {
-    if (!x || !w || !cu_seqlens || !seqlens_host || batch < 0 || num_heads <= 0 || kernel_size <= 0 || kernel_stride <= 0)
-        return FSA_ERR_BAD_ARG;
-    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
-    if (head_dim != 64 && head_dim != 128) return FSA_ERR_UNSUPPORTED;
-    if (kernel_size % kernel_stride != 0 || (kernel_stride & (kernel_stride - 1)) != 0 || (kernel_size & 1)) return FSA_ERR_UNSUPPORTED;
-    if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)dy & 15) || ((uintptr_t)dx & 15) || ((uintptr_t)dw & 15) || (x_stride_n % 8))
-        return FSA_ERR_BAD_ARG;
-    if (x_stride_n < (int64_t)num_heads * head_dim) return FSA_ERR_BAD_ARG;
-    int64_t total_y = 0;
-    for (int b = 0; b < batch; ++b)
-        if (seqlens_host[b] >= kernel_size) total_y += (seqlens_host[b] - kernel_size) / kernel_stride + 1;
-    if (total_y > 0 && !dy) return FSA_ERR_BAD_ARG;
+    const LcGrad g{x, x_stride_n, w, dy, dx, {nullptr, nullptr}, dw};
+    int64_t total = 0;
+    int rc = check_bwd(g, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, &total);
+    if (rc) return rc;
     (void)cudaGetLastError();
-    if (int rc_ctx = ensure_context()) return rc_ctx;
+    if ((rc = ensure_context())) return rc;
+    const LcPeGrad none{nullptr, nullptr, nullptr, 0};
     cudaStream_t stream = (cudaStream_t)stream_;
     return dtype == FSA_DTYPE_BF16
-               ? run_bwd<__nv_bfloat16>(x, x_stride_n, w, dy, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size,
-                                        kernel_stride, dtype, dx, dw, status, stream)
-               : run_bwd<__half>(x, x_stride_n, w, dy, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size,
-                                 kernel_stride, dtype, dx, dw, status, stream);
+               ? run_bwd<__nv_bfloat16>(&g, 1, none, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream)
+               : run_bwd<__half>(&g, 1, none, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream);
+}
+
+extern "C" int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kBiasParts * num_heads * head_dim * 4; }
+
+extern "C" int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
+                                   const void* pe, const void* dyk, const void* dyv, const void* dk_add, const void* dv_add0, const void* dv_add1,
+                                   const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
+                                   int kernel_stride, int dtype, void* dk, void* dv, void* dw_key, void* dw_value, void* dpe, float* scratch,
+                                   void* stream_) {
+    const LcGrad g[2] = {{k, k_stride_n, w_key, dyk, dk, {dk_add, nullptr}, dw_key}, {v, v_stride_n, w_value, dyv, dv, {dv_add0, dv_add1}, dw_value}};
+    int64_t total = 0;
+    for (int i = 0; i < 2; ++i) {
+        const int rc = check_bwd(g[i], cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, &total);
+        if (rc) return rc;
+    }
+    if (!dk || !dv || !pe || !scratch) return FSA_ERR_BAD_ARG;
+    (void)cudaGetLastError();
+    int rc = ensure_context();
+    if (rc) return rc;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    const int parts = total < 32 * kBiasParts ? (total < 32 ? 1 : (int)(total / 32)) : kBiasParts;
+    if (launch_column_sum(dtype, head_dim, dyk, total, num_heads, parts, scratch, stream) != cudaSuccess) return FSA_ERR_CUDA;
+    const LcPeGrad pg{pe, dpe, scratch, parts};
+    return dtype == FSA_DTYPE_BF16
+               ? run_bwd<__nv_bfloat16>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, nullptr, stream)
+               : run_bwd<__half>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, nullptr, stream);
 }

@@ -526,7 +526,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         e = cudaMemsetAsync(a.dk_acc, 0, kv_elems * 4 * 2, stream);   // dk_acc and dv_acc are adjacent
         if (e != cudaSuccess) return e;
     }
-    if (rows > 0) {
+    if (rows > 0 && !a.have_delta) {
         const int64_t rows_per_cta = 2 * (256 / (D / 8));
         unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
         sel_bwd_delta<ET><<<grid, 256, 0, stream>>>((const ET*)a.o, a.o_sn, a.o_sh, (const ET*)a.d_o, a.do_sn, a.do_sh,

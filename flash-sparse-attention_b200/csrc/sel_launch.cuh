@@ -50,6 +50,7 @@ struct SelBwdArgs {
     int run;           // tiles per scheduling run
     // scratch
     float* delta;      // [Hq, N]
+    bool have_delta;   // delta is the caller's: sum_d o dO is there already (o may be null)
     void* dq_part;     // [max_tiles * nsub * 128, D] input dtype
     const CUtensorMap* dqmap;   // over dq_part, box {64, 32}: partial stores of the pipelined kernel (null: not built)
     float* dk_acc;     // [N, Hk, D]; dv_acc follows immediately (unpipelined kernel: fp32 accumulators)

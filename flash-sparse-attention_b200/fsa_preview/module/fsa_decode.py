@@ -11,13 +11,12 @@ from typing import Optional, Sequence
 import torch
 
 from fsa import _lib
-from fsa._host import host
+from fsa._host import host, plain_gate, plain_linear
 from fsa.module.rope import RopeConfig, RotaryEmbedding
 from fsa.ops.gate import gate_mix
 from fsa.ops.linear_compress import compressed_seqlens, linear_compress
 from fsa_preview.cache import DecodeCache
 from fsa_preview.ops.compat import _linear_compress_decode
-from fsa_preview.module.fsa_decode_kernel import plain_gate, plain_linear
 from fsa_preview.ops.decode import Shard, nsa_decode_attention, step_settings
 
 

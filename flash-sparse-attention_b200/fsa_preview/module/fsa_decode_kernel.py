@@ -6,21 +6,11 @@ from typing import Optional
 
 import torch
 
-from fsa._host import host
+from fsa._host import host, plain_gate
 from fsa.ops.gate import gate_mix
 from fsa_preview.cache import DecodeCache
 from fsa_preview.ops.compat import _linear_compress_decode
 from fsa_preview.ops.decode import Shard, nsa_decode_attention, step_settings
-
-
-def plain_linear(m: torch.nn.Module) -> bool:
-    """Nothing but ``x W^T``: no subclass, bias or hook that a call of the module would run."""
-    return type(m) is torch.nn.Linear and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks)
-
-
-def plain_gate(m: torch.nn.Module) -> bool:
-    return (type(m) is torch.nn.Sequential and len(m) == 2 and plain_linear(m[0]) and type(m[1]) is torch.nn.Sigmoid
-            and not (m._forward_hooks or m._forward_pre_hooks or m[1]._forward_hooks or m[1]._forward_pre_hooks))
 
 
 class FlashSparseAttentionDecodeKernel(torch.nn.Module):

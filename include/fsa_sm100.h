@@ -283,6 +283,54 @@ int fsa_gate_proj_mix_bwd(const void* x, int64_t x_stride_n, const void* w_gate,
                           const void* c, const void* d_out, int64_t total, int hidden, int row_elems, int dtype, void* da, void* db,
                           void* dc, void* dx, void* dw_gate, float* scratch, int64_t scratch_bytes, void* stream);
 
+/* ------------------------------------------------------------------------------------------------
+ * The layer's pieces between its GEMMs, fused (what fsa.module.fsa runs; fsa/module/fsa.py:71-171).
+ *
+ * cos / sin tables [max_len, head_dim / 2] in the activation dtype for positions 0 .. max_len - 1 (inv_freq fp32, device), and
+ * cu_cmp [batch + 1], the compressed offsets. */
+int fsa_layer_prep(const int32_t* cu_seqlens, int batch, int64_t max_len, const float* inv_freq, int head_dim, int kernel_size,
+                   int kernel_stride, int dtype, void* cos_tab, void* sin_tab, int32_t* cu_cmp, void* stream);
+
+/* q and k rotated to q_out, k_out (contiguous), the compressed keys rotated in place at c * kernel_stride, and the row ranges
+ * of the dense branches per token: hi_cmp (compressed branch, -1: none), lo_win / hi_win (window); hi_cmp may be null. */
+int fsa_layer_rope_fwd(const void* q, int64_t q_stride_n, const void* k, int64_t k_stride_n, void* cmp_k, const void* cos_tab,
+                       const void* sin_tab, const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch, int64_t total, int64_t total_cmp,
+                       int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int window, int dtype,
+                       void* q_out, void* k_out, int32_t* hi_cmp, int32_t* lo_win, int32_t* hi_win, void* stream);
+
+/* dq = inverse rotation of dq0 + dq1 + dq2, dk of dk0 + dk1 (may be written over an input), dcmp_k in place. */
+int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const void* dk0, const void* dk1, void* dcmp_k,
+                       const void* cos_tab, const void* sin_tab, const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch,
+                       int64_t total, int64_t total_cmp, int num_q_heads, int num_kv_heads, int head_dim, int kernel_stride, int dtype,
+                       void* dq, void* dk, void* stream);
+
+/* fsa_gate_proj_mix_bwd that also gives delta [3][num_heads][total] fp32, the sum of o dO over every head of every branch. */
+int fsa_gate_proj_mix_bwd_delta(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
+                                const void* c, const void* d_out, int64_t total, int hidden, int num_heads, int head_dim, int dtype,
+                                void* da, void* db, void* dc, void* dx, void* dw_gate, float* delta, float* scratch,
+                                int64_t scratch_bytes, void* stream);
+
+/* fsa_sel_bwd / fsa_range_attn_bwd with delta [Hq, N] (sum_d o dO) given instead of o. */
+int fsa_sel_bwd_delta(const void* q, const void* k, const void* v, const float* lse, const void* d_o, const float* delta,
+                      const int32_t* topk_idx, const int32_t* cu_seqlens, int64_t N, int B, int Hq, int Hk, int D, int T, int BK, int dtype,
+                      int64_t q_sn, int64_t q_sh, int64_t k_sn, int64_t v_sn, int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk,
+                      void* dv, void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream);
+int fsa_range_attn_bwd_delta(const void* q, const void* k, const void* v, const float* lse, const void* d_o, const float* delta,
+                             const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi, int64_t N,
+                             int64_t Nk, int B, int Hq, int Hk, int D, int max_blocks, int BK, int dtype, int64_t q_sn, int64_t q_sh,
+                             int64_t k_sn, int64_t v_sn, int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk, void* dv,
+                             void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream);
+
+/* Backward of fsa_compress_kv_fwd: dk = gradient through the compressor + dk_add, dv likewise + dv_add0 + dv_add1 (addends
+ * [total, H, D] contiguous, may be the output itself, or null), dw_key with the share of the bias, dw_value, dpe (each may be
+ * null).  scratch: fsa_compress_kv_bwd_scratch_bytes(). */
+int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim);
+int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
+                        const void* pe, const void* dyk, const void* dyv, const void* dk_add, const void* dv_add0, const void* dv_add1,
+                        const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
+                        int kernel_stride, int dtype, void* dk, void* dv, void* dw_key, void* dw_value, void* dpe, float* scratch,
+                        void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * One-step decode (fsa_preview)
  * ------------------------------------------------------------------------------------------- */
