@@ -1,9 +1,11 @@
 // The layer between x and its output projection as one native autograd function: projections, compression, rotation, the three
 // branches, block selection and the gate mix.  Seen as one function, the backward needs no pass over [N, hidden] or
 // [N, heads, d] just to add gradients: the gate's backward starts dx and the GEMMs accumulate into it, the rotation's backward
-// sums the branches' dq and dk, the compressor's backward adds its share to theirs, and the gate's backward delivers the
+// sums what the branches and the compressor give of dq, dk and dv, and the gate's backward delivers the
 // sums of o dO that the attention backwards start from.
 #include "host_common.h"
+
+#include <cuda_runtime_api.h>
 
 namespace fsa_host {
 
@@ -138,6 +140,7 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         const LayerCfg c = layer_cfg(ctx->saved_data["cfg"].toIntVector());
         const Lengths s(ctx->saved_data["seqlens"].toIntVector(), c);
         c10::cuda::CUDAGuard guard(x.device());
+        cudaSetDevice(x.get_device());      // (binds the context to the engine's thread: the first GEMM below wants one)
         const int64_t N = s.N, hidden = x.size(1);
         const int dt = dtype_code(x);
         const float scale = (float)(1.0 / std::sqrt((double)c.D));
@@ -161,20 +164,23 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         d_sel.reset();
         auto [dq2, dk2, dv2] = range_bwd(q, k, v, lse_win, d_win, dl + 2 * (int64_t)c.Hq * N, cu, cu, bd + N, bd + 2 * N, s.win_blocks(c), scale);
         d_win.reset();
-        check(fsa_layer_rope_bwd(ptr(dq0), ptr(dq1), ptr(dq2), ptr(dk), ptr(dk2), ptr(dck), ptr(cs), ptr(sn), iptr(cu), iptr(cu_cmp), s.B, N, s.Nc, c.Hq,
-                                 c.Hk, c.D, c.stride, dt, ptr(dq0), ptr(dk), st),
-              "fsa_layer_rope_bwd");
-        dq1.reset(); dq2.reset();
+        auto rope_bwd = [&](int64_t n, int64_t nc, const Tensor& dkc, const Tensor& dvc) {
+            check(fsa_layer_rope_bwd(ptr(dq0), ptr(dq1), ptr(dq2), ptr(dk), ptr(dk2), ptr(dkc), ptr(dv), ptr(dv2), ptr(dvc), ptr(dck), ptr(cs), ptr(sn),
+                                     iptr(cu), iptr(cu_cmp), s.B, n, nc, c.Hq, c.Hk, c.D, c.stride, dt, ptr(dq0), ptr(dk), ptr(dv), st),
+                  "fsa_layer_rope_bwd");
+        };
+        rope_bwd(0, s.Nc, Tensor(), Tensor());
         Tensor dw_key = ctx->needs_input_grad(5) ? at::empty_like(w_key) : Tensor(), dw_value = ctx->needs_input_grad(6) ? at::empty_like(w_value) : Tensor(),
                dpe = ctx->needs_input_grad(7) ? at::empty_like(pe) : Tensor();
         {
-            const Tensor scratch = bytes(fsa_compress_kv_bwd_scratch_bytes(c.Hk, c.D), x);
-            check(fsa_compress_kv_bwd(ptr(k_raw), k_raw.stride(0), ptr(v), v.stride(0), ptr(w_key), ptr(w_value), ptr(pe), ptr(dck), ptr(dcv), ptr(dk),
-                                      ptr(dv), ptr(dv2), iptr(cu), s.tok.data(), s.B, c.Hk, c.D, c.ks, c.stride, dt, ptr(dk), ptr(dv), ptr(dw_key),
-                                      ptr(dw_value), ptr(dpe), (float*)ptr(scratch), st),
+            const Tensor dkc = at::empty_like(dk), dvc = at::empty_like(dv), scratch = bytes(fsa_compress_kv_bwd_scratch_bytes(c.Hk, c.D), x);
+            check(fsa_compress_kv_bwd(ptr(k_raw), k_raw.stride(0), ptr(v), v.stride(0), ptr(w_key), ptr(w_value), ptr(pe), ptr(dck), ptr(dcv), iptr(cu),
+                                      s.tok.data(), s.B, c.Hk, c.D, c.ks, c.stride, dt, ptr(dkc), ptr(dvc), ptr(dw_key), ptr(dw_value), ptr(dpe),
+                                      (float*)ptr(scratch), st),
                   "fsa_compress_kv_bwd");
+            rope_bwd(N, 0, dkc, dvc);
         }
-        dk2.reset(); dv2.reset(); dck.reset(); dcv.reset();
+        dq1.reset(); dq2.reset(); dk2.reset(); dv2.reset(); dck.reset(); dcv.reset();
         const Tensor gq = dq0.view({N, -1}), gk = dk.view({N, -1}), gv = dv.view({N, -1});
         Tensor dwq, dwk, dwv;
         if (ctx->needs_input_grad(1)) dwq = at::mm(gq.t(), x);

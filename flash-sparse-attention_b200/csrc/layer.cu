@@ -42,19 +42,21 @@ __global__ void __launch_bounds__(256) layer_prep_kernel(const int* __restrict__
     }
 }
 
-// out1 = x1 cos - x2 sin, out2 = x1 sin + x2 cos on eight pairs
+// (x1, x2) = (x1 cos - x2 sin, x1 sin + x2 cos) on eight pairs
 template <typename ET>
-__device__ __forceinline__ void rotate8(const float (&x1)[8], const float (&x2)[8], const ET* cs, const ET* sn, float sign, uint4& o1, uint4& o2) {
+__device__ __forceinline__ void rotate8(float (&x1)[8], float (&x2)[8], const ET* cs, const ET* sn, float sign) {
     const uint4 co = __ldg(reinterpret_cast<const uint4*>(cs)), si = __ldg(reinterpret_cast<const uint4*>(sn));
     const uint32_t *pc = &co.x, *ps = &si.x;
-    uint32_t *q1 = &o1.x, *q2 = &o2.x;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float2 c = ElemTraits<ET>::unpack2(pc[i]);
         float2 s = ElemTraits<ET>::unpack2(ps[i]);
         s.x *= sign; s.y *= sign;
-        q1[i] = ElemTraits<ET>::pack2(x1[2 * i] * c.x - x2[2 * i] * s.x, x1[2 * i + 1] * c.y - x2[2 * i + 1] * s.y);
-        q2[i] = ElemTraits<ET>::pack2(x1[2 * i] * s.x + x2[2 * i] * c.x, x1[2 * i + 1] * s.y + x2[2 * i + 1] * c.y);
+        const float a0 = x1[2 * i], b0 = x2[2 * i], a1 = x1[2 * i + 1], b1 = x2[2 * i + 1];
+        x1[2 * i] = a0 * c.x - b0 * s.x;
+        x2[2 * i] = a0 * s.x + b0 * c.x;
+        x1[2 * i + 1] = a1 * c.y - b1 * s.y;
+        x2[2 * i + 1] = a1 * s.y + b1 * c.y;
     }
 }
 template <typename ET>
@@ -73,32 +75,30 @@ struct LayerRopeParams {
     int B, Hq, Hk, D, ks, stride, window;
     int64_t N, Nc;
     const void *cs, *sn;
-    // forward: q[0], k[0] in; backward: the gradients of the branches, summed before the rotation (q: 3, k: 2)
+    // forward: q[0], k[0] in; backward: the gradients of the branches, summed before the rotation (q: 3, k: 2; k[2], that of the
+    // unrotated keys, and all of v after it)
     const void* q[3];
-    const void* k[2];
+    const void* k[3];
+    const void* v[3];
     int64_t q_sn, k_sn;         // token strides of q[0], k[0] (forward; the gradients are contiguous)
-    void *q_out, *k_out;        // contiguous
+    void *q_out, *k_out, *v_out;     // contiguous
     void* cmp;                  // [Nc, Hk, D] rotated in place: compressed keys or their gradient
     int *hi_cmp, *lo_win, *hi_win;   // [N] or null: row ranges of the dense branches (nsa_ref/ops/compressed_attention.py:77-80; the window)
 };
 
 // One thread = eight pairs of one row; rows of q, then of k, then of the compressed keys (whose position is their row times the
-// stride, so the same tables serve them).
+// stride, so the same tables serve them), then of v (backward: sums only).
 template <bool BWD, typename ET>
 __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p) {
     const int half = p.D / 2, vec = half / 8;
     const int64_t nq = p.N * p.Hq * vec, nk = p.N * p.Hk * vec, nc = p.Nc * p.Hk * vec;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq + nk + nc) return;
-    const int kind = i < nq ? 0 : i < nq + nk ? 1 : 2;
-    i -= kind == 0 ? 0 : kind == 1 ? nq : nq + nk;
+    if (i >= nq + nk + nc + (BWD ? nk : 0)) return;
+    const int kind = i < nq ? 0 : i < nq + nk ? 1 : i < nq + nk + nc ? 2 : 3;
+    i -= kind == 0 ? 0 : kind == 1 ? nq : kind == 2 ? nq + nk : nq + nk + nc;
     const int H = kind == 0 ? p.Hq : p.Hk;
     const uint32_t i32 = (uint32_t)i;                  // (N * Hq * D / 16 fits in 32 bits: checked on the host)
     const int v = (int)(i32 % (uint32_t)vec), h = (int)(i32 / (uint32_t)vec % (uint32_t)H), n = (int)(i32 / (uint32_t)(vec * H));
-    const int* cu = kind == 2 ? p.cu_cmp : p.cu;
-    const int b = find_seq(cu, p.B, n);
-    const int pos = n - __ldg(cu + b);
-    const int64_t trow = (int64_t)(kind == 2 ? pos * p.stride : pos) * half + v * 8;
     const int64_t at = ((int64_t)n * H + h) * p.D + v * 8;       // contiguous element
     float x1[8], x2[8];
 #pragma unroll
@@ -108,6 +108,26 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
         add8<ET>(*reinterpret_cast<const uint4*>(s), x1);
         add8<ET>(*reinterpret_cast<const uint4*>(s + half), x2);
     };
+    auto put = [&](void* dst, const float (&y1)[8], const float (&y2)[8]) {
+        uint4 o1, o2;
+        uint32_t *q1 = &o1.x, *q2 = &o2.x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            q1[j] = ElemTraits<ET>::pack2(y1[2 * j], y1[2 * j + 1]);
+            q2[j] = ElemTraits<ET>::pack2(y2[2 * j], y2[2 * j + 1]);
+        }
+        *reinterpret_cast<uint4*>((ET*)dst + at) = o1;
+        *reinterpret_cast<uint4*>((ET*)dst + at + half) = o2;
+    };
+    if (BWD && kind == 3) {
+        take(p.v[0], at); take(p.v[1], at); take(p.v[2], at);
+        put(p.v_out, x1, x2);
+        return;
+    }
+    const int* cu = kind == 2 ? p.cu_cmp : p.cu;
+    const int b = find_seq(cu, p.B, n);
+    const int pos = n - __ldg(cu + b);
+    const int64_t trow = (int64_t)(kind == 2 ? pos * p.stride : pos) * half + v * 8;
     if (kind == 2) {
         take(p.cmp, at);
     } else if (!BWD) {
@@ -117,11 +137,9 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
     } else {
         take(p.k[0], at); take(p.k[1], at);
     }
-    uint4 o1, o2;
-    rotate8<ET>(x1, x2, (const ET*)p.cs + trow, (const ET*)p.sn + trow, BWD ? -1.f : 1.f, o1, o2);
-    ET* out = (ET*)(kind == 0 ? p.q_out : kind == 1 ? p.k_out : p.cmp) + at;
-    *reinterpret_cast<uint4*>(out) = o1;
-    *reinterpret_cast<uint4*>(out + half) = o2;
+    rotate8<ET>(x1, x2, (const ET*)p.cs + trow, (const ET*)p.sn + trow, BWD ? -1.f : 1.f);
+    if (BWD && kind == 1) take(p.k[2], at);
+    put(kind == 0 ? p.q_out : kind == 1 ? p.k_out : p.cmp, x1, x2);
     if (!BWD && kind == 1 && h == 0 && v == 0 && p.hi_cmp) {
         const int c0 = __ldg(p.cu_cmp + b), nb = __ldg(p.cu_cmp + b + 1) - c0;
         const int vis = pos >= p.ks - 1 ? min((pos - (p.ks - 1)) / p.stride + 1, nb) : 0;
@@ -182,7 +200,7 @@ template <bool BWD>
 static int run_rope(const LayerRopeParams& p, int dtype, cudaStream_t stream) {
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     if (p.D % 16) return FSA_ERR_BAD_ARG;
-    const int64_t threads = (p.N * (p.Hq + p.Hk) + p.Nc * p.Hk) * (p.D / 16);
+    const int64_t threads = (p.N * (p.Hq + (BWD ? 2 : 1) * p.Hk) + p.Nc * p.Hk) * (p.D / 16);
     if (threads >= ((int64_t)1 << 32)) return FSA_ERR_UNSUPPORTED;
     if (threads == 0) return FSA_OK;
     (void)cudaGetLastError();
@@ -205,16 +223,16 @@ extern "C" int fsa_layer_rope_fwd(const void* q, int64_t q_stride_n, const void*
     return run_rope<false>(p, dtype, (cudaStream_t)stream);
 }
 
-extern "C" int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const void* dk0, const void* dk1, void* dcmp_k,
-                                  const void* cos_tab, const void* sin_tab, const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch,
-                                  int64_t total, int64_t total_cmp, int num_q_heads, int num_kv_heads, int head_dim, int kernel_stride, int dtype,
-                                  void* dq, void* dk, void* stream) {
-    if (!dq0 || !dq1 || !dq2 || !dk0 || !dk1 || !cos_tab || !sin_tab || !cu_seqlens || !cu_cmp || !dq || !dk || (total_cmp > 0 && !dcmp_k))
-        return FSA_ERR_BAD_ARG;
+extern "C" int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const void* dk0, const void* dk1, const void* dk2,
+                                  const void* dv0, const void* dv1, const void* dv2, void* dcmp_k, const void* cos_tab, const void* sin_tab,
+                                  const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch, int64_t total, int64_t total_cmp, int num_q_heads,
+                                  int num_kv_heads, int head_dim, int kernel_stride, int dtype, void* dq, void* dk, void* dv, void* stream) {
+    if (total > 0 && (!dq0 || !dq1 || !dq2 || !dk0 || !dk1 || !dk2 || !dv0 || !dv1 || !dv2 || !dq || !dk || !dv)) return FSA_ERR_BAD_ARG;
+    if (!cos_tab || !sin_tab || !cu_seqlens || !cu_cmp || (total_cmp > 0 && !dcmp_k)) return FSA_ERR_BAD_ARG;
     LayerRopeParams p = {};
     p.cu = cu_seqlens; p.cu_cmp = cu_cmp; p.B = batch; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.D = head_dim; p.stride = kernel_stride;
-    p.N = total; p.Nc = total_cmp; p.cs = cos_tab; p.sn = sin_tab; p.q[0] = dq0; p.q[1] = dq1; p.q[2] = dq2; p.k[0] = dk0; p.k[1] = dk1;
-    p.q_out = dq; p.k_out = dk; p.cmp = dcmp_k;
+    p.N = total; p.Nc = total_cmp; p.cs = cos_tab; p.sn = sin_tab; p.q[0] = dq0; p.q[1] = dq1; p.q[2] = dq2; p.k[0] = dk0; p.k[1] = dk1; p.k[2] = dk2;
+    p.v[0] = dv0; p.v[1] = dv1; p.v[2] = dv2; p.q_out = dq; p.k_out = dk; p.v_out = dv; p.cmp = dcmp_k;
     return run_rope<true>(p, dtype, (cudaStream_t)stream);
 }
 

@@ -35,11 +35,10 @@ struct LcDxParams {
     int n_seq, H, ks, stride;
     int phases;                 // phases per CTA
     int tile0[kLbSeqs + 1];     // first tile (128 m) of every sequence
-    int n_cmp[kLbSeqs];         // windows of every sequence (0: no product, the gradient is the addends)
+    int n_cmp[kLbSeqs];         // windows of every sequence (0: no product, the gradient is zero)
     int L[kLbSeqs];             // tokens
     int64_t tok0[kLbSeqs];      // first token
     void* dx[kLbTensors];       // [N, H, D] contiguous
-    const void* add[kLbTensors][2];   // other gradients of the same tensor, added before the rounding (may be dx itself), or null
     int* status;
 };
 static_assert(sizeof(LcDxMaps) + sizeof(LcDxParams) <= 4096, "kernel parameters");
@@ -141,8 +140,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
             tc_fence_after();
             const int64_t t = (int64_t)(m0 + r) * p.stride + p0 + pi;
             const bool valid = ok && t < p.L[seq];
-            const int64_t at = ((p.tok0[seq] + t) * p.H + h) * D;
-            ET* dst = reinterpret_cast<ET*>(p.dx[tn]) + at;
+            ET* dst = reinterpret_cast<ET*>(p.dx[tn]) + ((p.tok0[seq] + t) * p.H + h) * D;
 #pragma unroll
             for (int cc = 0; cc < D; cc += 32) {
                 uint32_t v[32];
@@ -156,25 +154,12 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
                 if (valid) {
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
-                        float f[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[q4 * 8 + j]);
-#pragma unroll
-                        for (int a = 0; a < 2; ++a) {
-                            if (p.add[tn][a]) {
-                                const uint4 x = *reinterpret_cast<const uint4*>(reinterpret_cast<const ET*>(p.add[tn][a]) + at + cc + q4 * 8);
-                                const uint32_t* px = &x.x;
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float2 g = ElemTraits<ET>::unpack2(px[j]);
-                                    f[2 * j] += g.x;
-                                    f[2 * j + 1] += g.y;
-                                }
-                            }
-                        }
-                        *reinterpret_cast<uint4*>(dst + cc + q4 * 8) =
-                            make_uint4(ElemTraits<ET>::pack2(f[0], f[1]), ElemTraits<ET>::pack2(f[2], f[3]), ElemTraits<ET>::pack2(f[4], f[5]),
-                                       ElemTraits<ET>::pack2(f[6], f[7]));
+                        uint4 u;
+                        u.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
+                        u.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
+                        u.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
+                        u.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
+                        *reinterpret_cast<uint4*>(dst + cc + q4 * 8) = u;
                     }
                 }
             }
@@ -402,7 +387,6 @@ struct LcGrad {
     int64_t x_sn;
     const void *w, *dy;
     void* dx;
-    const void* add[2];
     void* dw;
 };
 struct LcPeGrad {
@@ -423,7 +407,7 @@ static int run_bwd(const LcGrad* t, int nt, const LcPeGrad& pe, const int32_t* c
         for (int i = 0; i < nt; ++i) {
             int rc = make_tile_map(&maps.w[i], t[i].w, dtype, (int64_t)H * ks * D, D, D, 64);
             if (rc) return rc;
-            p.dx[i] = t[i].dx; p.add[i][0] = t[i].add[0]; p.add[i][1] = t[i].add[1];
+            p.dx[i] = t[i].dx;
         }
         int64_t tok0 = 0, y0 = 0;
         const int64_t row_bytes = (int64_t)H * D * 2;
@@ -476,7 +460,6 @@ static int check_bwd(const LcGrad& g, const int32_t* cu, const int32_t* seqlens,
     if (ks % stride != 0 || (stride & (stride - 1)) != 0 || (ks & 1)) return FSA_ERR_UNSUPPORTED;
     if (((uintptr_t)g.x & 15) || ((uintptr_t)g.w & 15) || ((uintptr_t)g.dy & 15) || ((uintptr_t)g.dx & 15) || ((uintptr_t)g.dw & 15) || (g.x_sn % 8))
         return FSA_ERR_BAD_ARG;
-    if (((uintptr_t)g.add[0] & 15) || ((uintptr_t)g.add[1] & 15)) return FSA_ERR_BAD_ARG;
     if (g.x_sn < (int64_t)H * D) return FSA_ERR_BAD_ARG;
     *total = 0;
     for (int b = 0; b < batch; ++b)
@@ -491,7 +474,7 @@ using namespace fsa;
 extern "C" int fsa_linear_compress_bwd(const void* x, int64_t x_stride_n, const void* w, const void* dy, const int32_t* cu_seqlens,
                                        const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
                                        int kernel_stride, int dtype, void* dx, void* dw, int32_t* status, void* stream_) {
-    const LcGrad g{x, x_stride_n, w, dy, dx, {nullptr, nullptr}, dw};
+    const LcGrad g{x, x_stride_n, w, dy, dx, dw};
     int64_t total = 0;
     int rc = check_bwd(g, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, &total);
     if (rc) return rc;
@@ -507,11 +490,10 @@ extern "C" int fsa_linear_compress_bwd(const void* x, int64_t x_stride_n, const 
 extern "C" int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kBiasParts * num_heads * head_dim * 4; }
 
 extern "C" int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
-                                   const void* pe, const void* dyk, const void* dyv, const void* dk_add, const void* dv_add0, const void* dv_add1,
-                                   const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
+                                   const void* pe, const void* dyk, const void* dyv, const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
                                    int kernel_stride, int dtype, void* dk, void* dv, void* dw_key, void* dw_value, void* dpe, float* scratch,
                                    void* stream_) {
-    const LcGrad g[2] = {{k, k_stride_n, w_key, dyk, dk, {dk_add, nullptr}, dw_key}, {v, v_stride_n, w_value, dyv, dv, {dv_add0, dv_add1}, dw_value}};
+    const LcGrad g[2] = {{k, k_stride_n, w_key, dyk, dk, dw_key}, {v, v_stride_n, w_value, dyv, dv, dw_value}};
     int64_t total = 0;
     for (int i = 0; i < 2; ++i) {
         const int rc = check_bwd(g[i], cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, &total);

@@ -110,7 +110,7 @@ SIGNATURES = {
     "fsa_layer_prep": (c_int, [c_void_p, c_int, c_int64, c_void_p] + [c_int] * 4 + [c_void_p] * 4),
     "fsa_layer_rope_fwd": (
         c_int, [c_void_p, c_int64, c_void_p, c_int64] + [c_void_p] * 5 + [c_int, c_int64, c_int64] + [c_int] * 7 + [c_void_p] * 6),
-    "fsa_layer_rope_bwd": (c_int, [c_void_p] * 10 + [c_int, c_int64, c_int64] + [c_int] * 5 + [c_void_p] * 3),
+    "fsa_layer_rope_bwd": (c_int, [c_void_p] * 14 + [c_int, c_int64, c_int64] + [c_int] * 5 + [c_void_p] * 4),
     "fsa_gate_proj_mix_bwd_delta": (
         c_int, [c_void_p, c_int64] + [c_void_p] * 6 + [c_int64] + [c_int] * 4 + [c_void_p] * 7 + [c_int64, c_void_p]),
     "fsa_sel_bwd_delta": (
@@ -120,7 +120,7 @@ SIGNATURES = {
         [c_void_p] * 10 + [c_int64] * 2 + [c_int] * 7 + [c_int64] * 6 + [c_float] + [c_void_p] * 4 + [c_int64, c_void_p, c_int64, c_void_p]),
     "fsa_compress_kv_bwd_scratch_bytes": (c_int64, [c_int, c_int]),
     "fsa_compress_kv_bwd": (
-        c_int, [c_void_p, c_int64, c_void_p, c_int64] + [c_void_p] * 10 + [c_int] * 6 + [c_void_p] * 7),
+        c_int, [c_void_p, c_int64, c_void_p, c_int64] + [c_void_p] * 7 + [c_int] * 6 + [c_void_p] * 7),
     "fsa_decode_proj": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "fsa_decode_append": (
         c_int,

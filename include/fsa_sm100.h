@@ -298,11 +298,13 @@ int fsa_layer_rope_fwd(const void* q, int64_t q_stride_n, const void* k, int64_t
                        int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int window, int dtype,
                        void* q_out, void* k_out, int32_t* hi_cmp, int32_t* lo_win, int32_t* hi_win, void* stream);
 
-/* dq = inverse rotation of dq0 + dq1 + dq2, dk of dk0 + dk1 (may be written over an input), dcmp_k in place. */
-int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const void* dk0, const void* dk1, void* dcmp_k,
-                       const void* cos_tab, const void* sin_tab, const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch,
-                       int64_t total, int64_t total_cmp, int num_q_heads, int num_kv_heads, int head_dim, int kernel_stride, int dtype,
-                       void* dq, void* dk, void* stream);
+/* dq = inverse rotation of dq0 + dq1 + dq2; dk = that of dk0 + dk1, plus dk2 (the compressor's share, of the unrotated keys);
+ * dv = dv0 + dv1 + dv2; dcmp_k in place.  total 0: the compressed keys alone; total_cmp 0: everything else.  An output may be
+ * one of its inputs. */
+int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const void* dk0, const void* dk1, const void* dk2,
+                       const void* dv0, const void* dv1, const void* dv2, void* dcmp_k, const void* cos_tab, const void* sin_tab,
+                       const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch, int64_t total, int64_t total_cmp, int num_q_heads,
+                       int num_kv_heads, int head_dim, int kernel_stride, int dtype, void* dq, void* dk, void* dv, void* stream);
 
 /* fsa_gate_proj_mix_bwd that also gives delta [3][num_heads][total] fp32, the sum of o dO over every head of every branch. */
 int fsa_gate_proj_mix_bwd_delta(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
@@ -321,13 +323,11 @@ int fsa_range_attn_bwd_delta(const void* q, const void* k, const void* v, const 
                              int64_t k_sn, int64_t v_sn, int64_t do_sn, int64_t do_sh, float sm_scale, void* dq, void* dk, void* dv,
                              void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream);
 
-/* Backward of fsa_compress_kv_fwd: dk = gradient through the compressor + dk_add, dv likewise + dv_add0 + dv_add1 (addends
- * [total, H, D] contiguous, may be the output itself, or null), dw_key with the share of the bias, dw_value, dpe (each may be
+/* Backward of fsa_compress_kv_fwd: dk, dv (contiguous), dw_key with the share of the bias, dw_value, dpe (the last three may be
  * null).  scratch: fsa_compress_kv_bwd_scratch_bytes(). */
 int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim);
 int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
-                        const void* pe, const void* dyk, const void* dyv, const void* dk_add, const void* dv_add0, const void* dv_add1,
-                        const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
+                        const void* pe, const void* dyk, const void* dyv, const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
                         int kernel_stride, int dtype, void* dk, void* dv, void* dw_key, void* dw_value, void* dpe, float* scratch,
                         void* stream);
 
