@@ -166,7 +166,8 @@ static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 // (64 KB written and read), which is why long lists keep long runs.  A function of the shape alone: forward and backward
 // must cut the same list alike.
 static int sched_run(const SelShape& s, int most) {
-    const int64_t tiles = ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT;
+    // (a backward run is walked once per 64-key part of its blocks)
+    const int64_t tiles = ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT * (s.BK > 64 ? s.BK / 64 : 1);
     const int64_t run = tiles / (4 * 148);
     return (int)(run < 1 ? 1 : run > most ? most : run);
 }
@@ -209,7 +210,7 @@ static int64_t bwd_dq_part_bytes(const SelShape& s) {
 // fp32 dK / dV accumulators (unpipelined kernel) or per-segment slabs (pipelined kernel): the same region
 static int64_t bwd_dkdv_bytes(const SelShape& s) {
     const int64_t acc = align_up(2 * s.Nk * s.Hk * (int64_t)s.D * 4, 256);
-    const int64_t slabs = align_up(sel_max_segments(s) * 2 * 64 * (int64_t)s.D * 4, 256);
+    const int64_t slabs = align_up(sel_max_segments(s) * bwd_nsub(s.BK) * 2 * 64 * (int64_t)s.D * 4, 256);
     return acc > slabs ? acc : slabs;
 }
 static int64_t bwd_scratch_bytes(const SelShape& s) {
@@ -427,8 +428,9 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     a.dq_part = (void*)sp;  sp += bwd_dq_part_bytes(s);
     CUtensorMap dqmap;
     a.dqmap = nullptr;
-    if (D == 128 && BK <= 64) {
-        rc = make_tile_map(&dqmap, a.dq_part, dtype, sel_max_tiles(s) * kTileRows, D, D, 32);
+    const int64_t dq_rows = sel_max_tiles(s) * bwd_nsub(BK) * kTileRows;
+    if (D <= 128 && dq_rows < ((int64_t)1 << 31)) {
+        rc = make_tile_map(&dqmap, a.dq_part, dtype, dq_rows, D, D, 32);
         if (rc) return rc;
         a.dqmap = &dqmap;
     }

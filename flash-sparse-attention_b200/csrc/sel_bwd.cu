@@ -444,10 +444,11 @@ __global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ 
 // segments, rounded to the output dtype (replaces the `.sum(0)` over the group's copies of the reference,
 // fsa/ops/FSA_topk_sparse_attention.py:1854-1855).  The rows of a block that nobody selected (no segment) and those past
 // the last sequence (the last CTA) are written as zeros here: no pass over dk and dv before (26 us of 64K tokens x 4 heads).
-template <typename ET>
+template <int D, typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s,
-                                                           SelIndex ix, ET* __restrict__ dk, ET* __restrict__ dv) {
-    constexpr int D = 128, KT = 64;
+                                                           SelIndex ix, int nsub, ET* __restrict__ dk, ET* __restrict__ dv) {
+    constexpr int KT = 64, RV = D / 4;                // keys of a slab, float4 per row
+    constexpr int kShares = 2 * KT * RV / 1024;       // CTAs per slab: 1024 float4 each, four per thread in flight
     const int hg = blockIdx.x;
     if (hg == s.Hk * s.NBmax) {
         if (blockIdx.y > 0) return;
@@ -458,40 +459,37 @@ __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restri
         }
         return;
     }
-    const int h = hg / s.NBmax, gb = hg - h * s.NBmax;
+    const int h = hg / s.NBmax, gb = hg - h * s.NBmax, sub = blockIdx.y / kShares;
     const int2 rn = block_rows(ck, s.B, s.BK, gb);
-    const int row0 = rn.x, nkeys = min(KT, rn.y);     // rows past the end of the sequence belong to the next sequence's block
+    // rows past the end of the sequence belong to the next sequence's block
+    const int row0 = rn.x + sub * KT, nkeys = min(KT, rn.y - sub * KT);
+    if (nkeys <= 0) return;
     const int seg0 = ix.key_seg[hg], nseg = ix.key_seg[hg + 1] - seg0;
-    // a warp per K/V row (32 lanes x 16 bytes = the row's 128 floats), four rows in flight per warp; the CTA's 8 warps take 32
-    // of the 64 rows of dK and 64 rows of dV (blockIdx.y: a block with many short segments would be a serial chain otherwise)
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float4* base = reinterpret_cast<const float4*>(slabs + (int64_t)seg0 * (2 * KT * D)) + lane;
-    constexpr int kSegStride = 2 * KT * D / 4, kRowStride = D / 4;       // in float4
-    {
-        const int r0 = (blockIdx.y * 8 + warp) * 4;
-        float4 acc[4];
+    const int i0 = (blockIdx.y % kShares) * 1024 + threadIdx.x;
+    const float4* base = reinterpret_cast<const float4*>(slabs) + ((int64_t)seg0 * nsub + sub) * (2 * KT * RV);
+    const int64_t seg_stride = (int64_t)nsub * (2 * KT * RV);
+    float4 acc[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int sg = 0; sg < nseg; ++sg) {
-            float4 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int r = r0 + j;                        // row of the slab: which * 64 + key
-                v[j] = (r & (KT - 1)) < nkeys ? __ldcs(base + (int64_t)sg * kSegStride + r * kRowStride) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { acc[j].x += v[j].x; acc[j].y += v[j].y; acc[j].z += v[j].z; acc[j].w += v[j].w; }
-        }
+    for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int sg = 0; sg < nseg; ++sg) {
+        float4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int r = r0 + j, key = r & (KT - 1);
-            if (key < nkeys) {
-                ET* dst = (r < KT ? dk : dv) + ((int64_t)(row0 + key) * s.Hk + h) * D + lane * 4;
-                uint2 w;
-                w.x = ElemTraits<ET>::pack2(acc[j].x, acc[j].y);
-                w.y = ElemTraits<ET>::pack2(acc[j].z, acc[j].w);
-                *reinterpret_cast<uint2*>(dst) = w;
-            }
+            const int i = i0 + j * 256;                  // float4 of the slab: (which * 64 + key) * RV + column / 4
+            v[j] = (i / RV & (KT - 1)) < nkeys ? __ldcs(base + sg * seg_stride + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { acc[j].x += v[j].x; acc[j].y += v[j].y; acc[j].z += v[j].z; acc[j].w += v[j].w; }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = i0 + j * 256, r = i / RV, key = r & (KT - 1);
+        if (key < nkeys) {
+            ET* dst = (r < KT ? dk : dv) + ((int64_t)(row0 + key) * s.Hk + h) * D + (i % RV) * 4;
+            uint2 w;
+            w.x = ElemTraits<ET>::pack2(acc[j].x, acc[j].y);
+            w.y = ElemTraits<ET>::pack2(acc[j].z, acc[j].w);
+            *reinterpret_cast<uint2*>(dst) = w;
         }
     }
 }
@@ -520,7 +518,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     // the gather warps of the pipelined kernel address rows by 32-bit offsets in units of 8 elements
     const bool offsets_fit = ((s.N * a.q_sn + (int64_t)s.Hq * a.q_sh) >> 3) < 0x7fffffffll &&
                              ((s.N * a.do_sn + (int64_t)s.Hq * a.do_sh) >> 3) < 0x7fffffffll;
-    const bool pipelined = D == 128 && s.BK <= kKT && a.dqmap && offsets_fit;
+    const bool pipelined = D <= 128 && a.dqmap && offsets_fit;
     cudaError_t e;
     if (!pipelined) {
         e = cudaMemsetAsync(a.dk_acc, 0, kv_elems * 4 * 2, stream);   // dk_acc and dv_acc are adjacent
@@ -540,7 +538,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     p.scale = a.sm_scale; p.scale_log2 = a.sm_scale * 1.4426950408889634f;
     p.dq_part = (ET*)a.dq_part; p.dk_acc = a.dk_acc; p.dv_acc = a.dv_acc;
     // range attention (every token sees one contiguous range): dQ by the query-tile-major kernel, no partial dQ rows
-    const bool dq_dense = pipelined && a.bd.kv_hi != nullptr && s.G <= 32;
+    const bool dq_dense = pipelined && D == 128 && a.bd.kv_hi != nullptr && s.G <= 32;
     if (pipelined) {
         const int dt = ElemTraits<ET>::kIsBF16 ? (int)kBF16 : (int)kFP16;
         if (dq_dense && rows > 0) {
@@ -572,9 +570,8 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     }
     if (kv_elems > 0) {
         if (pipelined) {
-            if constexpr (D == 128)
-                sel_bwd_dkdv_reduce<ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), 4), 256, 0, stream>>>(a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix,
-                                                                                            (ET*)a.dk, (ET*)a.dv);
+            sel_bwd_dkdv_reduce<D, ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), (unsigned)(nsub * (2 * kKT * (D / 4) / 1024))), 256, 0, stream>>>(
+                a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix, nsub, (ET*)a.dk, (ET*)a.dv);
         } else {
             int64_t n4 = kv_elems / 4;
             sel_bwd_convert<ET><<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(a.dk_acc, a.dv_acc, (ET*)a.dk, (ET*)a.dv, n4);

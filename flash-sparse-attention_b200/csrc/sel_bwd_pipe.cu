@@ -1,6 +1,7 @@
-// Selected-attention backward, pipelined kernel for head_dim 128 and blocks of <= 64 keys
-// (the shapes of the benchmark configurations); other shapes use the unpipelined kernel in
-// sel_bwd.cu.  Same math and same outputs: per tile of <= 128 (head, token) rows of one KV block
+// Selected-attention backward, pipelined kernel for head_dim 64 and 128 (256: sel_bwd.cu).  Blocks of 128 and 256 keys are
+// walked as independent 64-key parts, every part a pass over the tiles of its own (the gathers are repeated, which costs less
+// than the registers and TMEM of a wider tile: 21008 tokens, 128-key blocks, 734 us in the unpipelined kernel before).
+// Per tile of <= 128 (head, token) rows of one part of a KV block
 //     S = Q K^T, dP = dO V^T | P = exp2(S c - lse), dS = scale P (dP - delta) | dQ = dS K,
 //     dK^T += Q^T dS, dV^T += dO^T P
 // Warp roles (768 threads in six warpgroups whose register budgets are rebalanced with setmaxnreg; one CTA per SM,
@@ -36,29 +37,32 @@ struct SelBwdPipeParams {
     float scale, scale_log2;
     int run;
     SelBounds bd;      // visible K/V rows per token
-    ET* dq_part;       // [max_tiles * 128, D] (written through dqmap)
-    float* slabs;      // [segments][2 (dK, dV)][64 keys][D] fp32: the partial sums of every segment of tiles
+    ET* dq_part;       // [max_tiles][nsub][128, D] (written through dqmap)
+    int nsub;          // 64-key parts of a block
+    float* slabs;      // [segments][nsub][2 (dK, dV)][64 keys][D] fp32: the partial sums of every segment of tiles
     int no_dq;         // 1: dQ is computed elsewhere (range attention: the query-tile-major dQ kernel); only dK / dV here
 };
 
 namespace bwdpipe {
-constexpr int D = 128, KT = 64;
+constexpr int KT = 64;
 constexpr int kKVStages = 1;                     // (a second K/V stage and the dQ staging area compete for the same 32 KB)
 constexpr int kThreads = 768, kLoaders = 256;
 constexpr int kWLoad = kLoaders / 32, kWMma1 = kWLoad, kWMma2 = kWLoad + 1, kWFlush = kWLoad + 4, kWGroups = kWLoad + 8;
 // registers per thread of each role (multiples of 8); 32 * sum over warps <= 768 * 80 = the CTA's allocation
 constexpr int kRegLoad = 40, kRegMma = 48, kRegFlush = 96, kRegGroup = 128;
 static_assert(8 * kRegLoad + 4 * kRegMma + 4 * kRegFlush + 8 * kRegGroup <= 24 * 80, "register budget");
-constexpr int kKV = 2 * KT * D * 2;              // K then V: 32 KB
-constexpr int kQD = 2 * kTileRows * D * 2;       // Q then dO: 64 KB
 constexpr int kPS = 2 * kTileRows * KT * 2;      // P then dS: 32 KB
-constexpr int kDQ = kTileRows * D * 2;           // dQ staging: 32 KB, 8 KB per TMEM lane quarter
 constexpr int kTail = 2560;
-constexpr int kBytes = kKVStages * kKV + 2 * kQD + kPS + kDQ + kTail;
 constexpr int cS = 0, cDP = 64;                  // + 128 * buffer
 constexpr int cDQ = 256, cDK = 384, cDV = 448;
 constexpr uint32_t kCols = 512;
-static_assert(kBytes <= 227 * 1024, "smem budget");
+template <int D> struct Cfg {
+    static constexpr int kKV = 2 * KT * D * 2;              // K then V
+    static constexpr int kQD = 2 * kTileRows * D * 2;       // Q then dO
+    static constexpr int kDQ = kTileRows * D * 2;           // dQ staging, a quarter per TMEM lane quarter
+    static constexpr int kBytes = kKVStages * kKV + 2 * kQD + kPS + kDQ + kTail;
+    static_assert(kBytes <= 227 * 1024, "smem budget");
+};
 }  // namespace bwdpipe
 
 // Optional cycle accounting per role (debug builds only, -DFSA_TIMING): a table [gridDim.x][64] of accumulated
@@ -89,12 +93,13 @@ __device__ __forceinline__ float ex2_approx_b(float x) {
     return y;
 }
 
-template <typename ET>
+template <int D, typename ET>
 __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBwdPipeParams<ET> p,
                                                                      const __grid_constant__ CUtensorMap kmap,
                                                                      const __grid_constant__ CUtensorMap vmap,
                                                                      const __grid_constant__ CUtensorMap dqmap) {
     using namespace bwdpipe;
+    constexpr int kKV = Cfg<D>::kKV, kQD = Cfg<D>::kQD, kDQ = Cfg<D>::kDQ;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sKV = smem;
     uint8_t* sQD = sKV + kKVStages * kKV;
@@ -149,18 +154,18 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    const TileSchedule sched(p.ix.header[1], p.run);
+    const TileSchedule sched(p.ix.header[1], p.run, p.nsub);
     const int nloc = sched.nloc;
     const int key_lim = min(KT, s.BK);
 
     if (warp < kWLoad) {
         // ------------------------------------------------------------------ gather warps
-        // Thread t copies 16-byte chunk t % 16 of the rows t / 16 + 16 i (a half-warp covers one 256-byte row) of Q and
+        // (D = 128) thread t copies 16-byte chunk t % 16 of the rows t / 16 + 16 i (a half-warp covers one 256-byte row) of Q and
         // dO.  Tokens come from the prepared ring; the head part of every row offset is a thread constant.
         reg_dec<kRegLoad>();
         const int t = tid;
         bool ok = true;
-        constexpr int CPR = D / 8, RSTEP = kLoaders / CPR, NIT = kTileRows / RSTEP;   // 16 chunks per row, 8 rows per thread
+        constexpr int CPR = D / 8, RSTEP = kLoaders / CPR, NIT = kTileRows / RSTEP;   // D = 128: 16 chunks per row, 8 rows per thread
         const int cchunk = t % CPR, rbase = t / CPR;
         const uint32_t slab_off = (uint32_t)(cchunk >> 3) * (kTileRows * 128);
         int gq[NIT], gd[NIT];                   // (head-in-group * head stride) / 8 of this thread's rows
@@ -215,7 +220,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         const int quarter = warp & 3;
         const int d_idx = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint8_t* my_stage = sDQ + quarter * (32 * 256);
+        uint8_t* my_stage = sDQ + quarter * (32 * D * 2);
         bool ok = true;
         int nflush = 0;
         BT_DECL;
@@ -264,7 +269,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             if (lane == 0) {
 #pragma unroll
                 for (int b = 0; b < D / 64; ++b)
-                    tma_store_2d(&dqmap, b * 64, j * kTileRows + quarter * 32, smem_u32(my_stage + b * (32 * 128)));
+                    tma_store_2d(&dqmap, b * 64, (j * p.nsub + sched.sub(k)) * kTileRows + quarter * 32, smem_u32(my_stage + b * (32 * 128)));
                 bulk_commit();
             }
             }
@@ -275,17 +280,20 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             const TileInfo ti = load_tile(p.ix, j0);
             // segments of a key are numbered by the scheduling run they fall into
             const int seg = ti.seg0 + j0 / sched.run - __ldg(p.ix.tile_aux + j0).x / sched.run;
-            float* slab = p.slabs + (int64_t)seg * (2 * KT * D) + d_idx;
+            float* slab = p.slabs + ((int64_t)seg * p.nsub + sched.sub(k)) * (2 * KT * D) + d_idx;
             ok = mbar_wait(acc_full, nflush & 1, status) && ok;
             BT_TOC(3);
             tc_fence_after();
 #pragma unroll
             for (int which = 0; which < 2; ++which) {
                 uint32_t v[KT];
+                // (D = 64: the upper half of the accumulator rows holds products of whatever follows the tile in shared memory)
+                if (quarter * 32 < D) {
 #pragma unroll
-                for (int c0 = 0; c0 < KT; c0 += 32)
-                    tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[c0]));
-                tmem_ld_wait();
+                    for (int c0 = 0; c0 < KT; c0 += 32)
+                        tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[c0]));
+                    tmem_ld_wait();
+                }
                 if (which == 1) {
                     // both accumulators are in registers now: the next segment may overwrite them
                     tc_fence_before();
@@ -293,8 +301,10 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                     ++nflush;
                 }
                 float* dst = slab + which * (KT * D);
+                if (quarter * 32 < D) {
 #pragma unroll
-                for (int key = 0; key < KT; ++key) dst[key * D] = __uint_as_float(v[key]);
+                    for (int key = 0; key < KT; ++key) dst[key * D] = __uint_as_float(v[key]);
+                }
             }
             BT_TOC(4);
         }
@@ -491,12 +501,13 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                 const int ks = kvn % kKVStages;
                 ok = mbar_wait(&kv_empty[ks], ((kvn / kKVStages) & 1) ^ 1, status) && ok;
                 mbar_expect_tx(&kv_full[ks], (uint32_t)kKV);
+                const int row = cur.row0 + sched.sub(k) * KT;
                 uint8_t* dK = sKV + ks * kKV;
                 uint8_t* dV = dK + KT * D * 2;
 #pragma unroll
                 for (int b = 0; b < D / 64; ++b) {
-                    tma_load_2d(smem_u32(dK + b * KT * 128), &kmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
-                    tma_load_2d(smem_u32(dV + b * KT * 128), &vmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
+                    tma_load_2d(smem_u32(dK + b * KT * 128), &kmap, cur.h * D + b * 64, row, &kv_full[ks]);
+                    tma_load_2d(smem_u32(dV + b * KT * 128), &vmap, cur.h * D + b * 64, row, &kv_full[ks]);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -529,6 +540,10 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ent = 0xFFFFFFFFu;
             if (row_exists) ent = __ldg(p.ix.entries + (int64_t)j * s.TPT + e);
         };
+        auto fetch = [&](int k, uint32_t& ent, int& row0, int& h) {      // ... and the first key of the tile's part
+            fetch_ent(sched.tile(k), ent, row0, h);
+            row0 += sched.sub(k) * KT;
+        };
         auto fetch_stats = [&](uint32_t ent, int h, int row0, float& lse_, float& delta_, int& c_lo, int& c_hi) {
             // padding rows: their Q and dO rows are zero, so they add nothing to dK / dV whatever P is, and their dQ
             // rows are never read: they count as fully visible with lse = delta = 0 (finite values everywhere)
@@ -542,10 +557,10 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
         };
         if (nloc > 0) {
-            fetch_ent(sched.tile(0), entA, row0A, hA);
+            fetch(0, entA, row0A, hA);
             fetch_stats(entA, hA, row0A, lseA, deltaA, cloA, chiA);
         }
-        if (nloc > 1) fetch_ent(sched.tile(1), entB, row0B, hB);
+        if (nloc > 1) fetch(1, entB, row0B, hB);
         BT_DECL;
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
@@ -554,7 +569,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             // rotate the prefetch registers
             entA = entB; row0A = row0B; hA = hB;
             if (k + 1 < nloc) fetch_stats(entA, hA, row0A, lseA, deltaA, cloA, chiA);
-            if (k + 2 < nloc) fetch_ent(sched.tile(k + 2), entB, row0B, hB);
+            if (k + 2 < nloc) fetch(k + 2, entB, row0B, hB);
             BT_TOC(0);
             ok = mbar_wait(&sdp_full[st], (k >> 1) & 1, status) && ok;
             BT_EV(k, 5, sb == 0 && quarter == 0 && lane == 0);
@@ -616,7 +631,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     if (warp == 0) tmem_dealloc(tbase, bwdpipe::kCols);
 }
 
-template <typename ET>
+template <int D, typename ET>
 static cudaError_t launch_pipe(const SelBwdArgs& a, const SelShape& s, const SelIndex& ix, const CUtensorMap& kmap,
                                const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms, bool no_dq, cudaStream_t stream) {
     SelBwdPipeParams<ET> p;
@@ -629,11 +644,13 @@ static cudaError_t launch_pipe(const SelBwdArgs& a, const SelShape& s, const Sel
     p.bd = a.bd;
     p.dq_part = (ET*)a.dq_part; p.slabs = a.slabs;
     p.no_dq = no_dq ? 1 : 0;
-    auto kern = sel_bwd_pipe<ET>;
-    cudaError_t e = allow_smem((const void*)kern, bwdpipe::kBytes);
+    p.nsub = s.BK > bwdpipe::KT ? s.BK / bwdpipe::KT : 1;
+    auto kern = sel_bwd_pipe<D, ET>;
+    constexpr int smem = bwdpipe::Cfg<D>::kBytes;
+    cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(2, stream);
-    kern<<<num_sms, bwdpipe::kThreads, bwdpipe::kBytes, stream>>>(p, kmap, vmap, dqmap);
+    kern<<<num_sms, bwdpipe::kThreads, smem, stream>>>(p, kmap, vmap, dqmap);
     prof_end(2, stream);
     return cudaGetLastError();
 }
@@ -652,8 +669,11 @@ namespace fsa {
 cudaError_t launch_sel_bwd_pipe(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix,
                                 const CUtensorMap& kmap, const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms,
                                 bool no_dq, cudaStream_t stream) {
-    return dtype == kBF16 ? launch_pipe<__nv_bfloat16>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream)
-                          : launch_pipe<__half>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream);
+    if (s.D == 64)
+        return dtype == kBF16 ? launch_pipe<64, __nv_bfloat16>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream)
+                              : launch_pipe<64, __half>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream);
+    return dtype == kBF16 ? launch_pipe<128, __nv_bfloat16>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream)
+                          : launch_pipe<128, __half>(a, s, ix, kmap, vmap, dqmap, num_sms, no_dq, stream);
 }
 
 }  // namespace fsa

@@ -78,7 +78,7 @@ __host__ __device__ inline int64_t align_up(int64_t x, int64_t a) { return (x + 
 inline int64_t sel_max_tiles(const SelShape& s) {
     return ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT + (int64_t)s.Hk * s.NBmax;
 }
-// upper bound on the number of segments: one per key plus one per scheduling run that cuts a key
+// upper bound on the number of segments (of every 64-key part): one per key plus one per scheduling run that cuts a key
 inline int64_t sel_max_segments(const SelShape& s) {
     return (int64_t)s.Hk * s.NBmax + sel_max_tiles(s) / s.RB + 1;
 }
@@ -219,16 +219,20 @@ __device__ __forceinline__ int upper_seg(const int* __restrict__ off, int n, int
 // Static tile schedule of a persistent grid: runs of `run` consecutive tiles are dealt to the
 // CTAs round-robin, so the whole grid advances through the tile list together (neighbouring
 // blocks of one kv head: their query rows stay in L2) while a CTA still reuses a resident K/V
-// block across the tiles of a run.
+// block across the tiles of a run.  nsub > 1 (blocks of more keys than a kernel takes at a time; a power of two): every
+// run is dealt nsub times, once for each part of the blocks.
 struct TileSchedule {
-    int total, grid, cta, run, nloc;
-    __device__ TileSchedule(int total_, int run_) : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_) {
-        const int NR = (total + run - 1) / run;                    // runs in the list
-        const int mine = cta < NR ? (NR - cta + grid - 1) / grid : 0;
+    int total, grid, cta, run, lsub, nloc;      // lsub: log2 of nsub
+    __device__ TileSchedule(int total_, int run_, int nsub_ = 1)
+        : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_), lsub(31 - __clz(nsub_)) {
+        const int NR = (total + run - 1) / run, NV = NR << lsub;    // runs in the list, dealt runs
+        const int mine = cta < NV ? (NV - cta + grid - 1) / grid : 0;
         nloc = mine * run;
-        if (mine > 0 && (NR - 1) % grid == cta) nloc -= NR * run - total;   // the last run may be short
+        // the last run may be short (nsub < grid: a CTA has at most one of its parts, as its own last)
+        if (mine > 0 && (cta + (mine - 1) * grid) >> lsub == NR - 1) nloc -= NR * run - total;
     }
-    __device__ __forceinline__ int tile(int k) const { return ((k / run) * grid + cta) * run + (k % run); }
+    __device__ __forceinline__ int tile(int k) const { return (((k / run) * grid + cta) >> lsub) * run + (k % run); }
+    __device__ __forceinline__ int sub(int k) const { return ((k / run) * grid + cta) & ((1 << lsub) - 1); }
 };
 
 // Query-tile-major kernels cut every sequence into tiles of TPT consecutive tokens.  Both helpers are warp-collective (every lane calls them and gets the same

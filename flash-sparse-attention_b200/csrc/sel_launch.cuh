@@ -55,13 +55,13 @@ struct SelBwdArgs {
     const CUtensorMap* dqmap;   // over dq_part, box {64, 32}: partial stores of the pipelined kernel (null: not built)
     float* dk_acc;     // [N, Hk, D]; dv_acc follows immediately (unpipelined kernel: fp32 accumulators)
     float* dv_acc;
-    float* slabs;      // [segments][2][64][D] fp32 (pipelined kernel: per-segment partial dK / dV); shares memory with dk_acc
+    float* slabs;      // [segments][parts][2][64][D] fp32 (pipelined kernel: per-segment partial dK / dV); shares memory with dk_acc
     // outputs (contiguous)
     void *dq, *dk, *dv;
     SelBounds bd;      // visible K/V rows per token (all null: causal rule of selected attention)
 };
 
-// pipelined main kernel for head_dim 128, block size <= 64 (sel_bwd_pipe.cu)
+// pipelined main kernel for head_dim 64 and 128 (sel_bwd_pipe.cu)
 cudaError_t launch_sel_bwd_pipe(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix,
                                 const CUtensorMap& kmap, const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms,
                                 bool no_dq, cudaStream_t stream);

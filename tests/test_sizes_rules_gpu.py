@@ -20,9 +20,11 @@ def _close(got, ref, name):
     assert float(err.mean()) <= 1e-3 * scale, f"{name}: mean-abs {float(err.mean()):.3e}"
 
 
-@pytest.mark.parametrize("seqlens,Hk,G,T", [([1], 1, 1, 2), ([1100], 1, 2, 16), ([2371, 200], 2, 2, 16), ([1500, 33], 2, 8, 16)])
-def test_scheduling_runs_of_short_lists(seqlens, Hk, G, T):
-    d, bs, N = 128, 64, sum(seqlens)
+@pytest.mark.parametrize("seqlens,Hk,G,T,d,bs", [([1], 1, 1, 2, 128, 64), ([1100], 1, 2, 16, 128, 64), ([2371, 200], 2, 2, 16, 128, 64),
+                                                 ([1500, 33], 2, 8, 16, 128, 64), ([2371, 200, 65], 2, 2, 8, 128, 128),
+                                                 ([1100, 129], 2, 4, 16, 64, 64), ([900, 257], 1, 4, 4, 64, 256)])
+def test_scheduling_runs_of_short_lists(seqlens, Hk, G, T, d, bs):
+    N = sum(seqlens)
     q, k, v, do = make_qkv(N, Hk * G, Hk, d, 300 + N)
     idx, cu = make_topk_idx(seqlens, Hk, T, bs, 301 + N), make_cu_seqlens(seqlens)
     ref = sel_attn_forward_backward(q, k, v, do, idx, bs, cu, d ** -0.5)
