@@ -219,12 +219,12 @@ __device__ __forceinline__ int upper_seg(const int* __restrict__ off, int n, int
 // Static tile schedule of a persistent grid: runs of `run` consecutive tiles are dealt to the
 // CTAs round-robin, so the whole grid advances through the tile list together (neighbouring
 // blocks of one kv head: their query rows stay in L2) while a CTA still reuses a resident K/V
-// block across the tiles of a run.  nsub > 1 (blocks of more keys than a kernel takes at a time; a power of two): every
+// block across the tiles of a run.  nsub > 1 (blocks of more keys than a kernel takes at a time; 1, 2 or 4): every
 // run is dealt nsub times, once for each part of the blocks.
 struct TileSchedule {
     int total, grid, cta, run, lsub, nloc;      // lsub: log2 of nsub
     __device__ TileSchedule(int total_, int run_, int nsub_ = 1)
-        : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_), lsub(31 - __clz(nsub_)) {
+        : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_), lsub(nsub_ >> 1) {
         const int NR = (total + run - 1) / run, NV = NR << lsub;    // runs in the list, dealt runs
         const int mine = cta < NV ? (NV - cta + grid - 1) / grid : 0;
         nloc = mine * run;

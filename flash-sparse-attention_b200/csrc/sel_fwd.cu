@@ -49,16 +49,19 @@ template <int D, int BK>
 struct SelFwdCfg {
     static constexpr int kQ = kTileRows * D * 2;
     static constexpr int kKV = 2 * BK * D * 2;         // K then V
-    static constexpr int kOS = kTileRows * D * 2;      // output staging per softmax warpgroup (input dtype)
+    // Output staging of a softmax warp (32 rows, input dtype): whole rows, or at head size 256 one 64-column slab at a time
+    static constexpr int kOSCols = D <= 128 ? D : 64;
+    static constexpr int kOS = kTileRows * kOSCols * 2;    // ... of a softmax group
     static constexpr int kTail = 2560;                 // barriers, TMEM slot, row-offset table
     static constexpr int kMax = 227 * 1024;
     static constexpr int NKV = (2 * kQ + 2 * kKV + 2 * kOS + kTail <= kMax) ? 2 : 1;    // K/V stages
-    static constexpr int NQ = (3 * kQ + NKV * kKV + 2 * kOS + kTail <= kMax) ? 3 : 2;   // Q stages
+    static constexpr int NQ = (3 * kQ + NKV * kKV + 2 * kOS + kTail <= kMax) ? 3 : (2 * kQ + NKV * kKV + 2 * kOS + kTail <= kMax) ? 2 : 1;   // Q stages
     static constexpr int kBytes = NQ * kQ + NKV * kKV + 2 * kOS + kTail;
-    static constexpr int NS = (4 * BK + 2 * D <= 512) ? 4 : 2;   // S buffers (BK columns each); two per softmax group when they fit
+    static constexpr int NO = D <= 128 ? 2 : 1;        // O buffers of D columns: one per softmax group, or one that they take in turns
+    static constexpr int NS = (4 * BK + NO * D <= 512) ? 4 : 2;   // S buffers (BK columns each); two per softmax group when they fit
     static constexpr int cS = 0;
-    static constexpr int cO = NS * BK;                 // two O buffers of D columns, one per softmax group
-    static constexpr uint32_t kCols = tmem_cols_pow2(NS * BK + 2 * D);
+    static constexpr int cO = NS * BK;
+    static constexpr uint32_t kCols = tmem_cols_pow2(NS * BK + NO * D);
 };
 
 // warps: 0..3 gather loaders | 4 issues S = Q K^T | 5 issues O = P V | 6..9 softmax group 0 | 10..13 softmax group 1
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                                                                const __grid_constant__ CUtensorMap vmap,
                                                                const __grid_constant__ CUtensorMap omap) {
     using C = SelFwdCfg<D, BK>;
-    static_assert(C::NS * BK + 2 * D <= 512, "TMEM budget");
+    static_assert(C::NS * BK + C::NO * D <= 512, "TMEM budget");
     static_assert(C::kBytes <= 227 * 1024, "smem budget");
     // The kernel uses no static shared memory: the dynamic region starts 1024-byte aligned, which
     // the swizzled tiles need, and every byte of the 227 KB is budgeted (checked below).
@@ -181,23 +184,29 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             if (t == 0) TR(0, k, 0);
             ok = mbar_wait(&off_full[slot], (k / kFwdRing) & 1, status) && ok;
             const int hq0 = (int)(((long long)s_h[slot] * s.G * q_sh) >> 3);
-            int tok[NIT];
-#pragma unroll
-            for (int it = 0; it < NIT; ++it) tok[it] = s_tok[slot][rbase + it * RSTEP];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&off_empty[slot]);
-            T_TOC(2);
             const uint32_t dstq = smem_u32(sQ + qs * C::kQ) + slab_off;
-#ifdef FSA_TIMING
-            if (!(p.dbg & 1))
-#endif
-            {
+            constexpr int NB = NIT < 16 ? NIT : 16;            // rows whose tokens are held at a time
 #pragma unroll
-                for (int it = 0; it < NIT; ++it) {
-                    const int r = rbase + it * RSTEP;
-                    const bool valid = tok[it] >= 0;
-                    const int tk = valid ? tok[it] : 0;
-                    cp_async16(dstq + sw128_chunk_off(r, cchunk & 7), qc + ((long long)(tk * qsn8 + hq0 + gq[it]) << 3), valid);
+            for (int i0 = 0; i0 < NIT; i0 += NB) {
+                int tok[NB];
+#pragma unroll
+                for (int it = 0; it < NB; ++it) tok[it] = s_tok[slot][rbase + (i0 + it) * RSTEP];
+                if (i0 + NB == NIT) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&off_empty[slot]);
+                    T_TOC(2);
+                }
+#ifdef FSA_TIMING
+                if (!(p.dbg & 1))
+#endif
+                {
+#pragma unroll
+                    for (int it = 0; it < NB; ++it) {
+                        const int r = rbase + (i0 + it) * RSTEP;
+                        const bool valid = tok[it] >= 0;
+                        const int tk = valid ? tok[it] : 0;
+                        cp_async16(dstq + sw128_chunk_off(r, cchunk & 7), qc + ((long long)(tk * qsn8 + hq0 + gq[i0 + it]) << 3), valid);
+                    }
                 }
             }
             // arrives on q_full when this thread's copies have landed; nobody waits here, so the
@@ -343,7 +352,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
         if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
         for (int k = 0; k < nloc && ok; ++k) {
-            const int sb = k & 1, sbuf = k % C::NS;
+            const int ob = k % C::NO, sbuf = k % C::NS;
             const int prev_hg = hg0;
             hg0 = hg1; hg1 = hg2;
             if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
@@ -354,17 +363,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             ok = mbar_wait(&p_full[sbuf], (k / C::NS) & 1, status) && ok;
             T_TOC(5);
             if (lane == 0) TR(2, k, 0);
-            ok = mbar_wait(&o_empty[sb], ((k >> 1) & 1) ^ 1, status) && ok;
+            ok = mbar_wait(&o_empty[ob], ((k / C::NO) & 1) ^ 1, status) && ok;
             T_TOC(6);
             if (lane == 0) TR(2, k, 1);
             tc_fence_after();
             const uint32_t b_lo = v_lo + (uint32_t)(kv_cur * (C::kKV >> 4));
-            const uint32_t d_o = tbase + C::cO + sb * D, a_p = tbase + C::cS + sbuf * BK;
+            const uint32_t d_o = tbase + C::cO + ob * D, a_p = tbase + C::cS + sbuf * BK;
             if (leader) {
 #pragma unroll
                 for (int ks = 0; ks < BK / 16; ++ks)
                     umma_ts(d_o, a_p + ks * 8, umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_o, ks > 0);
-                umma_commit(&o_full[sb]);
+                umma_commit(&o_full[ob]);
                 umma_commit(&s_empty[sbuf]);
                 if (last_of_block) umma_commit(&kv_empty[kv_cur]);
             }
@@ -378,20 +387,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
     } else {
         // ------------------------------------------------------------------ softmax + epilogue
         // Group sb (warps 6..9 / 10..13) owns the CTA's tiles with odd / even local index, hence TMEM
-        // buffers S[sb], O[sb] and its own staging area.  One row per thread.
+        // buffers S[sb], O[sb] (head size 256: the one O in turns) and its own staging area.  One row per thread.
         const int sb = (warp - 6) >> 2;
         const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
         const int r = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         const int g = r / s.TPT;
         const int e = r - g * s.TPT;
-        // this warp's 32 staged rows: D/64 slabs of 32 rows x 128 bytes, 128-byte swizzle
-        uint8_t* my_os = sOS + sb * C::kOS + quarter * (32 * D * 2);
+        // this warp's 32 staged rows: slabs of 32 rows x 128 bytes, 128-byte swizzle
+        uint8_t* my_os = sOS + sb * C::kOS + quarter * (32 * C::kOSCols * 2);
+        const int ob = C::NO == 2 ? sb : 0;
         // the (m, l) pairs of a (head, token) complete a 128-byte line over T tiles far apart in time: keep those lines in
         // L2; the partial rows are written once and read once by the merge: let them leave first
         const uint64_t pol_ml = l2_policy_evict_last(), pol_part = l2_policy_evict_first();
         const uint32_t tS0 = tbase + lane_off + C::cS;
-        const uint32_t tO = tbase + lane_off + C::cO + sb * D;
+        const uint32_t tO = tbase + lane_off + C::cO + ob * D;
         bool ok = true;
         T_DECL;
         // software pipeline over this group's tiles: the entry of this thread's row is fetched two
@@ -430,45 +440,50 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         // O / l -> staging -> TMA store, for the tile (prev_j) whose softmax ran one iteration ago
         auto epilogue = [&]() {
             T_TIC;
-            ok = mbar_wait(&o_full[sb], prev_u & 1, status) && ok;
+            ok = mbar_wait(&o_full[ob], (C::NO == 2 ? prev_u : 2 * prev_u + sb) & 1, status) && ok;
             T_TOC(3);
             if (quarter == 2 && lane == 0) TR(3, prev_u * 2 + sb, 2);
             tc_fence_after();
-            if (lane == 0) bulk_wait_read0();   // previous store of this warp has read its staging rows
-            __syncwarp();
-            T_TOC(4);
             // (two TMEM loads in flight per wait, 64 columns per round trip, measured 5 % slower than one)
 #pragma unroll
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tO + c0, v);
-                tmem_ld_wait();
+            for (int s0 = 0; s0 < D; s0 += C::kOSCols) {
+                if (lane == 0) bulk_wait_read0();   // previous store of this warp has read its staging rows
+                __syncwarp();
+                T_TOC(4);
 #pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    // unnormalised O (its row sum l travels in the statistics): rounding to a floating-point
-                    // format is scale-free, so dividing first would not make the partial more accurate
-                    uint4 x;
-                    x.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-                    x.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-                    x.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-                    x.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-                    const int chunk = (c0 >> 3) + q4;     // 16-byte chunk of the row
-                    *reinterpret_cast<uint4*>(my_os + (chunk >> 3) * (32 * 128) + sw128_chunk_off(lane, chunk & 7)) = x;
+                for (int c0 = 0; c0 < C::kOSCols; c0 += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tO + s0 + c0, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q4 = 0; q4 < 4; ++q4) {
+                        // unnormalised O (its row sum l travels in the statistics): rounding to a floating-point
+                        // format is scale-free, so dividing first would not make the partial more accurate
+                        uint4 x;
+                        x.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
+                        x.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
+                        x.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
+                        x.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
+                        const int chunk = (c0 >> 3) + q4;     // 16-byte chunk of the staged row
+                        *reinterpret_cast<uint4*>(my_os + (chunk >> 3) * (32 * 128) + sw128_chunk_off(lane, chunk & 7)) = x;
+                    }
                 }
-            }
-            tc_fence_before();
-            mbar_arrive(&o_empty[sb]);
-            if (prev_valid) st_float2_hint(p.ml + prev_mli, prev_m, prev_l, pol_ml);
-            fence_async_smem();
-            __syncwarp();
+                if (s0 + C::kOSCols == D) {
+                    tc_fence_before();
+                    mbar_arrive(&o_empty[ob]);
+                    if (prev_valid) st_float2_hint(p.ml + prev_mli, prev_m, prev_l, pol_ml);
+                }
+                fence_async_smem();
+                __syncwarp();
 #ifdef FSA_TIMING
-            if (!(p.dbg & 2))
+                if (!(p.dbg & 2))
 #endif
-            if (lane == 0) {
+                if (lane == 0) {
 #pragma unroll
-                for (int b = 0; b < D / 64; ++b)
-                    tma_store_2d_hint(&omap, b * 64, prev_j * kTileRows + quarter * 32, smem_u32(my_os + b * (32 * 128)), pol_part);
-                bulk_commit();
+                    for (int b = 0; b < C::kOSCols / 64; ++b)
+                        tma_store_2d_hint(&omap, s0 + b * 64, prev_j * kTileRows + quarter * 32, smem_u32(my_os + b * (32 * 128)), pol_part);
+                    bulk_commit();
+                }
             }
             T_TOC(5);
             if (quarter == 2 && lane == 0) TR(3, prev_u * 2 + sb, 3);
@@ -583,10 +598,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             if (quarter == 2 && lane == 0) TR(3, k, 1);
 
             // the epilogue of this group's previous tile runs now: its P V has had a whole softmax
-            // to finish, so the wait below is normally free
-            if (have_prev) epilogue();
-            have_prev = true;
+            // to finish, so the wait below is normally free.  (With one O buffer this tile's own: the other group's P V waits
+            // for the buffer.)
+            if (C::NO == 2 && have_prev) epilogue();
+            have_prev = C::NO == 2;
             prev_j = j; prev_u = u; prev_m = m; prev_l = l; prev_valid = row_valid; prev_mli = mli;
+            if (C::NO == 1) epilogue();
         }
         if (have_prev && ok) epilogue();
         if (lane == 0) bulk_wait0();
@@ -599,7 +616,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 
 // ------------------------------------------------------------------------------------------
 // Unpipelined variant (one tile at a time, 128 threads) for the shapes whose tiles do not fit
-// the staged layout above (head_dim 256, 256-key blocks).  Same partial layout.
+// the staged layout above (256-key blocks).  Same partial layout.
 template <int D, int BK>
 struct SelFwdSimpleSmem {
     static constexpr int kK = BK * D * 2;
@@ -898,7 +915,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     { const char* v = getenv("FSA_DBG"); p.dbg = v ? atoi(v) : 0; }
 #endif
     cudaError_t e;
-    constexpr bool kPipelined = (D <= 128 && BK <= 128);
+    constexpr bool kPipelined = BK <= 128;
     // the gather warps of the pipelined kernel address rows by 32-bit offsets in units of 8 elements
     const bool offsets_fit = ((s.N * a.q_sn + (int64_t)s.Hq * a.q_sh) >> 3) < 0x7fffffffll;
     if (kPipelined && a.omap && offsets_fit) {
