@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
     uint64_t* s_full = kv_empty + C::NKV;    // [NS]
     uint64_t* s_empty = s_full + C::NS;      // [NS]
     uint64_t* p_full = s_empty + C::NS;      // [NS]
-    uint64_t* o_full = p_full + C::NS;       // [2]
+    uint64_t* o_full = p_full + C::NS;       // [2] per softmax group
     uint64_t* o_empty = o_full + 2;          // [2]
     uint64_t* off_full = o_empty + 2;        // [4] ring of prepared tiles: tokens, kv head, new-block flag are valid
     uint64_t* off_empty = off_full + kFwdRing;   // [4] ... have been read by the gather warps and the S issuer
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 #pragma unroll
                 for (int ks = 0; ks < BK / 16; ++ks)
                     umma_ts(d_o, a_p + ks * 8, umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_o, ks > 0);
-                umma_commit(&o_full[ob]);
+                umma_commit(&o_full[k & 1]);           // (per group, also when they share one O: a group waits for its own tiles only)
                 umma_commit(&s_empty[sbuf]);
                 if (last_of_block) umma_commit(&kv_empty[kv_cur]);
             }
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         // O / l -> staging -> TMA store, for the tile (prev_j) whose softmax ran one iteration ago
         auto epilogue = [&]() {
             T_TIC;
-            ok = mbar_wait(&o_full[ob], (C::NO == 2 ? prev_u : 2 * prev_u + sb) & 1, status) && ok;
+            ok = mbar_wait(&o_full[sb], prev_u & 1, status) && ok;
             T_TOC(3);
             if (quarter == 2 && lane == 0) TR(3, prev_u * 2 + sb, 2);
             tc_fence_after();
