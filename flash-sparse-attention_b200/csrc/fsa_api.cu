@@ -429,7 +429,7 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     CUtensorMap dqmap;
     a.dqmap = nullptr;
     const int64_t dq_rows = sel_max_tiles(s) * bwd_nsub(BK) * kTileRows;
-    if (D <= 128 && dq_rows < ((int64_t)1 << 31)) {
+    if (dq_rows < ((int64_t)1 << 31)) {
         rc = make_tile_map(&dqmap, a.dq_part, dtype, dq_rows, D, D, 32);
         if (rc) return rc;
         a.dqmap = &dqmap;

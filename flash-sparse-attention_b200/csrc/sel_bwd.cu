@@ -518,7 +518,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     // the gather warps of the pipelined kernel address rows by 32-bit offsets in units of 8 elements
     const bool offsets_fit = ((s.N * a.q_sn + (int64_t)s.Hq * a.q_sh) >> 3) < 0x7fffffffll &&
                              ((s.N * a.do_sn + (int64_t)s.Hq * a.do_sh) >> 3) < 0x7fffffffll;
-    const bool pipelined = D <= 128 && a.dqmap && offsets_fit;
+    const bool pipelined = a.dqmap && offsets_fit;
     cudaError_t e;
     if (!pipelined) {
         e = cudaMemsetAsync(a.dk_acc, 0, kv_elems * 4 * 2, stream);   // dk_acc and dv_acc are adjacent
@@ -545,7 +545,8 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
             e = launch_range_bwd_dq(dt, a, s, kmap, vmap, ix.header, stream);
             if (e != cudaSuccess) return e;
         }
-        e = launch_sel_bwd_pipe(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, dq_dense, stream);
+        e = D == 256 ? launch_sel_bwd_wide(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, stream)
+                     : launch_sel_bwd_pipe(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, dq_dense, stream);
         if (e != cudaSuccess) return e;
     } else {
         auto kern = sel_bwd_main<D, ET>;

@@ -84,16 +84,13 @@ constexpr int kTraceTile0 = 200;
 #define BT_EV(k, ev, who)
 #endif
 
-template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 __device__ __forceinline__ float ex2_approx_b(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
-template <int D, typename ET>
+template <int D, bool PARTS, typename ET>
 __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBwdPipeParams<ET> p,
                                                                      const __grid_constant__ CUtensorMap kmap,
                                                                      const __grid_constant__ CUtensorMap vmap,
@@ -154,7 +151,8 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    const TileSchedule sched(p.ix.header[1], p.run, p.nsub);
+    const TileScheduleT<PARTS> sched(p.ix.header[1], p.run, p.nsub);
+    const int nsub = PARTS ? p.nsub : 1;
     const int nloc = sched.nloc;
     const int key_lim = min(KT, s.BK);
 
@@ -269,7 +267,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             if (lane == 0) {
 #pragma unroll
                 for (int b = 0; b < D / 64; ++b)
-                    tma_store_2d(&dqmap, b * 64, (j * p.nsub + sched.sub(k)) * kTileRows + quarter * 32, smem_u32(my_stage + b * (32 * 128)));
+                    tma_store_2d(&dqmap, b * 64, (j * nsub + sched.sub(k)) * kTileRows + quarter * 32, smem_u32(my_stage + b * (32 * 128)));
                 bulk_commit();
             }
             }
@@ -280,20 +278,17 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             const TileInfo ti = load_tile(p.ix, j0);
             // segments of a key are numbered by the scheduling run they fall into
             const int seg = ti.seg0 + j0 / sched.run - __ldg(p.ix.tile_aux + j0).x / sched.run;
-            float* slab = p.slabs + ((int64_t)seg * p.nsub + sched.sub(k)) * (2 * KT * D) + d_idx;
+            float* slab = p.slabs + ((int64_t)seg * nsub + sched.sub(k)) * (2 * KT * D) + d_idx;
             ok = mbar_wait(acc_full, nflush & 1, status) && ok;
             BT_TOC(3);
             tc_fence_after();
 #pragma unroll
             for (int which = 0; which < 2; ++which) {
                 uint32_t v[KT];
-                // (D = 64: the upper half of the accumulator rows holds products of whatever follows the tile in shared memory)
-                if (quarter * 32 < D) {
 #pragma unroll
-                    for (int c0 = 0; c0 < KT; c0 += 32)
-                        tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[c0]));
-                    tmem_ld_wait();
-                }
+                for (int c0 = 0; c0 < KT; c0 += 32)
+                    tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[c0]));
+                tmem_ld_wait();
                 if (which == 1) {
                     // both accumulators are in registers now: the next segment may overwrite them
                     tc_fence_before();
@@ -301,6 +296,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                     ++nflush;
                 }
                 float* dst = slab + which * (KT * D);
+                // (D = 64: the upper accumulator rows are products of whatever follows the tile in shared memory)
                 if (quarter * 32 < D) {
 #pragma unroll
                     for (int key = 0; key < KT; ++key) dst[key * D] = __uint_as_float(v[key]);
@@ -645,7 +641,7 @@ static cudaError_t launch_pipe(const SelBwdArgs& a, const SelShape& s, const Sel
     p.dq_part = (ET*)a.dq_part; p.slabs = a.slabs;
     p.no_dq = no_dq ? 1 : 0;
     p.nsub = s.BK > bwdpipe::KT ? s.BK / bwdpipe::KT : 1;
-    auto kern = sel_bwd_pipe<D, ET>;
+    auto kern = p.nsub > 1 ? sel_bwd_pipe<D, true, ET> : sel_bwd_pipe<D, false, ET>;
     constexpr int smem = bwdpipe::Cfg<D>::kBytes;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;

@@ -220,20 +220,26 @@ __device__ __forceinline__ int upper_seg(const int* __restrict__ off, int n, int
 // CTAs round-robin, so the whole grid advances through the tile list together (neighbouring
 // blocks of one kv head: their query rows stay in L2) while a CTA still reuses a resident K/V
 // block across the tiles of a run.  nsub > 1 (blocks of more keys than a kernel takes at a time; 1, 2 or 4): every
-// run is dealt nsub times, once for each part of the blocks.
-struct TileSchedule {
+// run is dealt nsub times, once for each part of the blocks.  (PARTS = false, nsub = 1, is compiled apart: the part
+// arithmetic in the index roles cost the backward kernel 9 %.)
+template <bool PARTS>
+struct TileScheduleT {
     int total, grid, cta, run, lsub, nloc;      // lsub: log2 of nsub
-    __device__ TileSchedule(int total_, int run_, int nsub_ = 1)
-        : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_), lsub(nsub_ >> 1) {
-        const int NR = (total + run - 1) / run, NV = NR << lsub;    // runs in the list, dealt runs
+    __device__ TileScheduleT(int total_, int run_, int nsub_ = 1)
+        : total(total_), grid((int)gridDim.x), cta((int)blockIdx.x), run(run_), lsub(PARTS ? nsub_ >> 1 : 0) {
+        const int NR = (total + run - 1) / run, NV = PARTS ? NR << lsub : NR;      // runs in the list, dealt runs
         const int mine = cta < NV ? (NV - cta + grid - 1) / grid : 0;
         nloc = mine * run;
         // the last run may be short (nsub < grid: a CTA has at most one of its parts, as its own last)
-        if (mine > 0 && (cta + (mine - 1) * grid) >> lsub == NR - 1) nloc -= NR * run - total;
+        if (mine > 0 && (cta + (mine - 1) * grid) >> (PARTS ? lsub : 0) == NR - 1) nloc -= NR * run - total;
     }
-    __device__ __forceinline__ int tile(int k) const { return (((k / run) * grid + cta) >> lsub) * run + (k % run); }
-    __device__ __forceinline__ int sub(int k) const { return ((k / run) * grid + cta) & ((1 << lsub) - 1); }
+    __device__ __forceinline__ int tile(int k) const {
+        const int r = (k / run) * grid + cta;
+        return (PARTS ? r >> lsub : r) * run + (k % run);
+    }
+    __device__ __forceinline__ int sub(int k) const { return PARTS ? ((k / run) * grid + cta) & ((1 << lsub) - 1) : 0; }
 };
+using TileSchedule = TileScheduleT<false>;
 
 // Query-tile-major kernels cut every sequence into tiles of TPT consecutive tokens.  Both helpers are warp-collective (every lane calls them and gets the same
 // answer) and walk the sequences 32 at a time, so that a packed batch of thousands of short sequences costs B / 32 steps.

@@ -66,6 +66,10 @@ cudaError_t launch_sel_bwd_pipe(int dtype, const SelBwdArgs& a, const SelShape& 
                                 const CUtensorMap& kmap, const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms,
                                 bool no_dq, cudaStream_t stream);
 
+// ... and for head_dim 256 (sel_bwd_wide.cu)
+cudaError_t launch_sel_bwd_wide(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix, const CUtensorMap& kmap,
+                                const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms, cudaStream_t stream);
+
 // dQ of a range-attention backward as one query-tile-major kernel (range_dense.cu; head_dim 128): the accumulator stays
 // in TMEM across the K/V tiles a tile of tokens sees, so the block-major kernel above runs with no_dq
 cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& s, const CUtensorMap& kmap, const CUtensorMap& vmap,

@@ -324,6 +324,10 @@ __device__ __forceinline__ uint32_t sw128_chunk_off(int row, int chunk) {
     return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
 }
 
+// ---------------------------------------------------------------- register budgets of warpgroups
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---------------------------------------------------------------- element types
 template <typename ET> struct ElemTraits;
 template <> struct ElemTraits<__nv_bfloat16> {
