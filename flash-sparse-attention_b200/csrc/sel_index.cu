@@ -108,6 +108,8 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
 template <bool FILL>
 __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* __restrict__ topk_idx, const int* __restrict__ cu,
                                                                      SelBounds bd, SelShape s, SelIndex ix) {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ int sm[];   // [nwarps][NBmax]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int c = blockIdx.x, h = blockIdx.y;
@@ -143,6 +145,8 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
 
 // Step 2: per key, exclusive prefix of the chunks' counts and the total (thread per key; eight loads in flight).
 __global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
+    pdl_trigger();
+    pdl_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= s.Hk * s.NBmax) return;
     const int h = k / s.NBmax, gb = k - h * s.NBmax;
@@ -164,6 +168,8 @@ __global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
 // Step 3: exclusive scans over the keys (a single CTA): first tile, then -- it depends on the first tile -- first segment.
 // A key with tiles [t0, t0 + nt) is cut by the backward's schedule at every multiple of RB.
 __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ int wsum_a[32], wsum_b[32], wsum_c[32];
     __shared__ int carry_a, carry_b, carry_c;
     const int HG = s.Hk * s.NBmax;
@@ -241,6 +247,8 @@ __device__ __forceinline__ void write_tiles(const SelShape& s, const SelIndex& i
 
 // Step 4: tile records and the padding of the tile-ordered entry list: one warp per key.
 __global__ void __launch_bounds__(256) sel_index_tiles(const int* __restrict__ cu, SelBounds bd, SelShape s, SelIndex ix) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int hg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (hg >= s.Hk * s.NBmax) return;
@@ -279,9 +287,11 @@ __device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total)
 
 __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* __restrict__ topk_idx, const int* __restrict__ cu, SelBounds bd,
                                                                   SelShape s, SelIndex ix) {
+    pdl_trigger();
+    pdl_wait();
     namespace cg = cooperative_groups;
     extern __shared__ int sm[];   // [warps][NBmax] counts, then positions; [NBmax] entries, [NBmax] first tile, [NBmax] first segment of a key
-    __shared__ int wsum[32], mine[2];
+    __shared__ int wsum[32], mine[3];       // tiles, entries, segments of this head
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, NB = s.NBmax;
     int *s_cnt = sm + kSmallWarps * NB, *s_t0 = s_cnt + NB, *s_seg = s_t0 + NB;
@@ -290,14 +300,20 @@ __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* _
     __syncthreads();
     chunk_pass<false>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
     __syncthreads();
-    int cnt = 0;
-    if (tid < NB) {
-        for (int w = 0; w < kSmallWarps; ++w) {
-            const int v = sm[w * NB + tid];
-            sm[w * NB + tid] = cnt;            // this warp's first position inside the key
-            cnt += v;
+    // a warp per key: lane w turns warp w's count into its first position inside the key
+    for (int gb = warp; gb < NB; gb += kSmallWarps) {
+        const int v = sm[lane * NB + gb];
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
         }
+        sm[lane * NB + gb] = incl - v;
+        if (lane == 31) s_cnt[gb] = incl;
     }
+    __syncthreads();
+    const int cnt = tid < NB ? s_cnt[tid] : 0;
     int entries = 0, tiles = 0, segs = 0;
     cta_prefix(cnt, wsum, tid, &entries);
     const int nt = (cnt + s.TPT - 1) / s.TPT;
@@ -305,39 +321,33 @@ __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* _
     // tiles and entries of the heads before this one, and of all
     if (tid == 0) { mine[0] = tiles; mine[1] = entries; }
     cluster.sync();
-    int all_tiles = 0, all_entries = 0;
-    for (int r = 0; r < s.Hk; ++r) {
-        const int* other = cluster.map_shared_rank(mine, r);
-        if (r < h) t0 += other[0];
-        all_tiles += other[0];
-        all_entries += other[1];
-    }
-    cluster.sync();                            // everybody has read before the words are used again
+    const int v0 = lane < s.Hk ? cluster.map_shared_rank(mine, lane)[0] : 0, v1 = lane < s.Hk ? cluster.map_shared_rank(mine, lane)[1] : 0;
+    t0 += __reduce_add_sync(0xffffffffu, lane < h ? v0 : 0);
+    const int all_tiles = __reduce_add_sync(0xffffffffu, v0), all_entries = __reduce_add_sync(0xffffffffu, v1);
     int seg = cta_prefix(nt > 0 ? (t0 + nt - 1) / s.RB - t0 / s.RB + 1 : 0, wsum, tid, &segs);
-    if (tid == 0) mine[0] = segs;
+    if (tid == 0) mine[2] = segs;
     if (tid == 0 && h == 0) {
         ix.header[0] = kStatusOk; ix.header[1] = all_tiles; ix.header[2] = all_entries;
         ix.key_tile[s.Hk * NB] = all_tiles;
     }
     cluster.sync();
-    int all_segs = 0;
-    for (int r = 0; r < s.Hk; ++r) {
-        const int v = cluster.map_shared_rank(mine, r)[0];
-        if (r < h) seg += v;
-        all_segs += v;
-    }
+    const int v2 = lane < s.Hk ? cluster.map_shared_rank(mine, lane)[2] : 0;
+    seg += __reduce_add_sync(0xffffffffu, lane < h ? v2 : 0);
+    const int all_segs = __reduce_add_sync(0xffffffffu, v2);
+    cluster.barrier_arrive();                  // (nothing of another CTA is read from here on; none leaves before all have come here)
     if (tid < NB) {
         const int hg = h * NB + tid;
         ix.key_cnt[hg] = cnt; ix.key_tile[hg] = t0; ix.key_seg[hg] = seg;
-        s_cnt[tid] = cnt; s_t0[tid] = t0; s_seg[tid] = seg;
-        for (int w = 0; w < kSmallWarps; ++w) sm[w * NB + tid] += t0 * s.TPT;
+        s_t0[tid] = t0; s_seg[tid] = seg;
     }
     if (tid == 0 && h == 0) { ix.header[3] = all_segs; ix.key_seg[s.Hk * NB] = all_segs; }
     __syncthreads();
     for (int gb = warp; gb < NB; gb += kSmallWarps)
         if (s_cnt[gb] > 0) write_tiles(s, ix, ck, h, gb, s_cnt[gb], s_t0[gb], s_seg[gb], lane);
+    for (int gb = lane; gb < NB; gb += 32) sm[warp * NB + gb] += s_t0[gb] * s.TPT;
+    __syncwarp();
     chunk_pass<true>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
-    cluster.sync();                            // no CTA leaves while another reads its shared memory
+    cluster.barrier_wait();
 }
 
 // warps per CTA of the chunk kernels so that the per-warp histograms fit in shared memory; 0: the problem does not fit
@@ -364,11 +374,13 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
         cfg.blockDim = dim3(kSmallWarps * 32);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = 1; at.val.clusterDim.y = (unsigned)s.Hk; at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)s.Hk; at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 2;
         return cudaLaunchKernelEx(&cfg, sel_index_small, topk_idx, cu, bd, s, ix);
     }
     const int nw = s.IW;
@@ -380,11 +392,11 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)s.NC, (unsigned)s.Hk);
     const int HG = s.Hk * s.NBmax;
-    sel_index_chunk<false><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
-    sel_index_keys<<<(unsigned)((HG + 63) / 64), 64, 0, stream>>>(s, ix);
-    sel_index_scan<<<1, 1024, 0, stream>>>(s, ix);
-    sel_index_tiles<<<(unsigned)((HG + 7) / 8), 256, 0, stream>>>(cu, bd, s, ix);
-    sel_index_chunk<true><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
+    launch_pdl(sel_index_chunk<false>, grid, nw * 32, smem, stream, topk_idx, cu, bd, s, ix);
+    launch_pdl(sel_index_keys, (unsigned)((HG + 63) / 64), 64, 0, stream, s, ix);
+    launch_pdl(sel_index_scan, 1, 1024, 0, stream, s, ix);
+    launch_pdl(sel_index_tiles, (unsigned)((HG + 7) / 8), 256, 0, stream, cu, bd, s, ix);
+    launch_pdl(sel_index_chunk<true>, grid, nw * 32, smem, stream, topk_idx, cu, bd, s, ix);
     return cudaGetLastError();
 }
 
