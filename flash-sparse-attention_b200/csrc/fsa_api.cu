@@ -3,7 +3,7 @@
 // no allocation, no synchronisation on the compute paths.
 #include "../../include/fsa_sm100.h"
 #include "sel_common.cuh"
-#include "sel_launch.cuh"
+#include "range_bwd.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -213,6 +213,11 @@ static int64_t bwd_dkdv_bytes(const SelShape& s) {
     const int64_t slabs = align_up(sel_max_segments(s) * bwd_nsub(s.BK) * 2 * 64 * (int64_t)s.D * 4, 256);
     return acc > slabs ? acc : slabs;
 }
+// ranges: the query-tile-major and key-tile-major kernels serve head_dim 128 (their TMEM layout), the block-major ones the others
+static bool range_bwd_dense(int D) { return D == 128; }
+static int64_t range_bwd_scratch_bytes(const SelShape& s) {
+    return align_up(s.N * s.Hq * 4, 1024) + align_up(range_kv_plan_bytes(s), 1024) + range_kv_slab_bytes(s);
+}
 static int64_t bwd_scratch_bytes(const SelShape& s) {
     return align_up(s.N * s.Hq * 4, 1024) + bwd_dq_part_bytes(s) + bwd_dkdv_bytes(s);
 }
@@ -404,8 +409,9 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     if ((q_sn % 8) || (q_sh % 8) || (k_sn % 8) || (v_sn % 8) || (o_sn % 8) || (o_sh % 8) || (do_sn % 8) || (do_sh % 8))
         return FSA_ERR_BAD_ARG;
     if (k_sn < (int64_t)Hk * D || v_sn < (int64_t)Hk * D) return FSA_ERR_BAD_ARG;
-    if (index_ws_bytes < sel_index_bytes(s)) return FSA_ERR_WORKSPACE;
-    if (scratch_bytes < bwd_scratch_bytes(s)) return FSA_ERR_WORKSPACE;
+    const bool dense = bd.kv_hi && range_bwd_dense(D);          // (of the index only the status word is used)
+    if (index_ws_bytes < (dense ? 16 : sel_index_bytes(s))) return FSA_ERR_WORKSPACE;
+    if (scratch_bytes < (dense ? range_bwd_scratch_bytes(s) : bwd_scratch_bytes(s))) return FSA_ERR_WORKSPACE;
 
     SelIndex ix = sel_index_carve(index_ws, s);
     CUtensorMap kmap, vmap;
@@ -425,9 +431,26 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     char* sp = (char*)scratch;
     a.delta = delta ? const_cast<float*>(delta) : (float*)sp;   sp += align_up(N * Hq * 4, 1024);
     a.have_delta = delta != nullptr;
-    a.dq_part = (void*)sp;  sp += bwd_dq_part_bytes(s);
+    a.bd = bd;
+    a.dq = dq; a.dk = dk; a.dv = dv;
     CUtensorMap dqmap;
-    a.dqmap = nullptr;
+    a.dqmap = nullptr; a.plan = nullptr;
+    if (dense) {
+        RangeKvPlan plan;
+        plan.cu_q = cu_seqlens; plan.cu_k = bd.cu_k ? bd.cu_k : cu_seqlens; plan.kv_lo = bd.kv_lo; plan.kv_hi = bd.kv_hi;
+        plan.N = N; plan.Nk = Nk; plan.B = B; plan.Hk = Hk; plan.TPT = s.TPT;
+        plan.max_tiles = (int)range_kv_max_tiles(s);
+        plan.counts = (int*)sp;
+        plan.tiles = (int4*)(sp + 256);
+        plan.multi = plan.tiles + plan.max_tiles;
+        plan.items = plan.multi + plan.max_tiles;
+        sp += align_up(range_kv_plan_bytes(s), 1024);
+        a.slabs = (float*)sp;
+        a.plan = &plan;
+        const cudaError_t e = dispatch_sel_bwd(dtype, a, s, ix, kmap, vmap, sms, stream);
+        return e == cudaSuccess ? FSA_OK : cuda_fail(e);
+    }
+    a.dq_part = (void*)sp;  sp += bwd_dq_part_bytes(s);
     const int64_t dq_rows = sel_max_tiles(s) * bwd_nsub(BK) * kTileRows;
     if (dq_rows < ((int64_t)1 << 31)) {
         rc = make_tile_map(&dqmap, a.dq_part, dtype, dq_rows, D, D, 32);
@@ -437,8 +460,6 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     a.dk_acc = (float*)sp;
     a.dv_acc = a.dk_acc + Nk * Hk * (int64_t)D;
     a.slabs = (float*)sp;
-    a.bd = bd;
-    a.dq = dq; a.dk = dk; a.dv = dv;
     cudaError_t e = dispatch_sel_bwd(dtype, a, s, ix, kmap, vmap, sms, stream);
     if (e != cudaSuccess) return cuda_fail(e);
     return FSA_OK;
@@ -517,9 +538,11 @@ int fsa_range_attn_bytes(int64_t N, int64_t Nk, int B, int Hq, int Hk, int D, in
     if (rc) return rc;
     if (index_bytes_out) *index_bytes_out = sel_index_bytes(s);
     if (fwd_scratch_bytes_out) *fwd_scratch_bytes_out = fwd_scratch_bytes(s);
-    if (bwd_scratch_bytes_out) *bwd_scratch_bytes_out = bwd_scratch_bytes(s);
+    if (bwd_scratch_bytes_out) *bwd_scratch_bytes_out = range_bwd_dense(D) ? range_bwd_scratch_bytes(s) : bwd_scratch_bytes(s);
     return FSA_OK;
 }
+
+int fsa_range_attn_bwd_indexed(int D) { return range_bwd_dense(D) ? 0 : 1; }
 
 static int sel_static_base(void** out);
 

@@ -104,8 +104,9 @@ static std::tuple<Tensor, Tensor, Tensor> range_bwd(const Tensor& q, const Tenso
     const int B = (int)cu_q.size(0) - 1, Hq = (int)q.size(1), Hk = (int)k.size(1), D = (int)q.size(2);
     int64_t ib = 0, fb = 0, bb = 0;
     check(fsa_range_attn_bytes(N, Nk, B, Hq, Hk, D, max_blocks, 64, &ib, &fb, &bb), "fsa_range_attn_bytes");
-    const Tensor ws = bytes(ib, q), scratch = bytes(bb, q);
-    check(fsa_range_attn_index(iptr(cu_q), iptr(cu_k), lo, hi, N, Nk, B, Hq, Hk, max_blocks, 64, ptr(ws), ws.numel(), stream_of(q)), "fsa_range_attn_index");
+    const bool indexed = fsa_range_attn_bwd_indexed(D) != 0;
+    const Tensor ws = bytes(indexed ? ib : 16, q), scratch = bytes(bb, q);
+    if (indexed) check(fsa_range_attn_index(iptr(cu_q), iptr(cu_k), lo, hi, N, Nk, B, Hq, Hk, max_blocks, 64, ptr(ws), ws.numel(), stream_of(q)), "fsa_range_attn_index");
     Tensor dq = at::empty_like(q), dk = at::empty({Nk, Hk, D}, q.options()), dv = at::empty_like(dk);
     check(fsa_range_attn_bwd_delta(ptr(q), ptr(k), ptr(v), lse.data_ptr<float>(), ptr(dout), delta, iptr(cu_q), iptr(cu_k), lo, hi, N, Nk, B, Hq, Hk, D,
                                    max_blocks, 64, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1),

@@ -15,7 +15,7 @@
 //
 // Blocks larger than 64 keys are walked as BK/64 independent 64-key sub-tiles (the backward has
 // no per-block softmax state); a 32-key block is a 64-key tile whose upper half is masked.
-#include "sel_launch.cuh"
+#include "range_bwd.cuh"
 
 namespace fsa {
 
@@ -530,7 +530,11 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
                              ((s.N * a.do_sn + (int64_t)s.Hq * a.do_sh) >> 3) < 0x7fffffffll;
     const bool pipelined = a.dqmap && offsets_fit;
     cudaError_t e;
-    if (!pipelined) {
+    const int dt = ElemTraits<ET>::kIsBF16 ? (int)kBF16 : (int)kFP16;
+    if (a.plan) {
+        e = launch_range_bwd_plan(*a.plan, a, ix.header, stream);
+        if (e != cudaSuccess) return e;
+    } else if (!pipelined) {
         e = cudaMemsetAsync(a.dk_acc, 0, kv_elems * 4 * 2, stream);   // dk_acc and dv_acc are adjacent
         if (e != cudaSuccess) return e;
     }
@@ -540,6 +544,10 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         launch_pdl(sel_bwd_delta<ET>, grid, 256, 0, stream, (const ET*)a.o, a.o_sn, a.o_sh, (const ET*)a.d_o, a.do_sn, a.do_sh,
                                                     s.N, s.Hq, D, a.delta);
     }
+    if (a.plan) {
+        e = launch_range_bwd_dq(dt, a, s, kmap, vmap, ix.header, stream);
+        return e == cudaSuccess ? launch_range_bwd_dkdv(dt, *a.plan, a, s, kmap, vmap, ix.header, stream) : e;
+    }
     SelBwdParams<ET> p;
     p.q = (const ET*)a.q; p.q_sn = a.q_sn; p.q_sh = a.q_sh;
     p.d_o = (const ET*)a.d_o; p.do_sn = a.do_sn; p.do_sh = a.do_sh;
@@ -547,16 +555,9 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     p.s = s; p.ix = ix; p.nsub = nsub; p.bd = a.bd;
     p.scale = a.sm_scale; p.scale_log2 = a.sm_scale * 1.4426950408889634f;
     p.dq_part = (ET*)a.dq_part; p.dk_acc = a.dk_acc; p.dv_acc = a.dv_acc;
-    // range attention (every token sees one contiguous range): dQ by the query-tile-major kernel, no partial dQ rows
-    const bool dq_dense = pipelined && D == 128 && a.bd.kv_hi != nullptr && s.G <= 32;
     if (pipelined) {
-        const int dt = ElemTraits<ET>::kIsBF16 ? (int)kBF16 : (int)kFP16;
-        if (dq_dense && rows > 0) {
-            e = launch_range_bwd_dq(dt, a, s, kmap, vmap, ix.header, stream);
-            if (e != cudaSuccess) return e;
-        }
         e = D == 256 ? launch_sel_bwd_wide(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, stream)
-                     : launch_sel_bwd_pipe(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, dq_dense, stream);
+                     : launch_sel_bwd_pipe(dt, a, s, ix, kmap, vmap, *a.dqmap, num_sms, stream);
         if (e != cudaSuccess) return e;
     } else {
         auto kern = sel_bwd_main<D, ET>;
@@ -573,7 +574,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (rows > 0 && !dq_dense) {
+    if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
         prof_begin(3, stream);
         launch_pdl(sel_bwd_dq_reduce<D, ET>, grid, 256, 0, stream, (const ET*)a.dq_part, ix.pos, s, nsub, (ET*)a.dq);

@@ -40,6 +40,8 @@ struct SelFwdArgs {
 cudaError_t dispatch_sel_fwd(int dtype, const SelFwdArgs& a, const SelShape& s, const SelIndex& ix, int num_sms,
                              cudaStream_t stream);
 
+struct RangeKvPlan;      // range_bwd.cuh
+
 struct SelBwdArgs {
     const void *q, *d_o, *o;
     int64_t q_sn, q_sh, do_sn, do_sh, o_sn, o_sh;
@@ -59,19 +61,20 @@ struct SelBwdArgs {
     // outputs (contiguous)
     void *dq, *dk, *dv;
     SelBounds bd;      // visible K/V rows per token (all null: causal rule of selected attention)
+    const RangeKvPlan* plan;    // range attention on the query-tile-major and key-tile-major kernels (null: block-major)
 };
 
 // pipelined main kernel for head_dim 64 and 128 (sel_bwd_pipe.cu)
 cudaError_t launch_sel_bwd_pipe(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix,
                                 const CUtensorMap& kmap, const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms,
-                                bool no_dq, cudaStream_t stream);
+                                cudaStream_t stream);
 
 // ... and for head_dim 256 (sel_bwd_wide.cu)
 cudaError_t launch_sel_bwd_wide(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix, const CUtensorMap& kmap,
                                 const CUtensorMap& vmap, const CUtensorMap& dqmap, int num_sms, cudaStream_t stream);
 
 // dQ of a range-attention backward as one query-tile-major kernel (range_dense.cu; head_dim 128): the accumulator stays
-// in TMEM across the K/V tiles a tile of tokens sees, so the block-major kernel above runs with no_dq
+// in TMEM across the K/V tiles a tile of tokens sees (dK and dV: range_bwd_dkdv.cu)
 cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& s, const CUtensorMap& kmap, const CUtensorMap& vmap,
                                 int* status, cudaStream_t stream);
 

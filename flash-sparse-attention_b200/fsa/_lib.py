@@ -55,6 +55,7 @@ SIGNATURES = {
     ),
     "fsa_range_attn_bytes": (c_int, [c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, POINTER(c_int64),
                                      POINTER(c_int64), POINTER(c_int64)]),
+    "fsa_range_attn_bwd_indexed": (c_int, [c_int]),
     "fsa_range_attn_fwd": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int,

@@ -91,7 +91,9 @@ class RangeAttention(torch.autograd.Function):
         dev = q.device
         ib, _, bb = _sizes(N, Nk, B, Hq, Hk, D, ctx.max_blocks)
         scratch = _alloc_bytes(bb, dev)
-        if not ctx.has_index:
+        if not ctx.has_index and not L.fsa_range_attn_bwd_indexed(D):
+            index_ws = _alloc_bytes(16, dev)
+        elif not ctx.has_index:
             index_ws = _alloc_bytes(ib, dev)
             with torch.cuda.device(dev):
                 rc = L.fsa_range_attn_index(_lib.ptr(cu_q), _lib.ptr(cu_k), _lib.ptr(kv_lo), _lib.ptr(kv_hi), N, Nk, B, Hq, Hk,

@@ -151,9 +151,10 @@ int fsa_sel_bwd(const void* q, const void* k, const void* v, const void* o, cons
  *       fsa/module/fsa.py:149-159: kv_lo[n] = max(cu[b], n - W), kv_hi[n] = n.
  * Tensors, strides, dtype, lse (log2 units), workspaces and return codes are as for fsa_sel_fwd / fsa_sel_bwd;
  * fsa_range_attn_bytes returns the three workspace sizes (any out pointer may be null).
- * fsa_range_attn_bwd at head_dim 128 computes dq with a query-tile-major kernel (accumulator in TMEM over the K/V tiles a
- * tile of tokens sees, written once) and dk / dv with the block-major kernel; other head sizes use the block-major kernel
- * for all three. */
+ * fsa_range_attn_bwd at head_dim 128 computes dq with a query-tile-major and dk / dv with a key-tile-major kernel
+ * (accumulators in TMEM over the K/V tiles a tile of tokens sees, and over the tokens that see a K/V tile); it needs no index,
+ * index_ws is then any 16 bytes or more (the status word).  Other head sizes use the block-major kernel for all three and
+ * the index; fsa_range_attn_bwd_indexed(head_dim) says which (1: the index is needed). */
 int fsa_range_attn_bytes(int64_t total_tokens, int64_t total_kv_rows, int batch, int num_q_heads, int num_kv_heads,
                          int head_dim, int max_blocks, int block_size, int64_t* index_bytes_out,
                          int64_t* fwd_scratch_bytes_out, int64_t* bwd_scratch_bytes_out);
@@ -178,13 +179,14 @@ int fsa_range_attn_bwd(const void* q, const void* k, const void* v, const void* 
  * forward of CompressedAttention, nsa_ref/ops/compressed_attention.py:33-190, :762-829, and the sliding-window
  * flash_attn_varlen_func call of fsa/module/fsa.py:149-159).  head_dim 64 or 128, GQA group <= 32.  status: a device int
  * (zeroed by the caller) that receives a non-zero code if a bounded wait ran out, or NULL.
- * fsa_range_attn_bwd needs the tile index that fsa_range_attn_fwd leaves in index_ws; after this forward, build it
- * with fsa_range_attn_index (same max_blocks / block_size as the backward call). */
+ * Where fsa_range_attn_bwd needs the tile index (fsa_range_attn_bwd_indexed), fsa_range_attn_fwd leaves it in index_ws; after
+ * this forward, build it with fsa_range_attn_index (same max_blocks / block_size as the backward call). */
 int fsa_range_attn_fwd_dense(const void* q, const void* k, const void* v, const int32_t* cu_seqlens_q,
                              const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi, int64_t total_tokens,
                              int64_t total_kv_rows, int batch, int num_q_heads, int num_kv_heads, int head_dim, int dtype,
                              int64_t q_stride_n, int64_t q_stride_h, int64_t k_stride_n, int64_t v_stride_n, float sm_scale,
                              void* o, int64_t o_stride_n, int64_t o_stride_h, float* lse, int32_t* status, void* stream);
+int fsa_range_attn_bwd_indexed(int head_dim);
 int fsa_range_attn_index(const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi,
                          int64_t total_tokens, int64_t total_kv_rows, int batch, int num_q_heads, int num_kv_heads,
                          int max_blocks, int block_size, void* index_ws, int64_t index_ws_bytes, void* stream);
