@@ -66,8 +66,6 @@ constexpr int kDecKT = 64;
 template <int D, bool HI, typename ET>
 __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                                                           const __grid_constant__ CUtensorMap vmap) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ __align__(1024) unsigned char dsm_raw[];
     constexpr int HALF_BYTES = 64 * 128;                 // one 64-column half of 64 rows
     constexpr int KV_BYTES = (D / 64) * HALF_BYTES;
@@ -316,8 +314,6 @@ template <> __device__ __forceinline__ void store4<__half>(__half* dst, float4 v
 template <typename OT>
 __global__ void __launch_bounds__(256) lse_merge_kernel(const float* __restrict__ o_part, const float2* __restrict__ ml, int64_t rows, int P,
                                                         int PS, int D, OT* __restrict__ o, float* __restrict__ lse) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -377,8 +373,6 @@ template <typename ET>
 __global__ void __launch_bounds__(256) decode_finish_kernel(const float* __restrict__ o_part, const float2* __restrict__ ml, int64_t rows,
                                                             int ns, int nw, int PS, int D, int Hq, const ET* __restrict__ o_cmp,
                                                             const ET* __restrict__ gate, ET* __restrict__ out) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -474,8 +468,6 @@ struct DecodeTopkParams {
 };
 
 __global__ void __launch_bounds__(256) decode_topk_kernel(const DecodeTopkParams p) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ float tsm[];
     float* bs = tsm;                                         // [max_blocks] bf16-rounded block scores
     int* sel = reinterpret_cast<int*>(bs + p.max_blocks);    // [64] winners in selection order
@@ -560,8 +552,6 @@ __global__ void __launch_bounds__(256) decode_topk_kernel(const DecodeTopkParams
 __global__ void decode_ranges_kernel(const int32_t* __restrict__ topk_idx, const int* __restrict__ seq_len, const int* __restrict__ seq_row0,
                                      int B, int Hk, int T, int BK, int window, int piece, int NW, int shard_lo, int shard_hi,
                                      int* __restrict__ lo_out, int* __restrict__ hi_out) {
-    pdl_trigger();
-    pdl_wait();
     const int R = T + NW;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B * Hk * R) return;
@@ -592,8 +582,6 @@ __global__ void decode_ranges_kernel(const int32_t* __restrict__ topk_idx, const
 // Visible compressed tokens of the decoded row and the cache rows of this GPU's share of them.
 __global__ void decode_cmp_ranges_kernel(const int* __restrict__ seq_len, const int* __restrict__ cmp_row0, int B, int Hk, int ks, int stride,
                                          int cmp_lo, int cmp_hi, int* __restrict__ num_cmp, int* __restrict__ lo_out, int* __restrict__ hi_out) {
-    pdl_trigger();
-    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B * Hk) return;
     const int b = i / Hk;
@@ -613,7 +601,7 @@ static cudaError_t launch_partial_tma(DecodeParams p, const CUtensorMap& kmap, c
     auto kern = decode_partial_tma<D, HI, ET>;
     const cudaError_t e = allow_smem((const void*)kern, 3 * STAGE_BYTES + 2048);
     if (e != cudaSuccess) return e;
-    launch_pdl(kern, (unsigned)((int64_t)p.B * p.Hk * p.NP * p.nchunk), 160, smem, stream, p, kmap, vmap);
+    kern<<<(unsigned)((int64_t)p.B * p.Hk * p.NP * p.nchunk), 160, smem, stream>>>(p, kmap, vmap);
     return cudaGetLastError();
 }
 
@@ -695,11 +683,11 @@ extern "C" int fsa_lse_merge(const float* o_part, const float* ml, int64_t rows,
     unsigned grid = (unsigned)((rows + 7) / 8);
     cudaStream_t st = (cudaStream_t)stream;
     if (out_dtype == FSA_DTYPE_BF16)
-        launch_pdl(lse_merge_kernel<__nv_bfloat16>, grid, 256, 0, st, o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (__nv_bfloat16*)o, lse);
+        lse_merge_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (__nv_bfloat16*)o, lse);
     else if (out_dtype == FSA_DTYPE_FP16)
-        launch_pdl(lse_merge_kernel<__half>, grid, 256, 0, st, o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (__half*)o, lse);
+        lse_merge_kernel<__half><<<grid, 256, 0, st>>>(o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (__half*)o, lse);
     else if (out_dtype == 2)
-        launch_pdl(lse_merge_kernel<float>, grid, 256, 0, st, o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (float*)o, lse);
+        lse_merge_kernel<float><<<grid, 256, 0, st>>>(o_part, (const float2*)ml, rows, num_partials, part_stride, head_dim, (float*)o, lse);
     else
         return FSA_ERR_BAD_ARG;
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
@@ -734,7 +722,7 @@ extern "C" int fsa_decode_select_topk(const float* scores, int64_t scores_ld, in
         cudaError_t e = allow_smem((const void*)decode_topk_kernel, (int)smem);
         if (e != cudaSuccess) return FSA_ERR_CUDA;
     }
-    launch_pdl(decode_topk_kernel, (unsigned)(batch * num_kv_heads), 256, smem, (cudaStream_t)stream, p);
+    decode_topk_kernel<<<(unsigned)(batch * num_kv_heads), 256, smem, (cudaStream_t)stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
@@ -747,7 +735,7 @@ extern "C" int fsa_decode_ranges(const int32_t* topk_idx, const int32_t* seq_len
     if ((int64_t)piece * num_window_pieces < (int64_t)window + 1 && num_window_pieces > 0) return FSA_ERR_BAD_ARG;
     const int total = batch * num_kv_heads * (topk + num_window_pieces);
     (void)cudaGetLastError();
-    launch_pdl(decode_ranges_kernel, (total + 255) / 256, 256, 0, (cudaStream_t)stream, topk_idx, seq_len, seq_row0, batch, num_kv_heads, topk,
+    decode_ranges_kernel<<<(total + 255) / 256, 256, 0, (cudaStream_t)stream>>>(topk_idx, seq_len, seq_row0, batch, num_kv_heads, topk,
                                                                              block_size, window, piece, num_window_pieces, shard_lo,
                                                                              shard_hi, rng_lo, rng_hi);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
@@ -760,7 +748,7 @@ extern "C" int fsa_decode_cmp_ranges(const int32_t* seq_len, const int32_t* cmp_
         return FSA_ERR_BAD_ARG;
     (void)cudaGetLastError();
     const int total = batch * num_kv_heads;
-    launch_pdl(decode_cmp_ranges_kernel, (total + 255) / 256, 256, 0, (cudaStream_t)stream, seq_len, cmp_row0, batch, num_kv_heads, kernel_size,
+    decode_cmp_ranges_kernel<<<(total + 255) / 256, 256, 0, (cudaStream_t)stream>>>(seq_len, cmp_row0, batch, num_kv_heads, kernel_size,
                                                                                  kernel_stride, cmp_lo, cmp_hi, num_cmp, rng_lo, rng_hi);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
@@ -781,11 +769,11 @@ extern "C" int fsa_decode_finish(const float* o_part, const float* ml, int64_t r
     unsigned grid = (unsigned)((rows + 7) / 8);
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == FSA_DTYPE_BF16)
-        launch_pdl(decode_finish_kernel<__nv_bfloat16>, grid, 256, 0, st, o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride,
+        decode_finish_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride,
                                                                  head_dim, num_q_heads, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)gate,
                                                                  (__nv_bfloat16*)out);
     else if (dtype == FSA_DTYPE_FP16)
-        launch_pdl(decode_finish_kernel<__half>, grid, 256, 0, st, o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride, head_dim,
+        decode_finish_kernel<__half><<<grid, 256, 0, st>>>(o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride, head_dim,
                                                           num_q_heads, (const __half*)o_cmp, (const __half*)gate, (__half*)out);
     else
         return FSA_ERR_BAD_ARG;

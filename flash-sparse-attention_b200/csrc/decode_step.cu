@@ -49,8 +49,6 @@ struct DecodeProjParams {
 
 template <int NT, typename ET>
 __global__ void __launch_bounds__(256) decode_proj_kernel(const DecodeProjParams p) {
-    pdl_trigger();
-    pdl_wait();
     __shared__ float red[8][16][8 * NT + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
     int m = 0;
@@ -123,8 +121,6 @@ __device__ __forceinline__ float sigmoid_et(float z) { return round_et<ET>(1.f /
 
 template <typename ET>
 __global__ void __launch_bounds__(256) decode_append_kernel(const DecodeAppendParams p) {
-    pdl_trigger();
-    pdl_wait();
     __shared__ float s_cos[128], s_sin[128];
     __shared__ float s_z[3][8];
     const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -228,8 +224,6 @@ constexpr int kDcSplit = 8, kDcSeqs = 8, kDcPitch = 12;
 
 template <int D, typename ET>
 __global__ void __launch_bounds__(256, 1) decode_compress_kernel(const DecodeCompressParams p) {
-    pdl_trigger();
-    pdl_wait();
     namespace cg = cooperative_groups;
     constexpr int CG = D / 8, KL = 256 / CG;          // 16-byte column groups, reduction lanes
     extern __shared__ __align__(16) float dcs[];      // [KS][kDcPitch] inputs, later [8][kDcSeqs + 1][D] sums of the warps
@@ -407,8 +401,6 @@ __device__ __forceinline__ void warp_largest(const uint32_t* in, int n, int want
 
 template <typename ET>
 __global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectParams p) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ uint32_t dks[];                 // [max_blocks] keys, the probabilities, [G][P] merge weights
     __shared__ float s_lse, s_inv[16];
     __shared__ uint32_t cand[8 * 64], s_best[8 * 64], sel[64];
@@ -565,11 +557,11 @@ extern "C" int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k
     (void)cudaGetLastError();
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == FSA_DTYPE_BF16) {
-        if (batch <= 8) launch_pdl(decode_proj_kernel<1, __nv_bfloat16>, tiles, 256, 0, st, p);
-        else launch_pdl(decode_proj_kernel<2, __nv_bfloat16>, tiles, 256, 0, st, p);
+        if (batch <= 8) decode_proj_kernel<1, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
+        else decode_proj_kernel<2, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
     } else {
-        if (batch <= 8) launch_pdl(decode_proj_kernel<1, __half>, tiles, 256, 0, st, p);
-        else launch_pdl(decode_proj_kernel<2, __half>, tiles, 256, 0, st, p);
+        if (batch <= 8) decode_proj_kernel<1, __half><<<tiles, 256, 0, st>>>(p);
+        else decode_proj_kernel<2, __half><<<tiles, 256, 0, st>>>(p);
     }
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
@@ -589,8 +581,8 @@ extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void*
     p.inv_freq = inv_freq; p.seq_len = seq_len; p.seq_row0 = seq_row0; p.spare_row = (int64_t)batch * cap; p.cap = cap; p.ks = kernel_size;
     p.z = gate_logits; p.gx = gate_x; p.gw = gate_w; p.glen = gate_dim; p.gate = gate; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.D = head_dim;
     (void)cudaGetLastError();
-    if (dtype == FSA_DTYPE_BF16) launch_pdl(decode_append_kernel<__nv_bfloat16>, batch, 256, 0, (cudaStream_t)stream, p);
-    else launch_pdl(decode_append_kernel<__half>, batch, 256, 0, (cudaStream_t)stream, p);
+    if (dtype == FSA_DTYPE_BF16) decode_append_kernel<__nv_bfloat16><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
+    else decode_append_kernel<__half><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
@@ -606,13 +598,11 @@ static cudaError_t launch_compress(const DecodeCompressParams& p, cudaStream_t s
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kDcSplit; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kDcSplit; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
@@ -666,7 +656,7 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
     const void* kern = dtype == FSA_DTYPE_BF16 ? (const void*)decode_select_kernel<__nv_bfloat16> : (const void*)decode_select_kernel<__half>;
     if (smem > 48 * 1024 && allow_smem(kern, (int)smem) != cudaSuccess) return FSA_ERR_CUDA;
     const unsigned grid = (unsigned)(batch * num_kv_heads);
-    if (dtype == FSA_DTYPE_BF16) launch_pdl(decode_select_kernel<__nv_bfloat16>, grid, 256, smem, (cudaStream_t)stream, p);
-    else launch_pdl(decode_select_kernel<__half>, grid, 256, smem, (cudaStream_t)stream, p);
+    if (dtype == FSA_DTYPE_BF16) decode_select_kernel<__nv_bfloat16><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
+    else decode_select_kernel<__half><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }

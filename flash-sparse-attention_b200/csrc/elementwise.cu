@@ -14,8 +14,6 @@ template <typename ET>
 __global__ void __launch_bounds__(256) rope_kernel(const ET* __restrict__ x, int64_t x_sn, int64_t x_sh, const ET* __restrict__ cs,
                                                    const ET* __restrict__ sn, const int* __restrict__ cu, int B, int64_t N, int H,
                                                    int D, int conj, ET* __restrict__ out) {
-    pdl_trigger();
-    pdl_wait();
     const int half = D / 2, vec = half / 8;           // 16-byte vectors per half row
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= N * H * vec) return;
@@ -55,8 +53,6 @@ template <typename ET>
 __global__ void __launch_bounds__(256) gate_mix_fwd_kernel(const ET* __restrict__ g, const ET* __restrict__ a,
                                                            const ET* __restrict__ b, const ET* __restrict__ c, int64_t N, int HD,
                                                            ET* __restrict__ out) {
-    pdl_trigger();
-    pdl_wait();
     const int vec = HD / 8;
     const int64_t total = N * vec;
     const int64_t base = (int64_t)blockIdx.x * (blockDim.x * 2) + threadIdx.x;
@@ -96,8 +92,6 @@ __global__ void __launch_bounds__(256) gate_mix_bwd_kernel(const ET* __restrict_
                                                            const ET* __restrict__ b, const ET* __restrict__ c,
                                                            const ET* __restrict__ d_o, int64_t N, int HD, ET* __restrict__ da,
                                                            ET* __restrict__ db, ET* __restrict__ dc, float* __restrict__ dg) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (n >= N) return;
@@ -176,8 +170,6 @@ __global__ void __launch_bounds__(256) gate_proj_mix_fwd_kernel(const ET* __rest
                                                                 const ET* __restrict__ a, const ET* __restrict__ b,
                                                                 const ET* __restrict__ c, int64_t N, int hidden, int HD,
                                                                 ET* __restrict__ out, ET* __restrict__ gate) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ __align__(16) uint8_t gsm[];
     uint4* sw = reinterpret_cast<uint4*>(gsm);                 // [3][hidden / 8]
     const int hv = hidden / 8, vec = HD / 8;
@@ -241,8 +233,6 @@ __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __rest
                                                                 int hidden, int HD, ET* __restrict__ da, ET* __restrict__ db,
                                                                 ET* __restrict__ dc, ET* __restrict__ dx, float* __restrict__ dz,
                                                                 float* __restrict__ delta) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ __align__(16) uint8_t gsm[];
     uint4* sw = reinterpret_cast<uint4*>(gsm);
     const int hv = hidden / 8, vec = HD / 8;
@@ -337,8 +327,6 @@ __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __rest
 template <typename ET>
 __global__ void __launch_bounds__(256) gate_dw_partial_kernel(const ET* __restrict__ x, int64_t x_sn, const float* __restrict__ dz,
                                                               int64_t N, int hidden, int chunk_tokens, float* __restrict__ partial) {
-    pdl_trigger();
-    pdl_wait();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;         // 16-byte column vector
     if (v >= hidden / 8) return;
     const int64_t n0 = (int64_t)blockIdx.y * chunk_tokens, n1 = n0 + chunk_tokens < N ? n0 + chunk_tokens : N;
@@ -370,8 +358,6 @@ __global__ void __launch_bounds__(256) gate_dw_partial_kernel(const ET* __restri
 // the chunks' partial sums added in chunk order (deterministic) and rounded
 template <typename ET>
 __global__ void __launch_bounds__(256) gate_dw_reduce_kernel(const float* __restrict__ partial, int chunks, int hidden, ET* __restrict__ dwg) {
-    pdl_trigger();
-    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 3 * hidden) return;
     float s = 0.f;
@@ -391,7 +377,7 @@ static int run_gate_fwd(const void* x, int64_t x_sn, const void* wg, const void*
     const int warps = N <= 148 * 8 ? 4 : 8;
     const int64_t want = (N + warps - 1) / warps;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
-    launch_pdl(kern, grid, warps * 32, smem, stream, (const ET*)x, x_sn, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, N, hidden, HD,
+    kern<<<grid, warps * 32, smem, stream>>>((const ET*)x, x_sn, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, N, hidden, HD,
                                       (ET*)out, (ET*)gate);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
@@ -405,13 +391,13 @@ static int run_gate_bwd(const void* x, int64_t x_sn, const void* wg, const void*
     if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
     const int64_t want = (N + 7) / 8;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
-    launch_pdl(kern, grid, 256, smem, stream, (const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,
+    kern<<<grid, 256, smem, stream>>>((const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,
                                       HD, (ET*)da, (ET*)db, (ET*)dc, (ET*)dx, dz, delta);
     const int chunk_tokens = (int)((N + kGateChunks - 1) / kGateChunks);
     const int chunks = (int)((N + chunk_tokens - 1) / chunk_tokens);
-    launch_pdl(gate_dw_partial_kernel<ET>, dim3((unsigned)((hidden / 8 + 255) / 256), (unsigned)chunks), 256, 0, stream, (const ET*)x, x_sn, dz, N, hidden,
+    gate_dw_partial_kernel<ET><<<dim3((unsigned)((hidden / 8 + 255) / 256), (unsigned)chunks), 256, 0, stream>>>((const ET*)x, x_sn, dz, N, hidden,
                                                                                                           chunk_tokens, partial);
-    launch_pdl(gate_dw_reduce_kernel<ET>, (unsigned)((3 * hidden + 255) / 256), 256, 0, stream, partial, chunks, hidden, (ET*)dwg);
+    gate_dw_reduce_kernel<ET><<<(unsigned)((3 * hidden + 255) / 256), 256, 0, stream>>>(partial, chunks, hidden, (ET*)dwg);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
@@ -429,11 +415,11 @@ extern "C" int fsa_rope(const void* x, int64_t x_sn, int64_t x_sh, const void* c
     int64_t threads = total * heads * (head_dim / 16);
     unsigned grid = (unsigned)((threads + 255) / 256);
     if (dtype == FSA_DTYPE_BF16)
-        launch_pdl(rope_kernel<__nv_bfloat16>, grid, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, x_sn, x_sh, (const __nv_bfloat16*)cos_tab,
+        rope_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, x_sn, x_sh, (const __nv_bfloat16*)cos_tab,
                                                                            (const __nv_bfloat16*)sin_tab, cu_seqlens, batch, total, heads,
                                                                            head_dim, conj, (__nv_bfloat16*)out);
     else if (dtype == FSA_DTYPE_FP16)
-        launch_pdl(rope_kernel<__half>, grid, 256, 0, (cudaStream_t)stream, (const __half*)x, x_sn, x_sh, (const __half*)cos_tab, (const __half*)sin_tab,
+        rope_kernel<__half><<<grid, 256, 0, (cudaStream_t)stream>>>((const __half*)x, x_sn, x_sh, (const __half*)cos_tab, (const __half*)sin_tab,
                                                                     cu_seqlens, batch, total, heads, head_dim, conj, (__half*)out);
     else
         return FSA_ERR_BAD_ARG;
@@ -448,11 +434,11 @@ extern "C" int fsa_gate_mix_fwd(const void* gate, const void* a, const void* b, 
     int64_t threads = total * (row_elems / 8);
     unsigned grid = (unsigned)((threads + 511) / 512);   // two vectors per thread
     if (dtype == FSA_DTYPE_BF16)
-        launch_pdl(gate_mix_fwd_kernel<__nv_bfloat16>, grid, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)a,
+        gate_mix_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate, (const __nv_bfloat16*)a,
                                                                                    (const __nv_bfloat16*)b, (const __nv_bfloat16*)c, total,
                                                                                    row_elems, (__nv_bfloat16*)out);
     else if (dtype == FSA_DTYPE_FP16)
-        launch_pdl(gate_mix_fwd_kernel<__half>, grid, 256, 0, (cudaStream_t)stream, (const __half*)gate, (const __half*)a, (const __half*)b,
+        gate_mix_fwd_kernel<__half><<<grid, 256, 0, (cudaStream_t)stream>>>((const __half*)gate, (const __half*)a, (const __half*)b,
                                                                             (const __half*)c, total, row_elems, (__half*)out);
     else
         return FSA_ERR_BAD_ARG;
@@ -466,11 +452,11 @@ extern "C" int fsa_gate_mix_bwd(const void* gate, const void* a, const void* b, 
     (void)cudaGetLastError();
     unsigned grid = (unsigned)((total + 7) / 8);
     if (dtype == FSA_DTYPE_BF16)
-        launch_pdl(gate_mix_bwd_kernel<__nv_bfloat16>, grid, 256, 0, (cudaStream_t)stream, 
+        gate_mix_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>(
             (const __nv_bfloat16*)gate, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (const __nv_bfloat16*)c,
             (const __nv_bfloat16*)d_out, total, row_elems, (__nv_bfloat16*)da, (__nv_bfloat16*)db, (__nv_bfloat16*)dc, dgate);
     else if (dtype == FSA_DTYPE_FP16)
-        launch_pdl(gate_mix_bwd_kernel<__half>, grid, 256, 0, (cudaStream_t)stream, (const __half*)gate, (const __half*)a, (const __half*)b,
+        gate_mix_bwd_kernel<__half><<<grid, 256, 0, (cudaStream_t)stream>>>((const __half*)gate, (const __half*)a, (const __half*)b,
                                                                             (const __half*)c, (const __half*)d_out, total, row_elems,
                                                                             (__half*)da, (__half*)db, (__half*)dc, dgate);
     else

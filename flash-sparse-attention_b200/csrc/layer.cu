@@ -11,8 +11,6 @@ namespace fsa {
 template <typename ET>
 __global__ void __launch_bounds__(256) layer_prep_kernel(const int* __restrict__ cu, int B, int64_t len, const float* __restrict__ inv_freq, int half,
                                                          int ks, int stride, ET* __restrict__ cs, ET* __restrict__ sn, int* __restrict__ cu_cmp) {
-    pdl_trigger();
-    pdl_wait();
     const int64_t total = len * half;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t pos = i / half;
@@ -92,8 +90,6 @@ struct LayerRopeParams {
 // stride, so the same tables serve them), then of v (backward: sums only).
 template <bool BWD, typename ET>
 __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p) {
-    pdl_trigger();
-    pdl_wait();
     const int half = p.D / 2, vec = half / 8;
     const int64_t nq = p.N * p.Hq * vec, nk = p.N * p.Hk * vec, nc = p.Nc * p.Hk * vec;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,8 +153,6 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
 // gradient of the compressor's bias, finished by its consumer.
 template <int D, typename ET>
 __global__ void __launch_bounds__(256) column_sum_kernel(const ET* __restrict__ dy, int64_t rows, int H, float* __restrict__ out) {
-    pdl_trigger();
-    pdl_wait();
     constexpr int CG = D / 8, KL = 256 / CG;
     __shared__ float red[8][D];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cgi = tid % CG, kl = tid / CG, h = blockIdx.x;
@@ -194,10 +188,10 @@ extern "C" int fsa_layer_prep(const int32_t* cu_seqlens, int batch, int64_t max_
     const int64_t want = (max_len * (head_dim / 2) + 255) / 256;
     const unsigned grid = (unsigned)(want < 1 ? 1 : want > 148 * 8 ? 148 * 8 : want);
     if (dtype == FSA_DTYPE_BF16)
-        launch_pdl(layer_prep_kernel<__nv_bfloat16>, grid, 256, 0, (cudaStream_t)stream, cu_seqlens, batch, max_len, inv_freq, head_dim / 2, kernel_size,
+        layer_prep_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>(cu_seqlens, batch, max_len, inv_freq, head_dim / 2, kernel_size,
                                                                                 kernel_stride, (__nv_bfloat16*)cos_tab, (__nv_bfloat16*)sin_tab, cu_cmp);
     else
-        launch_pdl(layer_prep_kernel<__half>, grid, 256, 0, (cudaStream_t)stream, cu_seqlens, batch, max_len, inv_freq, head_dim / 2, kernel_size, kernel_stride,
+        layer_prep_kernel<__half><<<grid, 256, 0, (cudaStream_t)stream>>>(cu_seqlens, batch, max_len, inv_freq, head_dim / 2, kernel_size, kernel_stride,
                                                                          (__half*)cos_tab, (__half*)sin_tab, cu_cmp);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
@@ -211,8 +205,8 @@ static int run_rope(const LayerRopeParams& p, int dtype, cudaStream_t stream) {
     if (threads == 0) return FSA_OK;
     (void)cudaGetLastError();
     const unsigned grid = (unsigned)((threads + 255) / 256);
-    if (dtype == FSA_DTYPE_BF16) launch_pdl(layer_rope_kernel<BWD, __nv_bfloat16>, grid, 256, 0, stream, p);
-    else launch_pdl(layer_rope_kernel<BWD, __half>, grid, 256, 0, stream, p);
+    if (dtype == FSA_DTYPE_BF16) layer_rope_kernel<BWD, __nv_bfloat16><<<grid, 256, 0, stream>>>(p);
+    else layer_rope_kernel<BWD, __half><<<grid, 256, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
@@ -247,11 +241,11 @@ namespace fsa {
 cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, cudaStream_t stream) {
     const dim3 grid((unsigned)H, (unsigned)parts);
     if (dtype == FSA_DTYPE_BF16) {
-        if (D == 128) launch_pdl(column_sum_kernel<128, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)dy, rows, H, out);
-        else launch_pdl(column_sum_kernel<64, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)dy, rows, H, out);
+        if (D == 128) column_sum_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out);
+        else column_sum_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out);
     } else {
-        if (D == 128) launch_pdl(column_sum_kernel<128, __half>, grid, 256, 0, stream, (const __half*)dy, rows, H, out);
-        else launch_pdl(column_sum_kernel<64, __half>, grid, 256, 0, stream, (const __half*)dy, rows, H, out);
+        if (D == 128) column_sum_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out);
+        else column_sum_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out);
     }
     return cudaGetLastError();
 }

@@ -88,8 +88,6 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const int quarter = warp & 3, r = quarter * 32 + lane;           // (epilogue warps) this thread's window
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     bool ok = true;
@@ -220,8 +218,6 @@ constexpr int kPeParts = 16;
 
 template <int D, typename ET>
 __global__ void __launch_bounds__(256) compress_bias_kernel(const ET* __restrict__ pe, const ET* __restrict__ w, int rows, float* __restrict__ part) {
-    pdl_trigger();
-    pdl_wait();
     constexpr int CG = D / 8, KL = 256 / CG;
     __shared__ float red[8][D];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, cgi = tid % CG, kl = tid / CG;
@@ -270,13 +266,11 @@ static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, i
     cfg.blockDim = dim3(192);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, maps, p);
 }
 
@@ -377,11 +371,11 @@ extern "C" int fsa_compress_kv_fwd(const void* k, int64_t k_stride_n, const void
         const dim3 grid(kPeParts, (unsigned)num_heads);
         const int rows = kernel_size * head_dim;
         if (dtype == FSA_DTYPE_BF16) {
-            if (head_dim == 128) launch_pdl(compress_bias_kernel<128, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
-            else launch_pdl(compress_bias_kernel<64, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
+            if (head_dim == 128) compress_bias_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
+            else compress_bias_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
         } else {
-            if (head_dim == 128) launch_pdl(compress_bias_kernel<128, __half>, grid, 256, 0, stream, (const __half*)pe, (const __half*)w_key, rows, scratch);
-            else launch_pdl(compress_bias_kernel<64, __half>, grid, 256, 0, stream, (const __half*)pe, (const __half*)w_key, rows, scratch);
+            if (head_dim == 128) compress_bias_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch);
+            else compress_bias_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch);
         }
         if (cudaGetLastError() != cudaSuccess) return FSA_ERR_CUDA;
     }

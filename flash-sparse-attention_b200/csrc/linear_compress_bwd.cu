@@ -81,8 +81,6 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     if (warp == 0) {
         // ---- producer: (dy shifted by j, W slice of offset p + j * stride), 64 reduction columns per stage
         bool ok = true;
@@ -180,7 +178,7 @@ static cudaError_t launch_dx(const LcDxMaps& maps, const LcDxParams& p, int nt, 
     auto kern = linear_compress_dx_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    launch_pdl(kern, dim3((unsigned)p.tile0[p.n_seq], (unsigned)(p.H * nt), (unsigned)(p.stride / p.phases)), 192, smem, stream, maps, p);
+    kern<<<dim3((unsigned)p.tile0[p.n_seq], (unsigned)(p.H * nt), (unsigned)(p.stride / p.phases)), 192, smem, stream>>>(maps, p);
     return cudaGetLastError();
 }
 
@@ -234,8 +232,6 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     // tiles of 128 windows over all sequences
     int nitems = 0;
     for (int b = 0; b < p.batch; ++b) {
@@ -381,7 +377,7 @@ static cudaError_t launch_dw(const LcDwParams<ET>& p, int nt, cudaStream_t strea
     auto kern = linear_compress_dw_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    launch_pdl(kern, dim3((unsigned)(p.ks / (128 / D)), (unsigned)p.H, (unsigned)nt), 256, smem, stream, p);
+    kern<<<dim3((unsigned)(p.ks / (128 / D)), (unsigned)p.H, (unsigned)nt), 256, smem, stream>>>(p);
     return cudaGetLastError();
 }
 

@@ -39,8 +39,6 @@ constexpr int kRkTile = kTileRows * 128 * 2;
 // monotone, so every token is looked at: 8 loads in flight per thread, 2 x 128 KB of L2 reads at 32768 tokens).  The last CTA
 // zeroes the rows of dk and dv past the last sequence and the status word.
 __global__ void __launch_bounds__(512) range_key_tiles(const RangeKvPlan p, uint4* __restrict__ dk, uint4* __restrict__ dv, int* __restrict__ status) {
-    pdl_trigger();
-    pdl_wait();
     __shared__ int s_lo[16], s_hi[16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (blockIdx.x == gridDim.x - 1) {
@@ -87,8 +85,6 @@ __global__ void __launch_bounds__(512) range_key_tiles(const RangeKvPlan p, uint
 // smallest length that leaves about kRkItems items (times heads), and at least kRkMinTiles: below that an item's epilogue weighs
 // more than an idle SM.
 __global__ void __launch_bounds__(1024) range_plan_items(const RangeKvPlan p) {
-    pdl_trigger();
-    pdl_wait();
     __shared__ int wa[32], wb[32], wc[32];
     __shared__ long long total;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -136,8 +132,6 @@ __global__ void __launch_bounds__(1024) range_plan_items(const RangeKvPlan p) {
 // dk / dv rows of the K/V tiles that were cut: the sum of the slabs in order.  Slab: [dV, dK][column / 4][row] float4.
 template <typename ET>
 __global__ void __launch_bounds__(256) range_dkdv_reduce(const RangeKvPlan p, const float4* __restrict__ slabs, ET* __restrict__ dk, ET* __restrict__ dv) {
-    pdl_trigger();
-    pdl_wait();
     const int64_t units = (int64_t)__ldg(p.counts + 1) * p.Hk * 16;       // 2 x 16 x 128 chunks of 8 columns per tile and head, 256 a CTA
     for (int64_t w = blockIdx.x; w < units; w += gridDim.x) {
         const int part = (int)(w & 15), h = (int)((w >> 4) % p.Hk);
@@ -252,8 +246,6 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const int nitems = __ldg(p.plan.counts) * p.plan.Hk;
     const int TPT = p.plan.TPT;
 
@@ -522,8 +514,8 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
 }
 
 cudaError_t launch_range_bwd_plan(const RangeKvPlan& p, const SelBwdArgs& a, int* status, cudaStream_t stream) {
-    launch_pdl(range_key_tiles, (unsigned)p.max_tiles + 1, 512, 0, stream, p, (uint4*)a.dk, (uint4*)a.dv, status);
-    launch_pdl(range_plan_items, 1, 1024, 0, stream, p);
+    range_key_tiles<<<(unsigned)p.max_tiles + 1, 512, 0, stream>>>(p, (uint4*)a.dk, (uint4*)a.dv, status);
+    range_plan_items<<<1, 1024, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
@@ -535,9 +527,9 @@ static cudaError_t launch_rk(const RangeKvParams& p, const CUtensorMap& qmap, co
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(FSA_KERNEL_SEL_BWD_MAIN, stream);
-    launch_pdl(kern, (unsigned)(max_items < sms ? max_items : sms), kRkThreads, smem, stream, p, qmap, domap, kmap, vmap);
+    kern<<<(unsigned)(max_items < sms ? max_items : sms), kRkThreads, smem, stream>>>(p, qmap, domap, kmap, vmap);
     prof_end(FSA_KERNEL_SEL_BWD_MAIN, stream);
-    launch_pdl(range_dkdv_reduce<ET>, (unsigned)(4 * sms), 256, 0, stream, p.plan, (const float4*)p.slabs, (ET*)p.dk, (ET*)p.dv);
+    range_dkdv_reduce<ET><<<(unsigned)(4 * sms), 256, 0, stream>>>(p.plan, (const float4*)p.slabs, (ET*)p.dk, (ET*)p.dv);
     return cudaGetLastError();
 }
 

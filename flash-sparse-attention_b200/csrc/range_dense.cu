@@ -97,7 +97,6 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
         tma_prefetch_desc(&vmap);
         tma_prefetch_desc(&omap);
     }
-    pdl_wait();
     if (warp == 0) {
         // which tile is this: the heaviest (last) tiles of the list start first
         const int total = count_seq_tiles(p.cu_q, p.B, p.TPT, lane);
@@ -130,7 +129,6 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
     const int seq = s_meta[0], tok0 = s_meta[1], ne = s_meta[2], row_lo = s_meta[3], nblk = s_meta[4];
 
     if (seq >= 0) {
@@ -356,7 +354,7 @@ static cudaError_t launch_rd(const RangeDenseParams& p, const CUtensorMap& qmap,
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(FSA_KERNEL_RANGE_DENSE, stream);
-    launch_pdl(kern, dim3((unsigned)max_tiles, (unsigned)p.Hk), kRdThreads, smem, stream, p, qmap, kmap, vmap, omap);
+    kern<<<dim3((unsigned)max_tiles, (unsigned)p.Hk), kRdThreads, smem, stream>>>(p, qmap, kmap, vmap, omap);
     prof_end(FSA_KERNEL_RANGE_DENSE, stream);
     return cudaGetLastError();
 }
@@ -475,8 +473,6 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const int ntiles = count_seq_tiles(p.cu_q, p.B, p.TPT, lane);
     const int nitems = ntiles * p.Hk;
 
@@ -728,14 +724,14 @@ cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& 
         e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         prof_begin(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
-        launch_pdl(kern, grid, kDqThreads, smem, stream, p, qmap, domap, kmap, vmap, dqmap);
+        kern<<<grid, kDqThreads, smem, stream>>>(p, qmap, domap, kmap, vmap, dqmap);
         prof_end(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
     } else {
         auto kern = range_bwd_dq_dense<__half>;
         e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         prof_begin(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
-        launch_pdl(kern, grid, kDqThreads, smem, stream, p, qmap, domap, kmap, vmap, dqmap);
+        kern<<<grid, kDqThreads, smem, stream>>>(p, qmap, domap, kmap, vmap, dqmap);
         prof_end(FSA_KERNEL_SEL_BWD_DQ_REDUCE, stream);
     }
     return cudaGetLastError();

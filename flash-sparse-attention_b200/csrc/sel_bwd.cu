@@ -93,8 +93,6 @@ __global__ void __launch_bounds__(128, 1) sel_bwd_main(const SelBwdParams<ET> p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
 
     const int total = p.ix.header[1] * p.nsub;
@@ -343,8 +341,6 @@ template <typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_delta(const ET* __restrict__ o, int64_t o_sn, int64_t o_sh,
                                                      const ET* __restrict__ d_o, int64_t do_sn, int64_t do_sh,
                                                      int64_t N, int Hq, int D, float* __restrict__ delta) {
-    pdl_trigger();
-    pdl_wait();
     const int tpr = D >> 3;                                  // threads per row: 8, 16 or 32 (a power of two)
     const int rpc = 256 / tpr;                               // rows per pass of the CTA
     const int part = threadIdx.x & (tpr - 1), rloc = threadIdx.x / tpr;
@@ -389,8 +385,6 @@ __global__ void __launch_bounds__(256) sel_bwd_delta(const ET* __restrict__ o, i
 template <int D, typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ dq_part, const int* __restrict__ pos, SelShape s,
                                                          int nsub, ET* __restrict__ dq) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= s.N * s.Hq) return;
@@ -453,8 +447,6 @@ __global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ 
 template <int D, typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s,
                                                            SelIndex ix, int nsub, ET* __restrict__ dk, ET* __restrict__ dv) {
-    pdl_trigger();
-    pdl_wait();
     constexpr int KT = 64, RV = D / 4;                // keys of a slab, float4 per row
     constexpr int kShares = 2 * KT * RV / 1024;       // CTAs per slab: 1024 float4 each, four per thread in flight
     const int hg = blockIdx.x;
@@ -506,8 +498,6 @@ __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restri
 template <typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_convert(const float* __restrict__ a, const float* __restrict__ b,
                                                        ET* __restrict__ oa, ET* __restrict__ ob, int64_t n4) {
-    pdl_trigger();
-    pdl_wait();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
     float4 x = reinterpret_cast<const float4*>(a)[i];
@@ -541,7 +531,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     if (rows > 0 && !a.have_delta) {
         const int64_t rows_per_cta = 2 * (256 / (D / 8));
         unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
-        launch_pdl(sel_bwd_delta<ET>, grid, 256, 0, stream, (const ET*)a.o, a.o_sn, a.o_sh, (const ET*)a.d_o, a.do_sn, a.do_sh,
+        sel_bwd_delta<ET><<<grid, 256, 0, stream>>>((const ET*)a.o, a.o_sn, a.o_sh, (const ET*)a.d_o, a.do_sn, a.do_sh,
                                                     s.N, s.Hq, D, a.delta);
     }
     if (a.plan) {
@@ -569,7 +559,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         if (by_smem < per_sm) per_sm = by_smem;
         if (per_sm < 1) per_sm = 1;
         prof_begin(2, stream);
-        launch_pdl(kern, num_sms * per_sm, 128, smem, stream, p, kmap, vmap);
+        kern<<<num_sms * per_sm, 128, smem, stream>>>(p, kmap, vmap);
         prof_end(2, stream);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -577,16 +567,16 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
         prof_begin(3, stream);
-        launch_pdl(sel_bwd_dq_reduce<D, ET>, grid, 256, 0, stream, (const ET*)a.dq_part, ix.pos, s, nsub, (ET*)a.dq);
+        sel_bwd_dq_reduce<D, ET><<<grid, 256, 0, stream>>>((const ET*)a.dq_part, ix.pos, s, nsub, (ET*)a.dq);
         prof_end(3, stream);
     }
     if (kv_elems > 0) {
         if (pipelined) {
-            launch_pdl(sel_bwd_dkdv_reduce<D, ET>, dim3((unsigned)(s.Hk * s.NBmax + 1), (unsigned)(nsub * (2 * kKT * (D / 4) / 1024))), 256, 0, stream, 
+            sel_bwd_dkdv_reduce<D, ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), (unsigned)(nsub * (2 * kKT * (D / 4) / 1024))), 256, 0, stream>>>(
                 a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix, nsub, (ET*)a.dk, (ET*)a.dv);
         } else {
             int64_t n4 = kv_elems / 4;
-            launch_pdl(sel_bwd_convert<ET>, (unsigned)((n4 + 255) / 256), 256, 0, stream, a.dk_acc, a.dv_acc, (ET*)a.dk, (ET*)a.dv, n4);
+            sel_bwd_convert<ET><<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(a.dk_acc, a.dv_acc, (ET*)a.dk, (ET*)a.dv, n4);
         }
     }
     return cudaGetLastError();

@@ -150,8 +150,6 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const TileScheduleT<PARTS> sched(p.ix.header[1], p.run, p.nsub);
     const int nsub = PARTS ? p.nsub : 1;
     const int nloc = sched.nloc;
@@ -640,7 +638,7 @@ static cudaError_t launch_pipe(const SelBwdArgs& a, const SelShape& s, const Sel
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(2, stream);
-    launch_pdl(kern, num_sms, bwdpipe::kThreads, smem, stream, p, kmap, vmap, dqmap);
+    kern<<<num_sms, bwdpipe::kThreads, smem, stream>>>(p, kmap, vmap, dqmap);
     prof_end(2, stream);
     return cudaGetLastError();
 }

@@ -112,8 +112,6 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const TileScheduleT<true> sched(p.ix.header[1], p.run, p.nsub);
     const int nloc = sched.nloc;
     const int key_lim = min(KT, s.BK);
@@ -465,7 +463,7 @@ static cudaError_t launch_wide(const SelBwdArgs& a, const SelShape& s, const Sel
     cudaError_t e = allow_smem((const void*)kern, bwdwide::kBytes);
     if (e != cudaSuccess) return e;
     prof_begin(2, stream);
-    launch_pdl(kern, num_sms, bwdwide::kThreads, bwdwide::kBytes, stream, p, kmap, vmap, dqmap);
+    kern<<<num_sms, bwdwide::kThreads, bwdwide::kBytes, stream>>>(p, kmap, vmap, dqmap);
     prof_end(2, stream);
     return cudaGetLastError();
 }

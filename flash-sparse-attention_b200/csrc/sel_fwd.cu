@@ -154,8 +154,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();      // (not before the TMEM columns are held: a waiting kernel's CTA could take them)
-    pdl_wait();
 
     const TileSchedule sched(p.ix.header[1], p.run);
     const int nloc = sched.nloc;
@@ -654,8 +652,6 @@ __global__ void __launch_bounds__(128, 1) sel_fwd_simple(const SelFwdParams<ET> 
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
-    pdl_wait();
     const uint32_t tS = tbase, tO = tbase + BK;
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     const int total = p.ix.header[1];
@@ -798,8 +794,6 @@ template <int D, typename ET>
 __global__ void __launch_bounds__(256) sel_fwd_reduce(const ET* __restrict__ opart, const float2* __restrict__ ml,
                                                       const int* __restrict__ pos, SelShape s, ET* __restrict__ o,
                                                       int64_t o_sn, int64_t o_sh, float* __restrict__ lse) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // n * Hq + hq
     if (row >= s.N * s.Hq) return;
@@ -931,7 +925,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
             e = allow_smem((const void*)kern, smem);
             if (e != cudaSuccess) return e;
             prof_begin(0, stream);
-            launch_pdl(kern, num_sms, kFwdThreads, smem, stream, p, (const ET*)a.q, a.q_sn, a.q_sh, *a.kmap, *a.vmap, *a.omap);
+            kern<<<num_sms, kFwdThreads, smem, stream>>>(p, (const ET*)a.q, a.q_sn, a.q_sh, *a.kmap, *a.vmap, *a.omap);
             prof_end(0, stream);
         }
     } else {
@@ -945,7 +939,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
         if (by_smem < per_sm) per_sm = by_smem;
         if (per_sm < 1) per_sm = 1;
         prof_begin(0, stream);
-        launch_pdl(kern, num_sms * per_sm, 128, smem, stream, p, (const ET*)a.q, a.q_sn, a.q_sh, *a.kmap, *a.vmap);
+        kern<<<num_sms * per_sm, 128, smem, stream>>>(p, (const ET*)a.q, a.q_sn, a.q_sh, *a.kmap, *a.vmap);
         prof_end(0, stream);
     }
     e = cudaGetLastError();
@@ -954,7 +948,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
         prof_begin(1, stream);
-        launch_pdl(sel_fwd_reduce<D, ET>, grid, 256, 0, stream, (const ET*)a.opart, a.ml, ix.pos, s, (ET*)a.o, a.o_sn, a.o_sh, a.lse);
+        sel_fwd_reduce<D, ET><<<grid, 256, 0, stream>>>((const ET*)a.opart, a.ml, ix.pos, s, (ET*)a.o, a.o_sn, a.o_sh, a.lse);
         prof_end(1, stream);
     }
     return cudaGetLastError();

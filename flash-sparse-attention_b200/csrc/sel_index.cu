@@ -108,8 +108,6 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
 template <bool FILL>
 __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* __restrict__ topk_idx, const int* __restrict__ cu,
                                                                      SelBounds bd, SelShape s, SelIndex ix) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ int sm[];   // [nwarps][NBmax]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int c = blockIdx.x, h = blockIdx.y;
@@ -145,8 +143,6 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
 
 // Step 2: per key, exclusive prefix of the chunks' counts and the total (thread per key; eight loads in flight).
 __global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
-    pdl_trigger();
-    pdl_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= s.Hk * s.NBmax) return;
     const int h = k / s.NBmax, gb = k - h * s.NBmax;
@@ -168,8 +164,6 @@ __global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
 // Step 3: exclusive scans over the keys (a single CTA): first tile, then -- it depends on the first tile -- first segment.
 // A key with tiles [t0, t0 + nt) is cut by the backward's schedule at every multiple of RB.
 __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) {
-    pdl_trigger();
-    pdl_wait();
     __shared__ int wsum_a[32], wsum_b[32], wsum_c[32];
     __shared__ int carry_a, carry_b, carry_c;
     const int HG = s.Hk * s.NBmax;
@@ -247,8 +241,6 @@ __device__ __forceinline__ void write_tiles(const SelShape& s, const SelIndex& i
 
 // Step 4: tile records and the padding of the tile-ordered entry list: one warp per key.
 __global__ void __launch_bounds__(256) sel_index_tiles(const int* __restrict__ cu, SelBounds bd, SelShape s, SelIndex ix) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int hg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (hg >= s.Hk * s.NBmax) return;
@@ -287,8 +279,6 @@ __device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total)
 
 __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* __restrict__ topk_idx, const int* __restrict__ cu, SelBounds bd,
                                                                   SelShape s, SelIndex ix) {
-    pdl_trigger();
-    pdl_wait();
     namespace cg = cooperative_groups;
     extern __shared__ int sm[];   // [warps][NBmax] counts, then positions; [NBmax] entries, [NBmax] first tile, [NBmax] first segment of a key
     __shared__ int wsum[32], mine[3];       // tiles, entries, segments of this head
@@ -374,13 +364,11 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
         cfg.blockDim = dim3(kSmallWarps * 32);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)s.Hk; at[0].val.clusterDim.z = 1;
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 2;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1; at.val.clusterDim.y = (unsigned)s.Hk; at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, sel_index_small, topk_idx, cu, bd, s, ix);
     }
     const int nw = s.IW;
@@ -392,11 +380,11 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)s.NC, (unsigned)s.Hk);
     const int HG = s.Hk * s.NBmax;
-    launch_pdl(sel_index_chunk<false>, grid, nw * 32, smem, stream, topk_idx, cu, bd, s, ix);
-    launch_pdl(sel_index_keys, (unsigned)((HG + 63) / 64), 64, 0, stream, s, ix);
-    launch_pdl(sel_index_scan, 1, 1024, 0, stream, s, ix);
-    launch_pdl(sel_index_tiles, (unsigned)((HG + 7) / 8), 256, 0, stream, cu, bd, s, ix);
-    launch_pdl(sel_index_chunk<true>, grid, nw * 32, smem, stream, topk_idx, cu, bd, s, ix);
+    sel_index_chunk<false><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
+    sel_index_keys<<<(unsigned)((HG + 63) / 64), 64, 0, stream>>>(s, ix);
+    sel_index_scan<<<1, 1024, 0, stream>>>(s, ix);
+    sel_index_tiles<<<(unsigned)((HG + 7) / 8), 256, 0, stream>>>(cu, bd, s, ix);
+    sel_index_chunk<true><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
     return cudaGetLastError();
 }
 

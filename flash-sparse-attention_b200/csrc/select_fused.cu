@@ -59,7 +59,6 @@ struct TapWeights {
 template <int D, typename ET, int A, int BS, int TL>
 __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedParams p, const __grid_constant__ CUtensorMap qmap,
                                                                const __grid_constant__ CUtensorMap kmap) {
-    pdl_wait();
     constexpr int kQ = kSfRows * D * 2, kK = kSfKeys * D * 2;
     constexpr int PAD = A - 1, NWT = A + BS - 1;
     static_assert(32 % BS == 0, "a group of 32 key columns holds whole blocks");
@@ -98,7 +97,6 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    pdl_trigger();
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
 
     auto load_k = [&](int kt) {
@@ -244,12 +242,12 @@ static cudaError_t launch_tl(const SelFusedParams& p, const CUtensorMap& qmap, c
         auto kern = select_topk_fused_kernel<D, ET, A, BS, 16>;
         e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
-        launch_pdl(kern, grid, 128, smem, stream, p, qmap, kmap);
+        kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
     } else {
         auto kern = select_topk_fused_kernel<D, ET, A, BS, 32>;
         e = allow_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
-        launch_pdl(kern, grid, 128, smem, stream, p, qmap, kmap);
+        kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
     }
     return cudaGetLastError();
 }

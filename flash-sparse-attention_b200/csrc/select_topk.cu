@@ -36,8 +36,6 @@ struct TopkParams {
 };
 
 __global__ void __launch_bounds__(128) select_topk_kernel(const TopkParams p) {
-    pdl_trigger();
-    pdl_wait();
     extern __shared__ float smem_f[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* ps = smem_f + (size_t)warp * (p.smem_p + p.max_blocks + 64);
@@ -146,6 +144,6 @@ extern "C" int fsa_select_topk_seq(const float* qk, int64_t ld, const float* lse
     cudaError_t e = allow_smem((const void*)select_topk_kernel, (int)smem);
     if (e != cudaSuccess) return FSA_ERR_CUDA;
     int64_t warps = (int64_t)num_kv_heads * seq_len;
-    launch_pdl(select_topk_kernel, (unsigned)((warps + 3) / 4), 128, smem, (cudaStream_t)stream_, p);
+    select_topk_kernel<<<(unsigned)((warps + 3) / 4), 128, smem, (cudaStream_t)stream_>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }

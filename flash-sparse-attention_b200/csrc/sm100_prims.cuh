@@ -20,28 +20,6 @@ namespace fsa {
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize), once per thread, device and kernel (the driver call costs about as much
 // as a launch)
 cudaError_t allow_smem(const void* kern, int bytes);
-// Launch with programmatic stream serialization: the kernel may start (barrier and TMEM set-up, descriptor fetches) while the
-// kernel before it drains, and waits in pdl_wait for that one's results.  Every kernel calls pdl_trigger first -- or,
-// if it allocates TMEM, when it holds it: the waiting kernel's CTA could take the columns otherwise -- and pdl_wait before its
-// first access to global memory, reads and writes alike; kernels of a few microseconds in a row otherwise spend a
-// third of their time between launches.  Ordinary neighbours (a copy, a library kernel) are serialized as ever.
-template <typename... KA, typename... A>
-inline cudaError_t launch_pdl(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
-}
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
 int ensure_context();
 
