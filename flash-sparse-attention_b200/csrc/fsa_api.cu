@@ -7,7 +7,9 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <utility>
 
 namespace fsa {
 
@@ -94,9 +96,19 @@ cudaError_t allow_smem(const void* kern, int bytes) {
     if (e != cudaSuccess) return e;
     Seen& c = seen[(((uintptr_t)kern >> 4) ^ ((uintptr_t)kern >> 11)) & 127];      // a collision only costs the call
     if (c.kern == kern && c.dev == dev && c.bytes >= bytes) return cudaSuccess;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) c = Seen{kern, dev, bytes};
-    return e;
+    // the attribute belongs to the kernel, not to the thread: it is only ever raised, or a thread with a smaller size would
+    // take from another one what that one has seen granted
+    static std::mutex mutex;
+    static std::map<std::pair<const void*, int>, int> granted;
+    std::lock_guard<std::mutex> lock(mutex);
+    int& most = granted[{kern, dev}];
+    if (most < bytes) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+        most = bytes;
+    }
+    c = Seen{kern, dev, most};
+    return cudaSuccess;
 }
 
 int device_sm_count(int* out) {
