@@ -111,6 +111,19 @@ cudaError_t allow_smem(const void* kern, int bytes) {
     return cudaSuccess;
 }
 
+cudaError_t prefer_l1(const void* kern) {
+    struct Seen { const void* kern; int dev; };
+    static thread_local Seen seen[128];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    Seen& c = seen[(((uintptr_t)kern >> 4) ^ ((uintptr_t)kern >> 11)) & 127];
+    if (c.kern == kern && c.dev == dev) return cudaSuccess;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+    if (e == cudaSuccess) c = Seen{kern, dev};
+    return e;
+}
+
 int device_sm_count(int* out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);

@@ -11,12 +11,12 @@
 // the sequence's rows of x -- dims (column, window c, offset k), strides (1, stride * row, row): overlapping -- lets TMA
 // fetch the 64-column slab (k, half of d) of 128 consecutive windows straight into a swizzled K-major tile; windows
 // past n_b are out of the map's bounds and read as zero.  One CTA = 128 windows of one sequence x one head of one tensor (K and
-// V in the same launch) x a share of the reduction; a producer warp streams (A slab, W slab) stages through a four-stage
+// V in the same launch) x a share of the reduction; a producer warp streams (A slab, W slab) stages through a six-stage
 // mbarrier ring, one elected thread issues the MMAs (M = 128, N = d, fp32 in TMEM), four warps round the sum to the
 // activation dtype, add the bias and store the rows.
 //
 // The reduction over ks * d is one serial chain of MMAs behind a ring of loads: 26 us at ks * d = 4096 however few windows
-// there are.  When the tiles leave SMs idle the chain is cut in up to eight, one CTA of a cluster each, whose fp32 sums meet
+// there are.  When short sequences leave SMs idle the chain is cut in up to eight, one CTA of a cluster each, whose fp32 sums meet
 // through distributed shared memory (517 tokens, 8 heads, K and V: two launches of 26 us before).  One launch takes up to
 // kLcSeqs sequences, whose tensor maps travel as kernel parameters.
 #include "../../include/fsa_sm100.h"
@@ -30,7 +30,7 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int64_t rows, i
 int make_tile_map_3d(CUtensorMap* map, const void* base, int dtype, int64_t d0, int64_t d1, int64_t d2, int64_t stride1,
                      int64_t stride2, int box1);
 
-constexpr int kLcStages = 4, kLcSeqs = 12, kLcTensors = 2, kLcSplits = 8;
+constexpr int kLcStages = 6, kLcSeqs = 12, kLcTensors = 2, kLcSplits = 8, kLcShort = 64;
 
 struct LcMaps {
     CUtensorMap a[kLcTensors][kLcSeqs];      // overlapping windows of every sequence
@@ -258,9 +258,12 @@ static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, i
     auto kern = linear_compress_fwd_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    // CTAs per tile: as many as still find an SM of their own (the ring takes one SM's shared memory)
-    int S = 1;
-    while (S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= 148) S *= 2;
+    // CTAs per tile: as many as still find an SM of their own (the ring takes one SM's shared memory).  Short sequences only: another
+    // order of the sum moves the last bit of a compressed row, and with it near ties of a block selection where there is
+    // something to select; up to kLcShort windows (about 1000 tokens, 16 blocks of 64) a selection takes about everything.
+    int S = 1, longest = 0;
+    for (int b = 0; b < p.n_seq; ++b) longest = p.n_cmp[b] > longest ? p.n_cmp[b] : longest;
+    while (longest <= kLcShort && S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= 148) S *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)S, (unsigned)tiles, (unsigned)(p.H * nt));
     cfg.blockDim = dim3(192);

@@ -529,6 +529,8 @@ static cudaError_t launch_rk(const RangeKvParams& p, const CUtensorMap& qmap, co
     prof_begin(FSA_KERNEL_SEL_BWD_MAIN, stream);
     kern<<<(unsigned)(max_items < sms ? max_items : sms), kRkThreads, smem, stream>>>(p, qmap, domap, kmap, vmap);
     prof_end(FSA_KERNEL_SEL_BWD_MAIN, stream);
+    e = prefer_l1((const void*)range_dkdv_reduce<ET>);
+    if (e != cudaSuccess) return e;
     range_dkdv_reduce<ET><<<(unsigned)(4 * sms), 256, 0, stream>>>(p.plan, (const float4*)p.slabs, (ET*)p.dk, (ET*)p.dv);
     return cudaGetLastError();
 }

@@ -531,6 +531,8 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     if (rows > 0 && !a.have_delta) {
         const int64_t rows_per_cta = 2 * (256 / (D / 8));
         unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
+        e = prefer_l1((const void*)sel_bwd_delta<ET>);
+        if (e != cudaSuccess) return e;
         sel_bwd_delta<ET><<<grid, 256, 0, stream>>>((const ET*)a.o, a.o_sn, a.o_sh, (const ET*)a.d_o, a.do_sn, a.do_sh,
                                                     s.N, s.Hq, D, a.delta);
     }
@@ -566,12 +568,16 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     }
     if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
+        e = prefer_l1((const void*)sel_bwd_dq_reduce<D, ET>);
+        if (e != cudaSuccess) return e;
         prof_begin(3, stream);
         sel_bwd_dq_reduce<D, ET><<<grid, 256, 0, stream>>>((const ET*)a.dq_part, ix.pos, s, nsub, (ET*)a.dq);
         prof_end(3, stream);
     }
     if (kv_elems > 0) {
         if (pipelined) {
+            e = prefer_l1((const void*)sel_bwd_dkdv_reduce<D, ET>);
+            if (e != cudaSuccess) return e;
             sel_bwd_dkdv_reduce<D, ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), (unsigned)(nsub * (2 * kKT * (D / 4) / 1024))), 256, 0, stream>>>(
                 a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix, nsub, (ET*)a.dk, (ET*)a.dv);
         } else {

@@ -947,6 +947,8 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     int64_t rows = s.N * s.Hq;
     if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
+        e = prefer_l1((const void*)sel_fwd_reduce<D, ET>);
+        if (e != cudaSuccess) return e;
         prof_begin(1, stream);
         sel_fwd_reduce<D, ET><<<grid, 256, 0, stream>>>((const ET*)a.opart, a.ml, ix.pos, s, (ET*)a.o, a.o_sn, a.o_sh, a.lse);
         prof_end(1, stream);

@@ -20,6 +20,11 @@ namespace fsa {
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize), once per thread, device and kernel (the driver call costs about as much
 // as a launch)
 cudaError_t allow_smem(const void* kern, int bytes);
+// Gives a kernel that streams from global memory and has no shared memory to speak of the whole L1 (once per thread, device and
+// kernel).  Without a preference the SMs keep the split of the kernel before, and after one with 227 KB of shared memory the
+// 28 KB that are left hold too few loads in flight: the merges of the partial rows took 467 us instead of 390 us (16K tokens,
+// 32 heads, 16 rows each).
+cudaError_t prefer_l1(const void* kern);
 // Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
 int ensure_context();
 
