@@ -15,7 +15,8 @@
 //   4. tiles   one warp per key: tile records, padding of the last tile;
 //   5. fill    the CTAs of step 1 again: the same counting pass gives every warp its first position inside each key,
 //              a second pass over the same tokens writes entries and positions.
-// Entries of a key are in ascending order of (chunk, warp range, 32-token group, slot): ascending token groups.
+// Entries of a key are in ascending order of (chunk, warp range, 32-token group): ascending token groups, and inside a group
+// ascending tokens (short lists without repeated ids), else slot by slot.
 // Short problems run all steps in one launch (sel_index_small).
 #include <cooperative_groups.h>
 
@@ -28,16 +29,33 @@ constexpr int kIdxMaxSlots = 16;   // top-k lists up to this length are held in 
 
 // Count (FILL = false: hw[gb] += entries) or place (FILL = true: hw[gb] is this warp's next position in the
 // tile-ordered entry list) the entries of this warp's share of the chunk [n0, n1).
+// Bound by the latency of a warp's chain through shared memory.  Counts are shared-memory adds that nothing waits for.  To place
+// a group of 32 tokens, every lane sets its bit in the word mk[gb] of each of its blocks; a token's place among the
+// group's entries of a block is the number of bits below its own, so the slots do not wait for one another: three round trips
+// a group.  (Slot by slot, with __match_any_sync and a running position, took 16 dependent rounds: 89 us for 3661 tokens x 2
+// heads in the one-launch build.)  A list that names a block twice finds the bit set already; its group, long lists,
+// ranges and tables of more keys than have room for mk (null) go slot by slot.
 template <bool FILL>
 __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, const int* __restrict__ cu, const SelBounds& bd,
-                                           const SelShape& s, const SelIndex& ix, int h, int c, int n0, int n1, int* hw, int warp,
-                                           int nwarps, int lane) {
+                                           const SelShape& s, const SelIndex& ix, int h, int c, int n0, int n1, int* hw, unsigned* mk,
+                                           int warp, int nwarps, int lane) {
     const int ngroups = (n1 - n0 + 31) >> 5;
     const int gpw = (ngroups + nwarps - 1) / nwarps;
     const int g_lo = warp * gpw, g_hi = min(ngroups, g_lo + gpw);
     const bool list = bd.kv_hi == nullptr;
-    const bool in_regs = list && s.T <= kIdxMaxSlots && (s.T & 3) == 0 && (reinterpret_cast<uintptr_t>(topk_idx) & 15) == 0;
+    const bool in_regs = list && s.T <= kIdxMaxSlots, by4 = (s.T & 3) == 0 && (reinterpret_cast<uintptr_t>(topk_idx) & 15) == 0;
     const unsigned lt = (1u << lane) - 1;
+    auto store_pos = [&](const int (&ids)[kIdxMaxSlots], int n) {
+        int* prow = ix.pos + ((int64_t)h * s.N + n) * s.T;
+        if (!by4) {
+#pragma unroll
+            for (int j = 0; j < kIdxMaxSlots; ++j)
+                if (j < s.T) prow[j] = ids[j];
+        }
+#pragma unroll
+        for (int i = 0; i < kIdxMaxSlots / 4; ++i)
+            if (by4 && i * 4 < s.T) reinterpret_cast<int4*>(prow)[i] = make_int4(ids[i * 4], ids[i * 4 + 1], ids[i * 4 + 2], ids[i * 4 + 3]);
+    };
     for (int g = g_lo; g < g_hi; ++g) {
         const int n = n0 + g * 32 + lane;
         const bool active = n < n1;
@@ -46,13 +64,56 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
         const int* row = topk_idx + ((int64_t)h * s.N + n) * s.T;
         int ids[kIdxMaxSlots];
         if (in_regs && active) {
-            // the whole list in one round trip (rows are 16-byte aligned: T is a multiple of 4)
+            // the whole list in one round trip (by4: rows are 16-byte aligned)
+            if (!by4) {
+#pragma unroll
+                for (int j = 0; j < kIdxMaxSlots; ++j) ids[j] = j < s.T ? __ldg(row + j) : -1;
+            }
 #pragma unroll
             for (int i = 0; i < kIdxMaxSlots / 4; ++i) {
-                if (i * 4 < s.T) {
+                if (by4 && i * 4 < s.T) {
                     const int4 v = __ldg(reinterpret_cast<const int4*>(row) + i);
                     ids[i * 4] = v.x; ids[i * 4 + 1] = v.y; ids[i * 4 + 2] = v.z; ids[i * 4 + 3] = v.w;
                 }
+            }
+        }
+        if (FILL && in_regs && mk) {
+            int gb[kIdxMaxSlots];
+            unsigned twice = 0;
+#pragma unroll
+            for (int j = 0; j < kIdxMaxSlots; ++j) {
+                int r0;
+                gb[j] = active && j < s.T ? entry_block_ctx(tc, bd, s.BK, n, j, ids[j], &r0) : -1;
+                if (gb[j] >= 0) twice |= atomicOr(&mk[gb[j]], 1u << lane) >> lane & 1u;
+            }
+            __syncwarp();
+            const bool again = __any_sync(0xffffffffu, twice);
+            unsigned leads = 0;                    // slots in which this lane is the first of its block's entries
+#pragma unroll
+            for (int j = 0; j < kIdxMaxSlots; ++j) {
+                const int key = gb[j];
+                if (key >= 0 && !again) {
+                    const unsigned m = mk[key];
+                    const int ps = hw[key] + __popc(m & lt);
+                    if ((m & lt) == 0) leads |= 1u << j;
+                    ix.entries[ps] = ((uint32_t)n << kSlotBits) | (uint32_t)j;
+                    ids[j] = ps;
+                } else if (!again) {
+                    ids[j] = -1;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < kIdxMaxSlots; ++j) {
+                if (again ? gb[j] >= 0 : (leads >> j & 1u) != 0) {
+                    if (!again) hw[gb[j]] += __popc(mk[gb[j]]);
+                    mk[gb[j]] = 0u;
+                }
+            }
+            __syncwarp();
+            if (!again) {
+                if (active) store_pos(ids, n);
+                continue;
             }
         }
 #pragma unroll 1
@@ -68,14 +129,12 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
                     if (FILL) atomicMax(ix.header, (int)kStatusBadIndex);      // cleared between the two passes)
                     gb = -1;
                 }
-                __syncwarp();
-                const unsigned m = __match_any_sync(0xffffffffu, gb);
-                const int leader = __ffs(m) - 1;
                 if (!FILL) {
-                    if (gb >= 0 && lane == leader) {
-                        hw[gb] += __popc(m);
-                    }
+                    if (gb >= 0) atomicAdd(&hw[gb], 1);
                 } else {
+                    __syncwarp();
+                    const unsigned m = __match_any_sync(0xffffffffu, gb);
+                    const int leader = __ffs(m) - 1;
                     int base = 0;
                     if (gb >= 0 && lane == leader) {
                         base = hw[gb];
@@ -91,24 +150,25 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
                         if (in_regs) ids[j] = ps;      // the slot's id is used up: keep its position, written as whole rows below
                         else ix.pos[((int64_t)h * s.N + n) * s.T + sl] = ps;
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
         }
-        if (FILL && in_regs && active) {
-            int4* prow = reinterpret_cast<int4*>(ix.pos + ((int64_t)h * s.N + n) * s.T);
-#pragma unroll
-            for (int i = 0; i < kIdxMaxSlots / 4; ++i)
-                if (i * 4 < s.T) prow[i] = make_int4(ids[i * 4], ids[i * 4 + 1], ids[i * 4 + 2], ids[i * 4 + 3]);
-        }
+        if (FILL && in_regs && active) store_pos(ids, n);
     }
+}
+
+// Is there room for the words of lane bits?
+constexpr int kIdxSmem = 200 * 1024;
+__host__ __device__ __forceinline__ bool sel_index_masks(const SelShape& s, int nwarps) {
+    return (int64_t)nwarps * s.NBmax * 8 <= kIdxSmem && s.T <= kIdxMaxSlots;
 }
 
 // Step 1 (FILL = false) and step 5 (FILL = true).
 template <bool FILL>
 __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* __restrict__ topk_idx, const int* __restrict__ cu,
                                                                      SelBounds bd, SelShape s, SelIndex ix) {
-    extern __shared__ int sm[];   // [nwarps][NBmax]
+    extern __shared__ int sm[];   // [nwarps][NBmax] counts or positions, then, if there is room, [nwarps][NBmax] words of lane bits
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int c = blockIdx.x, h = blockIdx.y;
     const int n0 = (int)min((int64_t)c * s.C, s.N), n1 = (int)min((int64_t)(c + 1) * s.C, s.N);
@@ -117,7 +177,7 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
     if (!FILL) {
         for (int i = tid; i < nwarps * s.NBmax; i += nthreads) sm[i] = 0;
         __syncthreads();
-        chunk_pass<false>(topk_idx, cu, bd, s, ix, h, c, n0, n1, sm + warp * s.NBmax, warp, nwarps, lane);
+        chunk_pass<false>(topk_idx, cu, bd, s, ix, h, c, n0, n1, sm + warp * s.NBmax, nullptr, warp, nwarps, lane);
         __syncthreads();
         for (int gb = tid; gb < s.NBmax; gb += nthreads) {
             int run = 0;
@@ -136,8 +196,11 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
             const int base = kt[gb] * s.TPT + cc[gb];
             for (int i = 0; i < nwarps; ++i) sm[i * s.NBmax + gb] = base + wo[i * s.NBmax + gb];
         }
+        unsigned* mk = sel_index_masks(s, nwarps) ? reinterpret_cast<unsigned*>(sm) + nwarps * s.NBmax : nullptr;
+        if (mk)
+            for (int i = tid; i < nwarps * s.NBmax; i += nthreads) mk[i] = 0u;
         __syncthreads();
-        chunk_pass<true>(topk_idx, cu, bd, s, ix, h, c, n0, n1, sm + warp * s.NBmax, warp, nwarps, lane);
+        chunk_pass<true>(topk_idx, cu, bd, s, ix, h, c, n0, n1, sm + warp * s.NBmax, mk ? mk + warp * s.NBmax : nullptr, warp, nwarps, lane);
     }
 }
 
@@ -253,9 +316,10 @@ __global__ void __launch_bounds__(256) sel_index_tiles(const int* __restrict__ c
 // All five steps in one launch, for short problems: one CTA per kv head, the CTAs of a cluster exchange the numbers of tiles
 // and segments of their heads through distributed shared memory.  What bounds a short build is the latency of its launches
 // and dependent steps: 512 tokens x 2 heads took 24 us in five kernels and a memset.  The list is the same one (a warp takes
-// a contiguous range of 32-token groups either way).  Used up to kSmallTokens tokens, where the passes over the tokens (four
-// groups a warp) cost about what the launches do, and up to 8 heads (the cluster) and kSmallKeys blocks (a thread each).
-constexpr int kSmallTokens = 4096, kSmallKeys = 1024, kSmallWarps = 32;
+// a contiguous range of 32-token groups either way).  A head's entries all leave through one SM, scattered, at about one a clock:
+// used up to kSmallEntries of them (6 us + 1.1 ns each, against 28 us for the five launches), and up to 8 heads (the cluster) and
+// kSmallKeys blocks (a thread each).
+constexpr int kSmallEntries = 20000, kSmallKeys = 700, kSmallWarps = 32;
 
 // Exclusive prefix of v over the CTA's 1024 threads; *total = the sum.
 __device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total) {
@@ -280,15 +344,16 @@ __device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total)
 __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* __restrict__ topk_idx, const int* __restrict__ cu, SelBounds bd,
                                                                   SelShape s, SelIndex ix) {
     namespace cg = cooperative_groups;
-    extern __shared__ int sm[];   // [warps][NBmax] counts, then positions; [NBmax] entries, [NBmax] first tile, [NBmax] first segment of a key
+    extern __shared__ int sm[];   // [warps][NBmax] counts, then positions; [warps][NBmax] lane bits; [NBmax] entries, first tile, first segment of a key
     __shared__ int wsum[32], mine[3];       // tiles, entries, segments of this head
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, NB = s.NBmax;
-    int *s_cnt = sm + kSmallWarps * NB, *s_t0 = s_cnt + NB, *s_seg = s_t0 + NB;
+    unsigned* mk = reinterpret_cast<unsigned*>(sm) + kSmallWarps * NB;
+    int *s_cnt = sm + 2 * kSmallWarps * NB, *s_t0 = s_cnt + NB, *s_seg = s_t0 + NB;
     const int* ck = bd.cu_k ? bd.cu_k : cu;
-    for (int i = tid; i < kSmallWarps * NB; i += blockDim.x) sm[i] = 0;
+    for (int i = tid; i < 2 * kSmallWarps * NB; i += blockDim.x) sm[i] = 0;
     __syncthreads();
-    chunk_pass<false>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
+    chunk_pass<false>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, nullptr, warp, kSmallWarps, lane);
     __syncthreads();
     // a warp per key: lane w turns warp w's count into its first position inside the key
     for (int gb = warp; gb < NB; gb += kSmallWarps) {
@@ -336,13 +401,13 @@ __global__ void __launch_bounds__(kSmallWarps * 32) sel_index_small(const int* _
         if (s_cnt[gb] > 0) write_tiles(s, ix, ck, h, gb, s_cnt[gb], s_t0[gb], s_seg[gb], lane);
     for (int gb = lane; gb < NB; gb += 32) sm[warp * NB + gb] += s_t0[gb] * s.TPT;
     __syncwarp();
-    chunk_pass<true>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, warp, kSmallWarps, lane);
+    chunk_pass<true>(topk_idx, cu, bd, s, ix, h, 0, 0, (int)s.N, sm + warp * NB, mk + warp * NB, warp, kSmallWarps, lane);
     cluster.barrier_wait();
 }
 
 // warps per CTA of the chunk kernels so that the per-warp histograms fit in shared memory; 0: the problem does not fit
 int sel_index_warps(const SelShape& s) {
-    const int64_t ints = (200 * 1024) / 4;
+    const int64_t ints = kIdxSmem / 4;
     int64_t nw = ints / (s.NBmax > 0 ? s.NBmax : 1);
     if (nw < 1) return 0;
     if (nw > kIdxMaxWarps) nw = kIdxMaxWarps;
@@ -355,8 +420,8 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
                             cudaStream_t stream) {
     cudaError_t e;
     if ((int64_t)s.Hk * s.N == 0) return cudaMemsetAsync(ix.header, 0, 64 * 4, stream);
-    if (s.N <= kSmallTokens && s.Hk <= 8 && s.NBmax <= kSmallKeys) {
-        const int smem = (kSmallWarps + 3) * s.NBmax * 4;
+    if (s.N * s.T <= kSmallEntries && s.Hk <= 8 && s.NBmax <= kSmallKeys) {
+        const int smem = (2 * kSmallWarps + 3) * s.NBmax * 4;
         e = allow_smem((const void*)sel_index_small, smem);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
@@ -373,10 +438,10 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     }
     const int nw = s.IW;
     if (nw == 0) return cudaErrorInvalidValue;
-    const int smem = nw * s.NBmax * 4;
+    const int smem = nw * s.NBmax * 4, smem_fill = sel_index_masks(s, nw) ? 2 * smem : smem;
     e = allow_smem((const void*)sel_index_chunk<false>, smem);
     if (e != cudaSuccess) return e;
-    e = allow_smem((const void*)sel_index_chunk<true>, smem);
+    e = allow_smem((const void*)sel_index_chunk<true>, smem_fill);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)s.NC, (unsigned)s.Hk);
     const int HG = s.Hk * s.NBmax;
@@ -384,7 +449,7 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     sel_index_keys<<<(unsigned)((HG + 63) / 64), 64, 0, stream>>>(s, ix);
     sel_index_scan<<<1, 1024, 0, stream>>>(s, ix);
     sel_index_tiles<<<(unsigned)((HG + 7) / 8), 256, 0, stream>>>(cu, bd, s, ix);
-    sel_index_chunk<true><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
+    sel_index_chunk<true><<<grid, nw * 32, smem_fill, stream>>>(topk_idx, cu, bd, s, ix);
     return cudaGetLastError();
 }
 
