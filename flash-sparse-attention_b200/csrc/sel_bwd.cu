@@ -566,7 +566,12 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (rows > 0) {
+    if (rows > 0 && sel_merge_fits(s, nsub)) {
+        prof_begin(3, stream);
+        e = launch_sel_merge_dq(dt, a.dq_part, ix.pos, s, nsub, a.dq, ix.header, num_sms, stream);
+        prof_end(3, stream);
+        if (e != cudaSuccess) return e;
+    } else if (rows > 0) {
         unsigned grid = (unsigned)((rows + 7) / 8);
         e = prefer_l1((const void*)sel_bwd_dq_reduce<D, ET>);
         if (e != cudaSuccess) return e;

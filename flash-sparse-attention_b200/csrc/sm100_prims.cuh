@@ -171,6 +171,12 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
                  "r"(x), "r"(y), "r"(z), "r"(src_smem)
                  : "memory");
 }
+// Untiled copy global -> shared memory; both addresses and the size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem), "l"(src), "r"(bytes),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
 // L2 eviction policies for data with a known lifetime: evict_first for rows that are written once and read once much
 // later (they should not push anything else out), evict_last for lines that are completed by many small writes.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
