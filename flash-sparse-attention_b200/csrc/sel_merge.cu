@@ -2,13 +2,14 @@
 // partial outputs and their (m, l), dQ as the plain sum of the backward's partial rows.  (In the reference: the reduction of
 // fsa/ops/FSA_topk_sparse_attention.py:741-818 and the dQ accumulation of :1416-1545.)
 //
-// 2 KB or 4 KB have to come in per output row, as 16 pieces of 128 or 256 bytes from all over 2 GB.  As one warp per row that
+// 4 KB have to come in per output row, as 16 pieces of 256 bytes from all over 2 GB.  As one warp per row that
 // loads positions, then rows, then sums up and ends, the merge was bound by that chain of round trips, not by memory (partial
 // rows laid out in one contiguous piece took it no less time).  Here a CTA stays on its SM and each of 24 warps keeps 8 KB of
 // rows in flight: one bulk copy per partial row into the warp's own ring of stages, whose positions were loaded two rows before;
 // nothing passes through registers.  (With 12 warps and 16 KB each the arithmetic of a warp holds its stages up: dQ 503 us.)
-// 64K tokens x 8 heads x 16 rows of 256 bytes: forward 502 -> 425 us, dQ 476 -> 361 us = 6 TB/s.  At head size 256 the
-// warp per row already moves 5.9 TB/s, and stages of 8 KB would leave a warp one: it keeps the other kernels.
+// 64K tokens x 8 heads x 16 rows of 256 bytes: forward 502 -> 425 us, dQ 476 -> 361 us = 6 TB/s.  At head size 256 a
+// warp per row already moves 5.9 TB/s, and at 64 a row's arithmetic is too much for 24 warps (151 -> 193 us at 16384 tokens x 16
+// heads): they keep the other kernels.
 #include "sel_launch.cuh"
 
 namespace fsa {
@@ -20,8 +21,8 @@ template <int D>
 struct MergeCfg {
     static constexpr int kRow = D * 2;                      // bytes of a partial row
     static constexpr int kStage = kMgSlots * kRow;
-    static constexpr int S = 8192 / kStage;                 // stages of a warp: 4 or 2 for head sizes 64 and 128
-    static constexpr int kBytes = kMgWarps * S * (kStage + 8 + 4) + 16;
+    static constexpr int S = 8192 / kStage;                 // stages of a warp
+    static constexpr int kBytes = kMgWarps * (S * (kStage + 8 + 4) + kMgSlots * 4);
 };
 
 // An output row (token, kv head, head of the group) and the step from one of a warp's rows to the next.
@@ -52,7 +53,8 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* ring = smem + warp * (S * C::kStage);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kMgWarps * S * C::kStage) + warp * S;
-    unsigned* masks = reinterpret_cast<unsigned*>(smem + kMgWarps * S * (C::kStage + 8)) + warp * S;
+    float* wts = reinterpret_cast<float*>(smem + kMgWarps * S * (C::kStage + 8)) + warp * kMgSlots;
+    unsigned* masks = reinterpret_cast<unsigned*>(smem + kMgWarps * (S * (C::kStage + 8) + kMgSlots * 4)) + warp * S;
     if (lane < S) mbar_init(&bars[lane], 1);
     mbar_init_fence();
     __syncwarp();
@@ -113,36 +115,37 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
         float acc[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] = 0.f;
-        float w = 1.f, M = 0.f, L = 1.f;
+        float M = 0.f, L = 1.f;
         if (FWD) {
+            // (lanes from 16 on hold no slot: four steps, and the sum handed to them)
             const float m0 = (mask >> lane & 1u) ? v.x : -INFINITY;
             M = m0;
 #pragma unroll
-            for (int o = 16; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-            w = m0 == -INFINITY ? 0.f : exp2f(m0 - M);
+            for (int o = 8; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+            const float w = m0 == -INFINITY ? 0.f : exp2f(m0 - M);
+            if (lane < kMgSlots) wts[lane] = w;
             L = m0 == -INFINITY ? 0.f : w * v.y;
 #pragma unroll
-            for (int o = 16; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+            for (int o = 8; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+            L = __shfl_sync(0xffffffffu, L, 0);
+            __syncwarp();
         }
-        if (mask == 0xffffu) {
+        const bool all = mask == (1u << R) - 1u && (R & 3) == 0;
+        auto four = [&](int j0) {
+            const float4 w = FWD ? *reinterpret_cast<const float4*>(wts + j0) : make_float4(1.f, 1.f, 1.f, 1.f);
+            fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j0 * D), w.x);
+            fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + (j0 + 1) * D), w.y);
+            fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + (j0 + 2) * D), w.z);
+            fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + (j0 + 3) * D), w.w);
+        };
+        if (all && R == kMgSlots) {
 #pragma unroll
-            for (int j = 0; j < kMgSlots; ++j) {
-                const float wj = FWD ? __shfl_sync(0xffffffffu, w, j) : 1.f;
-                fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), wj);
-            }
-        } else if (mask == (1u << R) - 1u && (R & 3) == 0) {
-            for (int j0 = 0; j0 < R; j0 += 4) {
-#pragma unroll
-                for (int j = j0; j < j0 + 4; ++j) {
-                    const float wj = FWD ? __shfl_sync(0xffffffffu, w, j) : 1.f;
-                    fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), wj);
-                }
-            }
+            for (int j0 = 0; j0 < kMgSlots; j0 += 4) four(j0);
+        } else if (all) {
+            for (int j0 = 0; j0 < R; j0 += 4) four(j0);
         } else {
-            for (int j = 0; j < R; ++j) {
-                const float wj = FWD ? __shfl_sync(0xffffffffu, w, j) : 1.f;
-                if (mask >> j & 1u) fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), wj);
-            }
+            for (int j = 0; j < R; ++j)
+                if (mask >> j & 1u) fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), FWD ? wts[j] : 1.f);
         }
         __syncwarp();                            // the stage has been read
         if (k + S < cnt) {
@@ -157,8 +160,7 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) x[i] = ElemTraits<ET>::pack2(acc[2 * i] * inv, acc[2 * i + 1] * inv);
         if (ok) {
-            if constexpr (V == 2) *reinterpret_cast<uint32_t*>(dst) = x[0];
-            else *reinterpret_cast<uint2*>(dst) = make_uint2(x[0], x[1]);
+            *reinterpret_cast<uint2*>(dst) = make_uint2(x[0], x[1]);
             if (FWD && lane == 0) lse[(int64_t)hq * s.N + at.n] = L > 0.f ? M + log2f(L) : -INFINITY;
         }
         at.next(step, s.Hk, s.G);
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
 }
 
 bool sel_merge_fits(const SelShape& s, int nsub) {
-    return s.D <= 128 && s.T * nsub <= kMgSlots && s.N * s.Hq >= kMgRows && s.N * s.Hq < (1ll << 30);
+    return s.D == 128 && s.T * nsub <= kMgSlots && s.N * s.Hq >= kMgRows && s.N * s.Hq < (1ll << 30);
 }
 
 template <int D, typename ET, bool FWD>
@@ -189,7 +191,7 @@ static cudaError_t merge(int dtype, const void* part, const float2* ml, const in
     if (s.D == DD)                                                                                                                              \
         return dtype == kBF16 ? launch_merge<DD, __nv_bfloat16, FWD>(part, ml, pos, s, nsub, out, o_sn, o_sh, lse, status, sms, stream)         \
                               : launch_merge<DD, __half, FWD>(part, ml, pos, s, nsub, out, o_sn, o_sh, lse, status, sms, stream);
-    FSA_CASE(64) FSA_CASE(128)
+    FSA_CASE(128)
 #undef FSA_CASE
     return cudaErrorInvalidValue;
 }
