@@ -173,14 +173,29 @@ __global__ void __launch_bounds__(256) gate_proj_mix_fwd_kernel(const ET* __rest
     extern __shared__ __align__(16) uint8_t gsm[];
     uint4* sw = reinterpret_cast<uint4*>(gsm);                 // [3][hidden / 8]
     const int hv = hidden / 8, vec = HD / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // the first kAhead vectors of a token's row are on their way while the weights are copied or the token before is mixed
+    constexpr int kAhead = 8;
+    uint4 xa[kAhead];
+    auto ahead = [&](int64_t n) {
+        const uint4* xr = reinterpret_cast<const uint4*>(x + n * x_sn);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) xa[i] = n < N && lane + 32 * i < hv ? ld_stream16(xr + lane + 32 * i) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    ahead((int64_t)blockIdx.x * nw + warp);
     for (int i = threadIdx.x; i < 3 * hv; i += blockDim.x) sw[i] = reinterpret_cast<const uint4*>(wg)[i];
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int64_t n = (int64_t)blockIdx.x * nw + warp; n < N; n += (int64_t)gridDim.x * nw) {
         float z0 = 0.f, z1 = 0.f, z2 = 0.f;
         const uint4* xr = reinterpret_cast<const uint4*>(x + n * x_sn);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int v = lane + 32 * i;
+            if (v < hv) dot8x3<ET>(xa[i], sw[v], sw[hv + v], sw[2 * hv + v], z0, z1, z2);
+        }
 #pragma unroll 8
-        for (int v = lane; v < hv; v += 32) dot8x3<ET>(__ldg(xr + v), sw[v], sw[hv + v], sw[2 * hv + v], z0, z1, z2);
+        for (int v = lane + 32 * kAhead; v < hv; v += 32) dot8x3<ET>(ld_stream16(xr + v), sw[v], sw[hv + v], sw[2 * hv + v], z0, z1, z2);
+        ahead(n + (int64_t)gridDim.x * nw);
 #pragma unroll
         for (int o = 16; o; o >>= 1) {
             z0 += __shfl_xor_sync(0xffffffffu, z0, o);
@@ -372,7 +387,7 @@ static int run_gate_fwd(const void* x, int64_t x_sn, const void* wg, const void*
                         int HD, void* out, void* gate, cudaStream_t stream) {
     const int smem = 3 * hidden * 2;
     auto kern = gate_proj_mix_fwd_kernel<ET>;
-    if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
+    if (allow_smem((const void*)kern, smem) != cudaSuccess || prefer_l1((const void*)kern, 50) != cudaSuccess) return FSA_ERR_CUDA;
     // a warp per token: four per CTA while eight would leave SMs idle
     const int warps = N <= 148 * 8 ? 4 : 8;
     const int64_t want = (N + warps - 1) / warps;
@@ -388,7 +403,7 @@ static int run_gate_bwd(const void* x, int64_t x_sn, const void* wg, const void*
                         float* partial, float* delta, int head_dim, cudaStream_t stream) {
     const int smem = 3 * hidden * 2;
     auto kern = !delta ? gate_proj_mix_bwd_kernel<0, ET> : head_dim == 128 ? gate_proj_mix_bwd_kernel<16, ET> : gate_proj_mix_bwd_kernel<8, ET>;
-    if (allow_smem((const void*)kern, smem) != cudaSuccess) return FSA_ERR_CUDA;
+    if (allow_smem((const void*)kern, smem) != cudaSuccess || prefer_l1((const void*)kern, 50) != cudaSuccess) return FSA_ERR_CUDA;
     const int64_t want = (N + 7) / 8;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
     kern<<<grid, 256, smem, stream>>>((const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,

@@ -111,7 +111,7 @@ cudaError_t allow_smem(const void* kern, int bytes) {
     return cudaSuccess;
 }
 
-cudaError_t prefer_l1(const void* kern) {
+cudaError_t prefer_l1(const void* kern, int smem_percent) {
     struct Seen { const void* kern; int dev; };
     static thread_local Seen seen[128];
     int dev = 0;
@@ -119,7 +119,7 @@ cudaError_t prefer_l1(const void* kern) {
     if (e != cudaSuccess) return e;
     Seen& c = seen[(((uintptr_t)kern >> 4) ^ ((uintptr_t)kern >> 11)) & 127];
     if (c.kern == kern && c.dev == dev) return cudaSuccess;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, smem_percent);
     if (e == cudaSuccess) c = Seen{kern, dev};
     return e;
 }

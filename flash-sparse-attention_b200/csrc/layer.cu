@@ -70,6 +70,9 @@ __device__ __forceinline__ void add8(const uint4& v, float (&a)[8]) {
     }
 }
 
+// (read once; q may be rotated in place, so not through the read-only path)
+__device__ __forceinline__ uint4 ld_stream(const uint4* p) { return __ldcs(p); }
+
 struct LayerRopeParams {
     const int *cu, *cu_cmp;
     int B, Hq, Hk, D, ks, stride, window;
@@ -103,11 +106,24 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
     float x1[8], x2[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) x1[j] = x2[j] = 0.f;
-    auto take = [&](const void* src, int64_t off) {
-        const ET* s = (const ET*)src + off;
-        add8<ET>(*reinterpret_cast<const uint4*>(s), x1);
-        add8<ET>(*reinterpret_cast<const uint4*>(s + half), x2);
+    // everything that does not depend on the position is loaded before the sequence is looked for
+    uint4 a1[3], a2[3];
+    auto load = [&](int j, const void* src, int64_t off) {
+        a1[j] = ld_stream(reinterpret_cast<const uint4*>((const ET*)src + off));
+        a2[j] = ld_stream(reinterpret_cast<const uint4*>((const ET*)src + off + half));
     };
+    auto take = [&](int j) {
+        add8<ET>(a1[j], x1);
+        add8<ET>(a2[j], x2);
+    };
+    if (kind == 2) {
+        load(0, p.cmp, at);
+    } else if (!BWD) {
+        load(0, kind == 0 ? p.q[0] : p.k[0], (int64_t)n * (kind == 0 ? p.q_sn : p.k_sn) + h * p.D + v * 8);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) load(j, kind == 0 ? p.q[j] : kind == 1 ? p.k[j] : p.v[j], at);
+    }
     auto put = [&](void* dst, const float (&y1)[8], const float (&y2)[8]) {
         uint4 o1, o2;
         uint32_t *q1 = &o1.x, *q2 = &o2.x;
@@ -120,7 +136,7 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
         *reinterpret_cast<uint4*>((ET*)dst + at + half) = o2;
     };
     if (BWD && kind == 3) {
-        take(p.v[0], at); take(p.v[1], at); take(p.v[2], at);
+        take(0); take(1); take(2);
         put(p.v_out, x1, x2);
         return;
     }
@@ -128,17 +144,11 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
     const int b = find_seq(cu, p.B, n);
     const int pos = n - __ldg(cu + b);
     const int64_t trow = (int64_t)(kind == 2 ? pos * p.stride : pos) * half + v * 8;
-    if (kind == 2) {
-        take(p.cmp, at);
-    } else if (!BWD) {
-        take(kind == 0 ? p.q[0] : p.k[0], (int64_t)n * (kind == 0 ? p.q_sn : p.k_sn) + h * p.D + v * 8);
-    } else if (kind == 0) {
-        take(p.q[0], at); take(p.q[1], at); take(p.q[2], at);
-    } else {
-        take(p.k[0], at); take(p.k[1], at);
-    }
+    take(0);
+    if (BWD && kind < 2) take(1);
+    if (BWD && kind == 0) take(2);
     rotate8<ET>(x1, x2, (const ET*)p.cs + trow, (const ET*)p.sn + trow, BWD ? -1.f : 1.f);
-    if (BWD && kind == 1) take(p.k[2], at);
+    if (BWD && kind == 1) take(2);
     put(kind == 0 ? p.q_out : kind == 1 ? p.k_out : p.cmp, x1, x2);
     if (!BWD && kind == 1 && h == 0 && v == 0 && p.hi_cmp) {
         const int c0 = __ldg(p.cu_cmp + b), nb = __ldg(p.cu_cmp + b + 1) - c0;
@@ -205,6 +215,8 @@ static int run_rope(const LayerRopeParams& p, int dtype, cudaStream_t stream) {
     if (threads == 0) return FSA_OK;
     (void)cudaGetLastError();
     const unsigned grid = (unsigned)((threads + 255) / 256);
+    if (prefer_l1(dtype == FSA_DTYPE_BF16 ? (const void*)layer_rope_kernel<BWD, __nv_bfloat16> : (const void*)layer_rope_kernel<BWD, __half>) != cudaSuccess)
+        return FSA_ERR_CUDA;
     if (dtype == FSA_DTYPE_BF16) layer_rope_kernel<BWD, __nv_bfloat16><<<grid, 256, 0, stream>>>(p);
     else layer_rope_kernel<BWD, __half><<<grid, 256, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;

@@ -24,7 +24,8 @@ cudaError_t allow_smem(const void* kern, int bytes);
 // kernel).  Without a preference the SMs keep the split of the kernel before, and after one with 227 KB of shared memory the
 // 28 KB that are left hold too few loads in flight: the merges of the partial rows took 467 us instead of 390 us (16K tokens,
 // 32 heads, 16 rows each).
-cudaError_t prefer_l1(const void* kern);
+// smem_percent: the share that stays shared memory, for a kernel that uses some.
+cudaError_t prefer_l1(const void* kern, int smem_percent = 0);
 // Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
 int ensure_context();
 
