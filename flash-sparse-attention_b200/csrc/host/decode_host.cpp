@@ -50,7 +50,7 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, co
     int32_t* lo = (int32_t*)take(b_r);
     int32_t* hi = (int32_t*)take(b_r);
     void* oc = take(b_oc);
-    Tensor topk = i32({B, Hk, c.topk}, q), out = at::empty_like(q);
+    Tensor topk = i32({B, Hk, c.topk}, q), out = fresh_like(q);
     check(fsa_decode_cmp_partial(ptr(q), ptr(cmp_k), ptr(cmp_v), cmp_k.size(0), cmp_k.stride(0), iptr(seq_len), iptr(cmp_row0), B, Hq, Hk, D,
                                  c.ks, c.stride, chunk, nchunk, dt, scale, o1, m1, sc, ld, st),
           "fsa_decode_cmp_partial");
@@ -85,7 +85,7 @@ static std::tuple<Tensor, Tensor> step(const Tensor& q_in, const Tensor& k_new, 
     const int cap = (int)((t[0].size(0) - 1) / B), cmp_cap = (int)((t[2].size(0) - 1) / B);
     const float* freq = inv_freq.defined() ? inv_freq.data_ptr<float>() : nullptr;
     void* st = stream_of(k_new);
-    const Tensor gate = at::empty({B, 3}, k_new.options());
+    const Tensor gate = fresh({B, 3}, k_new);
     check(fsa_decode_append(ptr(q_in), ptr(k_new), ptr(v_new), ptr(q), ptr(t[0]), ptr(t[1]), ptr(t[4]), ptr(t[5]), freq,
                             t[6].data_ptr<int32_t>(), iptr(t[7]), B, cap, Hq, Hk, D, c.ks, ptr(z), ptr(gx), ptr(gw),
                             gx.defined() ? (int)gx.size(-1) : 0, ptr(gate), dt, st),
@@ -133,10 +133,10 @@ std::tuple<Tensor, Tensor> decode_layer_step(const Tensor& x_, const Tensor& wq,
     const bool skinny = B <= kProjRows && x.size(1) % 256 == 0 && nq % 256 == 0 && ((uintptr_t)x.data_ptr() & 15) == 0;
     Tensor q, k, v, z;
     if (skinny) {
-        q = at::empty({B, nq}, x.options());
-        k = at::empty({B, nk}, x.options());
-        v = at::empty({B, nk}, x.options());
-        z = at::empty({B, 3}, x.options());
+        q = fresh({B, nq}, x);
+        k = fresh({B, nk}, x);
+        v = fresh({B, nk}, x);
+        z = fresh({B, 3}, x);
         project(x, {wq, wk, wv, gw}, {q, k, v, z});
     } else {
         q = at::linear(x, wq);
@@ -148,7 +148,7 @@ std::tuple<Tensor, Tensor> decode_layer_step(const Tensor& x_, const Tensor& wq,
                              compress, cfg_of(cfg, scale));
     const Tensor m = mixed.view({B, nq});
     if (!skinny) return {at::linear(m, wo), ids};
-    Tensor y = at::empty({B, wo.size(0)}, x.options());
+    Tensor y = fresh({B, wo.size(0)}, x);
     project(m, {wo}, {y});
     return {y, ids};
 }

@@ -3,6 +3,7 @@
 #pragma once
 #include <torch/extension.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -34,9 +35,15 @@ inline bool rows_ok(const Tensor& t, bool packed) {
 }
 inline Tensor rows(const Tensor& t, bool packed = false) { return rows_ok(t, packed) ? t : t.contiguous(); }
 
-inline Tensor bytes(int64_t n, const Tensor& like) { return at::empty({std::max<int64_t>(n, 16)}, like.options().dtype(at::kByte)); }
-inline Tensor f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
-inline Tensor i32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kInt)); }
+// Memory straight from the allocator: a layer's step makes some fifty tensors, and the dispatcher's share of each is as long as the rest.
+inline Tensor fresh(at::IntArrayRef shape, at::ScalarType type, const Tensor& like) {
+    return Tensor(at::detail::empty_cuda(shape, type, like.device(), std::nullopt));
+}
+inline Tensor fresh(at::IntArrayRef shape, const Tensor& like) { return fresh(shape, like.scalar_type(), like); }
+inline Tensor fresh_like(const Tensor& like) { return fresh(like.sizes(), like); }      // (contiguous)
+inline Tensor bytes(int64_t n, const Tensor& like) { return fresh({std::max<int64_t>(n, 16)}, at::kByte, like); }
+inline Tensor f32(at::IntArrayRef shape, const Tensor& like) { return fresh(shape, at::kFloat, like); }
+inline Tensor i32(at::IntArrayRef shape, const Tensor& like) { return fresh(shape, at::kInt, like); }
 inline const int32_t* iptr(const Tensor& t) { return t.defined() ? t.data_ptr<int32_t>() : nullptr; }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 

@@ -41,7 +41,7 @@ struct Kept {
 static std::pair<Tensor, Tensor> range_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, const int32_t* lo,
                                            const int32_t* hi, float scale) {
     const int64_t N = q.size(0);
-    Tensor o = at::empty_like(q), lse = f32({q.size(1), N}, q);
+    Tensor o = fresh_like(q), lse = f32({q.size(1), N}, q);
     check(fsa_range_attn_fwd_dense(ptr(q), ptr(k), ptr(v), iptr(cu_q), iptr(cu_k), lo, hi, N, k.size(0), (int)cu_q.size(0) - 1, (int)q.size(1),
                                    (int)k.size(1), (int)q.size(2), dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), scale, ptr(o),
                                    o.stride(0), o.stride(1), lse.data_ptr<float>(), nullptr, stream_of(q)),
@@ -56,8 +56,8 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     const int dt = dtype_code(x);
     const float scale = (float)(1.0 / std::sqrt((double)c.D));
     void* st = stream_of(x);
-    t.cs = at::empty({s.max_len, c.D / 2}, x.options());
-    t.sn = at::empty({s.max_len, c.D / 2}, x.options());
+    t.cs = fresh({s.max_len, c.D / 2}, x);
+    t.sn = fresh({s.max_len, c.D / 2}, x);
     t.cu_cmp = i32({s.B + 1}, x);
     check(fsa_layer_prep(iptr(cu), s.B, s.max_len, inv_freq.data_ptr<float>(), c.D, c.ks, c.stride, dt, ptr(t.cs), ptr(t.sn),
                          t.cu_cmp.data_ptr<int32_t>(), st),
@@ -65,15 +65,15 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     t.k_raw = at::mm(x, wk.t()).view({N, c.Hk, c.D});
     t.v = at::mm(x, wv.t()).view({N, c.Hk, c.D});
     t.q = at::mm(x, wq.t()).view({N, c.Hq, c.D});
-    t.ck = at::empty({s.Nc, c.Hk, c.D}, x.options());
-    t.cv = at::empty_like(t.ck);
+    t.ck = fresh({s.Nc, c.Hk, c.D}, x);
+    t.cv = fresh_like(t.ck);
     {
         const Tensor scratch = bytes(fsa_compress_bias_scratch_bytes(c.Hk, c.D), x);
         check(fsa_compress_kv_fwd(ptr(t.k_raw), t.k_raw.stride(0), ptr(t.v), t.v.stride(0), ptr(w_key), ptr(w_value), ptr(pe), s.tok.data(), s.B, c.Hk,
                                   c.D, c.ks, c.stride, dt, ptr(t.ck), ptr(t.cv), (float*)ptr(scratch), st),
               "fsa_compress_kv_fwd");
     }
-    t.k = at::empty_like(t.k_raw);
+    t.k = fresh_like(t.k_raw);
     t.bounds = i32({3, N}, x);
     int32_t* bd = t.bounds.data_ptr<int32_t>();
     check(fsa_layer_rope_fwd(ptr(t.q), t.q.stride(0), ptr(t.k_raw), t.k_raw.stride(0), ptr(t.ck), ptr(t.cs), ptr(t.sn), iptr(cu), iptr(t.cu_cmp), s.B,
@@ -88,8 +88,8 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
           "fsa_select_topk_fused");
     std::tie(t.o_sel, t.lse_sel, t.ws) = sel_fwd(t.q, t.k, t.v, t.topk, c.bs, cu, scale);
     std::tie(t.o_win, t.lse_win) = range_fwd(t.q, t.k, t.v, cu, cu, bd + N, bd + 2 * N, scale);
-    t.gate = at::empty({N, 3}, x.options());
-    Tensor out = at::empty({N, (int64_t)c.Hq * c.D}, x.options());
+    t.gate = fresh({N, 3}, x);
+    Tensor out = fresh({N, (int64_t)c.Hq * c.D}, x);
     check(fsa_gate_proj_mix_fwd(ptr(x), x.stride(0), ptr(wg), ptr(t.o_cmp), ptr(t.o_sel), ptr(t.o_win), N, (int)hidden, c.Hq * c.D, dt, ptr(out),
                                 ptr(t.gate), st),
           "fsa_gate_proj_mix_fwd");
@@ -107,7 +107,7 @@ static std::tuple<Tensor, Tensor, Tensor> range_bwd(const Tensor& q, const Tenso
     const bool indexed = fsa_range_attn_bwd_indexed(D) != 0;
     const Tensor ws = bytes(indexed ? ib : 16, q), scratch = bytes(bb, q);
     if (indexed) check(fsa_range_attn_index(iptr(cu_q), iptr(cu_k), lo, hi, N, Nk, B, Hq, Hk, max_blocks, 64, ptr(ws), ws.numel(), stream_of(q)), "fsa_range_attn_index");
-    Tensor dq = at::empty_like(q), dk = at::empty({Nk, Hk, D}, q.options()), dv = at::empty_like(dk);
+    Tensor dq = fresh_like(q), dk = fresh({Nk, Hk, D}, q), dv = fresh_like(dk);
     check(fsa_range_attn_bwd_delta(ptr(q), ptr(k), ptr(v), lse.data_ptr<float>(), ptr(dout), delta, iptr(cu_q), iptr(cu_k), lo, hi, N, Nk, B, Hq, Hk, D,
                                    max_blocks, 64, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1),
                                    scale, ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
@@ -129,6 +129,7 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         ctx->saved_data["seqlens"] = seqlens;
         ctx->saved_data["cfg"] = cfg;
         ctx->mark_non_differentiable({t.topk});
+        ctx->set_materialize_grads(false);          // (no zeros for the ids)
         return {out, t.topk};
     }
 
@@ -138,6 +139,7 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
                      &q = sv[9], &k_raw = sv[10], &k = sv[11], &v = sv[12], &ck = sv[13], &cv = sv[14], &cs = sv[15], &sn = sv[16], &cu_cmp = sv[17],
                      &bounds = sv[18], &o_cmp = sv[19], &lse_cmp = sv[20], &topk = sv[21], &o_sel = sv[22], &lse_sel = sv[23], &ws = sv[24],
                      &o_win = sv[25], &lse_win = sv[26], &gate = sv[27];
+        if (!grads[0].defined()) return torch::autograd::variable_list(12);
         const LayerCfg c = layer_cfg(ctx->saved_data["cfg"].toIntVector());
         const Lengths s(ctx->saved_data["seqlens"].toIntVector(), c);
         c10::cuda::CUDAGuard guard(x.device());
@@ -148,8 +150,8 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         void* st = stream_of(x);
         const int32_t* bd = iptr(bounds);
 
-        Tensor dx = at::empty({N, hidden}, x.options()), dwg = at::empty_like(wg), delta = f32({3, c.Hq, N}, x);
-        Tensor d_cmp = at::empty_like(q), d_sel = at::empty_like(q), d_win = at::empty_like(q);
+        Tensor dx = fresh({N, hidden}, x), dwg = fresh_like(wg), delta = f32({3, c.Hq, N}, x);
+        Tensor d_cmp = fresh_like(q), d_sel = fresh_like(q), d_win = fresh_like(q);
         {
             const Tensor dout = grads[0].contiguous();
             const Tensor scratch = bytes(fsa_gate_proj_mix_scratch_bytes(N, (int)hidden), x);
@@ -171,10 +173,10 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
                   "fsa_layer_rope_bwd");
         };
         rope_bwd(0, s.Nc, Tensor(), Tensor());
-        Tensor dw_key = ctx->needs_input_grad(5) ? at::empty_like(w_key) : Tensor(), dw_value = ctx->needs_input_grad(6) ? at::empty_like(w_value) : Tensor(),
-               dpe = ctx->needs_input_grad(7) ? at::empty_like(pe) : Tensor();
+        Tensor dw_key = ctx->needs_input_grad(5) ? fresh_like(w_key) : Tensor(), dw_value = ctx->needs_input_grad(6) ? fresh_like(w_value) : Tensor(),
+               dpe = ctx->needs_input_grad(7) ? fresh_like(pe) : Tensor();
         {
-            const Tensor dkc = at::empty_like(dk), dvc = at::empty_like(dv), scratch = bytes(fsa_compress_kv_bwd_scratch_bytes(c.Hk, c.D), x);
+            const Tensor dkc = fresh_like(dk), dvc = fresh_like(dv), scratch = bytes(fsa_compress_kv_bwd_scratch_bytes(c.Hk, c.D), x);
             check(fsa_compress_kv_bwd(ptr(k_raw), k_raw.stride(0), ptr(v), v.stride(0), ptr(w_key), ptr(w_value), ptr(pe), ptr(dck), ptr(dcv), iptr(cu),
                                       s.tok.data(), s.B, c.Hk, c.D, c.ks, c.stride, dt, ptr(dkc), ptr(dvc), ptr(dw_key), ptr(dw_value), ptr(dpe),
                                       (float*)ptr(scratch), st),

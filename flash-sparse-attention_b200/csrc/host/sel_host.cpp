@@ -25,7 +25,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_fwd(const Tensor& q_, const Tensor& k_, c
     Tensor ws = bytes(nb, q);
     check(fsa_sel_fwd_scratch_bytes(s.N, s.B, s.Hq, s.Hk, s.D, s.T, s.bs, &nb), "fsa_sel_fwd_scratch_bytes");
     const Tensor scratch = bytes(nb, q);
-    Tensor o = at::empty({s.N, s.Hq, s.D}, q.options()), lse = f32({s.Hq, s.N}, q);
+    Tensor o = fresh({s.N, s.Hq, s.D}, q), lse = f32({s.Hq, s.N}, q);
     check(fsa_sel_fwd(ptr(q), ptr(k), ptr(v), iptr(idx), iptr(cu), s.N, s.B, s.Hq, s.Hk, s.D, s.T, s.bs, dtype_code(q), q.stride(0),
                       q.stride(1), k.stride(0), v.stride(0), (float)scale, ptr(o), o.stride(0), o.stride(1), lse.data_ptr<float>(),
                       ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
@@ -43,7 +43,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q_, const Tensor& k_, c
     int64_t nb = 0;
     check(fsa_sel_bwd_scratch_bytes(s.N, s.B, s.Hq, s.Hk, s.D, s.T, s.bs, &nb), "fsa_sel_bwd_scratch_bytes");
     const Tensor scratch = bytes(nb, q);
-    Tensor dq = at::empty({s.N, s.Hq, s.D}, q.options()), dk = at::empty({s.N, s.Hk, s.D}, q.options()), dv = at::empty_like(dk);
+    Tensor dq = fresh({s.N, s.Hq, s.D}, q), dk = fresh({s.N, s.Hk, s.D}, q), dv = fresh_like(dk);
     check(fsa_sel_bwd(ptr(q), ptr(k), ptr(v), ptr(o), lse.data_ptr<float>(), ptr(dout), iptr(idx), iptr(cu), s.N, s.B, s.Hq, s.Hk, s.D,
                       s.T, s.bs, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), o.stride(0), o.stride(1),
                       dout.stride(0), dout.stride(1), (float)scale, ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch),
@@ -59,7 +59,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd_delta(const Tensor& q, const Tensor& 
     int64_t nb = 0;
     check(fsa_sel_bwd_scratch_bytes(s.N, s.B, s.Hq, s.Hk, s.D, s.T, s.bs, &nb), "fsa_sel_bwd_scratch_bytes");
     const Tensor scratch = bytes(nb, q);
-    Tensor dq = at::empty_like(q), dk = at::empty({s.N, s.Hk, s.D}, q.options()), dv = at::empty_like(dk);
+    Tensor dq = fresh_like(q), dk = fresh({s.N, s.Hk, s.D}, q), dv = fresh_like(dk);
     check(fsa_sel_bwd_delta(ptr(q), ptr(k), ptr(v), lse.data_ptr<float>(), ptr(dout), delta, iptr(idx), iptr(cu), s.N, s.B, s.Hq, s.Hk, s.D, s.T,
                             s.bs, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1), (float)scale,
                             ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
