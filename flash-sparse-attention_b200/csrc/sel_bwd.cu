@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ 
 // fsa/ops/FSA_topk_sparse_attention.py:1854-1855).  The rows of a block that nobody selected (no segment) and those past
 // the last sequence (the last CTA) are written as zeros here: no pass over dk and dv before (26 us of 64K tokens x 4 heads).
 template <int D, typename ET>
-__global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s,
+__global__ void __launch_bounds__(256, 4) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s,
                                                            SelIndex ix, int nsub, ET* __restrict__ dk, ET* __restrict__ dv) {
     constexpr int KT = 64, RV = D / 4;                // keys of a slab, float4 per row
     constexpr int kShares = 2 * KT * RV / 1024;       // CTAs per slab: 1024 float4 each, four per thread in flight
@@ -471,11 +471,28 @@ __global__ void __launch_bounds__(256) sel_bwd_dkdv_reduce(const float* __restri
     float4 acc[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int sg = 0; sg < nseg; ++sg) {
+    // two segments in flight: a block that every token selects has many (20 of a 3661-token sequence took 27 us one by one; four in
+    // flight cost the registers that hide the latency of everybody else)
+    int sg = 0;
+    for (; sg + 2 <= nseg; sg += 2) {
+        float4 v[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * 256;              // float4 of the slab: (which * 64 + key) * RV + column / 4
+                v[u][j] = (i / RV & (KT - 1)) < nkeys ? __ldcs(base + (sg + u) * seg_stride + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
+    }
+    for (; sg < nseg; ++sg) {
         float4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int i = i0 + j * 256;                  // float4 of the slab: (which * 64 + key) * RV + column / 4
+            const int i = i0 + j * 256;
             v[j] = (i / RV & (KT - 1)) < nkeys ? __ldcs(base + sg * seg_stride + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
