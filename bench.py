@@ -424,7 +424,7 @@ def run_decode(args, dd, steps, sub=False):
             "e2e": ({"value": B / (e2e_ms * 1e-3), "unit": "tokens/s", "ms_per_step": e2e_ms,
                      "h2d_bytes_per_step": (qh.numel() + knh.numel() + vnh.numel()) * 2, "d2h_bytes_per_step": B * Hq * d * 2}
                     if e2e_n else None),
-            "gpu_launches": (7 if world == 1 else 9) * steps, "cuda_graph": use_graph,
+            "gpu_launches": (4 if world == 1 else 9) * steps, "cuda_graph": use_graph,
             "clocks": clocks,
         }
     del cache, mod

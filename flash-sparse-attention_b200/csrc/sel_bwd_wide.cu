@@ -8,7 +8,7 @@
 //   * dQ takes the columns of S and dP (they have been read when dS is there); the drain empties them behind the gather of dO;
 //   * the drain stages dQ in the P / dS buffers (their readers are done), half a row at a time.
 // The unpipelined kernel walked the same chain with 128 threads and no overlap at all: 17.5 us a tile.
-// 16384 tokens, 4 KV heads, G = 2: see the table of cases for the measured times.
+// 16384 tokens, 4 KV heads, G = 2: 1967 -> 736 us (6.5 us a tile).
 // Blocks of more than 64 keys are walked in 64-key parts as in sel_bwd_pipe.cu.
 #include "sel_launch.cuh"
 
