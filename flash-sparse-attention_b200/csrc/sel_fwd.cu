@@ -49,8 +49,9 @@ template <int D, int BK>
 struct SelFwdCfg {
     static constexpr int kQ = kTileRows * D * 2;
     static constexpr int kKV = 2 * BK * D * 2;         // K then V
-    // Output staging of a softmax warp (32 rows, input dtype): whole rows, or at head size 256 one 64-column slab at a time
-    static constexpr int kOSCols = D <= 128 ? D : 64;
+    // Output staging of a softmax warp (32 rows, input dtype): whole rows, or one 64-column slab at a time where that makes room
+    // (head size 256: at all; 128-key blocks at 128: for a second K/V stage)
+    static constexpr int kOSCols = D > 128 || (D == 128 && BK == 128) ? 64 : D;
     static constexpr int kOS = kTileRows * kOSCols * 2;    // ... of a softmax group
     static constexpr int kTail = 2560;                 // barriers, TMEM slot, row-offset table
     static constexpr int kMax = 227 * 1024;

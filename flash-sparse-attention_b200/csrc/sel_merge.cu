@@ -2,14 +2,14 @@
 // partial outputs and their (m, l), dQ as the plain sum of the backward's partial rows.  (In the reference: the reduction of
 // fsa/ops/FSA_topk_sparse_attention.py:741-818 and the dQ accumulation of :1416-1545.)
 //
-// 4 KB have to come in per output row, as 16 pieces of 256 bytes from all over 2 GB.  As one warp per row that
+// 4 KB (head size 64: 2 KB) have to come in per output row, as 16 pieces of 256 bytes from all over 2 GB.  As one warp per row that
 // loads positions, then rows, then sums up and ends, the merge was bound by that chain of round trips, not by memory (partial
 // rows laid out in one contiguous piece took it no less time).  Here a CTA stays on its SM and each of 24 warps keeps 8 KB of
 // rows in flight: one bulk copy per partial row into the warp's own ring of stages, whose positions were loaded two rows before;
 // nothing passes through registers.  (With 12 warps and 16 KB each the arithmetic of a warp holds its stages up: dQ 503 us.)
 // 64K tokens x 8 heads x 16 rows of 256 bytes: forward 502 -> 425 us, dQ 476 -> 361 us = 6 TB/s.  At head size 256 a
-// warp per row already moves 5.9 TB/s, and at 64 a row's arithmetic is too much for 24 warps (151 -> 193 us at 16384 tokens x 16
-// heads): they keep the other kernels.
+// warp per row already moves 5.9 TB/s and keeps the other kernels; at 64 a row's arithmetic is too much for 24 warps (151 -> 193 us
+// forward at 16384 tokens x 16 heads), so that half a warp takes a row there (forward 144 us, dQ 157 -> 137 us).
 #include "sel_launch.cuh"
 
 namespace fsa {
@@ -20,9 +20,10 @@ constexpr int64_t kMgRows = 24000;      // output rows from which a warp has eno
 template <int D>
 struct MergeCfg {
     static constexpr int kRow = D * 2;                      // bytes of a partial row
-    static constexpr int kStage = kMgSlots * kRow;
+    static constexpr int H = 128 / D;                       // output rows that a warp takes at a time: one, or at head size 64 one per half warp
+    static constexpr int kStage = H * kMgSlots * kRow;
     static constexpr int S = 8192 / kStage;                 // stages of a warp
-    static constexpr int kBytes = kMgWarps * (S * (kStage + 8 + 4) + kMgSlots * 4);
+    static constexpr int kBytes = kMgWarps * (S * (kStage + 8 + 4) + H * kMgSlots * 4);
 };
 
 // An output row (token, kv head, head of the group) and the step from one of a warp's rows to the next.
@@ -48,28 +49,28 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
                                                              SelShape s, int nsub, ET* __restrict__ out, int64_t o_sn, int64_t o_sh,
                                                              float* __restrict__ lse, int* status) {
     using C = MergeCfg<D>;
-    constexpr int S = C::S, V = D / 32;
+    constexpr int S = C::S, H = C::H, LPR = 32 / H, V = D / LPR;          // LPR: lanes of an output row
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % LPR, half = lane / LPR;
     uint8_t* ring = smem + warp * (S * C::kStage);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kMgWarps * S * C::kStage) + warp * S;
-    float* wts = reinterpret_cast<float*>(smem + kMgWarps * S * (C::kStage + 8)) + warp * kMgSlots;
-    unsigned* masks = reinterpret_cast<unsigned*>(smem + kMgWarps * (S * (C::kStage + 8) + kMgSlots * 4)) + warp * S;
+    float* wts = reinterpret_cast<float*>(smem + kMgWarps * S * (C::kStage + 8)) + (warp * H + half) * kMgSlots;
+    unsigned* masks = reinterpret_cast<unsigned*>(smem + kMgWarps * (S * (C::kStage + 8) + H * kMgSlots * 4)) + warp * S;
     if (lane < S) mbar_init(&bars[lane], 1);
     mbar_init_fence();
     __syncwarp();
-    const int rows = (int)(s.N * s.Hq), W = (int)gridDim.x * kMgWarps, first = (int)blockIdx.x * kMgWarps + warp;
-    const int cnt = first < rows ? (rows - first + W - 1) / W : 0;
-    const MergeRow step = merge_row(W, s);
-    const int R = s.T * nsub, sl = lane % s.T, sub = lane / s.T;        // partial rows; lane: row sub * T + sl
-    MergeRow at_pos = merge_row(first, s), at_ml = at_pos, at = at_pos;
+    const int rows = (int)(s.N * s.Hq), items = (rows + H - 1) / H, W = (int)gridDim.x * kMgWarps, first = (int)blockIdx.x * kMgWarps + warp;
+    const int cnt = first < items ? (items - first + W - 1) / W : 0;
+    const MergeRow step = merge_row(W * H, s);
+    const int R = s.T * nsub, sl = l % s.T, sub = l / s.T;              // partial rows; lane: row sub * T + sl
+    MergeRow at_pos = merge_row(first * H + half, s), at_ml = at_pos, at = at_pos;      // (n = N: the odd row out at the end)
     auto load_pos = [&](int& ps, int& g) {
-        ps = lane < R ? __ldg(pos + ((int64_t)at_pos.h * s.N + at_pos.n) * s.T + sl) : -1;
+        ps = l < R && at_pos.n < s.N ? __ldg(pos + ((int64_t)at_pos.h * s.N + at_pos.n) * s.T + sl) : -1;
         g = at_pos.g;
         at_pos.next(step, s.Hk, s.G);
     };
     auto load_ml = [&]() {
-        const float2 v = lane < s.T ? __ldg(ml + ((int64_t)(at_ml.h * s.G + at_ml.g) * s.N + at_ml.n) * s.T + lane) : make_float2(0.f, 0.f);
+        const float2 v = l < s.T && at_ml.n < s.N ? __ldg(ml + ((int64_t)(at_ml.h * s.G + at_ml.g) * s.N + at_ml.n) * s.T + l) : make_float2(0.f, 0.f);
         at_ml.next(step, s.Hk, s.G);
         return v;
     };
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
         if (ps >= 0) {
             const int tile = ps / s.TPT;
             const int64_t row = ((int64_t)tile * nsub + sub) * kTileRows + g * s.TPT + (ps - tile * s.TPT);
-            bulk_load(smem_u32(ring + st * C::kStage + lane * C::kRow), part + row * D, C::kRow, &bars[st]);
+            bulk_load(smem_u32(ring + st * C::kStage + (half * kMgSlots + l) * C::kRow), part + row * D, C::kRow, &bars[st]);
         }
     };
     int ps[S], gs[S];
@@ -111,26 +112,26 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
         }
         ok = mbar_wait(&bars[st], (k / S) & 1, status) && ok;
         const unsigned mask = masks[st];
-        const ET* src = reinterpret_cast<const ET*>(ring + st * C::kStage) + lane * V;
+        const ET* src = reinterpret_cast<const ET*>(ring + st * C::kStage) + half * kMgSlots * D + l * V;
         float acc[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] = 0.f;
         float M = 0.f, L = 1.f;
         if (FWD) {
-            // (lanes from 16 on hold no slot: four steps, and the sum handed to them)
+            // (16 lanes hold the slots of a row: four steps, and at head size 128 the sum handed to the others)
             const float m0 = (mask >> lane & 1u) ? v.x : -INFINITY;
             M = m0;
 #pragma unroll
             for (int o = 8; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
             const float w = m0 == -INFINITY ? 0.f : exp2f(m0 - M);
-            if (lane < kMgSlots) wts[lane] = w;
+            if (l < kMgSlots) wts[l] = w;
             L = m0 == -INFINITY ? 0.f : w * v.y;
 #pragma unroll
             for (int o = 8; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-            L = __shfl_sync(0xffffffffu, L, 0);
+            L = __shfl_sync(0xffffffffu, L, lane & ~(LPR - 1));
             __syncwarp();
         }
-        const bool all = mask == (1u << R) - 1u && (R & 3) == 0;
+        const bool all = mask == ((1u << R) - 1u) * (H == 2 ? 0x10001u : 1u) && (R & 3) == 0;
         auto four = [&](int j0) {
             const float4 w = FWD ? *reinterpret_cast<const float4*>(wts + j0) : make_float4(1.f, 1.f, 1.f, 1.f);
             fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j0 * D), w.x);
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
             for (int j0 = 0; j0 < R; j0 += 4) four(j0);
         } else {
             for (int j = 0; j < R; ++j)
-                if (mask >> j & 1u) fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), FWD ? wts[j] : 1.f);
+                if (mask >> (half * 16 + j) & 1u) fma_row_vec<V, ET>(acc, ld_row_vec<V, ET>(src + j * D), FWD ? wts[j] : 1.f);
         }
         __syncwarp();                            // the stage has been read
         if (k + S < cnt) {
@@ -155,13 +156,13 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
         }
         const int hq = at.h * s.G + at.g;
         const float inv = FWD ? (L > 0.f ? 1.f / L : 0.f) : 1.f;
-        ET* dst = out + (int64_t)at.n * o_sn + (int64_t)hq * o_sh + lane * V;
+        ET* dst = out + (int64_t)at.n * o_sn + (int64_t)hq * o_sh + l * V;
         uint32_t x[V / 2];
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) x[i] = ElemTraits<ET>::pack2(acc[2 * i] * inv, acc[2 * i + 1] * inv);
-        if (ok) {
+        if (ok && at.n < s.N) {
             *reinterpret_cast<uint2*>(dst) = make_uint2(x[0], x[1]);
-            if (FWD && lane == 0) lse[(int64_t)hq * s.N + at.n] = L > 0.f ? M + log2f(L) : -INFINITY;
+            if (FWD && l == 0) lse[(int64_t)hq * s.N + at.n] = L > 0.f ? M + log2f(L) : -INFINITY;
         }
         at.next(step, s.Hk, s.G);
     }
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
 }
 
 bool sel_merge_fits(const SelShape& s, int nsub) {
-    return s.D == 128 && s.T * nsub <= kMgSlots && s.N * s.Hq >= kMgRows && s.N * s.Hq < (1ll << 30);
+    return s.D <= 128 && s.T * nsub <= kMgSlots && s.N * s.Hq >= kMgRows && s.N * s.Hq < (1ll << 30);
 }
 
 template <int D, typename ET, bool FWD>
@@ -191,7 +192,7 @@ static cudaError_t merge(int dtype, const void* part, const float2* ml, const in
     if (s.D == DD)                                                                                                                              \
         return dtype == kBF16 ? launch_merge<DD, __nv_bfloat16, FWD>(part, ml, pos, s, nsub, out, o_sn, o_sh, lse, status, sms, stream)         \
                               : launch_merge<DD, __half, FWD>(part, ml, pos, s, nsub, out, o_sn, o_sh, lse, status, sms, stream);
-    FSA_CASE(128)
+    FSA_CASE(64) FSA_CASE(128)
 #undef FSA_CASE
     return cudaErrorInvalidValue;
 }

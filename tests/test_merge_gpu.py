@@ -13,7 +13,8 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("seqlens,Hk,G,T,d,bs,dtype", [([1499, 1000, 502], 2, 4, 16, 128, 64, "bf16"), ([2999, 1, 70], 1, 8, 9, 64, 32, "fp16"),
                                                        ([1300, 1333], 3, 4, 8, 128, 128, "bf16"), ([1100, 900], 2, 7, 4, 128, 256, "bf16"),
-                                                       ([1700, 1350], 8, 1, 3, 128, 64, "fp16")])
+                                                       ([1700, 1350], 8, 1, 3, 128, 64, "fp16"), ([2701, 2600], 1, 5, 16, 64, 64, "bf16"),
+                                                       ([1999, 1001, 1], 3, 3, 7, 64, 128, "fp16")])
 def test_resident_merge(seqlens, Hk, G, T, d, bs, dtype):
     N = sum(seqlens)
     assert N * Hk * G >= 24000 > max(seqlens) * Hk * G
