@@ -17,10 +17,13 @@
 //           A = ks / stride, BS = block_size / stride, w = histogram of i + j, i < A, j < BS                  (:1105-1115)
 //   bs[b] = +inf for b < init_blocks and for b <= t / block_size < b + local_blocks                           (:1068-1075)
 //   bs rounded to bf16                                                                                         (:1307-1308)
-// and keeps the best min(T, causal blocks) of its row in registers, ordered by (score descending, block ascending):
-// blocks arrive in ascending order, so a candidate only enters when it is strictly greater than the current worst
-// and bubbles up while strictly greater -- ties go to the lower block index (the reference leaves the tie order to
-// torch.topk).  Ascending ids, -1 tail (:1309-1313).
+// and keeps the best min(T, causal blocks) of its row in registers, ordered by (score descending, block ascending) -- ties
+// go to the lower block index (the reference leaves the tie order to torch.topk).  Ascending ids, -1 tail (:1309-1313).
+//
+// Score and block are one integer key (scores are >= 0, so their bf16 words order like them), and a candidate x enters the
+// descending list k by k[i] = max(k[i], min(k[i - 1], x)): two instructions a place, none of which waits for another or
+// branches.  Bubbling score and id up while greater was a chain of fifteen dependent steps that some lane of a warp nearly always
+// took, and bound the kernel: @@ us for 2 x 32768 tokens, 8 kv heads.
 //
 // Accumulation order of q.k: the tensor core's (products of 16-bit inputs are exact in fp32; the sums are not
 // associative), so a score can differ from another implementation's in its last bits, and an id can differ where two
@@ -31,6 +34,19 @@
 namespace fsa {
 
 int make_tile_map(CUtensorMap* map, const void* base, int dtype, int64_t rows, int64_t cols, int64_t row_stride, int box_rows);
+
+// WIDE: block ids beyond 16 bits (sequences of millions of tokens)
+template <bool WIDE> struct BlockKey;
+template <> struct BlockKey<false> {
+    using T = uint32_t;
+    __device__ static __forceinline__ T make(uint32_t score, int blk) { return score << 16 | (uint32_t)(0xffff - blk); }
+    __device__ static __forceinline__ int block(T k) { return 0xffff - (int)(k & 0xffffu); }
+};
+template <> struct BlockKey<true> {
+    using T = unsigned long long;
+    __device__ static __forceinline__ T make(uint32_t score, int blk) { return (T)score << 32 | (T)(0x7fffffff - blk); }
+    __device__ static __forceinline__ int block(T k) { return 0x7fffffff - (int)(k & 0x7fffffffu); }
+};
 
 struct SelFusedParams {
     const float* lse;        // [Hq, N] log2 units (compressed branch)
@@ -56,7 +72,7 @@ struct TapWeights {
     }
 };
 
-template <int D, typename ET, int A, int BS, int TL>
+template <int D, typename ET, int A, int BS, int TL, bool WIDE>
 __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedParams p, const __grid_constant__ CUtensorMap qmap,
                                                                const __grid_constant__ CUtensorMap kmap) {
     constexpr int kQ = kSfRows * D * 2, kK = kSfKeys * D * 2;
@@ -74,7 +90,7 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     const int tid = threadIdx.x, warp = tid >> 5;
     // which (sequence, query tile) is this CTA's (every warp finds it, 32 sequences per step)
     int b, n0, ne;
-    find_seq_tile(p.cu_q, p.B, kSfRows, (int)blockIdx.x, tid & 31, b, n0, ne);
+    find_seq_tile(p.cu_q, p.B, kSfRows, (int)(gridDim.x - 1 - blockIdx.x), tid & 31, b, n0, ne);      // (late tiles see the most keys: first)
     if (b < 0) return;
     const int h = blockIdx.y;
     const int L = __ldg(p.cu_q + b + 1) - __ldg(p.cu_q + b);
@@ -140,10 +156,10 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     const int nb = valid ? min(bq + 1, p.max_blocks) : 0;          // causal candidate blocks
     const float lse = nvis > 0 ? __ldg(p.lse + (int64_t)(h * p.G) * p.N + n0 + tid) : 0.f;
     const int nb_warp = __reduce_max_sync(0xffffffffu, nb);       // the TMEM loads below are warp-wide: uniform trip counts
-    float best_s[TL];
-    int best_i[TL];
+    using Key = typename BlockKey<WIDE>::T;
+    Key best[TL];
 #pragma unroll
-    for (int i = 0; i < TL; ++i) { best_s[i] = -1.f; best_i[i] = -1; }     // scores are >= 0
+    for (int i = 0; i < TL; ++i) best[i] = 0;              // (no block: below every key)
     float carry[PAD > 0 ? PAD : 1];
 #pragma unroll
     for (int i = 0; i < (PAD > 0 ? PAD : 1); ++i) carry[i] = 0.f;
@@ -186,23 +202,14 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
 #pragma unroll
             for (int j = 0; j < 32 / BS; ++j) {
                 const int blk = c0 / BS + j;
-                if (blk < nb) {
-                    float sc = 0.f;
+                float sc = 0.f;
 #pragma unroll
-                    for (int o = 0; o < NWT; ++o) sc = __fadd_rn(sc, __fmul_rn(pv[j * BS + o], TapWeights<A, BS>::w(o)));   // (no fused multiply-add: the order and rounding of the sum are part of the result)
-                    if (blk < p.init_blocks || (bq >= blk && bq < blk + p.local_blocks)) sc = INFINITY;
-                    sc = __bfloat162float(__float2bfloat16(sc));
-                    if (sc > best_s[TL - 1]) {
-                        best_s[TL - 1] = sc; best_i[TL - 1] = blk;
+                for (int o = 0; o < NWT; ++o) sc = __fadd_rn(sc, __fmul_rn(pv[j * BS + o], TapWeights<A, BS>::w(o)));   // (no fused multiply-add: the order and rounding of the sum are part of the result)
+                if (blk < p.init_blocks || (bq >= blk && bq < blk + p.local_blocks)) sc = INFINITY;
+                const Key x = blk < nb && sc >= 0.f ? BlockKey<WIDE>::make(__bfloat16_as_ushort(__float2bfloat16(sc)), blk) : (Key)0;
 #pragma unroll
-                        for (int i = TL - 1; i > 0; --i) {
-                            if (best_s[i] > best_s[i - 1]) {
-                                const float ts = best_s[i]; best_s[i] = best_s[i - 1]; best_s[i - 1] = ts;
-                                const int ti = best_i[i]; best_i[i] = best_i[i - 1]; best_i[i - 1] = ti;
-                            }
-                        }
-                    }
-                }
+                for (int i = TL - 1; i > 0; --i) best[i] = max(best[i], min(best[i - 1], x));
+                best[0] = max(best[0], x);
             }
         }
         tc_fence_before();
@@ -213,9 +220,9 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     if (valid) {
         // the first min(T_out, nb) entries are the selection; ascending ids, -1 tail
         const int nsel = min(p.T_out, nb);
+        int best_i[TL];
 #pragma unroll
-        for (int i = 0; i < TL; ++i)
-            if (i >= nsel) best_i[i] = 0x7fffffff;
+        for (int i = 0; i < TL; ++i) best_i[i] = i < nsel && best[i] != 0 ? BlockKey<WIDE>::block(best[i]) : 0x7fffffff;
 #pragma unroll
         for (int pass = 0; pass < TL; ++pass) {
 #pragma unroll
@@ -237,18 +244,12 @@ template <int D, typename ET, int A, int BS>
 static cudaError_t launch_tl(const SelFusedParams& p, const CUtensorMap& qmap, const CUtensorMap& kmap, int64_t n_items, cudaStream_t stream) {
     constexpr int smem = kSfRows * D * 2 + 2 * kSfKeys * D * 2 + 64;
     const dim3 grid((unsigned)n_items, (unsigned)p.Hk);
-    cudaError_t e;
-    if (p.T_out <= 16) {
-        auto kern = select_topk_fused_kernel<D, ET, A, BS, 16>;
-        e = allow_smem((const void*)kern, smem);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
-    } else {
-        auto kern = select_topk_fused_kernel<D, ET, A, BS, 32>;
-        e = allow_smem((const void*)kern, smem);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
-    }
+    const bool wide = p.max_blocks > 0xffff;
+    auto kern = p.T_out <= 16 ? (wide ? select_topk_fused_kernel<D, ET, A, BS, 16, true> : select_topk_fused_kernel<D, ET, A, BS, 16, false>)
+                              : (wide ? select_topk_fused_kernel<D, ET, A, BS, 32, true> : select_topk_fused_kernel<D, ET, A, BS, 32, false>);
+    const cudaError_t e = allow_smem((const void*)kern, smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, 128, smem, stream>>>(p, qmap, kmap);
     return cudaGetLastError();
 }
 
