@@ -9,8 +9,9 @@
 //
 // One CTA (128 threads) = 128 consecutive query tokens of one sequence x one KV head (the FIRST query head of the group
 // scores for the whole group, :897-912 with the slicing at :1280-1283).  The Q tile is loaded once by TMA; the
-// compressed keys of the sequence stream through a two-stage TMA ring in tiles of 128 keys; S = Q K^T (M = N = 128,
-// tcgen05, fp32 in one of two TMEM buffers) for tile kt + 1 is issued before tile kt is evaluated.  One thread owns one
+// compressed keys of the sequence stream through one TMA tile of 64 keys; S = Q K^T (M = 128, N = 64, tcgen05, fp32 in one
+// of two TMEM buffers) for tile kt + 1 is issued while tile kt is evaluated.  What bounds it is the evaluation, arithmetic of long
+// latency: 48 KB of shared memory, 128 TMEM columns and 128 registers a thread let four CTAs share an SM.  One thread owns one
 // query row:
 //   p[c]  = exp2(s[c] * scale * log2e - lse)   for visible c (t >= c * stride + ks - 1), else 0              (:897-912)
 //   bs[b] = sum_o w[o] * p[b * BS - (A - 1) + o], added in ascending o, out-of-range terms 0                  (:1046-1067)
@@ -23,7 +24,7 @@
 // Score and block are one integer key (scores are >= 0, so their bf16 words order like them), and a candidate x enters the
 // descending list k by k[i] = max(k[i], min(k[i - 1], x)): two instructions a place, none of which waits for another or
 // branches.  Bubbling score and id up while greater was a chain of fifteen dependent steps that some lane of a warp nearly always
-// took, and bound the kernel: @@ us for 2 x 32768 tokens, 8 kv heads.
+// took, and bound the kernel: 2 x 32768 tokens, 8 kv heads 1791 -> 1393 us, with four CTAs an SM instead of two 881 us.
 //
 // Accumulation order of q.k: the tensor core's (products of 16-bit inputs are exact in fp32; the sums are not
 // associative), so a score can differ from another implementation's in its last bits, and an id can differ where two
@@ -60,7 +61,7 @@ struct SelFusedParams {
     int* status;             // device status word or null
 };
 
-constexpr int kSfRows = 128, kSfKeys = 128;
+constexpr int kSfRows = 128, kSfKeys = 64;
 
 template <int A, int BS>
 struct TapWeights {
@@ -73,7 +74,7 @@ struct TapWeights {
 };
 
 template <int D, typename ET, int A, int BS, int TL, bool WIDE>
-__global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedParams p, const __grid_constant__ CUtensorMap qmap,
+__global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFusedParams p, const __grid_constant__ CUtensorMap qmap,
                                                                const __grid_constant__ CUtensorMap kmap) {
     constexpr int kQ = kSfRows * D * 2, kK = kSfKeys * D * 2;
     constexpr int PAD = A - 1, NWT = A + BS - 1;
@@ -81,11 +82,11 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + kQ;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sK + 2 * kK);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sK + kK);
     uint64_t* q_full = bars;          // [1]
-    uint64_t* k_full = bars + 1;      // [2]
-    uint64_t* s_full = bars + 3;      // [2]
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 5);
+    uint64_t* k_full = bars + 1;      // [1]
+    uint64_t* s_full = bars + 2;      // [2]
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 4);
 
     const int tid = threadIdx.x, warp = tid >> 5;
     // which (sequence, query tile) is this CTA's (every warp finds it, 32 sequences per step)
@@ -103,12 +104,13 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
 
     if (tid == 0) {
         mbar_init(q_full, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&s_full[i], 1); }
+        mbar_init(k_full, 1);
+        for (int i = 0; i < 2; ++i) mbar_init(&s_full[i], 1);
         mbar_init_fence();
         tma_prefetch_desc(&qmap);
         tma_prefetch_desc(&kmap);
     }
-    if (warp == 0) tmem_alloc(&tmem_slot, 256);
+    if (warp == 0) tmem_alloc(&tmem_slot, 2 * kSfKeys);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -116,11 +118,10 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
 
     auto load_k = [&](int kt) {
-        const int buf = kt & 1;
-        mbar_expect_tx(&k_full[buf], (uint32_t)kK);
+        mbar_expect_tx(k_full, (uint32_t)kK);
 #pragma unroll
         for (int sl = 0; sl < D / 64; ++sl)
-            tma_load_2d(smem_u32(sK + buf * kK + sl * kSfKeys * 128), &kmap, h * D + sl * 64, kbase + kt * kSfKeys, &k_full[buf]);
+            tma_load_2d(smem_u32(sK + sl * kSfKeys * 128), &kmap, h * D + sl * 64, kbase + kt * kSfKeys, k_full);
     };
     constexpr uint32_t idesc = umma_idesc(ElemTraits<ET>::kIsBF16, 128, kSfKeys, false, false);
     auto issue_mma = [&](int kt) {
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
             const uint32_t a = smem_u32(sQ + (ks >> 2) * (kSfRows * 128)) + (ks & 3) * 32;
-            const uint32_t bb = smem_u32(sK + buf * kK + (ks >> 2) * (kSfKeys * 128)) + (ks & 3) * 32;
+            const uint32_t bb = smem_u32(sK + (ks >> 2) * (kSfKeys * 128)) + (ks & 3) * 32;
             umma_ss(tbase + buf * kSfKeys, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(bb, 16, 1024), idesc, ks > 0);
         }
         umma_commit(&s_full[buf]);
@@ -141,9 +142,8 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
         for (int sl = 0; sl < D / 64; ++sl)
             tma_load_2d(smem_u32(sQ + sl * kSfRows * 128), &qmap, (h * p.G) * D + sl * 64, n0, q_full);
         load_k(0);
-        if (nkt > 1) load_k(1);
         ok = mbar_wait(q_full, 0, status) && ok;
-        ok = mbar_wait(&k_full[0], 0, status) && ok;
+        ok = mbar_wait(k_full, 0, status) && ok;
         tc_fence_after();
         issue_mma(0);
     }
@@ -166,56 +166,59 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
 
     for (int kt = 0; kt < nkt; ++kt) {
         const int buf = kt & 1;
-        // S(kt) done: its K stage is free; S(kt + 1) can be issued at once (its TMEM buffer was read in iteration kt - 1,
-        // before the barrier that ended it)
+        // S(kt) done: the K tile may be loaded over.  S(kt + 1) is issued between the two groups of columns of this tile: the keys have
+        // landed by then, and its TMEM buffer was read in iteration kt - 1, before the barrier that ended it
         if (have_keys) ok = mbar_wait(&s_full[buf], (kt >> 1) & 1, status) && ok;
         tc_fence_after();
-        if (tid == 0 && have_keys) {
-            if (kt + 1 < nkt) {
-                ok = mbar_wait(&k_full[buf ^ 1], ((kt + 1) >> 1) & 1, status) && ok;
-                tc_fence_after();
-                issue_mma(kt + 1);
-            }
-            if (kt + 2 < nkt) load_k(kt + 2);
-        }
+        if (tid == 0 && have_keys && kt + 1 < nkt) load_k(kt + 1);
         __syncwarp();
 #pragma unroll 1
         for (int c32 = 0; c32 < kSfKeys / 32; ++c32) {
             const int c0 = kt * kSfKeys + c32 * 32;      // first compressed token of this group of columns
-            if (c0 - PAD >= nb_warp * BS) break;         // no causal block of any row of this warp is left
-            uint32_t v[32];
-            if (have_keys) {
-                tmem_ld32(tbase + lane_off + buf * kSfKeys + c32 * 32, v);
-                tmem_ld_wait();
-            } else {
+            if (c0 - PAD < nb_warp * BS) {               // (else no causal block of any row of this warp is left)
+                uint32_t v[32];
+                if (have_keys) {
+                    tmem_ld32(tbase + lane_off + buf * kSfKeys + c32 * 32, v);
+                    tmem_ld_wait();
+                } else {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = 0u;
+                    for (int i = 0; i < 32; ++i) v[i] = 0u;
+                }
+                float pv[PAD + 32];
+#pragma unroll
+                for (int i = 0; i < PAD; ++i) pv[i] = carry[i];
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    pv[PAD + i] = (c0 + i < nvis) ? exp2f(fmaf(__uint_as_float(v[i]), p.scale_log2, -lse)) : 0.f;
+#pragma unroll
+                for (int i = 0; i < PAD; ++i) carry[i] = pv[32 + i];
+#pragma unroll
+                for (int j = 0; j < 32 / BS; ++j) {
+                    const int blk = c0 / BS + j;
+                    float sc = 0.f;
+#pragma unroll
+                    for (int o = 0; o < NWT; ++o) sc = __fadd_rn(sc, __fmul_rn(pv[j * BS + o], TapWeights<A, BS>::w(o)));   // (no fused multiply-add: the order and rounding of the sum are part of the result)
+                    if (blk < p.init_blocks || (bq >= blk && bq < blk + p.local_blocks)) sc = INFINITY;
+                    const Key x = blk < nb && sc >= 0.f ? BlockKey<WIDE>::make(__bfloat16_as_ushort(__float2bfloat16(sc)), blk) : (Key)0;
+#pragma unroll
+                    for (int i = TL - 1; i > 0; --i) best[i] = max(best[i], min(best[i - 1], x));
+                    best[0] = max(best[0], x);
+                }
             }
-            float pv[PAD + 32];
-#pragma unroll
-            for (int i = 0; i < PAD; ++i) pv[i] = carry[i];
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                pv[PAD + i] = (c0 + i < nvis) ? exp2f(fmaf(__uint_as_float(v[i]), p.scale_log2, -lse)) : 0.f;
-#pragma unroll
-            for (int i = 0; i < PAD; ++i) carry[i] = pv[32 + i];
-#pragma unroll
-            for (int j = 0; j < 32 / BS; ++j) {
-                const int blk = c0 / BS + j;
-                float sc = 0.f;
-#pragma unroll
-                for (int o = 0; o < NWT; ++o) sc = __fadd_rn(sc, __fmul_rn(pv[j * BS + o], TapWeights<A, BS>::w(o)));   // (no fused multiply-add: the order and rounding of the sum are part of the result)
-                if (blk < p.init_blocks || (bq >= blk && bq < blk + p.local_blocks)) sc = INFINITY;
-                const Key x = blk < nb && sc >= 0.f ? BlockKey<WIDE>::make(__bfloat16_as_ushort(__float2bfloat16(sc)), blk) : (Key)0;
-#pragma unroll
-                for (int i = TL - 1; i > 0; --i) best[i] = max(best[i], min(best[i - 1], x));
-                best[0] = max(best[0], x);
+            if (c32 == 0 && tid == 0 && have_keys && kt + 1 < nkt) {
+                ok = mbar_wait(k_full, (kt + 1) & 1, status) && ok;
+                tc_fence_after();
+                issue_mma(kt + 1);
             }
+            __syncwarp();
         }
         tc_fence_before();
         ok = __syncthreads_and(ok);
         if (!ok) break;
     }
+    // (on a wait that ran out: a key tile in flight lands before the CTA ends)
+    if (!ok && tid == 0 && have_keys)
+        for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait(k_full, ph, nullptr);
 
     if (valid) {
         // the first min(T_out, nb) entries are the selection; ascending ids, -1 tail
@@ -237,12 +240,12 @@ __global__ void __launch_bounds__(128) select_topk_fused_kernel(const SelFusedPa
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, 256);
+    if (warp == 0) tmem_dealloc(tbase, 2 * kSfKeys);
 }
 
 template <int D, typename ET, int A, int BS>
 static cudaError_t launch_tl(const SelFusedParams& p, const CUtensorMap& qmap, const CUtensorMap& kmap, int64_t n_items, cudaStream_t stream) {
-    constexpr int smem = kSfRows * D * 2 + 2 * kSfKeys * D * 2 + 64;
+    constexpr int smem = kSfRows * D * 2 + kSfKeys * D * 2 + 64;
     const dim3 grid((unsigned)n_items, (unsigned)p.Hk);
     const bool wide = p.max_blocks > 0xffff;
     auto kern = p.T_out <= 16 ? (wide ? select_topk_fused_kernel<D, ET, A, BS, 16, true> : select_topk_fused_kernel<D, ET, A, BS, 16, false>)
