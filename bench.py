@@ -782,7 +782,7 @@ def run_sel(args, dd):
                      "overlap": "copies of step i+1 on a second stream while step i computes"} if e2e_ms else None),
             # kernels of this library per step: 5 of the index build, forward main + merge, delta, backward main,
             # dQ merge, dK/dV slab reduce (the two memsets of dk / dv are not kernels)
-            "gpu_launches": 11 * args.steps,
+            "gpu_launches": 10 * args.steps,
             "clocks": clocks,
         }
     del qd, kd, vd, dod, idxd, dev_bufs, host

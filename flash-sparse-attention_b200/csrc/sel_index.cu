@@ -12,9 +12,9 @@
 //   2. keys    one thread per (kv head, block): exclusive prefix of chunk_cnt over the chunks (every chunk's first
 //              position inside the key) and the key's total;
 //   3. scan    one CTA: first tile and first segment of every key;
-//   4. tiles   one warp per key: tile records, padding of the last tile;
-//   5. fill    the CTAs of step 1 again: the same counting pass gives every warp its first position inside each key,
-//              a second pass over the same tokens writes entries and positions.
+//   4. fill    the CTAs of step 1 again: tile records and the padding of a key's last tile (a warp per key); then every warp's
+//              first position inside each key is known, and a second pass over the same tokens writes entries and positions.
+// Where a thread has few chunks to add up, step 3 does step 2 as well (a launch costs about 4 us of a short build).
 // Entries of a key are in ascending order of (chunk, warp range, 32-token group): ascending token groups, and inside a group
 // ascending tokens (short lists without repeated ids), else slot by slot.
 // Short problems run all steps in one launch (sel_index_small).
@@ -158,13 +158,26 @@ __device__ __forceinline__ void chunk_pass(const int* __restrict__ topk_idx, con
     }
 }
 
+// Tile records of one key (a warp), and the unused slots of its last tile.
+__device__ __forceinline__ void write_tiles(const SelShape& s, const SelIndex& ix, const int* __restrict__ ck, int h, int gb, int cnt,
+                                            int t0, int seg0, int lane) {
+    const int hg = h * s.NBmax + gb, nt = (cnt + s.TPT - 1) / s.TPT;
+    const int row0 = block_rows(ck, s.B, s.BK, gb).x;
+    for (int t = lane; t < nt; t += 32) {
+        ix.tile_rec[t0 + t] = make_int4(row0, min(s.TPT, cnt - t * s.TPT) | (h << 8), hg, seg0);
+        ix.tile_aux[t0 + t] = make_int2(t0, nt);
+    }
+    const int used = cnt - (nt - 1) * s.TPT;
+    for (int e = used + lane; e < s.TPT; e += 32) ix.entries[(int64_t)(t0 + nt - 1) * s.TPT + e] = 0xFFFFFFFFu;
+}
+
 // Is there room for the words of lane bits?
 constexpr int kIdxSmem = 200 * 1024;
 __host__ __device__ __forceinline__ bool sel_index_masks(const SelShape& s, int nwarps) {
     return (int64_t)nwarps * s.NBmax * 8 <= kIdxSmem && s.T <= kIdxMaxSlots;
 }
 
-// Step 1 (FILL = false) and step 5 (FILL = true).
+// Step 1 (FILL = false) and step 4 (FILL = true).
 template <bool FILL>
 __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* __restrict__ topk_idx, const int* __restrict__ cu,
                                                                      SelBounds bd, SelShape s, SelIndex ix) {
@@ -189,6 +202,12 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
             cc[gb] = run;
         }
     } else {
+        // the tile records of this warp's share of the keys
+        const int* ck = bd.cu_k ? bd.cu_k : cu;
+        for (int gb = c * nwarps + warp; gb < s.NBmax; gb += gridDim.x * nwarps) {
+            const int hg = h * s.NBmax + gb, cnt = ix.key_cnt[hg];
+            if (cnt > 0) write_tiles(s, ix, ck, h, gb, cnt, ix.key_tile[hg], ix.key_seg[hg], lane);
+        }
         // every warp's first position in the tile-ordered entry list: first entry of the key (step 3) + the chunk's first
         // position inside the key (step 2) + the warp's inside the chunk (step 1)
         const int* kt = ix.key_tile + (int64_t)h * s.NBmax;
@@ -204,10 +223,8 @@ __global__ void __launch_bounds__(kIdxMaxWarps * 32) sel_index_chunk(const int* 
     }
 }
 
-// Step 2: per key, exclusive prefix of the chunks' counts and the total (thread per key; eight loads in flight).
-__global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= s.Hk * s.NBmax) return;
+// Exclusive prefix of the chunks' counts of one key, and the total (eight loads in flight).
+__device__ __forceinline__ int prefix_chunks(const SelShape& s, const SelIndex& ix, int k) {
     const int h = k / s.NBmax, gb = k - h * s.NBmax;
     int* p = ix.chunk_cnt + (int64_t)h * s.NC * s.NBmax + gb;
     int run = 0;
@@ -221,11 +238,19 @@ __global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
             run += v[j];
         }
     }
-    ix.key_cnt[k] = run;
+    return run;
+}
+
+// Step 2: per key, exclusive prefix of the chunks' counts and the total (thread per key; eight loads in flight).
+__global__ void __launch_bounds__(64) sel_index_keys(SelShape s, SelIndex ix) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= s.Hk * s.NBmax) return;
+    ix.key_cnt[k] = prefix_chunks(s, ix, k);
 }
 
 // Step 3: exclusive scans over the keys (a single CTA): first tile, then -- it depends on the first tile -- first segment.
 // A key with tiles [t0, t0 + nt) is cut by the backward's schedule at every multiple of RB.
+template <bool KEYS>
 __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) {
     __shared__ int wsum_a[32], wsum_b[32], wsum_c[32];
     __shared__ int carry_a, carry_b, carry_c;
@@ -235,7 +260,8 @@ __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) 
     __syncthreads();
     for (int base = 0; base < HG; base += 1024) {
         const int i = base + tid;
-        const int a = i < HG ? ix.key_cnt[i] : 0;
+        const int a = i >= HG ? 0 : KEYS ? prefix_chunks(s, ix, i) : ix.key_cnt[i];
+        if (KEYS && i < HG) ix.key_cnt[i] = a;
         const int b = (a + s.TPT - 1) / s.TPT;
         int sa = a, sb = b;
         for (int o = 1; o < 32; o <<= 1) {
@@ -289,37 +315,13 @@ __global__ void __launch_bounds__(1024) sel_index_scan(SelShape s, SelIndex ix) 
     }
 }
 
-// Tile records of one key (a warp), and the unused slots of its last tile.
-__device__ __forceinline__ void write_tiles(const SelShape& s, const SelIndex& ix, const int* __restrict__ ck, int h, int gb, int cnt,
-                                            int t0, int seg0, int lane) {
-    const int hg = h * s.NBmax + gb, nt = (cnt + s.TPT - 1) / s.TPT;
-    const int row0 = block_rows(ck, s.B, s.BK, gb).x;
-    for (int t = lane; t < nt; t += 32) {
-        ix.tile_rec[t0 + t] = make_int4(row0, min(s.TPT, cnt - t * s.TPT) | (h << 8), hg, seg0);
-        ix.tile_aux[t0 + t] = make_int2(t0, nt);
-    }
-    const int used = cnt - (nt - 1) * s.TPT;
-    for (int e = used + lane; e < s.TPT; e += 32) ix.entries[(int64_t)(t0 + nt - 1) * s.TPT + e] = 0xFFFFFFFFu;
-}
-
-// Step 4: tile records and the padding of the tile-ordered entry list: one warp per key.
-__global__ void __launch_bounds__(256) sel_index_tiles(const int* __restrict__ cu, SelBounds bd, SelShape s, SelIndex ix) {
-    const int lane = threadIdx.x & 31;
-    const int hg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (hg >= s.Hk * s.NBmax) return;
-    const int cnt = ix.key_cnt[hg];
-    if (cnt == 0) return;
-    const int h = hg / s.NBmax;
-    write_tiles(s, ix, bd.cu_k ? bd.cu_k : cu, h, hg - h * s.NBmax, cnt, ix.key_tile[hg], ix.key_seg[hg], lane);
-}
-
-// All five steps in one launch, for short problems: one CTA per kv head, the CTAs of a cluster exchange the numbers of tiles
+// All steps in one launch, for short problems: one CTA per kv head, the CTAs of a cluster exchange the numbers of tiles
 // and segments of their heads through distributed shared memory.  What bounds a short build is the latency of its launches
 // and dependent steps: 512 tokens x 2 heads took 24 us in five kernels and a memset.  The list is the same one (a warp takes
 // a contiguous range of 32-token groups either way).  A head's entries all leave through one SM, scattered, at about one a clock:
-// used up to kSmallEntries of them (6 us + 1.1 ns each, against 28 us for the five launches), and up to 8 heads (the cluster) and
+// used up to kSmallEntries of them (6 us + 1.1 ns each, against 20-28 us for the launches of the steps), and up to 8 heads (the cluster) and
 // kSmallKeys blocks (a thread each).
-constexpr int kSmallEntries = 20000, kSmallKeys = 700, kSmallWarps = 32;
+constexpr int kSmallEntries = 16000, kSmallKeys = 700, kSmallWarps = 32;
 
 // Exclusive prefix of v over the CTA's 1024 threads; *total = the sum.
 __device__ __forceinline__ int cta_prefix(int v, int* wsum, int tid, int* total) {
@@ -446,9 +448,12 @@ cudaError_t sel_build_index(const int* topk_idx, const int* cu, const SelBounds&
     const dim3 grid((unsigned)s.NC, (unsigned)s.Hk);
     const int HG = s.Hk * s.NBmax;
     sel_index_chunk<false><<<grid, nw * 32, smem, stream>>>(topk_idx, cu, bd, s, ix);
-    sel_index_keys<<<(unsigned)((HG + 63) / 64), 64, 0, stream>>>(s, ix);
-    sel_index_scan<<<1, 1024, 0, stream>>>(s, ix);
-    sel_index_tiles<<<(unsigned)((HG + 7) / 8), 256, 0, stream>>>(cu, bd, s, ix);
+    if ((HG + 1023) / 1024 * s.NC <= 16) {                  // (two rounds of loads a thread)
+        sel_index_scan<true><<<1, 1024, 0, stream>>>(s, ix);
+    } else {
+        sel_index_keys<<<(unsigned)((HG + 63) / 64), 64, 0, stream>>>(s, ix);
+        sel_index_scan<false><<<1, 1024, 0, stream>>>(s, ix);
+    }
     sel_index_chunk<true><<<grid, nw * 32, smem_fill, stream>>>(topk_idx, cu, bd, s, ix);
     return cudaGetLastError();
 }
