@@ -238,9 +238,10 @@ __global__ void __launch_bounds__(256) gate_proj_mix_fwd_kernel(const ET* __rest
 
 // Backward, per token: da = g0 do, db = g1 do, dc = g2 do; dg_j = sum(do * branch_j) rounded; dz_j = dg_j g_j (1 - g_j)
 // rounded (the sigmoid's backward in the activation dtype); dx[n, :] = sum_j dz_j Wg[j, :]; dz kept in fp32 for dWg.
-// HV > 0: heads of HV 16-byte vectors; delta[j, h, n] = g_j sum over head h of do * branch_j, which is the sum of o dO that the
+// HV > 0: heads of HV 16-byte vectors; delta[j, h, n] = sum over head h of branch_j * (da, db, dc), which is the sum of o dO that the
 // attention backward of branch j starts from (three passes over o and dO of their own otherwise: 0.79 ms of 64K tokens x 32
-// heads).
+// heads).  It is summed from the gradient as it is stored: that is the dO whose products the attention backward subtracts it from, and
+// with another one the dS of a row no longer sum to zero (a token that sees one key gets a dq).
 template <int HV, typename ET>
 __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __restrict__ gate, const ET* __restrict__ wg,
                                                                 const ET* __restrict__ a, const ET* __restrict__ b,
@@ -276,21 +277,28 @@ __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __rest
                 if (v >= vec) continue;
                 const int64_t idx = n * vec + v;
                 const uint32_t *pd = &vd[u].x, *pa = &va[u].x, *pb = &vb[u].x, *pc = &vc[u].x;
-                float h0 = 0.f, h1 = 0.f, h2 = 0.f;       // this vector's share of its head
+                float t0 = 0.f, t1 = 0.f, t2 = 0.f;       // this vector's share of the gate's gradient
+                float h0 = 0.f, h1 = 0.f, h2 = 0.f;       // ... and of its head's delta
                 uint4 oa, ob, oc;
                 uint32_t *qa = &oa.x, *qb = &ob.x, *qc = &oc.x;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     float2 d = ElemTraits<ET>::unpack2(pd[i]);
                     float2 p = ElemTraits<ET>::unpack2(pa[i]), q = ElemTraits<ET>::unpack2(pb[i]), r = ElemTraits<ET>::unpack2(pc[i]);
-                    h0 += d.x * p.x + d.y * p.y;
-                    h1 += d.x * q.x + d.y * q.y;
-                    h2 += d.x * r.x + d.y * r.y;
+                    t0 += d.x * p.x + d.y * p.y;
+                    t1 += d.x * q.x + d.y * q.y;
+                    t2 += d.x * r.x + d.y * r.y;
                     qa[i] = ElemTraits<ET>::pack2(g0 * d.x, g0 * d.y);
                     qb[i] = ElemTraits<ET>::pack2(g1 * d.x, g1 * d.y);
                     qc[i] = ElemTraits<ET>::pack2(g2 * d.x, g2 * d.y);
+                    if constexpr (HV > 0) {
+                        const float2 u = ElemTraits<ET>::unpack2(qa[i]), w = ElemTraits<ET>::unpack2(qb[i]), z = ElemTraits<ET>::unpack2(qc[i]);
+                        h0 += u.x * p.x + u.y * p.y;
+                        h1 += w.x * q.x + w.y * q.y;
+                        h2 += z.x * r.x + z.y * r.y;
+                    }
                 }
-                s0 += h0; s1 += h1; s2 += h2;
+                s0 += t0; s1 += t1; s2 += t2;
                 if constexpr (HV > 0) {
                     // (vec is a multiple of HV and HV divides 32: a head's vectors sit in neighbouring lanes of one iteration)
                     const unsigned mask = HV == 32 ? 0xffffffffu : ((1u << HV) - 1) << (lane & ~(HV - 1));
@@ -302,9 +310,9 @@ __global__ void __launch_bounds__(256) gate_proj_mix_bwd_kernel(const ET* __rest
                     }
                     if ((lane & (HV - 1)) == 0) {
                         const int64_t head = v / HV, heads = vec / HV;
-                        delta[head * N + n] = g0 * h0;
-                        delta[(heads + head) * N + n] = g1 * h1;
-                        delta[(2 * heads + head) * N + n] = g2 * h2;
+                        delta[head * N + n] = h0;
+                        delta[(heads + head) * N + n] = h1;
+                        delta[(2 * heads + head) * N + n] = h2;
                     }
                 }
                 st_stream16(reinterpret_cast<uint4*>(da) + idx, oa);

@@ -308,7 +308,8 @@ int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* dq2, const 
                        const int32_t* cu_seqlens, const int32_t* cu_cmp, int batch, int64_t total, int64_t total_cmp, int num_q_heads,
                        int num_kv_heads, int head_dim, int kernel_stride, int dtype, void* dq, void* dk, void* dv, void* stream);
 
-/* fsa_gate_proj_mix_bwd that also gives delta [3][num_heads][total] fp32, the sum of o dO over every head of every branch. */
+/* fsa_gate_proj_mix_bwd that also gives delta [3][num_heads][total] fp32, the sum of o dO over every head of every branch (dO: the
+ * branch's gradient as it is stored). */
 int fsa_gate_proj_mix_bwd_delta(const void* x, int64_t x_stride_n, const void* w_gate, const void* gate, const void* a, const void* b,
                                 const void* c, const void* d_out, int64_t total, int hidden, int num_heads, int head_dim, int dtype,
                                 void* da, void* db, void* dc, void* dx, void* dw_gate, float* delta, float* scratch,

@@ -9,6 +9,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from fsa import _lib
 from fsa.ops.gate import gate_mix, gate_proj_mix
 
 DEV = "cuda:0"
@@ -51,3 +52,26 @@ def test_gate_proj_mix_matches_modules(N, hidden, H, d, dtype):
     out2 = gate_proj_mix(xg, wg, a, b, c)
     out2.backward(dout)
     assert torch.equal(out2, out) and torch.equal(xg.grad, xf.grad) and torch.equal(wg.grad, wf.grad)
+
+
+@pytest.mark.parametrize("N,hidden,H,d,dtype", [(1, 256, 1, 64, torch.bfloat16), (333, 512, 3, 128, torch.bfloat16), (77, 256, 5, 64, torch.float16),
+                                                (600, 1024, 16, 128, torch.float16)])
+def test_delta_is_the_sum_over_the_stored_gradient(N, hidden, H, d, dtype):
+    """delta[j, h, n] = sum_d branch_j * (the gradient of branch_j as it was rounded and stored): the products of 16-bit values
+    are exact in fp32, so the sum of d of them, in any order, is off by less than d * 2^-24 of the sum of their magnitudes."""
+    g = torch.Generator(device=DEV).manual_seed(N + d)
+    x, a, b, c, dout = (torch.randn(s, device=DEV, generator=g).to(dtype) for s in ((N, hidden), (N, H, d), (N, H, d), (N, H, d), (N, H, d)))
+    w = (torch.randn(3, hidden, device=DEV, generator=g) * hidden ** -0.5).to(dtype)
+    gate = torch.sigmoid(x.float() @ w.float().t()).to(dtype)
+    da, db, dc, dx, dw = (torch.empty_like(t) for t in (a, b, c, x, w))
+    delta = torch.empty(3, H, N, device=DEV)
+    L = _lib.lib()
+    scratch = torch.empty(max(int(L.fsa_gate_proj_mix_scratch_bytes(N, hidden)), 16), dtype=torch.uint8, device=DEV)
+    _lib.check(L.fsa_gate_proj_mix_bwd_delta(_lib.ptr(x), x.stride(0), _lib.ptr(w), _lib.ptr(gate), _lib.ptr(a), _lib.ptr(b), _lib.ptr(c),
+                                             _lib.ptr(dout), N, hidden, H, d, _lib.DTYPE_CODE[dtype], _lib.ptr(da), _lib.ptr(db), _lib.ptr(dc),
+                                             _lib.ptr(dx), _lib.ptr(dw), _lib.ptr(delta), _lib.ptr(scratch), scratch.numel(),
+                                             _lib.current_stream(x.device)), "fsa_gate_proj_mix_bwd_delta")
+    for j, (o, do) in enumerate(((a, da), (b, db), (c, dc))):
+        terms = o.double() * do.double()
+        err = (delta[j].double() - terms.sum(-1).t()).abs()
+        assert bool((err <= d * 2.0 ** -24 * terms.abs().sum(-1).t()).all()), f"branch {j}: {float(err.max()):.3e}"
