@@ -68,6 +68,11 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd_delta(const Tensor& q, const Tensor& 
                                                  const float* delta, const Tensor& idx, int64_t bs, const Tensor& cu, double scale,
                                                  const Tensor& ws);
 
+// FSA_CHECK_STATUS=1: after their launches the operators read the status words of their kernels (one synchronisation each) and
+// raise when a bounded wait ran out.
+bool checking_status();
+void check_status(const void* word, const Tensor& like, const char* what);
+
 void bind_sel(pybind11::module& m);
 void bind_decode(pybind11::module& m);
 void bind_layer(pybind11::module& m);

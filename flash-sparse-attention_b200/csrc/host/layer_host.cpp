@@ -39,12 +39,12 @@ struct Kept {
 };
 
 static std::pair<Tensor, Tensor> range_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, const int32_t* lo,
-                                           const int32_t* hi, float scale) {
+                                           const int32_t* hi, float scale, int32_t* status) {
     const int64_t N = q.size(0);
     Tensor o = fresh_like(q), lse = f32({q.size(1), N}, q);
     check(fsa_range_attn_fwd_dense(ptr(q), ptr(k), ptr(v), iptr(cu_q), iptr(cu_k), lo, hi, N, k.size(0), (int)cu_q.size(0) - 1, (int)q.size(1),
                                    (int)k.size(1), (int)q.size(2), dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), scale, ptr(o),
-                                   o.stride(0), o.stride(1), lse.data_ptr<float>(), nullptr, stream_of(q)),
+                                   o.stride(0), o.stride(1), lse.data_ptr<float>(), status, stream_of(q)),
           "fsa_range_attn_fwd_dense");
     return {o, lse};
 }
@@ -56,6 +56,8 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     const int dt = dtype_code(x);
     const float scale = (float)(1.0 / std::sqrt((double)c.D));
     void* st = stream_of(x);
+    const Tensor word = checking_status() ? at::zeros({4}, x.options().dtype(at::kInt)) : Tensor();
+    int32_t* status = word.defined() ? word.data_ptr<int32_t>() : nullptr;      // one for the two ranges and the selection
     t.cs = fresh({s.max_len, c.D / 2}, x);
     t.sn = fresh({s.max_len, c.D / 2}, x);
     t.cu_cmp = i32({s.B + 1}, x);
@@ -72,6 +74,7 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
         check(fsa_compress_kv_fwd(ptr(t.k_raw), t.k_raw.stride(0), ptr(t.v), t.v.stride(0), ptr(w_key), ptr(w_value), ptr(pe), s.tok.data(), s.B, c.Hk,
                                   c.D, c.ks, c.stride, dt, ptr(t.ck), ptr(t.cv), (float*)ptr(scratch), st),
               "fsa_compress_kv_fwd");
+        check_status((char*)ptr(scratch) + scratch.numel() - 16, x, "fsa_compress_kv_fwd status");
     }
     t.k = fresh_like(t.k_raw);
     t.bounds = i32({3, N}, x);
@@ -79,20 +82,22 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     check(fsa_layer_rope_fwd(ptr(t.q), t.q.stride(0), ptr(t.k_raw), t.k_raw.stride(0), ptr(t.ck), ptr(t.cs), ptr(t.sn), iptr(cu), iptr(t.cu_cmp), s.B,
                              N, s.Nc, c.Hq, c.Hk, c.D, c.ks, c.stride, c.window, dt, ptr(t.q), ptr(t.k), bd, bd + N, bd + 2 * N, st),
           "fsa_layer_rope_fwd");
-    std::tie(t.o_cmp, t.lse_cmp) = range_fwd(t.q, t.ck, t.cv, cu, t.cu_cmp, nullptr, bd, scale);
+    std::tie(t.o_cmp, t.lse_cmp) = range_fwd(t.q, t.ck, t.cv, cu, t.cu_cmp, nullptr, bd, scale, status);
     const int max_blocks = (s.max_len + c.bs - 1) / c.bs, t_out = std::min(c.topk, max_blocks);
     t.topk = i32({c.Hk, N, t_out}, x);
     check(fsa_select_topk_fused(ptr(t.q), t.q.stride(0), ptr(t.ck), t.ck.stride(0), t.lse_cmp.data_ptr<float>(), iptr(cu), iptr(t.cu_cmp), N, s.Nc,
                                 s.B, c.Hq, c.Hk, c.D, dt, scale, c.ks, c.stride, c.bs, c.init_blocks, c.local_blocks, max_blocks, t_out,
-                                t.topk.data_ptr<int32_t>(), nullptr, st),
+                                t.topk.data_ptr<int32_t>(), status, st),
           "fsa_select_topk_fused");
     std::tie(t.o_sel, t.lse_sel, t.ws) = sel_fwd(t.q, t.k, t.v, t.topk, c.bs, cu, scale);
-    std::tie(t.o_win, t.lse_win) = range_fwd(t.q, t.k, t.v, cu, cu, bd + N, bd + 2 * N, scale);
+    std::tie(t.o_win, t.lse_win) = range_fwd(t.q, t.k, t.v, cu, cu, bd + N, bd + 2 * N, scale, status);
     t.gate = fresh({N, 3}, x);
     Tensor out = fresh({N, (int64_t)c.Hq * c.D}, x);
     check(fsa_gate_proj_mix_fwd(ptr(x), x.stride(0), ptr(wg), ptr(t.o_cmp), ptr(t.o_sel), ptr(t.o_win), N, (int)hidden, c.Hq * c.D, dt, ptr(out),
                                 ptr(t.gate), st),
           "fsa_gate_proj_mix_fwd");
+    check_status(ptr(t.ws), x, "fsa_sel_fwd status");
+    check_status(status, x, "range attention and block selection status");
     return out;
 }
 
@@ -112,6 +117,7 @@ static std::tuple<Tensor, Tensor, Tensor> range_bwd(const Tensor& q, const Tenso
                                    max_blocks, 64, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1),
                                    scale, ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
           "fsa_range_attn_bwd_delta");
+    check_status(ptr(ws), q, "fsa_range_attn_bwd_delta status");
     return {dq, dk, dv};
 }
 
@@ -164,6 +170,7 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         auto [dq0, dck, dcv] = range_bwd(q, ck, cv, lse_cmp, d_cmp, dl, cu, cu_cmp, nullptr, bd, s.cmp_blocks(), scale);
         d_cmp.reset();
         auto [dq1, dk, dv] = sel_bwd_delta(q, k, v, lse_sel, d_sel, dl + (int64_t)c.Hq * N, topk, c.bs, cu, scale, ws);
+        check_status(ptr(ws), q, "fsa_sel_bwd_delta status");
         d_sel.reset();
         auto [dq2, dk2, dv2] = range_bwd(q, k, v, lse_win, d_win, dl + 2 * (int64_t)c.Hq * N, cu, cu, bd + N, bd + 2 * N, s.win_blocks(c), scale);
         d_win.reset();
@@ -181,6 +188,7 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
                                       s.tok.data(), s.B, c.Hk, c.D, c.ks, c.stride, dt, ptr(dkc), ptr(dvc), ptr(dw_key), ptr(dw_value), ptr(dpe),
                                       (float*)ptr(scratch), st),
                   "fsa_compress_kv_bwd");
+            check_status((char*)ptr(scratch) + scratch.numel() - 16, x, "fsa_compress_kv_bwd status");
             rope_bwd(N, 0, dkc, dvc);
         }
         dq1.reset(); dq2.reset(); dk2.reset(); dv2.reset(); dck.reset(); dcv.reset();

@@ -67,21 +67,25 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd_delta(const Tensor& q, const Tensor& 
     return {dq, dk, dv};
 }
 
-static void check_status(const Tensor& ws, const char* what) {
+bool checking_status() {
     static const bool on = [] {
         const char* v = getenv("FSA_CHECK_STATUS");
         return v && v[0] == '1' && !v[1];
     }();
-    if (!on) return;
+    return on;
+}
+
+void check_status(const void* word, const Tensor& like, const char* what) {
+    if (!checking_status()) return;
     int st = 0;
-    check(fsa_read_status(ptr(ws), stream_of(ws), &st), what);
+    check(fsa_read_status(word, stream_of(like), &st), what);
 }
 
 struct SelAttention : torch::autograd::Function<SelAttention> {
     static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
                           const Tensor& cu, int64_t bs, double scale) {
         auto [o, lse, ws] = sel_fwd(q, k, v, idx, bs, cu, scale);
-        check_status(ws, "fsa_sel_fwd status");
+        check_status(ptr(ws), q, "fsa_sel_fwd status");
         ctx->save_for_backward({q, k, v, o, lse, idx, cu, ws});
         ctx->saved_data["bs"] = bs;
         ctx->saved_data["scale"] = scale;
@@ -91,7 +95,7 @@ struct SelAttention : torch::autograd::Function<SelAttention> {
         const auto t = ctx->get_saved_variables();
         auto [dq, dk, dv] = sel_bwd(t[0], t[1], t[2], t[3], t[4], g[0], t[5], ctx->saved_data["bs"].toInt(), t[6],
                                     ctx->saved_data["scale"].toDouble(), t[7]);
-        check_status(t[7], "fsa_sel_bwd status");
+        check_status(ptr(t[7]), t[0], "fsa_sel_bwd status");
         return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
@@ -99,7 +103,7 @@ struct SelAttention : torch::autograd::Function<SelAttention> {
 Tensor sel_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, int64_t bs, const Tensor& cu, double scale) {
     if (wants_grad({&q, &k, &v})) return SelAttention::apply(q, k, v, idx, cu, bs, scale);
     auto [o, lse, ws] = sel_fwd(q, k, v, idx, bs, cu, scale);
-    check_status(ws, "fsa_sel_fwd status");
+    check_status(ptr(ws), q, "fsa_sel_fwd status");
     return o;
 }
 

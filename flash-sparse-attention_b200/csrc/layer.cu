@@ -160,12 +160,13 @@ __global__ void __launch_bounds__(256) layer_rope_kernel(const LayerRopeParams p
 }
 
 // Partial column sums over contiguous shares of the rows, out[part, h, :] = sum of dy[row, h, :] (fp32, fixed order): the
-// gradient of the compressor's bias, finished by its consumer.
+// gradient of the compressor's bias, finished by its consumer (whose status word is cleared here).
 template <int D, typename ET>
-__global__ void __launch_bounds__(256) column_sum_kernel(const ET* __restrict__ dy, int64_t rows, int H, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) column_sum_kernel(const ET* __restrict__ dy, int64_t rows, int H, float* __restrict__ out, int* __restrict__ status) {
     constexpr int CG = D / 8, KL = 256 / CG;
     __shared__ float red[8][D];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cgi = tid % CG, kl = tid / CG, h = blockIdx.x;
+    if (tid == 0 && h == 0 && blockIdx.y == 0) *status = kStatusOk;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const int64_t per = (rows + gridDim.y - 1) / gridDim.y, r1 = min(rows, per * (blockIdx.y + 1));
 #pragma unroll 4
@@ -250,14 +251,14 @@ extern "C" int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* 
 
 // partial column sums [parts][H][D]; called by the compressor's backward
 namespace fsa {
-cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, cudaStream_t stream) {
+cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, int* status, cudaStream_t stream) {
     const dim3 grid((unsigned)H, (unsigned)parts);
     if (dtype == FSA_DTYPE_BF16) {
-        if (D == 128) column_sum_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out);
-        else column_sum_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out);
+        if (D == 128) column_sum_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out, status);
+        else column_sum_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, rows, H, out, status);
     } else {
-        if (D == 128) column_sum_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out);
-        else column_sum_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out);
+        if (D == 128) column_sum_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out, status);
+        else column_sum_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)dy, rows, H, out, status);
     }
     return cudaGetLastError();
 }

@@ -217,10 +217,12 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
 constexpr int kPeParts = 16;
 
 template <int D, typename ET>
-__global__ void __launch_bounds__(256) compress_bias_kernel(const ET* __restrict__ pe, const ET* __restrict__ w, int rows, float* __restrict__ part) {
+__global__ void __launch_bounds__(256) compress_bias_kernel(const ET* __restrict__ pe, const ET* __restrict__ w, int rows, float* __restrict__ part,
+                                                           int* __restrict__ status) {
     constexpr int CG = D / 8, KL = 256 / CG;
     __shared__ float red[8][D];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, cgi = tid % CG, kl = tid / CG;
+    if (tid == 0 && blockIdx.x == 0 && h == 0) *status = kStatusOk;
     const int share = rows / kPeParts, r0 = blockIdx.x * share;
     const ET* wr = w + ((int64_t)h * rows + r0) * D + cgi * 8;
     const ET* pr = pe + (int64_t)h * rows + r0;
@@ -359,7 +361,7 @@ extern "C" int fsa_linear_compress_fwd(const void* x, int64_t x_stride_n, const 
     return run_compress(&t, 1, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, (cudaStream_t)stream);
 }
 
-extern "C" int64_t fsa_compress_bias_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kPeParts * num_heads * head_dim * 4; }
+extern "C" int64_t fsa_compress_bias_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kPeParts * num_heads * head_dim * 4 + 16; }
 
 extern "C" int fsa_compress_kv_fwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
                                    const void* pe, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
@@ -370,18 +372,19 @@ extern "C" int fsa_compress_kv_fwd(const void* k, int64_t k_stride_n, const void
     if (pe && (!scratch || (kernel_size * head_dim) % kPeParts)) return FSA_ERR_BAD_ARG;
     (void)cudaGetLastError();
     cudaStream_t stream = (cudaStream_t)stream_;
+    int* status = pe ? (int*)(scratch + (int64_t)kPeParts * num_heads * head_dim) : nullptr;
     if (pe) {
         const dim3 grid(kPeParts, (unsigned)num_heads);
         const int rows = kernel_size * head_dim;
         if (dtype == FSA_DTYPE_BF16) {
-            if (head_dim == 128) compress_bias_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
-            else compress_bias_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch);
+            if (head_dim == 128) compress_bias_kernel<128, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch, status);
+            else compress_bias_kernel<64, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pe, (const __nv_bfloat16*)w_key, rows, scratch, status);
         } else {
-            if (head_dim == 128) compress_bias_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch);
-            else compress_bias_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch);
+            if (head_dim == 128) compress_bias_kernel<128, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch, status);
+            else compress_bias_kernel<64, __half><<<grid, 256, 0, stream>>>((const __half*)pe, (const __half*)w_key, rows, scratch, status);
         }
         if (cudaGetLastError() != cudaSuccess) return FSA_ERR_CUDA;
     }
     const LcTensor t[2] = {{k, k_stride_n, w_key, pe ? scratch : nullptr, pe ? kPeParts : 0, yk}, {v, v_stride_n, w_value, nullptr, 0, yv}};
-    return run_compress(t, v ? 2 : 1, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, nullptr, stream);
+    return run_compress(t, v ? 2 : 1, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream);
 }

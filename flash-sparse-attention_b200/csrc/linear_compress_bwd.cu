@@ -449,7 +449,7 @@ static int run_bwd(const LcGrad* t, int nt, const LcPeGrad& pe, const int32_t* c
     return FSA_OK;
 }
 
-cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, cudaStream_t stream);
+cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, int* status, cudaStream_t stream);
 
 constexpr int kBiasParts = 32;      // shares of the windows in the sum that is the bias's gradient
 
@@ -487,7 +487,7 @@ extern "C" int fsa_linear_compress_bwd(const void* x, int64_t x_stride_n, const 
                : run_bwd<__half>(&g, 1, none, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream);
 }
 
-extern "C" int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kBiasParts * num_heads * head_dim * 4; }
+extern "C" int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim) { return (int64_t)kBiasParts * num_heads * head_dim * 4 + 16; }
 
 extern "C" int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
                                    const void* pe, const void* dyk, const void* dyv, const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
@@ -505,9 +505,10 @@ extern "C" int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void
     if (rc) return rc;
     cudaStream_t stream = (cudaStream_t)stream_;
     const int parts = total < 32 * kBiasParts ? (total < 32 ? 1 : (int)(total / 32)) : kBiasParts;
-    if (launch_column_sum(dtype, head_dim, dyk, total, num_heads, parts, scratch, stream) != cudaSuccess) return FSA_ERR_CUDA;
+    int* status = (int*)(scratch + (int64_t)kBiasParts * num_heads * head_dim);
+    if (launch_column_sum(dtype, head_dim, dyk, total, num_heads, parts, scratch, status, stream) != cudaSuccess) return FSA_ERR_CUDA;
     const LcPeGrad pg{pe, dpe, scratch, parts};
     return dtype == FSA_DTYPE_BF16
-               ? run_bwd<__nv_bfloat16>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, nullptr, stream)
-               : run_bwd<__half>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, nullptr, stream);
+               ? run_bwd<__nv_bfloat16>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream)
+               : run_bwd<__half>(g, 2, pg, cu_seqlens, seqlens_host, batch, num_heads, head_dim, kernel_size, kernel_stride, dtype, status, stream);
 }

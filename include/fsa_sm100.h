@@ -205,7 +205,8 @@ int fsa_linear_compress_fwd(const void* x, int64_t x_stride_n, const void* w, co
 
 /* K and V compressed in one launch per 12 sequences, with the bias of the position embedding pe [H, ks, D] (or null) of the
  * keys computed on the way: fsa_linear_compress_fwd twice plus the einsum of nsa_ref/ops/linear_compress.py:497-501.  v null:
- * one tensor only.  scratch: fsa_compress_bias_scratch_bytes(), needed with pe. */
+ * one tensor only.  scratch: fsa_compress_bias_scratch_bytes(), needed with pe; its last 16 bytes start with the call's status word
+ * (fsa_read_status). */
 int64_t fsa_compress_bias_scratch_bytes(int num_heads, int head_dim);
 int fsa_compress_kv_fwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
                         const void* pe, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
@@ -327,7 +328,7 @@ int fsa_range_attn_bwd_delta(const void* q, const void* k, const void* v, const 
                              void* index_ws, int64_t index_ws_bytes, void* scratch, int64_t scratch_bytes, void* stream);
 
 /* Backward of fsa_compress_kv_fwd: dk, dv (contiguous), dw_key with the share of the bias, dw_value, dpe (the last three may be
- * null).  scratch: fsa_compress_kv_bwd_scratch_bytes(). */
+ * null).  scratch: fsa_compress_kv_bwd_scratch_bytes(); its last 16 bytes start with the call's status word. */
 int64_t fsa_compress_kv_bwd_scratch_bytes(int num_heads, int head_dim);
 int fsa_compress_kv_bwd(const void* k, int64_t k_stride_n, const void* v, int64_t v_stride_n, const void* w_key, const void* w_value,
                         const void* pe, const void* dyk, const void* dyv, const int32_t* cu_seqlens, const int32_t* seqlens_host, int batch, int num_heads, int head_dim, int kernel_size,
