@@ -213,6 +213,16 @@ std::tuple<Tensor, Tensor> nsa_layer(const Tensor& x_, const Tensor& wq, const T
                                      const std::vector<int64_t>& seqlens, const std::vector<int64_t>& cfg) {
     c10::cuda::CUDAGuard guard(x_.device());
     same_kind(x_, {&wq, &wk, &wv, &wg, &w_key, &w_value, &pe}, "layer");
+    {
+        // (raw pointers from here on; the lengths agree with x and cu: _native of fsa/module/fsa.py)
+        const LayerCfg c = layer_cfg(cfg);
+        const int64_t hidden = x_.size(1), q = (int64_t)c.Hq * c.D, kv = (int64_t)c.Hk * c.D;
+        TORCH_CHECK_VALUE(wq.sizes() == at::IntArrayRef({q, hidden}) && wk.sizes() == at::IntArrayRef({kv, hidden}) &&
+                              wv.sizes() == wk.sizes() && wg.sizes() == at::IntArrayRef({3, hidden}) &&
+                              w_key.sizes() == at::IntArrayRef({c.Hk, (int64_t)c.ks * c.D, c.D}) && w_value.sizes() == w_key.sizes() &&
+                              pe.sizes() == at::IntArrayRef({c.Hk, c.ks, c.D}),
+                          "layer: a weight has another shape than the layer's settings");
+    }
     const Tensor x = x_.stride(1) == 1 && x_.stride(0) % 8 == 0 && ((uintptr_t)x_.data_ptr() & 15) == 0 ? x_ : x_.contiguous();
     if (wants_grad({&x, &wq, &wk, &wv, &wg, &w_key, &w_value, &pe})) {
         auto r = NsaLayer::apply(x, wq, wk, wv, wg, w_key, w_value, pe, inv_freq, cu, seqlens, cfg);

@@ -34,13 +34,18 @@ def host():
 def plain_linear(m: torch.nn.Module) -> bool:
     """Nothing but ``x W^T``: no subclass, bias or hook that a call of the module would run.  Modules made of such parts run as
     one native function on their weights, others as their parts."""
-    return type(m) is torch.nn.Linear and m.bias is None and not _hooked(m)
+    return type(m) is torch.nn.Linear and m.bias is None and not hooked(m)
 
 
 def plain_gate(m: torch.nn.Module) -> bool:
     return (type(m) is torch.nn.Sequential and len(m) == 2 and plain_linear(m[0]) and type(m[1]) is torch.nn.Sigmoid
-            and not _hooked(m) and not _hooked(m[1]))
+            and not hooked(m) and not hooked(m[1]))
 
 
-def _hooked(m: torch.nn.Module):
+def plain_weights(x: torch.Tensor, *weights: torch.Tensor) -> bool:
+    """Weights whose memory the native functions can take as it is, beside an input ``x``."""
+    return all(w.dtype == x.dtype and w.device == x.device and w.is_contiguous() for w in weights)
+
+
+def hooked(m: torch.nn.Module):
     return m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks

@@ -10,7 +10,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from fsa._host import host, plain_gate, plain_linear
+from fsa._host import host, plain_gate, plain_linear, plain_weights
 from fsa.module.rope import RopeConfig, RotaryEmbedding
 from fsa.ops.compressed_attention import _FUSED_TAPS, compressed_attention
 from fsa.ops.FSA_topk_sparse_attention import FSA_topk_sparse_attention
@@ -69,18 +69,20 @@ class FlashSparseAttention(torch.nn.Module):
         for p in self.parameters():
             torch.nn.init.xavier_uniform_(p)
 
-    def _native(self, x: torch.Tensor, seqlens, n_cmp: int) -> bool:
+    def _native(self, x: torch.Tensor, cu_seqlens: torch.Tensor, seqlens, n_cmp: int) -> bool:
         """Does the one native function serve this call?  It needs the modules to be what the constructor made of them, one type
         throughout and the shapes that the fused kernels are compiled for; anything else runs as its parts below."""
         return (x.is_cuda and x.dim() == 2 and n_cmp > 0 and self.head_dim in (64, 128) and sum(seqlens) == x.shape[0]
+                and cu_seqlens.numel() == len(seqlens) + 1 and cu_seqlens.device == x.device
                 and self.kernel_size in (16, 32, 64, 128) and self.kernel_size % self.kernel_stride == 0
                 and self.block_size % self.kernel_stride == 0
                 and (self.kernel_size // self.kernel_stride, self.block_size // self.kernel_stride) in _FUSED_TAPS
                 and self.kernel_stride & (self.kernel_stride - 1) == 0
                 and max(1, self.init_blocks + self.local_blocks) <= self.topk <= 32 and self.num_q_heads <= 32 * self.num_kv_heads
-                and self.hidden_size % 8 == 0 and self.hidden_size <= 16384 and type(self.rope) is RotaryEmbedding
+                and self.hidden_size % 8 == 0 and self.hidden_size <= 16384 and type(self.rope) is RotaryEmbedding and self.rope.plain(self.head_dim)
                 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v) and plain_gate(self.gate)
-                and all(p.dtype == x.dtype and p.is_contiguous() for p in (self.proj_q.weight, self.compress_key, self.intra_block_pe))
+                and plain_weights(x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.gate[0].weight, self.compress_key,
+                                  self.compress_value, self.intra_block_pe)
                 and not torch.is_autocast_enabled())
 
     def forward(self, x: torch.Tensor, cu_seqlens: torch.Tensor, seqlens: Optional[Sequence[int]] = None):
@@ -95,7 +97,7 @@ class FlashSparseAttention(torch.nn.Module):
         cmp_lens = compressed_seqlens(seqlens, self.kernel_size, self.kernel_stride)
         max_cmp = max(cmp_lens) if len(cmp_lens) else 0
 
-        if self._native(x, seqlens, sum(cmp_lens)):
+        if self._native(x, cu_seqlens, seqlens, sum(cmp_lens)):
             attn_output, self.last_topk_idx = host().nsa_layer(
                 x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.gate[0].weight, self.compress_key, self.compress_value,
                 self.intra_block_pe, self.rope.inv_freq_on(x.device), cu_seqlens.contiguous(), seqlens,
@@ -129,7 +131,7 @@ class FlashSparseAttention(torch.nn.Module):
         sliding_attn_output, _ = sliding_window_attention(q, k, v, cu_seqlens, self.window_size)
 
         # gate = sigmoid(Linear(hidden, 3)(x)) and the mix of the three branches, fused (same rounding points as the modules)
-        if x.is_cuda and self.hidden_size % 8 == 0 and self.hidden_size <= 16384:
+        if x.is_cuda and self.hidden_size % 8 == 0 and self.hidden_size <= 16384 and self.gate[0].weight.dtype == x.dtype:
             attn_output = gate_proj_mix(x, self.gate[0].weight, compressed_attn_output, sparse_attn_output, sliding_attn_output)
         else:
             attn_output = gate_mix(self.gate(x), compressed_attn_output, sparse_attn_output, sliding_attn_output)

@@ -17,6 +17,7 @@ import torch
 from torch import nn
 
 from fsa import _lib
+from fsa._host import hooked
 
 
 @dataclass
@@ -76,6 +77,7 @@ def _rotate(x, cos, sin, cu_seqlens, conj):
     if x.stride(2) != 1 or x.stride(0) % 8 or x.stride(1) % 8 or x.data_ptr() % 16:
         x = x.contiguous()
     N, H, D = x.shape
+    assert cos.shape[1] * 2 == D, "the rotary embedding is made for another head size"
     out = torch.empty((N, H, D), dtype=x.dtype, device=x.device)
     with torch.cuda.device(x.device):
         rc = _lib.lib().fsa_rope(_lib.ptr(x), x.stride(0), x.stride(1), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(cu_seqlens),
@@ -102,6 +104,10 @@ class RotaryEmbedding(nn.Module):
         if self._inv_freq.device != device:
             self._inv_freq = self._inv_freq.to(device)
         return self._inv_freq
+
+    def plain(self, head_dim: int) -> bool:
+        """Are cos and sin of position * inv_freq all that a call does?  (The native functions form the angles themselves.)"""
+        return self.attention_scaling == 1.0 and 2 * self._inv_freq.numel() == head_dim and not hooked(self)
 
     @torch.no_grad()
     def generate_cos_sin(self, x: torch.Tensor, position_ids: torch.Tensor):

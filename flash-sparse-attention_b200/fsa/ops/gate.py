@@ -48,6 +48,7 @@ class GateProjMix(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_gate, a, b, c):
         assert a.is_cuda, "the sm_100a kernels need CUDA tensors (no CPU fallback)"
+        assert x.dtype == w_gate.dtype == a.dtype == b.dtype == c.dtype
         xk = x if (x.stride(-1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0) else x.contiguous()
         wk, a, b, c = w_gate.contiguous(), a.contiguous(), b.contiguous(), c.contiguous()
         N, hidden = xk.shape
