@@ -539,6 +539,32 @@ static bool misaligned(std::initializer_list<const void*> ps) {
     return false;
 }
 
+// Shared memory of decode_select_kernel: keys, probabilities that the blocks can touch, merge weights.
+static int64_t select_smem(int max_blocks, int taps, int blocks_per, int group, int num_partials) {
+    return 4 * ((int64_t)max_blocks + (int64_t)max_blocks * blocks_per + taps + (int64_t)group * num_partials);
+}
+
+static bool select_sizes(int num_q_heads, int num_kv_heads, int kernel_size, int kernel_stride, int block_size, int topk, int max_blocks, int num_partials) {
+    if (kernel_size % kernel_stride || block_size % kernel_stride || topk > 64 || max_blocks > 65535 || num_q_heads / num_kv_heads > 16) return false;
+    const int bb = block_size / kernel_stride, nw = kernel_size / kernel_stride + bb - 1;
+    return nw <= 16 && select_smem(max_blocks, nw, bb, num_q_heads / num_kv_heads, num_partials) <= 200 * 1024;
+}
+
+static bool compress_sizes(int num_kv_heads, int head_dim, int kernel_size) {
+    return (head_dim == 64 || head_dim == 128) && kernel_size % 8 == 0 && kernel_size <= 128 && num_kv_heads <= 65535;
+}
+
+extern "C" int fsa_decode_step_sizes(int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int block_size, int topk,
+                                     int max_blocks, int num_partials, int gate_dim) {
+    if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads || head_dim <= 0 || kernel_size <= 0 || kernel_stride <= 0 || block_size <= 0 ||
+        topk <= 0 || max_blocks <= 0 || num_partials <= 0 || gate_dim < -1)
+        return FSA_ERR_BAD_ARG;
+    return (head_dim == 64 || head_dim == 128) && (gate_dim < 0 || (compress_sizes(num_kv_heads, head_dim, kernel_size) && gate_dim % 8 == 0)) &&
+                   select_sizes(num_q_heads, num_kv_heads, kernel_size, kernel_stride, block_size, topk, max_blocks, num_partials)
+               ? FSA_OK
+               : FSA_ERR_UNSUPPORTED;
+}
+
 extern "C" int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k_dim, int num, const void* const* w, const int* rows,
                                void* const* y, const int64_t* y_stride, int dtype, void* stream) {
     if (!x || !w || !rows || !y || !y_stride || batch <= 0 || num <= 0 || k_dim <= 0) return FSA_ERR_BAD_ARG;
@@ -611,7 +637,7 @@ extern "C" int fsa_decode_compress(const void* k_tail, const void* v_tail, const
                                    int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int cmp_cap, int dtype, void* stream) {
     if (!k_tail || !v_tail || !w_key || !w_value || !seq_len || !cmp_row0 || !cmp_k || !cmp_v || batch <= 0 || num_kv_heads <= 0) return FSA_ERR_BAD_ARG;
     if (kernel_size <= 0 || kernel_stride <= 0 || misaligned({w_key, w_value})) return FSA_ERR_BAD_ARG;
-    if ((head_dim != 64 && head_dim != 128) || kernel_size % 8 || kernel_size > 128 || num_kv_heads > 65535) return FSA_ERR_UNSUPPORTED;
+    if (!compress_sizes(num_kv_heads, head_dim, kernel_size)) return FSA_ERR_UNSUPPORTED;
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     DecodeCompressParams p;
     p.k_tail = k_tail; p.v_tail = v_tail; p.wk = w_key; p.wv = w_value; p.pe = pe; p.inv_freq = inv_freq; p.seq_len = seq_len; p.cmp_row0 = cmp_row0;
@@ -634,8 +660,7 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
         return FSA_ERR_BAD_ARG;
     if (num_window_pieces > 0 && (int64_t)block_size * num_window_pieces < (int64_t)window + 1) return FSA_ERR_BAD_ARG;
     if (head_dim % 4 || misaligned({o_part}) || ((uintptr_t)o_cmp & 7)) return FSA_ERR_BAD_ARG;
-    if (kernel_size % kernel_stride || block_size % kernel_stride || topk > 64 || max_blocks > 65535 || num_q_heads / num_kv_heads > 16)
-        return FSA_ERR_UNSUPPORTED;
+    if (!select_sizes(num_q_heads, num_kv_heads, kernel_size, kernel_stride, block_size, topk, max_blocks, num_partials)) return FSA_ERR_UNSUPPORTED;
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     DecodeSelectParams p;
     p.o_part = o_part; p.ml = (const float2*)ml; p.scores = scores; p.ld = scores_ld; p.seq_len = seq_len; p.seq_row0 = seq_row0;
@@ -644,14 +669,11 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
     p.max_blocks = max_blocks; p.window = window; p.npieces = num_window_pieces;
     const int a = kernel_size / kernel_stride, bb = block_size / kernel_stride;
     p.nw = a + bb - 1;
-    if (p.nw > 16) return FSA_ERR_UNSUPPORTED;
     for (int i = 0; i < 16; ++i) p.w[i] = 0.f;
     for (int i = 0; i < a; ++i)
         for (int j = 0; j < bb; ++j) p.w[i + j] += 1.f;
     p.o_cmp = o_cmp; p.topk = topk_idx; p.rng_lo = rng_lo; p.rng_hi = rng_hi;
-    // keys, probabilities that the blocks can touch, merge weights
-    const int64_t smem = 4 * ((int64_t)max_blocks + (int64_t)max_blocks * bb + p.nw + (int64_t)p.G * num_partials);
-    if (smem > 200 * 1024) return FSA_ERR_UNSUPPORTED;
+    const int64_t smem = select_smem(max_blocks, p.nw, bb, p.G, num_partials);
     (void)cudaGetLastError();
     const void* kern = dtype == FSA_DTYPE_BF16 ? (const void*)decode_select_kernel<__nv_bfloat16> : (const void*)decode_select_kernel<__half>;
     if (smem > 48 * 1024 && allow_smem(kern, (int)smem) != cudaSuccess) return FSA_ERR_CUDA;

@@ -2,6 +2,9 @@
 // that a CUDA graph can hold it).
 #include "host_common.h"
 
+#include <climits>
+#include <optional>
+
 namespace fsa_host {
 
 struct DecodeCfg {
@@ -15,21 +18,44 @@ static DecodeCfg cfg_of(const std::vector<int64_t>& c, double scale) {
     return {(int)c[0], (int)c[1], (int)c[2], (int)c[3], (int)c[4], (int)c[5], (int)c[6], c[7], scale};
 }
 
+// Chunks of the compressed rows.  Work per CTA of the two attention passes: as long as possible (few partials, a ring of loads that
+// stays full) while about four CTAs per SM are left for each pass: a small batch is split finely, a full one takes 1024 rows /
+// 16 blocks at a time.
+struct Chunks {
+    int rows, n;
+    Chunks(const DecodeCfg& c, int64_t heads) {
+        const int64_t max_cmp = std::max<int64_t>(c.max_len >= c.ks ? (c.max_len - c.ks) / c.stride + 1 : 0, 1);
+        const int64_t per = (max_cmp * heads + 4 * 148 - 1) / (4 * 148);
+        rows = (int)std::min<int64_t>(1024, std::max<int64_t>(64, (per + 63) / 64 * 64));
+        n = (int)((max_cmp + rows - 1) / rows);
+    }
+};
+
+static int max_blocks(const DecodeCfg& c) { return (int)std::min<int64_t>((c.max_len + c.bs - 1) / c.bs, INT_MAX); }
+
+// Do the kernels take these sizes?  (gate_dim: see fsa_decode_step_sizes)
+static bool takes_sizes(int64_t B, int64_t Hq, int64_t Hk, int64_t D, const DecodeCfg& c, int64_t gate_dim) {
+    return B > 0 && Hk > 0 && c.ks > 0 && c.stride > 0 && c.bs > 0 &&
+           fsa_decode_step_sizes((int)Hq, (int)Hk, (int)D, c.ks, c.stride, c.bs, c.topk, max_blocks(c), Chunks(c, B * Hk).n, (int)gate_dim) == FSA_OK;
+}
+
+static bool packed_like(const Tensor& t, const Tensor& q, int64_t Hk) {
+    return t.dim() == 3 && t.scalar_type() == q.scalar_type() && t.device() == q.device() && t.size(1) == Hk && t.size(2) == q.size(2) &&
+           t.stride(2) == 1 && t.stride(1) == t.size(2) && t.stride(0) % 8 == 0 && ((uintptr_t)t.data_ptr() & 15) == 0;
+}
+static bool lengths_like(const Tensor& t, const Tensor& q, int64_t B) {
+    return t.scalar_type() == at::kInt && t.device() == q.device() && t.numel() == B && t.is_contiguous();
+}
+
 // Three branches of one token per sequence and their gate mix; q [B, Hq, D] rotated, gate [B, 3].
 static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cmp_k, const Tensor& cmp_v,
                                             const Tensor& seq_len, const Tensor& seq_row0, const Tensor& cmp_row0, const Tensor& gate,
                                             const DecodeCfg& c) {
     const int B = (int)q.size(0), Hq = (int)q.size(1), D = (int)q.size(2), Hk = (int)k.size(1), dt = dtype_code(q);
-    TORCH_CHECK_VALUE(k.stride(2) == 1 && k.stride(1) == D && v.strides() == k.strides() && cmp_k.stride(2) == 1 && cmp_k.stride(1) == D &&
-                          cmp_v.strides() == cmp_k.strides(), "cache rows must be packed");
     const float scale = (float)(c.scale > 0 ? c.scale : 1.0 / std::sqrt((double)D));
     void* st = stream_of(q);
-    // Work per CTA of the two attention passes: as long as possible (few partials, a ring of loads that stays full) while about
-    // four CTAs per SM are left for each pass: a small batch is split finely, a full one takes 1024 rows / 16 blocks at a time.
-    const int64_t max_cmp = std::max<int64_t>(c.max_len >= c.ks ? (c.max_len - c.ks) / c.stride + 1 : 0, 1);
-    const int64_t per = (max_cmp * B * Hk + 4 * 148 - 1) / (4 * 148);
-    const int chunk = (int)std::min<int64_t>(1024, std::max<int64_t>(64, (per + 63) / 64 * 64));
-    const int nchunk = (int)((max_cmp + chunk - 1) / chunk);
+    const Chunks chunks(c, (int64_t)B * Hk);
+    const int chunk = chunks.rows, nchunk = chunks.n;
     const int npieces = (c.window + 1 + c.bs - 1) / c.bs, R = c.topk + npieces;
     int rpp = 16;
     while (rpp > 1 && (c.topk % rpp || (int64_t)B * Hk * ((R + rpp - 1) / rpp) < 2 * 148)) rpp /= 2;
@@ -55,7 +81,7 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, co
                                  c.ks, c.stride, chunk, nchunk, dt, scale, o1, m1, sc, ld, st),
           "fsa_decode_cmp_partial");
     check(fsa_decode_merge_select(o1, m1, nchunk, sc, ld, iptr(seq_len), iptr(seq_row0), B, Hq, Hk, D, c.ks, c.stride, c.bs, c.init_blocks,
-                                  c.local_blocks, c.topk, (int)((c.max_len + c.bs - 1) / c.bs), c.window, npieces, dt, oc,
+                                  c.local_blocks, c.topk, max_blocks(c), c.window, npieces, dt, oc,
                                   topk.data_ptr<int32_t>(), lo, hi, st),
           "fsa_decode_merge_select");
     check(fsa_decode_attn_partial(ptr(q), ptr(k), ptr(v), k.size(0), k.stride(0), lo, hi, B, Hq, Hk, D, R, rpp, c.bs, 1, dt, scale, o2, m2,
@@ -65,22 +91,55 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, co
     return {out, topk};
 }
 
-std::tuple<Tensor, Tensor> decode_mixed(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cmp_k, const Tensor& cmp_v,
-                                        const Tensor& seq_len, const Tensor& seq_row0, const Tensor& cmp_row0, const Tensor& gate,
-                                        const std::vector<int64_t>& cfg, double scale) {
-    c10::cuda::CUDAGuard guard(q.device());
-    return attention(q.contiguous(), k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate.to(q.scalar_type()).contiguous(), cfg_of(cfg, scale));
+// What these functions return: the outputs, or nothing where the kernels do not take the call (before anything was launched).
+using Outcome = std::optional<std::tuple<Tensor, Tensor>>;
+
+Outcome decode_mixed(const Tensor& q_, const Tensor& k, const Tensor& v, const Tensor& cmp_k, const Tensor& cmp_v, const Tensor& seq_len,
+                     const Tensor& seq_row0, const Tensor& cmp_row0, const Tensor& gate, const std::vector<int64_t>& cfg, double scale) {
+    c10::cuda::CUDAGuard guard(q_.device());
+    const DecodeCfg c = cfg_of(cfg, scale);
+    const Tensor q = q_.contiguous();
+    TORCH_CHECK_VALUE(q.dim() == 3 && k.dim() == 3 && gate.numel() == 3 * q.size(0), "decode: q [B, Hq, D], cache rows [rows, Hk, D], gate [B, 3]");
+    const int64_t B = q.size(0), Hk = k.size(1);
+    if (!takes_sizes(B, q.size(1), Hk, q.size(2), c, -1)) return std::nullopt;
+    for (auto* t : {&k, &v, &cmp_k, &cmp_v})
+        if (!packed_like(*t, q, Hk)) return std::nullopt;
+    if (v.strides() != k.strides() || cmp_v.strides() != cmp_k.strides()) return std::nullopt;
+    for (auto* t : {&seq_len, &seq_row0, &cmp_row0})
+        if (!lengths_like(*t, q, B)) return std::nullopt;
+    return attention(q, k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate.to(q.scalar_type()).contiguous(), c);
 }
 
 // The buffers of a DecodeCache, in this order: k, v, cmp_k, cmp_v, k_tail, v_tail, seq_len, seq_row0, cmp_row0.
 using Cache = std::vector<Tensor>;
 
+// Does the native step take this call?  k_new stands for the type and the device of everything.
+static bool served(const Cache& t, int64_t Hq, const Tensor& k_new, const Tensor& v_new, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
+                   const DecodeCfg& c, int64_t gate_dim) {
+    if (t.size() != 9 || k_new.dim() != 3 || !k_new.is_cuda()) return false;
+    const int64_t B = k_new.size(0), Hk = k_new.size(1), D = k_new.size(2);
+    if (!takes_sizes(B, Hq, Hk, D, c, gate_dim)) return false;
+    for (int i = 0; i < 6; ++i)
+        if (!packed_like(t[i], k_new, Hk) || !t[i].is_contiguous()) return false;
+    for (int i = 6; i < 9; ++i)
+        if (!lengths_like(t[i], k_new, B)) return false;
+    for (auto* w : {&v_new, &w_key, &w_value, &pe})
+        if (w->scalar_type() != k_new.scalar_type() || w->device() != k_new.device() || !w->is_contiguous() || ((uintptr_t)w->data_ptr() & 15)) return false;
+    const int64_t rows = t[0].size(0) - 1;        // (the last row of a buffer is a spare one)
+    return v_new.sizes() == k_new.sizes() && rows > 0 && rows % B == 0 && t[1].size(0) == rows + 1 && (t[2].size(0) - 1) % B == 0 &&
+           t[3].size(0) == t[2].size(0) && t[4].size(0) == B * c.ks + 1 && t[5].size(0) == t[4].size(0) &&
+           w_key.sizes() == at::IntArrayRef({Hk, c.ks * D, D}) && w_value.sizes() == w_key.sizes() && pe.sizes() == at::IntArrayRef({Hk, c.ks, D});
+}
+
+static bool weight(const Tensor& w, const Tensor& x, int64_t rows, int64_t cols) {
+    return w.scalar_type() == x.scalar_type() && w.device() == x.device() && w.is_contiguous() && w.sizes() == at::IntArrayRef({rows, cols}) &&
+           ((uintptr_t)w.data_ptr() & 15) == 0;
+}
+
 // Append (with the gate from logits z, or from gx and its weight), compressor, attention.
 static std::tuple<Tensor, Tensor> step(const Tensor& q_in, const Tensor& k_new, const Tensor& v_new, Tensor q, const Tensor& inv_freq,
                                        const Tensor& z, const Tensor& gx, const Tensor& gw, const Cache& t, const Tensor& w_key,
                                        const Tensor& w_value, const Tensor& pe, bool compress, const DecodeCfg& c) {
-    TORCH_CHECK_VALUE(t.size() == 9, "cache buffers");
-    same_kind(k_new, {&v_new, &q, &gw, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &w_key, &w_value, &pe}, "decode step");
     const int B = (int)k_new.size(0), Hk = (int)k_new.size(1), D = (int)k_new.size(2), Hq = (int)q.size(1), dt = dtype_code(k_new);
     const int cap = (int)((t[0].size(0) - 1) / B), cmp_cap = (int)((t[2].size(0) - 1) / B);
     const float* freq = inv_freq.defined() ? inv_freq.data_ptr<float>() : nullptr;
@@ -98,13 +157,18 @@ static std::tuple<Tensor, Tensor> step(const Tensor& q_in, const Tensor& k_new, 
 }
 
 // FlashSparseAttentionDecodeKernel.step: q, k_new, v_new in, [B, Hq * D] and the block ids out.
-std::tuple<Tensor, Tensor> decode_kernel_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gw, const Cache& t,
-                                              const Tensor& w_key, const Tensor& w_value, const Tensor& pe, bool compress,
-                                              const std::vector<int64_t>& cfg, double scale) {
+Outcome decode_kernel_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gw, const Cache& t, const Tensor& w_key,
+                           const Tensor& w_value, const Tensor& pe, bool compress, const std::vector<int64_t>& cfg, double scale) {
     c10::cuda::CUDAGuard guard(q_.device());
+    const DecodeCfg c = cfg_of(cfg, scale);
     const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
-    auto [y, ids] = step(q, k, v, q, Tensor(), Tensor(), q.view({q.size(0), -1}), gw, t, w_key, w_value, pe, compress, cfg_of(cfg, scale));
-    return {y.view({y.size(0), -1}), ids};
+    if (q.dim() != 3 || k.dim() != 3 || q.size(0) != k.size(0) || q.size(2) != k.size(2) || q.scalar_type() != k.scalar_type() || q.device() != k.device() ||
+        ((uintptr_t)q.data_ptr() & 15) || ((uintptr_t)k.data_ptr() & 15))
+        return std::nullopt;
+    const Tensor gx = q.view({q.size(0), -1});
+    if (!weight(gw, q, 3, gx.size(1)) || !served(t, q.size(1), k, v, w_key, w_value, pe, c, gx.size(1))) return std::nullopt;
+    auto [y, ids] = step(q, k, v, q, Tensor(), Tensor(), gx, gw, t, w_key, w_value, pe, compress, c);
+    return std::make_tuple(y.view({y.size(0), -1}), ids);
 }
 
 // Rows up to which the library's own skinny projection is used (one MMA tile of rows; above it a library GEMM's tiles are fuller).
@@ -123,14 +187,21 @@ static void project(const Tensor& x, std::initializer_list<Tensor> ws, std::init
 }
 
 // FlashSparseAttentionDecode.step: x [B, hidden] in, [B, hidden] and the block ids out.
-std::tuple<Tensor, Tensor> decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo,
-                                             const Tensor& gw, const Tensor& inv_freq, int64_t D, const Cache& t, const Tensor& w_key,
-                                             const Tensor& w_value, const Tensor& pe, bool compress, const std::vector<int64_t>& cfg, double scale) {
+Outcome decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo, const Tensor& gw,
+                          const Tensor& inv_freq, int64_t D, const Cache& t, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
+                          bool compress, const std::vector<int64_t>& cfg, double scale) {
     c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous();
-    same_kind(x, {&wq, &wk, &wv, &wo, &gw}, "decode step");
-    const int64_t B = x.size(0), nq = wq.size(0), nk = wk.size(0);
-    const bool skinny = B <= kProjRows && x.size(1) % 256 == 0 && nq % 256 == 0 && ((uintptr_t)x.data_ptr() & 15) == 0;
+    const DecodeCfg c = cfg_of(cfg, scale);
+    const Tensor x = x_.contiguous().view({x_.size(0), -1});
+    const int64_t B = x.size(0), hidden = x.size(1), nq = wq.size(0), nk = wk.size(0);
+    const bool skinny = B <= kProjRows && hidden % 256 == 0 && nq % 256 == 0 && ((uintptr_t)x.data_ptr() & 15) == 0;
+    if (t.size() != 9 || t[0].dim() != 3 || D <= 0 || nq % D || nk != t[0].size(1) * D || t[0].size(2) != D || ((uintptr_t)x.data_ptr() & 15) ||
+        inv_freq.scalar_type() != at::kFloat || inv_freq.device() != x.device() || inv_freq.numel() != D / 2 || !weight(wq, x, nq, hidden) ||
+        !weight(wk, x, nk, hidden) || !weight(wv, x, nk, hidden) || !weight(wo, x, wo.size(0), nq) || !weight(gw, x, 3, hidden))
+        return std::nullopt;
+    // (stands for the new keys and values, which are not projected yet)
+    const Tensor like = t[0].narrow(0, 0, std::min<int64_t>(B, t[0].size(0)));
+    if (like.size(0) != B || !served(t, nq / D, like, like, w_key, w_value, pe, c, skinny ? 0 : hidden)) return std::nullopt;
     Tensor q, k, v, z;
     if (skinny) {
         q = fresh({B, nq}, x);
@@ -145,12 +216,12 @@ std::tuple<Tensor, Tensor> decode_layer_step(const Tensor& x_, const Tensor& wq,
     }
     q = q.view({B, nq / D, D});
     auto [mixed, ids] = step(q, k.view({B, nk / D, D}), v.view({B, nk / D, D}), q, inv_freq, z, skinny ? Tensor() : x, gw, t, w_key, w_value, pe,
-                             compress, cfg_of(cfg, scale));
+                             compress, c);
     const Tensor m = mixed.view({B, nq});
-    if (!skinny) return {at::linear(m, wo), ids};
+    if (!skinny) return std::make_tuple(at::linear(m, wo), ids);
     Tensor y = fresh({B, wo.size(0)}, x);
     project(m, {wo}, {y});
-    return {y, ids};
+    return std::make_tuple(y, ids);
 }
 
 void bind_decode(pybind11::module& m) {

@@ -122,6 +122,7 @@ SIGNATURES = {
     "fsa_compress_kv_bwd_scratch_bytes": (c_int64, [c_int, c_int]),
     "fsa_compress_kv_bwd": (
         c_int, [c_void_p, c_int64, c_void_p, c_int64] + [c_void_p] * 7 + [c_int] * 6 + [c_void_p] * 7),
+    "fsa_decode_step_sizes": (c_int, [c_int] * 10),
     "fsa_decode_proj": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "fsa_decode_append": (
         c_int,

@@ -79,12 +79,16 @@ class DecodeCache:
         """The tensors that the native step works on."""
         return [self.k, self.v, self.cmp_k, self.cmp_v, self.k_tail, self.v_tail, self.seq_len, self.seq_row0, self.cmp_row0]
 
-    def advance(self) -> bool:
-        """Count one more token per sequence on the host; does the compressor have to run (it looks at the device-side lengths
-        itself, so it may run for nothing)?"""
+    def advanced(self):
+        """The host's lengths after one more token per sequence, and whether the compressor has to run for it (it looks at the
+        device-side lengths itself, so it may run for nothing)."""
         ks, stride = self.ks, self.stride
-        self.host_len = new = [L + 1 for L in self.host_len]
-        return self.always_compress or any(L >= ks and (L - ks) % stride == 0 for L in new)
+        new = [L + 1 for L in self.host_len]
+        return new, self.always_compress or any(L >= ks and (L - ks) % stride == 0 for L in new)
+
+    def advance(self) -> bool:
+        self.host_len, compress = self.advanced()
+        return compress
 
     @torch.no_grad()
     def append(self, k_raw: torch.Tensor, k_rot: torch.Tensor, v: torch.Tensor, compress_key: torch.Tensor,

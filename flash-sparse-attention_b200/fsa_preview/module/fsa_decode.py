@@ -87,14 +87,18 @@ class FlashSparseAttentionDecode(torch.nn.Module):
     def step(self, x: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """``x [B, hidden]``: one new token per sequence -> ``[B, hidden]``; appends to ``cache``."""
         B = x.shape[0]
-        if (cache.shard.world == 1 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v)
-                and plain_linear(self.proj_o) and plain_gate(self.gate) and type(self.rope) is RotaryEmbedding):
-            compress = cache.advance()
-            y, self.last_topk_idx = host().decode_layer_step(
+        if (x.is_cuda and cache.shard.world == 1 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v)
+                and plain_linear(self.proj_o) and plain_gate(self.gate) and type(self.rope) is RotaryEmbedding and self.rope.plain(self.head_dim)
+                and not torch.is_autocast_enabled()):
+            new_len, compress = cache.advanced()
+            done = host().decode_layer_step(
                 x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.proj_o.weight, self.gate[0].weight,
                 self.rope.inv_freq_on(x.device), self.head_dim, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
                 compress, step_settings(self, cache.max_len), 0.0)
-            return y
+            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts)
+                cache.host_len = new_len
+                y, self.last_topk_idx = done
+                return y
         pos = cache.seq_len.clone()                                   # position of the new token
         q = self.proj_q(x).view(B, self.num_q_heads, self.head_dim)
         k_new = self.proj_k(x).view(B, self.num_kv_heads, self.head_dim)

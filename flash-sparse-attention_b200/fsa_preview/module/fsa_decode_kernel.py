@@ -44,12 +44,15 @@ class FlashSparseAttentionDecodeKernel(torch.nn.Module):
     @torch.no_grad()
     def step(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """One token per sequence: ``q [B, Hq, d]``, ``k_new / v_new [B, Hk, d]`` -> ``[B, Hq*d]``; appends to ``cache``."""
-        if cache.shard.world == 1 and plain_gate(self.gate):
-            compress = cache.advance()
-            out, self.last_topk_idx = host().decode_kernel_step(
+        if q.is_cuda and cache.shard.world == 1 and plain_gate(self.gate) and not torch.is_autocast_enabled():
+            new_len, compress = cache.advanced()
+            done = host().decode_kernel_step(
                 q, k_new, v_new, self.gate[0].weight, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
                 compress, step_settings(self, cache.max_len), 0.0)
-            return out
+            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts)
+                cache.host_len = new_len
+                out, self.last_topk_idx = done
+                return out
         cache.append(k_new, k_new, v_new, self.compress_key, self.compress_value, self.intra_block_pe, None)
         q = q.contiguous()
         gate = self.gate(q.view(q.shape[0], -1))

@@ -15,6 +15,7 @@ import torch
 
 from fsa import _lib
 from fsa._host import host
+from fsa.ops.gate import gate_mix
 
 OUT_CODE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
@@ -262,11 +263,21 @@ def step_settings(m, max_len: int):
 
 
 def nsa_decode_mixed(q, k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate, *, kernel_size, kernel_stride, block_size, topk, init_blocks,
-                     local_blocks, window_size, max_len, sm_scale=None):
+                     local_blocks, window_size, max_len, sm_scale=None, shard: Optional[Shard] = None, ops=None, cmp_chunk: Optional[int] = None):
     """One-GPU decode step ending in the gate mix: ``g0 o_cmp + g1 o_sel + g2 o_win`` ``[B, Hq, D]`` and the top-k ids.
     Same arguments as ``nsa_decode_attention`` plus ``gate [B, 3]`` (after the sigmoid); four launches: compressed pass,
-    merge + top-k + ranges, selected and window pass, merges + mix."""
-    CudaDecodeOps._need_cuda(q)
-    return host().decode_mixed(q, k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate,
-                               [kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks, window_size, max_len],
-                               0.0 if sm_scale is None else float(sm_scale))
+    merge + top-k + ranges, selected and window pass, merges + mix.  With operators or chunks of the caller's, or sizes that these
+    kernels do not take, it is ``nsa_decode_attention`` and the mix."""
+    assert shard is None or shard.world == 1, "the fused finish is the one-GPU path; sharded steps merge across ranks first"
+    if ops is None and cmp_chunk is None and shard is None:
+        CudaDecodeOps._need_cuda(q)
+        done = host().decode_mixed(q, k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, gate,
+                                   [kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks, window_size, max_len],
+                                   0.0 if sm_scale is None else float(sm_scale))
+        if done is not None:
+            return done
+    oc, os_, ow, *_, idx = nsa_decode_attention(
+        q.contiguous(), k, v, cmp_k, cmp_v, seq_len, seq_row0, cmp_row0, kernel_size=kernel_size, kernel_stride=kernel_stride, block_size=block_size,
+        topk=topk, init_blocks=init_blocks, local_blocks=local_blocks, window_size=window_size, max_len=max_len, sm_scale=sm_scale, shard=shard,
+        ops=ops, cmp_chunk=cmp_chunk or 1024)
+    return gate_mix(gate.to(q.dtype), oc, os_.contiguous(), ow.contiguous()), idx

@@ -381,6 +381,12 @@ int fsa_decode_finish(const float* o_part, const float* ml, int64_t rows, int nu
 
 /* ---- the fused kernels of a one-GPU step (what fsa_preview.module's step runs; the calls above are its parts) ----
  *
+ * Do they all take these sizes?  FSA_OK or FSA_ERR_UNSUPPORTED, without a GPU, so that a caller knows before the first launch changes
+ * the cache.  gate_dim: as in fsa_decode_append, 0 with logits, -1: the attention part alone (no append, no compressor). */
+int fsa_decode_step_sizes(int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int block_size,
+                          int topk, int max_blocks, int num_partials, int gate_dim);
+
+/*
  * y_i[b, :] = x[b, :] W_i^T for up to four weight matrices [rows_i, k_dim] (contiguous) in one launch; batch <= 16,
  * k_dim a multiple of 256 (else FSA_ERR_UNSUPPORTED: use a library GEMM).  Replaces the projections of
  * fsa_preview/module/fsa_decode.py:76-83, :196. */

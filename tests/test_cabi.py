@@ -64,6 +64,22 @@ def test_argument_checks_return_codes():
         _lib.check(_lib.FSA_ERR_WORKSPACE, "x")
 
 
+def test_decode_step_sizes():
+    """One size on each side of every limit: the answer is known before a step's first launch."""
+    L = _lib.lib()
+    base = dict(Hq=32, Hk=8, D=128, ks=32, st=16, bs=64, T=16, blocks=2048, partials=64, gate=4096)
+    ok = lambda **kw: L.fsa_decode_step_sizes(*{**base, **kw}.values())          # noqa: E731
+    assert ok() == 0 and ok(gate=0) == 0
+    for inside, outside in ((dict(D=64), dict(D=96)), (dict(ks=24, st=8), dict(ks=20, st=4)), (dict(ks=128), dict(ks=144)), (dict(T=64), dict(T=65)),
+                            (dict(Hq=128), dict(Hq=136)), (dict(gate=8), dict(gate=12)), (dict(st=8, bs=64, ks=72), dict(st=8, bs=64, ks=80)),
+                            (dict(blocks=10187), dict(blocks=10188)), (dict(st=16, bs=48), dict(st=16, bs=40))):
+        assert ok(**inside) == 0, inside
+        assert ok(**outside) == _lib.FSA_ERR_UNSUPPORTED, outside
+    # the attention part alone has no compressor and no gate
+    assert ok(gate=-1, ks=4, st=4, bs=32) == 0 and ok(gate=-1, D=96) == _lib.FSA_ERR_UNSUPPORTED
+    assert ok(Hq=33) == ok(gate=-2) == ok(T=0) == _lib.FSA_ERR_BAD_ARG
+
+
 def test_operator_refuses_cpu_tensors():
     from fsa.ops import FSA_topk_sparse_attention
 

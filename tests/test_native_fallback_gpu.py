@@ -8,6 +8,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 from fsa.module.fsa import FlashSparseAttention, RopeConfig
+from fsa_preview.module import FlashSparseAttentionDecode, FlashSparseAttentionDecodeKernel
+from fsa_preview.ops.decode import nsa_decode_mixed
 
 DEV = "cuda:0"
 
@@ -78,3 +80,76 @@ def test_layer_keeps_a_scaled_or_hooked_rotation():
     layer.rope.register_forward_hook(lambda m, i, o: calls.append(1))
     assert torch.equal(layer(x, cu, [500, 200]), y) and len(calls) == 3
     assert not torch.equal(scaled(x, cu, [500, 200]), y)
+
+
+NSA = dict(kernel_size=32, kernel_stride=16, block_size=64, topk=8, init_blocks=1, local_blocks=2, window_size=100)
+
+
+def _decode(hidden, Hq, Hk, D, lens, max_len, **over):
+    torch.manual_seed(8)
+    cfg = {**NSA, **over}
+    mod = (FlashSparseAttentionDecode(hidden, Hq, Hk, D, rope_config=RopeConfig(head_dim=D), **cfg) if hidden
+           else FlashSparseAttentionDecodeKernel(Hq * D, Hq, Hk, D, **cfg)).to(DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.normal_(0, 0.05)
+
+    def cache(dtype=torch.bfloat16):
+        torch.manual_seed(9)
+        c = mod.new_cache(len(lens), max_len, dtype=dtype, device=DEV)
+        for t in c.buffers()[:6]:
+            t.normal_()
+        c.host_len = list(lens)
+        c.seq_len.copy_(torch.tensor(lens, dtype=torch.int32))
+        return c
+
+    def new():
+        B = len(lens)
+        shapes = [(B, hidden)] if hidden else [(B, Hq, D), (B, Hk, D), (B, Hk, D)]
+        return [torch.randn(s, device=DEV).to(torch.bfloat16) for s in shapes]
+
+    return mod, cache, new
+
+
+@pytest.mark.parametrize("hidden,Hq,Hk,D,lens,max_len,over", [
+    (0, 2, 1, 64, [30, 63], 200, dict(kernel_size=4, kernel_stride=4, block_size=32)),     # a window that is not a multiple of 8
+    (0, 2, 1, 64, [200, 143], 400, dict(kernel_size=144, kernel_stride=16)),               # one above 128
+    (260, 2, 2, 64, [70, 90, 31], 200, {}),                                                # a gate input that is not a multiple of 8
+    (0, 16, 1, 64, [700, 652000], 652800, {}),                                             # more merge weights than shared memory holds
+])
+def test_decode_sizes_outside_the_native_step_run_as_parts(hidden, Hq, Hk, D, lens, max_len, over):
+    mod, cache, new = _decode(hidden, Hq, Hk, D, lens, max_len, **over)
+    a, b = cache(), cache()
+    for _ in range(3):
+        ins = new()
+        y, ids = mod.step(*ins, a), mod.last_topk_idx
+        hook = mod.gate.register_forward_hook(lambda *x: None)
+        ref = mod.step(*ins, b)
+        hook.remove()
+        assert torch.equal(y, ref) and torch.equal(ids, mod.last_topk_idx) and bool(torch.isfinite(y).all())
+    assert a.host_len == b.host_len == [n + 3 for n in lens]
+    for x, z in zip(a.buffers(), b.buffers()):
+        assert torch.equal(x, z)
+
+
+@pytest.mark.parametrize("name", ["proj_q.weight", "proj_v.weight", "proj_o.weight", "gate.0.weight", "compress_key", "compress_value", "intra_block_pe"])
+def test_decode_takes_a_weight_in_another_memory_order_as_parts(name):
+    mod, cache, new = _decode(256, 4, 2, 128, [95, 130], 300)
+    owner, leaf = _holder(mod, name)
+    setattr(owner, leaf, _reordered(getattr(owner, leaf)))
+    a, b, ins = cache(), cache(), new()
+    y = mod.step(*ins, a)
+    hook = mod.gate.register_forward_hook(lambda *x: None)
+    assert torch.equal(mod.step(*ins, b), y)
+    hook.remove()
+    assert a.host_len == b.host_len == [96, 131]
+
+
+def test_decode_mixed_keeps_its_options_as_parts():
+    mod, cache, new = _decode(0, 4, 2, 128, [95, 130], 300)
+    c, (q, _, _) = cache(), new()
+    gate = torch.rand(2, 3, device=DEV).to(torch.bfloat16)
+    args = (q, c.k, c.v, c.cmp_k, c.cmp_v, c.seq_len, c.seq_row0, c.cmp_row0, gate)
+    y, ids = nsa_decode_mixed(*args, max_len=300, **NSA)
+    y2, ids2 = nsa_decode_mixed(*args, max_len=300, cmp_chunk=64, shard=None, ops=None, **NSA)
+    assert torch.equal(ids, ids2) and float((y - y2).abs().max()) <= 2.0 ** -6 * float(y.abs().max())
