@@ -87,6 +87,8 @@ class FlashSparseAttentionDecode(torch.nn.Module):
     def step(self, x: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """``x [B, hidden]``: one new token per sequence -> ``[B, hidden]``; appends to ``cache``."""
         B = x.shape[0]
+        if B != cache.B or x.numel() != B * self.hidden_size:
+            raise ValueError(f"x [{cache.B}, {self.hidden_size}] expected (one token for every sequence of the cache), got {list(x.shape)}")
         if (x.is_cuda and cache.shard.world == 1 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v)
                 and plain_linear(self.proj_o) and plain_gate(self.gate) and type(self.rope) is RotaryEmbedding and self.rope.plain(self.head_dim)
                 and not torch.is_autocast_enabled()):

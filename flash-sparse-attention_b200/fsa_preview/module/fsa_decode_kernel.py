@@ -44,6 +44,10 @@ class FlashSparseAttentionDecodeKernel(torch.nn.Module):
     @torch.no_grad()
     def step(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """One token per sequence: ``q [B, Hq, d]``, ``k_new / v_new [B, Hk, d]`` -> ``[B, Hq*d]``; appends to ``cache``."""
+        kv = (cache.B, self.num_kv_heads, self.head_dim)
+        if q.shape != (cache.B, self.num_q_heads, self.head_dim) or k_new.shape != kv or v_new.shape != kv:
+            raise ValueError(f"q [{cache.B}, {self.num_q_heads}, {self.head_dim}] and k_new, v_new {list(kv)} expected (one token for every "
+                             f"sequence of the cache), got {list(q.shape)}, {list(k_new.shape)}, {list(v_new.shape)}")
         if q.is_cuda and cache.shard.world == 1 and plain_gate(self.gate) and not torch.is_autocast_enabled():
             new_len, compress = cache.advanced()
             done = host().decode_kernel_step(

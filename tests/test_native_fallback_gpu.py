@@ -153,3 +153,23 @@ def test_decode_mixed_keeps_its_options_as_parts():
     y, ids = nsa_decode_mixed(*args, max_len=300, **NSA)
     y2, ids2 = nsa_decode_mixed(*args, max_len=300, cmp_chunk=64, shard=None, ops=None, **NSA)
     assert torch.equal(ids, ids2) and float((y - y2).abs().max()) <= 2.0 ** -6 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("hidden", [256, 0])
+def test_decode_refuses_what_does_not_fit_the_cache_and_leaves_it_alone(hidden):
+    mod, cache, new = _decode(hidden, 4, 2, 128, [95, 130, 64], 300)
+    c = cache()
+    before = [t.clone() for t in c.buffers()]
+    ins = new()
+    short, wide = [t[:2] for t in ins], [torch.cat([t, t]) for t in ins]
+    other = [t[..., :-64].contiguous() for t in ins]
+    for bad in (short, wide, other):
+        with pytest.raises(ValueError):
+            mod.step(*bad, c)
+    half = cache(torch.float16)
+    with pytest.raises((RuntimeError, ValueError, AssertionError)):
+        mod.step(*ins, half)
+    assert c.host_len == half.host_len == [95, 130, 64]
+    for x, z in zip(c.buffers(), before):
+        assert torch.equal(x, z)
+    assert torch.equal(half.seq_len, before[6])
