@@ -102,15 +102,15 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
     for (int k = 0; k < S; ++k)
         if (k < cnt) issue(k, ps[k], gs[k]);
 
-    bool ok = true;
-    for (int k = 0; k < cnt && ok; ++k) {
+    int k = 0;
+    for (; k < cnt; ++k) {
         const int st = k % S;
         const float2 v = mA;
         if (FWD) {
             mA = mB;
             if (k + 2 < cnt) mB = load_ml();
         }
-        ok = mbar_wait(&bars[st], (k / S) & 1, status) && ok;
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars[st], (k / S) & 1, status))) break;      // (the warp stays together)
         const unsigned mask = masks[st];
         const ET* src = reinterpret_cast<const ET*>(ring + st * C::kStage) + half * kMgSlots * D + l * V;
         float acc[V];
@@ -160,15 +160,15 @@ __global__ void __launch_bounds__(kMgWarps * 32, 1) sel_merge(const ET* __restri
         uint32_t x[V / 2];
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) x[i] = ElemTraits<ET>::pack2(acc[2 * i] * inv, acc[2 * i + 1] * inv);
-        if (ok && at.n < s.N) {
+        if (at.n < s.N) {
             *reinterpret_cast<uint2*>(dst) = make_uint2(x[0], x[1]);
             if (FWD && l == 0) lse[(int64_t)hq * s.N + at.n] = L > 0.f ? M + log2f(L) : -INFINITY;
         }
         at.next(step, s.Hk, s.G);
     }
-    // (on a wait that ran out: the copies in flight of this warp land before the CTA ends)
-    for (int k = 0; !ok && k < S; ++k)
-        if (lane == 0) mbar_wait(&bars[k], 0, nullptr);
+    // (on a wait that ran out: the copies in flight, those of this row and the S - 1 behind it, land before the CTA ends)
+    for (int j = k; j < cnt && j < k + S; ++j)
+        if (lane == 0) mbar_wait(&bars[j % S], (j / S) & 1, nullptr);
 }
 
 bool sel_merge_fits(const SelShape& s, int nsub) {
