@@ -46,3 +46,31 @@ def test_long_rows_are_the_same_every_time():
     for _ in range(4):
         o, lse = compressed_attention_core(q, k, v, ks, st, cu_q, cu_k, C)
         assert torch.equal(o, o0) and torch.equal(lse, lse0)
+
+
+@pytest.mark.parametrize("d,bs,T,dtype", [(64, 32, 8, torch.float16), (128, 64, 16, torch.bfloat16), (128, 256, 2, torch.bfloat16), (256, 128, 3, torch.bfloat16)])
+def test_row_strides_beyond_32_bit_offsets(d, bs, T, dtype):
+    """q and dO whose rows lie more than 2^34 elements apart in all: the pipelined kernels address rows by 32-bit offsets in units of 8
+    elements and leave these to the unpipelined ones (34 GB are reserved for them, of which only the rows are touched)."""
+    seqlens, Hk, G = [333, 80], 2, 2
+    N, Hq = sum(seqlens), Hk * G
+    q, k, v, do = (t.to(dtype) for t in make_qkv(N, Hq, Hk, d, 77 + d))
+    idx, cu = make_topk_idx(seqlens, Hk, T, bs, 78 + d), make_cu_seqlens(seqlens)
+    step = (2 ** 34 // N + 8) // 8 * 8
+    assert step * N >= 2 ** 34
+    try:
+        room = torch.empty(N * step, dtype=dtype, device=DEV)
+    except torch.OutOfMemoryError:
+        pytest.skip("less than 34 GB free")
+    far = []
+    for i, t in enumerate((q, do)):
+        far.append(room.as_strided((N, Hq, d), (step, d, 1), i * Hq * d))
+        far[-1].copy_(t)
+    ref = sel_attn_forward_backward(q, k, v, do, idx, bs, cu, d ** -0.5)
+    kc, vc, ic, cc = (x.to(DEV) for x in (k, v, idx, cu))
+    o, lse, ws = sel_attn_fwd(far[0], kc, vc, ic, bs, cc, d ** -0.5, check_status=True)
+    # q far away alone, dO alone, and both
+    for qx, dx in ((far[0], do.to(DEV)), (q.to(DEV), far[1]), tuple(far)):
+        grads = sel_attn_bwd(qx, kc, vc, o, lse, dx, ic, bs, cc, d ** -0.5, ws, check_status=True)
+        for name, got, want in zip(("o", "dq", "dk", "dv"), (o, *grads), (ref[0], *ref[2:])):
+            _close(got, want, name)
