@@ -397,9 +397,10 @@ static int run_gate_fwd(const void* x, int64_t x_sn, const void* wg, const void*
     auto kern = gate_proj_mix_fwd_kernel<ET>;
     if (allow_smem((const void*)kern, smem) != cudaSuccess || prefer_l1((const void*)kern, 50) != cudaSuccess) return FSA_ERR_CUDA;
     // a warp per token: four per CTA while eight would leave SMs idle
-    const int warps = N <= 148 * 8 ? 4 : 8;
+    const int64_t most = sm_count() * 8;
+    const int warps = N <= most ? 4 : 8;
     const int64_t want = (N + warps - 1) / warps;
-    const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
+    const unsigned grid = (unsigned)(want < most ? want : most);
     kern<<<grid, warps * 32, smem, stream>>>((const ET*)x, x_sn, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, N, hidden, HD,
                                       (ET*)out, (ET*)gate);
     return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
@@ -412,8 +413,8 @@ static int run_gate_bwd(const void* x, int64_t x_sn, const void* wg, const void*
     const int smem = 3 * hidden * 2;
     auto kern = !delta ? gate_proj_mix_bwd_kernel<0, ET> : head_dim == 128 ? gate_proj_mix_bwd_kernel<16, ET> : gate_proj_mix_bwd_kernel<8, ET>;
     if (allow_smem((const void*)kern, smem) != cudaSuccess || prefer_l1((const void*)kern, 50) != cudaSuccess) return FSA_ERR_CUDA;
-    const int64_t want = (N + 7) / 8;
-    const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
+    const int64_t want = (N + 7) / 8, most = sm_count() * 8;
+    const unsigned grid = (unsigned)(want < most ? want : most);
     kern<<<grid, 256, smem, stream>>>((const ET*)gate, (const ET*)wg, (const ET*)a, (const ET*)b, (const ET*)c, (const ET*)d_o, N, hidden,
                                       HD, (ET*)da, (ET*)db, (ET*)dc, (ET*)dx, dz, delta);
     const int chunk_tokens = (int)((N + kGateChunks - 1) / kGateChunks);

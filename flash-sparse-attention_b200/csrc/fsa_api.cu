@@ -138,6 +138,11 @@ int device_sm_count(int* out) {
     return FSA_OK;
 }
 
+int sm_count() {
+    int n = 0;
+    return device_sm_count(&n) == FSA_OK && n > 0 ? n : 148;
+}
+
 // ---- optional kernel timing: a ring of event pairs per kernel id
 constexpr int kProfKernels = 16;
 constexpr int kProfRing = 64;
@@ -193,7 +198,7 @@ static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 static int sched_run(const SelShape& s, int most) {
     // (a backward run is walked once per 64-key part of its blocks)
     const int64_t tiles = ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT * (s.BK > 64 ? s.BK / 64 : 1);
-    const int64_t run = tiles / (4 * 148);
+    const int64_t run = tiles / (4 * sm_count());
     return (int)(run < 1 ? 1 : run > most ? most : run);
 }
 
@@ -463,7 +468,7 @@ static int sel_bwd_impl(const SelBounds& bd, int64_t Nk, const float* delta, con
     if (dense) {
         RangeKvPlan plan;
         plan.cu_q = cu_seqlens; plan.cu_k = bd.cu_k ? bd.cu_k : cu_seqlens; plan.kv_lo = bd.kv_lo; plan.kv_hi = bd.kv_hi;
-        plan.N = N; plan.Nk = Nk; plan.B = B; plan.Hk = Hk; plan.TPT = s.TPT;
+        plan.N = N; plan.Nk = Nk; plan.B = B; plan.Hk = Hk; plan.TPT = s.TPT; plan.aim = range_kv_items();
         plan.max_tiles = (int)range_kv_max_tiles(s);
         plan.counts = (int*)sp;
         plan.tiles = (int4*)(sp + 256);

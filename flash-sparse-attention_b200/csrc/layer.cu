@@ -196,8 +196,8 @@ extern "C" int fsa_layer_prep(const int32_t* cu_seqlens, int batch, int64_t max_
         return FSA_ERR_BAD_ARG;
     if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
     (void)cudaGetLastError();
-    const int64_t want = (max_len * (head_dim / 2) + 255) / 256;
-    const unsigned grid = (unsigned)(want < 1 ? 1 : want > 148 * 8 ? 148 * 8 : want);
+    const int64_t want = (max_len * (head_dim / 2) + 255) / 256, most = sm_count() * 8;
+    const unsigned grid = (unsigned)(want < 1 ? 1 : want > most ? most : want);
     if (dtype == FSA_DTYPE_BF16)
         layer_prep_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>(cu_seqlens, batch, max_len, inv_freq, head_dim / 2, kernel_size,
                                                                                 kernel_stride, (__nv_bfloat16*)cos_tab, (__nv_bfloat16*)sin_tab, cu_cmp);

@@ -265,7 +265,7 @@ static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, i
     // something to select; up to kLcShort windows (about 1000 tokens, 16 blocks of 64) a selection takes about everything.
     int S = 1, longest = 0;
     for (int b = 0; b < p.n_seq; ++b) longest = p.n_cmp[b] > longest ? p.n_cmp[b] : longest;
-    while (longest <= kLcShort && S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= 148) S *= 2;
+    while (longest <= kLcShort && S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= sm_count()) S *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)S, (unsigned)tiles, (unsigned)(p.H * nt));
     cfg.blockDim = dim3(192);

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(512) range_key_tiles(const RangeKvPlan p, uint
 }
 
 // Work items from the stretches (one CTA): a tile of n row tiles becomes ceil(n / C) items of about equal length, C the
-// smallest length that leaves about kRkItems items (times heads), and at least kRkMinTiles: below that an item's epilogue weighs
+// smallest length that leaves about p.aim items (times heads), and at least kRkMinTiles: below that an item's epilogue weighs
 // more than an idle SM.
 __global__ void __launch_bounds__(1024) range_plan_items(const RangeKvPlan p) {
     __shared__ int wa[32], wb[32], wc[32];
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(1024) range_plan_items(const RangeKvPlan p) {
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0) atomicAdd(reinterpret_cast<unsigned long long*>(&total), (unsigned long long)mine);
     __syncthreads();
-    const int C = max(kRkMinTiles, (int)((total * p.Hk + kRkItems - 1) / kRkItems));
+    const int C = max(kRkMinTiles, (int)((total * p.Hk + p.aim - 1) / p.aim));
     int items = 0, slabs = 0, multi = 0;              // so far
     for (int base = 0; base < p.max_tiles; base += 1024) {
         const int i = base + tid;
