@@ -2,6 +2,8 @@
 // that a CUDA graph can hold it).
 #include "host_common.h"
 
+#include <ATen/cuda/CUDAContext.h>
+
 #include <climits>
 #include <optional>
 
@@ -18,6 +20,8 @@ static DecodeCfg cfg_of(const std::vector<int64_t>& c, double scale) {
     return {(int)c[0], (int)c[1], (int)c[2], (int)c[3], (int)c[4], (int)c[5], (int)c[6], c[7], scale};
 }
 
+static int64_t sms() { return at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
+
 // Chunks of the compressed rows.  Work per CTA of the two attention passes: as long as possible (few partials, a ring of loads that
 // stays full) while about four CTAs per SM are left for each pass: a small batch is split finely, a full one takes 1024 rows /
 // 16 blocks at a time.
@@ -25,7 +29,7 @@ struct Chunks {
     int rows, n;
     Chunks(const DecodeCfg& c, int64_t heads) {
         const int64_t max_cmp = std::max<int64_t>(c.max_len >= c.ks ? (c.max_len - c.ks) / c.stride + 1 : 0, 1);
-        const int64_t per = (max_cmp * heads + 4 * 148 - 1) / (4 * 148);
+        const int64_t ctas = 4 * sms(), per = (max_cmp * heads + ctas - 1) / ctas;
         rows = (int)std::min<int64_t>(1024, std::max<int64_t>(64, (per + 63) / 64 * 64));
         n = (int)((max_cmp + rows - 1) / rows);
     }
@@ -58,7 +62,7 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, co
     const int chunk = chunks.rows, nchunk = chunks.n;
     const int npieces = (c.window + 1 + c.bs - 1) / c.bs, R = c.topk + npieces;
     int rpp = 16;
-    while (rpp > 1 && (c.topk % rpp || (int64_t)B * Hk * ((R + rpp - 1) / rpp) < 2 * 148)) rpp /= 2;
+    while (rpp > 1 && (c.topk % rpp || (int64_t)B * Hk * ((R + rpp - 1) / rpp) < 2 * sms())) rpp /= 2;
     const int ns = c.topk / rpp, nw = (npieces + rpp - 1) / rpp, P2 = ns + nw;
     const int64_t ld = (int64_t)chunk * nchunk;
     auto al = [](int64_t n) { return (n + 255) / 256 * 256; };
@@ -113,27 +117,23 @@ Outcome decode_mixed(const Tensor& q_, const Tensor& k, const Tensor& v, const T
 // The buffers of a DecodeCache, in this order: k, v, cmp_k, cmp_v, k_tail, v_tail, seq_len, seq_row0, cmp_row0.
 using Cache = std::vector<Tensor>;
 
-// Does the native step take this call?  k_new stands for the type and the device of everything.
-static bool served(const Cache& t, int64_t Hq, const Tensor& k_new, const Tensor& v_new, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
-                   const DecodeCfg& c, int64_t gate_dim) {
-    if (t.size() != 9 || k_new.dim() != 3 || !k_new.is_cuda()) return false;
-    const int64_t B = k_new.size(0), Hk = k_new.size(1), D = k_new.size(2);
-    if (!takes_sizes(B, Hq, Hk, D, c, gate_dim)) return false;
-    for (int i = 0; i < 6; ++i)
-        if (!packed_like(t[i], k_new, Hk) || !t[i].is_contiguous()) return false;
-    for (int i = 6; i < 9; ++i)
-        if (!lengths_like(t[i], k_new, B)) return false;
-    for (auto* w : {&v_new, &w_key, &w_value, &pe})
-        if (w->scalar_type() != k_new.scalar_type() || w->device() != k_new.device() || !w->is_contiguous() || ((uintptr_t)w->data_ptr() & 15)) return false;
-    const int64_t rows = t[0].size(0) - 1;        // (the last row of a buffer is a spare one)
-    return v_new.sizes() == k_new.sizes() && rows > 0 && rows % B == 0 && t[1].size(0) == rows + 1 && (t[2].size(0) - 1) % B == 0 &&
-           t[3].size(0) == t[2].size(0) && t[4].size(0) == B * c.ks + 1 && t[5].size(0) == t[4].size(0) &&
-           w_key.sizes() == at::IntArrayRef({Hk, c.ks * D, D}) && w_value.sizes() == w_key.sizes() && pe.sizes() == at::IntArrayRef({Hk, c.ks, D});
+static bool weight(const Tensor& w, const Tensor& x, at::IntArrayRef shape) {
+    return w.scalar_type() == x.scalar_type() && w.device() == x.device() && w.is_contiguous() && w.sizes() == shape && ((uintptr_t)w.data_ptr() & 15) == 0;
 }
 
-static bool weight(const Tensor& w, const Tensor& x, int64_t rows, int64_t cols) {
-    return w.scalar_type() == x.scalar_type() && w.device() == x.device() && w.is_contiguous() && w.sizes() == at::IntArrayRef({rows, cols}) &&
-           ((uintptr_t)w.data_ptr() & 15) == 0;
+// Does the native step take this call?  x stands for the type and the device of everything.
+static bool served(const Cache& t, const Tensor& x, int64_t Hq, int64_t D, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
+                   const DecodeCfg& c, int64_t gate_dim) {
+    if (t.size() != 9 || t[0].dim() != 3 || !x.is_cuda()) return false;
+    const int64_t B = x.size(0), Hk = t[0].size(1), rows = t[0].size(0) - 1;        // (the last row of a buffer is a spare one)
+    if (!takes_sizes(B, Hq, Hk, D, c, gate_dim) || rows <= 0 || rows % B || t[2].dim() != 3 || (t[2].size(0) - 1) % B) return false;
+    const int64_t cmp_rows = t[2].size(0) - 1, ring = B * c.ks;
+    const int64_t want[6] = {rows, rows, cmp_rows, cmp_rows, ring, ring};
+    for (int i = 0; i < 6; ++i)
+        if (!weight(t[i], x, {want[i] + 1, Hk, D})) return false;
+    for (int i = 6; i < 9; ++i)
+        if (!lengths_like(t[i], x, B)) return false;
+    return weight(w_key, x, {Hk, c.ks * D, D}) && weight(w_value, x, {Hk, c.ks * D, D}) && weight(pe, x, {Hk, c.ks, D});
 }
 
 // Append (with the gate from logits z, or from gx and its weight), compressor, attention.
@@ -162,11 +162,11 @@ Outcome decode_kernel_step(const Tensor& q_, const Tensor& k_, const Tensor& v_,
     c10::cuda::CUDAGuard guard(q_.device());
     const DecodeCfg c = cfg_of(cfg, scale);
     const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
-    if (q.dim() != 3 || k.dim() != 3 || q.size(0) != k.size(0) || q.size(2) != k.size(2) || q.scalar_type() != k.scalar_type() || q.device() != k.device() ||
-        ((uintptr_t)q.data_ptr() & 15) || ((uintptr_t)k.data_ptr() & 15))
+    if (q.dim() != 3 || k.dim() != 3 || !weight(k, q, {q.size(0), k.size(1), q.size(2)}) || !weight(v, q, k.sizes()) || ((uintptr_t)q.data_ptr() & 15) ||
+        t.size() != 9 || t[0].dim() != 3 || t[0].size(1) != k.size(1))
         return std::nullopt;
     const Tensor gx = q.view({q.size(0), -1});
-    if (!weight(gw, q, 3, gx.size(1)) || !served(t, q.size(1), k, v, w_key, w_value, pe, c, gx.size(1))) return std::nullopt;
+    if (!weight(gw, q, {3, gx.size(1)}) || !served(t, q, q.size(1), q.size(2), w_key, w_value, pe, c, gx.size(1))) return std::nullopt;
     auto [y, ids] = step(q, k, v, q, Tensor(), Tensor(), gx, gw, t, w_key, w_value, pe, compress, c);
     return std::make_tuple(y.view({y.size(0), -1}), ids);
 }
@@ -192,16 +192,14 @@ Outcome decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, 
                           bool compress, const std::vector<int64_t>& cfg, double scale) {
     c10::cuda::CUDAGuard guard(x_.device());
     const DecodeCfg c = cfg_of(cfg, scale);
-    const Tensor x = x_.contiguous().view({x_.size(0), -1});
+    const Tensor flat = x_.contiguous(), x = flat.dim() == 2 ? flat : flat.view({flat.size(0), -1});
     const int64_t B = x.size(0), hidden = x.size(1), nq = wq.size(0), nk = wk.size(0);
-    const bool skinny = B <= kProjRows && hidden % 256 == 0 && nq % 256 == 0 && ((uintptr_t)x.data_ptr() & 15) == 0;
-    if (t.size() != 9 || t[0].dim() != 3 || D <= 0 || nq % D || nk != t[0].size(1) * D || t[0].size(2) != D || ((uintptr_t)x.data_ptr() & 15) ||
-        inv_freq.scalar_type() != at::kFloat || inv_freq.device() != x.device() || inv_freq.numel() != D / 2 || !weight(wq, x, nq, hidden) ||
-        !weight(wk, x, nk, hidden) || !weight(wv, x, nk, hidden) || !weight(wo, x, wo.size(0), nq) || !weight(gw, x, 3, hidden))
+    const bool skinny = B <= kProjRows && hidden % 256 == 0 && nq % 256 == 0;
+    if (((uintptr_t)x.data_ptr() & 15) || t.size() != 9 || t[0].dim() != 3 || D <= 0 || nq % D || nk != t[0].size(1) * D ||
+        inv_freq.scalar_type() != at::kFloat || inv_freq.device() != x.device() || inv_freq.numel() != D / 2 || !weight(wq, x, {nq, hidden}) ||
+        !weight(wk, x, {nk, hidden}) || !weight(wv, x, {nk, hidden}) || !weight(wo, x, {wo.size(0), nq}) || !weight(gw, x, {3, hidden}) ||
+        !served(t, x, nq / D, D, w_key, w_value, pe, c, skinny ? 0 : hidden))
         return std::nullopt;
-    // (stands for the new keys and values, which are not projected yet)
-    const Tensor like = t[0].narrow(0, 0, std::min<int64_t>(B, t[0].size(0)));
-    if (like.size(0) != B || !served(t, nq / D, like, like, w_key, w_value, pe, c, skinny ? 0 : hidden)) return std::nullopt;
     Tensor q, k, v, z;
     if (skinny) {
         q = fresh({B, nq}, x);
