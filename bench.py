@@ -34,7 +34,7 @@ import torch  # noqa: E402
 
 # DRAM bytes (read + write) per launch of the main kernels from one ncu capture of the small case (one 16384-token
 # sequence of config 1); traffic grows with the token count, so config 1 is 4 x that.
-NCU_TRAFFIC_SMALL = {"sel_bwd_main": 210.3e6 + 582.7e6, "sel_fwd_main": 73.3e6 + 479.6e6}
+NCU_TRAFFIC_SMALL = {"sel_bwd_pipe": 210.3e6 + 582.7e6, "sel_fwd_main": 73.3e6 + 479.6e6}
 # the compressed pass of the decode step at batch 8, from one ncu capture; grows with the batch
 NCU_TRAFFIC_DECODE_B8 = 268.5e6 + 6.7e6
 
@@ -690,7 +690,9 @@ def run_sel(args, dd):
     ms_step = dd.max_ms(ev0.elapsed_time(ev1)) / args.steps
     # per-kernel durations recorded inside the timed region (library-owned events around each launch, this rank's)
     kern = {}
-    for name, kid in (("sel_fwd_main", 0), ("sel_fwd_reduce", 1), ("sel_bwd_main", 2), ("sel_bwd_dq_reduce", 3), ("sel_index_build", 4)):
+    bwd = "sel_bwd_wide" if d == 256 else "sel_bwd_pipe"
+    merges = ("sel_fwd_reduce", "sel_bwd_dq_reduce") if d == 256 else ("sel_merge (o)", "sel_merge (dQ)")
+    for name, kid in (("sel_fwd_main", 0), (merges[0], 1), (bwd, 2), (merges[1], 3), ("sel_index_build", 4)):
         ms, n = c_float(0), c_int(0)
         _lib.check(L.fsa_profile_read(kid, byref(ms), byref(n)), "fsa_profile_read")
         kern[name] = {"ms_avg": (ms.value / n.value if n.value else None), "launches": n.value}
@@ -750,8 +752,8 @@ def run_sel(args, dd):
         # the timed region is tens of milliseconds at full clocks: the burst figure is the denominator
         peak_tf, peak_src = tensor_peak(burst=True)
         # dominant kernel: the backward main kernel (10*d*P useful FLOPs per launch, P of this rank's shard)
-        dom = "sel_bwd_main" if (kern["sel_bwd_main"]["ms_avg"] or 0) >= (kern["sel_fwd_main"]["ms_avg"] or 0) else "sel_fwd_main"
-        dom_flops = (10 if dom == "sel_bwd_main" else 4) * d * P_r
+        dom = bwd if (kern[bwd]["ms_avg"] or 0) >= (kern["sel_fwd_main"]["ms_avg"] or 0) else "sel_fwd_main"
+        dom_flops = (10 if dom == bwd else 4) * d * P_r
         dom_ms = kern[dom]["ms_avg"]
         achieved = dom_flops / (dom_ms * 1e-3) / 1e12 if dom_ms else None
         cpu = None
@@ -774,14 +776,14 @@ def run_sel(args, dd):
             "kernels": kern,
             "roofline": {"bound": "tensor", "kernel": dom, "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s",
                          "frac": (achieved / peak_tf if achieved else None),
-                         "traffic": (NCU_TRAFFIC_SMALL[dom] * (4 if args.case == "cfg1" else 1) * P_r / P_all) if args.case != "cfg2" else None,
+                         "traffic": (NCU_TRAFFIC_SMALL[dom] * (4 if args.case == "cfg1" else 1) * P_r / P_all) if args.case != "cfg2" and dom in NCU_TRAFFIC_SMALL else None,
                          "traffic_source": "ncu capture of the small case scaled by the token count", "peak_source": peak_src},
             "cpu_baseline": cpu,
             "e2e": ({"value": flops_step / (e2e_ms * 1e-3) / 1e12, "unit": UNIT, "ms_per_step": e2e_ms,
                      "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 12 * world,
                      "overlap": "copies of step i+1 on a second stream while step i computes"} if e2e_ms else None),
-            # kernels of this library per step: 5 of the index build, forward main + merge, delta, backward main,
-            # dQ merge, dK/dV slab reduce (the two memsets of dk / dv are not kernels)
+            # kernels of this library per step: 4 of the index build, forward main + merge, delta, backward main,
+            # dQ merge, dK/dV slab reduce
             "gpu_launches": 10 * args.steps,
             "clocks": clocks,
         }
