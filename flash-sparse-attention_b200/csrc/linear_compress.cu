@@ -17,7 +17,7 @@
 //
 // The reduction over ks * d is one serial chain of MMAs behind a ring of loads: 26 us at ks * d = 4096 however few windows
 // there are.  When short sequences leave SMs idle the chain is cut in up to eight, one CTA of a cluster each, whose fp32 sums meet
-// through distributed shared memory (517 tokens, 8 heads, K and V: two launches of 26 us before).  One launch takes up to
+// through distributed shared memory (517 tokens, 8 heads, K and V, inside a layer: 19 us for both, two launches of 26 us before).  One launch takes up to
 // kLcSeqs sequences, whose tensor maps travel as kernel parameters.
 #include "../../include/fsa_sm100.h"
 #include <cooperative_groups.h>
@@ -261,8 +261,9 @@ static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, i
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     // CTAs per tile: as many as still find an SM of their own (the ring takes one SM's shared memory).  Short sequences only: another
-    // order of the sum moves the last bit of a compressed row, and with it near ties of a block selection where there is
-    // something to select; up to kLcShort windows (about 1000 tokens, 16 blocks of 64) a selection takes about everything.
+    // order of the sum moves the last bit of a compressed row, and with it near ties of a block selection.  Up to kLcShort windows
+    // (about 1000 tokens at stride 16, 16 blocks of 64) a selection of 16 blocks of 64 takes them all; a smaller one, or one of 32-key
+    // blocks, does choose there.  The split goes by all sequences of the launch, so a sequence's last bits may depend on its batch.
     int S = 1, longest = 0;
     for (int b = 0; b < p.n_seq; ++b) longest = p.n_cmp[b] > longest ? p.n_cmp[b] : longest;
     while (longest <= kLcShort && S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= sm_count()) S *= 2;

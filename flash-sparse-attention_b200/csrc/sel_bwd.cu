@@ -1,4 +1,6 @@
-// Selected-attention backward for sm_100a.
+// Selected-attention backward for sm_100a: delta, the unpipelined main kernel, the sums of its partial results, and the dispatch.
+// The main kernels in ordinary use are sel_bwd_pipe.cu (head sizes 64 and 128) and sel_bwd_wide.cu (256); the one here serves q or
+// dO whose rows lie further apart than their 32-bit offsets reach (2^34 elements in all).
 //
 // One KV-major kernel does all five products of the backward (the reference runs S and dP
 // twice: once in backward_dkdv, fsa/ops/FSA_topk_sparse_attention.py:1548-1712, once in

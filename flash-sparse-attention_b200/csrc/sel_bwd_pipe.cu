@@ -1,4 +1,4 @@
-// Selected-attention backward, pipelined kernel for head_dim 64 and 128 (256: sel_bwd.cu).  Blocks of 128 and 256 keys are
+// Selected-attention backward, pipelined kernel for head_dim 64 and 128 (256: sel_bwd_wide.cu).  Blocks of 128 and 256 keys are
 // walked as independent 64-key parts, every part a pass over the tiles of its own (the gathers are repeated, which costs less
 // than the registers and TMEM of a wider tile: 21008 tokens, 128-key blocks, 734 us in the unpipelined kernel before).
 // Per tile of <= 128 (head, token) rows of one part of a KV block

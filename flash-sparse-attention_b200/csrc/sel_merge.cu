@@ -7,7 +7,7 @@
 // rows laid out in one contiguous piece took it no less time).  Here a CTA stays on its SM and each of 24 warps keeps 8 KB of
 // rows in flight: one bulk copy per partial row into the warp's own ring of stages, whose positions were loaded two rows before;
 // nothing passes through registers.  (With 12 warps and 16 KB each the arithmetic of a warp holds its stages up: dQ 503 us.)
-// 64K tokens x 8 heads x 16 rows of 256 bytes: forward 502 -> 425 us, dQ 476 -> 361 us = 6 TB/s.  At head size 256 a
+// 64K tokens x 8 heads x 16 rows of 256 bytes: forward 502 -> 420 us, dQ 476 -> 361 us = 5.1 and 5.9 TB/s of partial rows.  At head size 256 a
 // warp per row already moves 5.9 TB/s and keeps the other kernels; at 64 a row's arithmetic is too much for 24 warps (151 -> 193 us
 // forward at 16384 tokens x 16 heads), so that half a warp takes a row there (forward 144 us, dQ 157 -> 137 us).
 #include "sel_launch.cuh"
