@@ -93,6 +93,8 @@ class FlashSparseAttention(torch.nn.Module):
         cu_seqlens = cu_seqlens.to(torch.int32)
         if seqlens is None:
             seqlens = (cu_seqlens[1:] - cu_seqlens[:-1]).tolist()
+        elif not isinstance(seqlens, (list, tuple)):
+            seqlens = [int(n) for n in seqlens]
         max_len = max(seqlens) if len(seqlens) else 0
         cmp_lens = compressed_seqlens(seqlens, self.kernel_size, self.kernel_stride)
         max_cmp = max(cmp_lens) if len(cmp_lens) else 0

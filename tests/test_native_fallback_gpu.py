@@ -2,6 +2,7 @@
 and what no path takes raises."""
 import copy
 
+import numpy as np
 import pytest
 import torch
 
@@ -80,6 +81,29 @@ def test_layer_keeps_a_scaled_or_hooked_rotation():
     layer.rope.register_forward_hook(lambda m, i, o: calls.append(1))
     assert torch.equal(layer(x, cu, [500, 200]), y) and len(calls) == 3
     assert not torch.equal(scaled(x, cu, [500, 200]), y)
+
+
+@pytest.mark.parametrize("kind", ["list", "tuple", "array", "tensor", "none"])
+@pytest.mark.parametrize("lens", [[500, 200], [300, 0, 400], [0, 31, 669, 0]])
+def test_layer_takes_lengths_of_any_kind(kind, lens):
+    layer, x, _ = _layer()
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    given = dict(list=lens, tuple=tuple(lens), array=np.asarray(lens), tensor=torch.tensor(lens), none=None)[kind]
+
+    def grads():
+        xl = x.clone().requires_grad_(True)
+        layer.zero_grad(set_to_none=True)
+        y = layer(xl, cu, given)
+        y.backward(x.flip(0) if y.shape == x.shape else torch.ones_like(y))
+        return [y.detach(), layer.last_topk_idx, xl.grad] + [p.grad for p in layer.parameters()]
+
+    got = grads()
+    hook = layer.gate.register_forward_hook(lambda m, i, o: None)
+    want = grads()
+    hook.remove()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    for a, b in zip(got[2:], want[2:]):       # (sums of the branches' gradients rounded once here, at every sum there)
+        assert float((a.float() - b.float()).norm()) <= 1e-2 * float(b.float().norm())
 
 
 NSA = dict(kernel_size=32, kernel_stride=16, block_size=64, topk=8, init_blocks=1, local_blocks=2, window_size=100)
