@@ -5,6 +5,7 @@
 #include "sel_common.cuh"
 #include "range_bwd.cuh"
 
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -139,8 +140,13 @@ int device_sm_count(int* out) {
 }
 
 int sm_count() {
-    int n = 0;
-    return device_sm_count(&n) == FSA_OK && n > 0 ? n : 148;
+    // (asked for several times a call: the first device's answer stands for the process, whose size queries and launches must agree)
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    if (device_sm_count(&n) != FSA_OK || n <= 0) return 148;
+    known.store(n, std::memory_order_relaxed);
+    return n;
 }
 
 // ---- optional kernel timing: a ring of event pairs per kernel id

@@ -2,6 +2,7 @@
 // that a CUDA graph can hold it).
 #include "host_common.h"
 
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 
 #include <climits>
@@ -20,7 +21,10 @@ static DecodeCfg cfg_of(const std::vector<int64_t>& c, double scale) {
     return {(int)c[0], (int)c[1], (int)c[2], (int)c[3], (int)c[4], (int)c[5], (int)c[6], c[7], scale};
 }
 
-static int64_t sms() { return at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
+static int64_t sms() {
+    static const int64_t n = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    return n;
+}
 
 // Chunks of the compressed rows.  Work per CTA of the two attention passes: as long as possible (few partials, a ring of loads that
 // stays full) while about four CTAs per SM are left for each pass: a small batch is split finely, a full one takes 1024 rows /
@@ -121,10 +125,13 @@ static bool weight(const Tensor& w, const Tensor& x, at::IntArrayRef shape) {
     return w.scalar_type() == x.scalar_type() && w.device() == x.device() && w.is_contiguous() && w.sizes() == shape && ((uintptr_t)w.data_ptr() & 15) == 0;
 }
 
+// (under autocast the parts' library products take other types than their operands')
+static bool native_call(const Tensor& x) { return x.is_cuda() && !at::autocast::is_autocast_enabled(at::kCUDA); }
+
 // Does the native step take this call?  x stands for the type and the device of everything.
 static bool served(const Cache& t, const Tensor& x, int64_t Hq, int64_t D, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
                    const DecodeCfg& c, int64_t gate_dim) {
-    if (t.size() != 9 || t[0].dim() != 3 || !x.is_cuda()) return false;
+    if (t.size() != 9 || t[0].dim() != 3) return false;
     const int64_t B = x.size(0), Hk = t[0].size(1), rows = t[0].size(0) - 1;        // (the last row of a buffer is a spare one)
     if (!takes_sizes(B, Hq, Hk, D, c, gate_dim) || rows <= 0 || rows % B || t[2].dim() != 3 || (t[2].size(0) - 1) % B) return false;
     const int64_t cmp_rows = t[2].size(0) - 1, ring = B * c.ks;
@@ -159,6 +166,7 @@ static std::tuple<Tensor, Tensor> step(const Tensor& q_in, const Tensor& k_new, 
 // FlashSparseAttentionDecodeKernel.step: q, k_new, v_new in, [B, Hq * D] and the block ids out.
 Outcome decode_kernel_step(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gw, const Cache& t, const Tensor& w_key,
                            const Tensor& w_value, const Tensor& pe, bool compress, const std::vector<int64_t>& cfg, double scale) {
+    if (!native_call(q_)) return std::nullopt;
     c10::cuda::CUDAGuard guard(q_.device());
     const DecodeCfg c = cfg_of(cfg, scale);
     const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
@@ -190,6 +198,7 @@ static void project(const Tensor& x, std::initializer_list<Tensor> ws, std::init
 Outcome decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo, const Tensor& gw,
                           const Tensor& inv_freq, int64_t D, const Cache& t, const Tensor& w_key, const Tensor& w_value, const Tensor& pe,
                           bool compress, const std::vector<int64_t>& cfg, double scale) {
+    if (!native_call(x_)) return std::nullopt;
     c10::cuda::CUDAGuard guard(x_.device());
     const DecodeCfg c = cfg_of(cfg, scale);
     const Tensor flat = x_.contiguous(), x = flat.dim() == 2 ? flat : flat.view({flat.size(0), -1});

@@ -47,13 +47,6 @@ inline Tensor i32(at::IntArrayRef shape, const Tensor& like) { return fresh(shap
 inline const int32_t* iptr(const Tensor& t) { return t.defined() ? t.data_ptr<int32_t>() : nullptr; }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
-// Every tensor is contiguous, on x's device and of x's type (the kernels take raw pointers).
-inline void same_kind(const Tensor& x, std::initializer_list<const Tensor*> ts, const char* what) {
-    for (auto* t : ts)
-        TORCH_CHECK(t->scalar_type() == x.scalar_type() && t->device() == x.device() && t->is_contiguous(), what, ": expected contiguous ",
-                    x.scalar_type(), " on ", x.device(), ", got ", t->scalar_type(), " on ", t->device());
-}
-
 inline bool wants_grad(std::initializer_list<const Tensor*> ts) {
     if (!at::GradMode::is_enabled()) return false;
     for (auto* t : ts)

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime_api.h>
 
+#include <optional>
+
 namespace fsa_host {
 
 struct LayerCfg {
@@ -208,11 +210,13 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
     }
 };
 
-std::tuple<Tensor, Tensor> nsa_layer(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wg, const Tensor& w_key,
+// Nothing where a weight is of another type, device or memory order than the kernels read (the layer then runs as its parts).
+std::optional<std::tuple<Tensor, Tensor>> nsa_layer(const Tensor& x_, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wg, const Tensor& w_key,
                                      const Tensor& w_value, const Tensor& pe, const Tensor& inv_freq, const Tensor& cu,
                                      const std::vector<int64_t>& seqlens, const std::vector<int64_t>& cfg) {
     c10::cuda::CUDAGuard guard(x_.device());
-    same_kind(x_, {&wq, &wk, &wv, &wg, &w_key, &w_value, &pe}, "layer");
+    for (auto* w : {&wq, &wk, &wv, &wg, &w_key, &w_value, &pe})
+        if (w->scalar_type() != x_.scalar_type() || w->device() != x_.device() || !w->is_contiguous()) return std::nullopt;
     {
         // (raw pointers from here on; the lengths agree with x and cu: _native of fsa/module/fsa.py)
         const LayerCfg c = layer_cfg(cfg);
@@ -220,19 +224,19 @@ std::tuple<Tensor, Tensor> nsa_layer(const Tensor& x_, const Tensor& wq, const T
         TORCH_CHECK_VALUE(wq.sizes() == at::IntArrayRef({q, hidden}) && wk.sizes() == at::IntArrayRef({kv, hidden}) &&
                               wv.sizes() == wk.sizes() && wg.sizes() == at::IntArrayRef({3, hidden}) &&
                               w_key.sizes() == at::IntArrayRef({c.Hk, (int64_t)c.ks * c.D, c.D}) && w_value.sizes() == w_key.sizes() &&
-                              pe.sizes() == at::IntArrayRef({c.Hk, c.ks, c.D}),
-                          "layer: a weight has another shape than the layer's settings");
+                              pe.sizes() == at::IntArrayRef({c.Hk, c.ks, c.D}) && inv_freq.numel() == c.D / 2,
+                          "layer: a weight or the rotation has another shape than the layer's settings");
     }
     const Tensor x = x_.stride(1) == 1 && x_.stride(0) % 8 == 0 && ((uintptr_t)x_.data_ptr() & 15) == 0 ? x_ : x_.contiguous();
     if (wants_grad({&x, &wq, &wk, &wv, &wg, &w_key, &w_value, &pe})) {
         auto r = NsaLayer::apply(x, wq, wk, wv, wg, w_key, w_value, pe, inv_freq, cu, seqlens, cfg);
-        return {r[0], r[1]};
+        return std::make_tuple(r[0], r[1]);
     }
     const LayerCfg c = layer_cfg(cfg);
     const Lengths s(seqlens, c);
     Kept t;
     Tensor out = layer_fwd(x, wq, wk, wv, wg, w_key, w_value, pe, inv_freq, cu, s, c, t);
-    return {out, t.topk};
+    return std::make_tuple(out, t.topk);
 }
 
 void bind_layer(pybind11::module& m) { m.def("nsa_layer", &nsa_layer); }

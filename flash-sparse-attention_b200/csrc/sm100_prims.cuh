@@ -26,7 +26,7 @@ cudaError_t allow_smem(const void* kern, int bytes);
 // 32 heads, 16 rows each).
 // smem_percent: the share that stays shared memory, for a kernel that uses some.
 cudaError_t prefer_l1(const void* kern, int smem_percent = 0);
-// SMs of the current device; a B200's where no device answers (the size queries need none).
+// SMs of this process's device, for the rules that sizes and launches share; a B200's where no device answers (size queries need none).
 int sm_count();
 // Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
 int ensure_context();

@@ -42,10 +42,5 @@ def plain_gate(m: torch.nn.Module) -> bool:
             and not hooked(m) and not hooked(m[1]))
 
 
-def plain_weights(x: torch.Tensor, *weights: torch.Tensor) -> bool:
-    """Weights whose memory the native functions can take as it is, beside an input ``x``."""
-    return all(w.dtype == x.dtype and w.device == x.device and w.is_contiguous() for w in weights)
-
-
 def hooked(m: torch.nn.Module):
     return m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks

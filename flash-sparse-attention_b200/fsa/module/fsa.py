@@ -10,7 +10,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from fsa._host import host, plain_gate, plain_linear, plain_weights
+from fsa._host import host, plain_gate, plain_linear
 from fsa.module.rope import RopeConfig, RotaryEmbedding
 from fsa.ops.compressed_attention import _FUSED_TAPS, compressed_attention
 from fsa.ops.FSA_topk_sparse_attention import FSA_topk_sparse_attention
@@ -70,8 +70,9 @@ class FlashSparseAttention(torch.nn.Module):
             torch.nn.init.xavier_uniform_(p)
 
     def _native(self, x: torch.Tensor, cu_seqlens: torch.Tensor, seqlens, n_cmp: int) -> bool:
-        """Does the one native function serve this call?  It needs the modules to be what the constructor made of them, one type
-        throughout and the shapes that the fused kernels are compiled for; anything else runs as its parts below."""
+        """Does the one native function serve this call?  It needs the modules to be what the constructor made of them and the shapes
+        that the fused kernels are compiled for; anything else runs as its parts below.  (Whether the weights are of x's type and in
+        order the function sees itself.)"""
         return (x.is_cuda and x.dim() == 2 and n_cmp > 0 and self.head_dim in (64, 128) and sum(seqlens) == x.shape[0]
                 and cu_seqlens.numel() == len(seqlens) + 1 and cu_seqlens.device == x.device
                 and self.kernel_size in (16, 32, 64, 128) and self.kernel_size % self.kernel_stride == 0
@@ -79,10 +80,8 @@ class FlashSparseAttention(torch.nn.Module):
                 and (self.kernel_size // self.kernel_stride, self.block_size // self.kernel_stride) in _FUSED_TAPS
                 and self.kernel_stride & (self.kernel_stride - 1) == 0
                 and max(1, self.init_blocks + self.local_blocks) <= self.topk <= 32 and self.num_q_heads <= 32 * self.num_kv_heads
-                and self.hidden_size % 8 == 0 and self.hidden_size <= 16384 and type(self.rope) is RotaryEmbedding and self.rope.plain(self.head_dim)
+                and self.hidden_size % 8 == 0 and self.hidden_size <= 16384 and type(self.rope) is RotaryEmbedding and self.rope.plain()
                 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v) and plain_gate(self.gate)
-                and plain_weights(x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.gate[0].weight, self.compress_key,
-                                  self.compress_value, self.intra_block_pe)
                 and not torch.is_autocast_enabled())
 
     def forward(self, x: torch.Tensor, cu_seqlens: torch.Tensor, seqlens: Optional[Sequence[int]] = None):
@@ -100,12 +99,14 @@ class FlashSparseAttention(torch.nn.Module):
         max_cmp = max(cmp_lens) if len(cmp_lens) else 0
 
         if self._native(x, cu_seqlens, seqlens, sum(cmp_lens)):
-            attn_output, self.last_topk_idx = host().nsa_layer(
+            done = host().nsa_layer(
                 x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.gate[0].weight, self.compress_key, self.compress_value,
                 self.intra_block_pe, self.rope.inv_freq_on(x.device), cu_seqlens.contiguous(), seqlens,
                 [self.num_q_heads, self.num_kv_heads, self.head_dim, self.kernel_size, self.kernel_stride, self.block_size, self.topk,
                  self.init_blocks, self.local_blocks, self.window_size])
-            return self.proj_o(attn_output)
+            if done is not None:
+                attn_output, self.last_topk_idx = done
+                return self.proj_o(attn_output)
 
         q = self.proj_q(x).view(-1, self.num_q_heads, self.head_dim)
         k = self.proj_k(x).view(-1, self.num_kv_heads, self.head_dim)

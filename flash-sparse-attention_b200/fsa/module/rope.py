@@ -105,9 +105,9 @@ class RotaryEmbedding(nn.Module):
             self._inv_freq = self._inv_freq.to(device)
         return self._inv_freq
 
-    def plain(self, head_dim: int) -> bool:
+    def plain(self) -> bool:
         """Are cos and sin of position * inv_freq all that a call does?  (The native functions form the angles themselves.)"""
-        return self.attention_scaling == 1.0 and 2 * self._inv_freq.numel() == head_dim and not hooked(self)
+        return self.attention_scaling == 1.0 and not hooked(self)
 
     @torch.no_grad()
     def generate_cos_sin(self, x: torch.Tensor, position_ids: torch.Tensor):

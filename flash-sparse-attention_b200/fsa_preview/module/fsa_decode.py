@@ -86,21 +86,21 @@ class FlashSparseAttentionDecode(torch.nn.Module):
     @torch.no_grad()
     def step(self, x: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """``x [B, hidden]``: one new token per sequence -> ``[B, hidden]``; appends to ``cache``."""
-        B = x.shape[0]
-        if B != cache.B or x.numel() != B * self.hidden_size:
-            raise ValueError(f"x [{cache.B}, {self.hidden_size}] expected (one token for every sequence of the cache), got {list(x.shape)}")
-        if (x.is_cuda and cache.shard.world == 1 and plain_linear(self.proj_q) and plain_linear(self.proj_k) and plain_linear(self.proj_v)
-                and plain_linear(self.proj_o) and plain_gate(self.gate) and type(self.rope) is RotaryEmbedding and self.rope.plain(self.head_dim)
-                and not torch.is_autocast_enabled()):
+        # (every look-up of a sub-module costs a step a quarter of a microsecond: once each)
+        pq, pk, pv, po, gate, rope = self.proj_q, self.proj_k, self.proj_v, self.proj_o, self.gate, self.rope
+        if (cache.shard.world == 1 and plain_linear(pq) and plain_linear(pk) and plain_linear(pv) and plain_linear(po) and plain_gate(gate)
+                and type(rope) is RotaryEmbedding and rope.plain()):
             new_len, compress = cache.advanced()
             done = host().decode_layer_step(
-                x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight, self.proj_o.weight, self.gate[0].weight,
-                self.rope.inv_freq_on(x.device), self.head_dim, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
-                compress, step_settings(self, cache.max_len), 0.0)
-            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts)
+                x, pq.weight, pk.weight, pv.weight, po.weight, gate[0].weight, rope.inv_freq_on(x.device), self.head_dim, cache.buffers(),
+                self.compress_key, self.compress_value, self.intra_block_pe, compress, step_settings(self, cache.max_len), 0.0)
+            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts, or an error)
                 cache.host_len = new_len
                 y, self.last_topk_idx = done
                 return y
+        B = x.shape[0]
+        if B != cache.B or x.numel() != B * self.hidden_size:
+            raise ValueError(f"x [{cache.B}, {self.hidden_size}] expected (one token for every sequence of the cache), got {list(x.shape)}")
         pos = cache.seq_len.clone()                                   # position of the new token
         q = self.proj_q(x).view(B, self.num_q_heads, self.head_dim)
         k_new = self.proj_k(x).view(B, self.num_kv_heads, self.head_dim)

@@ -44,19 +44,20 @@ class FlashSparseAttentionDecodeKernel(torch.nn.Module):
     @torch.no_grad()
     def step(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, cache: DecodeCache) -> torch.Tensor:
         """One token per sequence: ``q [B, Hq, d]``, ``k_new / v_new [B, Hk, d]`` -> ``[B, Hq*d]``; appends to ``cache``."""
+        gate = self.gate
+        if cache.shard.world == 1 and plain_gate(gate):
+            new_len, compress = cache.advanced()
+            done = host().decode_kernel_step(
+                q, k_new, v_new, gate[0].weight, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
+                compress, step_settings(self, cache.max_len), 0.0)
+            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts, or an error)
+                cache.host_len = new_len
+                out, self.last_topk_idx = done
+                return out
         kv = (cache.B, self.num_kv_heads, self.head_dim)
         if q.shape != (cache.B, self.num_q_heads, self.head_dim) or k_new.shape != kv or v_new.shape != kv:
             raise ValueError(f"q [{cache.B}, {self.num_q_heads}, {self.head_dim}] and k_new, v_new {list(kv)} expected (one token for every "
                              f"sequence of the cache), got {list(q.shape)}, {list(k_new.shape)}, {list(v_new.shape)}")
-        if q.is_cuda and cache.shard.world == 1 and plain_gate(self.gate) and not torch.is_autocast_enabled():
-            new_len, compress = cache.advanced()
-            done = host().decode_kernel_step(
-                q, k_new, v_new, self.gate[0].weight, cache.buffers(), self.compress_key, self.compress_value, self.intra_block_pe,
-                compress, step_settings(self, cache.max_len), 0.0)
-            if done is not None:          # (else the kernels do not take these sizes, types or layouts: the step as its parts)
-                cache.host_len = new_len
-                out, self.last_topk_idx = done
-                return out
         cache.append(k_new, k_new, v_new, self.compress_key, self.compress_value, self.intra_block_pe, None)
         q = q.contiguous()
         gate = self.gate(q.view(q.shape[0], -1))

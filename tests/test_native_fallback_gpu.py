@@ -197,3 +197,14 @@ def test_decode_refuses_what_does_not_fit_the_cache_and_leaves_it_alone(hidden):
     for x, z in zip(c.buffers(), before):
         assert torch.equal(x, z)
     assert torch.equal(half.seq_len, before[6])
+
+
+def test_decode_under_autocast_runs_as_parts():
+    """Weights of 32 bits under autocast: the parts' products take 16-bit operands."""
+    mod, cache, new = _decode(256, 4, 2, 128, [95, 130], 300)
+    wide = copy.deepcopy(mod).float()
+    a, b, ins = cache(), cache(), new()
+    y = mod.step(*ins, a)
+    with torch.autocast("cuda", torch.bfloat16):
+        y2 = wide.step(*ins, b)
+    assert float((y2 - y).abs().max()) <= 2.0 ** -6 * float(y.abs().max()) and b.host_len == [96, 131]
