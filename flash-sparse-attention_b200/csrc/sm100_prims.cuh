@@ -83,32 +83,29 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity
         : "memory");
     return ok;
 }
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+__device__ __forceinline__ uint32_t clock32() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t)::"memory");
     return t;
 }
-// Bounded wait: polls until the phase completes, FSA_WAIT_NS nanoseconds have passed, or
-// another thread of the grid has already recorded a failure in the status word.  Returns false
-// (and records the failure) in the last two cases; the caller keeps going so that TMEM is
-// freed and the kernel returns.
-#ifndef FSA_WAIT_NS
-#define FSA_WAIT_NS 200000000ull   // 0.2 s
+// Bounded wait: polls until the phase completes or FSA_WAIT_CLOCKS cycles of the SM have passed (each try_wait already
+// sleeps for a while in hardware) and returns false in the second case; the caller keeps going so that TMEM is freed and
+// the kernel returns.  mbar_wait records the failure in the status word; mbar_poll leaves that to the caller, once for all
+// its waits.  Kept short on purpose: a warp-specialised kernel has some 25 waits, and the loops of its roles together have
+// to stay in the SM's instruction cache (sel_bwd_pipe.cu).
+#ifndef FSA_WAIT_CLOCKS
+#define FSA_WAIT_CLOCKS 400000000u   // 0.2 s at 1.965 GHz; less than the 2^32 at which the counter comes round
 #endif
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
+    const uint32_t t0 = clock32();
+#pragma unroll 1
+    do {
+        if (mbar_try_wait(bar, parity)) return true;
+    } while (clock32() - t0 < FSA_WAIT_CLOCKS);
+    return false;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status) {
-    // fast path: no timer, no status read (each try_wait already sleeps for a while in hardware)
-#pragma unroll 1
-    for (int it = 0; it < 256; ++it)
-        if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = global_timer_ns();
-#pragma unroll 1
-    for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 63u) == 0) {
-            if (status && *reinterpret_cast<volatile int*>(status) != 0) return false;
-            if (global_timer_ns() - t0 > FSA_WAIT_NS) break;
-        }
-    }
+    if (mbar_poll(bar, parity)) return true;
     if (status) atomicMax(status, (int)kStatusWaitTimeout);
     return false;
 }
