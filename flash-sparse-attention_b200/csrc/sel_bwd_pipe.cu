@@ -6,12 +6,12 @@
 //     dK^T += Q^T dS, dV^T += dO^T P
 // Warp roles (768 threads in six warpgroups whose register budgets are rebalanced with setmaxnreg; one CTA per SM,
 // persistent over a round-robin run schedule):
-//   warps 0..7   gather Q and dO rows with 16-byte async copies (two stages);
-//   warp 8       issues S and dP (tcgen05, fp32 in TMEM, two buffers);
-//   warp 9       issues dQ, dK^T, dV^T;
-//   warp 10      prepares, up to four tiles ahead, the token of every tile row (the gather warps then run without
+//   warps 0..7   gather the dO rows, then the Q rows with 16-byte async copies (two stages);
+//   warp 8       issues dP, then S (tcgen05, fp32 in TMEM, two buffers);
+//   warp 9       issues dV^T, dK^T, dQ;
+//   warp 10      prepares, two tiles ahead, the offset of every tile row (the gather warps then run without
 //                any global load of their own: a plain load issued behind a burst of async copies waits for it);
-//   warp 11      loads the K/V block of every run of tiles by TMA;
+//   warp 11      loads the K/V block of every segment by TMA;
 //   warps 12..15 the accumulator drain, one row / one head-dim index per thread: for every tile the dQ partial from TMEM
 //                through a swizzled staging area to global memory by TMA store (input dtype, tile order: the load/store
 //                unit is left to the row gathers); at the end of a segment (the tiles of one block inside one
@@ -22,6 +22,18 @@
 //   warps 16..23 two groups, one row per thread, each on half of the 64 key columns of every tile: P / dS to swizzled smem
 //                and nothing else -- they are the critical path of a tile (the exp2 and the dS arithmetic between two
 //                MMA phases), so both groups shorten the same tile instead of alternating tiles.
+// What bounds it: the dependent chain of a tile (gather of 64 KB, S / dP, P / dS, dV / dK) with two stages of Q / dO.  Hence
+//   - dO and Q are separate stages: dV is issued before dK and gives dO back first, the gather brings dO back first, and dP,
+//     the factor scale (dP - delta) and the product of the tile before run under the gather of Q (in one stage, and with dK
+//     and dV interleaved: 1115 and 1060 us instead of 1000);
+//   - K has two stages and V is given back after the last dP of a segment, so that a segment starts while the one before it
+//     ends; the 16 KB come from staging dQ 64 columns at a time;
+//   - the loops of all roles together stay in the SM's instruction cache: no division per tile (cursors), rolled loops where
+//     nothing waits for the issue, short waits, segment records from the preparation warp instead of in every role.  With
+//     65 KB of code the issue slots found no instruction 1.7 times per instruction issued, with 43 KB 0.2 times; the new
+//     stages in 74 KB of code: 7.6 times, 1600 us.
+// 64K tokens x 8 heads x 16 blocks (CUDA events): 1190 us; with the short waits alone 1099; now 1000.  21K ragged tokens,
+// 128-key blocks: 235 -> 205 us.
 #include "sel_launch.cuh"
 
 namespace fsa {
@@ -44,22 +56,22 @@ struct SelBwdPipeParams {
 
 namespace bwdpipe {
 constexpr int KT = 64;
-constexpr int kKVStages = 1;                     // (a second K/V stage and the dQ staging area compete for the same 32 KB)
+constexpr int kKStages = 2;                      // K; V has one: its last reader, dP, is early in a tile
 constexpr int kThreads = 768, kLoaders = 256;
 constexpr int kWLoad = kLoaders / 32, kWMma1 = kWLoad, kWMma2 = kWLoad + 1, kWFlush = kWLoad + 4, kWGroups = kWLoad + 8;
 // registers per thread of each role (multiples of 8); 32 * sum over warps <= 768 * 80 = the CTA's allocation
-constexpr int kRegLoad = 40, kRegMma = 48, kRegFlush = 96, kRegGroup = 128;
+constexpr int kRegLoad = 32, kRegMma = 64, kRegFlush = 96, kRegGroup = 128;
 static_assert(8 * kRegLoad + 4 * kRegMma + 4 * kRegFlush + 8 * kRegGroup <= 24 * 80, "register budget");
 constexpr int kPS = 2 * kTileRows * KT * 2;      // P then dS: 32 KB
-constexpr int kTail = 2560;
+constexpr int kTail = 2624;
 constexpr int cS = 0, cDP = 64;                  // + 128 * buffer
 constexpr int cDQ = 256, cDK = 384, cDV = 448;
 constexpr uint32_t kCols = 512;
 template <int D> struct Cfg {
-    static constexpr int kKV = 2 * KT * D * 2;              // K then V
+    static constexpr int kK = KT * D * 2;                   // one of K, V
     static constexpr int kQD = 2 * kTileRows * D * 2;       // Q then dO
-    static constexpr int kDQ = kTileRows * D * 2;           // dQ staging, a quarter per TMEM lane quarter
-    static constexpr int kBytes = kKVStages * kKV + 2 * kQD + kPS + kDQ + kTail;
+    static constexpr int kDQ = kTileRows * 64 * 2;          // dQ staging, 64 columns at a time, a quarter per TMEM lane quarter
+    static constexpr int kBytes = (kKStages + 1) * kK + 2 * kQD + kPS + kDQ + kTail;
     static_assert(kBytes <= 227 * 1024, "smem budget");
 };
 }  // namespace bwdpipe
@@ -95,33 +107,43 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                                                                      const __grid_constant__ CUtensorMap vmap,
                                                                      const __grid_constant__ CUtensorMap dqmap) {
     using namespace bwdpipe;
-    constexpr int kKV = Cfg<D>::kKV, kQD = Cfg<D>::kQD, kDQ = Cfg<D>::kDQ;
+    constexpr int kK = Cfg<D>::kK, kQD = Cfg<D>::kQD, kDQ = Cfg<D>::kDQ;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sKV = smem;
-    uint8_t* sQD = sKV + kKVStages * kKV;
+    uint8_t* sK = smem;                                     // K stages, then V
+    uint8_t* sV = sK + kKStages * kK;
+    uint8_t* sQD = sV + kK;
     uint8_t* sP = sQD + 2 * kQD;
     uint8_t* sDS = sP + kTileRows * KT * 2;
     uint8_t* sDQ = sP + kPS;
     uint8_t* tail = sDQ + kDQ;
-    int (*s_tok)[kTileRows] = reinterpret_cast<int (*)[kTileRows]>(tail);                // [4][128] token of every tile row, -1 padding
+    int2 (*s_off)[kTileRows] = reinterpret_cast<int2 (*)[kTileRows]>(tail);              // [2][128] offset of every tile row in q and dO (units of
+                                                                                        // 8 elements), -1: padding
     uint64_t* bars = reinterpret_cast<uint64_t*>(tail + 2048);
-    uint64_t* qd_full = bars;            // [2]
-    uint64_t* qd_empty = bars + 2;       // [2]
-    uint64_t* kv_full = bars + 4;        // [2]
-    uint64_t* kv_empty = bars + 6;       // [2]
-    uint64_t* sdp_full = bars + 10;      // [2]
-    uint64_t* sdp_empty = bars + 12;     // [2]
-    uint64_t* pds_full = bars + 14;
-    uint64_t* pds_empty = bars + 15;
-    uint64_t* dq_full = bars + 16;
-    uint64_t* dq_empty = bars + 17;
-    uint64_t* acc_full = bars + 18;
-    uint64_t* acc_empty = bars + 19;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 20);
-    uint64_t* off_full = bars + 26;      // [4] ring of prepared tiles: tokens, kv head and new-block flag are valid
-    uint64_t* off_empty = bars + 30;     // [4] ... have been read by the eight gather warps and the S/dP issuer
-    int* s_h = reinterpret_cast<int*>(bars + 34);    // [4] kv head of the prepared tile
-    int* s_nb = s_h + 4;                             // [4] 1: the tile starts a new K/V block
+    uint64_t* do_full = bars;            // [2] the dO rows of a stage have landed
+    uint64_t* do_empty = bars + 2;       // [2] ... have been read (dV)
+    uint64_t* q_full = bars + 4;         // [2]
+    uint64_t* q_empty = bars + 6;        // [2] (dK)
+    uint64_t* k_full = bars + 8;         // [2]
+    uint64_t* k_empty = bars + 10;       // [2]
+    uint64_t* v_full = bars + 12;
+    uint64_t* v_empty = bars + 13;
+    uint64_t* dp_full = bars + 14;       // [2]
+    uint64_t* s_full = bars + 16;        // [2]
+    uint64_t* sdp_empty = bars + 18;     // [2]
+    uint64_t* p_full = bars + 20;
+    uint64_t* p_empty = bars + 21;
+    uint64_t* ds_full = bars + 22;
+    uint64_t* ds_empty = bars + 23;
+    uint64_t* dq_full = bars + 24;
+    uint64_t* dq_empty = bars + 25;
+    uint64_t* acc_full = bars + 26;
+    uint64_t* acc_empty = bars + 27;
+    uint64_t* off_full = bars + 28;      // [2] ring of prepared tiles: row offsets and record are valid
+    uint64_t* off_empty = bars + 32;     // [2] ... have been read by the eight gather warps and the S/dP issuer
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 36);
+    int4* s_rec = reinterpret_cast<int4*>(bars + 38);    // [16] prepared tiles: {bit 0: first tile of a segment (K and V are loaded for it),
+                                                         // bit 1: last one, tile of partial dQ rows, tile, run}.  16: the drain may be eight behind
+    static_assert(2 * kTileRows * 8 + 38 * 8 + 16 * 16 <= kTail, "tail budget");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const SelShape& s = p.s;
@@ -132,14 +154,17 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     }
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&qd_full[i], kLoaders); mbar_init(&qd_empty[i], 1);
-            mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1);
-            mbar_init(&sdp_full[i], 1); mbar_init(&sdp_empty[i], 256);
+            mbar_init(&do_full[i], kLoaders); mbar_init(&do_empty[i], 1);
+            mbar_init(&q_full[i], kLoaders); mbar_init(&q_empty[i], 1);
+            mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
+            mbar_init(&dp_full[i], 1); mbar_init(&s_full[i], 1); mbar_init(&sdp_empty[i], 256);
         }
-        mbar_init(pds_full, 256); mbar_init(pds_empty, 1);
+        mbar_init(v_full, 1); mbar_init(v_empty, 1);
+        mbar_init(p_full, 256); mbar_init(p_empty, 1);
+        mbar_init(ds_full, 256); mbar_init(ds_empty, 1);
         mbar_init(dq_full, 1); mbar_init(dq_empty, 128);
         mbar_init(acc_full, 1); mbar_init(acc_empty, 128);
-        for (int i = 0; i < 4; ++i) { mbar_init(&off_full[i], 1); mbar_init(&off_empty[i], kWLoad + 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&off_full[i], 1); mbar_init(&off_empty[i], kWLoad + 1); }
         mbar_init_fence();
         tma_prefetch_desc(&kmap);
         tma_prefetch_desc(&vmap);
@@ -154,55 +179,51 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
     const int nsub = PARTS ? p.nsub : 1;
     const int nloc = sched.nloc;
     const int key_lim = min(KT, s.BK);
+    bool ok = true;                         // no wait of this thread has run out
 
     if (warp < kWLoad) {
         // ------------------------------------------------------------------ gather warps
         // (D = 128) thread t copies 16-byte chunk t % 16 of the rows t / 16 + 16 i (a half-warp covers one 256-byte row) of Q and
-        // dO.  Tokens come from the prepared ring; the head part of every row offset is a thread constant.
+        // dO.  The rows' offsets come from the prepared ring.
         reg_dec<kRegLoad>();
         const int t = tid;
-        bool ok = true;
         constexpr int CPR = D / 8, RSTEP = kLoaders / CPR, NIT = kTileRows / RSTEP;   // D = 128: 16 chunks per row, 8 rows per thread
         const int cchunk = t % CPR, rbase = t / CPR;
         const uint32_t slab_off = (uint32_t)(cchunk >> 3) * (kTileRows * 128);
-        int gq[NIT], gd[NIT];                   // (head-in-group * head stride) / 8 of this thread's rows
-#pragma unroll
-        for (int it = 0; it < NIT; ++it) {
-            const int g = (rbase + it * RSTEP) / s.TPT;
-            gq[it] = (int)((g * p.q_sh) >> 3);
-            gd[it] = (int)((g * p.do_sh) >> 3);
-        }
-        const int qsn8 = (int)(p.q_sn >> 3), dsn8 = (int)(p.do_sn >> 3);
         const ET* qc = p.q + cchunk * 8;
         const ET* dc = p.d_o + cchunk * 8;
         BT_DECL;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            const int st = k & 1, slot = k & 3;
+            const int st = k & 1;
             BT_TOC(0);
-            ok = mbar_wait(&off_full[slot], (k >> 2) & 1, status) && ok;
+            ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
             BT_TOC(2);
-            const int hq0 = (int)(((long long)s_h[slot] * s.G * p.q_sh) >> 3), hd0 = (int)(((long long)s_h[slot] * s.G * p.do_sh) >> 3);
-            int tok[NIT];
-#pragma unroll
-            for (int it = 0; it < NIT; ++it) tok[it] = s_tok[slot][rbase + it * RSTEP];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&off_empty[slot]);
-            BT_TOC(3);
-            ok = mbar_wait(&qd_empty[st], ((k >> 1) & 1) ^ 1, status) && ok;
+            const int2* off = s_off[st] + rbase;
+            // dO first: dV, its last reader, is issued before dK, the last reader of Q
+            // (RSTEP is a multiple of 8: the rows of a thread have one swizzle)
+            const uint32_t dq_ = smem_u32(sQD + st * kQD) + slab_off + sw128_chunk_off(rbase, cchunk & 7);
+            const uint32_t dd_ = dq_ + kTileRows * D * 2;
+            ok = mbar_poll(&do_empty[st], ((k >> 1) & 1) ^ 1) && ok;
             BT_EV(k, 0, t == 0);
             BT_TOC(1);
-            const uint32_t dq_ = smem_u32(sQD + st * kQD) + slab_off;
-            const uint32_t dd_ = dq_ + kTileRows * D * 2;
 #pragma unroll
             for (int it = 0; it < NIT; ++it) {
-                const int r = rbase + it * RSTEP;
-                const bool valid = tok[it] >= 0;
-                const int tk = valid ? tok[it] : 0;
-                const uint32_t so = sw128_chunk_off(r, cchunk & 7);
-                cp_async16(dq_ + so, qc + ((long long)(tk * qsn8 + hq0 + gq[it]) << 3), valid);
-                cp_async16(dd_ + so, dc + ((long long)(tk * dsn8 + hd0 + gd[it]) << 3), valid);
+                const int o = off[it * RSTEP].y;
+                cp_async16(dd_ + it * (RSTEP * 128), dc + ((int64_t)max(o, 0) << 3), o >= 0);
             }
-            cp_async_mbar_arrive_noinc(&qd_full[st]);
+            cp_async_mbar_arrive_noinc(&do_full[st]);
+            BT_TOC(4);
+            ok = mbar_poll(&q_empty[st], ((k >> 1) & 1) ^ 1) && ok;
+            BT_TOC(1);
+#pragma unroll
+            for (int it = 0; it < NIT; ++it) {
+                const int o = off[it * RSTEP].x;
+                cp_async16(dq_ + it * (RSTEP * 128), qc + ((int64_t)max(o, 0) << 3), o >= 0);
+            }
+            cp_async_mbar_arrive_noinc(&q_full[st]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&off_empty[st]);
             BT_EV(k, 1, t == 0);
             BT_TOC(4);
         }
@@ -217,87 +238,76 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         const int quarter = warp & 3;
         const int d_idx = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint8_t* my_stage = sDQ + quarter * (32 * D * 2);
-        bool ok = true;
+        uint8_t* my_stage = sDQ + quarter * (32 * 128);
         int nflush = 0;
         BT_DECL;
-        // key ids of the CTA's tiles, fetched two tiles ahead
-        int hg0 = -1, hg1 = -1, hg2 = -1;
-        if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
-        if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
-        int seg_first = 0;                 // local index of the first tile of the running segment
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            const int prev_hg = hg0;
-            hg0 = hg1; hg1 = hg2;
-            if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
-            if (hg0 != prev_hg || (k % sched.run) == 0) seg_first = k;
-            const bool last_of_seg = (k + 1 >= nloc) || (hg1 != hg0) || ((k + 1) % sched.run) == 0;
-            const int j = sched.tile(k);
             // ---- dQ partial of this tile
             BT_TOC(0);
-            ok = mbar_wait(dq_full, k & 1, status) && ok;
+            ok = mbar_poll(dq_full, k & 1) && ok;
             BT_EV(k, 13, warp == kWFlush && lane == 0);
             BT_TOC(1);
             tc_fence_after();
-            if (lane == 0) bulk_wait_read0();          // the store of the previous tile has read this warp's staging rows
-            __syncwarp();
+            const int4 rec = s_rec[k & 15];
+            // (rolled loops here and below: see the note on code size)
+#pragma unroll 1
+            for (int b = 0; b < D / 64; ++b) {
+                if (lane == 0) bulk_wait_read0();          // the store before this one has read this warp's staging rows
+                __syncwarp();
+#pragma unroll 1
+                for (int c0 = 0; c0 < 64; c0 += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tbase + lane_off + cDQ + b * 64 + c0, v);
+                    tmem_ld_wait();
 #pragma unroll
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tbase + lane_off + cDQ + c0, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    uint4 u;
-                    u.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-                    u.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-                    u.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-                    u.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-                    const int chunk = (c0 >> 3) + q4;
-                    *reinterpret_cast<uint4*>(my_stage + (chunk >> 3) * (32 * 128) + sw128_chunk_off(lane, chunk & 7)) = u;
+                    for (int q4 = 0; q4 < 4; ++q4) {
+                        uint4 u;
+                        u.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
+                        u.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
+                        u.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
+                        u.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
+                        *reinterpret_cast<uint4*>(my_stage + sw128_chunk_off(lane, (c0 >> 3) + q4)) = u;
+                    }
+                }
+                if (b == D / 64 - 1) {
+                    tc_fence_before();
+                    mbar_arrive(dq_empty);
+                    BT_EV(k, 14, warp == kWFlush && lane == 0);
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&dqmap, b * 64, rec.y * kTileRows + quarter * 32, smem_u32(my_stage));
+                    bulk_commit();
                 }
             }
-            tc_fence_before();
-            mbar_arrive(dq_empty);
-            BT_EV(k, 14, warp == kWFlush && lane == 0);
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-#pragma unroll
-                for (int b = 0; b < D / 64; ++b)
-                    tma_store_2d(&dqmap, b * 64, (j * nsub + sched.sub(k)) * kTileRows + quarter * 32, smem_u32(my_stage + b * (32 * 128)));
-                bulk_commit();
-            }
             BT_TOC(2);
-            if (!last_of_seg) continue;
-            // ---- dK^T / dV^T of the finished segment
-            const int j0 = sched.tile(seg_first);
-            const TileInfo ti = load_tile(p.ix, j0);
-            // segments of a key are numbered by the scheduling run they fall into
-            const int seg = ti.seg0 + j0 / sched.run - __ldg(p.ix.tile_aux + j0).x / sched.run;
-            float* slab = p.slabs + ((int64_t)seg * nsub + sched.sub(k)) * (2 * KT * D) + d_idx;
-            ok = mbar_wait(acc_full, nflush & 1, status) && ok;
+            if (!(rec.x & 2)) continue;
+            // ---- dK^T / dV^T of the finished segment (the segments of a key are numbered by the scheduling run they fall into)
+            const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
+            float* slab = p.slabs + ((int64_t)seg * nsub + (rec.y - rec.z * nsub)) * (2 * KT * D) + d_idx;
+            ok = mbar_poll(acc_full, nflush & 1) && ok;
             BT_TOC(3);
             tc_fence_after();
-#pragma unroll
+#pragma unroll 1
             for (int which = 0; which < 2; ++which) {
                 uint32_t v[KT];
-#pragma unroll
-                for (int c0 = 0; c0 < KT; c0 += 32)
-                    tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[c0]));
+                tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV), *reinterpret_cast<uint32_t (*)[32]>(&v[0]));
+                tmem_ld32(tbase + lane_off + (which == 0 ? cDK : cDV) + 32, *reinterpret_cast<uint32_t (*)[32]>(&v[32]));
                 tmem_ld_wait();
                 if (which == 1) {
-                    // both accumulators are in registers now: the next segment may overwrite them
+                    // both accumulators have been read: the next segment may overwrite them
                     tc_fence_before();
                     mbar_arrive(acc_empty);
                     ++nflush;
                 }
-                float* dst = slab + which * (KT * D);
                 // (D = 64: the upper accumulator rows are products of whatever follows the tile in shared memory)
                 if (quarter * 32 < D) {
 #pragma unroll
-                    for (int key = 0; key < KT; ++key) dst[key * D] = __uint_as_float(v[key]);
+                    for (int key = 0; key < KT; ++key) slab[key * D] = __uint_as_float(v[key]);
                 }
+                slab += KT * D;
             }
             BT_TOC(4);
         }
@@ -311,47 +321,58 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, KT, false, false);
         constexpr uint32_t hi_1024 = umma_desc_hi(1024);
         const uint32_t qd_lo = umma_desc_lo(smem_u32(sQD), 16);
-        const uint32_t kv_lo = umma_desc_lo(smem_u32(sKV), 16);
+        const uint32_t k_lo = umma_desc_lo(smem_u32(sK), 16), v_lo = umma_desc_lo(smem_u32(sV), 16);
         int kvn = -1;
-        bool ok = true;
         BT_DECL;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
             BT_TOC(0);
-            ok = mbar_wait(&off_full[k & 3], (k >> 2) & 1, status) && ok;
+            ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
             BT_TOC(1);
-            const int new_block = s_nb[k & 3];
+            const int seg = s_rec[k & 15].x;
             __syncwarp();
-            if (lane == 0) mbar_arrive(&off_empty[k & 3]);
-            if (new_block != 0) {
+            if (lane == 0) mbar_arrive(&off_empty[st]);
+            if (seg & 1) {
                 ++kvn;
-                ok = mbar_wait(&kv_full[kvn % kKVStages], (kvn / kKVStages) & 1, status) && ok;
+                ok = mbar_poll(v_full, kvn & 1) && ok;
             }
             BT_TOC(2);
-            ok = mbar_wait(&qd_full[st], (k >> 1) & 1, status) && ok;
+            ok = mbar_poll(&sdp_empty[st], ((k >> 1) & 1) ^ 1) && ok;
+            BT_EV(k, 3, lane == 0);
+            BT_TOC(4);
+            ok = mbar_poll(&do_full[st], (k >> 1) & 1) && ok;
             BT_EV(k, 2, lane == 0);
             BT_TOC(3);
             fence_async_smem();
-            ok = mbar_wait(&sdp_empty[st], ((k >> 1) & 1) ^ 1, status) && ok;
-            BT_EV(k, 3, lane == 0);
-            BT_TOC(4);
             tc_fence_after();
             const uint32_t aq = qd_lo + (uint32_t)(st * (kQD >> 4));
             const uint32_t ad = aq + (uint32_t)((kTileRows * D * 2) >> 4);
-            const uint32_t bk = kv_lo + (uint32_t)((kvn % kKVStages) * (kKV >> 4));
-            const uint32_t bv = bk + (uint32_t)((KT * D * 2) >> 4);
+            const uint32_t bk = k_lo + (uint32_t)((kvn % kKStages) * (kK >> 4));
             const uint32_t dS_ = tbase + cS + st * 128, dP_ = tbase + cDP + st * 128;
+            constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (KT * 128) >> 4;
             if (leader) {
-                constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (KT * 128) >> 4;
-#pragma unroll
+#pragma unroll 4
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ss(dP_, umma_desc_pack(ad + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
+                            umma_desc_pack(v_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
+                umma_commit(&dp_full[st]);
+                if (seg & 2) umma_commit(v_empty);
+            }
+            __syncwarp();
+            BT_TOC(5);
+            if (seg & 1) ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
+            BT_TOC(2);
+            ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
+            BT_TOC(3);
+            fence_async_smem();
+            tc_fence_after();
+            if (leader) {
+#pragma unroll 4
                 for (int ks = 0; ks < D / 16; ++ks)
                     umma_ss(dS_, umma_desc_pack(aq + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
                             umma_desc_pack(bk + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(dP_, umma_desc_pack(ad + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
-                            umma_desc_pack(bv + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
-                umma_commit(&sdp_full[st]);
+                umma_commit(&s_full[st]);
             }
             __syncwarp();
             BT_EV(k, 4, lane == 0);
@@ -367,55 +388,59 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         const uint32_t ds_k_lo = umma_desc_lo(smem_u32(sDS), 16);                       // dS as K-major A
         const uint32_t ds_mn_lo = umma_desc_lo(smem_u32(sDS), 8192);                    // dS as MN-major B (one slab)
         const uint32_t p_mn_lo = umma_desc_lo(smem_u32(sP), 8192);
-        const uint32_t k_mn_lo = umma_desc_lo(smem_u32(sKV), KT * 128);                 // K as MN-major B: slabs KT*128 apart
+        const uint32_t k_mn_lo = umma_desc_lo(smem_u32(sK), KT * 128);                  // K as MN-major B: slabs KT*128 apart
         const uint32_t qd_mn_lo = umma_desc_lo(smem_u32(sQD), kTileRows * 128);         // Q / dO as MN-major A
-        int kvn = -1, blk = -1;
-        bool ok = true;
-        int hg0 = -1, hg1 = -1, hg2 = -1;
-        if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
-        if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
+        int kvn = -1, blk = -1;            // K/V loads, segments
         BT_DECL;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
-            const int prev_hg = hg0;
-            hg0 = hg1; hg1 = hg2;
-            if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
-            // a segment ends where the block changes or the scheduling run ends
-            const bool first_of_block = hg0 != prev_hg || (k % sched.run) == 0;
-            const bool last_of_block = (k + 1 >= nloc) || (hg1 != hg0) || ((k + 1) % sched.run) == 0;
-            if (first_of_block) { ++kvn; ++blk; }
             BT_TOC(0);
-            ok = mbar_wait(pds_full, k & 1, status) && ok;
+            // (the record is complete: its tile has been through the S / dP issuer when P is there)
+            ok = mbar_poll(p_full, k & 1) && ok;
             BT_EV(k, 9, lane == 0);
             BT_TOC(1);
-            BT_TOC(2);
-            ok = mbar_wait(&qd_full[st], (k >> 1) & 1, status) && ok;     // already complete: acquire only
-            ok = mbar_wait(&kv_full[kvn % kKVStages], (kvn / kKVStages) & 1, status) && ok;
-            BT_TOC(3);
-            if (first_of_block && blk > 0) ok = mbar_wait(acc_empty, (blk - 1) & 1, status) && ok;
+            const int seg = s_rec[k & 15].x;
+            const bool first_of_block = seg & 1, last_of_block = seg & 2;
+            if (first_of_block) { ++kvn; ++blk; }
+            if (first_of_block && blk > 0) ok = mbar_poll(acc_empty, (blk - 1) & 1) && ok;
             BT_TOC(4);
+            ok = mbar_poll(&do_full[st], (k >> 1) & 1) && ok;     // already complete: acquire only
+            ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
+            ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
+            BT_TOC(3);
             fence_async_smem();
             tc_fence_after();
-            const uint32_t bk = k_mn_lo + (uint32_t)((kvn % kKVStages) * (kKV >> 4));
+            const uint32_t bk = k_mn_lo + (uint32_t)((kvn % kKStages) * (kK >> 4));
             const uint32_t aq = qd_mn_lo + (uint32_t)(st * (kQD >> 4));
             const uint32_t ad = aq + (uint32_t)((kTileRows * D * 2) >> 4);
-            // dK^T / dV^T first: they are the last readers of the Q / dO stage, which goes back to the gather warps as
-            // soon as they are done; dQ (which reads dS and K only) follows
+            // dV, then dK: they are the last readers of the dO and Q rows, which go back to the gather warps as soon as each is
+            // done; dQ (which reads dS and K only) follows
             if (leader) {
-#pragma unroll
-                for (int ks = 0; ks < kTileRows / 16; ++ks) {
-                    const uint32_t acc = (!first_of_block || ks > 0) ? 1u : 0u;
-                    umma_ss(tbase + cDK, umma_desc_pack(aq + ks * (2048 >> 4), hi_1024),
-                            umma_desc_pack(ds_mn_lo + ks * (2048 >> 4), hi_1024), idesc_dk, acc);
-                    umma_ss(tbase + cDV, umma_desc_pack(ad + ks * (2048 >> 4), hi_1024),
-                            umma_desc_pack(p_mn_lo + ks * (2048 >> 4), hi_1024), idesc_dk, acc);
-                }
-                umma_commit(&qd_empty[st]);
+#pragma unroll 4
+                for (int ks = 0; ks < kTileRows / 16; ++ks)
+                    umma_ss(tbase + cDV, umma_desc_pack(ad + ks * (2048 >> 4), hi_1024), umma_desc_pack(p_mn_lo + ks * (2048 >> 4), hi_1024),
+                            idesc_dk, (!first_of_block || ks > 0) ? 1u : 0u);
+                umma_commit(&do_empty[st]);
+                umma_commit(p_empty);
+            }
+            __syncwarp();
+            BT_TOC(5);
+            ok = mbar_poll(ds_full, k & 1) && ok;
+            BT_TOC(2);
+            fence_async_smem();
+            tc_fence_after();
+            if (leader) {
+#pragma unroll 4
+                for (int ks = 0; ks < kTileRows / 16; ++ks)
+                    umma_ss(tbase + cDK, umma_desc_pack(aq + ks * (2048 >> 4), hi_1024), umma_desc_pack(ds_mn_lo + ks * (2048 >> 4), hi_1024),
+                            idesc_dk, (!first_of_block || ks > 0) ? 1u : 0u);
+                umma_commit(&q_empty[st]);
                 if (last_of_block) umma_commit(acc_full);
             }
             __syncwarp();
             BT_EV(k, 10, lane == 0);
-            ok = mbar_wait(dq_empty, (k & 1) ^ 1, status) && ok;
+            ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
             BT_EV(k, 11, lane == 0);
             tc_fence_after();
             if (leader) {
@@ -423,9 +448,9 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                 for (int ks = 0; ks < KT / 16; ++ks)
                     umma_ss(tbase + cDQ, umma_desc_pack(ds_k_lo + ks * 2, hi_1024), umma_desc_pack(bk + ks * (2048 >> 4), hi_1024),
                             idesc_dq, ks > 0);
-                umma_commit(pds_empty);
+                umma_commit(ds_empty);
                 umma_commit(dq_full);
-                if (last_of_block) umma_commit(&kv_empty[kvn % kKVStages]);
+                if (last_of_block) umma_commit(&k_empty[kvn % kKStages]);
             }
             __syncwarp();
             BT_EV(k, 12, lane == 0);
@@ -435,69 +460,77 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
       } else if (warp == kWMma2 + 1) {
         // ------------------------------------------------------------------ tile preparation (tokens of the rows)
         // lane l owns rows l, l + 32, l + 64, l + 96; records and entries are fetched three tiles ahead
-        bool ok = true;
-        int gg[4], ee[4];
+        uint32_t gg = 0;                    // head (of the group) of the lane's rows, a byte each
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = lane + 32 * i;
-            gg[i] = r / s.TPT;
-            ee[i] = r - gg[i] * s.TPT;
-        }
+        for (int i = 0; i < 4; ++i) gg |= (uint32_t)((lane + 32 * i) / s.TPT) << (8 * i);
+        const int qsn8 = (int)(p.q_sn >> 3), dsn8 = (int)(p.do_sn >> 3), qsh8 = (int)(p.q_sh >> 3), dsh8 = (int)(p.do_sh >> 3);
         struct Pre { int h, hg; uint32_t e[4]; };
-        auto fetch = [&](int k, Pre& m) {
-            const int j = sched.tile(k);
-            const TileInfo ti = load_tile(p.ix, j);
+        TileCursorT<PARTS> ahead(sched), cur_t(sched);
+        auto fetch = [&](Pre& m) {
+            const TileInfo ti = load_tile(p.ix, ahead.j);
             m.h = ti.h; m.hg = ti.hg;
+            const uint32_t* ent = p.ix.entries + (int64_t)ahead.j * s.TPT + lane;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) m.e[i] = gg[i] < s.G ? __ldg(p.ix.entries + (int64_t)j * s.TPT + ee[i]) : 0xFFFFFFFFu;
+            for (int i = 0; i < 4; ++i) {
+                const int g = gg >> (8 * i) & 255;
+                m.e[i] = g < s.G ? __ldg(ent + 32 * i - g * s.TPT) : 0xFFFFFFFFu;
+            }
+            ahead.next(sched);
         };
         Pre m1{0, -1, {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}}, m2 = m1, m3 = m1;
-        if (nloc > 0) fetch(0, m1);
-        if (nloc > 1) fetch(1, m2);
-        if (nloc > 2) fetch(2, m3);
+        if (nloc > 0) fetch(m1);
+        if (nloc > 1) fetch(m2);
+        if (nloc > 2) fetch(m3);
         int prev_hg = -1;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            const int slot = k & 3;
+            const int slot = k & 1;
             const Pre cur = m1;
             m1 = m2; m2 = m3;
-            if (k + 3 < nloc) fetch(k + 3, m3);
-            ok = mbar_wait(&off_empty[slot], ((k >> 2) & 1) ^ 1, status) && ok;
+            if (k + 3 < nloc) fetch(m3);
+            ok = mbar_poll(&off_empty[slot], ((k >> 1) & 1) ^ 1) && ok;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s_tok[slot][lane + 32 * i] = cur.e[i] != 0xFFFFFFFFu ? (int)(cur.e[i] >> kSlotBits) : -1;
-            if (lane == 0) {
-                s_h[slot] = cur.h;
-                s_nb[slot] = (cur.hg != prev_hg || (k % sched.run) == 0) ? 1 : 0;
+            for (int i = 0; i < 4; ++i) {
+                const int hq = cur.h * s.G + (int)(gg >> (8 * i) & 255), tok = (int)(cur.e[i] >> kSlotBits);
+                s_off[slot][lane + 32 * i] = cur.e[i] != 0xFFFFFFFFu ? make_int2(tok * qsn8 + hq * qsh8, tok * dsn8 + hq * dsh8) : make_int2(-1, -1);
             }
+            if (lane == 0)
+                s_rec[k & 15] = make_int4((cur.hg != prev_hg || cur_t.r == 0 ? 1 : 0) | (k + 1 >= nloc || m1.hg != cur.hg || cur_t.r + 1 == sched.run ? 2 : 0),
+                                          cur_t.j * nsub + cur_t.sub(sched), cur_t.j, cur_t.run(sched));
+            cur_t.next(sched);
             prev_hg = cur.hg;
             __syncwarp();
             if (lane == 0) mbar_arrive(&off_full[slot]);
         }
       } else {
         // ------------------------------------------------------------------ K/V blocks by TMA
-        bool ok = true;
         int kvn = -1, prev_hg = -1;
         TileInfo t1{0, 0, 0, -1, 0}, t2 = t1;
-        if (nloc > 0) t1 = load_tile(p.ix, sched.tile(0));
-        if (nloc > 1) t2 = load_tile(p.ix, sched.tile(1));
+        TileCursorT<PARTS> ahead(sched), cur_t(sched);
+        auto fetch = [&](TileInfo& t) { t = load_tile(p.ix, ahead.j); ahead.next(sched); };
+        if (nloc > 0) fetch(t1);
+        if (nloc > 1) fetch(t2);
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
             const TileInfo cur = t1;
             t1 = t2;
-            if (k + 2 < nloc) t2 = load_tile(p.ix, sched.tile(k + 2));
-            if (cur.hg == prev_hg && (k % sched.run) != 0) continue;     // (every segment loads its K/V block)
+            if (k + 2 < nloc) fetch(t2);
+            const int row = cur.row0 + cur_t.sub(sched) * KT;
+            const bool first = cur.hg != prev_hg || cur_t.r == 0;     // (every segment loads its K/V block)
+            cur_t.next(sched);
+            if (!first) continue;
             prev_hg = cur.hg;
             ++kvn;
             if (lane == 0) {
-                const int ks = kvn % kKVStages;
-                ok = mbar_wait(&kv_empty[ks], ((kvn / kKVStages) & 1) ^ 1, status) && ok;
-                mbar_expect_tx(&kv_full[ks], (uint32_t)kKV);
-                const int row = cur.row0 + sched.sub(k) * KT;
-                uint8_t* dK = sKV + ks * kKV;
-                uint8_t* dV = dK + KT * D * 2;
+                const int ks = kvn % kKStages;
+                ok = mbar_poll(&k_empty[ks], ((kvn / kKStages) & 1) ^ 1) && ok;
+                mbar_expect_tx(&k_full[ks], (uint32_t)kK);
 #pragma unroll
-                for (int b = 0; b < D / 64; ++b) {
-                    tma_load_2d(smem_u32(dK + b * KT * 128), &kmap, cur.h * D + b * 64, row, &kv_full[ks]);
-                    tma_load_2d(smem_u32(dV + b * KT * 128), &vmap, cur.h * D + b * 64, row, &kv_full[ks]);
-                }
+                for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sK + ks * kK + b * KT * 128), &kmap, cur.h * D + b * 64, row, &k_full[ks]);
+                ok = mbar_poll(v_empty, (kvn & 1) ^ 1) && ok;
+                mbar_expect_tx(v_full, (uint32_t)kK);
+#pragma unroll
+                for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sV + b * KT * 128), &vmap, cur.h * D + b * 64, row, v_full);
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
@@ -516,7 +549,6 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         const bool row_exists = g < s.G;
         constexpr int HC = KT / 2;              // columns of this group
         const int cb = sb * HC;
-        bool ok = true;
         // software pipeline over the tiles: entries two tiles ahead, lse / delta one ahead
         uint32_t entB = 0xFFFFFFFFu;            // entry of tile k + 2
         uint32_t entA = 0xFFFFFFFFu;            // entry of tile k + 1 (after rotation)
@@ -529,9 +561,11 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ent = 0xFFFFFFFFu;
             if (row_exists) ent = __ldg(p.ix.entries + (int64_t)j * s.TPT + e);
         };
-        auto fetch = [&](int k, uint32_t& ent, int& row0, int& h) {      // ... and the first key of the tile's part
-            fetch_ent(sched.tile(k), ent, row0, h);
-            row0 += sched.sub(k) * KT;
+        TileCursorT<PARTS> ahead(sched);
+        auto fetch = [&](uint32_t& ent, int& row0, int& h) {      // ... and the first key of the tile's part
+            fetch_ent(ahead.j, ent, row0, h);
+            row0 += ahead.sub(sched) * KT;
+            ahead.next(sched);
         };
         auto fetch_stats = [&](uint32_t ent, int h, int row0, float& lse_, float& delta_, int& c_lo, int& c_hi) {
             // padding rows: their Q and dO rows are zero, so they add nothing to dK / dV whatever P is, and their dQ
@@ -546,11 +580,12 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
         };
         if (nloc > 0) {
-            fetch(0, entA, row0A, hA);
+            fetch(entA, row0A, hA);
             fetch_stats(entA, hA, row0A, lseA, deltaA, cloA, chiA);
         }
-        if (nloc > 1) fetch(1, entB, row0B, hB);
+        if (nloc > 1) fetch(entB, row0B, hB);
         BT_DECL;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
             const float lse_r = lseA, delta_s = deltaA;
@@ -558,63 +593,69 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             // rotate the prefetch registers
             entA = entB; row0A = row0B; hA = hB;
             if (k + 1 < nloc) fetch_stats(entA, hA, row0A, lseA, deltaA, cloA, chiA);
-            if (k + 2 < nloc) fetch(k + 2, entB, row0B, hB);
+            if (k + 2 < nloc) fetch(entB, row0B, hB);
             BT_TOC(0);
-            ok = mbar_wait(&sdp_full[st], (k >> 1) & 1, status) && ok;
+            // most tiles are fully visible to all their rows (only a token's own block is cut by causality)
+            const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == KT);
+            // dP comes first (its rows are gathered first): scale (dP - delta) is ready when S arrives
+            ok = mbar_poll(&dp_full[st], (k >> 1) & 1) && ok;
+            tc_fence_after();
+            uint32_t sv[32], dv[32], pp[HC / 2];
+            tmem_ld32(tbase + lane_off + cDP + st * 128 + cb, dv);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) dv[i] = __float_as_uint(fmaf(__uint_as_float(dv[i]), p.scale, -delta_s));
+            BT_TOC(5);
+            ok = mbar_poll(&s_full[st], (k >> 1) & 1) && ok;
             BT_EV(k, 5, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(1);
             tc_fence_after();
-            uint32_t pp[HC / 2], dd[HC / 2];
-            // most tiles are fully visible to all their rows (only a token's own block is cut by causality)
-            const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == KT);
-            {
-                uint32_t sv[32], dv[32];
-                tmem_ld32(tbase + lane_off + cS + st * 128 + cb, sv);
-                tmem_ld32(tbase + lane_off + cDP + st * 128 + cb, dv);
-                tmem_ld_wait();
-                if (all_visible) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float p0 = ex2_approx_b(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r));
-                        const float p1 = ex2_approx_b(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse_r));
-                        const float d0 = p0 * fmaf(__uint_as_float(dv[i]), p.scale, -delta_s);
-                        const float d1 = p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s);
-                        pp[i >> 1] = ElemTraits<ET>::pack2(p0, p1);
-                        dd[i >> 1] = ElemTraits<ET>::pack2(d0, d1);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float p0 = (cb + i >= c_lo && cb + i < c_hi) ? ex2_approx_b(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r)) : 0.f;
-                        const float p1 = (cb + i + 1 >= c_lo && cb + i + 1 < c_hi) ? ex2_approx_b(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse_r)) : 0.f;
-                        const float d0 = p0 * fmaf(__uint_as_float(dv[i]), p.scale, -delta_s);
-                        const float d1 = p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s);
-                        pp[i >> 1] = ElemTraits<ET>::pack2(p0, p1);
-                        dd[i >> 1] = ElemTraits<ET>::pack2(d0, d1);
-                    }
-                }
-            }
+            tmem_ld32(tbase + lane_off + cS + st * 128 + cb, sv);
+            tmem_ld_wait();
             tc_fence_before();
             mbar_arrive(&sdp_empty[st]);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sv[i] = __float_as_uint(ex2_approx_b(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r)));
+            if (!all_visible) {
+                // (bit i: column cb + i is visible)
+                const int lo = min(max(c_lo - cb, 0), 32), hi = min(max(c_hi - cb, 0), 32);
+                const uint32_t vis = (uint32_t)((1ull << hi) - 1) & ~(uint32_t)((1ull << lo) - 1);
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    if (!(vis >> i & 1u)) sv[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                const float p0 = __uint_as_float(sv[i]), p1 = __uint_as_float(sv[i + 1]);
+                pp[i >> 1] = ElemTraits<ET>::pack2(p0, p1);
+                sv[i >> 1] = ElemTraits<ET>::pack2(p0 * __uint_as_float(dv[i]), p1 * __uint_as_float(dv[i + 1]));      // (dS over what has been read)
+            }
             BT_EV(k, 6, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(2);
-            ok = mbar_wait(pds_empty, (k & 1) ^ 1, status) && ok;
+            // P first: dV starts while dS is being written
+            ok = mbar_poll(p_empty, (k & 1) ^ 1) && ok;
             BT_EV(k, 7, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(3);
 #pragma unroll
-            for (int c4 = 0; c4 < HC / 8; ++c4) {
-                const uint32_t off = sw128_chunk_off(r, sb * (HC / 8) + c4);
-                *reinterpret_cast<uint4*>(sP + off) = make_uint4(pp[c4 * 4], pp[c4 * 4 + 1], pp[c4 * 4 + 2], pp[c4 * 4 + 3]);
-                *reinterpret_cast<uint4*>(sDS + off) = make_uint4(dd[c4 * 4], dd[c4 * 4 + 1], dd[c4 * 4 + 2], dd[c4 * 4 + 3]);
-            }
+            for (int c4 = 0; c4 < HC / 8; ++c4)
+                *reinterpret_cast<uint4*>(sP + sw128_chunk_off(r, sb * (HC / 8) + c4)) = make_uint4(pp[c4 * 4], pp[c4 * 4 + 1], pp[c4 * 4 + 2], pp[c4 * 4 + 3]);
             fence_async_smem();
-            mbar_arrive(pds_full);
+            mbar_arrive(p_full);
+            BT_TOC(4);
+            ok = mbar_poll(ds_empty, (k & 1) ^ 1) && ok;
+            BT_TOC(3);
+#pragma unroll
+            for (int c4 = 0; c4 < HC / 8; ++c4)
+                *reinterpret_cast<uint4*>(sDS + sw128_chunk_off(r, sb * (HC / 8) + c4)) = make_uint4(sv[c4 * 4], sv[c4 * 4 + 1], sv[c4 * 4 + 2], sv[c4 * 4 + 3]);
+            fence_async_smem();
+            mbar_arrive(ds_full);
             BT_EV(k, 8, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(4);
             BT_TOC(6);
         }
         if (quarter == 0 && lane == 0) BT_DUMP(32 + sb * 8, 7);
     }
+    if (!ok) atomicMax(status, (int)kStatusWaitTimeout);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, bwdpipe::kCols);

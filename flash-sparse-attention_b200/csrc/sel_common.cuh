@@ -240,6 +240,18 @@ struct TileScheduleT {
     __device__ __forceinline__ int sub(int k) const { return PARTS ? ((k / run) * grid + cta) & ((1 << lsub) - 1) : 0; }
 };
 using TileSchedule = TileScheduleT<false>;
+// Walks a CTA's tiles in order without a division per tile (a role of a warp-specialised kernel keeps one or two).
+template <bool PARTS>
+struct TileCursorT {
+    int j, r, q;                                 // tile, its place in the run, dealt run
+    __device__ explicit TileCursorT(const TileScheduleT<PARTS>& c) : j((PARTS ? c.cta >> c.lsub : c.cta) * c.run), r(0), q(c.cta) {}
+    __device__ __forceinline__ void next(const TileScheduleT<PARTS>& c) {
+        ++j;
+        if (++r == c.run) { r = 0; q += c.grid; j = run(c) * c.run; }
+    }
+    __device__ __forceinline__ int run(const TileScheduleT<PARTS>& c) const { return PARTS ? q >> c.lsub : q; }
+    __device__ __forceinline__ int sub(const TileScheduleT<PARTS>& c) const { return PARTS ? q & ((1 << c.lsub) - 1) : 0; }
+};
 
 // Query-tile-major kernels cut every sequence into tiles of TPT consecutive tokens.  Both helpers are warp-collective (every lane calls them and gets the same
 // answer) and walk the sequences 32 at a time, so that a packed batch of thousands of short sequences costs B / 32 steps.
