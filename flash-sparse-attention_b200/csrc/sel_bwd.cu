@@ -587,7 +587,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
     }
     if (rows > 0 && sel_merge_fits(s, nsub)) {
         prof_begin(3, stream);
-        e = launch_sel_merge_dq(dt, a.dq_part, ix.pos, s, nsub, a.dq, ix.header, num_sms, stream);
+        e = launch_sel_merge_dq(dt, a.dq_part, ix.pos, s, nsub, a.dq, num_sms, stream);
         prof_end(3, stream);
         if (e != cudaSuccess) return e;
     } else if (rows > 0) {

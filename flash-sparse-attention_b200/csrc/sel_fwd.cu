@@ -927,8 +927,7 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     int64_t rows = s.N * s.Hq;
     if (rows > 0 && sel_merge_fits(s, 1)) {
         prof_begin(1, stream);
-        e = launch_sel_merge_fwd(ElemTraits<ET>::kIsBF16 ? (int)kBF16 : (int)kFP16, a.opart, a.ml, ix.pos, s, a.o, a.o_sn, a.o_sh, a.lse, ix.header,
-                                 num_sms, stream);
+        e = launch_sel_merge_fwd(ElemTraits<ET>::kIsBF16 ? (int)kBF16 : (int)kFP16, a.opart, a.ml, ix.pos, s, a.o, a.o_sn, a.o_sh, a.lse, num_sms, stream);
         prof_end(1, stream);
         return e;
     }

@@ -67,9 +67,8 @@ struct SelBwdArgs {
 // merges for up to 16 partial rows a token (sel_merge.cu)
 bool sel_merge_fits(const SelShape& s, int nsub);
 cudaError_t launch_sel_merge_fwd(int dtype, const void* part, const float2* ml, const int* pos, const SelShape& s, void* o, int64_t o_sn,
-                                 int64_t o_sh, float* lse, int* status, int sms, cudaStream_t stream);
-cudaError_t launch_sel_merge_dq(int dtype, const void* part, const int* pos, const SelShape& s, int nsub, void* dq, int* status, int sms,
-                                cudaStream_t stream);
+                                 int64_t o_sh, float* lse, int sms, cudaStream_t stream);
+cudaError_t launch_sel_merge_dq(int dtype, const void* part, const int* pos, const SelShape& s, int nsub, void* dq, int sms, cudaStream_t stream);
 
 // pipelined main kernel for head_dim 64 and 128 (sel_bwd_pipe.cu)
 cudaError_t launch_sel_bwd_pipe(int dtype, const SelBwdArgs& a, const SelShape& s, const SelIndex& ix,

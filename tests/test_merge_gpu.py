@@ -35,3 +35,10 @@ def test_resident_merge(seqlens, Hk, G, T, d, bs, dtype):
         o1, lse1, dq1 = run(a, a + n)
         assert torch.equal(o[a : a + n], o1) and torch.equal(lse[:, a : a + n], lse1) and torch.equal(dq[a : a + n], dq1)
         a += n
+
+
+@pytest.mark.parametrize("seqlens,Hk,G,T,d", [([1500, 1503], 2, 4, 12, 128), ([1500, 1503], 2, 4, 13, 128), ([2000, 1100], 8, 1, 15, 64),
+                                              ([1999, 1300], 1, 8, 1, 64), ([2701, 1400], 2, 3, 14, 64)])
+def test_resident_merge_row_counts(seqlens, Hk, G, T, d):
+    """Counts of partial rows around the one from which all 16 are taken without a test, and tokens that have fewer than that."""
+    test_resident_merge(seqlens, Hk, G, T, d, 64, "bf16")
