@@ -199,7 +199,11 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_TOC(0);
             ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
             BT_TOC(2);
-            const int2* off = s_off[st] + rbase;
+            int2 off[NIT];                              // (all of them ahead of the copies)
+#pragma unroll
+            for (int it = 0; it < NIT; ++it) off[it] = s_off[st][rbase + it * RSTEP];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&off_empty[st]);
             // dO first: dV, its last reader, is issued before dK, the last reader of Q
             // (RSTEP is a multiple of 8: the rows of a thread have one swizzle)
             const uint32_t dq_ = smem_u32(sQD + st * kQD) + slab_off + sw128_chunk_off(rbase, cchunk & 7);
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_TOC(1);
 #pragma unroll
             for (int it = 0; it < NIT; ++it) {
-                const int o = off[it * RSTEP].y;
+                const int o = off[it].y;
                 cp_async16(dd_ + it * (RSTEP * 128), dc + ((int64_t)max(o, 0) << 3), o >= 0);
             }
             cp_async_mbar_arrive_noinc(&do_full[st]);
@@ -218,12 +222,10 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_TOC(1);
 #pragma unroll
             for (int it = 0; it < NIT; ++it) {
-                const int o = off[it * RSTEP].x;
+                const int o = off[it].x;
                 cp_async16(dq_ + it * (RSTEP * 128), qc + ((int64_t)max(o, 0) << 3), o >= 0);
             }
             cp_async_mbar_arrive_noinc(&q_full[st]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&off_empty[st]);
             BT_EV(k, 1, t == 0);
             BT_TOC(4);
         }
@@ -345,6 +347,8 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_EV(k, 2, lane == 0);
             BT_TOC(3);
             fence_async_smem();
+            __syncwarp();             // no lane is still to see a phase that the products end
+            __syncwarp();
             tc_fence_after();
             const uint32_t aq = qd_lo + (uint32_t)(st * (kQD >> 4));
             const uint32_t ad = aq + (uint32_t)((kTileRows * D * 2) >> 4);
@@ -366,6 +370,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
             BT_TOC(3);
             fence_async_smem();
+            __syncwarp();
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -410,6 +415,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
             BT_TOC(3);
             fence_async_smem();
+            __syncwarp();
             tc_fence_after();
             const uint32_t bk = k_mn_lo + (uint32_t)((kvn % kKStages) * (kK >> 4));
             const uint32_t aq = qd_mn_lo + (uint32_t)(st * (kQD >> 4));
@@ -429,6 +435,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(ds_full, k & 1) && ok;
             BT_TOC(2);
             fence_async_smem();
+            __syncwarp();
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -442,6 +449,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_EV(k, 10, lane == 0);
             ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
             BT_EV(k, 11, lane == 0);
+            __syncwarp();
             tc_fence_after();
             if (leader) {
 #pragma unroll

@@ -4,18 +4,23 @@
 // fsa/ops/FSA_topk_sparse_attention.py:285-566): KV blocks are the outer loop.  A persistent
 // CTA owns a contiguous range of tiles; a tile is <= 128 rows = (query head of the group,
 // selecting token).  Warp-specialised:
-//   warps 0..3  gather the query rows by token id with 16-byte async copies into a ring of swizzled Q stages
-//               (TMA gather4 was measured at ~70 cycles per 512-byte instruction: too slow);
-//   warp 4      one elected thread issues tcgen05.mma S = Q K^T into one of two TMEM S buffers;
-//   warp 5      one elected thread issues O = P V (P read from TMEM, V MN-major from smem) into one
-//               of two TMEM O buffers; two issuing warps keep the two streams from blocking each other;
-//   warps 6..13 two softmax groups, each owning every other tile: one thread per row, row
-//               max / exp2 / row sum from TMEM, P written back to TMEM over S (16-bit), then the
-//               epilogue: O / l rounded to the input dtype, staged in swizzled smem and written
-//               with TMA tile stores (one per warp and 64-column slab);
-//   warp 14     prepares the tokens of the tile rows up to four tiles ahead (the gather warps then issue
-//               no global load of their own);
-//   warp 15     loads the K/V blocks by tiled TMA (128-byte swizzle, double-buffered).
+//   warps 0..3   gather the query rows by token id with 16-byte async copies into a ring of swizzled Q stages
+//                (TMA gather4 was measured at ~70 cycles per 512-byte instruction: too slow);
+//   warp 4       one elected thread issues tcgen05.mma S = Q K^T into one of the TMEM S buffers;
+//   warp 5       one elected thread issues O = P V (P read from TMEM, V MN-major from smem) into one
+//                of two TMEM O buffers; two issuing warps keep the two streams from blocking each other;
+//   warp 6       prepares the entries of the tile rows up to four tiles ahead (the other warps then issue
+//                no global load of their own);
+//   warp 7       loads the K/V blocks by tiled TMA (128-byte swizzle, double-buffered);
+//   warps 8..15  two softmax groups, each owning every other tile: one thread per row, row max / exp2 / row sum
+//                from TMEM, P written back to TMEM over S (16-bit), (m, l) to memory;
+//   warps 16..19 the epilogue of every tile: unnormalised O rounded to the input dtype, staged in swizzled smem 64 columns
+//                at a time and written with TMA tile stores.
+// What bounds it: getting rows in and out; gather, preparation and epilogue warps are each busy for three quarters of the
+// time.  With the epilogue in the softmax groups and 512 threads of one register budget those groups were busy for 0.9 of it.
+// 64K tokens x 8 heads x 16 blocks of 64 keys: 575 -> 520 us (2.1 GB of partial rows at 4.1 TB/s); 21K ragged tokens, 4 heads,
+// 128-key blocks 94 -> 65; head size 256, 16K tokens, 8 heads 300 -> 272.  Eight gather warps (registers: spills) 557 us, two epilogue groups
+// 581, 64 columns per TMEM read of the epilogue 519.
 // Partial rows are stored in TILE ORDER (contiguous 128-row slabs); their (m, l) statistics go to
 // ml[(query head, token, slot)] so that the merge reads a token's pairs as one line.  No atomics, no
 // cross-block state.
@@ -27,7 +32,6 @@
 #include <type_traits>
 
 #include "sel_launch.cuh"
-#include <cstdlib>
 
 namespace fsa {
 
@@ -38,58 +42,36 @@ struct SelFwdParams {
     float scale_log2;        // softmax scale * log2(e)
     int run;                 // tiles per scheduling run (see TileSchedule)
     SelBounds bd;            // visible K/V rows per token
-    int dbg;                 // debug builds only: bit 0 skip Q copies, bit 1 skip partial stores
     ET* opart;               // [max_tiles * 128, D]  unnormalised partial outputs, tile order
     float2* ml;              // [Hq, N, T] (fits in max_tiles * 128 pairs): row max in log2 units, row sum
 };
 
 __host__ __device__ constexpr uint32_t tmem_cols_pow2(int c) { return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512; }
 
+constexpr int kFwdThreads = 640;
+constexpr int kFwdLoaders = 128;
+constexpr int kFwdRing = 4;             // prepared tiles
+// registers per thread of the five warpgroups (gather, issuers, two of softmax, epilogue), out of 96 each at the launch
+constexpr int kFwdRegLoad = 40, kFwdRegMma = 64, kFwdRegSoft = 136, kFwdRegEpi = 96;
+static_assert(kFwdRegLoad + kFwdRegMma + 2 * kFwdRegSoft + kFwdRegEpi <= 5 * 96, "register budget");
+
 template <int D, int BK>
 struct SelFwdCfg {
     static constexpr int kQ = kTileRows * D * 2;
     static constexpr int kKV = 2 * BK * D * 2;         // K then V
-    // Output staging of a softmax warp (32 rows, input dtype): whole rows, or one 64-column slab at a time where that makes room
-    // (head size 256: at all; 128-key blocks at 128: for a second K/V stage)
-    static constexpr int kOSCols = D > 128 || (D == 128 && BK == 128) ? 64 : D;
-    static constexpr int kOS = kTileRows * kOSCols * 2;    // ... of a softmax group
-    static constexpr int kTail = 2560;                 // barriers, TMEM slot, row-offset table
+    static constexpr int kSlab = kTileRows * 128;      // output staging of 64 columns (a quarter per epilogue warp)
+    static constexpr int kTail = 3072;                 // ring of entries, head offsets, records, barriers, TMEM slot
     static constexpr int kMax = 227 * 1024;
-    static constexpr int NKV = (2 * kQ + 2 * kKV + 2 * kOS + kTail <= kMax) ? 2 : 1;    // K/V stages
-    static constexpr int NQ = (3 * kQ + NKV * kKV + 2 * kOS + kTail <= kMax) ? 3 : (2 * kQ + NKV * kKV + 2 * kOS + kTail <= kMax) ? 2 : 1;   // Q stages
-    static constexpr int kBytes = NQ * kQ + NKV * kKV + 2 * kOS + kTail;
-    static constexpr int NO = D <= 128 ? 2 : 1;        // O buffers of D columns: one per softmax group, or one that they take in turns
+    static constexpr int NKV = (2 * kQ + 2 * kKV + 2 * kSlab + kTail <= kMax) ? 2 : 1;    // K/V stages
+    static constexpr int NQ = (3 * kQ + NKV * kKV + 2 * kSlab + kTail <= kMax) ? 3 : (2 * kQ + NKV * kKV + 2 * kSlab + kTail <= kMax) ? 2 : 1;   // Q stages
+    static constexpr int NSL = (NQ * kQ + NKV * kKV + 4 * kSlab + kTail <= kMax) ? 4 : 2; // staged slabs
+    static constexpr int kBytes = NQ * kQ + NKV * kKV + NSL * kSlab + kTail;
+    static constexpr int NO = D <= 128 ? 2 : 1;        // O buffers of D columns
     static constexpr int NS = (4 * BK + NO * D <= 512) ? 4 : 2;   // S buffers (BK columns each); two per softmax group when they fit
     static constexpr int cS = 0;
     static constexpr int cO = NS * BK;
     static constexpr uint32_t kCols = tmem_cols_pow2(NS * BK + NO * D);
 };
-
-// warps: 0..3 gather loaders | 4 issues S = Q K^T | 5 issues O = P V | 6..9 softmax group 0 | 10..13 softmax group 1
-// (any four consecutive warps cover the four TMEM lane quarters, warp % 4) | 14 prepares the tokens of the tile rows up
-// to four tiles ahead | 15 loads the K/V blocks by TMA.  The gather warps issue no global load of their own: a plain
-// load issued behind a burst of async copies waits for the burst.
-constexpr int kFwdThreads = 512;
-constexpr int kFwdLoaders = 128;
-constexpr int kFwdRing = 4;
-
-// Optional cycle accounting per role (debug builds only): FSA_TIMING defines a global table
-// [gridDim.x][32] of accumulated clock64() deltas.
-#ifdef FSA_TIMING
-__device__ unsigned long long g_fwd_timing[512 * 32];
-#define T_DECL unsigned long long _t0 = 0, _acc[12] = {0,0,0,0,0,0,0,0,0,0,0,0}
-#define T_TIC _t0 = clock64()
-#define T_TOC(i) do { unsigned long long _t1 = clock64(); _acc[i] += _t1 - _t0; _t0 = _t1; } while (0)
-#define T_DUMP(base, n) do { for (int _i = 0; _i < (n); ++_i) g_fwd_timing[blockIdx.x * 32 + (base) + _i] = _acc[_i]; } while (0)
-#define TR(role, k, ev) do { if (blockIdx.x == 3 && (k) >= 64 && (k) < 96) g_fwd_trace[((role) * 32 + ((k) - 64)) * 4 + (ev)] = clock64(); } while (0)
-__device__ long long g_fwd_trace[6 * 32 * 4];
-#else
-#define TR(role, k, ev)
-#define T_DECL
-#define T_TIC
-#define T_TOC(i)
-#define T_DUMP(base, n)
-#endif
 
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
@@ -111,9 +93,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
     uint8_t* sQ = smem;
     uint8_t* sKV = sQ + C::NQ * C::kQ;
     uint8_t* sOS = sKV + C::NKV * C::kKV;
-    uint8_t* tail = sOS + 2 * C::kOS;
-    int (*s_tok)[kTileRows] = reinterpret_cast<int (*)[kTileRows]>(tail);   // [4][128] token of every tile row (-1: padding)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tail + kFwdRing * kTileRows * 4);
+    uint8_t* tail = sOS + C::NSL * C::kSlab;
+    uint32_t (*s_ent)[kTileRows] = reinterpret_cast<uint32_t (*)[kTileRows]>(tail);     // [4][128] entry of every tile row (all ones: padding)
+    int* s_goff = reinterpret_cast<int*>(tail + kFwdRing * kTileRows * 4);              // [128] head part of a row's offset (units of 8 elements)
+    int4* s_rec = reinterpret_cast<int4*>(s_goff + kTileRows);   // [4] {kv head, bit 0: first tile of a K/V block, bit 1: last one, first row of the block, -}
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_rec + kFwdRing);
     uint64_t* q_full = bars;                 // [NQ]
     uint64_t* q_empty = q_full + C::NQ;      // [NQ]
     uint64_t* kv_full = q_empty + C::NQ;     // [NKV]
@@ -121,14 +105,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
     uint64_t* s_full = kv_empty + C::NKV;    // [NS]
     uint64_t* s_empty = s_full + C::NS;      // [NS]
     uint64_t* p_full = s_empty + C::NS;      // [NS]
-    uint64_t* o_full = p_full + C::NS;       // [2] per softmax group
-    uint64_t* o_empty = o_full + 2;          // [2]
-    uint64_t* off_full = o_empty + 2;        // [4] ring of prepared tiles: tokens, kv head, new-block flag are valid
-    uint64_t* off_empty = off_full + kFwdRing;   // [4] ... have been read by the gather warps and the S issuer
+    uint64_t* o_full = p_full + C::NS;       // [NO]
+    uint64_t* o_empty = o_full + C::NO;      // [NO]
+    uint64_t* off_full = o_empty + C::NO;    // [4] ring of prepared tiles: entries and record are valid
+    uint64_t* off_empty = off_full + kFwdRing;   // [4] ... have been read by the gather warps, both issuers and the tile's softmax group
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(off_empty + kFwdRing);
-    int* s_h = reinterpret_cast<int*>(off_empty + kFwdRing) + 2;   // [4] kv head of the prepared tile
-    int* s_nb = s_h + kFwdRing;                                    // [4] 1: the tile starts a new K/V block
-    static_assert(kFwdRing * kTileRows * 4 + (2 * C::NQ + 2 * C::NKV + 3 * C::NS + 4 + 2 * kFwdRing) * 8 + 8 + 8 * kFwdRing <= C::kTail,
+    static_assert((kFwdRing + 1) * kTileRows * 4 + kFwdRing * 16 + (2 * C::NQ + 2 * C::NKV + 3 * C::NS + 2 * C::NO + 2 * kFwdRing) * 8 + 8 <= C::kTail,
                   "tail budget");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -141,16 +123,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 
     if (tid == 0) {
         for (int i = 0; i < C::NQ; ++i) { mbar_init(&q_full[i], kFwdLoaders); mbar_init(&q_empty[i], 1); }
-        for (int i = 0; i < kFwdRing; ++i) { mbar_init(&off_full[i], 1); mbar_init(&off_empty[i], kFwdLoaders / 32 + 1); }
+        for (int i = 0; i < kFwdRing; ++i) { mbar_init(&off_full[i], 1); mbar_init(&off_empty[i], kFwdLoaders / 32 + 2 + 4); }
         for (int i = 0; i < C::NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
         for (int i = 0; i < C::NS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 1); mbar_init(&p_full[i], 128); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 128); }
+        for (int i = 0; i < C::NO; ++i) { mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 128); }
         mbar_init_fence();
         tma_prefetch_desc(&kmap);
         tma_prefetch_desc(&vmap);
         tma_prefetch_desc(&omap);
     }
     if (warp == 0) tmem_alloc(&tmem_slot, C::kCols);
+    if (tid < kTileRows) s_goff[tid] = (int)(((tid / s.TPT) * q_sh) >> 3);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -158,379 +141,259 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 
     const TileSchedule sched(p.ix.header[1], p.run);
     const int nloc = sched.nloc;
+    bool ok = true;                          // no wait of this thread has run out
 
     if (warp < 4) {
         // ------------------------------------------------------------------ gather warps (128 threads)
         // Thread t copies 16-byte chunk (t % CPR) of the rows t / CPR, t / CPR + RSTEP, ... (a half-warp covers one
-        // 256-byte row).  Tokens come from the prepared ring; the head part of a row offset is a thread constant.
-        T_DECL;
-        const int t = tid;
-        bool ok = true;
+        // 256-byte row).
+        reg_dec<kFwdRegLoad>();
         constexpr int CPR = D / 8;                         // 16-byte chunks per row
         constexpr int RSTEP = kFwdLoaders / CPR;           // rows advanced per iteration
         constexpr int NIT = kTileRows / RSTEP;
-        const int cchunk = t % CPR, rbase = t / CPR;
-        const uint32_t slab_off = (uint32_t)(cchunk >> 3) * (kTileRows * 128);
-        int gq[NIT];                                       // (head-in-group * head stride) / 8 of this thread's rows
-#pragma unroll
-        for (int it = 0; it < NIT; ++it) gq[it] = (int)((((rbase + it * RSTEP) / s.TPT) * q_sh) >> 3);
-        const int qsn8 = (int)(q_sn >> 3);
+        const int cchunk = tid % CPR, rbase = tid / CPR;
+        const uint32_t dst0 = smem_u32(sQ) + (uint32_t)(cchunk >> 3) * (kTileRows * 128);
+        const int qsn8 = (int)(q_sn >> 3), qsh8 = (int)(q_sh >> 3);
         const ET* qc = q + cchunk * 8;
+        int qs = 0, qph = 1;                               // Q stage and the parity of its release
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            const int qs = k % C::NQ, slot = k % kFwdRing;
-            T_TIC;
+            const int slot = k % kFwdRing;
             // the Q stage is free once the S MMA of the tile that used it is done
-            ok = mbar_wait(&q_empty[qs], ((k / C::NQ) & 1) ^ 1, status) && ok;
-            T_TOC(1);
-            if (t == 0) TR(0, k, 0);
-            ok = mbar_wait(&off_full[slot], (k / kFwdRing) & 1, status) && ok;
-            const int hq0 = (int)(((long long)s_h[slot] * s.G * q_sh) >> 3);
-            const uint32_t dstq = smem_u32(sQ + qs * C::kQ) + slab_off;
-            constexpr int NB = NIT < 16 ? NIT : 16;            // rows whose tokens are held at a time
-#pragma unroll
+            ok = mbar_poll(&q_empty[qs], qph) && ok;
+            ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+            const int hq0 = s_rec[slot].x * s.G * qsh8;
+            const uint32_t dst = dst0 + qs * C::kQ;
+            constexpr int NB = 8;                              // rows whose offsets are read together, ahead of their copies
+#pragma unroll 1
             for (int i0 = 0; i0 < NIT; i0 += NB) {
-                int tok[NB];
+                int off[NB];
 #pragma unroll
-                for (int it = 0; it < NB; ++it) tok[it] = s_tok[slot][rbase + (i0 + it) * RSTEP];
-                if (i0 + NB == NIT) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&off_empty[slot]);
-                    T_TOC(2);
+                for (int it = 0; it < NB; ++it) {
+                    const int r = rbase + (i0 + it) * RSTEP;
+                    const uint32_t ent = s_ent[slot][r];
+                    off[it] = ent != 0xFFFFFFFFu ? (int)(ent >> kSlotBits) * qsn8 + hq0 + s_goff[r] : -1;
                 }
-#ifdef FSA_TIMING
-                if (!(p.dbg & 1))
-#endif
-                {
 #pragma unroll
-                    for (int it = 0; it < NB; ++it) {
-                        const int r = rbase + (i0 + it) * RSTEP;
-                        const bool valid = tok[it] >= 0;
-                        const int tk = valid ? tok[it] : 0;
-                        cp_async16(dstq + sw128_chunk_off(r, cchunk & 7), qc + ((long long)(tk * qsn8 + hq0 + gq[i0 + it]) << 3), valid);
-                    }
-                }
+                for (int it = 0; it < NB; ++it)
+                    cp_async16(dst + sw128_chunk_off(rbase + (i0 + it) * RSTEP, cchunk & 7), qc + ((int64_t)max(off[it], 0) << 3), off[it] >= 0);
             }
             // arrives on q_full when this thread's copies have landed; nobody waits here, so the
             // loader never holds a finished tile back behind a later wait
             cp_async_mbar_arrive_noinc(&q_full[qs]);
-            T_TOC(3);
-            if (t == 0) TR(0, k, 1);
-        }
-        if (t == 0) T_DUMP(0, 5);
-    } else if (warp == 14) {
-        // ------------------------------------------------------------------ tile preparation (tokens of the rows)
-        // lane l owns rows l, l + 32, l + 64, l + 96; records and entries are fetched three tiles ahead
-        bool ok = true;
-        int gg[4], ee[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = lane + 32 * i;
-            gg[i] = r / s.TPT;
-            ee[i] = r - gg[i] * s.TPT;
-        }
-        struct Pre { int h, hg; uint32_t e[4]; };
-        auto fetch = [&](int k, Pre& m) {
-            const int j = sched.tile(k);
-            const TileInfo ti = load_tile(p.ix, j);
-            m.h = ti.h; m.hg = ti.hg;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) m.e[i] = gg[i] < s.G ? __ldg(p.ix.entries + (int64_t)j * s.TPT + ee[i]) : 0xFFFFFFFFu;
-        };
-        Pre m1{0, -1, {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}}, m2 = m1, m3 = m1;
-        if (nloc > 0) fetch(0, m1);
-        if (nloc > 1) fetch(1, m2);
-        if (nloc > 2) fetch(2, m3);
-        int prev_hg = -1;
-        for (int k = 0; k < nloc && ok; ++k) {
-            const int slot = k % kFwdRing;
-            const Pre cur = m1;
-            m1 = m2; m2 = m3;
-            if (k + 3 < nloc) fetch(k + 3, m3);
-            ok = mbar_wait(&off_empty[slot], ((k / kFwdRing) & 1) ^ 1, status) && ok;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s_tok[slot][lane + 32 * i] = cur.e[i] != 0xFFFFFFFFu ? (int)(cur.e[i] >> kSlotBits) : -1;
-            if (lane == 0) {
-                s_h[slot] = cur.h;
-                s_nb[slot] = cur.hg != prev_hg ? 1 : 0;
-            }
-            prev_hg = cur.hg;
             __syncwarp();
-            if (lane == 0) mbar_arrive(&off_full[slot]);
+            if (lane == 0) mbar_arrive(&off_empty[slot]);
+            if (++qs == C::NQ) { qs = 0; qph ^= 1; }
         }
-    } else if (warp == 15) {
-        // ------------------------------------------------------------------ K/V blocks by TMA
-        bool ok = true;
-        int kvn = -1, prev_hg = -1;
-        TileInfo t1{0, 0, 0, -1, 0}, t2 = t1;
-        if (nloc > 0) t1 = load_tile(p.ix, sched.tile(0));
-        if (nloc > 1) t2 = load_tile(p.ix, sched.tile(1));
-        for (int k = 0; k < nloc && ok; ++k) {
-            const TileInfo cur = t1;
-            t1 = t2;
-            if (k + 2 < nloc) t2 = load_tile(p.ix, sched.tile(k + 2));
-            if (cur.hg == prev_hg) continue;
-            prev_hg = cur.hg;
-            ++kvn;
-            if (lane == 0) {
-                const int ks = kvn % C::NKV;
-                ok = mbar_wait(&kv_empty[ks], ((kvn / C::NKV) & 1) ^ 1, status) && ok;
-                mbar_expect_tx(&kv_full[ks], (uint32_t)C::kKV);
-                uint8_t* dK = sKV + ks * C::kKV;
-                uint8_t* dV = dK + BK * D * 2;
-#pragma unroll
-                for (int b = 0; b < D / 64; ++b) {
-                    tma_load_2d(smem_u32(dK + b * BK * 128), &kmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
-                    tma_load_2d(smem_u32(dV + b * BK * 128), &vmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
-                }
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        }
-    } else if (warp == 4) {
-        // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T
-        // The whole warp walks the loop (uniform control flow); one elected lane issues.  S and P V
-        // are issued by different warps so that neither waits behind the other's barriers.
-        const bool leader = elect_one();
-        constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, BK, false, false);
-        // descriptor words: constant high word (SBO 1024, version, swizzle), low words of the bases
-        constexpr uint32_t hi_1024 = umma_desc_hi(1024);
-        const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16);
-        const uint32_t k_lo = umma_desc_lo(smem_u32(sKV), 16);
-        int kvn = -1;
-        bool ok = true;
-        T_DECL;
-        for (int k = 0; k < nloc && ok; ++k) {
-            const int qs = k % C::NQ, sbuf = k % C::NS;
-            T_TIC;
-            // "does this tile start a new K/V block": published by the loader with the Q stage
-            ok = mbar_wait(&off_full[k % kFwdRing], (k / kFwdRing) & 1, status) && ok;
-            const int new_block = s_nb[k % kFwdRing];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&off_empty[k % kFwdRing]);
-            if (new_block != 0) {
-                ++kvn;
-                ok = mbar_wait(&kv_full[kvn % C::NKV], (kvn / C::NKV) & 1, status) && ok;
-            }
-            T_TOC(1);
-            if (lane == 0) TR(1, k, 0);
-            ok = mbar_wait(&q_full[qs], (k / C::NQ) & 1, status) && ok;
-            fence_async_smem();   // the Q rows were written by cp.async (generic proxy)
-            T_TOC(2);
-            if (lane == 0) TR(1, k, 1);
-            ok = mbar_wait(&s_empty[sbuf], ((k / C::NS) & 1) ^ 1, status) && ok;
-            T_TOC(3);
-            if (lane == 0) TR(1, k, 2);
-            tc_fence_after();
-            const uint32_t a_lo = q_lo + (uint32_t)(qs * (C::kQ >> 4));
-            const uint32_t b_lo = k_lo + (uint32_t)((kvn % C::NKV) * (C::kKV >> 4));
-            const uint32_t d_s = tbase + C::cS + sbuf * BK;
-            if (leader) {
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    // k-step ks: 64-column slab ks / 4, 32-byte step (ks % 4) inside the 128-byte swizzle row
-                    constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
-                    umma_ss(d_s, umma_desc_pack(a_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
-                            umma_desc_pack(b_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
-                }
-                umma_commit(&q_empty[qs]);
-                umma_commit(&s_full[sbuf]);
-            }
-            __syncwarp();
-            T_TOC(4);
-            if (lane == 0) TR(1, k, 3);
-        }
-        if (lane == 0) T_DUMP(8, 5);
-    } else if (warp == 5) {
-        // ------------------------------------------------------------------ MMA issuer 2: O = P V
-        const bool leader = elect_one();
-        constexpr uint32_t idesc_o = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
-        constexpr uint32_t hi_1024 = umma_desc_hi(1024);
-        const uint32_t v_lo = umma_desc_lo(smem_u32(sKV + BK * D * 2), BK * 128);   // MN-major: LBO = slab stride
-        int kvn = -1;
-        bool ok = true;
-        T_DECL;
-        // block ids of the CTA's tiles, fetched two tiles ahead (needed to know when a K/V stage is done)
-        int hg0 = -1, hg1 = -1, hg2 = -1;
-        if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
-        if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
-        for (int k = 0; k < nloc && ok; ++k) {
-            const int ob = k % C::NO, sbuf = k % C::NS;
-            const int prev_hg = hg0;
-            hg0 = hg1; hg1 = hg2;
-            if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
-            if (hg0 != prev_hg) ++kvn;
-            const bool last_of_block = (k + 1 >= nloc) || (hg1 != hg0);
-            const int kv_cur = kvn % C::NKV;
-            T_TIC;
-            ok = mbar_wait(&p_full[sbuf], (k / C::NS) & 1, status) && ok;
-            T_TOC(5);
-            if (lane == 0) TR(2, k, 0);
-            ok = mbar_wait(&o_empty[ob], ((k / C::NO) & 1) ^ 1, status) && ok;
-            T_TOC(6);
-            if (lane == 0) TR(2, k, 1);
-            tc_fence_after();
-            const uint32_t b_lo = v_lo + (uint32_t)(kv_cur * (C::kKV >> 4));
-            const uint32_t d_o = tbase + C::cO + ob * D, a_p = tbase + C::cS + sbuf * BK;
-            if (leader) {
-#pragma unroll
-                for (int ks = 0; ks < BK / 16; ++ks)
-                    umma_ts(d_o, a_p + ks * 8, umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_o, ks > 0);
-                umma_commit(&o_full[k & 1]);           // (per group, also when they share one O: a group waits for its own tiles only)
-                umma_commit(&s_empty[sbuf]);
-                if (last_of_block) umma_commit(&kv_empty[kv_cur]);
-            }
-            __syncwarp();
-            T_TOC(7);
-            if (lane == 0) TR(2, k, 2);
-        }
-#ifdef FSA_TIMING
-        if (lane == 0) for (int i = 5; i < 8; ++i) g_fwd_timing[blockIdx.x * 32 + 8 + i] = _acc[i];
-#endif
-    } else {
-        // ------------------------------------------------------------------ softmax + epilogue
-        // Group sb (warps 6..9 / 10..13) owns the CTA's tiles with odd / even local index, hence TMEM
-        // buffers S[sb], O[sb] (head size 256: the one O in turns) and its own staging area.  One row per thread.
-        const int sb = (warp - 6) >> 2;
-        const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
-        const int r = quarter * 32 + lane;
-        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        const int g = r / s.TPT;
-        const int e = r - g * s.TPT;
-        // this warp's 32 staged rows: slabs of 32 rows x 128 bytes, 128-byte swizzle
-        uint8_t* my_os = sOS + sb * C::kOS + quarter * (32 * C::kOSCols * 2);
-        const int ob = C::NO == 2 ? sb : 0;
-        // the (m, l) pairs of a (head, token) complete a 128-byte line over T tiles far apart in time: keep those lines in
-        // L2; the partial rows are written once and read once by the merge: let them leave first
-        const uint64_t pol_ml = l2_policy_evict_last(), pol_part = l2_policy_evict_first();
-        const uint32_t tS0 = tbase + lane_off + C::cS;
-        const uint32_t tO = tbase + lane_off + C::cO + ob * D;
-        bool ok = true;
-        T_DECL;
-        // software pipeline over this group's tiles: the entry of this thread's row is fetched two
-        // own tiles ahead, the visible-column bounds (which may need the token's row limits) one ahead
-        const bool row_exists = g < s.G;
-        uint32_t entA = 0xFFFFFFFFu, entB = 0xFFFFFFFFu;
-        int row0A = 0, row0B = 0, cloA = 0, chiA = BK, hA = 0, hB = 0;
-        // tile indices of this group's tiles k, k + 2, k + 4 without a division per tile: a cursor (run index, offset
-        // in the run) that advances by two
-        int cq = sb / sched.run, cr = sb % sched.run;
-        auto cursor_next = [&]() {
-            const int j = (cq * sched.grid + sched.cta) * sched.run + cr;
-            cr += 2;
-            while (cr >= sched.run) { cr -= sched.run; ++cq; }
-            return j;
-        };
-        int jA = 0, jB = 0;
-        auto fetch_ent = [&](int j, uint32_t& ent, int& row0, int& h) {
-            const TileInfo ti = load_tile(p.ix, j);
-            row0 = ti.row0; h = ti.h;
-            ent = 0xFFFFFFFFu;
-            if (row_exists) ent = __ldg(p.ix.entries + (int64_t)j * s.TPT + e);
-        };
-        // statistics go to ml[(head, token, slot)]: the merge kernel reads a token's T pairs as one contiguous line
-        auto ml_index = [&](uint32_t ent, int h) {
-            return ((int64_t)(h * s.G + g) * s.N + (int64_t)(ent >> kSlotBits)) * s.T + (int)(ent & ((1u << kSlotBits) - 1));
-        };
-        auto fetch_bounds = [&](uint32_t ent, int row0, int& c_lo, int& c_hi) {
-            c_lo = 0; c_hi = BK;   // padding rows: anything finite
-            if (ent != 0xFFFFFFFFu) visible_cols(p.bd, (int)(ent >> kSlotBits), row0, BK, c_lo, c_hi);
-        };
-        bool have_prev = false, prev_valid = false;
-        int prev_j = 0, prev_u = 0;
-        float prev_m = 0.f, prev_l = 0.f;
-        int64_t prev_mli = 0;
-        // O / l -> staging -> TMA store, for the tile (prev_j) whose softmax ran one iteration ago
-        auto epilogue = [&]() {
-            T_TIC;
-            ok = mbar_wait(&o_full[sb], prev_u & 1, status) && ok;
-            T_TOC(3);
-            if (quarter == 2 && lane == 0) TR(3, prev_u * 2 + sb, 2);
-            tc_fence_after();
-            // (two TMEM loads in flight per wait, 64 columns per round trip, measured 5 % slower than one)
-#pragma unroll
-            for (int s0 = 0; s0 < D; s0 += C::kOSCols) {
-                if (lane == 0) bulk_wait_read0();   // previous store of this warp has read its staging rows
+    } else if (warp < 8) {
+        reg_dec<kFwdRegMma>();
+        if (warp == 4) {
+            // -------------------------------------------------------------- MMA issuer 1: S = Q K^T
+            // The whole warp walks the loop (uniform control flow); one elected lane issues.  S and P V
+            // are issued by different warps so that neither waits behind the other's barriers.
+            const bool leader = elect_one();
+            constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, BK, false, false);
+            // descriptor words: constant high word (SBO 1024, version, swizzle), low words of the bases
+            constexpr uint32_t hi_1024 = umma_desc_hi(1024);
+            const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16);
+            const uint32_t k_lo = umma_desc_lo(smem_u32(sKV), 16);
+            int kvn = -1, qs = 0, qph = 0;
+#pragma unroll 1
+            for (int k = 0; k < nloc && ok; ++k) {
+                const int sbuf = k % C::NS, slot = k % kFwdRing;
+                ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+                const int blk = s_rec[slot].y;
                 __syncwarp();
-                T_TOC(4);
+                if (lane == 0) mbar_arrive(&off_empty[slot]);
+                if (blk & 1) {
+                    ++kvn;
+                    ok = mbar_poll(&kv_full[kvn % C::NKV], (kvn / C::NKV) & 1) && ok;
+                }
+                ok = mbar_poll(&q_full[qs], qph) && ok;
+                fence_async_smem();   // the Q rows were written by cp.async (generic proxy)
+                ok = mbar_poll(&s_empty[sbuf], ((k / C::NS) & 1) ^ 1) && ok;
+                __syncwarp();         // no lane is still to see a phase that the products end
+                tc_fence_after();
+                const uint32_t a_lo = q_lo + (uint32_t)(qs * (C::kQ >> 4));
+                const uint32_t b_lo = k_lo + (uint32_t)((kvn % C::NKV) * (C::kKV >> 4));
+                const uint32_t d_s = tbase + C::cS + sbuf * BK;
+                if (leader) {
+#pragma unroll 4
+                    for (int ks = 0; ks < D / 16; ++ks) {
+                        // k-step ks: 64-column slab ks / 4, 32-byte step (ks % 4) inside the 128-byte swizzle row
+                        constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
+                        umma_ss(d_s, umma_desc_pack(a_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
+                                umma_desc_pack(b_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
+                    }
+                    umma_commit(&q_empty[qs]);
+                    umma_commit(&s_full[sbuf]);
+                }
+                __syncwarp();
+                if (++qs == C::NQ) { qs = 0; qph ^= 1; }
+            }
+        } else if (warp == 5) {
+            // -------------------------------------------------------------- MMA issuer 2: O = P V
+            const bool leader = elect_one();
+            constexpr uint32_t idesc_o = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
+            constexpr uint32_t hi_1024 = umma_desc_hi(1024);
+            const uint32_t v_lo = umma_desc_lo(smem_u32(sKV + BK * D * 2), BK * 128);   // MN-major: LBO = slab stride
+            int kvn = -1;
+#pragma unroll 1
+            for (int k = 0; k < nloc && ok; ++k) {
+                const int ob = k % C::NO, sbuf = k % C::NS, slot = k % kFwdRing;
+                ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+                const int blk = s_rec[slot].y;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&off_empty[slot]);
+                if (blk & 1) ++kvn;
+                ok = mbar_poll(&o_empty[ob], ((k / C::NO) & 1) ^ 1) && ok;
+                ok = mbar_poll(&p_full[sbuf], (k / C::NS) & 1) && ok;
+                __syncwarp();
+                tc_fence_after();
+                const int kv_cur = kvn % C::NKV;
+                const uint32_t b_lo = v_lo + (uint32_t)(kv_cur * (C::kKV >> 4));
+                const uint32_t d_o = tbase + C::cO + ob * D, a_p = tbase + C::cS + sbuf * BK;
+                if (leader) {
 #pragma unroll
-                for (int c0 = 0; c0 < C::kOSCols; c0 += 32) {
-                    uint32_t v[32];
-                    tmem_ld32(tO + s0 + c0, v);
-                    tmem_ld_wait();
+                    for (int ks = 0; ks < BK / 16; ++ks)
+                        umma_ts(d_o, a_p + ks * 8, umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_o, ks > 0);
+                    umma_commit(&o_full[ob]);
+                    umma_commit(&s_empty[sbuf]);
+                    if (blk & 2) umma_commit(&kv_empty[kv_cur]);
+                }
+                __syncwarp();
+            }
+        } else if (warp == 6) {
+            // -------------------------------------------------------------- tile preparation (entries of the rows)
+            // lane l owns rows l, l + 32, l + 64, l + 96; records and entries are fetched three tiles ahead
+            uint32_t gg = 0;                    // head (of the group) of the lane's rows, a byte each
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        // unnormalised O (its row sum l travels in the statistics): rounding to a floating-point
-                        // format is scale-free, so dividing first would not make the partial more accurate
-                        uint4 x;
-                        x.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-                        x.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-                        x.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-                        x.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-                        const int chunk = (c0 >> 3) + q4;     // 16-byte chunk of the staged row
-                        *reinterpret_cast<uint4*>(my_os + (chunk >> 3) * (32 * 128) + sw128_chunk_off(lane, chunk & 7)) = x;
+            for (int i = 0; i < 4; ++i) gg |= (uint32_t)((lane + 32 * i) / s.TPT) << (8 * i);
+            struct Pre { int h, hg, row0; uint32_t e[4]; };
+            TileCursorT<false> ahead(sched);
+            auto fetch = [&](Pre& m) {
+                const TileInfo ti = load_tile(p.ix, ahead.j);
+                m.h = ti.h; m.hg = ti.hg; m.row0 = ti.row0;
+                const uint32_t* ent = p.ix.entries + (int64_t)ahead.j * s.TPT + lane;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int g = gg >> (8 * i) & 255;
+                    m.e[i] = g < s.G ? __ldg(ent + 32 * i - g * s.TPT) : 0xFFFFFFFFu;
+                }
+                ahead.next(sched);
+            };
+            Pre m1{0, -1, 0, {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}}, m2 = m1, m3 = m1;
+            if (nloc > 0) fetch(m1);
+            if (nloc > 1) fetch(m2);
+            if (nloc > 2) fetch(m3);
+            int prev_hg = -1;
+            // publishes tile k from m and fetches tile k + 3 into it (three in turn: handing the registers on would wait for the loads)
+            auto publish = [&](int k, Pre& m, const Pre& next) {
+                const int slot = k % kFwdRing;
+                ok = mbar_poll(&off_empty[slot], ((k / kFwdRing) & 1) ^ 1) && ok;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s_ent[slot][lane + 32 * i] = m.e[i];
+                if (lane == 0)
+                    s_rec[slot] = make_int4(m.h, (m.hg != prev_hg ? 1 : 0) | (k + 1 >= nloc || next.hg != m.hg ? 2 : 0), m.row0, 0);
+                prev_hg = m.hg;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&off_full[slot]);
+                if (k + 3 < nloc) fetch(m);
+            };
+#pragma unroll 1
+            for (int k = 0; k < nloc && ok; k += 3) {
+                publish(k, m1, m2);
+                if (k + 1 < nloc) publish(k + 1, m2, m3);
+                if (k + 2 < nloc) publish(k + 2, m3, m1);
+            }
+        } else {
+            // -------------------------------------------------------------- K/V blocks by TMA
+            int kvn = -1, prev_hg = -1;
+            TileInfo t1{0, 0, 0, -1, 0}, t2 = t1;
+            TileCursorT<false> ahead(sched);
+            auto fetch = [&](TileInfo& t) { t = load_tile(p.ix, ahead.j); ahead.next(sched); };
+            if (nloc > 0) fetch(t1);
+            if (nloc > 1) fetch(t2);
+#pragma unroll 1
+            for (int k = 0; k < nloc && ok; ++k) {
+                const TileInfo cur = t1;
+                t1 = t2;
+                if (k + 2 < nloc) fetch(t2);
+                if (cur.hg == prev_hg) continue;
+                prev_hg = cur.hg;
+                ++kvn;
+                if (lane == 0) {
+                    const int ks = kvn % C::NKV;
+                    ok = mbar_poll(&kv_empty[ks], ((kvn / C::NKV) & 1) ^ 1) && ok;
+                    mbar_expect_tx(&kv_full[ks], (uint32_t)C::kKV);
+                    uint8_t* dK = sKV + ks * C::kKV;
+                    uint8_t* dV = dK + BK * D * 2;
+#pragma unroll
+                    for (int b = 0; b < D / 64; ++b) {
+                        tma_load_2d(smem_u32(dK + b * BK * 128), &kmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
+                        tma_load_2d(smem_u32(dV + b * BK * 128), &vmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
                     }
                 }
-                if (s0 + C::kOSCols == D) {
-                    tc_fence_before();
-                    mbar_arrive(&o_empty[ob]);
-                    if (prev_valid) st_float2_hint(p.ml + prev_mli, prev_m, prev_l, pol_ml);
-                }
-                fence_async_smem();
-                __syncwarp();
-#ifdef FSA_TIMING
-                if (!(p.dbg & 2))
-#endif
-                if (lane == 0) {
-#pragma unroll
-                    for (int b = 0; b < C::kOSCols / 64; ++b)
-                        tma_store_2d_hint(&omap, s0 + b * 64, prev_j * kTileRows + quarter * 32, smem_u32(my_os + b * (32 * 128)), pol_part);
-                    bulk_commit();
-                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
-            T_TOC(5);
-            if (quarter == 2 && lane == 0) TR(3, prev_u * 2 + sb, 3);
+        }
+    } else if (warp < 16) {
+        // ------------------------------------------------------------------ softmax
+        // Group sb (warps 8..11 / 12..15) owns the CTA's tiles with even / odd local index.  One row per thread.
+        reg_inc<kFwdRegSoft>();
+        const int sb = (warp - 8) >> 2;
+        const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
+        const int r = quarter * 32 + lane;
+        const int g = r / s.TPT;
+        // the (m, l) pairs of a (head, token) complete a 128-byte line over T tiles far apart in time: keep those lines in L2
+        const uint64_t pol_ml = l2_policy_evict_last();
+        const uint32_t tS0 = tbase + ((uint32_t)(quarter * 32) << 16) + C::cS;
+        // entry, (m, l) place and visible key columns of this thread's row of the group's next tile
+        uint32_t ent = 0xFFFFFFFFu;
+        int64_t mli = 0;
+        int c_lo = 0, c_hi = BK;
+        auto fetch = [&](int k) {
+            const int slot = k % kFwdRing;
+            ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+            ent = s_ent[slot][r];
+            const int4 rec = s_rec[slot];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&off_empty[slot]);
+            c_lo = 0; c_hi = BK;                      // padding rows: anything finite
+            if (ent != 0xFFFFFFFFu) {
+                const int tok = (int)(ent >> kSlotBits);
+                visible_cols(p.bd, tok, rec.z, BK, c_lo, c_hi);
+                // statistics go to ml[(head, token, slot)]: the merge kernel reads a token's T pairs as one contiguous line
+                mli = ((int64_t)(rec.x * s.G + g) * s.N + tok) * s.T + (int)(ent & ((1u << kSlotBits) - 1));
+            }
         };
-        if (sb < nloc) {
-            jA = cursor_next();
-            fetch_ent(jA, entA, row0A, hA);
-            fetch_bounds(entA, row0A, cloA, chiA);
-        }
-        if (sb + 2 < nloc) {
-            jB = cursor_next();
-            fetch_ent(jB, entB, row0B, hB);
-        }
+        if (sb < nloc) fetch(sb);
+#pragma unroll 1
         for (int k = sb; k < nloc && ok; k += 2) {
-            const int j = jA;
-            const int u = k >> 1;                     // use count of this group's O buffer
             const int sbuf = k % C::NS;
             const uint32_t tS = tS0 + sbuf * BK;
-            const bool row_valid = entA != 0xFFFFFFFFu;
-            const int c_lo = cloA, c_hi = chiA;            // visible key columns of this row
-            const int64_t mli = row_valid ? ml_index(entA, hA) : 0;
-            entA = entB; row0A = row0B; hA = hB; jA = jB;
-            T_TIC;
-            if (k + 2 < nloc) fetch_bounds(entA, row0A, cloA, chiA);
-            if (k + 4 < nloc) {
-                jB = cursor_next();
-                fetch_ent(jB, entB, row0B, hB);
-            }
-            T_TOC(0);
-            ok = mbar_wait(&s_full[sbuf], (k / C::NS) & 1, status) && ok;
-            T_TOC(1);
-            if (quarter == 2 && lane == 0) TR(3, k, 0);
+            ok = mbar_poll(&s_full[sbuf], (k / C::NS) & 1) && ok;
             tc_fence_after();
             // A row is held in registers W = 32 or 64 columns at a time: one TMEM read for a block of that size.  128 columns: the upper half
             // is read for its maximum, then the lower one, which stays, then (P of the lower half is in its place, over S) the upper one
             // again.  (Four 32-column reads twice over, one running maximum and sum: 140 -> 101 us for 21K ragged tokens x 4 heads.)
             constexpr int W = BK < 64 ? BK : 64;
+            const bool masked = __any_sync(0xffffffffu, c_lo > 0 || c_hi < BK);
             uint32_t v[W];
             auto load = [&](int c0) {
                 tmem_ld32(tS + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[0]));
                 if constexpr (W == 64) tmem_ld32(tS + c0 + 32, *reinterpret_cast<uint32_t (*)[32]>(&v[W - 32]));
                 tmem_ld_wait();
-                if (c_lo > c0 || c_hi < c0 + W) {
+                if (masked) {
 #pragma unroll
-                    for (int i = 0; i < W; ++i)
-                        if (c0 + i < c_lo || c0 + i >= c_hi) v[i] = 0xff800000u;   // -inf: exp2 gives exactly 0
+                    for (int i0 = 0; i0 < W; i0 += 32) {
+                        // (bit i: column c0 + i0 + i is visible)
+                        const int lo = min(max(c_lo - c0 - i0, 0), 32), hi = min(max(c_hi - c0 - i0, 0), 32);
+                        const uint32_t vis = (uint32_t)((1ull << hi) - 1) & ~(uint32_t)((1ull << lo) - 1);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (!(vis >> i & 1u)) v[i0 + i] = 0xff800000u;   // -inf: exp2 gives exactly 0
+                    }
                 }
             };
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, ls[4] = {0.f, 0.f, 0.f, 0.f};
@@ -570,25 +433,66 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 load(W);
                 probabilities(W);
             }
-            const float l = (ls[0] + ls[1]) + (ls[2] + ls[3]);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&p_full[sbuf]);
-            T_TOC(2);
-            if (quarter == 2 && lane == 0) TR(3, k, 1);
-
-            // the epilogue of this group's previous tile runs now: its P V has had a whole softmax
-            // to finish, so the wait below is normally free.  (With one O buffer this tile's own: the other group's P V waits
-            // for the buffer.)
-            if (C::NO == 2 && have_prev) epilogue();
-            have_prev = C::NO == 2;
-            prev_j = j; prev_u = u; prev_m = m; prev_l = l; prev_valid = row_valid; prev_mli = mli;
-            if (C::NO == 1) epilogue();
+            if (ent != 0xFFFFFFFFu) st_float2_hint(p.ml + mli, m, (ls[0] + ls[1]) + (ls[2] + ls[3]), pol_ml);
+            if (k + 2 < nloc) fetch(k + 2);
         }
-        if (have_prev && ok) epilogue();
+    } else {
+        // ------------------------------------------------------------------ epilogue: O -> staging -> TMA store
+        // unnormalised O (its row sum l travels in the statistics): rounding to a floating-point format is scale-free, so
+        // dividing first would not make the partial more accurate
+        const int quarter = warp & 3;
+        // this warp's 32 staged rows: slabs of 32 rows x 128 bytes, 128-byte swizzle
+        uint8_t* my_os = sOS + quarter * (32 * 128);
+        // the partial rows are written once and read once by the merge: let them leave L2 first
+        const uint64_t pol_part = l2_policy_evict_first();
+        const uint32_t tO0 = tbase + ((uint32_t)(quarter * 32) << 16) + C::cO;
+        TileCursorT<false> cur(sched);
+        int slab = 0;
+#pragma unroll 1
+        for (int k = 0; k < nloc && ok; ++k) {
+            const int ob = k % C::NO;
+            ok = mbar_poll(&o_full[ob], (k / C::NO) & 1) && ok;
+            tc_fence_after();
+#pragma unroll 1
+            for (int b = 0; b < D / 64; ++b) {
+                uint8_t* stage = my_os + slab * C::kSlab;
+                if (lane == 0) bulk_wait_read<C::NSL - 1>();    // the store that used this slab has read it
+                __syncwarp();
+#pragma unroll
+                for (int c0 = 0; c0 < 64; c0 += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tO0 + ob * D + b * 64 + c0, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q4 = 0; q4 < 4; ++q4) {
+                        uint4 x;
+                        x.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
+                        x.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
+                        x.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
+                        x.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
+                        *reinterpret_cast<uint4*>(stage + sw128_chunk_off(lane, (c0 >> 3) + q4)) = x;
+                    }
+                }
+                if (b == D / 64 - 1) {
+                    tc_fence_before();
+                    mbar_arrive(&o_empty[ob]);
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d_hint(&omap, b * 64, cur.j * kTileRows + quarter * 32, smem_u32(stage), pol_part);
+                    bulk_commit();
+                }
+                if (++slab == C::NSL) slab = 0;
+            }
+            cur.next(sched);
+        }
         if (lane == 0) bulk_wait0();
-        if (warp == 6 && lane == 0) T_DUMP(16, 6);
     }
+    if (!ok) atomicMax(status, (int)kStatusWaitTimeout);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, C::kCols);
@@ -890,10 +794,6 @@ static cudaError_t launch_sel_fwd(const SelFwdArgs& a, const SelShape& s, const 
     p.opart = (ET*)a.opart; p.ml = a.ml;
     p.run = a.run;
     p.bd = a.bd;
-    p.dbg = 0;
-#ifdef FSA_TIMING
-    { const char* v = getenv("FSA_DBG"); p.dbg = v ? atoi(v) : 0; }
-#endif
     cudaError_t e;
     constexpr bool kPipelined = BK <= 128;
     // the gather warps of the pipelined kernel address rows by 32-bit offsets in units of 8 elements
@@ -960,12 +860,3 @@ cudaError_t dispatch_sel_fwd(int dtype, const SelFwdArgs& a, const SelShape& s, 
 }
 
 }  // namespace fsa
-
-#ifdef FSA_TIMING
-extern "C" int fsa_debug_read_fwd_trace(long long* host, int n) {
-    return (int)cudaMemcpyFromSymbol(host, fsa::g_fwd_trace, (size_t)n * sizeof(long long));
-}
-extern "C" int fsa_debug_read_fwd_timing(unsigned long long* host, int n) {
-    return (int)cudaMemcpyFromSymbol(host, fsa::g_fwd_timing, (size_t)n * sizeof(unsigned long long));
-}
-#endif
