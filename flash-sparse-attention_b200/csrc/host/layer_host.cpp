@@ -33,6 +33,12 @@ struct Lengths {
     }
     int win_blocks(const LayerCfg& c) const { return (c.window + 1 + 63) / 64 + 1; }       // 64-row blocks that a token's range can touch
     int cmp_blocks() const { return (max_cmp + 63) / 64 + 1; }
+    // Does every token select every block up to its own?  The selection then is causal attention over its whole sequence, for which
+    // the query-tile-major kernels need no scores, no index and no partial rows.  32 / 8 heads, prefill of 517 tokens 202 -> 158 us, of 1024
+    // 275 -> 195; 16 / 4 heads, training step on 8 x 1000 tokens 1909 -> 1640, on 64 x 200 2745 -> 2560.  From the first longer sequence on
+    // the selection has to run for it.  (Head size 128: their backward; the block-major one that serves the others gains nothing.)
+    bool every_block(const LayerCfg& c) const { return c.D == 128 && max_len <= (int64_t)c.topk * c.bs; }
+    int own_blocks() const { return (max_len + 63) / 64 + 1; }
 };
 
 // What a forward leaves for the backward.
@@ -87,18 +93,24 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     std::tie(t.o_cmp, t.lse_cmp) = range_fwd(t.q, t.ck, t.cv, cu, t.cu_cmp, nullptr, bd, scale, status);
     const int max_blocks = (s.max_len + c.bs - 1) / c.bs, t_out = std::min(c.topk, max_blocks);
     t.topk = i32({c.Hk, N, t_out}, x);
-    check(fsa_select_topk_fused(ptr(t.q), t.q.stride(0), ptr(t.ck), t.ck.stride(0), t.lse_cmp.data_ptr<float>(), iptr(cu), iptr(t.cu_cmp), N, s.Nc,
-                                s.B, c.Hq, c.Hk, c.D, dt, scale, c.ks, c.stride, c.bs, c.init_blocks, c.local_blocks, max_blocks, t_out,
-                                t.topk.data_ptr<int32_t>(), status, st),
-          "fsa_select_topk_fused");
-    std::tie(t.o_sel, t.lse_sel, t.ws) = sel_fwd(t.q, t.k, t.v, t.topk, c.bs, cu, scale);
+    if (s.every_block(c)) {
+        check(fsa_layer_every_block(iptr(cu), s.B, N, c.Hk, t_out, c.bs, t.topk.data_ptr<int32_t>(), st), "fsa_layer_every_block");
+        if (checking_status()) t.ws = at::zeros({4}, x.options().dtype(at::kInt));      // (the branch's own word, read as the operator's is)
+        std::tie(t.o_sel, t.lse_sel) = range_fwd(t.q, t.k, t.v, cu, cu, nullptr, bd + 2 * N, scale, t.ws.defined() ? t.ws.data_ptr<int32_t>() : nullptr);
+    } else {
+        check(fsa_select_topk_fused(ptr(t.q), t.q.stride(0), ptr(t.ck), t.ck.stride(0), t.lse_cmp.data_ptr<float>(), iptr(cu), iptr(t.cu_cmp), N, s.Nc,
+                                    s.B, c.Hq, c.Hk, c.D, dt, scale, c.ks, c.stride, c.bs, c.init_blocks, c.local_blocks, max_blocks, t_out,
+                                    t.topk.data_ptr<int32_t>(), status, st),
+              "fsa_select_topk_fused");
+        std::tie(t.o_sel, t.lse_sel, t.ws) = sel_fwd(t.q, t.k, t.v, t.topk, c.bs, cu, scale);
+    }
     std::tie(t.o_win, t.lse_win) = range_fwd(t.q, t.k, t.v, cu, cu, bd + N, bd + 2 * N, scale, status);
     t.gate = fresh({N, 3}, x);
     Tensor out = fresh({N, (int64_t)c.Hq * c.D}, x);
     check(fsa_gate_proj_mix_fwd(ptr(x), x.stride(0), ptr(wg), ptr(t.o_cmp), ptr(t.o_sel), ptr(t.o_win), N, (int)hidden, c.Hq * c.D, dt, ptr(out),
                                 ptr(t.gate), st),
           "fsa_gate_proj_mix_fwd");
-    check_status(ptr(t.ws), x, "fsa_sel_fwd status");
+    if (t.ws.defined()) check_status(ptr(t.ws), x, "fsa_sel_fwd status");
     check_status(status, x, "range attention and block selection status");
     return out;
 }
@@ -106,7 +118,7 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
 // dq, dk, dv of one of the dense branches
 static std::tuple<Tensor, Tensor, Tensor> range_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& lse, const Tensor& dout,
                                                     const float* delta, const Tensor& cu_q, const Tensor& cu_k, const int32_t* lo, const int32_t* hi,
-                                                    int max_blocks, float scale) {
+                                                    int max_blocks, float scale, const char* what = "fsa_range_attn_bwd_delta status") {
     const int64_t N = q.size(0), Nk = k.size(0);
     const int B = (int)cu_q.size(0) - 1, Hq = (int)q.size(1), Hk = (int)k.size(1), D = (int)q.size(2);
     int64_t ib = 0, fb = 0, bb = 0;
@@ -119,7 +131,7 @@ static std::tuple<Tensor, Tensor, Tensor> range_bwd(const Tensor& q, const Tenso
                                    max_blocks, 64, dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), dout.stride(0), dout.stride(1),
                                    scale, ptr(dq), ptr(dk), ptr(dv), ptr(ws), ws.numel(), ptr(scratch), scratch.numel(), stream_of(q)),
           "fsa_range_attn_bwd_delta");
-    check_status(ptr(ws), q, "fsa_range_attn_bwd_delta status");
+    check_status(ptr(ws), q, what);
     return {dq, dk, dv};
 }
 
@@ -171,8 +183,11 @@ struct NsaLayer : torch::autograd::Function<NsaLayer> {
         const float* dl = delta.data_ptr<float>();
         auto [dq0, dck, dcv] = range_bwd(q, ck, cv, lse_cmp, d_cmp, dl, cu, cu_cmp, nullptr, bd, s.cmp_blocks(), scale);
         d_cmp.reset();
-        auto [dq1, dk, dv] = sel_bwd_delta(q, k, v, lse_sel, d_sel, dl + (int64_t)c.Hq * N, topk, c.bs, cu, scale, ws);
-        check_status(ptr(ws), q, "fsa_sel_bwd_delta status");
+        const float* dl_sel = dl + (int64_t)c.Hq * N;
+        auto [dq1, dk, dv] = s.every_block(c) ? range_bwd(q, k, v, lse_sel, d_sel, dl_sel, cu, cu, nullptr, bd + 2 * N, s.own_blocks(), scale,
+                                                          "fsa_sel_bwd_delta status")
+                                              : sel_bwd_delta(q, k, v, lse_sel, d_sel, dl_sel, topk, c.bs, cu, scale, ws);
+        if (!s.every_block(c)) check_status(ptr(ws), q, "fsa_sel_bwd_delta status");
         d_sel.reset();
         auto [dq2, dk2, dv2] = range_bwd(q, k, v, lse_win, d_win, dl + 2 * (int64_t)c.Hq * N, cu, cu, bd + N, bd + 2 * N, s.win_blocks(c), scale);
         d_win.reset();

@@ -249,6 +249,27 @@ extern "C" int fsa_layer_rope_bwd(const void* dq0, const void* dq1, const void* 
     return run_rope<true>(p, dtype, (cudaStream_t)stream);
 }
 
+namespace fsa {
+__global__ void __launch_bounds__(256) layer_every_block_kernel(const int* __restrict__ cu, int B, int N, int Hk, int T, int BK, int* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;       // row (kv head, token), slot
+    if (i >= (int64_t)Hk * N * T) return;
+    const int64_t row = i / T;
+    const int slot = (int)(i - row * T), n = (int)(row % N);
+    out[i] = slot <= (n - __ldg(cu + find_seq(cu, B, n))) / BK ? slot : -1;
+}
+}  // namespace fsa
+
+extern "C" int fsa_layer_every_block(const int32_t* cu_seqlens, int batch, int64_t total, int num_kv_heads, int topk, int block_size, int32_t* topk_idx,
+                                     void* stream) {
+    if (!cu_seqlens || batch < 0 || total < 0 || total >= kMaxTokens || num_kv_heads <= 0 || topk <= 0 || block_size <= 0 || (total > 0 && !topk_idx))
+        return FSA_ERR_BAD_ARG;
+    if (total == 0 || batch == 0) return FSA_OK;
+    (void)cudaGetLastError();
+    const int64_t n = total * num_kv_heads * topk;
+    layer_every_block_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(cu_seqlens, batch, (int)total, num_kv_heads, topk, block_size, topk_idx);
+    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
 // partial column sums [parts][H][D]; called by the compressor's backward
 namespace fsa {
 cudaError_t launch_column_sum(int dtype, int D, const void* dy, int64_t rows, int H, int parts, float* out, int* status, cudaStream_t stream) {

@@ -301,6 +301,11 @@ int fsa_layer_rope_fwd(const void* q, int64_t q_stride_n, const void* k, int64_t
                        int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride, int window, int dtype,
                        void* q_out, void* k_out, int32_t* hi_cmp, int32_t* lo_win, int32_t* hi_win, void* stream);
 
+/* Block ids [num_kv_heads, total, topk] of tokens that select every block up to their own, ascending, -1 behind them: what a
+ * selection of topk blocks comes to in sequences of at most topk blocks. */
+int fsa_layer_every_block(const int32_t* cu_seqlens, int batch, int64_t total, int num_kv_heads, int topk, int block_size, int32_t* topk_idx,
+                          void* stream);
+
 /* dq = inverse rotation of dq0 + dq1 + dq2; dk = that of dk0 + dk1, plus dk2 (the compressor's share, of the unrotated keys);
  * dv = dv0 + dv1 + dv2; dcmp_k in place.  total 0: the compressed keys alone; total_cmp 0: everything else.  An output may be
  * one of its inputs. */
