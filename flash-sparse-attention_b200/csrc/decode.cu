@@ -97,14 +97,21 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
         if (p.rng_lo) {
             lo_r = rlo[j]; hi_r = rhi[j];
         } else {
-            const int len = __ldg(p.seq_len + b);
-            lo_r = __ldg(p.row0 + b);
+            const int len = p.seq_len[b];
+            lo_r = p.row0[b];
             hi_r = lo_r + (len >= p.ks ? (len - p.ks) / p.stride + 1 : 0);
         }
         lo = lo_r + c * p.chunk;
         n = lo_r < 0 ? 0 : max(min(hi_r, lo + p.chunk) - lo, 0);
     };
     const int64_t pbase = ((int64_t)b * p.Hq + h * G) * P + pidx;
+    if (tid == 0) {
+        for (int s = 0; s < nst; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        mbar_init_fence();
+        tma_prefetch_desc(&kmap);
+        tma_prefetch_desc(&vmap);
+    }
+    follow();
     int total = 0;
     for (int j = j0; j < j1; ++j) {
         int lo, n;
@@ -114,10 +121,6 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
     if (total == 0) {
         if (tid < G) p.ml[pbase + (int64_t)tid * P] = make_float2(-INFINITY, 0.f);
         return;
-    }
-    if (tid == 0) {
-        for (int s = 0; s < nst; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
-        mbar_init_fence();
     }
     __syncthreads();
     const uint32_t sbase = smem_u32(base);
@@ -372,9 +375,9 @@ __global__ void __launch_bounds__(256) lse_merge_kernel(const float* __restrict_
 constexpr int kFinishThreads = 64, kFinishAhead = 1024;      // rows up to which the many registers of AHEAD still let all warps run at once
 
 template <bool AHEAD, typename ET>
-__global__ void __launch_bounds__(kFinishThreads) decode_finish_kernel(const float* __restrict__ o_part, const float2* __restrict__ ml, int64_t rows,
-                                                            int ns, int nw, int PS, int D, int Hq, const ET* __restrict__ o_cmp,
-                                                            const ET* __restrict__ gate, ET* __restrict__ out) {
+__global__ void __launch_bounds__(kFinishThreads) decode_finish_kernel(const float* o_part, const float2* ml, int64_t rows, int ns, int nw, int PS,
+                                                                      int D, int Hq, const ET* o_cmp, const ET* gate, ET* out) {
+    follow();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -623,8 +626,7 @@ static cudaError_t launch_partial_tma(DecodeParams p, const CUtensorMap& kmap, c
     auto kern = decode_partial_tma<D, HI, ET>;
     const cudaError_t e = allow_smem((const void*)kern, 3 * STAGE_BYTES + 2048);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)((int64_t)p.B * p.Hk * p.NP * p.nchunk), 160, smem, stream>>>(p, kmap, vmap);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3((unsigned)((int64_t)p.B * p.Hk * p.NP * p.nchunk)), 160, smem, stream, 1, p, kmap, vmap);
 }
 
 template <int D, typename ET>
@@ -791,15 +793,17 @@ extern "C" int fsa_decode_finish(const float* o_part, const float* ml, int64_t r
     unsigned grid = (unsigned)((rows + kFinishThreads / 32 - 1) / (kFinishThreads / 32));
     cudaStream_t st = (cudaStream_t)stream;
     auto run = [&](auto kern, auto* o_, const auto* c, const auto* g) {
-        kern<<<grid, kFinishThreads, 0, st>>>(o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride, head_dim, num_q_heads, c, g, o_);
+        return launch_dependent(kern, dim3(grid), kFinishThreads, 0, st, 1, o_part, (const float2*)ml, rows, num_sel_partials, num_win_partials, part_stride, head_dim,
+                                num_q_heads, c, g, o_);
     };
+    cudaError_t e;
     const bool few = rows <= kFinishAhead;
     if (dtype == FSA_DTYPE_BF16)
-        run(few ? decode_finish_kernel<true, __nv_bfloat16> : decode_finish_kernel<false, __nv_bfloat16>, (__nv_bfloat16*)out,
-            (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)gate);
+        e = run(few ? decode_finish_kernel<true, __nv_bfloat16> : decode_finish_kernel<false, __nv_bfloat16>, (__nv_bfloat16*)out,
+                (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)gate);
     else if (dtype == FSA_DTYPE_FP16)
-        run(few ? decode_finish_kernel<true, __half> : decode_finish_kernel<false, __half>, (__half*)out, (const __half*)o_cmp, (const __half*)gate);
+        e = run(few ? decode_finish_kernel<true, __half> : decode_finish_kernel<false, __half>, (__half*)out, (const __half*)o_cmp, (const __half*)gate);
     else
         return FSA_ERR_BAD_ARG;
-    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }

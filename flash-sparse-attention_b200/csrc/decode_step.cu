@@ -3,6 +3,10 @@
 // kernels of a few microseconds, so what bounds it is the number of launches and dependent steps: 63 launches (torch glue
 // around the library's kernels) took 180 us of GPU time for eight requests whose bytes need 25.
 //
+// Every kernel of a step is launched as a dependent one (sm100_prims.cuh): its CTAs come up while the kernel before it ends, and the
+// projections fetch their weights into L2 meanwhile (one request of 8191 tokens, 32 / 8 heads with projections: 58.0 -> 49.7 us a
+// step, 33 MB of weights being on their way under the merge; from a graph, where launches cost less, 72.5 -> 71.0 for eight requests).
+//
 // Replaces the host-side glue of the reference's step (fsa_preview/module/fsa_decode.py:84-199: projections, torch.cat of
 // the caches, the incremental compressor fsa_preview/ops/linear_compress_decode.py:14-76, gate).
 #include "../../include/fsa_sm100.h"
@@ -61,6 +65,13 @@ __global__ void __launch_bounds__(256) decode_proj_kernel(const DecodeProjParams
     const ET* xr[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) xr[t] = (const ET*)p.x + (int64_t)min(t * 8 + gid, p.B - 1) * p.x_stride + warp * kw + tig * 8;
+    // the CTA's 16 rows of W are fetched while the kernel before this one ends (a hint: nothing is read yet)
+    {
+        const char* wb = reinterpret_cast<const char*>((const ET*)p.w[m] + (int64_t)row0 * p.K);
+        const int lines = min(16, rows - row0) * (p.K / 64);            // of 128 bytes
+        for (int i = tid; i < lines; i += 256) prefetch_l2(wb + (int64_t)i * 128);
+    }
+    follow();
     float c[NT][4];
 #pragma unroll
     for (int t = 0; t < NT; ++t) c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
@@ -69,7 +80,7 @@ __global__ void __launch_bounds__(256) decode_proj_kernel(const DecodeProjParams
         const uint4 a = __ldcs(reinterpret_cast<const uint4*>(w0 + k)), b = __ldcs(reinterpret_cast<const uint4*>(w1 + k));
         uint4 xv[NT];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) xv[t] = __ldg(reinterpret_cast<const uint4*>(xr[t] + k));
+        for (int t = 0; t < NT; ++t) xv[t] = __ldcg(reinterpret_cast<const uint4*>(xr[t] + k));
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             mma_16816<ET>(c[t], a.x, b.x, a.y, b.y, xv[t].x, xv[t].y);
@@ -124,6 +135,7 @@ __global__ void __launch_bounds__(256) decode_append_kernel(const DecodeAppendPa
     __shared__ float s_cos[128], s_sin[128];
     __shared__ float s_z[3][8];
     const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    follow();
     const int t = p.seq_len[b];
     const int half = p.D / 2;
     const bool rot = p.inv_freq != nullptr;
@@ -138,11 +150,11 @@ __global__ void __launch_bounds__(256) decode_append_kernel(const DecodeAppendPa
         const int nv = p.glen / 8;
         float acc[3] = {0.f, 0.f, 0.f};
         for (int i = tid; i < nv; i += 256) {
-            const uint4 xv = __ldg(x + i);
+            const uint4 xv = __ldcg(x + i);
             const uint32_t* px = &xv.x;
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                const uint4 wv = __ldg(w + (int64_t)j * nv + i);
+                const uint4 wv = __ldcg(w + (int64_t)j * nv + i);
                 const uint32_t* pw = &wv.x;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -238,6 +250,7 @@ __global__ void __launch_bounds__(256, 1) decode_compress_kernel(const DecodeCom
     const ET* w = (const ET*)(is_k ? p.wk : p.wv) + ((int64_t)h * p.ks * D + (int64_t)rank * KS) * D;
     const ET* pe = is_k && p.pe ? (const ET*)p.pe + (int64_t)h * p.ks * D + (int64_t)rank * KS : nullptr;
     const int cgi = tid % CG, kl = tid / CG;
+    follow();
     for (int next = 0;;) {
         if (warp == 0) {
             int n = 0, b0 = next;
@@ -285,7 +298,7 @@ __global__ void __launch_bounds__(256, 1) decode_compress_kernel(const DecodeCom
             for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
 #pragma unroll 8
         for (int e = kl; e < KS; e += KL) {
-            const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)e * D) + cgi);
+            const uint4 wv = __ldcg(reinterpret_cast<const uint4*>(w + (int64_t)e * D) + cgi);
             const uint32_t* pw = &wv.x;
             float f[8];
 #pragma unroll
@@ -406,6 +419,7 @@ __global__ void __launch_bounds__(256) decode_select_kernel(const DecodeSelectPa
     __shared__ uint32_t cand[8 * 64], s_best[8 * 64], sel[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x / p.Hk, h = blockIdx.x % p.Hk;
+    follow();
     const int len = p.seq_len[b], t = len - 1;
     const int ncmp = len >= p.ks ? (len - p.ks) / p.stride + 1 : 0;
     const int bq = t / p.BK, nb = t >= 0 ? min(bq + 1, p.max_blocks) : 0;
@@ -582,14 +596,9 @@ extern "C" int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k
     p.tile0[num] = tiles;
     (void)cudaGetLastError();
     cudaStream_t st = (cudaStream_t)stream;
-    if (dtype == FSA_DTYPE_BF16) {
-        if (batch <= 8) decode_proj_kernel<1, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
-        else decode_proj_kernel<2, __nv_bfloat16><<<tiles, 256, 0, st>>>(p);
-    } else {
-        if (batch <= 8) decode_proj_kernel<1, __half><<<tiles, 256, 0, st>>>(p);
-        else decode_proj_kernel<2, __half><<<tiles, 256, 0, st>>>(p);
-    }
-    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+    auto kern = dtype == FSA_DTYPE_BF16 ? (batch <= 8 ? decode_proj_kernel<1, __nv_bfloat16> : decode_proj_kernel<2, __nv_bfloat16>)
+                                        : (batch <= 8 ? decode_proj_kernel<1, __half> : decode_proj_kernel<2, __half>);
+    return launch_dependent(kern, dim3((unsigned)tiles), 256, 0, st, 1, p) == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
 extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void* v_in, void* q_out, void* k_cache, void* v_cache, void* k_tail,
@@ -607,9 +616,8 @@ extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void*
     p.inv_freq = inv_freq; p.seq_len = seq_len; p.seq_row0 = seq_row0; p.spare_row = (int64_t)batch * cap; p.cap = cap; p.ks = kernel_size;
     p.z = gate_logits; p.gx = gate_x; p.gw = gate_w; p.glen = gate_dim; p.gate = gate; p.Hq = num_q_heads; p.Hk = num_kv_heads; p.D = head_dim;
     (void)cudaGetLastError();
-    if (dtype == FSA_DTYPE_BF16) decode_append_kernel<__nv_bfloat16><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
-    else decode_append_kernel<__half><<<batch, 256, 0, (cudaStream_t)stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+    auto kern = dtype == FSA_DTYPE_BF16 ? decode_append_kernel<__nv_bfloat16> : decode_append_kernel<__half>;
+    return launch_dependent(kern, dim3((unsigned)batch), 256, 0, (cudaStream_t)stream, 1, p) == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
 template <int D, typename ET>
@@ -619,17 +627,7 @@ static cudaError_t launch_compress(const DecodeCompressParams& p, cudaStream_t s
     auto kern = decode_compress_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kDcSplit, (unsigned)p.Hk, 2);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kDcSplit; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return launch_dependent(kern, dim3(kDcSplit, (unsigned)p.Hk, 2), 256, smem, stream, kDcSplit, p);
 }
 
 extern "C" int fsa_decode_compress(const void* k_tail, const void* v_tail, const void* w_key, const void* w_value, const void* pe,
@@ -678,7 +676,6 @@ extern "C" int fsa_decode_merge_select(const float* o_part, const float* ml, int
     const void* kern = dtype == FSA_DTYPE_BF16 ? (const void*)decode_select_kernel<__nv_bfloat16> : (const void*)decode_select_kernel<__half>;
     if (smem > 48 * 1024 && allow_smem(kern, (int)smem) != cudaSuccess) return FSA_ERR_CUDA;
     const unsigned grid = (unsigned)(batch * num_kv_heads);
-    if (dtype == FSA_DTYPE_BF16) decode_select_kernel<__nv_bfloat16><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
-    else decode_select_kernel<__half><<<grid, 256, smem, (cudaStream_t)stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+    auto run = dtype == FSA_DTYPE_BF16 ? decode_select_kernel<__nv_bfloat16> : decode_select_kernel<__half>;
+    return launch_dependent(run, dim3(grid), 256, smem, (cudaStream_t)stream, 1, p) == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }

@@ -28,6 +28,24 @@ cudaError_t allow_smem(const void* kern, int bytes);
 cudaError_t prefer_l1(const void* kern, int smem_percent = 0);
 // SMs of this process's device, for the rules that sizes and launches share; a B200's where no device answers (size queries need none).
 int sm_count();
+// Launch of a kernel that begins with follow(): its CTAs are brought up, and its weights fetched, while the kernel before it ends.
+// cluster: CTAs (in x) of a cluster.
+template <typename... KA, typename... A>
+static inline cudaError_t launch_dependent(void (*kern)(KA...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, unsigned cluster, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
 // Binds the current device's primary context to the calling thread: tensor-map encoding is a driver call and needs one.
 int ensure_context();
 
@@ -56,6 +74,16 @@ __device__ __forceinline__ bool elect_one() {
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(pred));
     return pred != 0;
+}
+
+// ---------------------------------------------------------------- dependent launches
+// A kernel launched by launch_dependent (below) may start while the one before it in the stream still runs.  Every thread of it calls
+// follow() before it reads or writes anything of a kernel before it, and before it may return: from there on all of them have
+// ended and their writes are seen.  The kernel after it may start from then on too, so that only one kernel is ever ahead.  What the
+// kernel before wrote is not read through the non-coherent path (__ldg, const __restrict__): such a load may be moved before this.
+__device__ __forceinline__ void follow() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- mbarrier
@@ -130,6 +158,9 @@ __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// A hint: the line of p into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---------------------------------------------------------------- TMA
 // 2-D tiled load: box of the tensor map starting at (x = innermost element, y = row).

@@ -81,3 +81,34 @@ def test_compressor_reductions(seqlens, H, D, ks, st):
             assert float((y[at : at + n].double() - ref).norm() / ref.norm()) <= 5e-3, f"sequence {i}"
         at += n
     assert at == y.shape[0] == int(ycu[-1])
+
+
+@pytest.mark.parametrize("B,Hk,G,D,hidden", [(1, 8, 4, 128, 4096), (12, 2, 4, 64, 1024), (20, 4, 4, 128, 2048)])
+def test_steps_in_a_row_match_steps_one_by_one(B, Hk, G, D, hidden):
+    """The kernels of a step start while the one before them ends: steps without a wait between them, each fed with the output of the
+    one before, against the same steps with a wait after each -- outputs and caches bit for bit."""
+    torch.manual_seed(B)
+    mod = FlashSparseAttentionDecode(hidden, Hk * G, Hk, D, 32, 16, 64, 8, 1, 2, 100, rope_config=RopeConfig(head_dim=D)).to(DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        for p in mod.parameters():
+            torch.nn.init.xavier_uniform_(p)
+    lens = [600 + 37 * b for b in range(B)]
+    x0 = torch.randn(B, hidden, device=DEV).to(torch.bfloat16)
+
+    def run(wait):
+        torch.manual_seed(1)
+        c = mod.new_cache(B, 2048, dtype=torch.bfloat16, device=DEV)
+        for t in (c.k, c.v, c.cmp_k, c.cmp_v, c.k_tail, c.v_tail):
+            t.normal_()
+        c.host_len = list(lens)
+        c.seq_len.copy_(torch.tensor(lens, dtype=torch.int32))
+        x, ys = x0, []
+        for _ in range(40):
+            x = (x + mod.step(x, c)).clamp(-4, 4)
+            ys.append(x)
+            if wait:
+                torch.cuda.synchronize()
+        return ys + [getattr(c, n)[:-1] for n in ("k", "v", "cmp_k", "cmp_v", "k_tail", "v_tail")] + [c.seq_len]
+
+    with torch.no_grad():
+        assert all(torch.equal(a, b) for a, b in zip(run(False), run(True)))
