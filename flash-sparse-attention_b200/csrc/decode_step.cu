@@ -219,8 +219,12 @@ __global__ void __launch_bounds__(256) decode_append_kernel(const DecodeAppendPa
 // For every sequence whose length seq_len[b] (after the append) completes a window: y = ring rows (oldest first) W[h], rounded,
 // plus the position-embedding bias pe W (keys), rotated at m * stride (keys, with inv_freq), to row m of the compressed
 // cache.  A cluster of 8 CTAs per (kv head, K or V) splits the ks * D reduction; their partial sums meet in distributed
-// shared memory.  Sequences are taken eight at a time; when none completes a window, which is most steps of a small batch,
-// no weight is read and the launch ends at once (a batched library GEMM over all sequences read 17 MB every step: 35 us).
+// shared memory.  When no sequence completes a window, which is most steps of a small batch, no weight is read and the launch
+// ends at once (a batched library GEMM over all sequences read 17 MB every step: 35 us).
+// Bound by reading W once (17 MB for 8 heads of 128): a CTA takes its 512 rows of it to shared memory, the ring rows of up to
+// 79 sequences and pe beside them, and the warp-level MMA (fp32 sums) goes over both; a warp has D / 8 columns.  (As multiply-adds
+// of a thread, eight sequences at a time and W read again for each eight, the average step of 64 sequences of one length took 460 us
+// instead of 438, that of eight sequences 71.0 instead of 66.7.)
 struct DecodeCompressParams {
     const void *k_tail, *v_tail;         // [B * ks + 1, Hk, D] rings
     const void *wk, *wv;                 // [Hk, ks * D, D]
@@ -232,131 +236,145 @@ struct DecodeCompressParams {
     int B, Hk, ks, stride, cmp_cap;
 };
 
-constexpr int kDcSplit = 8, kDcSeqs = 8, kDcPitch = 12;
+// CTAs of a cluster; rows of a turn (sequences, and pe behind them); rows of W that are staged at a time; padding of a staged row
+constexpr int kDcSplit = 8, kDcRows = 80, kDcChunk = 512, kDcPad = 8;
+template <int D> constexpr int dc_smem() { return (kDcChunk * (D + kDcPad) + kDcRows * (kDcChunk + kDcPad)) * 2; }
+
+__device__ __forceinline__ void ldsm_x2_trans(uint32_t addr, uint32_t& r0, uint32_t& r1) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+}
 
 template <int D, typename ET>
 __global__ void __launch_bounds__(256, 1) decode_compress_kernel(const DecodeCompressParams p) {
     namespace cg = cooperative_groups;
-    constexpr int CG = D / 8, KL = 256 / CG;          // 16-byte column groups, reduction lanes
-    extern __shared__ __align__(16) float dcs[];      // [KS][kDcPitch] inputs, later [8][kDcSeqs + 1][D] sums of the warps
-    __shared__ float part[(kDcSeqs + 1) * D], s_y[D];
-    __shared__ int s_act[kDcSeqs], s_n, s_next;
+    constexpr int WP = D + kDcPad, AP = kDcChunk + kDcPad;      // pitches: 8 rows of a fragment lie in 8 different groups of banks
+    constexpr int MT = kDcRows / 16, NT = D / 64;               // 16-row tiles of a turn; 8-column tiles of a warp
+    constexpr int PAR = 256 / D;                                // rows that are finished at a time
+    extern __shared__ __align__(128) unsigned char dcs[];
+    ET* sw = reinterpret_cast<ET*>(dcs);                        // [kDcChunk][WP]
+    ET* sa = sw + kDcChunk * WP;                                // [kDcRows][AP], later [kDcRows][D] sums
+    float* part = reinterpret_cast<float*>(sa);
+    __shared__ float s_y[PAR][D];
+    __shared__ int s_act[kDcRows], s_len[kDcRows], s_n, s_next;
     cg::cluster_group cluster = cg::this_cluster();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
     const int rank = blockIdx.x, h = blockIdx.y;
     const bool is_k = blockIdx.z == 0;
-    const int KS = p.ks * D / kDcSplit;
+    const int KS = p.ks * D / kDcSplit;                         // a multiple of 64
     const ET* tail = (const ET*)(is_k ? p.k_tail : p.v_tail);
     const ET* w = (const ET*)(is_k ? p.wk : p.wv) + ((int64_t)h * p.ks * D + (int64_t)rank * KS) * D;
     const ET* pe = is_k && p.pe ? (const ET*)p.pe + (int64_t)h * p.ks * D + (int64_t)rank * KS : nullptr;
-    const int cgi = tid % CG, kl = tid / CG;
     follow();
     for (int next = 0;;) {
         if (warp == 0) {
             int n = 0, b0 = next;
-            for (; b0 < p.B && n < kDcSeqs; b0 += 32) {
+            for (; b0 < p.B && n < kDcRows - 1; b0 += 32) {
                 const int b = b0 + lane;
                 const int len = b < p.B ? p.seq_len[b] : 0;
                 unsigned m = __ballot_sync(0xffffffffu, len >= p.ks && (len - p.ks) % p.stride == 0);
                 int last = 31;
-                while (m && n < kDcSeqs) {
+                while (m && n < kDcRows - 1) {
                     last = __ffs(m) - 1;
-                    if (lane == 0) s_act[n] = b0 + last;
+                    if (lane == last) { s_act[n] = b; s_len[n] = len; }
                     ++n;
                     m &= m - 1;
                 }
-                if (n == kDcSeqs) { b0 += last + 1; break; }
+                if (n == kDcRows - 1) { b0 += last + 1; break; }
             }
             if (lane == 0) { s_n = n; s_next = b0; }
         }
         __syncthreads();
         const int n = s_n;
         if (n == 0) break;                             // (the same for every CTA of the cluster)
-        // eight inputs of one sequence (or of pe) per thread, transposed: the sequences of one input are adjacent
-        for (int i = tid; i < (kDcSeqs + 1) * (KS / 8); i += 256) {
-            const int a = i % (kDcSeqs + 1), e = i / (kDcSeqs + 1) * 8;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (a < n) {
-                const int b = s_act[a], kk = rank * KS + e, o = kk / D, d = kk - o * D;
-                x = *reinterpret_cast<const uint4*>(tail + (((int64_t)b * p.ks + (p.seq_len[b] + o) % p.ks) * p.Hk + h) * D + d);
-            } else if (a == kDcSeqs && pe) {
-                x = *reinterpret_cast<const uint4*>(pe + e);
-            }
-            const uint32_t* px = &x.x;
+        const int mt = (n + (pe ? 1 : 0) + 15) / 16;
+        float acc[MT][NT][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = ElemTraits<ET>::unpack2(px[j]);
-                dcs[(e + 2 * j) * kDcPitch + a] = f.x;
-                dcs[(e + 2 * j + 1) * kDcPitch + a] = f.y;
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+        for (int k0 = 0; k0 < KS; k0 += kDcChunk) {
+            const int kc = min(kDcChunk, KS - k0);
+            if (k0) __syncthreads();                   // the chunk before has been read
+            for (int i = tid; i < kc * (D / 8); i += 256) {
+                const int e = i / (D / 8), c = i % (D / 8) * 8;
+                cp_async16(smem_u32(sw + e * WP + c), w + (int64_t)(k0 + e) * D + c, true);
+            }
+            for (int i = tid; i < mt * 16 * (kc / 8); i += 256) {
+                const int a = i / (kc / 8), e = i % (kc / 8) * 8;
+                const ET* src = tail;                  // (rows behind the last one: zeros)
+                if (a < n) {
+                    const int kk = rank * KS + k0 + e, o = kk / D;
+                    src = tail + (((int64_t)s_act[a] * p.ks + (s_len[a] + o) % p.ks) * p.Hk + h) * D + (kk - o * D);
+                } else if (a == n && pe) {
+                    src = pe + k0 + e;
+                }
+                cp_async16(smem_u32(sa + a * AP + e), src, a < n || (a == n && pe));
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncthreads();
+            const uint32_t wb = smem_u32(sw + (lane & 15) * WP + warp * (D / 8) + (lane >> 4) * 8);
+            const uint32_t ab = smem_u32(sa + (lane & 15) * AP + (lane >> 4) * 8);
+#pragma unroll 2
+            for (int k = 0; k < kc; k += 16) {
+                uint32_t b[2 * NT];
+                if constexpr (NT == 2)
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(wb + k * WP * 2));
+                else ldsm_x2_trans(wb + k * WP * 2, b[0], b[1]);
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    if (i >= mt) break;
+                    uint32_t a0, a1, a2, a3;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(ab + (i * 16 * AP + k) * 2));
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) mma_16816<ET>(acc[i][j], a0, a1, a2, a3, b[2 * j], b[2 * j + 1]);
+                }
             }
         }
-        __syncthreads();
-        float acc[kDcSeqs + 1][8];
+        __syncthreads();                               // the inputs have been read: the sums take their place
 #pragma unroll
-        for (int a = 0; a <= kDcSeqs; ++a)
+        for (int i = 0; i < MT; ++i) {
+            if (i >= mt) break;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
-#pragma unroll 8
-        for (int e = kl; e < KS; e += KL) {
-            const uint4 wv = __ldcg(reinterpret_cast<const uint4*>(w + (int64_t)e * D) + cgi);
-            const uint32_t* pw = &wv.x;
-            float f[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 t = ElemTraits<ET>::unpack2(pw[j]);
-                f[2 * j] = t.x; f[2 * j + 1] = t.y;
+            for (int j = 0; j < NT; ++j) {
+                float* at = part + (i * 16 + gid) * D + warp * (D / 8) + j * 8 + tig * 2;
+                *reinterpret_cast<float2*>(at) = make_float2(acc[i][j][0], acc[i][j][1]);
+                *reinterpret_cast<float2*>(at + 8 * D) = make_float2(acc[i][j][2], acc[i][j][3]);
             }
-            const float4 x0 = *reinterpret_cast<const float4*>(dcs + e * kDcPitch), x1 = *reinterpret_cast<const float4*>(dcs + e * kDcPitch + 4);
-            const float xs[kDcSeqs + 1] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, dcs[e * kDcPitch + 8]};
-#pragma unroll
-            for (int a = 0; a <= kDcSeqs; ++a)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[a][j] = fmaf(xs[a], f[j], acc[a][j]);
-        }
-        __syncthreads();
-        // lanes of a warp that share a column group, then the warps, then the cluster
-#pragma unroll
-        for (int a = 0; a <= kDcSeqs; ++a)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-#pragma unroll
-                for (int o = CG; o < 32; o <<= 1) acc[a][j] += __shfl_xor_sync(0xffffffffu, acc[a][j], o);
-                if (lane < CG) dcs[(warp * (kDcSeqs + 1) + a) * D + cgi * 8 + j] = acc[a][j];
-            }
-        __syncthreads();
-        for (int i = tid; i < (kDcSeqs + 1) * D; i += 256) {
-            float s = 0.f;
-#pragma unroll
-            for (int v = 0; v < 8; ++v) s += dcs[v * (kDcSeqs + 1) * D + i];
-            part[i] = s;
         }
         cluster.sync();
-        if (rank < n) {
-            const int b = s_act[rank], m = (p.seq_len[b] - p.ks) / p.stride;
-            if (tid < D) {
+        // row a is finished by CTA a % 8
+        const int sub = tid / D, col = tid % D;
+        for (int a0 = rank; a0 < n; a0 += kDcSplit * PAR) {
+            const int a = a0 + kDcSplit * sub;
+            const int m = a < n ? (s_len[a] - p.ks) / p.stride : 0;
+            if (a < n) {
                 float y = 0.f, bias = 0.f;
 #pragma unroll
                 for (int r = 0; r < kDcSplit; ++r) {
                     const float* other = cluster.map_shared_rank(part, r);
-                    y += other[rank * D + tid];
-                    bias += other[kDcSeqs * D + tid];
+                    y += other[a * D + col];
+                    if (pe) bias += other[n * D + col];
                 }
                 y = round_et<ET>(y);
                 if (pe) y = round_et<ET>(y + round_et<ET>(bias));
-                s_y[tid] = y;
+                s_y[sub][col] = y;
             }
             __syncthreads();
-            if (tid < D && m < p.cmp_cap) {
-                float y = s_y[tid];
+            if (a < n && m < p.cmp_cap) {
+                float y = s_y[sub][col];
                 if (is_k && p.inv_freq) {
-                    const int i = tid % (D / 2);
+                    const int i = col % (D / 2);
                     const float ang = (float)(m * p.stride) * p.inv_freq[i];
                     const float c = round_et<ET>(cosf(ang)), s = round_et<ET>(sinf(ang));
-                    const float x1 = s_y[i], x2 = s_y[i + D / 2];
-                    y = tid < D / 2 ? x1 * c - x2 * s : x1 * s + x2 * c;
+                    const float x1 = s_y[sub][i], x2 = s_y[sub][i + D / 2];
+                    y = col < D / 2 ? x1 * c - x2 * s : x1 * s + x2 * c;
                 }
-                ((ET*)(is_k ? p.cmp_k : p.cmp_v))[((int64_t)(p.cmp_row0[b] + m) * p.Hk + h) * D + tid] = (ET)y;
+                ((ET*)(is_k ? p.cmp_k : p.cmp_v))[((int64_t)(p.cmp_row0[s_act[a]] + m) * p.Hk + h) * D + col] = (ET)y;
             }
+            __syncthreads();
         }
         next = s_next;
         cluster.sync();                                // the partial sums have been read
@@ -622,8 +640,8 @@ extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void*
 
 template <int D, typename ET>
 static cudaError_t launch_compress(const DecodeCompressParams& p, cudaStream_t stream) {
-    const int in = p.ks * D / kDcSplit * kDcPitch, sums = 8 * (kDcSeqs + 1) * D;
-    const int smem = (in > sums ? in : sums) * 4;
+    constexpr int smem = dc_smem<D>();
+    static_assert(kDcRows * D * 4 <= kDcRows * (kDcChunk + kDcPad) * 2 && smem <= 225 * 1024, "shared memory");
     auto kern = decode_compress_kernel<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;

@@ -112,3 +112,39 @@ def test_steps_in_a_row_match_steps_one_by_one(B, Hk, G, D, hidden):
 
     with torch.no_grad():
         assert all(torch.equal(a, b) for a, b in zip(run(False), run(True)))
+
+
+@pytest.mark.parametrize("B,D,ks,st,dtype", [(250, 64, 32, 16, torch.bfloat16), (3, 128, 64, 16, torch.float16), (17, 128, 40, 8, torch.bfloat16),
+                                             (5, 64, 24, 8, torch.bfloat16), (16, 128, 32, 16, torch.bfloat16), (79, 128, 16, 8, torch.bfloat16)])
+def test_compressor_turns_and_chunks(B, D, ks, st, dtype):
+    """The incremental compressor against the prefill one on the window that ends with the new token: around the rows of an MMA tile,
+    more sequences than a turn takes, reductions of one, two and one and a half chunks; rows of other sequences stay as they were."""
+    torch.manual_seed(B + ks)
+    Hk = 2
+    mod = FlashSparseAttentionDecodeKernel(2 * Hk * D, 2 * Hk, Hk, D, ks, st, 64, 8, 1, 2, 100).to(DEV).to(dtype)
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.normal_(0, 0.05)
+    lens = [ks - 1 + st * (b % 5) + (7 if b % 16 == 3 else 0) for b in range(B)]        # all but a few complete a window now
+    cache = mod.new_cache(B, 400, dtype=dtype, device=DEV)
+    for t in (cache.k, cache.v, cache.cmp_k, cache.cmp_v, cache.k_tail, cache.v_tail):
+        t.normal_()
+    cache.host_len = list(lens)
+    cache.seq_len.copy_(torch.tensor(lens, dtype=torch.int32))
+    before = cache.cmp_k.clone(), cache.cmp_v.clone()
+    with torch.no_grad():
+        mod.step(*(torch.randn(B, H, D, device=DEV).to(dtype) for H in (2 * Hk, Hk, Hk)), cache)
+    for got, old, tail, w, pe in ((cache.cmp_k, before[0], cache.k_tail, mod.compress_key, mod.intra_block_pe), (cache.cmp_v, before[1], cache.v_tail, mod.compress_value, None)):
+        want = old.clone()
+        ring = tail[:-1].view(B, ks, Hk, D)
+        for b, L in enumerate(lens):
+            if (L + 1 - ks) % st == 0:
+                x = torch.cat([ring[b, (L + 1) % ks :], ring[b, : (L + 1) % ks]]).double()
+                y = torch.einsum("khd,hkde->he", x, w.double().view(Hk, ks, D, D)).to(dtype)
+                if pe is not None:
+                    y = y + torch.einsum("hkd,hkde->he", pe.double(), w.double().view(Hk, ks, D, D)).to(dtype)
+                want[int(cache.cmp_row0[b]) + (L + 1 - ks) // st] = y
+        changed = (want != old).any(-1).any(-1)
+        assert torch.equal(got[~changed], old[~changed])
+        # fp32 sums of exact products: the result is one rounding (keys: two and their sum's) from the 64-bit one
+        assert float((got[changed].double() - want[changed].double()).norm() / want[changed].double().norm()) <= (6e-4 if dtype == torch.float16 else 4e-3)
