@@ -105,6 +105,26 @@ __global__ void __launch_bounds__(256) decode_proj_kernel(const DecodeProjParams
     }
 }
 
+// ------------------------------------------------------------------------------------------------ copies
+struct CopyParams {
+    const char* src[8];
+    char* dst[8];
+    int64_t bytes[8], first[9];          // first: 16-byte units before a buffer's own
+    int n;
+};
+__global__ void __launch_bounds__(256) copy_kernel(const CopyParams p) {
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < p.first[p.n]; i += (int64_t)gridDim.x * 256) {
+        int m = 0;
+        while (i >= p.first[m + 1]) ++m;
+        const int64_t at = (i - p.first[m]) * 16;
+        const char* s = p.src[m] + at;
+        char* d = p.dst[m] + at;
+        if ((((uintptr_t)s | (uintptr_t)d) & 15) == 0 && at + 16 <= p.bytes[m]) *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(s);
+        else
+            for (int64_t j = 0; j < 16 && at + j < p.bytes[m]; ++j) d[j] = s[j];
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ append
 // One CTA per sequence: rotates q and k of the new token at its position t = seq_len[b] (inv_freq null: they come rotated),
 // writes k, v to row t of the cache and the raw k, v to the compressor's ring, gate = sigmoid(z) with z given or computed
@@ -617,6 +637,23 @@ extern "C" int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k
     auto kern = dtype == FSA_DTYPE_BF16 ? (batch <= 8 ? decode_proj_kernel<1, __nv_bfloat16> : decode_proj_kernel<2, __nv_bfloat16>)
                                         : (batch <= 8 ? decode_proj_kernel<1, __half> : decode_proj_kernel<2, __half>);
     return launch_dependent(kern, dim3((unsigned)tiles), 256, 0, st, 1, p) == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
+extern "C" int fsa_copy(int num, const void* const* src, void* const* dst, const int64_t* bytes, void* stream) {
+    if (num < 0 || num > 8 || (num > 0 && (!src || !dst || !bytes))) return FSA_ERR_BAD_ARG;
+    CopyParams p = {};
+    p.n = num;
+    for (int i = 0; i < num; ++i) {
+        if (bytes[i] < 0 || (bytes[i] > 0 && (!src[i] || !dst[i]))) return FSA_ERR_BAD_ARG;
+        p.src[i] = (const char*)src[i]; p.dst[i] = (char*)dst[i]; p.bytes[i] = bytes[i];
+        p.first[i + 1] = p.first[i] + (bytes[i] + 15) / 16;
+    }
+    const int64_t units = p.first[num];
+    if (units == 0) return FSA_OK;
+    (void)cudaGetLastError();
+    const int64_t ctas = (units + 255) / 256;
+    copy_kernel<<<(unsigned)(ctas < 4096 ? ctas : 4096), 256, 0, (cudaStream_t)stream>>>(p);
+    return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
 }
 
 extern "C" int fsa_decode_append(const void* q_in, const void* k_in, const void* v_in, void* q_out, void* k_cache, void* v_cache, void* k_tail,

@@ -231,7 +231,31 @@ Outcome decode_layer_step(const Tensor& x_, const Tensor& wq, const Tensor& wk, 
     return std::make_tuple(y, ids);
 }
 
+// dst[i].copy_(src[i]) of a captured step's inputs in one launch; false, and nothing done, where that is more than a copy of bytes.
+static bool copy_inputs(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
+    const size_t n = dst.size();
+    if (n != src.size() || n == 0 || n > 8) return false;
+    const void* s[8];
+    void* d[8];
+    int64_t b[8];
+    for (size_t i = 0; i < n; ++i) {
+        if (!dst[i].is_cuda() || src[i].device() != dst[0].device() || dst[i].device() != dst[0].device() || src[i].scalar_type() != dst[i].scalar_type() ||
+            src[i].sizes() != dst[i].sizes() || !src[i].is_contiguous() || !dst[i].is_contiguous() || src[i].is_conj() || src[i].is_neg() ||
+            dst[i].is_conj() || dst[i].is_neg() || (dst[i].requires_grad() && at::GradMode::is_enabled()) || wants_grad({&src[i]}))
+            return false;
+        s[i] = src[i].data_ptr();
+        d[i] = dst[i].data_ptr();
+        b[i] = (int64_t)src[i].nbytes();
+        for (size_t j = 0; j < n; ++j)      // (a source in another's destination: one after the other)
+            if ((const char*)s[i] < (const char*)dst[j].data_ptr() + dst[j].nbytes() && (const char*)dst[j].data_ptr() < (const char*)s[i] + b[i]) return false;
+    }
+    c10::cuda::CUDAGuard guard(dst[0].device());
+    check(fsa_copy((int)n, s, d, b, stream_of(dst[0])), "fsa_copy");
+    return true;
+}
+
 void bind_decode(pybind11::module& m) {
+    m.def("copy_inputs", &copy_inputs);
     m.def("decode_mixed", &decode_mixed);
     m.def("decode_kernel_step", &decode_kernel_step);
     m.def("decode_layer_step", &decode_layer_step);

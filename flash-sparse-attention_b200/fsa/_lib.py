@@ -111,6 +111,7 @@ SIGNATURES = {
     "fsa_layer_prep": (c_int, [c_void_p, c_int, c_int64, c_void_p] + [c_int] * 4 + [c_void_p] * 4),
     "fsa_layer_rope_fwd": (
         c_int, [c_void_p, c_int64, c_void_p, c_int64] + [c_void_p] * 5 + [c_int, c_int64, c_int64] + [c_int] * 7 + [c_void_p] * 6),
+    "fsa_copy": (c_int, [c_int] + [c_void_p] * 4),
     "fsa_layer_every_block": (c_int, [c_void_p, c_int, c_int64] + [c_int] * 3 + [c_void_p] * 2),
     "fsa_layer_rope_bwd": (c_int, [c_void_p] * 14 + [c_int, c_int64, c_int64] + [c_int] * 5 + [c_void_p] * 4),
     "fsa_gate_proj_mix_bwd_delta": (

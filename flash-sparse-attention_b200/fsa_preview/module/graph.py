@@ -11,6 +11,7 @@ from typing import Callable, Sequence
 
 import torch
 
+from fsa._host import host
 from fsa_preview.cache import DecodeCache
 
 
@@ -41,8 +42,9 @@ class GraphedStep:
         cache.host_len = host0
 
     def __call__(self, *inputs: torch.Tensor) -> torch.Tensor:
-        for dst, src in zip(self.static_in, inputs):
-            dst.copy_(src, non_blocking=True)
+        if not host().copy_inputs(self.static_in[: len(inputs)], inputs):
+            for dst, src in zip(self.static_in, inputs):
+                dst.copy_(src, non_blocking=True)
         self.graph.replay()
         self.cache.host_len = [L + 1 for L in self.cache.host_len]
         return self.static_out

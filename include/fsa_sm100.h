@@ -398,6 +398,10 @@ int fsa_decode_step_sizes(int num_q_heads, int num_kv_heads, int head_dim, int k
 int fsa_decode_proj(const void* x, int64_t x_stride, int batch, int k_dim, int num, const void* const* w, const int* rows,
                     void* const* y, const int64_t* y_stride, int dtype, void* stream);
 
+/* Up to 8 copies between buffers of one device in one launch (the inputs of a captured step: a copy each takes longer to launch
+ * than to run).  Any alignment; the buffers of a call do not overlap. */
+int fsa_copy(int num, const void* const* src, void* const* dst, const int64_t* bytes, void* stream);
+
 /* Append one token per sequence: rotates q and k at position seq_len[b] (inv_freq null: they are rotated already and q is
  * not touched), writes k and v to row seq_row0[b] + seq_len[b] of the caches and the raw k, v to the compressor's rings,
  * gate[b, :] = sigmoid(gate_logits[b, :]) or sigmoid(gate_x[b, :] gate_w^T), then seq_len[b] += 1.  A token past `cap` goes

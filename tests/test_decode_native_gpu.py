@@ -148,3 +148,17 @@ def test_compressor_turns_and_chunks(B, D, ks, st, dtype):
         assert torch.equal(got[~changed], old[~changed])
         # fp32 sums of exact products: the result is one rounding (keys: two and their sum's) from the 64-bit one
         assert float((got[changed].double() - want[changed].double()).norm() / want[changed].double().norm()) <= (6e-4 if dtype == torch.float16 else 4e-3)
+
+
+def test_inputs_of_a_captured_step_are_copied_in_one_launch():
+    """fsa_copy at sizes and alignments that end within a 16-byte unit; what is more than a copy of bytes is left to copy_."""
+    from fsa._host import host
+
+    torch.manual_seed(3)
+    src = [torch.randn(s, device=DEV).to(torch.bfloat16) for s in ((3, 5), (1, 8, 128), (0, 4), (1,), (70000, 3))]
+    src.append(torch.randn(257, device=DEV).to(torch.bfloat16)[1:])
+    dst = [torch.zeros_like(t) for t in src]
+    assert host().copy_inputs(dst, src) and all(torch.equal(a, b) for a, b in zip(src, dst))
+    a, b = torch.zeros(4, 6, device=DEV), torch.randn(4, 6, device=DEV)
+    for d, s in ((a, b.double()), (a, b.t().contiguous().t()), (a, b[:1]), (a, b.cpu()), (a[:2], a[1:3])):
+        assert not host().copy_inputs([d], [s])
