@@ -5,10 +5,11 @@
 // (256 TMEM columns) leave 256 columns for S, dP and dQ together.  A tile is therefore a chain -- gather, S / dP, P / dS,
 // dK / dV / dQ -- that overlaps with its neighbours only where a resource is given back early:
 //   * dK first: it frees the Q stage, whose next rows are on their way while dV and dQ run; dV frees dO;
-//   * dQ takes the columns of S and dP (they have been read when dS is there); the drain empties them behind the gather of dO;
-//   * the drain stages dQ in the P / dS buffers (their readers are done), half a row at a time.
+//   * dQ takes the columns of S and dP (they have been read when dS is there).  The P / dS warps, which have nothing to do until
+//     the next S, read it into registers as one, so that S may follow at once, and stage it from there in the P / dS buffers (their
+//     readers are done).  Four drain warps that staged it half a row at a time held the columns for 4000 of a tile's 9300 cycles.
 // The unpipelined kernel walked the same chain with 128 threads and no overlap at all: 17.5 us a tile.
-// 16384 tokens, 4 KV heads, G = 2: 1967 -> 736 us (6.5 us a tile).
+// 16384 tokens, 4 KV heads, G = 2: 1967 -> 736 -> 704 us, with an even share of the tiles (sched_run) 598.
 // Blocks of more than 64 keys are walked in 64-key parts as in sel_bwd_pipe.cu.
 #include "sel_launch.cuh"
 
@@ -31,7 +32,7 @@ struct SelBwdWideParams {
 namespace bwdwide {
 constexpr int D = 256, KT = 64;
 constexpr int kThreads = 768, kLoaders = 256;
-constexpr int kWLoad = kLoaders / 32, kWMma1 = kWLoad, kWMma2 = kWLoad + 1, kWPrep = kWLoad + 2, kWKV = kWLoad + 3, kWDrain = kWLoad + 4,
+constexpr int kWLoad = kLoaders / 32, kWMma1 = kWLoad, kWMma2 = kWLoad + 1, kWPrep = kWLoad + 2, kWDrain = kWLoad + 4,
               kWGroups = kWLoad + 8;
 constexpr int kRegLoad = 40, kRegMma = 48, kRegDrain = 96, kRegGroup = 128;
 static_assert(8 * kRegLoad + 4 * kRegMma + 4 * kRegDrain + 8 * kRegGroup <= 24 * 80, "register budget");
@@ -77,15 +78,17 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
     uint64_t* kv_empty = bars + 5;       // every product of the segment is done
     uint64_t* sdp_full = bars + 6;
     uint64_t* pds_full = bars + 7;       // the 256 row threads have written P and dS
-    uint64_t* pds_free = bars + 8;       // the drain's stores have read their staging (the P / dS buffers)
+    uint64_t* pds_free = bars + 8;       // the stores of dQ have read their staging (the P / dS buffers)
     uint64_t* dq_full = bars + 9;        // every product of the tile is done
-    uint64_t* dq_empty = bars + 10;      // the drain has read dQ: its columns may take the next S and dP
+    uint64_t* dq_empty = bars + 10;      // dQ has been read: its columns may take the next S and dP
     uint64_t* acc_full = bars + 11;
     uint64_t* acc_empty = bars + 12;
     uint64_t* off_full = bars + 13;      // [ring]
     uint64_t* off_empty = bars + 15;     // [ring]
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 17);
-    int* s_nb = reinterpret_cast<int*>(bars + 18);     // [ring] 1: the tile starts a new segment (its own K/V block)
+    int4* s_rec = reinterpret_cast<int4*>(bars + 18);  // [8] prepared tiles: {bit 0: first tile of a segment (it loads its K/V block), bit 1: last
+                                                       // one, tile of partial dQ rows, tile, run}
+    static_assert(kRing * 2 * kTileRows * 4 + 18 * 8 + 8 * 16 <= kTail, "tail budget");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const SelShape& s = p.s;
@@ -98,8 +101,8 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         mbar_init(q_full, kLoaders); mbar_init(q_empty, 1);
         mbar_init(do_full, kLoaders); mbar_init(do_empty, 1);
         mbar_init(kv_full, 1); mbar_init(kv_empty, 1);
-        mbar_init(sdp_full, 1); mbar_init(pds_full, 256); mbar_init(pds_free, 4);
-        mbar_init(dq_full, 1); mbar_init(dq_empty, 128);
+        mbar_init(sdp_full, 1); mbar_init(pds_full, 256); mbar_init(pds_free, 8);
+        mbar_init(dq_full, 1); mbar_init(dq_empty, 256 + 4);
         mbar_init(acc_full, 1); mbar_init(acc_empty, 128);
         for (int i = 0; i < kRing; ++i) { mbar_init(&off_full[i], 1); mbar_init(&off_empty[i], kWLoad + 1); }
         mbar_init_fence();
@@ -115,103 +118,56 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
     const TileScheduleT<true> sched(p.ix.header[1], p.run, p.nsub);
     const int nloc = sched.nloc;
     const int key_lim = min(KT, s.BK);
+    bool ok = true;                          // no wait of this thread has run out
 
     if (warp < kWLoad) {
         // ------------------------------------------------------------------ gather warps: a warp copies whole 512-byte rows
         reg_dec<kRegLoad>();
-        bool ok = true;
         constexpr int NIT = kTileRows / kWLoad;                  // rows per warp
         const uint32_t slab_off = (uint32_t)(lane >> 3) * kSlab;
         auto copy = [&](const ET* base, uint8_t* dst, const int* off) {
             const ET* src = base + lane * 8;
             const uint32_t d = smem_u32(dst) + slab_off;
-#pragma unroll 8
-            for (int i = 0; i < NIT; ++i) {
-                const int r = warp + i * kWLoad;
-                const int o = off[r];
-                cp_async16(d + sw128_chunk_off(r, lane & 7), src + ((long long)(o < 0 ? 0 : o) << 3), o >= 0);
+#pragma unroll 1
+            for (int i0 = 0; i0 < NIT; i0 += 8) {                // (the offsets of eight rows are read ahead of their copies)
+                int o[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = off[warp + (i0 + i) * kWLoad];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    cp_async16(d + sw128_chunk_off(warp + (i0 + i) * kWLoad, lane & 7), src + ((int64_t)max(o[i], 0) << 3), o[i] >= 0);
             }
         };
         for (int k = 0; k < nloc && ok; ++k) {
             const int slot = k % kRing;
-            ok = mbar_wait(&off_full[slot], (k / kRing) & 1, status) && ok;
-            ok = mbar_wait(q_empty, (k & 1) ^ 1, status) && ok;
+            ok = mbar_poll(&off_full[slot], (k / kRing) & 1) && ok;
+            ok = mbar_poll(q_empty, (k & 1) ^ 1) && ok;
             copy(p.q, sQ, s_off[slot][0]);
             cp_async_mbar_arrive_noinc(q_full);
-            ok = mbar_wait(do_empty, (k & 1) ^ 1, status) && ok;
+            ok = mbar_poll(do_empty, (k & 1) ^ 1) && ok;
             copy(p.d_o, sDO, s_off[slot][1]);
             cp_async_mbar_arrive_noinc(do_full);
             __syncwarp();
             if (lane == 0) mbar_arrive(&off_empty[slot]);
         }
     } else if (warp >= kWDrain && warp < kWDrain + 4) {
-        // ------------------------------------------------------------------ drain: dQ per tile, dK / dV per segment
+        // ------------------------------------------------------------------ drain: dK / dV per segment
         reg_inc<kRegDrain>();
         const int quarter = warp & 3;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        uint8_t* my_stage = sP + quarter * (2 * 32 * 128);       // 32 rows x 128 columns: two slabs
-        bool ok = true;
         int nflush = 0;
-        int hg0 = -1, hg1 = -1, hg2 = -1;
-        if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
-        if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
-        int seg_first = 0;
+#pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            const int prev_hg = hg0;
-            hg0 = hg1; hg1 = hg2;
-            if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
-            if (hg0 != prev_hg || (k % sched.run) == 0) seg_first = k;
-            const bool last_of_seg = (k + 1 >= nloc) || (hg1 != hg0) || ((k + 1) % sched.run) == 0;
-            const int row = (sched.tile(k) * p.nsub + sched.sub(k)) * kTileRows + quarter * 32;
-            ok = mbar_wait(dq_full, k & 1, status) && ok;
-            tc_fence_after();
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (half == 1) {
-                    if (lane == 0) bulk_wait_read0();            // the first half's store has read the staging rows
-                    __syncwarp();
-                }
-#pragma unroll
-                for (int c0 = 0; c0 < 128; c0 += 32) {
-                    uint32_t v[32];
-                    tmem_ld32(tbase + lane_off + cDQ + half * 128 + c0, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        uint4 u;
-                        u.x = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-                        u.y = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-                        u.z = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-                        u.w = ElemTraits<ET>::pack2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-                        const int chunk = (c0 >> 3) + q4;
-                        *reinterpret_cast<uint4*>(my_stage + (chunk >> 3) * (32 * 128) + sw128_chunk_off(lane, chunk & 7)) = u;
-                    }
-                }
-                if (half == 1) {
-                    tc_fence_before();
-                    mbar_arrive(dq_empty);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) tma_store_2d(&dqmap, half * 128 + b * 64, row, smem_u32(my_stage + b * (32 * 128)));
-                    bulk_commit();
-                }
-            }
-            if (lane == 0) {
-                bulk_wait_read0();
-                mbar_arrive(pds_free);
-            }
+            ok = mbar_poll(dq_full, k & 1) && ok;
+            const int4 rec = s_rec[k & 7];
             __syncwarp();
-            if (!last_of_seg) continue;
-            const int j0 = sched.tile(seg_first);
-            const TileInfo ti = load_tile(p.ix, j0);
-            const int seg = ti.seg0 + j0 / sched.run - __ldg(p.ix.tile_aux + j0).x / sched.run;
-            float* slab = p.slabs + ((int64_t)seg * p.nsub + sched.sub(k)) * (2 * KT * D) + quarter * 32 + lane;
-            ok = mbar_wait(acc_full, nflush & 1, status) && ok;
+            if (lane == 0) mbar_arrive(dq_empty);                // (no tile gets two ahead of this warp)
+            if (!(rec.x & 2)) continue;
+            const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
+            float* slab = p.slabs + ((int64_t)seg * p.nsub + (rec.y - rec.z * p.nsub)) * (2 * KT * D) + quarter * 32 + lane;
+            ok = mbar_poll(acc_full, nflush & 1) && ok;
             tc_fence_after();
-#pragma unroll
+#pragma unroll 1
             for (int part = 0; part < 4; ++part) {               // dK low, dK high, dV low, dV high half of the head dimension
                 uint32_t v[KT];
 #pragma unroll
@@ -228,7 +184,6 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 for (int key = 0; key < KT; ++key) dst[key * D] = __uint_as_float(v[key]);
             }
         }
-        if (lane == 0) bulk_wait0();
     } else if (warp < kWDrain) {
         reg_dec<kRegMma>();
         if (warp == kWMma1) {
@@ -240,33 +195,32 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16), do_lo = umma_desc_lo(smem_u32(sDO), 16);
             const uint32_t k_lo = umma_desc_lo(smem_u32(sK), 16), v_lo = umma_desc_lo(smem_u32(sV), 16);
             int kvn = -1;
-            bool ok = true;
             for (int k = 0; k < nloc && ok; ++k) {
                 const int slot = k % kRing;
-                ok = mbar_wait(&off_full[slot], (k / kRing) & 1, status) && ok;
-                const int new_block = s_nb[slot];
+                ok = mbar_poll(&off_full[slot], (k / kRing) & 1) && ok;
+                const int seg = s_rec[k & 7].x;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
-                if (new_block != 0) {
+                if (seg & 1) {
                     ++kvn;
-                    ok = mbar_wait(kv_full, kvn & 1, status) && ok;
+                    ok = mbar_poll(kv_full, kvn & 1) && ok;
                 }
-                ok = mbar_wait(dq_empty, (k & 1) ^ 1, status) && ok;
-                ok = mbar_wait(q_full, k & 1, status) && ok;
+                ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
+                ok = mbar_poll(q_full, k & 1) && ok;
                 fence_async_smem();
                 tc_fence_after();
                 if (leader) {
-#pragma unroll
+#pragma unroll 4
                     for (int ks = 0; ks < D / 16; ++ks)
                         umma_ss(tbase + cS, umma_desc_pack(q_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
                                 umma_desc_pack(k_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc, ks > 0);
                 }
                 __syncwarp();
-                ok = mbar_wait(do_full, k & 1, status) && ok;
+                ok = mbar_poll(do_full, k & 1) && ok;
                 fence_async_smem();
                 tc_fence_after();
                 if (leader) {
-#pragma unroll
+#pragma unroll 4
                     for (int ks = 0; ks < D / 16; ++ks)
                         umma_ss(tbase + cDP, umma_desc_pack(do_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
                                 umma_desc_pack(v_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc, ks > 0);
@@ -285,34 +239,29 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             const uint32_t k_mn_lo = umma_desc_lo(smem_u32(sK), KT * 128);
             const uint32_t q_mn_lo = umma_desc_lo(smem_u32(sQ), kSlab), do_mn_lo = umma_desc_lo(smem_u32(sDO), kSlab);
             int blk = -1;
-            bool ok = true;
-            int hg0 = -1, hg1 = -1, hg2 = -1;
-            if (nloc > 0) hg1 = load_tile(p.ix, sched.tile(0)).hg;
-            if (nloc > 1) hg2 = load_tile(p.ix, sched.tile(1)).hg;
+#pragma unroll 1
             for (int k = 0; k < nloc && ok; ++k) {
-                const int prev_hg = hg0;
-                hg0 = hg1; hg1 = hg2;
-                if (k + 2 < nloc) hg2 = load_tile(p.ix, sched.tile(k + 2)).hg;
-                const bool first = hg0 != prev_hg || (k % sched.run) == 0;
-                const bool last = (k + 1 >= nloc) || (hg1 != hg0) || ((k + 1) % sched.run) == 0;
+                // (the record is complete: its tile has been through the S / dP issuer when P is there)
+                ok = mbar_poll(pds_full, k & 1) && ok;
+                const int seg = s_rec[k & 7].x;
+                const bool first = seg & 1, last = seg & 2;
                 if (first) ++blk;
-                ok = mbar_wait(pds_full, k & 1, status) && ok;
                 // (complete already: acquire only)
-                ok = mbar_wait(kv_full, blk & 1, status) && ok;
-                ok = mbar_wait(q_full, k & 1, status) && ok;
-                ok = mbar_wait(do_full, k & 1, status) && ok;
-                if (first && blk > 0) ok = mbar_wait(acc_empty, (blk - 1) & 1, status) && ok;
+                ok = mbar_poll(kv_full, blk & 1) && ok;
+                ok = mbar_poll(q_full, k & 1) && ok;
+                ok = mbar_poll(do_full, k & 1) && ok;
+                if (first && blk > 0) ok = mbar_poll(acc_empty, (blk - 1) & 1) && ok;
                 fence_async_smem();
                 tc_fence_after();
                 if (leader) {
-#pragma unroll
+#pragma unroll 2
                     for (int ks = 0; ks < kTileRows / 16; ++ks)
 #pragma unroll
                         for (int half = 0; half < 2; ++half)
                             umma_ss(tbase + cDK + half * KT, umma_desc_pack(q_mn_lo + half * ((2 * kSlab) >> 4) + ks * (2048 >> 4), hi_1024),
                                     umma_desc_pack(ds_mn_lo + ks * (2048 >> 4), hi_1024), idesc_dk, (!first || ks > 0) ? 1u : 0u);
                     umma_commit(q_empty);
-#pragma unroll
+#pragma unroll 2
                     for (int ks = 0; ks < kTileRows / 16; ++ks)
 #pragma unroll
                         for (int half = 0; half < 2; ++half)
@@ -331,7 +280,6 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             }
         } else if (warp == kWPrep) {
             // -------------------------------------------------------------- tile preparation: row offsets, two tiles ahead of the copies
-            bool ok = true;
             int gg[4], ee[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -341,37 +289,58 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             }
             const int qsn8 = (int)(p.q_sn >> 3), dsn8 = (int)(p.do_sn >> 3), qsh8 = (int)(p.q_sh >> 3), dsh8 = (int)(p.do_sh >> 3);
             int prev_hg = -1;
-            for (int k = 0; k < nloc && ok; ++k) {
-                const int slot = k % kRing, j = sched.tile(k);
-                const TileInfo ti = load_tile(p.ix, j);
-                uint32_t e[4];
+            // (two tiles in turn: handing the registers on would wait for the loads)
+            struct Pre { int h, hg; uint32_t e[4]; };
+            TileCursorT<true> ahead(sched), cur(sched);
+            auto fetch = [&](Pre& m) {
+                const TileInfo ti = load_tile(p.ix, ahead.j);
+                m.h = ti.h; m.hg = ti.hg;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) e[i] = gg[i] < s.G ? __ldg(p.ix.entries + (int64_t)j * s.TPT + ee[i]) : 0xFFFFFFFFu;
-                ok = mbar_wait(&off_empty[slot], ((k / kRing) & 1) ^ 1, status) && ok;
+                for (int i = 0; i < 4; ++i) m.e[i] = gg[i] < s.G ? __ldg(p.ix.entries + (int64_t)ahead.j * s.TPT + ee[i]) : 0xFFFFFFFFu;
+                ahead.next(sched);
+            };
+            auto publish = [&](int k, Pre& m, const Pre& next) {
+                const int slot = k % kRing;
+                ok = mbar_poll(&off_empty[slot], ((k / kRing) & 1) ^ 1) && ok;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int tok = (int)(e[i] >> kSlotBits), hq = ti.h * s.G + gg[i];
-                    s_off[slot][0][lane + 32 * i] = e[i] != 0xFFFFFFFFu ? tok * qsn8 + hq * qsh8 : -1;
-                    s_off[slot][1][lane + 32 * i] = e[i] != 0xFFFFFFFFu ? tok * dsn8 + hq * dsh8 : -1;
+                    const int tok = (int)(m.e[i] >> kSlotBits), hq = m.h * s.G + gg[i];
+                    s_off[slot][0][lane + 32 * i] = m.e[i] != 0xFFFFFFFFu ? tok * qsn8 + hq * qsh8 : -1;
+                    s_off[slot][1][lane + 32 * i] = m.e[i] != 0xFFFFFFFFu ? tok * dsn8 + hq * dsh8 : -1;
                 }
-                if (lane == 0) s_nb[slot] = (ti.hg != prev_hg || (k % sched.run) == 0) ? 1 : 0;
-                prev_hg = ti.hg;
+                if (lane == 0)
+                    s_rec[k & 7] = make_int4((m.hg != prev_hg || cur.r == 0 ? 1 : 0) | (k + 1 >= nloc || next.hg != m.hg || cur.r + 1 == sched.run ? 2 : 0),
+                                             cur.j * p.nsub + cur.sub(sched), cur.j, cur.run(sched));
+                cur.next(sched);
+                prev_hg = m.hg;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&off_full[slot]);
+                if (k + 2 < nloc) fetch(m);
+            };
+            Pre m1{0, -1, {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}}, m2 = m1;
+            if (nloc > 0) fetch(m1);
+            if (nloc > 1) fetch(m2);
+#pragma unroll 1
+            for (int k = 0; k < nloc && ok; k += 2) {
+                publish(k, m1, m2);
+                if (k + 1 < nloc) publish(k + 1, m2, m1);
             }
         } else {
             // -------------------------------------------------------------- K/V blocks by TMA
-            bool ok = true;
             int kvn = -1, prev_hg = -1;
+            TileCursorT<true> cur(sched);
+#pragma unroll 1
             for (int k = 0; k < nloc && ok; ++k) {
-                const TileInfo ti = load_tile(p.ix, sched.tile(k));
-                if (ti.hg == prev_hg && (k % sched.run) != 0) continue;
+                const TileInfo ti = load_tile(p.ix, cur.j);
+                const int row = ti.row0 + cur.sub(sched) * KT;
+                const bool first = ti.hg != prev_hg || cur.r == 0;
+                cur.next(sched);
+                if (!first) continue;
                 prev_hg = ti.hg;
                 ++kvn;
                 if (lane == 0) {
-                    ok = mbar_wait(kv_empty, (kvn & 1) ^ 1, status) && ok;
+                    ok = mbar_poll(kv_empty, (kvn & 1) ^ 1) && ok;
                     mbar_expect_tx(kv_full, (uint32_t)(2 * kK));
-                    const int row = ti.row0 + sched.sub(k) * KT;
 #pragma unroll
                     for (int b = 0; b < D / 64; ++b) {
                         tma_load_2d(smem_u32(sK + b * KT * 128), &kmap, ti.h * D + b * 64, row, kv_full);
@@ -392,30 +361,38 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         const bool row_exists = g < s.G;
         constexpr int HC = KT / 2;
         const int cb = sb * HC;
-        bool ok = true;
         uint32_t ent = 0xFFFFFFFFu;
         int row0 = 0, h = 0;
-        auto fetch_ent = [&](int k) {
-            const int j = sched.tile(k);
-            const TileInfo ti = load_tile(p.ix, j);
-            row0 = ti.row0 + sched.sub(k) * KT;
+        TileCursorT<true> ahead(sched);
+        auto fetch_ent = [&]() {
+            const TileInfo ti = load_tile(p.ix, ahead.j);
+            row0 = ti.row0 + ahead.sub(sched) * KT;
             h = ti.h;
-            ent = row_exists ? __ldg(p.ix.entries + (int64_t)j * s.TPT + e) : 0xFFFFFFFFu;
+            ent = row_exists ? __ldg(p.ix.entries + (int64_t)ahead.j * s.TPT + e) : 0xFFFFFFFFu;
+            ahead.next(sched);
         };
-        if (nloc > 0) fetch_ent(0);
-        for (int k = 0; k < nloc && ok; ++k) {
-            // padding rows: zero Q and dO rows, any finite P will do
-            float lse_r = 0.f, delta_s = 0.f;
-            int c_lo = 0, c_hi = key_lim;
+        if (nloc > 0) fetch_ent();
+        // lse, delta and visible columns of the next tile's row (padding rows: zero Q and dO rows, any finite P will do)
+        float lse_n = 0.f, delta_n = 0.f;
+        int lo_n = 0, hi_n = key_lim;
+        auto fetch_stats = [&]() {
+            lse_n = 0.f; delta_n = 0.f; lo_n = 0; hi_n = key_lim;
             if (ent != 0xFFFFFFFFu) {
                 const int tok = (int)(ent >> kSlotBits);
                 const int64_t idx = (int64_t)(h * s.G + g) * s.N + tok;
-                lse_r = __ldg(p.lse + idx);
-                delta_s = __ldg(p.delta + idx) * p.scale;
-                visible_cols(p.bd, tok, row0, key_lim, c_lo, c_hi);
+                lse_n = __ldg(p.lse + idx);
+                delta_n = __ldg(p.delta + idx);
+                visible_cols(p.bd, tok, row0, key_lim, lo_n, hi_n);
             }
-            if (k + 1 < nloc) fetch_ent(k + 1);
-            ok = mbar_wait(sdp_full, k & 1, status) && ok;
+        };
+        if (nloc > 0) fetch_stats();
+        uint8_t* my_stage = sP + (sb * 4 + quarter) * (32 * 128);        // 32 rows x 64 columns
+#pragma unroll 1
+        for (int k = 0; k < nloc && ok; ++k) {
+            const float lse_r = lse_n, delta_s = delta_n * p.scale;
+            const int c_lo = lo_n, c_hi = hi_n;
+            if (k + 1 < nloc) fetch_ent();
+            ok = mbar_poll(sdp_full, k & 1) && ok;
             tc_fence_after();
             uint32_t pp[HC / 2], dd[HC / 2];
             {
@@ -424,15 +401,24 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 tmem_ld32(tbase + lane_off + cDP + cb, dv);
                 tmem_ld_wait();
 #pragma unroll
+                for (int i = 0; i < 32; ++i) sv[i] = __float_as_uint(ex2_approx_w(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r)));
+                if (!__all_sync(0xffffffffu, c_lo <= cb && c_hi >= cb + HC)) {
+                    // (bit i: column cb + i is visible)
+                    const int lo = min(max(c_lo - cb, 0), 32), hi = min(max(c_hi - cb, 0), 32);
+                    const uint32_t vis = (uint32_t)((1ull << hi) - 1) & ~(uint32_t)((1ull << lo) - 1);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (!(vis >> i & 1u)) sv[i] = 0u;
+                }
+#pragma unroll
                 for (int i = 0; i < 32; i += 2) {
-                    const float p0 = (cb + i >= c_lo && cb + i < c_hi) ? ex2_approx_w(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r)) : 0.f;
-                    const float p1 = (cb + i + 1 >= c_lo && cb + i + 1 < c_hi) ? ex2_approx_w(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse_r)) : 0.f;
+                    const float p0 = __uint_as_float(sv[i]), p1 = __uint_as_float(sv[i + 1]);
                     pp[i >> 1] = ElemTraits<ET>::pack2(p0, p1);
                     dd[i >> 1] = ElemTraits<ET>::pack2(p0 * fmaf(__uint_as_float(dv[i]), p.scale, -delta_s), p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s));
                 }
             }
             tc_fence_before();
-            if (k > 0) ok = mbar_wait(pds_free, (k - 1) & 1, status) && ok;
+            if (k > 0) ok = mbar_poll(pds_free, (k - 1) & 1) && ok;
 #pragma unroll
             for (int c4 = 0; c4 < HC / 8; ++c4) {
                 const uint32_t off = sw128_chunk_off(r, sb * (HC / 8) + c4);
@@ -441,8 +427,43 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             }
             fence_async_smem();
             mbar_arrive(pds_full);
+            if (k + 1 < nloc) fetch_stats();
+            // ---- dQ of the tile: this group's 128 columns to registers, which frees its TMEM columns for the next S and dP, and from
+            // there 64 at a time through the P / dS buffers, which the products have read
+            ok = mbar_poll(dq_full, k & 1) && ok;
+            tc_fence_after();
+            const int row = s_rec[k & 7].y * kTileRows + quarter * 32;
+            uint32_t x[64];
+#pragma unroll
+            for (int c0 = 0; c0 < 128; c0 += 32) {
+                uint32_t v[32];
+                tmem_ld32(tbase + lane_off + cDQ + sb * 128 + c0, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[c0 / 2 + i] = ElemTraits<ET>::pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+            }
+            tc_fence_before();
+            mbar_arrive(dq_empty);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4*>(my_stage + sw128_chunk_off(lane, c)) =
+                        make_uint4(x[half * 32 + c * 4], x[half * 32 + c * 4 + 1], x[half * 32 + c * 4 + 2], x[half * 32 + c * 4 + 3]);
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&dqmap, sb * 128 + half * 64, row, smem_u32(my_stage));
+                    bulk_commit();
+                    bulk_wait_read0();
+                    if (half == 1) mbar_arrive(pds_free);
+                }
+                __syncwarp();
+            }
         }
+        if (lane == 0) bulk_wait0();
     }
+    if (!ok) atomicMax(status, (int)kStatusWaitTimeout);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, bwdwide::kCols);
