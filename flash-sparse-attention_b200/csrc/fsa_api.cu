@@ -195,17 +195,34 @@ static int env_int(const char* name, int dflt) {
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// Tiles per scheduling run of the persistent kernels: `most` when there are plenty of tiles, fewer when runs of that length
-// would leave SMs without work or with a last run of their own to wait for -- a run is a serial chain on one SM (a backward
-// tile takes about 2.7 us, so the 128 tiles of a 512-token problem took 86 us in four runs of 32 and take 12 in 128 runs of
-// one).  Four runs per SM keep the imbalance of the last round small; a shorter run costs the backward one more dK / dV slab
-// (64 KB written and read), which is why long lists keep long runs.  A function of the shape alone: forward and backward
-// must cut the same list alike.
-static int sched_run(const SelShape& s, int most) {
-    // (a backward run is walked once per 64-key part of its blocks)
-    const int64_t tiles = ((int64_t)s.Hk * s.N * s.T + s.TPT - 1) / s.TPT * (s.BK > 64 ? s.BK / 64 : 1);
-    const int64_t run = tiles / (4 * sm_count());
-    return (int)(run < 1 ? 1 : run > most ? most : run);
+// Tiles per scheduling run of the persistent kernels: about `want` when there are plenty of tiles, fewer when runs of that length
+// would leave SMs without work -- a run is a serial chain on one SM (a backward tile takes about 2.3 us, so the 128 tiles of a
+// 512-token problem took 86 us in four runs of 32 and take 12 in 128 runs of one).  Whole runs are dealt, so that the longest
+// share is ceil(runs / SMs) runs: the length is the one for which that comes nearest to an even share.  (Four runs an SM whatever
+// came of it before: 16384 tokens at head size 256, 4 KV heads had five runs of 27 tiles on some SMs where three of 38 do, backward 704 ->
+// 598 us; 21K ragged tokens with 128-key blocks 206 -> 188; 7192 tokens in four sequences four of 24 where three of 25 do.)  The number of tiles is known
+// on the device only, so it is estimated, from sequences of one length that select all they can, and the share looked at 2 %
+// to both sides.  A run costs as much as `own` tiles besides its own: the backward one more dK / dV slab (64 KB written and read,
+// 1.3 tiles), the forward a load of K and V; runs above `want` spread the CTAs over more query rows than L2 likes.  A function of the
+// shape alone: forward and backward must cut the same list alike.
+static int sched_run(const SelShape& s, int want, int parts, double own) {
+    if (s.N <= 0 || s.B <= 0) return 1;
+    const double L = (double)s.N / s.B, nb = L <= s.BK ? 1. : L / s.BK;
+    const double entries = nb <= s.T ? L * (nb + 1) / 2 : L * s.T - 0.5 * s.BK * s.T * (s.T - 1.);      // of a sequence and kv head
+    const double per_head = entries / s.TPT + 0.5 * nb, tiles = (double)s.Hk * s.B * (per_head > nb ? per_head : nb);
+    const int sms = sm_count();
+    int best = 1;
+    double least = 0;
+    for (int run = 1; run <= want + want / 2; ++run) {
+        double cost = 0;
+        for (int i = -1; i <= 1; ++i) {
+            const int64_t t = (int64_t)(tiles * (1 + 0.02 * i)) + 1, runs = (t + run - 1) / run * parts;
+            cost += (double)((runs + sms - 1) / sms * run);
+        }
+        cost *= 1 + own / run + (run > want ? 0.1 * (run - want) / want : 0);
+        if (run == 1 || cost <= least) { best = run; least = cost; }
+    }
+    return best;
 }
 
 static int make_shape(int64_t N, int B, int Hq, int Hk, int D, int T, int BK, SelShape* s, int64_t Nk = -1) {
@@ -228,7 +245,7 @@ static int make_shape(int64_t N, int B, int Hq, int Hk, int D, int T, int BK, Se
     if (s->NC < 1) s->NC = 1;
     // tiles per scheduling run of the backward (FSA_SEL_RUN overrides; read once): see sched_run
     static const int env_run = env_int("FSA_SEL_RUN", 0);
-    s->RB = env_run > 0 ? env_run : sched_run(*s, 32);
+    s->RB = env_run > 0 ? env_run : sched_run(*s, 32, BK > 64 ? BK / 64 : 1, 1.3);
     if ((int64_t)s->Hk * s->NBmax >= ((int64_t)1 << 30)) return FSA_ERR_UNSUPPORTED;
     if ((int64_t)s->Hk * s->NBmax * s->NC >= ((int64_t)1 << 31)) return FSA_ERR_UNSUPPORTED;
     if (Hk > 65535) return FSA_ERR_UNSUPPORTED;
@@ -369,7 +386,7 @@ static int sel_fwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
     SelFwdArgs a;
     a.q = q; a.q_sn = q_sn; a.q_sh = q_sh; a.sm_scale = sm_scale;
     static const int env_run = env_int("FSA_SEL_RUN", 0);
-    a.run = env_run > 0 ? env_run : sched_run(s, 8);
+    a.run = env_run > 0 ? env_run : sched_run(s, 8, 1, 0.3);
     a.opart = scratch;
     a.ml = (float2*)((char*)scratch + align_up(prow * D * 2, 1024));
     a.o = o; a.o_sn = o_sn; a.o_sh = o_sh; a.lse = lse;
