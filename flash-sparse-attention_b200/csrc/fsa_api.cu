@@ -210,17 +210,15 @@ static int sched_run(const SelShape& s, int want, int parts, double own) {
     const double L = (double)s.N / s.B, nb = L <= s.BK ? 1. : L / s.BK;
     const double entries = nb <= s.T ? L * (nb + 1) / 2 : L * s.T - 0.5 * s.BK * s.T * (s.T - 1.);      // of a sequence and kv head
     const double per_head = entries / s.TPT + 0.5 * nb, tiles = (double)s.Hk * s.B * (per_head > nb ? per_head : nb);
-    const int sms = sm_count();
+    const uint32_t sms = (uint32_t)sm_count();
+    if (tiles * parts <= sms) return 1;
     int best = 1;
     double least = 0;
-    for (int run = 1; run <= want + want / 2; ++run) {
-        double cost = 0;
-        for (int i = -1; i <= 1; ++i) {
-            const int64_t t = (int64_t)(tiles * (1 + 0.02 * i)) + 1, runs = (t + run - 1) / run * parts;
-            cost += (double)((runs + sms - 1) / sms * run);
-        }
-        cost *= 1 + own / run + (run > want ? 0.1 * (run - want) / want : 0);
-        if (run == 1 || cost <= least) { best = run; least = cost; }
+    for (uint32_t run = tiles * parts > 3. * want * sms ? 2 * want / 3 : 1; run <= (uint32_t)(want + want / 2); ++run) {
+        uint32_t cost = 0;
+        for (int i = -1; i <= 1; ++i) cost += (((uint32_t)(tiles * (1 + 0.02 * i)) + run) / run * parts + sms - 1) / sms * run;
+        const double c = cost * (1 + own / run + ((int)run > want ? 0.1 * ((int)run - want) / want : 0));
+        if (least == 0 || c <= least) { best = (int)run; least = c; }
     }
     return best;
 }
