@@ -385,8 +385,7 @@ __global__ void __launch_bounds__(256) sel_bwd_delta(const ET* __restrict__ o, i
 // dq[n, hq, :] = sum over usable slots (and sub-tiles) of the partial rows, looked up through
 // the `pos` map; one warp per (n, hq)
 template <int D, typename ET>
-__global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ dq_part, const int* __restrict__ pos, SelShape s,
-                                                         int nsub, ET* __restrict__ dq) {
+__device__ __forceinline__ void dq_reduce_rows(const ET* __restrict__ dq_part, const int* __restrict__ pos, const SelShape& s, int nsub, ET* __restrict__ dq) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= s.N * s.Hq) return;
@@ -446,14 +445,15 @@ __global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ 
 // segments, rounded to the output dtype (replaces the `.sum(0)` over the group's copies of the reference,
 // fsa/ops/FSA_topk_sparse_attention.py:1854-1855).  The rows of a block that nobody selected (no segment) and those past
 // the last sequence (the last CTA) are written as zeros here: no pass over dk and dv before (26 us of 64K tokens x 4 heads).
+// hg: block of a kv head; share: part of its 64-key slabs (dkdv_shares of each)
+__host__ __device__ constexpr int dkdv_shares(int D) { return 2 * 64 * (D / 4) / 1024; }      // CTAs per slab: 1024 float4 each, four per thread in flight
 template <int D, typename ET>
-__global__ void __launch_bounds__(256, 4) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s,
-                                                           SelIndex ix, int nsub, ET* __restrict__ dk, ET* __restrict__ dv) {
+__device__ __forceinline__ void dkdv_reduce_block(const float* __restrict__ slabs, const int* __restrict__ ck, const SelShape& s, const SelIndex& ix,
+                                                  int nsub, ET* __restrict__ dk, ET* __restrict__ dv, int hg, int share) {
     constexpr int KT = 64, RV = D / 4;                // keys of a slab, float4 per row
-    constexpr int kShares = 2 * KT * RV / 1024;       // CTAs per slab: 1024 float4 each, four per thread in flight
-    const int hg = blockIdx.x;
+    constexpr int kShares = dkdv_shares(D);
     if (hg == s.Hk * s.NBmax) {
-        if (blockIdx.y > 0) return;
+        if (share > 0) return;
         const int64_t first = (int64_t)__ldg(ck + s.B) * s.Hk * (D / 8), last = s.Nk * s.Hk * (D / 8);
         for (int64_t i = first + threadIdx.x; i < last; i += blockDim.x) {
             reinterpret_cast<uint4*>(dk)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -461,13 +461,13 @@ __global__ void __launch_bounds__(256, 4) sel_bwd_dkdv_reduce(const float* __res
         }
         return;
     }
-    const int h = hg / s.NBmax, gb = hg - h * s.NBmax, sub = blockIdx.y / kShares;
+    const int h = hg / s.NBmax, gb = hg - h * s.NBmax, sub = share / kShares;
     const int2 rn = block_rows(ck, s.B, s.BK, gb);
     // rows past the end of the sequence belong to the next sequence's block
     const int row0 = rn.x + sub * KT, nkeys = min(KT, rn.y - sub * KT);
     if (nkeys <= 0) return;
     const int seg0 = ix.key_seg[hg], nseg = ix.key_seg[hg + 1] - seg0;
-    const int i0 = (blockIdx.y % kShares) * 1024 + threadIdx.x;
+    const int i0 = (share % kShares) * 1024 + threadIdx.x;
     const float4* base = reinterpret_cast<const float4*>(slabs) + ((int64_t)seg0 * nsub + sub) * (2 * KT * RV);
     const int64_t seg_stride = (int64_t)nsub * (2 * KT * RV);
     float4 acc[4];
@@ -513,6 +513,28 @@ __global__ void __launch_bounds__(256, 4) sel_bwd_dkdv_reduce(const float* __res
     }
 }
 
+template <int D, typename ET>
+__global__ void __launch_bounds__(256) sel_bwd_dq_reduce(const ET* __restrict__ dq_part, const int* __restrict__ pos, SelShape s, int nsub, ET* __restrict__ dq) {
+    dq_reduce_rows<D, ET>(dq_part, pos, s, nsub, dq);
+}
+template <int D, typename ET>
+__global__ void __launch_bounds__(256, 4) sel_bwd_dkdv_reduce(const float* __restrict__ slabs, const int* __restrict__ ck, SelShape s, SelIndex ix, int nsub,
+                                                              ET* __restrict__ dk, ET* __restrict__ dv) {
+    dkdv_reduce_block<D, ET>(slabs, ck, s, ix, nsub, dk, dv, blockIdx.x, blockIdx.y);
+}
+// Both in one launch, for problems so small that a launch is as long as either (512 tokens, 4 heads: 3.1 + 4.1 us): the first `ndq` CTAs take dq.
+template <int D, typename ET>
+__global__ void __launch_bounds__(256) sel_bwd_reduce_few(const ET* __restrict__ dq_part, const float* __restrict__ slabs, const int* __restrict__ ck,
+                                                          SelShape s, SelIndex ix, int nsub, ET* __restrict__ dq, ET* __restrict__ dk,
+                                                          ET* __restrict__ dv, int ndq) {
+    if ((int)blockIdx.x < ndq) {
+        dq_reduce_rows<D, ET>(dq_part, ix.pos, s, nsub, dq);
+    } else {
+        const int i = (int)blockIdx.x - ndq, blocks = s.Hk * s.NBmax + 1;
+        dkdv_reduce_block<D, ET>(slabs, ck, s, ix, nsub, dk, dv, i % blocks, i / blocks);
+    }
+}
+
 // fp32 accumulators -> output dtype
 template <typename ET>
 __global__ void __launch_bounds__(256) sel_bwd_convert(const float* __restrict__ a, const float* __restrict__ b,
@@ -527,6 +549,8 @@ __global__ void __launch_bounds__(256) sel_bwd_convert(const float* __restrict__
     reinterpret_cast<uint2*>(oa)[i] = u;
     reinterpret_cast<uint2*>(ob)[i] = w;
 }
+
+constexpr int64_t kReduceFew = 24000;      // output rows up to which both reductions go in one launch (more: resident merges take dq)
 
 template <int D, typename ET>
 static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const SelIndex& ix, const CUtensorMap& kmap,
@@ -585,6 +609,18 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
+    const unsigned kv_blocks = (unsigned)(s.Hk * s.NBmax + 1), kv_shares = (unsigned)(nsub * dkdv_shares(D));
+    const int* kv_starts = a.bd.cu_k ? a.bd.cu_k : a.cu;
+    if (pipelined && rows > 0 && rows < kReduceFew && kv_elems > 0) {
+        const unsigned ndq = (unsigned)((rows + 7) / 8);
+        e = prefer_l1((const void*)sel_bwd_reduce_few<D, ET>);
+        if (e != cudaSuccess) return e;
+        prof_begin(3, stream);
+        sel_bwd_reduce_few<D, ET><<<ndq + kv_blocks * kv_shares, 256, 0, stream>>>((const ET*)a.dq_part, a.slabs, kv_starts, s, ix, nsub, (ET*)a.dq,
+                                                                                   (ET*)a.dk, (ET*)a.dv, (int)ndq);
+        prof_end(3, stream);
+        return cudaGetLastError();
+    }
     if (rows > 0 && sel_merge_fits(s, nsub)) {
         prof_begin(3, stream);
         e = launch_sel_merge_dq(dt, a.dq_part, ix.pos, s, nsub, a.dq, num_sms, stream);
@@ -602,8 +638,7 @@ static cudaError_t launch_sel_bwd(const SelBwdArgs& a, const SelShape& s, const 
         if (pipelined) {
             e = prefer_l1((const void*)sel_bwd_dkdv_reduce<D, ET>);
             if (e != cudaSuccess) return e;
-            sel_bwd_dkdv_reduce<D, ET><<<dim3((unsigned)(s.Hk * s.NBmax + 1), (unsigned)(nsub * (2 * kKT * (D / 4) / 1024))), 256, 0, stream>>>(
-                a.slabs, a.bd.cu_k ? a.bd.cu_k : a.cu, s, ix, nsub, (ET*)a.dk, (ET*)a.dv);
+            sel_bwd_dkdv_reduce<D, ET><<<dim3(kv_blocks, kv_shares), 256, 0, stream>>>(a.slabs, kv_starts, s, ix, nsub, (ET*)a.dk, (ET*)a.dv);
         } else {
             int64_t n4 = kv_elems / 4;
             sel_bwd_convert<ET><<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(a.dk_acc, a.dv_acc, (ET*)a.dk, (ET*)a.dv, n4);
