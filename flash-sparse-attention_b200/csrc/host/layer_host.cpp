@@ -46,15 +46,27 @@ struct Kept {
     Tensor q, k_raw, k, v, ck, cv, cs, sn, cu_cmp, bounds, o_cmp, lse_cmp, topk, o_sel, lse_sel, ws, o_win, lse_win, gate;
 };
 
-static std::pair<Tensor, Tensor> range_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, const int32_t* lo,
-                                           const int32_t* hi, float scale, int32_t* status) {
+// One of the dense branches: ranges of K/V rows in, o and lse out.
+struct Range {
+    const Tensor &k, &v, &cu_k;
+    const int32_t *lo, *hi;
+    Tensor &o, &lse;
+    int32_t* status;
+};
+// Branches that do not wait for one another, in one launch (the longest first).
+static void range_fwd(const Tensor& q, const Tensor& cu_q, std::initializer_list<Range> branches, float scale) {
     const int64_t N = q.size(0);
-    Tensor o = fresh_like(q), lse = f32({q.size(1), N}, q);
-    check(fsa_range_attn_fwd_dense(ptr(q), ptr(k), ptr(v), iptr(cu_q), iptr(cu_k), lo, hi, N, k.size(0), (int)cu_q.size(0) - 1, (int)q.size(1),
-                                   (int)k.size(1), (int)q.size(2), dtype_code(q), q.stride(0), q.stride(1), k.stride(0), v.stride(0), scale, ptr(o),
-                                   o.stride(0), o.stride(1), lse.data_ptr<float>(), status, stream_of(q)),
+    fsa_range_problem a[3];
+    int n = 0;
+    for (const Range& r : branches) {
+        r.o = fresh_like(q);
+        r.lse = f32({q.size(1), N}, q);
+        a[n++] = {ptr(q), ptr(r.k), ptr(r.v), iptr(cu_q), iptr(r.cu_k), r.lo, r.hi, N, r.k.size(0), q.stride(0), q.stride(1), r.k.stride(0), r.v.stride(0),
+                  ptr(r.o), r.o.stride(0), r.o.stride(1), r.lse.data_ptr<float>(), r.status};
+    }
+    const Tensor& k = branches.begin()->k;
+    check(fsa_range_attn_fwd_dense_several(n, a, (int)cu_q.size(0) - 1, (int)q.size(1), (int)k.size(1), (int)q.size(2), dtype_code(q), scale, stream_of(q)),
           "fsa_range_attn_fwd_dense");
-    return {o, lse};
 }
 
 static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wg, const Tensor& w_key,
@@ -90,21 +102,21 @@ static Tensor layer_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, con
     check(fsa_layer_rope_fwd(ptr(t.q), t.q.stride(0), ptr(t.k_raw), t.k_raw.stride(0), ptr(t.ck), ptr(t.cs), ptr(t.sn), iptr(cu), iptr(t.cu_cmp), s.B,
                              N, s.Nc, c.Hq, c.Hk, c.D, c.ks, c.stride, c.window, dt, ptr(t.q), ptr(t.k), bd, bd + N, bd + 2 * N, st),
           "fsa_layer_rope_fwd");
-    std::tie(t.o_cmp, t.lse_cmp) = range_fwd(t.q, t.ck, t.cv, cu, t.cu_cmp, nullptr, bd, scale, status);
+    const Range cmp{t.ck, t.cv, t.cu_cmp, nullptr, bd, t.o_cmp, t.lse_cmp, status}, win{t.k, t.v, cu, bd + N, bd + 2 * N, t.o_win, t.lse_win, status};
     const int max_blocks = (s.max_len + c.bs - 1) / c.bs, t_out = std::min(c.topk, max_blocks);
     t.topk = i32({c.Hk, N, t_out}, x);
     if (s.every_block(c)) {
         check(fsa_layer_every_block(iptr(cu), s.B, N, c.Hk, t_out, c.bs, t.topk.data_ptr<int32_t>(), st), "fsa_layer_every_block");
         if (checking_status()) t.ws = at::zeros({4}, x.options().dtype(at::kInt));      // (the branch's own word, read as the operator's is)
-        std::tie(t.o_sel, t.lse_sel) = range_fwd(t.q, t.k, t.v, cu, cu, nullptr, bd + 2 * N, scale, t.ws.defined() ? t.ws.data_ptr<int32_t>() : nullptr);
+        range_fwd(t.q, cu, {{t.k, t.v, cu, nullptr, bd + 2 * N, t.o_sel, t.lse_sel, t.ws.defined() ? t.ws.data_ptr<int32_t>() : nullptr}, win, cmp}, scale);
     } else {
+        range_fwd(t.q, cu, {cmp, win}, scale);
         check(fsa_select_topk_fused(ptr(t.q), t.q.stride(0), ptr(t.ck), t.ck.stride(0), t.lse_cmp.data_ptr<float>(), iptr(cu), iptr(t.cu_cmp), N, s.Nc,
                                     s.B, c.Hq, c.Hk, c.D, dt, scale, c.ks, c.stride, c.bs, c.init_blocks, c.local_blocks, max_blocks, t_out,
                                     t.topk.data_ptr<int32_t>(), status, st),
               "fsa_select_topk_fused");
         std::tie(t.o_sel, t.lse_sel, t.ws) = sel_fwd(t.q, t.k, t.v, t.topk, c.bs, cu, scale);
     }
-    std::tie(t.o_win, t.lse_win) = range_fwd(t.q, t.k, t.v, cu, cu, bd + N, bd + 2 * N, scale, status);
     t.gate = fresh({N, 3}, x);
     Tensor out = fresh({N, (int64_t)c.Hq * c.D}, x);
     check(fsa_gate_proj_mix_fwd(ptr(x), x.stride(0), ptr(wg), ptr(t.o_cmp), ptr(t.o_sel), ptr(t.o_win), N, (int)hidden, c.Hq * c.D, dt, ptr(out),

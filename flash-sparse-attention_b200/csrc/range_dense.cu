@@ -41,6 +41,14 @@ struct RangeDenseParams {
     int* status;
 };
 
+// Up to three problems in one launch (blockIdx.z): branches of a layer that do not wait for one another.  A short prompt has fewer tiles
+// than the SMs hold CTAs, and each launch of its own left most of them empty (517 tokens, 32 / 8 heads: 3 x 11 us, together 19: prefill 158 -> 138 us).
+constexpr int kRdProblems = 3;
+struct RangeDenseLaunch {
+    CUtensorMap q[kRdProblems], k[kRdProblems], v[kRdProblems], o[kRdProblems];
+    RangeDenseParams p[kRdProblems];
+};
+
 constexpr int kRdThreads = 192;
 constexpr int kRdBK = 64;
 constexpr float kRdLazy = 8.0f;       // raise a row's reference max only when exceeded by more than this (log2 units)
@@ -52,10 +60,9 @@ __device__ __forceinline__ float rd_ex2(float x) {
 }
 
 template <int D, typename ET>
-__global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDenseParams p, const __grid_constant__ CUtensorMap qmap,
-                                                                const __grid_constant__ CUtensorMap kmap,
-                                                                const __grid_constant__ CUtensorMap vmap,
-                                                                const __grid_constant__ CUtensorMap omap) {
+__global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_constant__ RangeDenseLaunch launch) {
+    const RangeDenseParams& p = launch.p[blockIdx.z];
+    const CUtensorMap &qmap = launch.q[blockIdx.z], &kmap = launch.k[blockIdx.z], &vmap = launch.v[blockIdx.z], &omap = launch.o[blockIdx.z];
     constexpr int BK = kRdBK;
     constexpr int kQ = kTileRows * D * 2;            // Q tile, later the output staging
     constexpr int kKt = BK * D * 2;                  // one K (or V) tile
@@ -347,14 +354,13 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const RangeDens
 }
 
 template <int D, typename ET>
-static cudaError_t launch_rd(const RangeDenseParams& p, const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap,
-                             const CUtensorMap& omap, int max_tiles, cudaStream_t stream) {
+static cudaError_t launch_rd(const RangeDenseLaunch& l, int num, int max_tiles, cudaStream_t stream) {
     constexpr int smem = kTileRows * D * 2 + 4 * kRdBK * D * 2 + 256;
     auto kern = range_fwd_dense<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     prof_begin(FSA_KERNEL_RANGE_DENSE, stream);
-    kern<<<dim3((unsigned)max_tiles, (unsigned)p.Hk), kRdThreads, smem, stream>>>(p, qmap, kmap, vmap, omap);
+    kern<<<dim3((unsigned)max_tiles, (unsigned)l.p[0].Hk, (unsigned)num), kRdThreads, smem, stream>>>(l);
     prof_end(FSA_KERNEL_RANGE_DENSE, stream);
     return cudaGetLastError();
 }
@@ -741,43 +747,53 @@ cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& 
 
 using namespace fsa;
 
+extern "C" int fsa_range_attn_fwd_dense_several(int num, const fsa_range_problem* problems, int B, int Hq, int Hk, int D, int dtype, float sm_scale,
+                                                void* stream_) {
+    if (num <= 0 || !problems || B < 0 || Hq <= 0 || Hk <= 0 || Hq % Hk != 0) return FSA_ERR_BAD_ARG;
+    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
+    const int G = Hq / Hk;
+    for (int i = 0; i < num; ++i)
+        if (problems[i].N < 0 || problems[i].Nk < 0) return FSA_ERR_BAD_ARG;
+    if ((D != 64 && D != 128) || G > 32 || num > kRdProblems) return FSA_ERR_UNSUPPORTED;
+    if (!(sm_scale > 0.f)) return FSA_ERR_BAD_ARG;
+    const int TPT = (kTileRows / G) & ~3;
+    RangeDenseLaunch l = {};
+    int used = 0, max_tiles = 0, rc;
+    for (int i = 0; i < num; ++i) {
+        const fsa_range_problem& a = problems[i];
+        if (a.N == 0 || B == 0) continue;
+        if (!a.q || !a.k || !a.v || !a.cu_seqlens_q || !a.cu_seqlens_k || !a.kv_hi || !a.o || !a.lse || a.Nk == 0) return FSA_ERR_BAD_ARG;
+        if (((uintptr_t)a.q & 15) || ((uintptr_t)a.k & 15) || ((uintptr_t)a.v & 15) || ((uintptr_t)a.o & 15)) return FSA_ERR_BAD_ARG;
+        if ((a.q_stride_n % 8) || (a.q_stride_h % 8) || (a.k_stride_n % 8) || (a.v_stride_n % 8) || (a.o_stride_n % 8) || (a.o_stride_h % 8))
+            return FSA_ERR_BAD_ARG;
+        if (a.k_stride_n < (int64_t)Hk * D || a.v_stride_n < (int64_t)Hk * D) return FSA_ERR_BAD_ARG;
+        if (used == 0) {
+            (void)cudaGetLastError();
+            if ((rc = ensure_context())) return rc;
+        }
+        if ((rc = make_tile_map_3d_box(&l.q[used], a.q, dtype, D, a.N, Hq, a.q_stride_n, a.q_stride_h, TPT, G))) return rc;
+        if ((rc = make_tile_map_3d_box(&l.o[used], a.o, dtype, D, a.N, Hq, a.o_stride_n, a.o_stride_h, TPT, G))) return rc;
+        if ((rc = make_tile_map(&l.k[used], a.k, dtype, a.Nk, (int64_t)Hk * D, a.k_stride_n, 64))) return rc;
+        if ((rc = make_tile_map(&l.v[used], a.v, dtype, a.Nk, (int64_t)Hk * D, a.v_stride_n, 64))) return rc;
+        RangeDenseParams& p = l.p[used++];
+        p.cu_q = a.cu_seqlens_q; p.cu_k = a.cu_seqlens_k; p.kv_lo = a.kv_lo; p.kv_hi = a.kv_hi;
+        p.N = a.N; p.Nk = a.Nk; p.B = B; p.Hq = Hq; p.Hk = Hk; p.G = G; p.TPT = TPT;
+        p.scale_log2 = sm_scale * 1.4426950408889634f;
+        p.o = a.o; p.o_sn = a.o_stride_n; p.o_sh = a.o_stride_h; p.lse = a.lse; p.status = a.status;
+        const int tiles = (int)((a.N + TPT - 1) / TPT) + B;
+        if (tiles > max_tiles) max_tiles = tiles;
+    }
+    if (used == 0) return FSA_OK;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    const cudaError_t e = dtype == FSA_DTYPE_BF16 ? (D == 128 ? launch_rd<128, __nv_bfloat16>(l, used, max_tiles, stream) : launch_rd<64, __nv_bfloat16>(l, used, max_tiles, stream))
+                                                  : (D == 128 ? launch_rd<128, __half>(l, used, max_tiles, stream) : launch_rd<64, __half>(l, used, max_tiles, stream));
+    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+}
+
 extern "C" int fsa_range_attn_fwd_dense(const void* q, const void* k, const void* v, const int32_t* cu_seqlens_q,
                                         const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi, int64_t N, int64_t Nk,
                                         int B, int Hq, int Hk, int D, int dtype, int64_t q_sn, int64_t q_sh, int64_t k_sn, int64_t v_sn,
-                                        float sm_scale, void* o, int64_t o_sn, int64_t o_sh, float* lse, int32_t* status, void* stream_) {
-    if (N < 0 || Nk < 0 || B < 0 || Hq <= 0 || Hk <= 0 || Hq % Hk != 0) return FSA_ERR_BAD_ARG;
-    if (dtype != FSA_DTYPE_BF16 && dtype != FSA_DTYPE_FP16) return FSA_ERR_BAD_ARG;
-    if (D != 64 && D != 128) return FSA_ERR_UNSUPPORTED;
-    const int G = Hq / Hk;
-    if (G > 32) return FSA_ERR_UNSUPPORTED;
-    if (!(sm_scale > 0.f)) return FSA_ERR_BAD_ARG;
-    if (N == 0 || B == 0) return FSA_OK;
-    if (!q || !k || !v || !cu_seqlens_q || !cu_seqlens_k || !kv_hi || !o || !lse || Nk == 0) return FSA_ERR_BAD_ARG;
-    if (((uintptr_t)q & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)o & 15)) return FSA_ERR_BAD_ARG;
-    if ((q_sn % 8) || (q_sh % 8) || (k_sn % 8) || (v_sn % 8) || (o_sn % 8) || (o_sh % 8)) return FSA_ERR_BAD_ARG;
-    if (k_sn < (int64_t)Hk * D || v_sn < (int64_t)Hk * D) return FSA_ERR_BAD_ARG;
-    (void)cudaGetLastError();
-    int rc = ensure_context();
-    if (rc) return rc;
-    const int TPT = (kTileRows / G) & ~3;
-    CUtensorMap qmap, kmap, vmap, omap;
-    if ((rc = make_tile_map_3d_box(&qmap, q, dtype, D, N, Hq, q_sn, q_sh, TPT, G))) return rc;
-    if ((rc = make_tile_map_3d_box(&omap, o, dtype, D, N, Hq, o_sn, o_sh, TPT, G))) return rc;
-    if ((rc = make_tile_map(&kmap, k, dtype, Nk, (int64_t)Hk * D, k_sn, 64))) return rc;
-    if ((rc = make_tile_map(&vmap, v, dtype, Nk, (int64_t)Hk * D, v_sn, 64))) return rc;
-    RangeDenseParams p;
-    p.cu_q = cu_seqlens_q; p.cu_k = cu_seqlens_k; p.kv_lo = kv_lo; p.kv_hi = kv_hi;
-    p.N = N; p.Nk = Nk; p.B = B; p.Hq = Hq; p.Hk = Hk; p.G = G; p.TPT = TPT;
-    p.scale_log2 = sm_scale * 1.4426950408889634f;
-    p.o = o; p.o_sn = o_sn; p.o_sh = o_sh; p.lse = lse; p.status = status;
-    const int max_tiles = (int)((N + TPT - 1) / TPT) + B;
-    cudaStream_t stream = (cudaStream_t)stream_;
-    cudaError_t e;
-    if (dtype == FSA_DTYPE_BF16)
-        e = D == 128 ? launch_rd<128, __nv_bfloat16>(p, qmap, kmap, vmap, omap, max_tiles, stream)
-                     : launch_rd<64, __nv_bfloat16>(p, qmap, kmap, vmap, omap, max_tiles, stream);
-    else
-        e = D == 128 ? launch_rd<128, __half>(p, qmap, kmap, vmap, omap, max_tiles, stream)
-                     : launch_rd<64, __half>(p, qmap, kmap, vmap, omap, max_tiles, stream);
-    return e == cudaSuccess ? FSA_OK : FSA_ERR_CUDA;
+                                        float sm_scale, void* o, int64_t o_sn, int64_t o_sh, float* lse, int32_t* status, void* stream) {
+    const fsa_range_problem a = {q, k, v, cu_seqlens_q, cu_seqlens_k, kv_lo, kv_hi, N, Nk, q_sn, q_sh, k_sn, v_sn, o, o_sn, o_sh, lse, status};
+    return fsa_range_attn_fwd_dense_several(1, &a, B, Hq, Hk, D, dtype, sm_scale, stream);
 }

@@ -68,6 +68,7 @@ SIGNATURES = {
          c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
          c_int64, c_int64, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p],
     ),
+    "fsa_range_attn_fwd_dense_several": (c_int, [c_int, c_void_p] + [c_int] * 5 + [c_float, c_void_p]),
     "fsa_range_attn_fwd_dense": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int,

@@ -186,6 +186,19 @@ int fsa_range_attn_fwd_dense(const void* q, const void* k, const void* v, const 
                              int64_t total_kv_rows, int batch, int num_q_heads, int num_kv_heads, int head_dim, int dtype,
                              int64_t q_stride_n, int64_t q_stride_h, int64_t k_stride_n, int64_t v_stride_n, float sm_scale,
                              void* o, int64_t o_stride_n, int64_t o_stride_h, float* lse, int32_t* status, void* stream);
+
+/* The same for up to three problems of one batch and head layout in one launch (the branches of a layer); arguments as above. */
+typedef struct {
+    const void *q, *k, *v;
+    const int32_t *cu_seqlens_q, *cu_seqlens_k, *kv_lo, *kv_hi;
+    int64_t N, Nk, q_stride_n, q_stride_h, k_stride_n, v_stride_n;
+    void* o;
+    int64_t o_stride_n, o_stride_h;
+    float* lse;
+    int32_t* status;
+} fsa_range_problem;
+int fsa_range_attn_fwd_dense_several(int num, const fsa_range_problem* problems, int batch, int num_q_heads, int num_kv_heads, int head_dim, int dtype,
+                                     float sm_scale, void* stream);
 int fsa_range_attn_bwd_indexed(int head_dim);
 int fsa_range_attn_index(const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* kv_lo, const int32_t* kv_hi,
                          int64_t total_tokens, int64_t total_kv_rows, int batch, int num_q_heads, int num_kv_heads,
