@@ -368,17 +368,23 @@ static cudaError_t launch_rd(const RangeDenseLaunch& l, int num, int max_tiles, 
 
 // ------------------------------------------------------------------------------------------------ dQ, query-tile-major
 // dQ of range attention with the same tiling as the forward above: per K/V tile S = Q K^T and dP = dO V^T, then
-// P = exp2(S c - lse), dS = scale P (dP - delta) to swizzled shared memory, dQ (+)= dS K accumulated in TMEM over the
-// tiles and written once.  (In the reference: the dQ part of _backward_kernel, nsa_ref/ops/compressed_attention.py:
+// P = exp2(S c - lse), dS = scale P (dP - delta), dQ (+)= dS K accumulated in TMEM over the tiles and written once.  (In the reference: the dQ part of _backward_kernel, nsa_ref/ops/compressed_attention.py:
 // 193-760, and of flash-attn's backward for the sliding window.)  With it the block-major backward kernel computes
-// only dK and dV and no partial dQ row is written or merged.  One CTA per SM, 352 threads:
+// only dK and dV and no partial dQ row is written or merged.  One CTA per SM, 384 threads:
 //   warp 0      TMA producer: Q and dO tiles of every item, (K, V) tiles through a four-stage ring (a stage comes free only
 //               when the tile's dQ product is done, and the next load needs a microsecond to land);
 //   warp 1      one elected thread issues S and dP (two TMEM buffers: they run a tile ahead of the row threads);
 //   warp 10     one elected thread issues dQ (a second issuer: see the MMA section);
-//   warps 2..9  two groups of 128 row threads, each on 32 of the 64 key columns: dS to one of two shared-memory buffers;
-//               epilogue: each group rounds 64 of the dQ columns, stages them (the Q tile's memory) and stores its slab by
-//               3-D TMA (plain stores for the last, partial tile of a sequence).
+//   warp 11     finds the items, up to four ahead (the search and its loads take ~3700 cycles, three tiles' worth);
+//   warps 2..9  two groups of 128 row threads: Q (group 0) and dO (group 1) of the next item to TMEM when the item's S / dP are
+//               done; 32 of the 64 key columns each, dS over dP; epilogue: each group rounds 64 of the dQ columns, stages them
+//               and stores its slab by 3-D TMA (plain stores for the last, partial tile of a sequence).
+// The left operand of every product (Q, dO, dS) comes from TMEM, so a tile of 64 keys takes three reads of 16 KB from shared
+// memory.  With all of them in shared memory it was 128 KB and the writes of dS, twice the cycles that the products take.
+// Measured at 2 x 32768 tokens, 32 / 8 heads (window of 512 and compressed branch together): operands in shared memory, items
+// found by every warp for itself 3.49 ms; operands in TMEM 2.92; items by a warp of their own and row numbers an item ahead 2.77
+// (6.4 thousand cycles between two items before, ten tiles of 1190).  A tile is now bound by its row threads (700 cycles) in
+// turn with the S / dP products, which two TMEM buffers let run one tile ahead; the products alone take 770.
 struct RangeDqParams {
     const int32_t* cu_q;
     const int32_t* cu_k;
@@ -393,8 +399,9 @@ struct RangeDqParams {
     int* status;
 };
 
-constexpr int kDqThreads = 352;     // producer, S/dP issuer, 8 row warps, dQ issuer
+constexpr int kDqThreads = 384;     // producer, S/dP issuer, 8 row warps, dQ issuer, item warp
 constexpr int kDqStages = 4;
+constexpr int kDqItems = 4;         // items known ahead
 
 // One work item of the dQ kernel: a tile of tokens x one KV head.
 struct DqItem {
@@ -437,36 +444,41 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     constexpr int D = 128, BK = kRdBK, KH = D / 64;
     constexpr int kQ = kTileRows * D * 2;            // Q tile, same for dO
     constexpr int kKt = BK * D * 2;
-    constexpr int kDS = kTileRows * BK * 2;          // one dS buffer; the two together stage a dQ tile in the epilogue
+    constexpr int kOut = kTileRows * 128;            // 64 columns of the dQ tile on their way out
     constexpr uint32_t kCols = 512;
-    constexpr int cDQ = 256;                         // S(b) at 128 b, dP(b) at 128 b + 64
+    constexpr int cDQ = 256, cQ = 384, cDO = 448;    // S(b) at 128 b, dP(b) / dS(b) at 128 b + 64; Q and dO two values a column
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;
     uint8_t* sDO = sQ + kQ;
     uint8_t* sKV = sDO + kQ;                         // stage: K then V
-    uint8_t* sDS = sKV + kDqStages * 2 * kKt;        // two buffers
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + 2 * kDS);
+    uint8_t* sOut = sKV + kDqStages * 2 * kKt;       // two slabs
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + 2 * kOut);
     uint64_t* qd_full = bars;           // Q and dO tiles of an item have landed
-    uint64_t* qd_empty = bars + 1;      // ... have been read by the item's last S / dP products
+    uint64_t* qd_empty = bars + 1;      // ... have been read by the 256 row threads
     uint64_t* kv_full = bars + 2;                        // [stages]
     uint64_t* kv_empty = kv_full + kDqStages;            // [stages] the dQ product of the tile is done
     uint64_t* sdp_full = kv_empty + kDqStages;           // [2]
     uint64_t* sdp_free = sdp_full + 2;                   // [2] the 256 row threads have read S and dP
-    uint64_t* ds_full = sdp_free + 2;                    // [2] ... have written dS
+    uint64_t* ds_full = sdp_free + 2;                    // [2] ... have written dS over dP
     uint64_t* ds_empty = ds_full + 2;                    // [2] the dQ product has read dS
     uint64_t* dq_free = ds_empty + 2;                    // the 256 row threads have read an item's dQ accumulator
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(dq_free + 1);
+    uint64_t* qt_full = dq_free + 1;                     // ... have written an item's Q and dO to TMEM
+    uint64_t* it_full = qt_full + 1;                     // [items]
+    uint64_t* it_empty = it_full + kDqItems;             // [items] the eleven other warps have read the entry
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(it_empty + kDqItems);
+    int4* s_item = reinterpret_cast<int4*>(bars + 32);   // [items][2]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = p.status;
     if (tid == 0) {
-        mbar_init(qd_full, 1); mbar_init(qd_empty, 1);
+        mbar_init(qd_full, 1); mbar_init(qd_empty, 256);
         for (int i = 0; i < kDqStages; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sdp_full[i], 1); mbar_init(&sdp_free[i], 256);
             mbar_init(&ds_full[i], 256); mbar_init(&ds_empty[i], 1);
         }
-        mbar_init(dq_free, 256);
+        for (int i = 0; i < kDqItems; ++i) { mbar_init(&it_full[i], 1); mbar_init(&it_empty[i], kDqThreads / 32 - 1); }
+        mbar_init(dq_free, 256); mbar_init(qt_full, 256);
         mbar_init_fence();
         tma_prefetch_desc(&qmap);
         tma_prefetch_desc(&domap);
@@ -481,13 +493,36 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     const uint32_t tbase = tmem_slot;
     const int ntiles = count_seq_tiles(p.cu_q, p.B, p.TPT, lane);
     const int nitems = ntiles * p.Hk;
+    // Entry n of this CTA's items: every warp but the one that fills the ring takes each of them once, in order.
+    auto take_item = [&](int n, bool& ok) {
+        ok = mbar_wait(&it_full[n % kDqItems], (n / kDqItems) & 1, status) && ok;
+        const int4 x = s_item[(n % kDqItems) * 2], y = s_item[(n % kDqItems) * 2 + 1];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&it_empty[n % kDqItems]);
+        DqItem m;
+        m.seq = x.x; m.tok0 = x.y; m.ne = x.z; m.row_lo = x.w; m.nblk = y.x; m.h = y.y;
+        return m;
+    };
 
-    if (warp == 0) {
+    if (warp == kDqThreads / 32 - 1) {
+        // ------------------------------------------------------------------ items
+        bool ok = true;
+        int n = 0;
+        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
+            const DqItem m = dq_item(p, ntiles, w, lane);
+            ok = mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status) && ok;
+            if (lane == 0) {
+                s_item[(n % kDqItems) * 2] = make_int4(m.seq, m.tok0, m.ne, m.row_lo);
+                s_item[(n % kDqItems) * 2 + 1] = make_int4(m.nblk, m.h, 0, 0);
+                mbar_arrive(&it_full[n % kDqItems]);
+            }
+        }
+    } else if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         bool ok = true;
-        int kvc = 0, qi = 0;           // K/V tiles and non-empty items so far
-        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-            const DqItem m = dq_item(p, ntiles, w, lane);
+        int kvc = 0, qi = 0, n = 0;    // K/V tiles and non-empty items so far
+        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
+            const DqItem m = take_item(n, ok);
             if (m.nblk == 0) continue;
             if (lane == 0) {
                 ok = mbar_wait(qd_empty, (qi & 1) ^ 1, status) && ok;
@@ -516,47 +551,48 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
-    } else if (warp == 1 || warp == kDqThreads / 32 - 1) {
+    } else if (warp == 1 || warp == kDqThreads / 32 - 2) {
         // ------------------------------------------------------------------ MMA issuers
-        // Two warps: the k-steps of one accumulator follow one another at ~100 cycles each, and a single issuing thread also
-        // waits on barriers between products; with dQ on a warp of its own its chain overlaps the S / dP chains of the next
-        // tile (measured: 20 % faster).  Warp 1 issues S and dP, the last warp issues dQ.  The K/V tiles of all items form one sequence
-        // c = 0, 1, ...; S / dP run ahead of dQ as far as their two TMEM buffers and the K/V ring allow, also across the
-        // boundary between two items (the next item's Q / dO are loaded as soon as this item's last S / dP are done).
+        // Two warps: a single issuing thread waits on barriers between products; with dQ on a warp of its own its chain overlaps
+        // the S / dP chains of the next tile (measured: 20 % faster).  Warp 1 issues S and dP, warp 10 dQ.  The K/V tiles of all
+        // items form one sequence c = 0, 1, ...; S / dP run ahead of dQ as far as their two TMEM buffers and the K/V ring allow,
+        // also across the boundary between two items (the next item's Q / dO replace this item's when its last S / dP are done).
         const bool leader = elect_one();
         constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, BK, false, false);
         constexpr uint32_t idesc_dq = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);     // dS (K-major) x K (MN-major)
         constexpr uint32_t hi_1024 = umma_desc_hi(1024);
-        constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
-        const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16), do_lo = umma_desc_lo(smem_u32(sDO), 16);
+        constexpr int kSlabB = (BK * 128) >> 4;
         const uint32_t kv_lo_ = umma_desc_lo(smem_u32(sKV), 16);
-        const uint32_t ds_lo = umma_desc_lo(smem_u32(sDS), 16);
         const uint32_t k_mn_lo = umma_desc_lo(smem_u32(sKV), BK * 128);
         bool ok = true;
-        int c = 0, qi = 0;
-        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-            const DqItem m = dq_item(p, ntiles, w, lane);
+        int c = 0, qi = 0, n = 0;
+        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
+            const DqItem m = take_item(n, ok);
             if (m.nblk == 0) continue;
             if (warp == 1) {
-                ok = mbar_wait(qd_full, qi & 1, status) && ok;
+                ok = mbar_wait(qt_full, qi & 1, status) && ok;
                 for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                     const int b = c & 1, st = c % kDqStages;
+                    const uint32_t k_lo = kv_lo_ + (uint32_t)(st * ((2 * kKt) >> 4));
+                    const uint32_t v_lo = k_lo + (uint32_t)(kKt >> 4);
                     ok = mbar_wait(&kv_full[st], (c / kDqStages) & 1, status) && ok;
                     ok = mbar_wait(&sdp_free[b], ((c >> 1) & 1) ^ 1, status) && ok;     // S / dP of tile c - 2 have been read
                     tc_fence_after();
                     if (leader) {
-                        const uint32_t k_lo = kv_lo_ + (uint32_t)(st * ((2 * kKt) >> 4));
-                        const uint32_t v_lo = k_lo + (uint32_t)(kKt >> 4);
 #pragma unroll
                         for (int ks = 0; ks < D / 16; ++ks)
-                            umma_ss(tbase + b * 128, umma_desc_pack(q_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
-                                    umma_desc_pack(k_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
+                            umma_ts(tbase + b * 128, tbase + cQ + ks * 8, umma_desc_pack(k_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024),
+                                    idesc_s, ks > 0);
+                    }
+                    __syncwarp();
+                    ok = mbar_wait(&ds_empty[b], ((c >> 1) & 1) ^ 1, status) && ok;     // the dQ product of tile c - 2 has read dS
+                    tc_fence_after();
+                    if (leader) {
 #pragma unroll
                         for (int ks = 0; ks < D / 16; ++ks)
-                            umma_ss(tbase + b * 128 + BK, umma_desc_pack(do_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
-                                    umma_desc_pack(v_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
+                            umma_ts(tbase + b * 128 + BK, tbase + cDO + ks * 8, umma_desc_pack(v_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024),
+                                    idesc_s, ks > 0);
                         umma_commit(&sdp_full[b]);
-                        if (j + 1 == m.nblk) umma_commit(qd_empty);          // every S / dP of this item has been issued
                     }
                     __syncwarp();
                 }
@@ -565,15 +601,13 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                     const int b = c & 1, st = c % kDqStages;
                     ok = mbar_wait(&ds_full[b], (c >> 1) & 1, status) && ok;      // (implies S / dP of the tile are done with K and V)
                     if (j == 0 && qi > 0) ok = mbar_wait(dq_free, (qi - 1) & 1, status) && ok;     // the previous item's dQ has been read
-                    fence_async_smem();
                     tc_fence_after();
                     if (leader) {
-                        const uint32_t a_lo = ds_lo + (uint32_t)(b * (kDS >> 4));
                         const uint32_t b_lo = k_mn_lo + (uint32_t)(st * ((2 * kKt) >> 4));
 #pragma unroll
-                        for (int ks = 0; ks < BK / 16; ++ks)
-                            umma_ss(tbase + cDQ, umma_desc_pack(a_lo + ks * 2, hi_1024), umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024),
-                                    idesc_dq, (j > 0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 0; ks < BK / 16; ++ks)      // the two row groups keep their halves 32 columns apart
+                            umma_ts(tbase + cDQ, tbase + b * 128 + BK + (ks >> 1) * 32 + (ks & 1) * 8,
+                                    umma_desc_pack(b_lo + ks * (2048 >> 4), hi_1024), idesc_dq, (j > 0 || ks > 0) ? 1u : 0u);
                         umma_commit(&kv_empty[st]);
                         umma_commit(&ds_empty[b]);
                     }
@@ -593,20 +627,54 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
         const int cb = sb * HC;
         bool ok = true;
         int c = 0, qi = 0;
+        // One row of an item's Q (group 0) or dO (group 1) to TMEM.  Not before the last S / dP products of the item before are done.
+        auto take_row = [&]() {
+            ok = mbar_wait(qd_full, qi & 1, status) && ok;
+            ++qi;
+            const uint8_t* src = sb ? sDO : sQ;
+            uint32_t x[2][32];
+#pragma unroll
+            for (int i = 0; i < D / 8; ++i)
+                *reinterpret_cast<uint4*>(&x[i >> 3][(i & 7) * 4]) = *reinterpret_cast<const uint4*>(src + (i >> 3) * (kTileRows * 128) + sw128_chunk_off(r, i & 7));
+            tmem_st32(tbase + lane_off + (sb ? cDO : cQ), x[0]);
+            tmem_st32(tbase + lane_off + (sb ? cDO : cQ) + 32, x[1]);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(qd_empty);
+            mbar_arrive(qt_full);
+        };
+        // This row's numbers, loaded an item ahead: item numbers and loads of their own between two items were a third of the kernel.
+        struct Row { int lo, hi; float lse, delta; };
+        auto load_numbers = [&](const DqItem& m) {
+            Row x = {0, -1, 0.f, 0.f};
+            if (g < p.G && e < m.ne) {
+                x.lo = p.kv_lo ? __ldg(p.kv_lo + m.tok0 + e) : __ldg(p.cu_k + m.seq);
+                x.hi = __ldg(p.kv_hi + m.tok0 + e);
+                const int64_t idx = (int64_t)(m.h * p.G + g) * p.N + m.tok0 + e;
+                x.lse = __ldg(p.lse + idx);
+                x.delta = __ldg(p.delta + idx);
+            }
+            return x;
+        };
+        DqItem m;
+        m.nblk = m.ne = 0;
+        int n = 0;
+        if ((int)blockIdx.x < nitems) {
+            m = take_item(n, ok);
+            if (m.nblk > 0) take_row();
+        }
+        Row row = load_numbers(m);
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-            const DqItem m = dq_item(p, ntiles, w, lane);
             const bool row_valid = g < p.G && e < m.ne;
             const int tok = m.tok0 + e;
-            int lo_r = 0, hi_r = -1;
-            float lse_r = 0.f, delta_s = 0.f;
-            if (row_valid) {
-                lo_r = p.kv_lo ? __ldg(p.kv_lo + tok) : __ldg(p.cu_k + m.seq);
-                hi_r = min(__ldg(p.kv_hi + tok), (int)p.Nk - 1);     // rows past the end of K/V do not exist
-                const int64_t idx = (int64_t)(m.h * p.G + g) * p.N + tok;
-                lse_r = __ldg(p.lse + idx);
-                delta_s = __ldg(p.delta + idx) * p.scale;
-                if (!(lse_r > -INFINITY)) hi_r = lo_r - 1;      // a row that saw nothing in the forward sees nothing here
-            }
+            const int lo_r = row.lo;
+            const float lse_r = row.lse, delta_s = row.delta * p.scale;
+            int hi_r = min(row.hi, (int)p.Nk - 1);              // rows past the end of K/V do not exist
+            if (!(lse_r > -INFINITY)) hi_r = lo_r - 1;          // a row that saw nothing in the forward sees nothing here
+            DqItem next;
+            next.nblk = next.ne = 0;
+            if (w + (int)gridDim.x < nitems) next = take_item(++n, ok);
+            row = load_numbers(next);
             for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                 const int b = c & 1;
                 const int R0 = m.row_lo + j * BK;
@@ -622,6 +690,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                     tmem_ld_wait();
                     tc_fence_before();
                     mbar_arrive(&sdp_free[b]);       // both rows are in registers: the buffer may take tile c + 2
+                    if (j + 1 == m.nblk && next.nblk > 0) take_row();      // the next item's S / dP run under this item's end
                     if (all_visible) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
@@ -631,25 +700,25 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                                                                p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s));
                         }
                     } else {
+                        // bit i: column cb + i is seen
+                        const int v_lo = min(max(c_lo - cb, 0), HC), v_hi = min(max(c_hi - cb, 0), HC);
+                        const uint32_t vis = v_hi > v_lo ? (0xffffffffu >> (HC - v_hi + v_lo)) << v_lo : 0u;
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
-                            const float p0 = (cb + i >= c_lo && cb + i < c_hi) ? rd_ex2(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r)) : 0.f;
-                            const float p1 = (cb + i + 1 >= c_lo && cb + i + 1 < c_hi) ? rd_ex2(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse_r)) : 0.f;
-                            const float d0 = p0 > 0.f ? p0 * fmaf(__uint_as_float(dv[i]), p.scale, -delta_s) : 0.f;
-                            const float d1 = p1 > 0.f ? p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s) : 0.f;
+                            const float p0 = rd_ex2(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse_r));
+                            const float p1 = rd_ex2(fmaf(__uint_as_float(sv[i + 1]), p.scale_log2, -lse_r));
+                            const float d0 = (vis >> i & 1u) && p0 > 0.f ? p0 * fmaf(__uint_as_float(dv[i]), p.scale, -delta_s) : 0.f;
+                            const float d1 = (vis >> (i + 1) & 1u) && p1 > 0.f ? p1 * fmaf(__uint_as_float(dv[i + 1]), p.scale, -delta_s) : 0.f;
                             dd[i >> 1] = ElemTraits<ET>::pack2(d0, d1);
                         }
                     }
                 }
-                ok = mbar_wait(&ds_empty[b], ((c >> 1) & 1) ^ 1, status) && ok;      // the dQ product of tile c - 2 has read this buffer
-                uint8_t* ds = sDS + b * kDS;
-#pragma unroll
-                for (int c4 = 0; c4 < HC / 8; ++c4)
-                    *reinterpret_cast<uint4*>(ds + sw128_chunk_off(r, sb * (HC / 8) + c4)) =
-                        make_uint4(dd[c4 * 4], dd[c4 * 4 + 1], dd[c4 * 4 + 2], dd[c4 * 4 + 3]);
-                fence_async_smem();
+                tmem_st16(tbase + lane_off + b * 128 + BK + cb, dd);
+                tmem_st_wait();
+                tc_fence_before();
                 mbar_arrive(&ds_full[b]);
             }
+            if (m.nblk == 0 && next.nblk > 0) take_row();
             // ---- epilogue of the item: this group's 64 of the 128 dQ columns
             const bool full_tile = m.ne == p.TPT && p.G * p.TPT == kTileRows && m.nblk > 0;
             if (m.nblk > 0) {
@@ -657,7 +726,12 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                 tc_fence_after();
             }
             ET* drow = reinterpret_cast<ET*>(p.dq) + ((int64_t)tok * p.Hq + (m.h * p.G + g)) * D + sb * 64;
-            uint8_t* stage = sDS + sb * kDS;            // (both dS buffers are free: every dQ product of the item is done)
+            uint8_t* stage = sOut + sb * kOut;
+            if (full_tile) {                             // the slab of the item before has left it
+                if (quarter == 0 && lane == 0) bulk_wait_read0();
+                if (sb == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+                else asm volatile("bar.sync 2, 128;" ::: "memory");
+            }
 #pragma unroll
             for (int c0 = 0; c0 < 64; c0 += 32) {
                 uint32_t a[32];
@@ -686,7 +760,6 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             if (m.nblk > 0) {
                 tc_fence_before();
                 mbar_arrive(dq_free);            // the accumulator may take the next item
-                ++qi;
             }
             if (full_tile) {
                 fence_async_smem();
@@ -695,12 +768,11 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                 if (quarter == 0 && lane == 0) {
                     if (ok) tma_store_3d(&dqmap, sb * 64, m.tok0, m.h * p.G, smem_u32(stage));
                     bulk_commit();
-                    bulk_wait_read0();           // the staging memory is a dS buffer again in the next item
                 }
-                asm volatile("bar.sync 3, 256;" ::: "memory");
             }
+            m = next;
         }
-        (void)qi;
+        if (quarter == 0 && lane == 0) bulk_wait_read0();      // the last slab has left shared memory
     }
     tc_fence_before();
     __syncthreads();
@@ -719,7 +791,7 @@ cudaError_t launch_range_bwd_dq(int dtype, const SelBwdArgs& a, const SelShape& 
     p.N = s.N; p.Nk = s.Nk; p.B = s.B; p.Hq = s.Hq; p.Hk = s.Hk; p.G = s.G; p.TPT = s.TPT;
     p.scale = a.sm_scale; p.scale_log2 = a.sm_scale * 1.4426950408889634f;
     p.lse = a.lse; p.delta = a.delta; p.dq = a.dq; p.status = status;
-    constexpr int smem = 2 * kTileRows * 128 * 2 + kDqStages * 2 * kRdBK * 128 * 2 + 2 * kTileRows * kRdBK * 2 + 256;
+    constexpr int smem = 2 * kTileRows * 128 * 2 + kDqStages * 2 * kRdBK * 128 * 2 + 2 * kTileRows * kRdBK * 2 + 256 + kDqItems * 32;
     const int64_t max_items = ((s.N + s.TPT - 1) / s.TPT + s.B) * (int64_t)s.Hk;
     int sms = 0;
     if (device_sm_count(&sms) != 0 || sms <= 0) return cudaErrorInvalidValue;
