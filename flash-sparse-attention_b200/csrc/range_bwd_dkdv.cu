@@ -7,9 +7,9 @@
 // group, token) that TMA reads in place: no index, no gather.  Everything is computed transposed -- a TMEM lane is a K/V row
 // -- so that P^T and dS^T are written over S^T and dP^T in TMEM and feed the products from there, never through shared memory:
 //   S^T = K Q^T, dP^T = V dO^T, P = exp2(S c - lse), dS = scale P (dP - delta), dV += P^T dO, dK += dS^T Q.
-// S^T / P^T, dP^T / dS^T, dV and dK take 128 columns each: all of TMEM, one buffer of each.  So the two chains
-// dV(i) -> S(i+1) and dK(i) -> dP(i+1) run in turns, each under the other's exp2 / dS arithmetic; each has an issuing warp of
-// its own, which also overlaps the k-steps of the two where both are ready.
+// S^T / P^T, dP^T / dS^T, dV and dK take 128 columns each: all of TMEM, one buffer of each.  The chains dV(i) -> S(i+1) and
+// dK(i) -> dP(i+1) go by halves of a row tile: a row group hands its 64 rows on and gets the next ones without waiting for the
+// other group, so that one group's exp2 / dS arithmetic runs under the products of the other.  Each chain has an issuing warp.
 //   warp 0       TMA producer: K and V of an item, and Q, dO, Q, dO, ... through a ring of five tiles (32 KB each; a tile
 //                comes free when both products that read it are done)
 //   warp 1       issues S(i) and dV(i)            warp 2    issues dP(i) and dK(i)
@@ -18,7 +18,10 @@
 // Items of few tiles would leave SMs idle at the end, items of one K/V tile are of very different length (the first
 // compressed rows are seen by the whole sequence): a plan on the device cuts the stretches so that an SM gets about eight.  The
 // parts of a K/V tile that was cut go to fp32 slabs that the last kernel adds in order (bit-reproducible); others are written in place.
-// Bound by the MMA chains (128 x 128 x 16 k-steps of one accumulator follow one another at ~100 cycles; 32 per tile).
+// A tile takes 3100 cycles where every row sees all K/V rows: its products read 256 KB of shared memory and the loads write 64 KB,
+// 2560 cycles (the products alone: 2050).  Tiles that need the mask are bound by the row threads (4700).  Measured at 2 x 32768
+// tokens, 32 / 8 heads (window of 512 and compressed branch together): whole tiles in turns 4.19 ms, halves 3.93; at 8 sequences
+// of about 1000 tokens 119 -> 108 us.
 #include "../../include/fsa_sm100.h"
 #include <climits>
 
@@ -202,8 +205,8 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
     uint8_t* sU = sV + kRkTile;                      // [kRkUnits] Q, dO, Q, dO, ...
     float* sLse = reinterpret_cast<float*>(sU + kRkUnits * kRkTile);      // [2][128]
     float* sDel = sLse + 2 * 128;                                         // [2][128] scale * delta
-    uint16_t* sVis = reinterpret_cast<uint16_t*>(sDel + 2 * 128);         // [2][128] first visible row | (rows - 1) << 8
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sVis + 2 * 128);
+    uint8_t* sVis = reinterpret_cast<uint8_t*>(sDel + 2 * 128);           // [2][2][128] first visible row; last one | 128
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sVis + 4 * 128);
     uint64_t* k_full = bars;            // K of an item has landed
     uint64_t* k_empty = bars + 1;       // ... has been read by the item's last S product
     uint64_t* v_full = bars + 2;
@@ -212,24 +215,26 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
     uint64_t* u_empty = u_full + kRkUnits;           // [units] the two products that read a Q or dO tile are done
     uint64_t* st_full = u_empty + kRkUnits;          // [2]
     uint64_t* st_empty = st_full + 2;                // [2]
-    uint64_t* s_full = st_empty + 2;    // S(i) is done
-    uint64_t* p_full = s_full + 1;      // P(i) is in its place
-    uint64_t* dp_full = s_full + 2;
-    uint64_t* ds_full = s_full + 3;
-    uint64_t* dv_done = s_full + 4;     // the item's last dV product is done
-    uint64_t* dk_done = s_full + 5;
-    uint64_t* dv_free = s_full + 6;     // the accumulator has been read
-    uint64_t* dk_free = s_full + 7;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(s_full + 8);
-    int* s_masked = reinterpret_cast<int*>(s_full + 8) + 2;               // [2] some row of the tile does not see all K/V rows
+    uint64_t* s_full = st_empty + 2;    // [2 halves] S(i) is done
+    uint64_t* p_full = s_full + 2;      // [2] P(i) is in its place
+    uint64_t* dp_full = s_full + 4;     // [2]
+    uint64_t* ds_full = s_full + 6;     // [2]
+    uint64_t* dv_done = s_full + 8;     // the item's last dV product is done
+    uint64_t* dk_done = s_full + 9;
+    uint64_t* dv_free = s_full + 10;    // the accumulator has been read
+    uint64_t* dk_free = s_full + 11;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(s_full + 12);
+    int* s_masked = reinterpret_cast<int*>(s_full + 12) + 2;              // [2] some row of the tile does not see all K/V rows
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = p.status;
     if (tid == 0) {
         mbar_init(k_full, 1); mbar_init(k_empty, 1); mbar_init(v_full, 1); mbar_init(v_empty, 1);
         for (int i = 0; i < kRkUnits; ++i) { mbar_init(&u_full[i], 1); mbar_init(&u_empty[i], 2); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&st_full[i], 32); mbar_init(&st_empty[i], 256); }
-        mbar_init(s_full, 1); mbar_init(p_full, 256); mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&st_full[i], 32); mbar_init(&st_empty[i], 256);
+            mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&dp_full[i], 1); mbar_init(&ds_full[i], 128);
+        }
         mbar_init(dv_done, 1); mbar_init(dk_done, 1); mbar_init(dv_free, 128); mbar_init(dk_free, 128);
         mbar_init_fence();
         tma_prefetch_desc(&qmap);
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         // ------------------------------------------------------------------ MMA issuers: warp 1 S and dV, warp 2 dP and dK
         const bool first = warp == 1;
         const bool leader = elect_one();
-        constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, 128, false, false);
+        constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, 64, false, false);
         constexpr uint32_t idesc_acc = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);     // P^T / dS^T (TMEM) x dO / Q (MN-major)
         constexpr uint32_t hi_1024 = umma_desc_hi(1024);
         const uint32_t a_lo = umma_desc_lo(smem_u32(first ? sK : sV), 16);
@@ -302,21 +307,21 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         uint64_t *acc_done = first ? dv_done : dk_done, *acc_free = first ? dv_free : dk_free;
         bool ok = true;
         int c = 0, qi = 0;
-        // S^T (dP^T) of row tile t into its place: in order after the product that read P^T (dS^T) of the tile before from there
-        auto issue_s = [&](int t, bool last) {
+        // S^T (dP^T) of half a row tile t into its place: in order after the product that read P^T (dS^T) of the tile before from there
+        auto issue_s = [&](int t, int half, bool last) {
             const int u = 2 * t + (first ? 0 : 1), st = u % kRkUnits;
-            ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
+            if (half == 0) ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
             tc_fence_after();
             if (leader) {
-                const uint32_t bu = b_lo + (uint32_t)(st * (kRkTile >> 4));
+                const uint32_t bu = b_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t off = (ks >> 2) * (kSlab >> 4) + (ks & 3) * 2;
-                    umma_ss(c_s, umma_desc_pack(a_lo + off, hi_1024), umma_desc_pack(bu + off, hi_1024), idesc_s, ks > 0);
+                    umma_ss(c_s + half * 64, umma_desc_pack(a_lo + off, hi_1024), umma_desc_pack(bu + off, hi_1024), idesc_s, ks > 0);
                 }
-                umma_commit(out_full);
-                umma_commit(&u_empty[st]);
-                if (last) umma_commit(kv_empty);
+                umma_commit(&out_full[half]);
+                if (half) umma_commit(&u_empty[st]);
+                if (half && last) umma_commit(kv_empty);
             }
             __syncwarp();
         };
@@ -324,24 +329,28 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
             const RkItem m = rk_item(p.plan, w);
             if (m.n == 0) continue;
             ok = mbar_wait(kv_full, qi & 1, status) && ok;
-            issue_s(c, m.n == 1);
+            issue_s(c, 0, m.n == 1);
+            issue_s(c, 1, m.n == 1);
             for (int i = 0; i < m.n && ok; ++i, ++c) {
                 const int u = 2 * c + (first ? 1 : 0), st = u % kRkUnits;       // dV takes dO, dK takes Q
                 ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
                 if (i == 0 && qi > 0) ok = mbar_wait(acc_free, (qi - 1) & 1, status) && ok;
-                ok = mbar_wait(in_full, c & 1, status) && ok;
-                tc_fence_after();
-                if (leader) {
-                    const uint32_t bu = b_mn_lo + (uint32_t)(st * (kRkTile >> 4));
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    ok = mbar_wait(&in_full[half], c & 1, status) && ok;
+                    tc_fence_after();
+                    if (leader) {
+                        const uint32_t bu = b_mn_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));
 #pragma unroll
-                    for (int ks = 0; ks < kTileRows / 16; ++ks)     // the two row groups keep their halves 64 columns apart
-                        umma_ts(c_acc, c_s + (ks >> 2) * 64 + (ks & 3) * 8, umma_desc_pack(bu + ks * (2048 >> 4), hi_1024), idesc_acc,
-                                (i > 0 || ks > 0) ? 1u : 0u);
-                    umma_commit(&u_empty[st]);
-                    if (i + 1 == m.n) umma_commit(acc_done);
+                        for (int ks = 0; ks < kTileRows / 32; ++ks)
+                            umma_ts(c_acc, c_s + half * 64 + ks * 8, umma_desc_pack(bu + ks * (2048 >> 4), hi_1024), idesc_acc,
+                                    (i > 0 || half > 0 || ks > 0) ? 1u : 0u);
+                        if (half) umma_commit(&u_empty[st]);
+                        if (half && i + 1 == m.n) umma_commit(acc_done);
+                    }
+                    __syncwarp();
+                    if (i + 1 < m.n) issue_s(c + 1, half, i + 2 == m.n);
                 }
-                __syncwarp();
-                if (i + 1 < m.n) issue_s(c + 1, i + 2 == m.n);
             }
             ++qi;
         }
@@ -370,14 +379,15 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                     }
                 }
                 bool masked = false;
-                uint32_t vis[4];
+                int vis[4][2];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int l = max(lo[j] - m.key0, 0), u = min(hi[j] - m.key0, kTileRows - 1);
                     const bool sees = u >= l && lse[j] > -INFINITY && lse[j] < INFINITY;     // a row that saw nothing in the forward sees nothing here
                     masked |= sees && (l > 0 || u < m.nkeys - 1);
                     if (!sees) { lse[j] = INFINITY; del[j] = 0.f; }                          // exp2(s - inf) = 0
-                    vis[j] = sees ? (uint32_t)l | (uint32_t)(u - l) << 8 : 255u;
+                    vis[j][0] = sees ? l : kTileRows - 1;
+                    vis[j][1] = sees ? u | 128 : 128;
                 }
                 masked = __any_sync(0xffffffffu, masked);
                 const int b = c & 1;
@@ -386,7 +396,8 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 for (int j = 0; j < 4; ++j) {
                     sLse[b * 128 + lane + 32 * j] = lse[j];
                     sDel[b * 128 + lane + 32 * j] = del[j];
-                    sVis[b * 128 + lane + 32 * j] = (uint16_t)vis[j];
+                    sVis[b * 256 + lane + 32 * j] = (uint8_t)vis[j][0];
+                    sVis[b * 256 + 128 + lane + 32 * j] = (uint8_t)vis[j][1];
                 }
                 if (lane == 0) s_masked[b] = masked;
                 mbar_arrive(&st_full[b]);
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
             for (int i = 0; i < m.n && ok; ++i, ++c) {
                 const int b = c & 1;
                 ok = mbar_wait(&st_full[b], (c >> 1) & 1, status) && ok;
-                ok = mbar_wait(s_full, c & 1, status) && ok;
+                ok = mbar_wait(&s_full[grp], c & 1, status) && ok;
                 tc_fence_after();
                 const bool masked = s_masked[b] != 0;
                 const float4* lse4 = reinterpret_cast<const float4*>(sLse + b * 128 + grp * 64);
@@ -427,16 +438,18 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                     v[4 * j + 2] = __float_as_uint(x2); v[4 * j + 3] = __float_as_uint(x3);
                 }
                 if (masked) {
-                    const uint4* vis4 = reinterpret_cast<const uint4*>(sVis + b * 128 + grp * 64);
+                    // four rows at a time: bit 7 of a byte of (128 | key) - first says key >= first, of (128 | last) - key that key <= last
+                    const uint32_t key4 = (uint32_t)key * 0x01010101u;
+                    const uint4* first4 = reinterpret_cast<const uint4*>(sVis + b * 256 + grp * 64);
+                    const uint4* last4 = first4 + 8;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint4 x = vis4[j];
-                        const uint32_t y[4] = {x.x, x.y, x.z, x.w};
+                    for (int j = 0; j < 4; ++j) {
+                        const uint4 f = first4[j], l = last4[j];
+                        const uint32_t seen[4] = {((key4 | 0x80808080u) - f.x) & (l.x - key4), ((key4 | 0x80808080u) - f.y) & (l.y - key4),
+                                                  ((key4 | 0x80808080u) - f.z) & (l.z - key4), ((key4 | 0x80808080u) - f.w) & (l.w - key4)};
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            if ((uint32_t)key - (y[q] & 255u) > ((y[q] >> 8) & 255u)) v[8 * j + 2 * q] = 0u;
-                            if ((uint32_t)key - ((y[q] >> 16) & 255u) > (y[q] >> 24)) v[8 * j + 2 * q + 1] = 0u;
-                        }
+                        for (int q = 0; q < 16; ++q)
+                            if (!(seen[q >> 2] & (0x80u << ((q & 3) * 8)))) v[16 * j + q] = 0u;
                     }
                 }
 #pragma unroll
@@ -444,8 +457,8 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 tmem_st32(tS, pk);
                 tmem_st_wait();
                 tc_fence_before();
-                mbar_arrive(p_full);
-                ok = mbar_wait(dp_full, c & 1, status) && ok;
+                mbar_arrive(&p_full[grp]);
+                ok = mbar_wait(&dp_full[grp], c & 1, status) && ok;
                 tc_fence_after();
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
@@ -465,7 +478,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 }
                 tmem_st_wait();
                 tc_fence_before();
-                mbar_arrive(ds_full);
+                mbar_arrive(&ds_full[grp]);
                 mbar_arrive(&st_empty[b]);
             }
             // ---- epilogue of the item: group 0 dV, group 1 dK
