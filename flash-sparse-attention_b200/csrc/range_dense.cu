@@ -3,19 +3,22 @@
 // nsa_ref/ops/compressed_attention.py:762-829, kernel :33-190) and in the sliding-window branch (replaces the
 // flash_attn_varlen_func call of fsa/module/fsa.py:149-159).
 //
-// One CTA = one tile of <= 128 rows = (query head of a GQA group, TPT consecutive tokens of one sequence) x one KV head.
+// One item = one tile of <= 128 rows = (query head of a GQA group, TPT consecutive tokens of one sequence) x one KV head.
 // The rows of the tile see neighbouring ranges, so the CTA walks the 64-row K/V tiles from the lowest row any of its rows
 // sees to the highest, keeps the output accumulator in TMEM across them (online softmax) and writes o and lse once: no
-// partial rows, no merge kernel, no index.  Two CTAs share an SM (96 KB of shared memory and 256 TMEM columns each), so
-// the softmax of one overlaps the MMAs of the other.
-//   warp 0      TMA producer: the Q tile once (3-D box: column, token, head -> head-major rows), K and V tiles through two
-//               rings of two stages (K is released by the S product, V by the P V product, so K runs a tile ahead);
+// partial rows, no merge kernel, no index.  Two CTAs share an SM (112 KB of shared memory and 256 TMEM columns each), so
+// the softmax of one overlaps the MMAs of the other.  The grid has a CTA per item, but a CTA that runs takes over items whose
+// CTA has not started (cluster launch control), one ahead: finding a tile, its ranges and the first loads take 7200 cycles and
+// the end of an item 4500, as long as seven of its K/V tiles, and run under the item before.  Measured at 1 x 32768 tokens, 32 / 8
+// heads, window of 512 and compressed branch: 788 -> 594 us (a CTA per item before).
+//   warp 0      finds the items; TMA producer: the Q tile (3-D box: column, token, head -> head-major rows), K and V tiles through
+//               two rings of two stages (K is released by the S product, V by the P V product, so K runs a tile ahead);
 //   warp 1      one elected thread issues S(j+1) = Q K^T before the softmax of tile j is done, then O (+)= P(j) V(j);
 //   warps 2..5  one row per thread: scaled logits from TMEM, per-row range mask, running max / sum, P -> TMEM (input dtype,
 //               over S).  The reference max of a row is only raised when a tile exceeds it by more than 2^8 (the final
 //               o = O / l does not depend on the reference); then the warp waits for the previous P V product and
-//               rescales its 32 accumulator rows in TMEM.  Epilogue: o = O / l through swizzled staging (the Q tile's
-//               memory) and a 3-D TMA store, or plain stores for the last, partial tile of a sequence; lse = m + log2 l.
+//               rescales its 32 accumulator rows in TMEM.  Epilogue: o = O / l through swizzled staging, 64 columns at a
+//               time, and 3-D TMA stores, or plain stores for the last, partial tile of a sequence; lse = m + log2 l.
 #include "../../include/fsa_sm100.h"
 #include <climits>
 
@@ -59,12 +62,42 @@ __device__ __forceinline__ float rd_ex2(float x) {
     return y;
 }
 
+// One item: a tile of tokens x one KV head of problem z.
+struct RdItem {
+    int z, h, seq, tok0, ne, row_lo, nblk;
+};
+
+// The K/V rows that a row of the item sees: [x, y].
+__device__ __forceinline__ int2 rd_row(const RangeDenseLaunch& launch, const RdItem& m, bool valid, int e) {
+    if (m.z < 0 || !valid) return make_int2(0, -1);
+    const RangeDenseParams& p = launch.p[m.z];
+    return make_int2(p.kv_lo ? __ldg(p.kv_lo + m.tok0 + e) : __ldg(p.cu_k + m.seq), __ldg(p.kv_hi + m.tok0 + e));
+}
+
+// Takes over a CTA of this launch that has not started yet (cluster launch control): 16 bytes of answer at dst, with bar as the
+// transaction barrier.  Not to be called again once the answer was no.
+__device__ __forceinline__ void claim_next_cta(uint32_t dst, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst),
+                 "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool claimed_cta(uint32_t src, int& x, int& y, int& z) {
+    uint32_t yes, cx, cy, cz;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+        "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+        "ld.shared.b128 a, [%4];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, a;\n\t}"
+        : "=r"(yes), "=r"(cx), "=r"(cy), "=r"(cz) : "r"(src) : "memory");
+    x = (int)cx; y = (int)cy; z = (int)cz;
+    return yes != 0;
+}
+
 template <int D, typename ET>
 __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_constant__ RangeDenseLaunch launch) {
-    const RangeDenseParams& p = launch.p[blockIdx.z];
-    const CUtensorMap &qmap = launch.q[blockIdx.z], &kmap = launch.k[blockIdx.z], &vmap = launch.v[blockIdx.z], &omap = launch.o[blockIdx.z];
     constexpr int BK = kRdBK;
-    constexpr int kQ = kTileRows * D * 2;            // Q tile, later the output staging
+    constexpr int kQ = kTileRows * D * 2;
     constexpr int kKt = BK * D * 2;                  // one K (or V) tile
     constexpr int KH = D / 64;
     constexpr uint32_t kCols = (2 * BK + D) <= 128 ? 128 : 256;
@@ -73,7 +106,8 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + kQ;
     uint8_t* sV = sK + 2 * kKt;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kKt);
+    uint8_t* sOut = sV + 2 * kKt;                    // 64 output columns on their way out
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + kTileRows * 128);
     uint64_t* q_full = bars;            // [1]
     uint64_t* k_full = bars + 1;        // [2]
     uint64_t* k_empty = bars + 3;       // [2]
@@ -84,14 +118,21 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
     // [2] P V of the even / odd tiles done.  Two, because a row warp may be two products ahead: it can finish the last softmax
     // before the product of the tile before has been issued, and one barrier's parity cannot tell that product from its own
     uint64_t* pv_done = bars + 13;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 15);
-    int* s_meta = reinterpret_cast<int*>(bars + 16);     // [0] sequence, [1] first token, [2] tokens, [3] first K/V row, [4] K/V tiles
+    uint64_t* q_empty = bars + 15;      // the item's last S product is done
+    uint64_t* o_free = bars + 16;       // the 128 row threads have read an item's accumulator
+    uint64_t* it_full = bars + 17;      // the next item is known
+    uint64_t* it_empty = bars + 18;     // ... has been taken by the five other warps
+    uint64_t* claim = bars + 19;        // the answer to a claim has arrived
+    int* s_claim = reinterpret_cast<int*>(bars + 20);    // 16 bytes
+    int4* s_item = reinterpret_cast<int4*>(bars + 22);   // [2 items][2]
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 30);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int* status = p.status;
-    const int h = blockIdx.y;
+    int* status = launch.p[blockIdx.z].status;
+    const int G = launch.p[0].G, TPT = launch.p[0].TPT;      // (the same for all problems)
     if (tid == 0) {
-        mbar_init(q_full, 1);
+        mbar_init(q_full, 1); mbar_init(q_empty, 1); mbar_init(o_free, 128);
+        mbar_init(it_full, 1); mbar_init(it_empty, 5); mbar_init(claim, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
             mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
@@ -99,113 +140,155 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             mbar_init(&pv_done[i], 1);
         }
         mbar_init_fence();
-        tma_prefetch_desc(&qmap);
-        tma_prefetch_desc(&kmap);
-        tma_prefetch_desc(&vmap);
-        tma_prefetch_desc(&omap);
     }
-    if (warp == 0) {
-        // which tile is this: the heaviest (last) tiles of the list start first
-        const int total = count_seq_tiles(p.cu_q, p.B, p.TPT, lane);
-        int seq, tok0, ne;
-        find_seq_tile(p.cu_q, p.B, p.TPT, total - 1 - (int)blockIdx.x, lane, seq, tok0, ne);
-        // lowest and highest K/V row any token of the tile sees
-        int lo = INT_MAX, hi = -1;
-        if (seq >= 0) {
-            const int k0 = __ldg(p.cu_k + seq);
-            for (int e = lane; e < ne; e += 32) {
-                const int l = p.kv_lo ? __ldg(p.kv_lo + tok0 + e) : k0;
-                const int u = __ldg(p.kv_hi + tok0 + e);
-                if (u >= l) { lo = min(lo, l); hi = max(hi, u); }
-            }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
-        }
-        if (lane == 0) {
-            lo = max(lo, 0);
-            hi = min(hi, (int)p.Nk - 1);
-            s_meta[0] = seq; s_meta[1] = tok0; s_meta[2] = ne; s_meta[3] = lo;
-            s_meta[4] = hi >= lo ? (hi - lo) / BK + 1 : 0;
-        }
-        tmem_alloc(&tmem_slot, kCols);
-    }
+    if (warp == 0) tmem_alloc(&tmem_slot, kCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = tmem_slot;
-    const int seq = s_meta[0], tok0 = s_meta[1], ne = s_meta[2], row_lo = s_meta[3], nblk = s_meta[4];
+    // Item n of this CTA.  Each of the five other warps takes every item once, in order; z < 0 ends the list.
+    auto read_item = [&](int n) {
+        const int4 x = s_item[(n & 1) * 2], y = s_item[(n & 1) * 2 + 1];
+        RdItem m;
+        m.z = x.x; m.h = x.y; m.seq = x.z; m.tok0 = x.w;
+        m.ne = y.x; m.row_lo = y.y; m.nblk = y.z;
+        return m;
+    };
+    auto take_item = [&](int n, bool& ok) {
+        ok = mbar_wait(it_full, n & 1, status) && ok;
+        RdItem m = read_item(n);
+        if (!ok) m.z = -1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(it_empty);
+        return m;
+    };
 
-    if (seq >= 0) {
-        if (warp == 0) {
-            // ------------------------------------------------------------------ TMA producer
-            bool ok = true;
-            if (lane == 0 && nblk > 0) {
-                mbar_expect_tx(q_full, (uint32_t)(KH * 128 * p.TPT * p.G));
-#pragma unroll
-                for (int b = 0; b < KH; ++b) tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &qmap, b * 64, tok0, h * p.G, q_full);
-            }
-            // K tile j and V tile j are loaded in the order the MMA warp needs them: K(0), K(1), V(0), K(2), V(1), ...
-            for (int step = 0; step < nblk + 1 && ok; ++step) {
-                if (lane == 0) {
-                    const int jk = step, jv = step - 1;
-                    if (jk < nblk) {
-                        const int st = jk & 1;
-                        ok = mbar_wait(&k_empty[st], ((jk >> 1) & 1) ^ 1, status) && ok;
-                        mbar_expect_tx(&k_full[st], (uint32_t)kKt);
-#pragma unroll
-                        for (int b = 0; b < KH; ++b)
-                            tma_load_2d(smem_u32(sK + st * kKt + b * (BK * 128)), &kmap, h * D + b * 64, row_lo + jk * BK, &k_full[st]);
-                    }
-                    if (jv >= 0) {
-                        const int st = jv & 1;
-                        ok = mbar_wait(&v_empty[st], ((jv >> 1) & 1) ^ 1, status) && ok;
-                        mbar_expect_tx(&v_full[st], (uint32_t)kKt);
-#pragma unroll
-                        for (int b = 0; b < KH; ++b)
-                            tma_load_2d(smem_u32(sV + st * kKt + b * (BK * 128)), &vmap, h * D + b * 64, row_lo + jv * BK, &v_full[st]);
-                    }
-                }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            }
-        } else if (warp == 1) {
-            // ------------------------------------------------------------------ MMA issuer
-            const bool leader = elect_one();
-            constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, BK, false, false);
-            constexpr uint32_t idesc_o = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
-            constexpr uint32_t hi_1024 = umma_desc_hi(1024);
-            const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16);
-            const uint32_t k_lo = umma_desc_lo(smem_u32(sK), 16);
-            const uint32_t v_lo = umma_desc_lo(smem_u32(sV), BK * 128);     // MN-major: LBO = slab stride
-            bool ok = true;
-            auto issue_s = [&](int j) {
-                const int st = j & 1;
-                ok = mbar_wait(&k_full[st], (j >> 1) & 1, status) && ok;
-                tc_fence_after();
-                if (leader) {
-                    constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
-                    const uint32_t b_lo = k_lo + (uint32_t)(st * (kKt >> 4));
-#pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        umma_ss(tbase + cS + st * BK, umma_desc_pack(q_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
-                                umma_desc_pack(b_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
-                    umma_commit(&k_empty[st]);
-                    umma_commit(&s_full[st]);
-                }
-                __syncwarp();
+    if (warp == 0) {
+        // ------------------------------------------------------------------ items and TMA producer
+        bool ok = true;
+        int n = 0, claims = 0, qi = 0, c = 0;           // items, claims, non-empty items, K/V tiles so far
+        int bx = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
+        while (ok) {
+            const RangeDenseParams& p = launch.p[z];
+            bool asked = false;
+            auto ask = [&]() {
+                mbar_expect_tx(claim, 16);
+                claim_next_cta(smem_u32(s_claim), claim);
+                asked = true;
             };
-            if (nblk > 0) {
-                ok = mbar_wait(q_full, 0, status) && ok;
-                issue_s(0);
+            // which tile is this: the heaviest (last) tiles of the list start first
+            const int total = count_seq_tiles(p.cu_q, p.B, TPT, lane);
+            int seq, tok0, ne;
+            find_seq_tile(p.cu_q, p.B, TPT, total - 1 - bx, lane, seq, tok0, ne);
+            if (seq >= 0) {
+                // lowest and highest K/V row any token of the tile sees
+                int lo = INT_MAX, hi = -1;
+                const int k0 = __ldg(p.cu_k + seq);
+                for (int e = lane; e < ne; e += 32) {
+                    const int l = p.kv_lo ? __ldg(p.kv_lo + tok0 + e) : k0;
+                    const int u = __ldg(p.kv_hi + tok0 + e);
+                    if (u >= l) { lo = min(lo, l); hi = max(hi, u); }
+                }
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) {
+                    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+                    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+                }
+                lo = max(lo, 0);
+                hi = min(hi, (int)p.Nk - 1);
+                const int nblk = hi >= lo ? (hi - lo) / BK + 1 : 0;
+                if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+                if (lane == 0) {
+                    s_item[(n & 1) * 2] = make_int4(z, h, seq, tok0);
+                    s_item[(n & 1) * 2 + 1] = make_int4(ne, lo, nblk, 0);
+                    mbar_arrive(it_full);
+                }
+                ++n;
+                if (lane == 0 && nblk > 0) {
+                    const CUtensorMap *kmap = &launch.k[z], *vmap = &launch.v[z];
+                    ok = mbar_wait(q_empty, (qi & 1) ^ 1, status) && ok;
+                    ask();                  // not earlier: a CTA is to be one item ahead, not to take the share of others
+                    mbar_expect_tx(q_full, (uint32_t)(KH * 128 * TPT * G));
+#pragma unroll
+                    for (int b = 0; b < KH; ++b) tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &launch.q[z], b * 64, tok0, h * G, q_full);
+                    // K tile j and V tile j are loaded in the order the MMA warp needs them: K(0), K(1), V(0), K(2), V(1), ...
+                    for (int step = 0; step < nblk + 1 && ok; ++step) {
+                        const int jk = c + step, jv = jk - 1;
+                        if (step < nblk) {
+                            const int st = jk & 1;
+                            ok = mbar_wait(&k_empty[st], ((jk >> 1) & 1) ^ 1, status) && ok;
+                            mbar_expect_tx(&k_full[st], (uint32_t)kKt);
+#pragma unroll
+                            for (int b = 0; b < KH; ++b)
+                                tma_load_2d(smem_u32(sK + st * kKt + b * (BK * 128)), kmap, h * D + b * 64, lo + step * BK, &k_full[st]);
+                        }
+                        if (step > 0) {
+                            const int st = jv & 1;
+                            ok = mbar_wait(&v_empty[st], ((jv >> 1) & 1) ^ 1, status) && ok;
+                            mbar_expect_tx(&v_full[st], (uint32_t)kKt);
+#pragma unroll
+                            for (int b = 0; b < KH; ++b)
+                                tma_load_2d(smem_u32(sV + st * kKt + b * (BK * 128)), vmap, h * D + b * 64, lo + (step - 1) * BK, &v_full[st]);
+                        }
+                    }
+                }
+                c += nblk;
+                qi += nblk > 0;
             }
-            for (int j = 0; j < nblk && ok; ++j) {
-                const int st = j & 1;
-                // S(j + 1) overwrites the buffer P(j - 1) was read from by the product issued one iteration ago (in order)
-                if (j + 1 < nblk) issue_s(j + 1);
-                ok = mbar_wait(&p_full[st], (j >> 1) & 1, status) && ok;
-                ok = mbar_wait(&v_full[st], (j >> 1) & 1, status) && ok;
+            if (lane == 0 && !asked) ask();
+            // (the answer is in shared memory before this CTA may end, whatever happened above)
+            ok = mbar_wait(claim, claims & 1, status) && ok;
+            ++claims;
+            const bool more = claimed_cta(smem_u32(s_claim), bx, h, z);
+            ok = __all_sync(0xffffffffu, ok);
+            fence_async_smem();
+            if (!more) break;
+        }
+        if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+        if (lane == 0) {
+            s_item[(n & 1) * 2] = make_int4(-1, 0, -1, 0);
+            s_item[(n & 1) * 2 + 1] = make_int4(0, 0, 0, 0);
+            mbar_arrive(it_full);
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        const bool leader = elect_one();
+        constexpr uint32_t idesc_s = umma_idesc(ElemTraits<ET>::kIsBF16, 128, BK, false, false);
+        constexpr uint32_t idesc_o = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
+        constexpr uint32_t hi_1024 = umma_desc_hi(1024);
+        const uint32_t q_lo = umma_desc_lo(smem_u32(sQ), 16);
+        const uint32_t k_lo = umma_desc_lo(smem_u32(sK), 16);
+        const uint32_t v_lo = umma_desc_lo(smem_u32(sV), BK * 128);     // MN-major: LBO = slab stride
+        bool ok = true;
+        int n = 0, qi = 0, c = 0;
+        auto issue_s = [&](int t, bool last) {
+            const int st = t & 1;
+            ok = mbar_wait(&k_full[st], (t >> 1) & 1, status) && ok;
+            tc_fence_after();
+            if (leader) {
+                constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
+                const uint32_t b_lo = k_lo + (uint32_t)(st * (kKt >> 4));
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ss(tbase + cS + st * BK, umma_desc_pack(q_lo + (ks >> 2) * kSlabA + (ks & 3) * 2, hi_1024),
+                            umma_desc_pack(b_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc_s, ks > 0);
+                umma_commit(&k_empty[st]);
+                umma_commit(&s_full[st]);
+                if (last) umma_commit(q_empty);
+            }
+            __syncwarp();
+        };
+        for (RdItem m = take_item(n, ok); m.z >= 0; m = take_item(++n, ok)) {
+            if (m.nblk == 0) continue;
+            ok = mbar_wait(q_full, qi & 1, status) && ok;
+            issue_s(c, m.nblk == 1);
+            for (int j = 0; j < m.nblk && ok; ++j, ++c) {
+                const int st = c & 1;
+                // S(c + 1) overwrites the buffer P(c - 1) was read from by the product issued one iteration ago (in order)
+                if (j + 1 < m.nblk) issue_s(c + 1, j + 2 == m.nblk);
+                if (j == 0 && qi > 0) ok = mbar_wait(o_free, (qi - 1) & 1, status) && ok;
+                ok = mbar_wait(&p_full[st], (c >> 1) & 1, status) && ok;
+                ok = mbar_wait(&v_full[st], (c >> 1) & 1, status) && ok;
                 tc_fence_after();
                 if (leader) {
                     const uint32_t b_lo = v_lo + (uint32_t)(st * (kKt >> 4));
@@ -218,35 +301,41 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 }
                 __syncwarp();
             }
-        } else {
-            // ------------------------------------------------------------------ softmax and epilogue: one row per thread
-            const int quarter = warp & 3;
-            const int r = quarter * 32 + lane;
-            const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-            const int g = r / p.TPT, e = r - g * p.TPT;
-            const bool row_valid = g < p.G && e < ne;
-            const int tok = tok0 + e;
-            int lo_r = 0, hi_r = -1;
-            if (row_valid) {
-                lo_r = p.kv_lo ? __ldg(p.kv_lo + tok) : __ldg(p.cu_k + seq);
-                hi_r = min(__ldg(p.kv_hi + tok), (int)p.Nk - 1);     // rows past the end of K/V do not exist
-            }
+            ++qi;
+        }
+    } else {
+        // ------------------------------------------------------------------ softmax and epilogue: one row per thread
+        const int quarter = warp & 3;
+        const int r = quarter * 32 + lane;
+        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+        const int g = r / TPT, e = r - g * TPT;
+        bool ok = true;
+        int n = 0, c = 0;
+        RdItem m = take_item(n, ok);
+        int2 sees = rd_row(launch, m, g < G && e < m.ne, e);
+        // (the four warps leave the loop together: they meet at barriers in it)
+        for (ok = bar_all(1, 128, ok); ok && m.z >= 0;) {
+            const float scale_log2 = launch.p[0].scale_log2;                 // (the same for all problems)
+            const int lo_r = sees.x - m.row_lo, hi_r = min(sees.y, (int)launch.p[m.z].Nk - 1) - m.row_lo;      // rows past the end of K/V do not exist
+            const int nblk = m.nblk;
             float m_ref = -INFINITY, l_run = 0.f;
-            bool ok = true;
-            for (int j = 0; j < nblk && ok; ++j) {
-                const int st = j & 1;
-                const int R0 = row_lo + j * BK;
-                const int c_lo = max(0, lo_r - R0), c_hi = min(BK, hi_r - R0 + 1);      // visible columns [c_lo, c_hi)
-                ok = mbar_wait(&s_full[st], (j >> 1) & 1, status) && ok;
+            for (int j = 0; j < nblk && ok; ++j, ++c) {
+                const int st = c & 1;
+                const int c_lo = max(0, lo_r - j * BK), c_hi = min(BK, hi_r - j * BK + 1);      // visible columns [c_lo, c_hi)
+                ok = mbar_wait(&s_full[st], (c >> 1) & 1, status) && ok;
                 tc_fence_after();
                 uint32_t v[BK];
                 tmem_ld32(tbase + lane_off + cS + st * BK, *reinterpret_cast<uint32_t (*)[32]>(&v[0]));
                 tmem_ld32(tbase + lane_off + cS + st * BK + 32, *reinterpret_cast<uint32_t (*)[32]>(&v[32]));
                 tmem_ld_wait();
                 if (c_lo > 0 || c_hi < BK) {
+                    // bit i: column i is seen
+                    const int v_hi = max(c_hi, 0), v_lo = min(c_lo, BK);
+                    const uint64_t vis = v_hi > v_lo ? (~0ull >> (BK - v_hi + v_lo)) << v_lo : 0ull;
+                    const uint32_t vis2[2] = {(uint32_t)vis, (uint32_t)(vis >> 32)};
 #pragma unroll
                     for (int i = 0; i < BK; ++i)
-                        if (i < c_lo || i >= c_hi) v[i] = 0xff800000u;      // -inf: exp2 gives exactly 0
+                        if (!(vis2[i >> 5] >> (i & 31) & 1u)) v[i] = 0xff800000u;      // -inf: exp2 gives exactly 0
                 }
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -256,7 +345,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                     mx[2] = fmaxf(mx[2], __uint_as_float(v[i + 2]));
                     mx[3] = fmaxf(mx[3], __uint_as_float(v[i + 3]));
                 }
-                const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+                const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
                 // raise the reference only when this tile exceeds it by a lot; the first finite maximum sets it
                 float alpha = 1.f;
                 const bool raise = m_blk > m_ref + kRdLazy;     // false when m_blk is -inf; true when m_ref is -inf and m_blk finite
@@ -267,7 +356,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 // accumulator rows already hold products (j > 0): rescale them when any row of the warp changes reference
                 const bool scale_acc = __any_sync(0xffffffffu, raise && j > 0);
                 if (scale_acc) {
-                    ok = mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, status) && ok;
+                    ok = mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status) && ok;
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < D; c0 += 32) {
@@ -285,10 +374,10 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 uint32_t pk[BK / 2];
 #pragma unroll
                 for (int i = 0; i < BK; i += 4) {
-                    const float p0 = rd_ex2(fmaf(__uint_as_float(v[i]), p.scale_log2, -m_use));
-                    const float p1 = rd_ex2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -m_use));
-                    const float p2 = rd_ex2(fmaf(__uint_as_float(v[i + 2]), p.scale_log2, -m_use));
-                    const float p3 = rd_ex2(fmaf(__uint_as_float(v[i + 3]), p.scale_log2, -m_use));
+                    const float p0 = rd_ex2(fmaf(__uint_as_float(v[i]), scale_log2, -m_use));
+                    const float p1 = rd_ex2(fmaf(__uint_as_float(v[i + 1]), scale_log2, -m_use));
+                    const float p2 = rd_ex2(fmaf(__uint_as_float(v[i + 2]), scale_log2, -m_use));
+                    const float p3 = rd_ex2(fmaf(__uint_as_float(v[i + 3]), scale_log2, -m_use));
                     ls[0] += p0; ls[1] += p1; ls[2] += p2; ls[3] += p3;
                     pk[i >> 1] = ElemTraits<ET>::pack2(p0, p1);
                     pk[(i >> 1) + 1] = ElemTraits<ET>::pack2(p2, p3);
@@ -299,25 +388,40 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 tc_fence_before();
                 mbar_arrive(&p_full[st]);
             }
+            m = read_item(n);
+            const RangeDenseParams& p = launch.p[m.z];
+            const bool row_valid = g < G && e < m.ne;
+            const int tok = m.tok0 + e;
+            // the next item's numbers arrive under this item's epilogue
+            const RdItem next = take_item(++n, ok);
+            sees = rd_row(launch, next, g < G && e < next.ne, e);
             // ---- epilogue
-            if (nblk > 0) {
-                ok = mbar_wait(&pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status) && ok;
+            if (m.nblk > 0) {
+                ok = mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status) && ok;
                 tc_fence_after();
             }
+            ok = bar_all(1, 128, ok);
             const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-            if (row_valid && ok) p.lse[(int64_t)(h * p.G + g) * p.N + tok] = l_run > 0.f ? m_ref + log2f(l_run) : -INFINITY;
-            const bool full_tile = ne == p.TPT && p.G * p.TPT == kTileRows;      // whole box inside the sequence, every row staged
-            uint8_t* my_stage = sQ + quarter * (32 * 128);     // per 64-column slab: rows of this warp at (slab base) + 32 * 128 * quarter
-            ET* orow = reinterpret_cast<ET*>(p.o) + (int64_t)tok * p.o_sn + (int64_t)(h * p.G + g) * p.o_sh;
+            if (row_valid && ok) p.lse[(int64_t)(m.h * G + g) * p.N + tok] = l_run > 0.f ? m_ref + log2f(l_run) : -INFINITY;
+            const bool full_tile = m.ne == TPT && G * TPT == kTileRows;      // whole box inside the sequence, every row staged
+            ET* orow = reinterpret_cast<ET*>(p.o) + (int64_t)tok * p.o_sn + (int64_t)(m.h * G + g) * p.o_sh;
 #pragma unroll
             for (int c0 = 0; c0 < D; c0 += 32) {
                 uint32_t a[32];
-                if (nblk > 0) {
+                if (m.nblk > 0) {
                     tmem_ld32(tbase + lane_off + cO + c0, a);
                     tmem_ld_wait();
+                    if (c0 + 32 == D) {
+                        tc_fence_before();
+                        mbar_arrive(o_free);            // the accumulator may take the next item
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) a[i] = 0u;
+                }
+                if (full_tile && c0 % 64 == 0) {        // the columns before have left the staging memory
+                    if (quarter == 0 && lane == 0) bulk_wait_read0();
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
@@ -326,27 +430,22 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                     x.y = ElemTraits<ET>::pack2(__uint_as_float(a[q4 * 8 + 2]) * inv_l, __uint_as_float(a[q4 * 8 + 3]) * inv_l);
                     x.z = ElemTraits<ET>::pack2(__uint_as_float(a[q4 * 8 + 4]) * inv_l, __uint_as_float(a[q4 * 8 + 5]) * inv_l);
                     x.w = ElemTraits<ET>::pack2(__uint_as_float(a[q4 * 8 + 6]) * inv_l, __uint_as_float(a[q4 * 8 + 7]) * inv_l);
-                    const int chunk = (c0 >> 3) + q4;
-                    if (full_tile) {
-                        *reinterpret_cast<uint4*>(sQ + (chunk >> 3) * (kTileRows * 128) + sw128_chunk_off(r, chunk & 7)) = x;
-                    } else if (row_valid && ok) {
-                        *reinterpret_cast<uint4*>(orow + chunk * 8) = x;
+                    if (full_tile) *reinterpret_cast<uint4*>(sOut + sw128_chunk_off(r, (c0 % 64) / 8 + q4)) = x;
+                    else if (row_valid && ok) *reinterpret_cast<uint4*>(orow + c0 + q4 * 8) = x;
+                }
+                if (full_tile && c0 % 64 == 32) {
+                    // all four warps have staged their rows: one 3-D store of 64 columns
+                    fence_async_smem();
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (quarter == 0 && lane == 0) {
+                        if (ok) tma_store_3d(&launch.o[m.z], c0 - 32, m.tok0, m.h * G, smem_u32(sOut));
+                        bulk_commit();
                     }
                 }
             }
-            (void)my_stage;
-            if (full_tile) {
-                // all four warps have staged their rows: one 3-D store per 64-column slab
-                fence_async_smem();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == 2 && lane == 0 && ok) {
-#pragma unroll
-                    for (int b = 0; b < KH; ++b) tma_store_3d(&omap, b * 64, tok0, h * p.G, smem_u32(sQ + b * (kTileRows * 128)));
-                    bulk_commit();
-                    bulk_wait_read0();     // the staging memory has been read; the global writes complete on their own
-                }
-            }
+            m = next;
         }
+        if (quarter == 0 && lane == 0) bulk_wait_read0();      // the last columns have left shared memory
     }
     tc_fence_before();
     __syncthreads();
@@ -355,7 +454,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
 
 template <int D, typename ET>
 static cudaError_t launch_rd(const RangeDenseLaunch& l, int num, int max_tiles, cudaStream_t stream) {
-    constexpr int smem = kTileRows * D * 2 + 4 * kRdBK * D * 2 + 256;
+    constexpr int smem = kTileRows * D * 2 + 4 * kRdBK * D * 2 + kTileRows * 128 + 256;
     auto kern = range_fwd_dense<D, ET>;
     cudaError_t e = allow_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
@@ -664,6 +763,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             if (m.nblk > 0) take_row();
         }
         Row row = load_numbers(m);
+        ok = bar_all(3, 256, ok);       // (the eight warps enter the loop together: they meet at barriers in it)
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
             const bool row_valid = g < p.G && e < m.ne;
             const int tok = m.tok0 + e;

@@ -138,6 +138,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     return false;
 }
 
+// Barrier `id` of `threads` threads that tells whether v held for all of them.
+__device__ __forceinline__ bool bar_all(int id, int threads, bool v) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all) : "r"((uint32_t)v), "r"(id), "r"(threads) : "memory");
+    return all != 0;
+}
+
 // ---------------------------------------------------------------- proxies / fences
 // Generic-proxy writes to shared memory (st.shared, cp.async) must be made visible to the
 // async proxy (TMA, tcgen05.mma operand reads) before those engines read them.
