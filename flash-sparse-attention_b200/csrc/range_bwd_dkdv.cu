@@ -19,9 +19,9 @@
 // compressed rows are seen by the whole sequence): a plan on the device cuts the stretches so that an SM gets about eight.  The
 // parts of a K/V tile that was cut go to fp32 slabs that the last kernel adds in order (bit-reproducible); others are written in place.
 // A tile takes 3100 cycles where every row sees all K/V rows: its products read 256 KB of shared memory and the loads write 64 KB,
-// 2560 cycles (the products alone: 2050).  Tiles that need the mask are bound by the row threads (4700).  Measured at 2 x 32768
-// tokens, 32 / 8 heads (window of 512 and compressed branch together): whole tiles in turns 4.19 ms, halves 3.93; at 8 sequences
-// of about 1000 tokens 119 -> 108 us.
+// 2560 cycles (the products alone: 2050).  Tiles that need the mask are bound by the row threads.  Measured at 2 x 32768
+// tokens, 32 / 8 heads (window of 512 and compressed branch together): whole tiles in turns 4.19 ms, halves 3.93; at four sequences
+// of 777 to 3001 tokens, 16 / 4 heads, 119 -> 106 us.
 #include "../../include/fsa_sm100.h"
 #include <climits>
 
