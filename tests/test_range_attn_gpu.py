@@ -1,5 +1,7 @@
 """Compressed-branch and sliding-window attention on the GPU against the CPU oracle.
 Tolerances as in test_sel_attn_gpu.py (bf16 in/out vs fp32 oracle)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -276,3 +278,54 @@ def test_random_shapes_forward_backward(seed):
     _tol_ok(qc.grad, dq_ref, "dq " + tag)
     _tol_ok(kc.grad, dk_ref, "dk " + tag)
     _tol_ok(vc.grad, dv_ref, "dv " + tag)
+
+
+class _Problem(ctypes.Structure):       # fsa_range_problem
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("q", "k", "v", "cu_q", "cu_k", "kv_lo", "kv_hi")] + [(n, ctypes.c_int64) for n in ("N", "Nk", "q_sn", "q_sh", "k_sn", "v_sn")]
+                + [("o", ctypes.c_void_p), ("o_sn", ctypes.c_int64), ("o_sh", ctypes.c_int64), ("lse", ctypes.c_void_p), ("status", ctypes.c_void_p)])
+
+
+@pytest.mark.parametrize("d,G", [(128, 4), (64, 4), (128, 3)])
+def test_items_do_not_depend_on_who_computes_them(d, G):
+    """Three problems in one launch, with several times as many items as CTAs run at once (CTAs take items over; the dQ kernel
+    walks a list): the same bits as a launch per sequence and problem, which has an SM's room for every item.  Ranges that
+    are empty for single tokens and for whole tiles, partial tiles, a sequence of one token."""
+    from fsa import _lib
+    from fsa.ops.range_attention import range_attention
+
+    lens, Hk = [4000, 1, 2500, 63, 3000], 2
+    N = sum(lens)
+    g = torch.Generator().manual_seed(d + G)
+    q, do = (torch.randn(N, Hk * G, d, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    k, v = (torch.randn(N, Hk, d, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    cu = make_cu_seqlens(lens)
+    first = torch.repeat_interleave(cu[:-1], torch.tensor(lens)).to(torch.int32)
+    tok = torch.arange(N, dtype=torch.int32)
+    near, far = torch.maximum(tok - 300, first), first + (tok - first) // 3       # at most 22 blocks of 64 rows
+    gaps = tok.clone()
+    gaps[500:900] = -1
+    gaps[torch.rand(N, generator=g) < 0.1] = -1
+    ranges = [(near, tok), (None, far), (near, gaps)]
+    ranges = [(None if lo is None else lo.to(DEV), hi.to(DEV)) for lo, hi in ranges]
+    cud = cu.to(DEV)
+    outs = [(torch.empty_like(q), torch.empty(Hk * G, N, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)) for _ in ranges]
+    problems = (_Problem * 3)(*[
+        _Problem(*(_lib.ptr(t) for t in (q, k, v, cud, cud, lo, hi)), N, N, q.stride(0), q.stride(1), k.stride(0), v.stride(0),
+                 _lib.ptr(o), o.stride(0), o.stride(1), _lib.ptr(lse), _lib.ptr(st)) for (lo, hi), (o, lse, st) in zip(ranges, outs)])
+    rc = _lib.lib().fsa_range_attn_fwd_dense_several(3, ctypes.byref(problems), len(lens), Hk * G, Hk, d, _lib.DTYPE_CODE[q.dtype], d ** -0.5,
+                                                     _lib.current_stream(q.device))
+    assert rc == 0
+    for (lo, hi), (o, lse, st) in zip(ranges, outs):
+        assert int(st[0]) == 0
+        qa = q.clone().requires_grad_(True)
+        oa, lsea = range_attention(qa, k, v, cud, cud, lo, hi, 24)
+        oa.backward(do)
+        assert torch.equal(oa, o) and torch.equal(lsea, lse)
+        for a, n in zip(cu[:-1].tolist(), lens):
+            qs = q[a : a + n].clone().requires_grad_(True)
+            c1 = make_cu_seqlens([n]).to(DEV)
+            os_, lses = range_attention(qs, k[a : a + n], v[a : a + n], c1, c1, None if lo is None else lo[a : a + n] - a, hi[a : a + n] - a, 24)
+            os_.backward(do[a : a + n])
+            assert torch.equal(os_, o[a : a + n]) and torch.equal(lses, lse[:, a : a + n])
+            if d == 128:
+                assert torch.equal(qs.grad, qa.grad[a : a + n])
