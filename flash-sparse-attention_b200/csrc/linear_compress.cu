@@ -17,7 +17,8 @@
 //
 // The reduction over ks * d is one serial chain of MMAs behind a ring of loads: 26 us at ks * d = 4096 however few windows
 // there are.  When short sequences leave SMs idle the chain is cut in up to eight, one CTA of a cluster each, whose fp32 sums meet
-// through distributed shared memory (517 tokens, 8 heads, K and V, inside a layer: 19 us for both, two launches of 26 us before).  One launch takes up to
+// through distributed shared memory (517 tokens, 8 heads, K and V, inside a layer: 11 us for both; two launches of 26 us before; 19 us with
+// six stages, an SM for every CTA, and the sums read one after the other).  One launch takes up to
 // kLcSeqs sequences, whose tensor maps travel as kernel parameters.
 #include "../../include/fsa_sm100.h"
 #include <cooperative_groups.h>
@@ -30,7 +31,7 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int64_t rows, i
 int make_tile_map_3d(CUtensorMap* map, const void* base, int dtype, int64_t d0, int64_t d1, int64_t d2, int64_t stride1,
                      int64_t stride2, int box1);
 
-constexpr int kLcStages = 6, kLcSeqs = 12, kLcTensors = 2, kLcSplits = 8, kLcShort = 64;
+constexpr int kLcStages = 6, kLcStagesSplit = 3, kLcSeqs = 12, kLcTensors = 2, kLcSplits = 8, kLcShort = 64;
 
 struct LcMaps {
     CUtensorMap a[kLcTensors][kLcSeqs];      // overlapping windows of every sequence
@@ -48,22 +49,22 @@ struct LcParams {
 };
 static_assert(sizeof(LcMaps) + sizeof(LcParams) <= 4096, "kernel parameters");
 
-template <int D, typename ET>
+template <int D, typename ET, int ST>
 __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_constant__ LcMaps maps, const LcParams p) {
     namespace cg = cooperative_groups;
     constexpr int kA = 128 * 128, kB = 64 * D * 2;        // one stage: 128 windows x 64 columns, 64 weight rows x D columns
     constexpr int kSlabsPerK = D / 64;
     constexpr int kPitch = D + 4;                         // floats per row of a partial tile (16-byte aligned, fewer bank conflicts)
-    static_assert(128 * kPitch * 4 <= kLcStages * (kA + kB), "the partial tile reuses the ring");
+    static_assert(128 * kPitch * 4 <= ST * (kA + kB), "the partial tile reuses the ring");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sA = smem;
-    uint8_t* sB = sA + kLcStages * kA;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kLcStages * kB);
+    uint8_t* sB = sA + ST * kA;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sB + ST * kB);
     uint64_t* full = bars;                  // [stages]
-    uint64_t* empty = bars + kLcStages;     // [stages]
-    uint64_t* acc_full = bars + 2 * kLcStages;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 2 * kLcStages + 1);
-    float* s_bias = reinterpret_cast<float*>(bars + 2 * kLcStages + 2);      // [D] rounded to the activation dtype
+    uint64_t* empty = bars + ST;     // [stages]
+    uint64_t* acc_full = bars + 2 * ST;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
+    float* s_bias = reinterpret_cast<float*>(bars + 2 * ST + 2);      // [D] rounded to the activation dtype
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = (int)gridDim.x, rank = (int)blockIdx.x;            // CTAs that share the reduction (= cluster size), this one
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
     const CUtensorMap* wmap = &maps.w[tn];
     int* status = p.status;
     if (tid == 0) {
-        for (int i = 0; i < kLcStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < ST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_init(acc_full, 1);
         mbar_init_fence();
         tma_prefetch_desc(amap);
@@ -94,9 +95,9 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
     if (warp == 0) {
         // ---- producer
         for (int i = 0; i < nslab && ok; ++i) {
-            const int st = i % kLcStages;
+            const int st = i % ST;
             if (lane == 0) {
-                ok = mbar_wait(&empty[st], ((i / kLcStages) & 1) ^ 1, status) && ok;
+                ok = mbar_wait(&empty[st], ((i / ST) & 1) ^ 1, status) && ok;
                 mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
                 const int k = (slab0 + i) / kSlabsPerK, dh = (slab0 + i) % kSlabsPerK;
                 tma_load_3d(smem_u32(sA + st * kA), amap, h * D + dh * 64, c0, k, &full[st]);
@@ -111,8 +112,8 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
         const bool leader = elect_one();
         constexpr uint32_t idesc = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
         for (int i = 0; i < nslab && ok; ++i) {
-            const int st = i % kLcStages;
-            ok = mbar_wait(&full[st], (i / kLcStages) & 1, status) && ok;
+            const int st = i % ST;
+            ok = mbar_wait(&full[st], (i / ST) & 1, status) && ok;
             tc_fence_after();
             if (leader) {
 #pragma unroll
@@ -194,14 +195,20 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
         for (int i = tid; i < (r_hi - r_lo) * (D / 8) && ok; i += 192) {
             const int row = r_lo + i / (D / 8), col = (i % (D / 8)) * 8;
             float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            float4 a[kLcSplits], b[kLcSplits];                   // all reads in flight at once: one after the other they took 3 us
 #pragma unroll
-            for (int q = 0; q < kLcSplits; ++q) {
-                if (q >= S) break;
-                const float* src = cluster.map_shared_rank(part, q) + row * kPitch + col;
-                const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-                sum[0] += a.x; sum[1] += a.y; sum[2] += a.z; sum[3] += a.w;
-                sum[4] += b.x; sum[5] += b.y; sum[6] += b.z; sum[7] += b.w;
-            }
+            for (int q = 0; q < kLcSplits; ++q)
+                if (q < S) {
+                    const float* src = cluster.map_shared_rank(part, q) + row * kPitch + col;
+                    a[q] = *reinterpret_cast<const float4*>(src);
+                    b[q] = *reinterpret_cast<const float4*>(src + 4);
+                }
+#pragma unroll
+            for (int q = 0; q < kLcSplits; ++q)
+                if (q < S) {
+                    sum[0] += a[q].x; sum[1] += a[q].y; sum[2] += a[q].z; sum[3] += a[q].w;
+                    sum[4] += b[q].x; sum[5] += b[q].y; sum[6] += b[q].z; sum[7] += b[q].w;
+                }
             *reinterpret_cast<uint4*>(y + (int64_t)row * p.H * D + col) = finish(sum, col);
         }
         cluster.sync();                                    // nobody leaves while its partial tile is being read
@@ -256,10 +263,6 @@ __global__ void __launch_bounds__(256) compress_bias_kernel(const ET* __restrict
 
 template <int D, typename ET>
 static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, int nt, cudaStream_t stream) {
-    constexpr int smem = kLcStages * (128 * 128 + 64 * D * 2) + 128 + D * 4;
-    auto kern = linear_compress_fwd_kernel<D, ET>;
-    cudaError_t e = allow_smem((const void*)kern, smem);
-    if (e != cudaSuccess) return e;
     // CTAs per tile: as many as still find an SM of their own (the ring takes one SM's shared memory).  Short sequences only: another
     // order of the sum moves the last bit of a compressed row, and with it near ties of a block selection.  Up to kLcShort windows
     // (about 1000 tokens at stride 16, 16 blocks of 64) a selection of 16 blocks of 64 takes them all; a smaller one, or one of 32-key
@@ -267,6 +270,13 @@ static cudaError_t launch_lc(const LcMaps& maps, const LcParams& p, int tiles, i
     int S = 1, longest = 0;
     for (int b = 0; b < p.n_seq; ++b) longest = p.n_cmp[b] > longest ? p.n_cmp[b] : longest;
     while (longest <= kLcShort && S < kLcSplits && (p.ks * (D / 64)) % (2 * S) == 0 && 2 * S * tiles * p.H * nt <= sm_count()) S *= 2;
+    // Three stages where the reduction is split, so that two CTAs share an SM: clusters of eight that need an SM for each CTA do not all
+    // find one at once (a GPU processing cluster has 16 to 20 SMs), and sixteen of them took two rounds.
+    const int stages = S > 1 ? kLcStagesSplit : kLcStages;
+    const int smem = stages * (128 * 128 + 64 * D * 2) + 128 + D * 4;
+    auto kern = S > 1 ? linear_compress_fwd_kernel<D, ET, kLcStagesSplit> : linear_compress_fwd_kernel<D, ET, kLcStages>;
+    cudaError_t e = allow_smem((const void*)kern, smem);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)S, (unsigned)tiles, (unsigned)(p.H * nt));
     cfg.blockDim = dim3(192);
