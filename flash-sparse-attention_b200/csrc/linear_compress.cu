@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
         for (int i = 0; i < nslab && ok; ++i) {
             const int st = i % ST;
             ok = mbar_wait(&full[st], (i / ST) & 1, status) && ok;
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
 #pragma unroll

@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
             for (int q = 0; q < per_phase && ok; ++q, ++i) {
                 const int st = i % kLcDxStages;
                 ok = mbar_wait(&full[st], (i / kLcDxStages) & 1, status) && ok;
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
 #pragma unroll
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
                 const int st = i % kLcDwStages;
                 ok = mbar_wait(&full[st], (i / kLcDwStages) & 1, status) && ok;
                 fence_async_smem();
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
                     const uint32_t a_lo = umma_desc_lo(smem_u32(smem + st * kStage), kSlab);

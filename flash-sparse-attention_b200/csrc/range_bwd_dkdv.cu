@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         auto issue_s = [&](int t, int half, bool last) {
             const int u = 2 * t + (first ? 0 : 1), st = u % kRkUnits;
             if (half == 0) ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
                 const uint32_t bu = b_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));
@@ -338,6 +339,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
 #pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
                     ok = mbar_wait(&in_full[half], c & 1, status) && ok;
+                    ok = warp_ok(ok);
                     tc_fence_after();
                     if (leader) {
                         const uint32_t bu = b_mn_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));

@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
     auto take_item = [&](int n, bool& ok) {
         ok = mbar_wait(it_full, n & 1, status) && ok;
         RdItem m = read_item(n);
+        ok = warp_ok(ok);
         if (!ok) m.z = -1;
-        __syncwarp();
         if (lane == 0) mbar_arrive(it_empty);
         return m;
     };
@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 hi = min(hi, (int)p.Nk - 1);
                 const int nblk = hi >= lo ? (hi - lo) / BK + 1 : 0;
                 if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+                ok = warp_ok(ok);
                 if (lane == 0) {
                     s_item[(n & 1) * 2] = make_int4(z, h, seq, tok0);
                     s_item[(n & 1) * 2 + 1] = make_int4(ne, lo, nblk, 0);
@@ -240,11 +241,12 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             ok = mbar_wait(claim, claims & 1, status) && ok;
             ++claims;
             const bool more = claimed_cta(smem_u32(s_claim), bx, h, z);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_ok(ok);
             fence_async_smem();
             if (!more) break;
         }
         if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+        ok = warp_ok(ok);
         if (lane == 0) {
             s_item[(n & 1) * 2] = make_int4(-1, 0, -1, 0);
             s_item[(n & 1) * 2 + 1] = make_int4(0, 0, 0, 0);
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
         auto issue_s = [&](int t, bool last) {
             const int st = t & 1;
             ok = mbar_wait(&k_full[st], (t >> 1) & 1, status) && ok;
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
                 constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 if (j == 0 && qi > 0) ok = mbar_wait(o_free, (qi - 1) & 1, status) && ok;
                 ok = mbar_wait(&p_full[st], (c >> 1) & 1, status) && ok;
                 ok = mbar_wait(&v_full[st], (c >> 1) & 1, status) && ok;
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
                     const uint32_t b_lo = v_lo + (uint32_t)(st * (kKt >> 4));
@@ -596,7 +600,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     auto take_item = [&](int n, bool& ok) {
         ok = mbar_wait(&it_full[n % kDqItems], (n / kDqItems) & 1, status) && ok;
         const int4 x = s_item[(n % kDqItems) * 2], y = s_item[(n % kDqItems) * 2 + 1];
-        __syncwarp();
+        ok = warp_ok(ok);
         if (lane == 0) mbar_arrive(&it_empty[n % kDqItems]);
         DqItem m;
         m.seq = x.x; m.tok0 = x.y; m.ne = x.z; m.row_lo = x.w; m.nblk = y.x; m.h = y.y;
@@ -610,6 +614,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
             const DqItem m = dq_item(p, ntiles, w, lane);
             ok = mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status) && ok;
+            ok = warp_ok(ok);
             if (lane == 0) {
                 s_item[(n % kDqItems) * 2] = make_int4(m.seq, m.tok0, m.ne, m.row_lo);
                 s_item[(n % kDqItems) * 2 + 1] = make_int4(m.nblk, m.h, 0, 0);
@@ -676,6 +681,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                     const uint32_t v_lo = k_lo + (uint32_t)(kKt >> 4);
                     ok = mbar_wait(&kv_full[st], (c / kDqStages) & 1, status) && ok;
                     ok = mbar_wait(&sdp_free[b], ((c >> 1) & 1) ^ 1, status) && ok;     // S / dP of tile c - 2 have been read
+                    ok = warp_ok(ok);
                     tc_fence_after();
                     if (leader) {
 #pragma unroll
@@ -685,6 +691,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                     }
                     __syncwarp();
                     ok = mbar_wait(&ds_empty[b], ((c >> 1) & 1) ^ 1, status) && ok;     // the dQ product of tile c - 2 has read dS
+                    ok = warp_ok(ok);
                     tc_fence_after();
                     if (leader) {
 #pragma unroll
@@ -700,6 +707,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                     const int b = c & 1, st = c % kDqStages;
                     ok = mbar_wait(&ds_full[b], (c >> 1) & 1, status) && ok;      // (implies S / dP of the tile are done with K and V)
                     if (j == 0 && qi > 0) ok = mbar_wait(dq_free, (qi - 1) & 1, status) && ok;     // the previous item's dQ has been read
+                    ok = warp_ok(ok);
                     tc_fence_after();
                     if (leader) {
                         const uint32_t b_lo = k_mn_lo + (uint32_t)(st * ((2 * kKt) >> 4));

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             int2 off[NIT];                              // (all of them ahead of the copies)
 #pragma unroll
             for (int it = 0; it < NIT; ++it) off[it] = s_off[st][rbase + it * RSTEP];
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(&off_empty[st]);
             // dO first: dV, its last reader, is issued before dK, the last reader of Q
             // (RSTEP is a multiple of 8: the rows of a thread have one swizzle)
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
             BT_TOC(1);
             const int seg = s_rec[k & 15].x;
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(&off_empty[st]);
             if (seg & 1) {
                 ++kvn;
@@ -347,8 +347,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_EV(k, 2, lane == 0);
             BT_TOC(3);
             fence_async_smem();
-            __syncwarp();             // no lane is still to see a phase that the products end
-            __syncwarp();
+            ok = warp_ok(ok);
             tc_fence_after();
             const uint32_t aq = qd_lo + (uint32_t)(st * (kQD >> 4));
             const uint32_t ad = aq + (uint32_t)((kTileRows * D * 2) >> 4);
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
             BT_TOC(3);
             fence_async_smem();
-            __syncwarp();
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -415,7 +414,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
             BT_TOC(3);
             fence_async_smem();
-            __syncwarp();
+            ok = warp_ok(ok);
             tc_fence_after();
             const uint32_t bk = k_mn_lo + (uint32_t)((kvn % kKStages) * (kK >> 4));
             const uint32_t aq = qd_mn_lo + (uint32_t)(st * (kQD >> 4));
@@ -435,7 +434,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = mbar_poll(ds_full, k & 1) && ok;
             BT_TOC(2);
             fence_async_smem();
-            __syncwarp();
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -449,7 +448,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_EV(k, 10, lane == 0);
             ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
             BT_EV(k, 11, lane == 0);
-            __syncwarp();
+            ok = warp_ok(ok);
             tc_fence_after();
             if (leader) {
 #pragma unroll
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                                           cur_t.j * nsub + cur_t.sub(sched), cur_t.j, cur_t.run(sched));
             cur_t.next(sched);
             prev_hg = cur.hg;
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(&off_full[slot]);
         }
       } else {

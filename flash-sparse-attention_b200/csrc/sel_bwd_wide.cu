@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             ok = mbar_poll(do_empty, (k & 1) ^ 1) && ok;
             copy(p.d_o, sDO, s_off[slot][1]);
             cp_async_mbar_arrive_noinc(do_full);
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(&off_empty[slot]);
         }
     } else if (warp >= kWDrain && warp < kWDrain + 4) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         for (int k = 0; k < nloc && ok; ++k) {
             ok = mbar_poll(dq_full, k & 1) && ok;
             const int4 rec = s_rec[k & 7];
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(dq_empty);                // (no tile gets two ahead of this warp)
             if (!(rec.x & 2)) continue;
             const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 const int slot = k % kRing;
                 ok = mbar_poll(&off_full[slot], (k / kRing) & 1) && ok;
                 const int seg = s_rec[k & 7].x;
-                __syncwarp();
+                ok = warp_ok(ok);
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (seg & 1) {
                     ++kvn;
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
                 ok = mbar_poll(q_full, k & 1) && ok;
                 fence_async_smem();
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 4
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 __syncwarp();
                 ok = mbar_poll(do_full, k & 1) && ok;
                 fence_async_smem();
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 4
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 ok = mbar_poll(do_full, k & 1) && ok;
                 if (first && blk > 0) ok = mbar_poll(acc_empty, (blk - 1) & 1) && ok;
                 fence_async_smem();
+                ok = warp_ok(ok);
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 2
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                                              cur.j * p.nsub + cur.sub(sched), cur.j, cur.run(sched));
                 cur.next(sched);
                 prev_hg = m.hg;
-                __syncwarp();
+                ok = warp_ok(ok);
                 if (lane == 0) mbar_arrive(&off_full[slot]);
                 if (k + 2 < nloc) fetch(m);
             };

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             // arrives on q_full when this thread's copies have landed; nobody waits here, so the
             // loader never holds a finished tile back behind a later wait
             cp_async_mbar_arrive_noinc(&q_full[qs]);
-            __syncwarp();
+            ok = warp_ok(ok);
             if (lane == 0) mbar_arrive(&off_empty[slot]);
             if (++qs == C::NQ) { qs = 0; qph ^= 1; }
         }
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 const int sbuf = k % C::NS, slot = k % kFwdRing;
                 ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
                 const int blk = s_rec[slot].y;
-                __syncwarp();
+                ok = warp_ok(ok);
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (blk & 1) {
                     ++kvn;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 ok = mbar_poll(&q_full[qs], qph) && ok;
                 fence_async_smem();   // the Q rows were written by cp.async (generic proxy)
                 ok = mbar_poll(&s_empty[sbuf], ((k / C::NS) & 1) ^ 1) && ok;
-                __syncwarp();         // no lane is still to see a phase that the products end
+                ok = warp_ok(ok);
                 tc_fence_after();
                 const uint32_t a_lo = q_lo + (uint32_t)(qs * (C::kQ >> 4));
                 const uint32_t b_lo = k_lo + (uint32_t)((kvn % C::NKV) * (C::kKV >> 4));
@@ -243,12 +243,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 const int ob = k % C::NO, sbuf = k % C::NS, slot = k % kFwdRing;
                 ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
                 const int blk = s_rec[slot].y;
-                __syncwarp();
+                ok = warp_ok(ok);
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (blk & 1) ++kvn;
                 ok = mbar_poll(&o_empty[ob], ((k / C::NO) & 1) ^ 1) && ok;
                 ok = mbar_poll(&p_full[sbuf], (k / C::NS) & 1) && ok;
-                __syncwarp();
+                ok = warp_ok(ok);
                 tc_fence_after();
                 const int kv_cur = kvn % C::NKV;
                 const uint32_t b_lo = v_lo + (uint32_t)(kv_cur * (C::kKV >> 4));
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 if (lane == 0)
                     s_rec[slot] = make_int4(m.h, (m.hg != prev_hg ? 1 : 0) | (k + 1 >= nloc || next.hg != m.hg ? 2 : 0), m.row0, 0);
                 prev_hg = m.hg;
-                __syncwarp();
+                ok = warp_ok(ok);
                 if (lane == 0) mbar_arrive(&off_full[slot]);
                 if (k + 3 < nloc) fetch(m);
             };

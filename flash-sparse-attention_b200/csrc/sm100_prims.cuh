@@ -138,6 +138,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     return false;
 }
 
+// Whether no wait of any lane of a warp has run out, for all its lanes alike.  Stands between waits that the whole warp makes and what an
+// elected lane then issues or announces: a phase that this leads to may be the next one of a barrier just waited for, and a lane that
+// has yet to look at the one before would see its parity gone by and wait until its limit.  And a lane that gave up must not
+// leave a loop in which the others go on to meet it.  (The vote alone does not order the lanes' accesses to shared memory.)
+__device__ __forceinline__ bool warp_ok(bool ok) {
+    const bool all = __all_sync(0xffffffffu, ok);
+    __syncwarp();
+    return all;
+}
+
 // Barrier `id` of `threads` threads that tells whether v held for all of them.
 __device__ __forceinline__ bool bar_all(int id, int threads, bool v) {
     uint32_t all;
