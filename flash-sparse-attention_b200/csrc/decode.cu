@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
     constexpr int NO = D / 8;                            // 8-column output tiles of P V
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
     const int nst = p.nst;
+    const uint32_t limit = wait_limit(&g_decode_status);
     uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)nst * STAGE_BYTES);
     uint64_t* empty = full + 4;
     float* smm = reinterpret_cast<float*>(empty + 4);    // [4][16]
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
                 bounds(j, lo, n);
                 for (int i = 0; i * kDecKT < n; ++i, ++it) {
                     const int s = it % nst;
-                    if (it >= nst && !mbar_wait(&empty[s], ((it / nst) - 1) & 1, &g_decode_status)) { ok = false; break; }
+                    if (it >= nst && !mbar_wait(&empty[s], ((it / nst) - 1) & 1, &g_decode_status, limit)) { ok = false; break; }
                     mbar_expect_tx(&full[s], STAGE_BYTES);
                     const uint32_t kb = sbase + s * STAGE_BYTES;
 #pragma unroll
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
         float* srow = want_scores ? p.scores + ((int64_t)b * p.Hk + h) * p.scores_ld + c * p.chunk : nullptr;
         for (int i = 0; i * kDecKT < n; ++i, ++it) {
             const int s = it % nst;
-            if (!mbar_wait(&full[s], (it / nst) & 1, &g_decode_status)) { ok_wait = false; break; }
+            if (!mbar_wait(&full[s], (it / nst) & 1, &g_decode_status, limit)) { ok_wait = false; break; }
             const int k0 = i * kDecKT + warp * 16;               // first key of this warp's tile
             if (k0 < n) {
                 const uint32_t kb = sbase + s * STAGE_BYTES, vb = kb + KV_BYTES;

@@ -646,14 +646,15 @@ int fsa_sel_index_dump(const void* index_ws, int64_t N, int B, int Hq, int Hk, i
 }
 
 // A bounded wait that runs out, on purpose and harmlessly: one thread waits on an mbarrier that nothing arrives on, gives
-// up after FSA_WAIT_CLOCKS like every wait of the library does, records kStatusWaitTimeout in the status word and returns.
+// up after FSA_WAIT_CLOCKS like every wait of the library does (earlier if the status word is set: see wait_limit), records
+// kStatusWaitTimeout in the status word and returns.
 // Lets a test walk the failure path of the status plumbing without hanging or faulting anything.
 static __global__ void wait_timeout_probe_kernel(int* status) {
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         mbar_init_fence();
-        if (mbar_wait(&bar, 0, status)) atomicMax(status, 99);   // cannot happen: nobody arrives
+        if (mbar_wait(&bar, 0, status, wait_limit(status))) atomicMax(status, 99);   // cannot happen: nobody arrives
     }
 }
 

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
     const CUtensorMap* amap = &maps.a[tn][seq];
     const CUtensorMap* wmap = &maps.w[tn];
     int* status = p.status;
+    const uint32_t limit = wait_limit(status);
     if (tid == 0) {
         for (int i = 0; i < ST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_init(acc_full, 1);
@@ -97,13 +98,15 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
         for (int i = 0; i < nslab && ok; ++i) {
             const int st = i % ST;
             if (lane == 0) {
-                ok = mbar_wait(&empty[st], ((i / ST) & 1) ^ 1, status) && ok;
-                mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
-                const int k = (slab0 + i) / kSlabsPerK, dh = (slab0 + i) % kSlabsPerK;
-                tma_load_3d(smem_u32(sA + st * kA), amap, h * D + dh * 64, c0, k, &full[st]);
+                ok = ok && mbar_wait(&empty[st], ((i / ST) & 1) ^ 1, status, limit);
+                if (ok) {
+                    mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
+                    const int k = (slab0 + i) / kSlabsPerK, dh = (slab0 + i) % kSlabsPerK;
+                    tma_load_3d(smem_u32(sA + st * kA), amap, h * D + dh * 64, c0, k, &full[st]);
 #pragma unroll
-                for (int nh = 0; nh < D / 64; ++nh)
-                    tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), wmap, nh * 64, (h * p.ks * D) + (slab0 + i) * 64, &full[st]);
+                    for (int nh = 0; nh < D / 64; ++nh)
+                        tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), wmap, nh * 64, (h * p.ks * D) + (slab0 + i) * 64, &full[st]);
+                }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
@@ -113,8 +116,9 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
         constexpr uint32_t idesc = umma_idesc(ElemTraits<ET>::kIsBF16, 128, D, false, true);
         for (int i = 0; i < nslab && ok; ++i) {
             const int st = i % ST;
-            ok = mbar_wait(&full[st], (i / ST) & 1, status) && ok;
+            ok = ok && mbar_wait(&full[st], (i / ST) & 1, status, limit);
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             if (leader) {
 #pragma unroll
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(192) linear_compress_fwd_kernel(const __grid_c
             s_bias[t] = v;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        ok = mbar_wait(acc_full, 0, status);
+        ok = ok && mbar_wait(acc_full, 0, status, limit);
         tc_fence_after();
     }
     ET* y = reinterpret_cast<ET*>(p.y[tn]) + ((int64_t)(p.y_row0[seq] + c0) * p.H + h) * D;      // row r at r * H * D

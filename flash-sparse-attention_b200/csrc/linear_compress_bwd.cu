@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
     const int J = p.ks / p.stride;
     const int per_phase = J * KH;
     int* status = p.status;
+    const uint32_t limit = wait_limit(status);
     if (tid == 0) {
         for (int i = 0; i < kLcDxStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 128); }
@@ -89,14 +90,16 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
             for (int q = 0; q < per_phase && ok; ++q, ++i) {
                 const int st = i % kLcDxStages;
                 if (lane == 0) {
-                    ok = mbar_wait(&empty[st], ((i / kLcDxStages) & 1) ^ 1, status) && ok;
-                    mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
-                    const int j = q / KH, kh = q % KH;
-                    const int k = p0 + pi + j * p.stride;
-                    tma_load_2d(smem_u32(sA + st * kA), ymap, h * D + kh * 64, m0 - j, &full[st]);
+                    ok = ok && mbar_wait(&empty[st], ((i / kLcDxStages) & 1) ^ 1, status, limit);
+                    if (ok) {
+                        mbar_expect_tx(&full[st], (uint32_t)(kA + kB));
+                        const int j = q / KH, kh = q % KH;
+                        const int k = p0 + pi + j * p.stride;
+                        tma_load_2d(smem_u32(sA + st * kA), ymap, h * D + kh * 64, m0 - j, &full[st]);
 #pragma unroll
-                    for (int nh = 0; nh < KH; ++nh)
-                        tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), wmap, kh * 64, (h * p.ks + k) * D + nh * 64, &full[st]);
+                        for (int nh = 0; nh < KH; ++nh)
+                            tma_load_2d(smem_u32(sB + st * kB + nh * (64 * 128)), wmap, kh * 64, (h * p.ks + k) * D + nh * 64, &full[st]);
+                    }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
@@ -109,12 +112,13 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
         int i = 0;
         for (int pi = 0; pi < p.phases && ok && product; ++pi) {
             const int buf = pi & 1;
-            ok = mbar_wait(&acc_empty[buf], ((pi >> 1) & 1) ^ 1, status) && ok;
+            ok = ok && mbar_wait(&acc_empty[buf], ((pi >> 1) & 1) ^ 1, status, limit);
             tc_fence_after();
             for (int q = 0; q < per_phase && ok; ++q, ++i) {
                 const int st = i % kLcDxStages;
-                ok = mbar_wait(&full[st], (i / kLcDxStages) & 1, status) && ok;
+                ok = ok && mbar_wait(&full[st], (i / kLcDxStages) & 1, status, limit);
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
 #pragma unroll
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
         bool ok = true;
         for (int pi = 0; pi < p.phases && ok; ++pi) {
             const int buf = pi & 1;
-            if (product) ok = mbar_wait(&acc_full[buf], (pi >> 1) & 1, status) && ok;
+            if (product) ok = ok && mbar_wait(&acc_full[buf], (pi >> 1) & 1, status, limit);
             tc_fence_after();
             const int64_t t = (int64_t)(m0 + r) * p.stride + p0 + pi;
             const bool valid = ok && t < p.L[seq];
@@ -223,6 +227,7 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
     const bool with_pe = tn == 0 && p.pe != nullptr;
     float* s_db = reinterpret_cast<float*>(bars + 2 * kLcDwStages + 2);      // [D] gradient of the bias
     int* status = p.status;
+    const uint32_t limit = wait_limit(status);
     if (tid == 0) {
         for (int i = 0; i < kLcDwStages; ++i) { mbar_init(&full[i], 128); mbar_init(&empty[i], 1); }
         mbar_init(acc_full, 1);
@@ -261,7 +266,7 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
             const int n = L >= p.ks ? (L - p.ks) / p.stride + 1 : 0;
             for (int c0 = 0; c0 < n && ok; c0 += 128, ++i) {
                 const int st = i % kLcDwStages;
-                ok = mbar_wait(&empty[st], ((i / kLcDwStages) & 1) ^ 1, status) && ok;
+                ok = ok && mbar_wait(&empty[st], ((i / kLcDwStages) & 1) ^ 1, status, limit);
                 const uint32_t sx = smem_u32(smem + st * kStage) + x_slab;
                 const uint32_t sy = smem_u32(smem + st * kStage + kX) + y_slab;
 #pragma unroll
@@ -291,9 +296,10 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
             bool ok = true;
             for (int i = 0; i < nitems && ok; ++i) {
                 const int st = i % kLcDwStages;
-                ok = mbar_wait(&full[st], (i / kLcDwStages) & 1, status) && ok;
+                ok = ok && mbar_wait(&full[st], (i / kLcDwStages) & 1, status, limit);
                 fence_async_smem();
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
                     const uint32_t a_lo = umma_desc_lo(smem_u32(smem + st * kStage), kSlab);
@@ -325,7 +331,7 @@ __global__ void __launch_bounds__(256) linear_compress_dw_kernel(const LcDwParam
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         if (nitems > 0) {
-            ok = mbar_wait(acc_full, 0, status);
+            ok = ok && mbar_wait(acc_full, 0, status, limit);
             tc_fence_after();
         }
         ET* dst = p.dw[tn] ? p.dw[tn] + wrow * D : nullptr;

@@ -265,14 +265,16 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 if (m.n == 0) continue;
                 auto load_unit = [&](const CUtensorMap* map, int tok) {
                     const int st = u % kRkUnits;
-                    ok = mbar_wait(&u_empty[st], ((u / kRkUnits) & 1) ^ 1, status) && ok;
+                    ok = ok && mbar_wait(&u_empty[st], ((u / kRkUnits) & 1) ^ 1, status);
+                    if (!ok) return;
                     mbar_expect_tx(&u_full[st], unit_bytes);
 #pragma unroll
                     for (int b = 0; b < 2; ++b) tma_load_3d(smem_u32(sU + st * kRkTile + b * kSlab), map, b * 64, tok, m.h * p.G, &u_full[st]);
                     ++u;
                 };
                 auto load_kv = [&](const CUtensorMap* map, uint8_t* dst, uint64_t* full, uint64_t* empty) {
-                    ok = mbar_wait(empty, (qi & 1) ^ 1, status) && ok;
+                    ok = ok && mbar_wait(empty, (qi & 1) ^ 1, status);
+                    if (!ok) return;
                     mbar_expect_tx(full, (uint32_t)kRkTile);
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
@@ -310,8 +312,9 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         // S^T (dP^T) of half a row tile t into its place: in order after the product that read P^T (dS^T) of the tile before from there
         auto issue_s = [&](int t, int half, bool last) {
             const int u = 2 * t + (first ? 0 : 1), st = u % kRkUnits;
-            if (half == 0) ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
+            if (half == 0) ok = ok && mbar_wait(&u_full[st], (u / kRkUnits) & 1, status);
             ok = warp_ok(ok);
+            if (!ok) return;
             tc_fence_after();
             if (leader) {
                 const uint32_t bu = b_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));
@@ -329,17 +332,18 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
             const RkItem m = rk_item(p.plan, w);
             if (m.n == 0) continue;
-            ok = mbar_wait(kv_full, qi & 1, status) && ok;
+            ok = ok && mbar_wait(kv_full, qi & 1, status);
             issue_s(c, 0, m.n == 1);
             issue_s(c, 1, m.n == 1);
             for (int i = 0; i < m.n && ok; ++i, ++c) {
                 const int u = 2 * c + (first ? 1 : 0), st = u % kRkUnits;       // dV takes dO, dK takes Q
-                ok = mbar_wait(&u_full[st], (u / kRkUnits) & 1, status) && ok;
-                if (i == 0 && qi > 0) ok = mbar_wait(acc_free, (qi - 1) & 1, status) && ok;
+                ok = ok && mbar_wait(&u_full[st], (u / kRkUnits) & 1, status);
+                if (i == 0 && qi > 0) ok = ok && mbar_wait(acc_free, (qi - 1) & 1, status);
 #pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
-                    ok = mbar_wait(&in_full[half], c & 1, status) && ok;
+                    ok = ok && mbar_wait(&in_full[half], c & 1, status);
                     ok = warp_ok(ok);
+                    if (!ok) break;
                     tc_fence_after();
                     if (leader) {
                         const uint32_t bu = b_mn_lo + (uint32_t)(st * (kRkTile >> 4) + half * (8192 >> 4));
@@ -393,7 +397,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 }
                 masked = __any_sync(0xffffffffu, masked);
                 const int b = c & 1;
-                ok = mbar_wait(&st_empty[b], ((c >> 1) & 1) ^ 1, status) && ok;
+                ok = ok && mbar_wait(&st_empty[b], ((c >> 1) & 1) ^ 1, status);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     sLse[b * 128 + lane + 32 * j] = lse[j];
@@ -418,8 +422,8 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
             const RkItem m = rk_item(p.plan, w);
             for (int i = 0; i < m.n && ok; ++i, ++c) {
                 const int b = c & 1;
-                ok = mbar_wait(&st_full[b], (c >> 1) & 1, status) && ok;
-                ok = mbar_wait(&s_full[grp], c & 1, status) && ok;
+                ok = ok && mbar_wait(&st_full[b], (c >> 1) & 1, status);
+                ok = ok && mbar_wait(&s_full[grp], c & 1, status);
                 tc_fence_after();
                 const bool masked = s_masked[b] != 0;
                 const float4* lse4 = reinterpret_cast<const float4*>(sLse + b * 128 + grp * 64);
@@ -460,7 +464,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&p_full[grp]);
-                ok = mbar_wait(&dp_full[grp], c & 1, status) && ok;
+                ok = ok && mbar_wait(&dp_full[grp], c & 1, status);
                 tc_fence_after();
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
@@ -485,7 +489,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
             }
             // ---- epilogue of the item: group 0 dV, group 1 dK
             if (m.n > 0) {
-                ok = mbar_wait(grp ? dk_done : dv_done, qi & 1, status) && ok;
+                ok = ok && mbar_wait(grp ? dk_done : dv_done, qi & 1, status);
                 tc_fence_after();
             }
             const bool write = ok && key < m.nkeys;

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = launch.p[blockIdx.z].status;
+    const uint32_t limit = wait_limit(status);
     const int G = launch.p[0].G, TPT = launch.p[0].TPT;      // (the same for all problems)
     if (tid == 0) {
         mbar_init(q_full, 1); mbar_init(q_empty, 1); mbar_init(o_free, 128);
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
         return m;
     };
     auto take_item = [&](int n, bool& ok) {
-        ok = mbar_wait(it_full, n & 1, status) && ok;
+        ok = ok && mbar_wait(it_full, n & 1, status, limit);
         RdItem m = read_item(n);
         ok = warp_ok(ok);
         if (!ok) m.z = -1;
@@ -197,9 +198,9 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 lo = max(lo, 0);
                 hi = min(hi, (int)p.Nk - 1);
                 const int nblk = hi >= lo ? (hi - lo) / BK + 1 : 0;
-                if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+                if (n > 0) ok = ok && mbar_wait(it_empty, (n - 1) & 1, status, limit);
                 ok = warp_ok(ok);
-                if (lane == 0) {
+                if (ok && lane == 0) {
                     s_item[(n & 1) * 2] = make_int4(z, h, seq, tok0);
                     s_item[(n & 1) * 2 + 1] = make_int4(ne, lo, nblk, 0);
                     mbar_arrive(it_full);
@@ -207,17 +208,20 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 ++n;
                 if (lane == 0 && nblk > 0) {
                     const CUtensorMap *kmap = &launch.k[z], *vmap = &launch.v[z];
-                    ok = mbar_wait(q_empty, (qi & 1) ^ 1, status) && ok;
+                    ok = ok && mbar_wait(q_empty, (qi & 1) ^ 1, status, limit);
                     ask();                  // not earlier: a CTA is to be one item ahead, not to take the share of others
-                    mbar_expect_tx(q_full, (uint32_t)(KH * 128 * TPT * G));
+                    if (ok) {
+                        mbar_expect_tx(q_full, (uint32_t)(KH * 128 * TPT * G));
 #pragma unroll
-                    for (int b = 0; b < KH; ++b) tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &launch.q[z], b * 64, tok0, h * G, q_full);
+                        for (int b = 0; b < KH; ++b) tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &launch.q[z], b * 64, tok0, h * G, q_full);
+                    }
                     // K tile j and V tile j are loaded in the order the MMA warp needs them: K(0), K(1), V(0), K(2), V(1), ...
                     for (int step = 0; step < nblk + 1 && ok; ++step) {
                         const int jk = c + step, jv = jk - 1;
                         if (step < nblk) {
                             const int st = jk & 1;
-                            ok = mbar_wait(&k_empty[st], ((jk >> 1) & 1) ^ 1, status) && ok;
+                            ok = ok && mbar_wait(&k_empty[st], ((jk >> 1) & 1) ^ 1, status, limit);
+                            if (!ok) break;
                             mbar_expect_tx(&k_full[st], (uint32_t)kKt);
 #pragma unroll
                             for (int b = 0; b < KH; ++b)
@@ -225,7 +229,8 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                         }
                         if (step > 0) {
                             const int st = jv & 1;
-                            ok = mbar_wait(&v_empty[st], ((jv >> 1) & 1) ^ 1, status) && ok;
+                            ok = ok && mbar_wait(&v_empty[st], ((jv >> 1) & 1) ^ 1, status, limit);
+                            if (!ok) break;
                             mbar_expect_tx(&v_full[st], (uint32_t)kKt);
 #pragma unroll
                             for (int b = 0; b < KH; ++b)
@@ -238,16 +243,17 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             }
             if (lane == 0 && !asked) ask();
             // (the answer is in shared memory before this CTA may end, whatever happened above)
-            ok = mbar_wait(claim, claims & 1, status) && ok;
+            const bool answered = mbar_wait(claim, claims & 1, status, limit);
+            ok = ok && answered;
             ++claims;
             const bool more = claimed_cta(smem_u32(s_claim), bx, h, z);
             ok = warp_ok(ok);
             fence_async_smem();
             if (!more) break;
         }
-        if (n > 0) ok = mbar_wait(it_empty, (n - 1) & 1, status) && ok;
+        if (n > 0) ok = ok && mbar_wait(it_empty, (n - 1) & 1, status, limit);
         ok = warp_ok(ok);
-        if (lane == 0) {
+        if (ok && lane == 0) {          // (else the other warps give up by themselves: one may still read this place)
             s_item[(n & 1) * 2] = make_int4(-1, 0, -1, 0);
             s_item[(n & 1) * 2 + 1] = make_int4(0, 0, 0, 0);
             mbar_arrive(it_full);
@@ -265,8 +271,9 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
         int n = 0, qi = 0, c = 0;
         auto issue_s = [&](int t, bool last) {
             const int st = t & 1;
-            ok = mbar_wait(&k_full[st], (t >> 1) & 1, status) && ok;
+            ok = ok && mbar_wait(&k_full[st], (t >> 1) & 1, status, limit);
             ok = warp_ok(ok);
+            if (!ok) return;
             tc_fence_after();
             if (leader) {
                 constexpr int kSlabA = (kTileRows * 128) >> 4, kSlabB = (BK * 128) >> 4;
@@ -283,16 +290,17 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
         };
         for (RdItem m = take_item(n, ok); m.z >= 0; m = take_item(++n, ok)) {
             if (m.nblk == 0) continue;
-            ok = mbar_wait(q_full, qi & 1, status) && ok;
+            ok = ok && mbar_wait(q_full, qi & 1, status, limit);
             issue_s(c, m.nblk == 1);
             for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                 const int st = c & 1;
                 // S(c + 1) overwrites the buffer P(c - 1) was read from by the product issued one iteration ago (in order)
                 if (j + 1 < m.nblk) issue_s(c + 1, j + 2 == m.nblk);
-                if (j == 0 && qi > 0) ok = mbar_wait(o_free, (qi - 1) & 1, status) && ok;
-                ok = mbar_wait(&p_full[st], (c >> 1) & 1, status) && ok;
-                ok = mbar_wait(&v_full[st], (c >> 1) & 1, status) && ok;
+                if (j == 0 && qi > 0) ok = ok && mbar_wait(o_free, (qi - 1) & 1, status, limit);
+                ok = ok && mbar_wait(&p_full[st], (c >> 1) & 1, status, limit);
+                ok = ok && mbar_wait(&v_full[st], (c >> 1) & 1, status, limit);
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
                     const uint32_t b_lo = v_lo + (uint32_t)(st * (kKt >> 4));
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             for (int j = 0; j < nblk && ok; ++j, ++c) {
                 const int st = c & 1;
                 const int c_lo = max(0, lo_r - j * BK), c_hi = min(BK, hi_r - j * BK + 1);      // visible columns [c_lo, c_hi)
-                ok = mbar_wait(&s_full[st], (c >> 1) & 1, status) && ok;
+                ok = ok && mbar_wait(&s_full[st], (c >> 1) & 1, status, limit);
                 tc_fence_after();
                 uint32_t v[BK];
                 tmem_ld32(tbase + lane_off + cS + st * BK, *reinterpret_cast<uint32_t (*)[32]>(&v[0]));
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                 // accumulator rows already hold products (j > 0): rescale them when any row of the warp changes reference
                 const bool scale_acc = __any_sync(0xffffffffu, raise && j > 0);
                 if (scale_acc) {
-                    ok = mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status) && ok;
+                    ok = ok && mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status, limit);
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < D; c0 += 32) {
@@ -401,7 +409,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             sees = rd_row(launch, next, g < G && e < next.ne, e);
             // ---- epilogue
             if (m.nblk > 0) {
-                ok = mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status) && ok;
+                ok = ok && mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status, limit);
                 tc_fence_after();
             }
             ok = bar_all(1, 128, ok);
@@ -598,12 +606,13 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     const int nitems = ntiles * p.Hk;
     // Entry n of this CTA's items: every warp but the one that fills the ring takes each of them once, in order.
     auto take_item = [&](int n, bool& ok) {
-        ok = mbar_wait(&it_full[n % kDqItems], (n / kDqItems) & 1, status) && ok;
+        ok = ok && mbar_wait(&it_full[n % kDqItems], (n / kDqItems) & 1, status);
         const int4 x = s_item[(n % kDqItems) * 2], y = s_item[(n % kDqItems) * 2 + 1];
         ok = warp_ok(ok);
         if (lane == 0) mbar_arrive(&it_empty[n % kDqItems]);
         DqItem m;
         m.seq = x.x; m.tok0 = x.y; m.ne = x.z; m.row_lo = x.w; m.nblk = y.x; m.h = y.y;
+        if (!ok) m.ne = m.nblk = 0;
         return m;
     };
 
@@ -613,9 +622,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
         int n = 0;
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
             const DqItem m = dq_item(p, ntiles, w, lane);
-            ok = mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status) && ok;
+            ok = ok && mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status);
             ok = warp_ok(ok);
-            if (lane == 0) {
+            if (ok && lane == 0) {
                 s_item[(n % kDqItems) * 2] = make_int4(m.seq, m.tok0, m.ne, m.row_lo);
                 s_item[(n % kDqItems) * 2 + 1] = make_int4(m.nblk, m.h, 0, 0);
                 mbar_arrive(&it_full[n % kDqItems]);
@@ -629,26 +638,30 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             const DqItem m = take_item(n, ok);
             if (m.nblk == 0) continue;
             if (lane == 0) {
-                ok = mbar_wait(qd_empty, (qi & 1) ^ 1, status) && ok;
-                mbar_expect_tx(qd_full, (uint32_t)(2 * KH * 128 * p.TPT * p.G));
+                ok = ok && mbar_wait(qd_empty, (qi & 1) ^ 1, status);
+                if (ok) {
+                    mbar_expect_tx(qd_full, (uint32_t)(2 * KH * 128 * p.TPT * p.G));
 #pragma unroll
-                for (int b = 0; b < KH; ++b) {
-                    tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &qmap, b * 64, m.tok0, m.h * p.G, qd_full);
-                    tma_load_3d(smem_u32(sDO + b * (kTileRows * 128)), &domap, b * 64, m.tok0, m.h * p.G, qd_full);
+                    for (int b = 0; b < KH; ++b) {
+                        tma_load_3d(smem_u32(sQ + b * (kTileRows * 128)), &qmap, b * 64, m.tok0, m.h * p.G, qd_full);
+                        tma_load_3d(smem_u32(sDO + b * (kTileRows * 128)), &domap, b * 64, m.tok0, m.h * p.G, qd_full);
+                    }
                 }
             }
             ++qi;
             for (int j = 0; j < m.nblk && ok; ++j, ++kvc) {
                 if (lane == 0) {
                     const int st = kvc % kDqStages;
-                    ok = mbar_wait(&kv_empty[st], ((kvc / kDqStages) & 1) ^ 1, status) && ok;
-                    mbar_expect_tx(&kv_full[st], (uint32_t)(2 * kKt));
-                    uint8_t* dK = sKV + st * 2 * kKt;
-                    uint8_t* dV = dK + kKt;
+                    ok = ok && mbar_wait(&kv_empty[st], ((kvc / kDqStages) & 1) ^ 1, status);
+                    if (ok) {
+                        mbar_expect_tx(&kv_full[st], (uint32_t)(2 * kKt));
+                        uint8_t* dK = sKV + st * 2 * kKt;
+                        uint8_t* dV = dK + kKt;
 #pragma unroll
-                    for (int b = 0; b < KH; ++b) {
-                        tma_load_2d(smem_u32(dK + b * (BK * 128)), &kmap, m.h * D + b * 64, m.row_lo + j * BK, &kv_full[st]);
-                        tma_load_2d(smem_u32(dV + b * (BK * 128)), &vmap, m.h * D + b * 64, m.row_lo + j * BK, &kv_full[st]);
+                        for (int b = 0; b < KH; ++b) {
+                            tma_load_2d(smem_u32(dK + b * (BK * 128)), &kmap, m.h * D + b * 64, m.row_lo + j * BK, &kv_full[st]);
+                            tma_load_2d(smem_u32(dV + b * (BK * 128)), &vmap, m.h * D + b * 64, m.row_lo + j * BK, &kv_full[st]);
+                        }
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -674,14 +687,15 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             const DqItem m = take_item(n, ok);
             if (m.nblk == 0) continue;
             if (warp == 1) {
-                ok = mbar_wait(qt_full, qi & 1, status) && ok;
+                ok = ok && mbar_wait(qt_full, qi & 1, status);
                 for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                     const int b = c & 1, st = c % kDqStages;
                     const uint32_t k_lo = kv_lo_ + (uint32_t)(st * ((2 * kKt) >> 4));
                     const uint32_t v_lo = k_lo + (uint32_t)(kKt >> 4);
-                    ok = mbar_wait(&kv_full[st], (c / kDqStages) & 1, status) && ok;
-                    ok = mbar_wait(&sdp_free[b], ((c >> 1) & 1) ^ 1, status) && ok;     // S / dP of tile c - 2 have been read
+                    ok = ok && mbar_wait(&kv_full[st], (c / kDqStages) & 1, status);
+                    ok = ok && mbar_wait(&sdp_free[b], ((c >> 1) & 1) ^ 1, status);     // S / dP of tile c - 2 have been read
                     ok = warp_ok(ok);
+                    if (!ok) break;
                     tc_fence_after();
                     if (leader) {
 #pragma unroll
@@ -690,8 +704,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                                     idesc_s, ks > 0);
                     }
                     __syncwarp();
-                    ok = mbar_wait(&ds_empty[b], ((c >> 1) & 1) ^ 1, status) && ok;     // the dQ product of tile c - 2 has read dS
+                    ok = ok && mbar_wait(&ds_empty[b], ((c >> 1) & 1) ^ 1, status);     // the dQ product of tile c - 2 has read dS
                     ok = warp_ok(ok);
+                    if (!ok) break;
                     tc_fence_after();
                     if (leader) {
 #pragma unroll
@@ -705,9 +720,10 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             } else {
                 for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                     const int b = c & 1, st = c % kDqStages;
-                    ok = mbar_wait(&ds_full[b], (c >> 1) & 1, status) && ok;      // (implies S / dP of the tile are done with K and V)
-                    if (j == 0 && qi > 0) ok = mbar_wait(dq_free, (qi - 1) & 1, status) && ok;     // the previous item's dQ has been read
+                    ok = ok && mbar_wait(&ds_full[b], (c >> 1) & 1, status);      // (implies S / dP of the tile are done with K and V)
+                    if (j == 0 && qi > 0) ok = ok && mbar_wait(dq_free, (qi - 1) & 1, status);     // the previous item's dQ has been read
                     ok = warp_ok(ok);
+                    if (!ok) break;
                     tc_fence_after();
                     if (leader) {
                         const uint32_t b_lo = k_mn_lo + (uint32_t)(st * ((2 * kKt) >> 4));
@@ -736,7 +752,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
         int c = 0, qi = 0;
         // One row of an item's Q (group 0) or dO (group 1) to TMEM.  Not before the last S / dP products of the item before are done.
         auto take_row = [&]() {
-            ok = mbar_wait(qd_full, qi & 1, status) && ok;
+            ok = ok && mbar_wait(qd_full, qi & 1, status);
             ++qi;
             const uint8_t* src = sb ? sDO : sQ;
             uint32_t x[2][32];
@@ -787,7 +803,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                 const int b = c & 1;
                 const int R0 = m.row_lo + j * BK;
                 const int c_lo = max(0, lo_r - R0), c_hi = min(BK, hi_r - R0 + 1);
-                ok = mbar_wait(&sdp_full[b], (c >> 1) & 1, status) && ok;
+                ok = ok && mbar_wait(&sdp_full[b], (c >> 1) & 1, status);
                 tc_fence_after();
                 uint32_t dd[HC / 2];
                 const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == BK);
@@ -830,16 +846,14 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             // ---- epilogue of the item: this group's 64 of the 128 dQ columns
             const bool full_tile = m.ne == p.TPT && p.G * p.TPT == kTileRows && m.nblk > 0;
             if (m.nblk > 0) {
-                ok = mbar_wait(&ds_empty[(c - 1) & 1], ((c - 1) >> 1) & 1, status) && ok;      // the item's last dQ product is done
+                ok = ok && mbar_wait(&ds_empty[(c - 1) & 1], ((c - 1) >> 1) & 1, status);      // the item's last dQ product is done
                 tc_fence_after();
             }
             ET* drow = reinterpret_cast<ET*>(p.dq) + ((int64_t)tok * p.Hq + (m.h * p.G + g)) * D + sb * 64;
             uint8_t* stage = sOut + sb * kOut;
-            if (full_tile) {                             // the slab of the item before has left it
-                if (quarter == 0 && lane == 0) bulk_wait_read0();
-                if (sb == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-                else asm volatile("bar.sync 2, 128;" ::: "memory");
-            }
+            // the slab of the item before has left its place; and the four warps go on, or give up, together
+            if (quarter == 0 && lane == 0) bulk_wait_read0();
+            ok = bar_all(1 + sb, 128, ok);
 #pragma unroll
             for (int c0 = 0; c0 < 64; c0 += 32) {
                 uint32_t a[32];

@@ -218,24 +218,26 @@ __global__ void __launch_bounds__(128, 1) sel_bwd_main(const SelBwdParams<ET> p,
 
         // ---- stage 3: S = Q K^T, dP = dO V^T
         if (tid == 0) {
-            if (new_kv) ok = mbar_wait(&bar_kv, kv_loads & 1, status);
+            if (new_kv) ok = ok && mbar_wait(&bar_kv, kv_loads & 1, status);
             tc_fence_after();
+            if (ok) {
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t a = smem_u32(sQ + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
-                uint32_t b = smem_u32(sK + (ks >> 2) * (kKT * 128)) + (ks & 3) * 32;
-                umma_ss(tbase + C::cS, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
-            }
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    uint32_t a = smem_u32(sQ + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
+                    uint32_t b = smem_u32(sK + (ks >> 2) * (kKT * 128)) + (ks & 3) * 32;
+                    umma_ss(tbase + C::cS, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
+                }
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t a = smem_u32(sDO + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
-                uint32_t b = smem_u32(sV + (ks >> 2) * (kKT * 128)) + (ks & 3) * 32;
-                umma_ss(tbase + C::cDP, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    uint32_t a = smem_u32(sDO + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
+                    uint32_t b = smem_u32(sV + (ks >> 2) * (kKT * 128)) + (ks & 3) * 32;
+                    umma_ss(tbase + C::cDP, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
+                }
+                umma_commit(&bar_a);
             }
-            umma_commit(&bar_a);
         }
         if (new_kv) ++kv_loads;
-        ok = mbar_wait(&bar_a, it & 1, status) && ok;
+        ok = ok && mbar_wait(&bar_a, it & 1, status);
         tc_fence_after();
 
         // ---- stage 4: P and dS rows -> smem (K-major rows of 64 keys)
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(128, 1) sel_bwd_main(const SelBwdParams<ET> p,
         __syncthreads();
 
         // ---- stage 5: dQ = dS K ; dK^T += Q^T dS ; dV^T += dO^T P
-        if (tid == 0) {
+        if (tid == 0 && ok) {
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < kKT / 16; ++ks) {
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(128, 1) sel_bwd_main(const SelBwdParams<ET> p,
         have_acc = true;
         cur_h = h;
         cur_row0 = row0;
-        ok = mbar_wait(&bar_b, it & 1, status) && ok;
+        ok = ok && mbar_wait(&bar_b, it & 1, status);
         tc_fence_after();
 
         // ---- stage 6: dQ partial -> global

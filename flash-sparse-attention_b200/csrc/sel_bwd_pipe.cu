@@ -197,18 +197,19 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
             BT_TOC(0);
-            ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&off_full[st], (k >> 1) & 1);
             BT_TOC(2);
             int2 off[NIT];                              // (all of them ahead of the copies)
 #pragma unroll
             for (int it = 0; it < NIT; ++it) off[it] = s_off[st][rbase + it * RSTEP];
             ok = warp_ok(ok);
+            if (!ok) break;
             if (lane == 0) mbar_arrive(&off_empty[st]);
             // dO first: dV, its last reader, is issued before dK, the last reader of Q
             // (RSTEP is a multiple of 8: the rows of a thread have one swizzle)
             const uint32_t dq_ = smem_u32(sQD + st * kQD) + slab_off + sw128_chunk_off(rbase, cchunk & 7);
             const uint32_t dd_ = dq_ + kTileRows * D * 2;
-            ok = mbar_poll(&do_empty[st], ((k >> 1) & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(&do_empty[st], ((k >> 1) & 1) ^ 1);
             BT_EV(k, 0, t == 0);
             BT_TOC(1);
 #pragma unroll
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
             cp_async_mbar_arrive_noinc(&do_full[st]);
             BT_TOC(4);
-            ok = mbar_poll(&q_empty[st], ((k >> 1) & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(&q_empty[st], ((k >> 1) & 1) ^ 1);
             BT_TOC(1);
 #pragma unroll
             for (int it = 0; it < NIT; ++it) {
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         for (int k = 0; k < nloc && ok; ++k) {
             // ---- dQ partial of this tile
             BT_TOC(0);
-            ok = mbar_poll(dq_full, k & 1) && ok;
+            ok = ok && mbar_poll(dq_full, k & 1);
             BT_EV(k, 13, warp == kWFlush && lane == 0);
             BT_TOC(1);
             tc_fence_after();
@@ -280,16 +281,16 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_2d(&dqmap, b * 64, rec.y * kTileRows + quarter * 32, smem_u32(my_stage));
+                    if (ok) tma_store_2d(&dqmap, b * 64, rec.y * kTileRows + quarter * 32, smem_u32(my_stage));
                     bulk_commit();
                 }
             }
             BT_TOC(2);
-            if (!(rec.x & 2)) continue;
+            if (!ok || !(rec.x & 2)) continue;
             // ---- dK^T / dV^T of the finished segment (the segments of a key are numbered by the scheduling run they fall into)
             const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
             float* slab = p.slabs + ((int64_t)seg * nsub + (rec.y - rec.z * nsub)) * (2 * KT * D) + d_idx;
-            ok = mbar_poll(acc_full, nflush & 1) && ok;
+            ok = ok && mbar_poll(acc_full, nflush & 1);
             BT_TOC(3);
             tc_fence_after();
 #pragma unroll 1
@@ -330,24 +331,25 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         for (int k = 0; k < nloc && ok; ++k) {
             const int st = k & 1;
             BT_TOC(0);
-            ok = mbar_poll(&off_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&off_full[st], (k >> 1) & 1);
             BT_TOC(1);
             const int seg = s_rec[k & 15].x;
-            ok = warp_ok(ok);
+            __syncwarp();
             if (lane == 0) mbar_arrive(&off_empty[st]);
             if (seg & 1) {
                 ++kvn;
-                ok = mbar_poll(v_full, kvn & 1) && ok;
+                ok = ok && mbar_poll(v_full, kvn & 1);
             }
             BT_TOC(2);
-            ok = mbar_poll(&sdp_empty[st], ((k >> 1) & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(&sdp_empty[st], ((k >> 1) & 1) ^ 1);
             BT_EV(k, 3, lane == 0);
             BT_TOC(4);
-            ok = mbar_poll(&do_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&do_full[st], (k >> 1) & 1);
             BT_EV(k, 2, lane == 0);
             BT_TOC(3);
             fence_async_smem();
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             const uint32_t aq = qd_lo + (uint32_t)(st * (kQD >> 4));
             const uint32_t ad = aq + (uint32_t)((kTileRows * D * 2) >> 4);
@@ -364,12 +366,13 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
             __syncwarp();
             BT_TOC(5);
-            if (seg & 1) ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
+            if (seg & 1) ok = ok && mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1);
             BT_TOC(2);
-            ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&q_full[st], (k >> 1) & 1);
             BT_TOC(3);
             fence_async_smem();
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -401,20 +404,21 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             const int st = k & 1;
             BT_TOC(0);
             // (the record is complete: its tile has been through the S / dP issuer when P is there)
-            ok = mbar_poll(p_full, k & 1) && ok;
+            ok = ok && mbar_poll(p_full, k & 1);
             BT_EV(k, 9, lane == 0);
             BT_TOC(1);
             const int seg = s_rec[k & 15].x;
             const bool first_of_block = seg & 1, last_of_block = seg & 2;
             if (first_of_block) { ++kvn; ++blk; }
-            if (first_of_block && blk > 0) ok = mbar_poll(acc_empty, (blk - 1) & 1) && ok;
+            if (first_of_block && blk > 0) ok = ok && mbar_poll(acc_empty, (blk - 1) & 1);
             BT_TOC(4);
-            ok = mbar_poll(&do_full[st], (k >> 1) & 1) && ok;     // already complete: acquire only
-            ok = mbar_poll(&q_full[st], (k >> 1) & 1) && ok;
-            ok = mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1) && ok;
+            ok = ok && mbar_poll(&do_full[st], (k >> 1) & 1);     // already complete: acquire only
+            ok = ok && mbar_poll(&q_full[st], (k >> 1) & 1);
+            ok = ok && mbar_poll(&k_full[kvn % kKStages], (kvn / kKStages) & 1);
             BT_TOC(3);
             fence_async_smem();
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             const uint32_t bk = k_mn_lo + (uint32_t)((kvn % kKStages) * (kK >> 4));
             const uint32_t aq = qd_mn_lo + (uint32_t)(st * (kQD >> 4));
@@ -431,10 +435,11 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
             __syncwarp();
             BT_TOC(5);
-            ok = mbar_poll(ds_full, k & 1) && ok;
+            ok = ok && mbar_poll(ds_full, k & 1);
             BT_TOC(2);
             fence_async_smem();
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             if (leader) {
 #pragma unroll 4
@@ -446,9 +451,10 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             }
             __syncwarp();
             BT_EV(k, 10, lane == 0);
-            ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(dq_empty, (k & 1) ^ 1);
             BT_EV(k, 11, lane == 0);
             ok = warp_ok(ok);
+            if (!ok) break;
             tc_fence_after();
             if (leader) {
 #pragma unroll
@@ -495,7 +501,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             const Pre cur = m1;
             m1 = m2; m2 = m3;
             if (k + 3 < nloc) fetch(m3);
-            ok = mbar_poll(&off_empty[slot], ((k >> 1) & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(&off_empty[slot], ((k >> 1) & 1) ^ 1);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int hq = cur.h * s.G + (int)(gg >> (8 * i) & 255), tok = (int)(cur.e[i] >> kSlotBits);
@@ -530,14 +536,18 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ++kvn;
             if (lane == 0) {
                 const int ks = kvn % kKStages;
-                ok = mbar_poll(&k_empty[ks], ((kvn / kKStages) & 1) ^ 1) && ok;
-                mbar_expect_tx(&k_full[ks], (uint32_t)kK);
+                ok = ok && mbar_poll(&k_empty[ks], ((kvn / kKStages) & 1) ^ 1);
+                if (ok) {
+                    mbar_expect_tx(&k_full[ks], (uint32_t)kK);
 #pragma unroll
-                for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sK + ks * kK + b * KT * 128), &kmap, cur.h * D + b * 64, row, &k_full[ks]);
-                ok = mbar_poll(v_empty, (kvn & 1) ^ 1) && ok;
-                mbar_expect_tx(v_full, (uint32_t)kK);
+                    for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sK + ks * kK + b * KT * 128), &kmap, cur.h * D + b * 64, row, &k_full[ks]);
+                }
+                ok = ok && mbar_poll(v_empty, (kvn & 1) ^ 1);
+                if (ok) {
+                    mbar_expect_tx(v_full, (uint32_t)kK);
 #pragma unroll
-                for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sV + b * KT * 128), &vmap, cur.h * D + b * 64, row, v_full);
+                    for (int b = 0; b < D / 64; ++b) tma_load_2d(smem_u32(sV + b * KT * 128), &vmap, cur.h * D + b * 64, row, v_full);
+                }
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
@@ -605,7 +615,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             // most tiles are fully visible to all their rows (only a token's own block is cut by causality)
             const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == KT);
             // dP comes first (its rows are gathered first): scale (dP - delta) is ready when S arrives
-            ok = mbar_poll(&dp_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&dp_full[st], (k >> 1) & 1);
             tc_fence_after();
             uint32_t sv[32], dv[32], pp[HC / 2];
             tmem_ld32(tbase + lane_off + cDP + st * 128 + cb, dv);
@@ -613,7 +623,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
 #pragma unroll
             for (int i = 0; i < 32; ++i) dv[i] = __float_as_uint(fmaf(__uint_as_float(dv[i]), p.scale, -delta_s));
             BT_TOC(5);
-            ok = mbar_poll(&s_full[st], (k >> 1) & 1) && ok;
+            ok = ok && mbar_poll(&s_full[st], (k >> 1) & 1);
             BT_EV(k, 5, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(1);
             tc_fence_after();
@@ -640,7 +650,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             BT_EV(k, 6, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(2);
             // P first: dV starts while dS is being written
-            ok = mbar_poll(p_empty, (k & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(p_empty, (k & 1) ^ 1);
             BT_EV(k, 7, sb == 0 && quarter == 0 && lane == 0);
             BT_TOC(3);
 #pragma unroll
@@ -649,7 +659,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             fence_async_smem();
             mbar_arrive(p_full);
             BT_TOC(4);
-            ok = mbar_poll(ds_empty, (k & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(ds_empty, (k & 1) ^ 1);
             BT_TOC(3);
 #pragma unroll
             for (int c4 = 0; c4 < HC / 8; ++c4)

@@ -140,14 +140,16 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         };
         for (int k = 0; k < nloc && ok; ++k) {
             const int slot = k % kRing;
-            ok = mbar_poll(&off_full[slot], (k / kRing) & 1) && ok;
-            ok = mbar_poll(q_empty, (k & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(&off_full[slot], (k / kRing) & 1);
+            ok = ok && mbar_poll(q_empty, (k & 1) ^ 1);
+            ok = warp_ok(ok);
+            if (!ok) break;
             copy(p.q, sQ, s_off[slot][0]);
             cp_async_mbar_arrive_noinc(q_full);
-            ok = mbar_poll(do_empty, (k & 1) ^ 1) && ok;
+            ok = ok && mbar_poll(do_empty, (k & 1) ^ 1);
             copy(p.d_o, sDO, s_off[slot][1]);
             cp_async_mbar_arrive_noinc(do_full);
-            ok = warp_ok(ok);
+            __syncwarp();
             if (lane == 0) mbar_arrive(&off_empty[slot]);
         }
     } else if (warp >= kWDrain && warp < kWDrain + 4) {
@@ -158,14 +160,15 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         int nflush = 0;
 #pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
-            ok = mbar_poll(dq_full, k & 1) && ok;
+            ok = ok && mbar_poll(dq_full, k & 1);
             const int4 rec = s_rec[k & 7];
             ok = warp_ok(ok);
+            if (!ok) break;
             if (lane == 0) mbar_arrive(dq_empty);                // (no tile gets two ahead of this warp)
             if (!(rec.x & 2)) continue;
             const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
             float* slab = p.slabs + ((int64_t)seg * p.nsub + (rec.y - rec.z * p.nsub)) * (2 * KT * D) + quarter * 32 + lane;
-            ok = mbar_poll(acc_full, nflush & 1) && ok;
+            ok = ok && mbar_poll(acc_full, nflush & 1);
             tc_fence_after();
 #pragma unroll 1
             for (int part = 0; part < 4; ++part) {               // dK low, dK high, dV low, dV high half of the head dimension
@@ -197,18 +200,19 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             int kvn = -1;
             for (int k = 0; k < nloc && ok; ++k) {
                 const int slot = k % kRing;
-                ok = mbar_poll(&off_full[slot], (k / kRing) & 1) && ok;
+                ok = ok && mbar_poll(&off_full[slot], (k / kRing) & 1);
                 const int seg = s_rec[k & 7].x;
-                ok = warp_ok(ok);
+                __syncwarp();
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (seg & 1) {
                     ++kvn;
-                    ok = mbar_poll(kv_full, kvn & 1) && ok;
+                    ok = ok && mbar_poll(kv_full, kvn & 1);
                 }
-                ok = mbar_poll(dq_empty, (k & 1) ^ 1) && ok;
-                ok = mbar_poll(q_full, k & 1) && ok;
+                ok = ok && mbar_poll(dq_empty, (k & 1) ^ 1);
+                ok = ok && mbar_poll(q_full, k & 1);
                 fence_async_smem();
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 4
@@ -217,9 +221,10 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                                 umma_desc_pack(k_lo + (ks >> 2) * kSlabB + (ks & 3) * 2, hi_1024), idesc, ks > 0);
                 }
                 __syncwarp();
-                ok = mbar_poll(do_full, k & 1) && ok;
+                ok = ok && mbar_poll(do_full, k & 1);
                 fence_async_smem();
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 4
@@ -244,17 +249,18 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
 #pragma unroll 1
             for (int k = 0; k < nloc && ok; ++k) {
                 // (the record is complete: its tile has been through the S / dP issuer when P is there)
-                ok = mbar_poll(pds_full, k & 1) && ok;
+                ok = ok && mbar_poll(pds_full, k & 1);
                 const int seg = s_rec[k & 7].x;
                 const bool first = seg & 1, last = seg & 2;
                 if (first) ++blk;
                 // (complete already: acquire only)
-                ok = mbar_poll(kv_full, blk & 1) && ok;
-                ok = mbar_poll(q_full, k & 1) && ok;
-                ok = mbar_poll(do_full, k & 1) && ok;
-                if (first && blk > 0) ok = mbar_poll(acc_empty, (blk - 1) & 1) && ok;
+                ok = ok && mbar_poll(kv_full, blk & 1);
+                ok = ok && mbar_poll(q_full, k & 1);
+                ok = ok && mbar_poll(do_full, k & 1);
+                if (first && blk > 0) ok = ok && mbar_poll(acc_empty, (blk - 1) & 1);
                 fence_async_smem();
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 if (leader) {
 #pragma unroll 2
@@ -304,7 +310,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             };
             auto publish = [&](int k, Pre& m, const Pre& next) {
                 const int slot = k % kRing;
-                ok = mbar_poll(&off_empty[slot], ((k / kRing) & 1) ^ 1) && ok;
+                ok = ok && mbar_poll(&off_empty[slot], ((k / kRing) & 1) ^ 1);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int tok = (int)(m.e[i] >> kSlotBits), hq = m.h * s.G + gg[i];
@@ -342,12 +348,14 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 prev_hg = ti.hg;
                 ++kvn;
                 if (lane == 0) {
-                    ok = mbar_poll(kv_empty, (kvn & 1) ^ 1) && ok;
-                    mbar_expect_tx(kv_full, (uint32_t)(2 * kK));
+                    ok = ok && mbar_poll(kv_empty, (kvn & 1) ^ 1);
+                    if (ok) {
+                        mbar_expect_tx(kv_full, (uint32_t)(2 * kK));
 #pragma unroll
-                    for (int b = 0; b < D / 64; ++b) {
-                        tma_load_2d(smem_u32(sK + b * KT * 128), &kmap, ti.h * D + b * 64, row, kv_full);
-                        tma_load_2d(smem_u32(sV + b * KT * 128), &vmap, ti.h * D + b * 64, row, kv_full);
+                        for (int b = 0; b < D / 64; ++b) {
+                            tma_load_2d(smem_u32(sK + b * KT * 128), &kmap, ti.h * D + b * 64, row, kv_full);
+                            tma_load_2d(smem_u32(sV + b * KT * 128), &vmap, ti.h * D + b * 64, row, kv_full);
+                        }
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -395,7 +403,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             const float lse_r = lse_n, delta_s = delta_n * p.scale;
             const int c_lo = lo_n, c_hi = hi_n;
             if (k + 1 < nloc) fetch_ent();
-            ok = mbar_poll(sdp_full, k & 1) && ok;
+            ok = ok && mbar_poll(sdp_full, k & 1);
             tc_fence_after();
             uint32_t pp[HC / 2], dd[HC / 2];
             {
@@ -421,7 +429,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 }
             }
             tc_fence_before();
-            if (k > 0) ok = mbar_poll(pds_free, (k - 1) & 1) && ok;
+            if (k > 0) ok = ok && mbar_poll(pds_free, (k - 1) & 1);
 #pragma unroll
             for (int c4 = 0; c4 < HC / 8; ++c4) {
                 const uint32_t off = sw128_chunk_off(r, sb * (HC / 8) + c4);
@@ -433,7 +441,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
             if (k + 1 < nloc) fetch_stats();
             // ---- dQ of the tile: this group's 128 columns to registers, which frees its TMEM columns for the next S and dP, and from
             // there 64 at a time through the P / dS buffers, which the products have read
-            ok = mbar_poll(dq_full, k & 1) && ok;
+            ok = ok && mbar_poll(dq_full, k & 1);
             tc_fence_after();
             const int row = s_rec[k & 7].y * kTileRows + quarter * 32;
             uint32_t x[64];
@@ -456,7 +464,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_2d(&dqmap, sb * 128 + half * 64, row, smem_u32(my_stage));
+                    if (ok) tma_store_2d(&dqmap, sb * 128 + half * 64, row, smem_u32(my_stage));
                     bulk_commit();
                     bulk_wait_read0();
                     if (half == 1) mbar_arrive(pds_free);

@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         for (int k = 0; k < nloc && ok; ++k) {
             const int slot = k % kFwdRing;
             // the Q stage is free once the S MMA of the tile that used it is done
-            ok = mbar_poll(&q_empty[qs], qph) && ok;
-            ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+            ok = ok && mbar_poll(&q_empty[qs], qph);
+            ok = ok && mbar_poll(&off_full[slot], (k / kFwdRing) & 1);
             const int hq0 = s_rec[slot].x * s.G * qsh8;
             const uint32_t dst = dst0 + qs * C::kQ;
             constexpr int NB = 8;                              // rows whose offsets are read together, ahead of their copies
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 for (int it = 0; it < NB; ++it) {
                     const int r = rbase + (i0 + it) * RSTEP;
                     const uint32_t ent = s_ent[slot][r];
-                    off[it] = ent != 0xFFFFFFFFu ? (int)(ent >> kSlotBits) * qsn8 + hq0 + s_goff[r] : -1;
+                    off[it] = ok && ent != 0xFFFFFFFFu ? (int)(ent >> kSlotBits) * qsn8 + hq0 + s_goff[r] : -1;
                 }
 #pragma unroll
                 for (int it = 0; it < NB; ++it)
@@ -201,18 +201,19 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 #pragma unroll 1
             for (int k = 0; k < nloc && ok; ++k) {
                 const int sbuf = k % C::NS, slot = k % kFwdRing;
-                ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+                ok = ok && mbar_poll(&off_full[slot], (k / kFwdRing) & 1);
                 const int blk = s_rec[slot].y;
-                ok = warp_ok(ok);
+                __syncwarp();
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (blk & 1) {
                     ++kvn;
-                    ok = mbar_poll(&kv_full[kvn % C::NKV], (kvn / C::NKV) & 1) && ok;
+                    ok = ok && mbar_poll(&kv_full[kvn % C::NKV], (kvn / C::NKV) & 1);
                 }
-                ok = mbar_poll(&q_full[qs], qph) && ok;
+                ok = ok && mbar_poll(&q_full[qs], qph);
                 fence_async_smem();   // the Q rows were written by cp.async (generic proxy)
-                ok = mbar_poll(&s_empty[sbuf], ((k / C::NS) & 1) ^ 1) && ok;
+                ok = ok && mbar_poll(&s_empty[sbuf], ((k / C::NS) & 1) ^ 1);
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 const uint32_t a_lo = q_lo + (uint32_t)(qs * (C::kQ >> 4));
                 const uint32_t b_lo = k_lo + (uint32_t)((kvn % C::NKV) * (C::kKV >> 4));
@@ -241,14 +242,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 #pragma unroll 1
             for (int k = 0; k < nloc && ok; ++k) {
                 const int ob = k % C::NO, sbuf = k % C::NS, slot = k % kFwdRing;
-                ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
+                ok = ok && mbar_poll(&off_full[slot], (k / kFwdRing) & 1);
                 const int blk = s_rec[slot].y;
-                ok = warp_ok(ok);
+                __syncwarp();
                 if (lane == 0) mbar_arrive(&off_empty[slot]);
                 if (blk & 1) ++kvn;
-                ok = mbar_poll(&o_empty[ob], ((k / C::NO) & 1) ^ 1) && ok;
-                ok = mbar_poll(&p_full[sbuf], (k / C::NS) & 1) && ok;
+                ok = ok && mbar_poll(&o_empty[ob], ((k / C::NO) & 1) ^ 1);
+                ok = ok && mbar_poll(&p_full[sbuf], (k / C::NS) & 1);
                 ok = warp_ok(ok);
+                if (!ok) break;
                 tc_fence_after();
                 const int kv_cur = kvn % C::NKV;
                 const uint32_t b_lo = v_lo + (uint32_t)(kv_cur * (C::kKV >> 4));
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             // publishes tile k from m and fetches tile k + 3 into it (three in turn: handing the registers on would wait for the loads)
             auto publish = [&](int k, Pre& m, const Pre& next) {
                 const int slot = k % kFwdRing;
-                ok = mbar_poll(&off_empty[slot], ((k / kFwdRing) & 1) ^ 1) && ok;
+                ok = ok && mbar_poll(&off_empty[slot], ((k / kFwdRing) & 1) ^ 1);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) s_ent[slot][lane + 32 * i] = m.e[i];
                 if (lane == 0)
@@ -324,14 +326,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 ++kvn;
                 if (lane == 0) {
                     const int ks = kvn % C::NKV;
-                    ok = mbar_poll(&kv_empty[ks], ((kvn / C::NKV) & 1) ^ 1) && ok;
-                    mbar_expect_tx(&kv_full[ks], (uint32_t)C::kKV);
-                    uint8_t* dK = sKV + ks * C::kKV;
-                    uint8_t* dV = dK + BK * D * 2;
+                    ok = ok && mbar_poll(&kv_empty[ks], ((kvn / C::NKV) & 1) ^ 1);
+                    if (ok) {
+                        mbar_expect_tx(&kv_full[ks], (uint32_t)C::kKV);
+                        uint8_t* dK = sKV + ks * C::kKV;
+                        uint8_t* dV = dK + BK * D * 2;
 #pragma unroll
-                    for (int b = 0; b < D / 64; ++b) {
-                        tma_load_2d(smem_u32(dK + b * BK * 128), &kmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
-                        tma_load_2d(smem_u32(dV + b * BK * 128), &vmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
+                        for (int b = 0; b < D / 64; ++b) {
+                            tma_load_2d(smem_u32(dK + b * BK * 128), &kmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
+                            tma_load_2d(smem_u32(dV + b * BK * 128), &vmap, cur.h * D + b * 64, cur.row0, &kv_full[ks]);
+                        }
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -354,8 +358,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         int c_lo = 0, c_hi = BK;
         auto fetch = [&](int k) {
             const int slot = k % kFwdRing;
-            ok = mbar_poll(&off_full[slot], (k / kFwdRing) & 1) && ok;
-            ent = s_ent[slot][r];
+            ok = ok && mbar_poll(&off_full[slot], (k / kFwdRing) & 1);
+            ent = ok ? s_ent[slot][r] : 0xFFFFFFFFu;
             const int4 rec = s_rec[slot];
             __syncwarp();
             if (lane == 0) mbar_arrive(&off_empty[slot]);
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         for (int k = sb; k < nloc && ok; k += 2) {
             const int sbuf = k % C::NS;
             const uint32_t tS = tS0 + sbuf * BK;
-            ok = mbar_poll(&s_full[sbuf], (k / C::NS) & 1) && ok;
+            ok = ok && mbar_poll(&s_full[sbuf], (k / C::NS) & 1);
             tc_fence_after();
             // A row is held in registers W = 32 or 64 columns at a time: one TMEM read for a block of that size.  128 columns: the upper half
             // is read for its maximum, then the lower one, which stays, then (P of the lower half is in its place, over S) the upper one
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
 #pragma unroll 1
         for (int k = 0; k < nloc && ok; ++k) {
             const int ob = k % C::NO;
-            ok = mbar_poll(&o_full[ob], (k / C::NO) & 1) && ok;
+            ok = ok && mbar_poll(&o_full[ob], (k / C::NO) & 1);
             tc_fence_after();
 #pragma unroll 1
             for (int b = 0; b < D / 64; ++b) {
@@ -483,7 +487,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_2d_hint(&omap, b * 64, cur.j * kTileRows + quarter * 32, smem_u32(stage), pol_part);
+                    if (ok) tma_store_2d_hint(&omap, b * 64, cur.j * kTileRows + quarter * 32, smem_u32(stage), pol_part);
                     bulk_commit();
                 }
                 if (++slab == C::NSL) slab = 0;
@@ -579,18 +583,20 @@ __global__ void __launch_bounds__(128, 1) sel_fwd_simple(const SelFwdParams<ET> 
         tc_fence_before();
         __syncthreads();
         if (tid == 0) {
-            if (new_kv) ok = mbar_wait(&bar_kv, kv_loads & 1, status);
+            if (new_kv) ok = ok && mbar_wait(&bar_kv, kv_loads & 1, status);
             tc_fence_after();
+            if (ok) {
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t a = smem_u32(sQ + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
-                uint32_t b = smem_u32(sK + (ks >> 2) * (BK * 128)) + (ks & 3) * 32;
-                umma_ss(tS, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    uint32_t a = smem_u32(sQ + (ks >> 2) * (kTileRows * 128)) + (ks & 3) * 32;
+                    uint32_t b = smem_u32(sK + (ks >> 2) * (BK * 128)) + (ks & 3) * 32;
+                    umma_ss(tS, umma_desc_sw128(a, 16, 1024), umma_desc_sw128(b, 16, 1024), idesc_s, ks > 0);
+                }
+                umma_commit(&bar_s);
             }
-            umma_commit(&bar_s);
         }
         if (new_kv) ++kv_loads;
-        ok = mbar_wait(&bar_s, it & 1, status) && ok;
+        ok = ok && mbar_wait(&bar_s, it & 1, status);
         tc_fence_after();
         const int r = tid;
         const int g = r / s.TPT, e = r - g * s.TPT;
@@ -628,7 +634,7 @@ __global__ void __launch_bounds__(128, 1) sel_fwd_simple(const SelFwdParams<ET> 
         tmem_st_wait();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
+        if (tid == 0 && ok) {
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < BK / 16; ++ks) {
@@ -637,7 +643,7 @@ __global__ void __launch_bounds__(128, 1) sel_fwd_simple(const SelFwdParams<ET> 
             }
             umma_commit(&bar_o);
         }
-        ok = mbar_wait(&bar_o, it & 1, status) && ok;
+        ok = ok && mbar_wait(&bar_o, it & 1, status);
         tc_fence_after();
         {
             const int64_t grow = (int64_t)item * kTileRows + r;

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFuse
     const int nkt = ((t_last / p.BK + 1) * BS + kSfKeys - 1) / kSfKeys;     // key tiles that hold a causal block of the tile
     const bool have_keys = ncmp > 0;       // a sequence shorter than the compression window has none: every probability is 0
     int* status = p.status;
+    const uint32_t limit = wait_limit(status);
 
     if (tid == 0) {
         mbar_init(q_full, 1);
@@ -142,10 +143,10 @@ __global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFuse
         for (int sl = 0; sl < D / 64; ++sl)
             tma_load_2d(smem_u32(sQ + sl * kSfRows * 128), &qmap, (h * p.G) * D + sl * 64, n0, q_full);
         load_k(0);
-        ok = mbar_wait(q_full, 0, status) && ok;
-        ok = mbar_wait(k_full, 0, status) && ok;
+        ok = ok && mbar_wait(q_full, 0, status, limit);
+        ok = ok && mbar_wait(k_full, 0, status, limit);
         tc_fence_after();
-        issue_mma(0);
+        if (ok) issue_mma(0);
     }
 
     // this thread's row
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFuse
         const int buf = kt & 1;
         // S(kt) done: the K tile may be loaded over.  S(kt + 1) is issued between the two groups of columns of this tile: the keys have
         // landed by then, and its TMEM buffer was read in iteration kt - 1, before the barrier that ended it
-        if (have_keys) ok = mbar_wait(&s_full[buf], (kt >> 1) & 1, status) && ok;
+        if (have_keys) ok = ok && mbar_wait(&s_full[buf], (kt >> 1) & 1, status, limit);
         tc_fence_after();
         if (tid == 0 && have_keys && kt + 1 < nkt) load_k(kt + 1);
         __syncwarp();
@@ -206,9 +207,9 @@ __global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFuse
                 }
             }
             if (c32 == 0 && tid == 0 && have_keys && kt + 1 < nkt) {
-                ok = mbar_wait(k_full, (kt + 1) & 1, status) && ok;
+                ok = ok && mbar_wait(k_full, (kt + 1) & 1, status, limit);
                 tc_fence_after();
-                issue_mma(kt + 1);
+                if (ok) issue_mma(kt + 1);
             }
             __syncwarp();
         }
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(128, 4) select_topk_fused_kernel(const SelFuse
     }
     // (on a wait that ran out: a key tile in flight lands before the CTA ends)
     if (!ok && tid == 0 && have_keys)
-        for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait(k_full, ph, nullptr);
+        for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait(k_full, ph, nullptr, limit);
 
     if (valid) {
         // the first min(T_out, nb) entries are the selection; ascending ids, -1 tail

@@ -116,24 +116,31 @@ __device__ __forceinline__ uint32_t clock32() {
     asm volatile("mov.u32 %0, %%clock;" : "=r"(t)::"memory");
     return t;
 }
-// Bounded wait: polls until the phase completes or FSA_WAIT_CLOCKS cycles of the SM have passed (each try_wait already
-// sleeps for a while in hardware) and returns false in the second case; the caller keeps going so that TMEM is freed and
-// the kernel returns.  mbar_wait records the failure in the status word; mbar_poll leaves that to the caller, once for all
-// its waits.  Kept short on purpose: a warp-specialised kernel has some 25 waits, and the loops of its roles together have
-// to stay in the SM's instruction cache (sel_bwd_pipe.cu).
+// Bounded wait: polls until the phase completes or `limit` cycles of the SM have passed (each try_wait already sleeps for a
+// while in hardware) and returns false in the second case.  A role's first wait that runs out is its last (`ok = ok && ...`): from
+// there on it issues nothing and uses no address that the wait was for, and leaves its loop, so that TMEM is freed and the
+// kernel returns.  mbar_wait records the failure in the status word; mbar_poll leaves that to the caller, once for all its
+// waits.  Kept short on purpose: a warp-specialised kernel has some 25 waits, and the loops of its roles together have to
+// stay in the SM's instruction cache (sel_bwd_pipe.cu).
 #ifndef FSA_WAIT_CLOCKS
 #define FSA_WAIT_CLOCKS 400000000u   // 0.2 s at 1.965 GHz; less than the 2^32 at which the counter comes round
 #endif
-__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, uint32_t limit = FSA_WAIT_CLOCKS) {
     const uint32_t t0 = clock32();
 #pragma unroll 1
     do {
         if (mbar_try_wait(bar, parity)) return true;
-    } while (clock32() - t0 < FSA_WAIT_CLOCKS);
+    } while (clock32() - t0 < limit);
     return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status) {
-    if (mbar_poll(bar, parity)) return true;
+// The limit of a CTA's waits in kernels of many waves of CTAs: 3 ms where the status word says that a wait has run out already (of a
+// CTA before it, as far as the launch's word was zero).  Read once, by every thread for itself, and not waited for until a wait is slow.
+__device__ __forceinline__ uint32_t wait_limit(const int* status) {
+    const int failed = status ? *reinterpret_cast<const volatile int*>(status) : 0;
+    return failed ? FSA_WAIT_CLOCKS / 64 : FSA_WAIT_CLOCKS;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, uint32_t limit = FSA_WAIT_CLOCKS) {
+    if (mbar_poll(bar, parity, limit)) return true;
     if (status) atomicMax(status, (int)kStatusWaitTimeout);
     return false;
 }

@@ -482,7 +482,7 @@ int fsa_decode_ranges(const int32_t* topk_idx, const int32_t* seq_len, const int
 int fsa_read_status(const void* index_ws, void* stream, int* status_out);
 
 /* Debug/inspection: launch one thread that waits on a barrier nothing will ever signal.  Like every wait of the library
- * it gives up after its bound (0.2 s), records status 1 in the int at status_ws (a zeroed device word, e.g. the start of
+ * it gives up after its bound (0.2 s; 3 ms if the word is set already), records status 1 in the int at status_ws (a zeroed device word, e.g. the start of
  * an index workspace) and returns: fsa_read_status(status_ws, ...) then reports FSA_ERR_DEVICE_STATUS.  Exists so that the
  * failure path of the status plumbing can be tested without hanging or faulting a GPU.  No reference counterpart. */
 int fsa_debug_wait_timeout(void* status_ws, void* stream);

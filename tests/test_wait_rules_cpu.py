@@ -29,3 +29,22 @@ def test_a_warp_meets_between_its_waits_and_what_one_lane_issues(name):
     for at in alone:
         last = max((w for w in waits if w < at), default=None)
         assert last is None or any(last < m < at for m in meets), f"{name}:{line(text, at)}"
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_a_wait_that_ran_out_is_a_roles_last(name):
+    text = code(name)
+    late = [line(text, m.start()) for m in re.finditer(WAIT + r"[^;]*\)\s*&&\s*ok\b", text)]
+    assert not late, f"{name}: lines {late} wait before they look whether an earlier wait ran out"
+
+
+def test_what_is_issued_depends_on_the_wait_before_it():
+    """A tensor copy or product whose wait ran out would be in flight when the CTA ends, or take its place from numbers nobody has written."""
+    for name in SOURCES:
+        text = code(name)
+        for m in re.finditer(r"ok = (?:ok && )?" + WAIT + r"[^;]*;", text):
+            rest = text[m.end():]
+            first = re.search(r"tma_load|tma_store|umma_ss|umma_ts|issue_mma", rest)
+            again = re.search(WAIT, rest)
+            if first and (again is None or first.start() < again.start()):
+                assert re.search(r"if \(!ok\)|if \(ok\)|if \(tid == 0 && ok\)|&& ok;|\bok &&", rest[: first.start()]), f"{name}:{line(text, m.start())}"
