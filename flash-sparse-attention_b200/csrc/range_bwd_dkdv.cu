@@ -21,7 +21,8 @@
 // A tile takes 3100 cycles where every row sees all K/V rows: its products read 256 KB of shared memory and the loads write 64 KB,
 // 2560 cycles (the products alone: 2050).  Tiles that need the mask are bound by the row threads.  Measured at 2 x 32768
 // tokens, 32 / 8 heads (window of 512 and compressed branch together): whole tiles in turns 4.19 ms, halves 3.93; at four sequences
-// of 777 to 3001 tokens, 16 / 4 heads, 119 -> 106 us.
+// of 777 to 3001 tokens, 16 / 4 heads, 119 -> 106 us (104 -> 110 with the waits of a half's S and dP for the product that reads the P
+// or dS in their place; nothing at the larger size, 3.85 ms).
 #include "../../include/fsa_sm100.h"
 #include <climits>
 
@@ -223,8 +224,10 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
     uint64_t* dk_done = s_full + 9;
     uint64_t* dv_free = s_full + 10;    // the accumulator has been read
     uint64_t* dk_free = s_full + 11;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(s_full + 12);
-    int* s_masked = reinterpret_cast<int*>(s_full + 12) + 2;              // [2] some row of the tile does not see all K/V rows
+    uint64_t* p_read = s_full + 12;     // [2 halves] dV(i) has read P
+    uint64_t* ds_read = s_full + 14;    // [2] dK(i) has read dS
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(s_full + 16);
+    int* s_masked = reinterpret_cast<int*>(s_full + 16) + 2;              // [2] some row of the tile does not see all K/V rows
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = p.status;
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         for (int i = 0; i < 2; ++i) {
             mbar_init(&st_full[i], 32); mbar_init(&st_empty[i], 256);
             mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&dp_full[i], 1); mbar_init(&ds_full[i], 128);
+            mbar_init(&p_read[i], 1); mbar_init(&ds_read[i], 1);
         }
         mbar_init(dv_done, 1); mbar_init(dk_done, 1); mbar_init(dv_free, 128); mbar_init(dk_free, 128);
         mbar_init_fence();
@@ -305,14 +309,16 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         const uint32_t b_mn_lo = umma_desc_lo(smem_u32(sU), kSlab);
         const uint32_t c_s = tbase + (first ? cS : cP), c_acc = tbase + (first ? cDV : cDK);
         uint64_t *kv_full = first ? k_full : v_full, *kv_empty = first ? k_empty : v_empty;
-        uint64_t *out_full = first ? s_full : dp_full, *in_full = first ? p_full : ds_full;
+        uint64_t *out_full = first ? s_full : dp_full, *in_full = first ? p_full : ds_full, *in_read = first ? p_read : ds_read;
         uint64_t *acc_done = first ? dv_done : dk_done, *acc_free = first ? dv_free : dk_free;
         bool ok = true;
         int c = 0, qi = 0;
-        // S^T (dP^T) of half a row tile t into its place: in order after the product that read P^T (dS^T) of the tile before from there
+        // S^T (dP^T) of half a row tile t into its place, when the product that reads P^T (dS^T) of the tile before from there is done
+        // (products of two shapes may run in another order than they were issued)
         auto issue_s = [&](int t, int half, bool last) {
             const int u = 2 * t + (first ? 0 : 1), st = u % kRkUnits;
             if (half == 0) ok = ok && mbar_wait(&u_full[st], (u / kRkUnits) & 1, status);
+            if (t > 0) ok = ok && mbar_wait(&in_read[half], (t - 1) & 1, status);
             ok = warp_ok(ok);
             if (!ok) return;
             tc_fence_after();
@@ -351,6 +357,7 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
                         for (int ks = 0; ks < kTileRows / 32; ++ks)
                             umma_ts(c_acc, c_s + half * 64 + ks * 8, umma_desc_pack(bu + ks * (2048 >> 4), hi_1024), idesc_acc,
                                     (i > 0 || half > 0 || ks > 0) ? 1u : 0u);
+                        umma_commit(&in_read[half]);
                         if (half) umma_commit(&u_empty[st]);
                         if (half && i + 1 == m.n) umma_commit(acc_done);
                     }

@@ -269,9 +269,12 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
         const uint32_t v_lo = umma_desc_lo(smem_u32(sV), BK * 128);     // MN-major: LBO = slab stride
         bool ok = true;
         int n = 0, qi = 0, c = 0;
+        // S(t) takes the place of P(t - 2): products of two shapes may run in another order than they were issued, so it waits for the one
+        // that reads P(t - 2) (it was issued before the softmax of tile t - 1 began, and is done by the time that this is reached)
         auto issue_s = [&](int t, bool last) {
             const int st = t & 1;
             ok = ok && mbar_wait(&k_full[st], (t >> 1) & 1, status, limit);
+            if (t >= 2) ok = ok && mbar_wait(&pv_done[st], ((t - 2) >> 1) & 1, status, limit);
             ok = warp_ok(ok);
             if (!ok) return;
             tc_fence_after();
@@ -294,7 +297,6 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             issue_s(c, m.nblk == 1);
             for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                 const int st = c & 1;
-                // S(c + 1) overwrites the buffer P(c - 1) was read from by the product issued one iteration ago (in order)
                 if (j + 1 < m.nblk) issue_s(c + 1, j + 2 == m.nblk);
                 if (j == 0 && qi > 0) ok = ok && mbar_wait(o_free, (qi - 1) & 1, status, limit);
                 ok = ok && mbar_wait(&p_full[st], (c >> 1) & 1, status, limit);

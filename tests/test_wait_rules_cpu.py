@@ -48,3 +48,21 @@ def test_what_is_issued_depends_on_the_wait_before_it():
             again = re.search(WAIT, rest)
             if first and (again is None or first.start() < again.start()):
                 assert re.search(r"if \(!ok\)|if \(ok\)|if \(tid == 0 && ok\)|&& ok;|\bok &&", rest[: first.start()]), f"{name}:{line(text, m.start())}"
+
+
+@pytest.mark.parametrize("name,writes,reads,barrier", [
+    ("sel_fwd.cu", "umma_ss(d_s", "umma_ts(d_o", "s_empty"),
+    ("range_dense.cu", "umma_ss(tbase + cS", "umma_ts(tbase + cO", "pv_done"),
+    ("range_dense.cu", "umma_ts(tbase + b * 128 + BK, tbase + cDO", "umma_ts(tbase + cDQ", "ds_empty"),
+    ("range_bwd_dkdv.cu", "umma_ss(c_s", "umma_ts(c_acc", "in_read"),
+])
+def test_a_product_waits_for_the_one_that_reads_what_it_overwrites(name, writes, reads, barrier):
+    """Products of one thread run in the order of their issue only where accumulator and shape are the same; a commit tells when one is done."""
+    text = code(name)
+    assert text.count(writes) == 1 and text.count(reads) == 1
+    before = text[: text.index(writes)]
+    waits = list(re.finditer(WAIT + r"&" + barrier + r"\[", before))
+    assert waits and "umma_" not in before[waits[-1].end():].replace("umma_desc", "").replace("umma_idesc", ""), f"{name}: {writes}"
+    after = text[text.index(reads):]
+    commit = re.search(r"umma_commit\(&" + barrier + r"\[", after)
+    assert commit and "mbar_" not in after[: commit.start()], f"{name}: {reads}"
