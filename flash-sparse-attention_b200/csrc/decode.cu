@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(160) decode_partial_tma(const DecodeParams p, 
         float* srow = want_scores ? p.scores + ((int64_t)b * p.Hk + h) * p.scores_ld + c * p.chunk : nullptr;
         for (int i = 0; i * kDecKT < n; ++i, ++it) {
             const int s = it % nst;
-            if (!mbar_wait(&full[s], (it / nst) & 1, &g_decode_status, limit)) { ok_wait = false; break; }
+            ok_wait = mbar_wait(&full[s], (it / nst) & 1, &g_decode_status, limit);
+            if (!warp_stays(ok_wait)) break;
             const int k0 = i * kDecKT + warp * 16;               // first key of this warp's tile
             if (k0 < n) {
                 const uint32_t kb = sbase + s * STAGE_BYTES, vb = kb + KV_BYTES;

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
             const int buf = pi & 1;
             ok = ok && mbar_wait(&acc_empty[buf], ((pi >> 1) & 1) ^ 1, status, limit);
             tc_fence_after();
-            for (int q = 0; q < per_phase && ok; ++q, ++i) {
+            for (int q = 0; q < per_phase; ++q, ++i) {       // (left by all lanes at the vote below)
                 const int st = i % kLcDxStages;
                 ok = ok && mbar_wait(&full[st], (i / kLcDxStages) & 1, status, limit);
                 ok = warp_ok(ok);
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(192) linear_compress_dx_kernel(const __grid_co
         const int r = quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         bool ok = true;
-        for (int pi = 0; pi < p.phases && ok; ++pi) {
+        for (int pi = 0; pi < p.phases && warp_stays(ok); ++pi) {
             const int buf = pi & 1;
             if (product) ok = ok && mbar_wait(&acc_full[buf], (pi >> 1) & 1, status, limit);
             tc_fence_after();

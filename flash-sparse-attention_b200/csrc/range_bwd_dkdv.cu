@@ -374,9 +374,9 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         int g[4], e[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) { g[j] = (lane + 32 * j) / TPT; e[j] = lane + 32 * j - g[j] * TPT; }
-        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+        for (int w = blockIdx.x; w < nitems && warp_stays(ok); w += gridDim.x) {
             const RkItem m = rk_item(p.plan, w);
-            for (int i = 0; i < m.n && ok; ++i, ++c) {
+            for (int i = 0; i < m.n && warp_stays(ok); ++i, ++c) {
                 float lse[4], del[4];
                 int lo[4], hi[4];
 #pragma unroll
@@ -425,9 +425,9 @@ __global__ void __launch_bounds__(kRkThreads, 1) range_bwd_dkdv(const RangeKvPar
         const uint32_t tS = tbase + lane_off + cS + grp * 64, tP = tbase + lane_off + cP + grp * 64;
         bool ok = true;
         int c = 0, qi = 0;
-        for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+        for (int w = blockIdx.x; w < nitems && warp_stays(ok); w += gridDim.x) {
             const RkItem m = rk_item(p.plan, w);
-            for (int i = 0; i < m.n && ok; ++i, ++c) {
+            for (int i = 0; i < m.n && warp_stays(ok); ++i, ++c) {
                 const int b = c & 1;
                 ok = ok && mbar_wait(&st_full[b], (c >> 1) & 1, status);
                 ok = ok && mbar_wait(&s_full[grp], c & 1, status);

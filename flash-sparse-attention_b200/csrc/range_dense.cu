@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             const int lo_r = sees.x - m.row_lo, hi_r = min(sees.y, (int)launch.p[m.z].Nk - 1) - m.row_lo;      // rows past the end of K/V do not exist
             const int nblk = m.nblk;
             float m_ref = -INFINITY, l_run = 0.f;
-            for (int j = 0; j < nblk && ok; ++j, ++c) {
+            for (int j = 0; j < nblk && warp_stays(ok); ++j, ++c) {
                 const int st = c & 1;
                 const int c_lo = max(0, lo_r - j * BK), c_hi = min(BK, hi_r - j * BK + 1);      // visible columns [c_lo, c_hi)
                 ok = ok && mbar_wait(&s_full[st], (c >> 1) & 1, status, limit);
@@ -651,6 +651,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                 }
             }
             ++qi;
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             for (int j = 0; j < m.nblk && ok; ++j, ++kvc) {
                 if (lane == 0) {
                     const int st = kvc % kDqStages;
@@ -668,7 +669,6 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
     } else if (warp == 1 || warp == kDqThreads / 32 - 2) {
         // ------------------------------------------------------------------ MMA issuers
@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             if (m.nblk == 0) continue;
             if (warp == 1) {
                 ok = ok && mbar_wait(qt_full, qi & 1, status);
+                ok = warp_ok(ok);
                 for (int j = 0; j < m.nblk && ok; ++j, ++c) {
                     const int b = c & 1, st = c % kDqStages;
                     const uint32_t k_lo = kv_lo_ + (uint32_t)(st * ((2 * kKt) >> 4));
@@ -801,7 +802,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             next.nblk = next.ne = 0;
             if (w + (int)gridDim.x < nitems) next = take_item(++n, ok);
             row = load_numbers(next);
-            for (int j = 0; j < m.nblk && ok; ++j, ++c) {
+            for (int j = 0; j < m.nblk && warp_stays(ok); ++j, ++c) {
                 const int b = c & 1;
                 const int R0 = m.row_lo + j * BK;
                 const int c_lo = max(0, lo_r - R0), c_hi = min(BK, hi_r - R0 + 1);

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         const ET* dc = p.d_o + cchunk * 8;
         BT_DECL;
 #pragma unroll 1
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc; ++k) {                // (left by all lanes at the vote below)
             const int st = k & 1;
             BT_TOC(0);
             ok = ok && mbar_poll(&off_full[st], (k >> 1) & 1);
@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             ok = ok && mbar_poll(dq_full, k & 1);
             BT_EV(k, 13, warp == kWFlush && lane == 0);
             BT_TOC(1);
+            ok = warp_ok(ok);
             tc_fence_after();
             const int4 rec = s_rec[k & 15];
             // (rolled loops here and below: see the note on code size)
@@ -291,6 +292,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             const int seg = load_tile(p.ix, rec.z).seg0 + rec.w - __ldg(p.ix.tile_aux + rec.z).x / sched.run;
             float* slab = p.slabs + ((int64_t)seg * nsub + (rec.y - rec.z * nsub)) * (2 * KT * D) + d_idx;
             ok = ok && mbar_poll(acc_full, nflush & 1);
+            ok = warp_ok(ok);
             BT_TOC(3);
             tc_fence_after();
 #pragma unroll 1
@@ -603,7 +605,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         if (nloc > 1) fetch(entB, row0B, hB);
         BT_DECL;
 #pragma unroll 1
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc && warp_stays(ok); ++k) {
             const int st = k & 1;
             const float lse_r = lseA, delta_s = deltaA;
             const int c_lo = cloA, c_hi = chiA;

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
                     cp_async16(d + sw128_chunk_off(warp + (i0 + i) * kWLoad, lane & 7), src + ((int64_t)max(o[i], 0) << 3), o[i] >= 0);
             }
         };
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc; ++k) {                         // (left by all lanes at the vote below)
             const int slot = k % kRing;
             ok = ok && mbar_poll(&off_full[slot], (k / kRing) & 1);
             ok = ok && mbar_poll(q_empty, (k & 1) ^ 1);
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         int nflush = 0;
 #pragma unroll 1
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc; ++k) {                         // (left by all lanes at the vote below)
             ok = ok && mbar_poll(dq_full, k & 1);
             const int4 rec = s_rec[k & 7];
             ok = warp_ok(ok);
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(bwdwide::kThreads, 1) sel_bwd_wide(const SelBw
         if (nloc > 0) fetch_stats();
         uint8_t* my_stage = sP + (sb * 4 + quarter) * (32 * 128);        // 32 rows x 64 columns
 #pragma unroll 1
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc && warp_stays(ok); ++k) {
             const float lse_r = lse_n, delta_s = delta_n * p.scale;
             const int c_lo = lo_n, c_hi = hi_n;
             if (k + 1 < nloc) fetch_ent();

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         };
         if (sb < nloc) fetch(sb);
 #pragma unroll 1
-        for (int k = sb; k < nloc && ok; k += 2) {
+        for (int k = sb; k < nloc && warp_stays(ok); k += 2) {
             const int sbuf = k % C::NS;
             const uint32_t tS = tS0 + sbuf * BK;
             ok = ok && mbar_poll(&s_full[sbuf], (k / C::NS) & 1);
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         TileCursorT<false> cur(sched);
         int slab = 0;
 #pragma unroll 1
-        for (int k = 0; k < nloc && ok; ++k) {
+        for (int k = 0; k < nloc && warp_stays(ok); ++k) {
             const int ob = k % C::NO;
             ok = ok && mbar_poll(&o_full[ob], (k / C::NO) & 1);
             tc_fence_after();

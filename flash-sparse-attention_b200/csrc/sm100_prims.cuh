@@ -155,6 +155,13 @@ __device__ __forceinline__ bool warp_ok(bool ok) {
     return all;
 }
 
+// The condition of a loop in which the lanes of a warp meet (TMEM accesses, votes, shuffles) while each of them waits for itself: they
+// leave it together.  A lane that gave up alone would leave the others to wait for it without end.
+__device__ __forceinline__ bool warp_stays(bool& ok) {
+    ok = __all_sync(0xffffffffu, ok);
+    return ok;
+}
+
 // Barrier `id` of `threads` threads that tells whether v held for all of them.
 __device__ __forceinline__ bool bar_all(int id, int threads, bool v) {
     uint32_t all;

@@ -66,3 +66,78 @@ def test_a_product_waits_for_the_one_that_reads_what_it_overwrites(name, writes,
     after = text[text.index(reads):]
     commit = re.search(r"umma_commit\(&" + barrier + r"\[", after)
     assert commit and "mbar_" not in after[: commit.start()], f"{name}: {reads}"
+
+
+COLLECTIVE = r"tmem_ld|tmem_st|_sync\(|__syncwarp|__syncthreads|warp_ok|warp_stays|bar_all|bar\.sync"
+VOTE = r"warp_ok\(|warp_stays\(|bar_all\(|__syncthreads_and\(|= __shfl_sync\(0xffffffffu, ok "
+
+
+def closing(text, at):
+    """The place behind the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] in "({[") - (text[i] in ")}]")
+        if depth == 0:
+            return i + 1
+    raise ValueError("unbalanced")
+
+
+def inlined(text):
+    """The lambdas that wait or vote in the place of their calls."""
+    while True:
+        for m in re.finditer(r"auto (\w+) = \[&\]\([^)]*\)\s*\{", text):
+            end = closing(text, m.end() - 1)
+            body = text[m.end() - 1 : end]
+            if re.search(WAIT + "|" + VOTE, body):
+                break
+        else:
+            return text
+        rest = re.sub(r"(?<![\w.])" + m.group(1) + r"\((?=[^)]*\))", lambda c: body.replace("return", "") + " (", text[end + 1 :])
+        text = text[: m.start()] + rest
+
+
+def lanes_apart(text):
+    """Walks a source in order, a loop's body twice: the loops in which lanes meet, but which a lane whose wait ran out may leave alone."""
+    loops = []
+    events = re.compile(r"(?P<loop>(?:for|while) \()|(?P<vote>" + VOTE + r")|(?P<wait>" + WAIT + r")|(?P<leave>if \([^()]*!ok[^()]*\) (?:break|continue))"
+                        r"|(?P<other>\} else (?:if \(warp|\{\s*(?:if \(warp|bool ok|const int)))|(?P<fresh>bool ok(?:_wait)? = true)")
+
+    def walk(a, b, apart, owner):
+        """apart: lanes may differ on whether a wait ran out; owner: the innermost loop, whether lanes meet in it."""
+        while True:
+            m = events.search(text, a, b)
+            if not m:
+                return apart
+            a = m.end()
+            if m.group("vote"):
+                apart = False
+            elif m.group("wait"):
+                apart = True
+            elif m.group("fresh") or m.group("other"):
+                apart = False
+            elif m.group("leave"):
+                if apart and owner and owner[1]:
+                    loops.append(owner[0])
+            else:
+                head_end = closing(text, m.end() - 1)
+                head = text[m.start() : head_end]
+                brace = re.compile(r"\s*\{").match(text, head_end)
+                if not brace:
+                    continue
+                end = closing(text, brace.end() - 1)
+                me = (head, re.search(COLLECTIVE, head + text[head_end:end]) is not None)
+                for _ in range(2):
+                    if "warp_stays" in head:
+                        apart = False
+                    elif re.search(r"\bok\b|ok_wait", head) and me[1] and apart:
+                        loops.append(head)
+                    apart = walk(brace.end(), end, apart, me)       # (a loop that ends by its count ends without the vote in its head)
+                a = end
+
+    walk(0, len(text), False, None)
+    return loops
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_lanes_leave_a_loop_in_which_they_meet_together(name):
+    assert not lanes_apart(inlined(code(name)))
