@@ -515,6 +515,10 @@ struct RangeDqParams {
 constexpr int kDqThreads = 384;     // producer, S/dP issuer, 8 row warps, dQ issuer, item warp
 constexpr int kDqStages = 4;
 constexpr int kDqItems = 4;         // items known ahead
+// The item warp is ahead, so that its wait for a free entry lasts as long as an item: a tile of 64 K/V rows takes some 1200 cycles, and
+// 0.2 s would end it at 21 million rows.  This many cycles more for each tile of the longest item so far.
+constexpr uint32_t kDqTileClocks = 4096;
+static_assert(kMaxTokens / kRdBK * kDqTileClocks + FSA_WAIT_CLOCKS < (int64_t)1 << 32, "the counter comes round");
 
 // One work item of the dQ kernel: a tile of tokens x one KV head.
 struct DqItem {
@@ -621,11 +625,12 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
     if (warp == kDqThreads / 32 - 1) {
         // ------------------------------------------------------------------ items
         bool ok = true;
-        int n = 0;
+        int n = 0, longest = 0;
         for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x, ++n) {
             const DqItem m = dq_item(p, ntiles, w, lane);
-            ok = ok && mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status);
+            ok = ok && mbar_wait(&it_empty[n % kDqItems], ((n / kDqItems) & 1) ^ 1, status, FSA_WAIT_CLOCKS + longest * kDqTileClocks);
             ok = warp_ok(ok);
+            longest = max(longest, m.nblk);
             if (ok && lane == 0) {
                 s_item[(n % kDqItems) * 2] = make_int4(m.seq, m.tok0, m.ne, m.row_lo);
                 s_item[(n % kDqItems) * 2 + 1] = make_int4(m.nblk, m.h, 0, 0);

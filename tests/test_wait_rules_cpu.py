@@ -68,6 +68,16 @@ def test_a_product_waits_for_the_one_that_reads_what_it_overwrites(name, writes,
     assert commit and "mbar_" not in after[: commit.start()], f"{name}: {reads}"
 
 
+def test_the_wait_for_an_item_outlasts_the_longest_one():
+    """The item warp of the dQ kernel waits through a whole item, up to 2^25 K/V rows in tiles of 64 that take some 1200 cycles."""
+    text = code("range_dense.cu")
+    wait = re.search(WAIT + r"&it_empty\[n % kDqItems\][^;]*;", text).group(0)
+    more = re.search(r"FSA_WAIT_CLOCKS \+ longest \* kDqTileClocks", wait) and int(re.search(r"kDqTileClocks = (\d+)", text).group(1))
+    least = int(re.search(r"define FSA_WAIT_CLOCKS (\d+)u", open(os.path.join(CSRC, "sm100_prims.cuh")).read()).group(1))
+    assert (1 << 25) // 64 * 1200 < least + (1 << 25) // 64 * (more or 0) < 1 << 32
+    assert re.search(r"longest = max\(longest, m\.nblk\)", text)
+
+
 COLLECTIVE = r"tmem_ld|tmem_st|_sync\(|__syncwarp|__syncthreads|warp_ok|warp_stays|bar_all|bar\.sync"
 VOTE = r"warp_ok\(|warp_stays\(|bar_all\(|__syncthreads_and\(|= __shfl_sync\(0xffffffffu, ok "
 
