@@ -126,12 +126,13 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
     int* s_claim = reinterpret_cast<int*>(bars + 20);    // 16 bytes
     int4* s_item = reinterpret_cast<int4*>(bars + 22);   // [2 items][2]
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 30);
+    int* status = reinterpret_cast<int*>(bars + 30) + 1;     // of this CTA
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int* status = launch.p[blockIdx.z].status;
-    const uint32_t limit = wait_limit(status);
+    const uint32_t limit = wait_limit(launch.p[blockIdx.z].status);
     const int G = launch.p[0].G, TPT = launch.p[0].TPT;      // (the same for all problems)
     if (tid == 0) {
+        *status = kStatusOk;
         mbar_init(q_full, 1); mbar_init(q_empty, 1); mbar_init(o_free, 128);
         mbar_init(it_full, 1); mbar_init(it_empty, 5); mbar_init(claim, 1);
         for (int i = 0; i < 2; ++i) {
@@ -464,6 +465,8 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tbase, kCols);
+    // (a CTA has taken over items of every problem of the launch, and gave up those that it would have taken)
+    if (tid < kRdProblems && *status != kStatusOk && launch.p[tid].status) atomicMax(launch.p[tid].status, *status);
 }
 
 template <int D, typename ET>

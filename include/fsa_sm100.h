@@ -187,7 +187,8 @@ int fsa_range_attn_fwd_dense(const void* q, const void* k, const void* v, const 
                              int64_t q_stride_n, int64_t q_stride_h, int64_t k_stride_n, int64_t v_stride_n, float sm_scale,
                              void* o, int64_t o_stride_n, int64_t o_stride_h, float* lse, int32_t* status, void* stream);
 
-/* The same for up to three problems of one batch and head layout in one launch (the branches of a layer); arguments as above. */
+/* The same for up to three problems of one batch and head layout in one launch (the branches of a layer); arguments as above.
+ * A wait that runs out is recorded in the status words of all of them. */
 typedef struct {
     const void *q, *k, *v;
     const int32_t *cu_seqlens_q, *cu_seqlens_k, *kv_lo, *kv_hi;

@@ -78,6 +78,15 @@ def test_the_wait_for_an_item_outlasts_the_longest_one():
     assert re.search(r"longest = max\(longest, m\.nblk\)", text)
 
 
+def test_a_failed_launch_of_several_problems_says_so_in_the_words_of_all():
+    """A CTA of range_fwd_dense takes over items of any problem: one that gave up has left work of each of them undone."""
+    text = code("range_dense.cu")
+    kernel = text[text.index("range_fwd_dense(const") : text.index("static cudaError_t launch_rd")]
+    assert set(re.findall(WAIT + r"[^;]*?, (status), limit\)", kernel)) == {"status"} and re.search(r"int\* status = reinterpret_cast<int\*>\(bars", kernel)
+    assert "*status = kStatusOk;" in kernel[: kernel.index("__syncthreads")]
+    assert re.search(r"__syncthreads\(\);[^}]*if \(tid < kRdProblems && \*status != kStatusOk && launch\.p\[tid\]\.status\) atomicMax", kernel)
+
+
 COLLECTIVE = r"tmem_ld|tmem_st|_sync\(|__syncwarp|__syncthreads|warp_ok|warp_stays|bar_all|bar\.sync"
 VOTE = r"warp_ok\(|warp_stays\(|bar_all\(|__syncthreads_and\(|= __shfl_sync\(0xffffffffu, ok "
 
