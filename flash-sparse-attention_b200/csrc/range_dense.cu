@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
             const int lo_r = sees.x - m.row_lo, hi_r = min(sees.y, (int)launch.p[m.z].Nk - 1) - m.row_lo;      // rows past the end of K/V do not exist
             const int nblk = m.nblk;
             float m_ref = -INFINITY, l_run = 0.f;
-            for (int j = 0; j < nblk && warp_stays(ok); ++j, ++c) {
+            for (int j = 0; j < nblk; ++j, ++c) {          // (left by all lanes at the vote below)
                 const int st = c & 1;
                 const int c_lo = max(0, lo_r - j * BK), c_hi = min(BK, hi_r - j * BK + 1);      // visible columns [c_lo, c_hi)
                 ok = ok && mbar_wait(&s_full[st], (c >> 1) & 1, status, limit);
@@ -369,9 +369,10 @@ __global__ void __launch_bounds__(kRdThreads, 2) range_fwd_dense(const __grid_co
                     m_ref = m_blk;
                 }
                 // accumulator rows already hold products (j > 0): rescale them when any row of the warp changes reference
-                const bool scale_acc = __any_sync(0xffffffffu, raise && j > 0);
+                const bool scale_acc = __any_sync(0xffffffffu, (raise && j > 0) || !ok);
                 if (scale_acc) {
                     ok = ok && mbar_wait(&pv_done[(c - 1) & 1], ((c - 1) >> 1) & 1, status, limit);
+                    if (!warp_stays(ok)) break;
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < D; c0 += 32) {
@@ -810,14 +811,15 @@ __global__ void __launch_bounds__(kDqThreads, 1) range_bwd_dq_dense(const RangeD
             next.nblk = next.ne = 0;
             if (w + (int)gridDim.x < nitems) next = take_item(++n, ok);
             row = load_numbers(next);
-            for (int j = 0; j < m.nblk && warp_stays(ok); ++j, ++c) {
+            for (int j = 0; j < m.nblk; ++j, ++c) {        // (left by all lanes at the vote below)
                 const int b = c & 1;
                 const int R0 = m.row_lo + j * BK;
                 const int c_lo = max(0, lo_r - R0), c_hi = min(BK, hi_r - R0 + 1);
                 ok = ok && mbar_wait(&sdp_full[b], (c >> 1) & 1, status);
                 tc_fence_after();
                 uint32_t dd[HC / 2];
-                const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == BK);
+                const bool all_visible = __all_sync(0xffffffffu, ok && c_lo == 0 && c_hi == BK);
+                if (!all_visible && !warp_stays(ok)) break;
                 {
                     uint32_t sv[32], dv[32];
                     tmem_ld32(tbase + lane_off + b * 128 + cb, sv);

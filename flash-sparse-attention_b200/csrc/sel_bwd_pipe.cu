@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
         if (nloc > 1) fetch(entB, row0B, hB);
         BT_DECL;
 #pragma unroll 1
-        for (int k = 0; k < nloc && warp_stays(ok); ++k) {
+        for (int k = 0; k < nloc; ++k) {               // (left by all lanes at the vote below)
             const int st = k & 1;
             const float lse_r = lseA, delta_s = deltaA;
             const int c_lo = cloA, c_hi = chiA;
@@ -615,7 +615,8 @@ __global__ void __launch_bounds__(bwdpipe::kThreads, 1) sel_bwd_pipe(const SelBw
             if (k + 2 < nloc) fetch(entB, row0B, hB);
             BT_TOC(0);
             // most tiles are fully visible to all their rows (only a token's own block is cut by causality)
-            const bool all_visible = __all_sync(0xffffffffu, c_lo == 0 && c_hi == KT);
+            const bool all_visible = __all_sync(0xffffffffu, ok && c_lo == 0 && c_hi == KT);
+            if (!all_visible && !warp_stays(ok)) break;
             // dP comes first (its rows are gathered first): scale (dP - delta) is ready when S arrives
             ok = ok && mbar_poll(&dp_full[st], (k >> 1) & 1);
             tc_fence_after();

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
         };
         if (sb < nloc) fetch(sb);
 #pragma unroll 1
-        for (int k = sb; k < nloc && warp_stays(ok); k += 2) {
+        for (int k = sb; k < nloc; k += 2) {               // (left by all lanes at the vote below)
             const int sbuf = k % C::NS;
             const uint32_t tS = tS0 + sbuf * BK;
             ok = ok && mbar_poll(&s_full[sbuf], (k / C::NS) & 1);
@@ -382,7 +382,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) sel_fwd_main(const SelFwdParam
             // is read for its maximum, then the lower one, which stays, then (P of the lower half is in its place, over S) the upper one
             // again.  (Four 32-column reads twice over, one running maximum and sum: 140 -> 101 us for 21K ragged tokens x 4 heads.)
             constexpr int W = BK < 64 ? BK : 64;
-            const bool masked = __any_sync(0xffffffffu, c_lo > 0 || c_hi < BK);
+            const bool masked = __any_sync(0xffffffffu, c_lo > 0 || c_hi < BK || !ok);
+            if (masked && !warp_stays(ok)) break;
             uint32_t v[W];
             auto load = [&](int c0) {
                 tmem_ld32(tS + c0, *reinterpret_cast<uint32_t (*)[32]>(&v[0]));

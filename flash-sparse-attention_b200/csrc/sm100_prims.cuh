@@ -156,7 +156,8 @@ __device__ __forceinline__ bool warp_ok(bool ok) {
 }
 
 // The condition of a loop in which the lanes of a warp meet (TMEM accesses, votes, shuffles) while each of them waits for itself: they
-// leave it together.  A lane that gave up alone would leave the others to wait for it without end.
+// leave it together.  A lane that gave up alone would leave the others to wait for it without end.  (A loop that votes in each turn on
+// something else counts `!ok` there and asks this only then: a vote more between two tiles cost the row threads up to 1 %.)
 __device__ __forceinline__ bool warp_stays(bool& ok) {
     ok = __all_sync(0xffffffffu, ok);
     return ok;

@@ -160,3 +160,12 @@ def lanes_apart(text):
 @pytest.mark.parametrize("name", SOURCES)
 def test_lanes_leave_a_loop_in_which_they_meet_together(name):
     assert not lanes_apart(inlined(code(name)))
+
+
+@pytest.mark.parametrize("name,votes", [("range_dense.cu", ["scale_acc", "all_visible"]), ("sel_fwd.cu", ["masked"]), ("sel_bwd_pipe.cu", ["all_visible"])])
+def test_a_vote_that_stands_for_the_loops_counts_the_lanes_that_gave_up(name, votes):
+    """Where a warp votes in each turn for another reason, that vote tells too whether one on the waits is due."""
+    text = code(name)
+    for v in votes:
+        m = re.search(r"const bool " + v + r" = __(?:any_sync\(0xffffffffu, [^;]*\|\| !ok|all_sync\(0xffffffffu, ok &&[^;]*)\);", text)
+        assert m and re.match(r"\s*if \((?:" + v + r"\) \{\s*ok = ok && [^;]*;\s*if \(!warp_stays|!?" + v + r" && !warp_stays)\(ok\)\) break;", text[m.end():]), v
