@@ -388,7 +388,7 @@ static int sel_fwd_impl(const SelBounds& bd, int64_t Nk, const void* q, const vo
     a.opart = scratch;
     a.ml = (float2*)((char*)scratch + align_up(prow * D * 2, 1024));
     a.o = o; a.o_sn = o_sn; a.o_sh = o_sh; a.lse = lse;
-    a.kmap = &kmap; a.vmap = &vmap; a.qmap = nullptr; a.omap = nullptr;
+    a.kmap = &kmap; a.vmap = &vmap; a.omap = nullptr;
     a.bd = bd;
     if (BK <= 128) {
         rc = make_tile_map(&omap, scratch, dtype, prow, D, D, 32);

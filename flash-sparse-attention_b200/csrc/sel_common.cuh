@@ -137,30 +137,7 @@ __device__ __forceinline__ int2 block_rows(const int* __restrict__ ck, int B, in
     return make_int2(row0, min(BK, k1 - row0));
 }
 
-// Block of slot `sl` of token n, or -1.  List mode: a slot is usable when 0 <= id <= t_local / BK
-// (nsa_ref/ops/topk_sparse_attention.py:116-119).  Range mode: slot sl is the sl-th block touched by
-// [kv_lo[n], kv_hi[n]].
-__device__ __forceinline__ int entry_block(const int* __restrict__ cu, const SelBounds& bd, int B, int BK, int n, int sl,
-                                           const int* __restrict__ idrow, int* row0_out) {
-    const int b = find_seq(cu, B, n);
-    const int c = __ldg(cu + b);
-    const int ck = bd.cu_k ? __ldg(bd.cu_k + b) : c;
-    int id;
-    if (bd.kv_hi) {
-        const int lo = bd.kv_lo ? __ldg(bd.kv_lo + n) : ck, hi = __ldg(bd.kv_hi + n);
-        if (hi < lo) return -1;
-        id = (lo - ck) / BK + sl;
-        if (id > (hi - ck) / BK) return -1;
-    } else {
-        id = __ldg(idrow + sl);
-        if (id < 0 || id > (n - c) / BK) return -1;
-    }
-    *row0_out = ck + id * BK;
-    return ck / BK + b + id;
-}
-
-// The same, with everything that depends only on the token looked up once (one binary search per token instead of
-// one per slot).
+// What the blocks of a token's slots depend on, looked up once a token.
 struct TokenCtx {
     int c, ck, kb, lo, hi;    // sequence start (q rows), K/V start, global id of block 0, visible range (range mode)
     int ke;                   // K/V end of the sequence
@@ -179,6 +156,9 @@ __device__ __forceinline__ TokenCtx token_ctx(const int* __restrict__ cu, const 
     }
     return t;
 }
+// Block of slot `sl` of token n, or -1.  List mode: a slot is usable when 0 <= id <= t_local / BK
+// (nsa_ref/ops/topk_sparse_attention.py:116-119).  Range mode: slot sl is the sl-th block touched by
+// [kv_lo[n], kv_hi[n]].
 __device__ __forceinline__ int entry_block_ctx(const TokenCtx& t, const SelBounds& bd, int BK, int n, int sl, int id_list,
                                                int* row0_out) {
     int id;
@@ -206,16 +186,6 @@ __device__ __forceinline__ void visible_cols(const SelBounds& bd, int tok, int r
     c_hi = min(klim, hi - row0 + 1);
 }
 
-// largest i in [0, n) with off[i] <= x  (off ascending, off[0] = 0)
-__device__ __forceinline__ int upper_seg(const int* __restrict__ off, int n, int x) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (off[mid] <= x) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
 // Static tile schedule of a persistent grid: runs of `run` consecutive tiles are dealt to the
 // CTAs round-robin, so the whole grid advances through the tile list together (neighbouring
 // blocks of one kv head: their query rows stay in L2) while a CTA still reuses a resident K/V
@@ -233,11 +203,6 @@ struct TileScheduleT {
         // the last run may be short (nsub < grid: a CTA has at most one of its parts, as its own last)
         if (mine > 0 && (cta + (mine - 1) * grid) >> (PARTS ? lsub : 0) == NR - 1) nloc -= NR * run - total;
     }
-    __device__ __forceinline__ int tile(int k) const {
-        const int r = (k / run) * grid + cta;
-        return (PARTS ? r >> lsub : r) * run + (k % run);
-    }
-    __device__ __forceinline__ int sub(int k) const { return PARTS ? ((k / run) * grid + cta) & ((1 << lsub) - 1) : 0; }
 };
 using TileSchedule = TileScheduleT<false>;
 // Walks a CTA's tiles in order without a division per tile (a role of a warp-specialised kernel keeps one or two).

@@ -30,7 +30,6 @@ struct SelFwdArgs {
     void* o;
     int64_t o_sn, o_sh;
     float* lse;
-    const CUtensorMap* qmap;  // [N, Hq*D] box {64,1} for gather4; null when q's head stride != D
     const CUtensorMap* kmap;  // [N, Hk*D] box {64, BK}
     const CUtensorMap* vmap;
     const CUtensorMap* omap;  // [max_tiles * 128, D] box {64, 32} for the partial stores

@@ -213,16 +213,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap
         ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
-// TMA gather4: four rows (y0..y3) of a 2-D tensor, box {cols, 1}, land in four consecutive
-// 128-byte rows of the destination (swizzled like a tiled load).
-__device__ __forceinline__ void tma_gather4(uint32_t dst_smem, const CUtensorMap* map, int x, int y0, int y1, int y2, int y3,
-                                            uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-        "%6}], [%7];" ::"r"(dst_smem),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(smem_u32(bar))
-        : "memory");
-}
 // 2-D tiled store smem -> global (bulk async-group completion).  x and y must be non-negative.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src_smem) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
@@ -235,12 +225,6 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
                      reinterpret_cast<uint64_t>(map)),
                  "r"(x), "r"(y), "r"(z), "r"(src_smem)
-                 : "memory");
-}
-// Untiled copy global -> shared memory; both addresses and the size are multiples of 16 bytes.
-__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem), "l"(src), "r"(bytes),
-                 "r"(smem_u32(bar))
                  : "memory");
 }
 // L2 eviction policies for data with a known lifetime: evict_first for rows that are written once and read once much
